@@ -96,7 +96,9 @@ int trs_device_count(void);
 int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, int k_cols, int window,
                          int validate, void* stream, trs_spmm_plan** out_plan);
 int trs_spmm_plan_destroy(trs_spmm_plan* plan);
-/* Scratch the run needs for feature width F (partial sums of windows split across CTAs). */
+/* Scratch the run needs for feature width F: the partial sums of windows split across CTAs and, when
+ * F % 8 != 0, room for a copy of B with padded rows.  (A workspace that holds the partial sums only,
+ * trs_spmm_static_scratch_bytes, is accepted too: such widths are then gathered with 2-byte loads.) */
 int trs_spmm_workspace_bytes(const trs_spmm_plan* plan, int F, size_t* bytes);
 /* C[m_rows, F] = A' * B[k_cols, F]; fp16 inputs, fp32 accumulate; C fully written (no memset
  * needed), fp32 or fp16 per out_dtype.  Asynchronous on `stream`; allocates nothing. */

@@ -55,6 +55,10 @@ struct Upload {
         *dev = (const T*)d;
         return 0;
     }
+    void drop(void* d) {
+        for (void*& p : ptrs)
+            if (p && p == d) { cudaFree(d); p = nullptr; }
+    }
     template <class T>
     int raw(size_t n, T** dev) {
         *dev = nullptr;
@@ -220,9 +224,37 @@ int resident_chunks(const trs_resident* h, size_t out_bytes) {
 
 // Enqueue one call on the three streams; returns without waiting.  `timed` records the six
 // timing events of the synchronous entry.
+int resident_drain(trs_resident* h) {
+    cudaError_t e1 = cudaStreamSynchronize(h->s_in);
+    cudaError_t e2 = cudaStreamSynchronize(h->stream);
+    cudaError_t e3 = cudaStreamSynchronize(h->s_out);
+    if (e1 != cudaSuccess) return (int)e1;
+    if (e2 != cudaSuccess) return (int)e2;
+    if (e3 != cudaSuccess) return (int)e3;
+    return TRS_OK;
+}
+
+// Workspace for a width that needs more than max_dimN does (a padded copy of B): grown once, after the
+// calls in flight have left the old one.
+int resident_workspace(trs_resident* h, int dimN) {
+    size_t need = 0;
+    int rc = trs_spmm_workspace_bytes(h->plan, dimN, &need);
+    if (rc || need <= h->ws_bytes) return rc;
+    rc = resident_drain(h);
+    if (rc) return rc;
+    void* grown = nullptr;
+    rc = h->up.raw<unsigned char>(need, (unsigned char**)&grown);
+    if (rc) return rc;
+    h->up.drop(h->d_ws);
+    h->d_ws = grown;
+    h->ws_bytes = need;
+    return TRS_OK;
+}
+
 int resident_enqueue(trs_resident* h, const trs_half* rhs_host, void* out_host, int dimN, int out_dtype, bool timed) {
     const int si = (int)(h->seq % kSlots);
     int rc = slot_init(h, si);
+    if (!rc) rc = resident_workspace(h, dimN);
     if (rc) return rc;
     ResidentSlot& s = h->slot[si];
     const size_t elt = out_dtype == TRS_OUT_F16 ? 2 : 4;
@@ -260,16 +292,6 @@ int resident_enqueue(trs_resident* h, const trs_half* rhs_host, void* out_host, 
     if (timed) cudaEventRecord(h->t_ev[5], h->s_out);
     TRS_CUDA(cudaEventRecord(s.out_done, h->s_out));
     ++h->seq;
-    return TRS_OK;
-}
-
-int resident_drain(trs_resident* h) {
-    cudaError_t e1 = cudaStreamSynchronize(h->s_in);
-    cudaError_t e2 = cudaStreamSynchronize(h->stream);
-    cudaError_t e3 = cudaStreamSynchronize(h->s_out);
-    if (e1 != cudaSuccess) return (int)e1;
-    if (e2 != cudaSuccess) return (int)e2;
-    if (e3 != cudaSuccess) return (int)e3;
     return TRS_OK;
 }
 

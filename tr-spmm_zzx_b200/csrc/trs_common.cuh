@@ -95,6 +95,20 @@ __device__ __forceinline__ uint32_t smem_u32(const void* p) {
 __device__ __forceinline__ void cp_async16(uint32_t dst, const void* src, int src_bytes) {
     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(dst), "l"(src), "r"(src_bytes));
 }
+__device__ __forceinline__ void cp_async16(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;\n" ::"r"(dst), "l"(src));
+}
+template <int OFF>
+__device__ __forceinline__ void cp_async16_at(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0+%2], [%1], 16;\n" ::"r"(dst), "l"(src), "n"(OFF));
+}
+template <int OFF>
+__device__ __forceinline__ void ldmatrix_x4_trans_at(uint32_t addr, uint32_t& r0, uint32_t& r1, uint32_t& r2,
+                                                     uint32_t& r3) {
+    asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4+%5];\n"
+                 : "=r"(r0), "=r"(r1), "=r"(r2), "=r"(r3)
+                 : "r"(addr), "n"(OFF));
+}
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
 __device__ __forceinline__ void cp_async_wait() {

@@ -4,29 +4,29 @@
 // features of it.  A "k-step" is 16 columns of the window:
 //   * a packed 2:4 tile  (s_tile_column / s_packed_a / s_packed_meta, block_online.cpp:796-841)
 //     -> one mma.sp m16n8k16 per 8 features, or
-//   * a pair of dense 16x8 TC blocks (t_column / t_binary / t_value, block_online.cpp:444-540)
-//     -> one dense mma m16n8k16 per 8 features, or
-//   * 16 entries of the window's CSR remainder -> one dense mma m16n8k16 per 8 features.
-// The default kernel gives every item to ONE warp: the warp gathers the 16 B rows of a step with
-// 16-byte cp.async into its own shared-memory ring, feeds them to the tensor cores with
-// ldmatrix.trans and keeps the fp32 accumulators of all 16 x FS outputs in registers across the
-// item.  No block-wide barrier exists anywhere in the loop; measured on B200, the barrier per
-// k-step of a CTA-cooperative gather, not the bytes in flight, was what held the gather rate at
-// 8.7 TB/s where warp-private rings reach 14 TB/s on the same column stream.
-// The CSR remainder parts of the window (c_* / cs_* arrays, block_online.cpp:397-439; kernels
-// mGCNkernel.cu:976-1042, 1119-1171) run through the same pipeline: the plan expands them into
-// groups of 16 entries, a group's 16 columns are gathered like a tile's and multiplied by a
-// 16 x 16 A tile holding entry k in column k (the fallback kernel for unaligned operands adds
-// them with scalar loads instead), and C is written exactly once:
-// no memset, no atomics, no second output buffer, no add kernel (compare
-// mGCNkernel_online.cu:1589-1590, 1689-1712).  Heavy windows are cut into several items that
-// write fp32 partial sums to scratch; a second kernel adds them in a fixed order, so results are
-// bit-identical from run to run.
+//   * a pair of dense 16x8 TC blocks (t_column / t_binary / t_value, block_online.cpp:444-540), or
+//   * 16 entries of the window's CSR remainder (c_* / cs_* arrays, block_online.cpp:397-439; kernels
+//     mGCNkernel.cu:976-1042, 1119-1171), entry k in column k of a 16 x 16 tile
+//     -> one dense mma m16n8k16 per 8 features.
+// The plan lays the steps of every item out as one stream: 16 column ids per step (64 bytes, the
+// items one after the other), and for the dense steps the 16 x 16 A tile expanded in fragment order
+// (512 bytes, 16 per lane).  A kernel then needs nothing but a running step number.
+//
+// Every item belongs to one warp; where the whole matrix is too small to give every SM its warps, to the
+// four warps of a CTA (a quarter of the steps each, added through shared memory at the end).  A warp gathers the 16 B rows of a step with 16-byte cp.async
+// into its own shared-memory ring, feeds them to the tensor cores with ldmatrix.trans and keeps
+// the fp32 accumulators of all 16 x FS outputs in registers across the item.  No block-wide barrier
+// exists in the loop.  C is written exactly once: no memset, no atomics, no second output buffer,
+// no add kernel (compare mGCNkernel_online.cu:1589-1590, 1689-1712).  Heavy windows are cut into
+// several items that write fp32 partial sums to scratch; a second kernel adds them in a fixed order,
+// so results are bit-identical from run to run.
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 
 #include <string.h>
 
+#include <atomic>
+#include <type_traits>
 #include <mutex>
 #include <vector>
 
@@ -34,28 +34,15 @@
 
 namespace trs {
 
-constexpr int kStages = 4;           // CTA-cooperative kernels (fallback for unaligned inputs)
-constexpr int kIdxAhead = 2 * kStages - 2;  // column ids are fetched this many steps ahead
-constexpr int kIdxRing = 8;                 // slots of 16 column ids; >= kIdxAhead + 1
-constexpr int kARegionBytes = 768;   // sparse: 256 B A + 32 B meta; dense: 16 rows x 48 B
-constexpr int kDenseRowHalfs = 24;   // 48-byte row stride of the expanded dense A tile
-
-struct Item {        // 64 bytes: everything a warp / CTA needs to start
+struct Item {        // 32 bytes: everything a warp needs to start
     int window;      // window id
-    int step_begin;  // k-steps of the window this item covers
-    int step_end;
     int slot;        // -1: write C; >=0: write partial sums to scratch slot
-    int tile0;       // first packed tile of the window
-    int ntiles;      // packed tiles of the window (steps [0, ntiles) are tiles, the rest TC pairs)
-    int blk0;        // TC block range of the window
-    int blk_end;
-    int c_begin;     // long CSR parts this item adds (a split window's parts are spread over its items)
-    int c_end;
-    int cs_begin;    // short CSR parts this item adds
-    int cs_end;
-    int ce0;         // the same CSR entries as groups of 16 (plan-owned expansion): first group, count
-    int ce_n;
-    int pad[2];
+    int step0;       // first step of the item in the plan's step stream
+    int nsparse;     // steps [0, nsparse) are packed tiles, the rest dense 16 x 16 tiles
+    int nsteps;
+    int tile0;       // packed tile of step 0
+    int dense0;      // dense tile of step nsparse
+    int pad;
 };
 
 struct Heavy {
@@ -71,21 +58,25 @@ struct WindowRanges {
     int* c_end;
     int* cs_begin;   // short CSR parts per window
     int* cs_end;
-    int* ce_begin;   // first group of 16 expanded CSR entries per window ([W + 1], exclusive scan of ce_count)
-    int* ce_count;
 };
 
 struct KernelArgs {
-    trs_format f;
-    const Item* items;
+    const Item* items;             // longest first
     int n_items;
+    int w_begin, w_end;            // window range of this run (RANGE instances: items outside return at once)
+    const int* ids;                // [steps + kIdBlock][16] column ids of the step stream
+    const uint32_t* packed_a;      // [tiles][64]
+    const uint32_t* packed_meta;   // [tiles][8]
+    const uint4* dense;            // [dense steps][32] A tiles in fragment order, one uint4 per lane
     const __half* B;
     void* C;
-    float* scratch;
-    const __half* tc_dense;        // [blocks][16][8] expanded TC blocks (plan-owned)
-    const int* ce_col;             // [groups][16] column ids of the CSR remainder entries, -1 = padding (plan-owned)
-    const unsigned* ce_rv;         // [groups][16] fp16 value | local row << 16
-    int m_rows, k_cols, window, F, out_half;
+    float* scratch;                // [slots][16][ldS]
+    int ldb;                       // elements from one row of B to the next
+    int ldS;
+    int F;                         // features of C
+    int bchunks;                   // 16-byte chunks a row of B really has
+    int m_rows, window, out_half;
+    int vec_out;                   // rows of C are 16-byte aligned
     int relu;                      // 1: C = max(A'B, 0) (GCN layer epilogue)
     void* peers[8];                // fused exchange: the fp16 rows are written into every one of these
     int n_peers;                   //   [N_total, F] buffers (this GPU's and its NVLink peers'), 0 = off
@@ -107,85 +98,159 @@ __global__ void k_part_ranges(const int* __restrict__ key, const int* __restrict
     if (p == n - 1 || key[p + 1] / div != w) end[w] = hi;
 }
 
-// CSR remainder entries of a window (long parts first, then short parts), expanded at plan time
-// into groups of 16 entries - column id and (fp16 value, local row) - so that the warp kernel can
-// run them through its gather pipeline as k-steps of their own: 16 gathered B rows times a
-// 16 x 16 A tile that holds entry k in column k (one non-zero per column).
-__global__ void k_ce_count(trs_format f, WindowRanges wr, int num_windows) {
+// Entries of a window's CSR remainder: long parts first, then short parts.
+__device__ __forceinline__ int csr_entries(const trs_format& f, const WindowRanges& wr, int w, int pass) {
+    const int b = pass ? wr.cs_begin[w] : wr.c_begin[w], e = pass ? wr.cs_end[w] : wr.c_end[w];
+    const int* off = pass ? f.cs_row_offset : f.c_row_offset;
+    return e > b ? max(off[e] - off[b], 0) : 0;
+}
+struct WindowSteps {
+    int tiles, tc, ce;  // packed tiles, pairs of TC blocks, groups of 16 CSR entries
+};
+__device__ __forceinline__ WindowSteps window_steps(const trs_format& f, const WindowRanges& wr, int w) {
+    WindowSteps s;
+    s.tiles = w < f.num_windows ? f.s_window_tile_offset[w + 1] - f.s_window_tile_offset[w] : 0;
+    s.tc = (wr.blk_end[w] - wr.blk_begin[w] + 1) / 2;
+    s.ce = (csr_entries(f, wr, w, 0) + csr_entries(f, wr, w, 1) + 15) / 16;
+    return s;
+}
+
+// Per-window counts (arrays of W + 1, the last entry zero, scanned afterwards): steps and dense
+// steps first, then items, split-window flag and scratch slots, which depend on the total.
+constexpr int kWindowCounts = 5;
+enum { WC_STEPS, WC_DENSE, WC_ITEMS, WC_HEAVY, WC_SLOTS };
+__global__ void k_count_steps(trs_format f, WindowRanges wr, int num_windows, int* __restrict__ cnt) {
     int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w > num_windows) return;
-    int n = 0;
-    if (w < num_windows) {
-        if (wr.c_end[w] > wr.c_begin[w]) n += f.c_row_offset[wr.c_end[w]] - f.c_row_offset[wr.c_begin[w]];
-        if (wr.cs_end[w] > wr.cs_begin[w]) n += f.cs_row_offset[wr.cs_end[w]] - f.cs_row_offset[wr.cs_begin[w]];
-    }
-    wr.ce_count[w] = n > 0 ? (n + 15) / 16 : 0;
-}
-__global__ void k_ce_fill(trs_format f, WindowRanges wr, int num_windows, int window, int pass, long long capacity,
-                          int* __restrict__ ce_col, unsigned* __restrict__ ce_rv) {
-    const int n = pass ? f.parts_c_short : f.parts_c;
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    const int* roff = pass ? f.cs_row_offset : f.c_row_offset;
-    const int* rrow = pass ? f.cs_row : f.c_row;
-    const int* rcol = pass ? f.cs_column : f.c_column;
-    const __half* rval = (const __half*)(pass ? f.cs_value : f.c_value);
-    const int w = rrow[p] / window;
-    if (w < 0 || w >= num_windows) return;  // reported by validation
-    const int lr = rrow[p] - w * window;
-    long long dst = (long long)wr.ce_begin[w] * 16 + (roff[p] - (pass ? f.cs_row_offset[wr.cs_begin[w]] : f.c_row_offset[wr.c_begin[w]]));
-    if (pass && wr.c_end[w] > wr.c_begin[w]) dst += f.c_row_offset[wr.c_end[w]] - f.c_row_offset[wr.c_begin[w]];
-    for (int e = roff[p]; e < roff[p + 1]; ++e, ++dst) {
-        if (dst < 0 || dst >= capacity) return;
-        ce_col[dst] = rcol[e];
-        ce_rv[dst] = (unsigned)__half_as_ushort(rval[e]) | ((unsigned)lr << 16);
-    }
+    const size_t stride = (size_t)num_windows + 1;
+    WindowSteps s = {0, 0, 0};
+    if (w < num_windows) s = window_steps(f, wr, w);
+    cnt[WC_STEPS * stride + w] = s.tiles + s.tc + s.ce;
+    cnt[WC_DENSE * stride + w] = s.tc + s.ce;
 }
 
-__global__ void k_count_items(trs_format f, WindowRanges wr, int num_windows, int chunk, int* __restrict__ n_items,
-                              int* __restrict__ n_heavy, int* __restrict__ n_slots) {
-    int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= num_windows) return;
-    int tiles = 0;
-    if (w < f.num_windows) tiles = f.s_window_tile_offset[w + 1] - f.s_window_tile_offset[w];
-    int blocks = wr.blk_end[w] - wr.blk_begin[w];
-    int steps = tiles + (blocks + 1) / 2;
-    int items = steps <= chunk ? 1 : (steps + chunk - 1) / chunk;
-    n_items[w] = items;
-    n_heavy[w] = items > 1 ? 1 : 0;
-    n_slots[w] = items > 1 ? items : 0;
+// Longest run of steps one item takes.  An item should not be longer than the average share of a warp
+// slot (16 warps per SM at 128 features), or the longest ones are still running when the rest is
+// done; below 32 steps the extra partial sums cost more than the shorter tail gives, above 512 nothing
+// is left to gain.  Measured best at R-MAT scale 14 / 16 / 17 / 18 / 19 / 20 / 21, F = 128: 32 / 48 / 96 / 192 / 256 / 384 / 512
+// steps; 256 for all of them took 57 / 66 / 118 / 148 / 277 / 589 / 2080 us against 21 / 43 / 74 / 143 / 277 / 554 / 2049.
+// A matrix with less than six steps per warp slot gives every item four warps instead (few_items).
+constexpr int kWarpsPerSm = 16, kFewSteps = 6;
+__host__ __device__ __forceinline__ int item_steps(int total_steps, int sms) {
+    const int share = total_steps / (sms * kWarpsPerSm);
+    return share < kFewSteps ? 128 : min(max(share, 32), 512);
 }
 
-__global__ void k_fill_items(trs_format f, WindowRanges wr, int num_windows, int chunk,
-                             const int* __restrict__ item_off, const int* __restrict__ heavy_off,
-                             const int* __restrict__ slot_off, Item* __restrict__ items, Heavy* __restrict__ heavy) {
+__global__ void k_count_items(int num_windows, int chunk, int sms, const int* __restrict__ step_off, int* __restrict__ cnt) {
+    int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w > num_windows) return;
+    const size_t stride = (size_t)num_windows + 1;
+    if (chunk <= 0) chunk = item_steps(step_off[num_windows], sms);
+    int items = 0;
+    if (w < num_windows) items = max(1, (step_off[w + 1] - step_off[w] + chunk - 1) / chunk);
+    cnt[WC_ITEMS * stride + w] = items;
+    cnt[WC_HEAVY * stride + w] = items > 1 ? 1 : 0;
+    cnt[WC_SLOTS * stride + w] = items > 1 ? items : 0;
+}
+
+__global__ void k_fill_items(trs_format f, WindowRanges wr, int num_windows, const int* __restrict__ off,
+                             Item* __restrict__ items, Heavy* __restrict__ heavy) {
     int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w >= num_windows) return;
-    int tiles = 0;
-    if (w < f.num_windows) tiles = f.s_window_tile_offset[w + 1] - f.s_window_tile_offset[w];
-    int blocks = wr.blk_end[w] - wr.blk_begin[w];
-    int steps = tiles + (blocks + 1) / 2;
-    int n = item_off[w + 1] - item_off[w];
-    const int tile0 = (w < f.num_windows) ? f.s_window_tile_offset[w] : 0;
-    const int blk0 = wr.blk_begin[w], blk_end = wr.blk_end[w];
-    const int cb = wr.c_begin[w], cn = wr.c_end[w] - cb, sb = wr.cs_begin[w], sn = wr.cs_end[w] - sb;
-    const int g0 = wr.ce_begin[w], gn = wr.ce_count[w];
-    if (n == 1) {
-        items[item_off[w]] = Item{w, 0, steps, -1, tile0, tiles, blk0, blk_end, cb, cb + cn, sb, sb + sn, g0, gn, {0, 0}};
-        return;
-    }
-    // split evenly so that no item is much shorter than the others; the window's CSR parts are
-    // spread over the items the same way
-    int per = (steps + n - 1) / n;
+    const size_t stride = (size_t)num_windows + 1;
+    const int i0 = off[WC_ITEMS * stride + w], n = off[WC_ITEMS * stride + w + 1] - i0;
+    const int heavy0 = off[WC_HEAVY * stride + w], slot0 = off[WC_SLOTS * stride + w];
+    const int step0 = off[WC_STEPS * stride + w], steps = off[WC_STEPS * stride + w + 1] - step0;
+    const int dense0 = off[WC_DENSE * stride + w];
+    const int tile0 = w < f.num_windows ? f.s_window_tile_offset[w] : 0;
+    const int tiles = w < f.num_windows ? f.s_window_tile_offset[w + 1] - tile0 : 0;
+    // split evenly so that no item is much shorter than the others
+    const int per = (steps + n - 1) / n;
     for (int i = 0; i < n; ++i) {
-        int b = min(i * per, steps), e = min(b + per, steps);
-        items[item_off[w] + i] = Item{w, b, e, slot_off[w] + i, tile0, tiles, blk0, blk_end,
-                                      cb + (int)((long long)cn * i / n), cb + (int)((long long)cn * (i + 1) / n),
-                                      sb + (int)((long long)sn * i / n), sb + (int)((long long)sn * (i + 1) / n),
-                                      g0 + (int)((long long)gn * i / n),
-                                      (int)((long long)gn * (i + 1) / n) - (int)((long long)gn * i / n), {0, 0}};
+        const int b = min(i * per, steps), e = min(b + per, steps);
+        items[i0 + i] = Item{w, n > 1 ? slot0 + i : -1, step0 + b, min(max(tiles - b, 0), e - b), e - b, tile0 + b,
+                             dense0 + max(b - tiles, 0), 0};
     }
-    heavy[heavy_off[w]] = Heavy{w, slot_off[w], slot_off[w] + n};
+    if (n > 1) heavy[heavy0] = Heavy{w, slot0, slot0 + n};
+}
+
+// The step stream, one warp per item.  An unused column slot of a step repeats the step's first
+// column (its A entries are zero), so that the gather needs no special case; a step without any
+// column takes column 0.
+__global__ void k_fill_steps(trs_format f, WindowRanges wr, const Item* __restrict__ items, int n_items,
+                             const int* __restrict__ off, int num_windows, int window, int* __restrict__ ids,
+                             uint4* __restrict__ dense) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+    const int lane = threadIdx.x & 31;
+    if (i >= n_items) return;
+    const Item it = items[i];
+    const int w = it.window;
+    for (int j = 0; j < it.nsparse; ++j) {
+        int c = -1;
+        if (lane < 16) c = f.s_tile_column[(size_t)(it.tile0 + j) * 16 + lane];
+        const unsigned have = __ballot_sync(0xffffffffu, c >= 0);
+        const int dup = have ? __shfl_sync(0xffffffffu, c, __ffs(have) - 1) : 0;
+        if (lane < 16) ids[((size_t)it.step0 + j) * 16 + lane] = c >= 0 ? c : dup;
+    }
+    if (it.nsteps == it.nsparse) return;
+    const WindowSteps ws = window_steps(f, wr, w);
+    const int blk0 = wr.blk_begin[w], blk_end = wr.blk_end[w];
+    const int n_long = csr_entries(f, wr, w, 0), n_short = csr_entries(f, wr, w, 1);
+    const int rel = it.dense0 - off[WC_DENSE * ((size_t)num_windows + 1) + w];  // dense steps of the window before this item
+    const int g = lane >> 2, t = lane & 3;
+    for (int j = it.nsparse; j < it.nsteps; ++j) {
+        const int d = rel + j - it.nsparse;
+        int c = -1;
+        uint32_t a[4] = {0u, 0u, 0u, 0u};
+        if (d < ws.tc) {
+            const int b = blk0 + 2 * d + ((lane >> 3) & 1);
+            if (lane < 16 && b < blk_end) c = f.t_column[(size_t)b * 8 + (lane & 7)];
+            // fragment word q: row g + 8 (q & 1), columns 2t, 2t + 1 of block q >> 1
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const int bq = blk0 + 2 * d + (q >> 1);
+                if (bq >= blk_end) continue;
+                const unsigned long long lo = (unsigned long long)f.t_binary[(size_t)bq * 2];
+                const unsigned long long hi = (unsigned long long)f.t_binary[(size_t)bq * 2 + 1];
+                const unsigned long long m = (q & 1) ? hi : lo;
+                const __half* v = (const __half*)f.t_value + f.t_block_offset[bq];
+                const int bit = g * 8 + 2 * t;
+                int rank = __popcll(m & ((1ull << bit) - 1ull)) + ((q & 1) ? __popcll(lo) : 0);
+                if ((m >> bit) & 1ull) { a[q] = __half_as_ushort(v[rank]); ++rank; }
+                if ((m >> (bit + 1)) & 1ull) a[q] |= (uint32_t)__half_as_ushort(v[rank]) << 16;
+            }
+        } else {
+            // lane k < 16 finds entry k of the group: its part by binary search in the window's prefix
+            const int e = (d - ws.tc) * 16 + lane;
+            uint32_t ent = 0xffffu << 16;  // value | local row << 16; row 0xffff matches no row
+            if (lane < 16 && e < n_long + n_short) {
+                const bool is_short = e >= n_long;
+                const int* roff = is_short ? f.cs_row_offset : f.c_row_offset;
+                int lo = is_short ? wr.cs_begin[w] : wr.c_begin[w], hi = is_short ? wr.cs_end[w] : wr.c_end[w];
+                const int at = roff[lo] + (is_short ? e - n_long : e);
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (roff[mid] <= at) lo = mid; else hi = mid;
+                }
+                const int row = (is_short ? f.cs_row : f.c_row)[lo];
+                c = (is_short ? f.cs_column : f.c_column)[at];
+                ent = (uint32_t)((is_short ? f.cs_value : f.c_value)[at]) | ((uint32_t)(row - w * window) << 16);
+            }
+            // fragment word q: row g + 8 (q & 1), entries 2t + 8 (q >> 1) and the next one
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+                const uint32_t row = (uint32_t)(g + 8 * (q & 1));
+                const uint32_t e0 = __shfl_sync(0xffffffffu, ent, 2 * t + 8 * (q >> 1));
+                const uint32_t e1 = __shfl_sync(0xffffffffu, ent, 2 * t + 8 * (q >> 1) + 1);
+                if ((e0 >> 16) == row) a[q] = e0 & 0xffffu;
+                if ((e1 >> 16) == row) a[q] |= e1 << 16;
+            }
+        }
+        const unsigned have = __ballot_sync(0xffffffffu, c >= 0);
+        const int dup = have ? __shfl_sync(0xffffffffu, c, __ffs(have) - 1) : 0;
+        if (lane < 16) ids[((size_t)it.step0 + j) * 16 + lane] = c >= 0 ? c : dup;
+        dense[((size_t)it.dense0 + j - it.nsparse) * 32 + lane] = make_uint4(a[0], a[1], a[2], a[3]);
+    }
 }
 
 // Validation: every violated rule ORs one bit into *err.
@@ -205,12 +270,11 @@ __global__ void k_check_range(const int* __restrict__ a, long long n, int lo, in
     if (v < lo || v >= hi) atomicOr(err, bit);
 }
 // Launch-order class of an item: long items first, so that the last wave of the grid consists of
-// short ones (one item per warp: a long item that starts late would keep its SM busy alone).
+// short ones.  Classes of 8 steps (four classes over the whole range measured 4 - 6 % slower).
+constexpr int kClassBits = 6;
 __global__ void k_item_class(const Item* __restrict__ items, int n, unsigned char* __restrict__ cls) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const int steps = items[i].step_end - items[i].step_begin + items[i].ce_n;
-    cls[i] = (unsigned char)(31 - min(steps, 255) / 8);   // 32 classes of 8 steps (four classes measured 4 - 6 % slower, 64 or 256 the same)
+    if (i < n) cls[i] = (unsigned char)(63 - min(items[i].nsteps / 8, 63));
 }
 
 // The TC kernels read t_value[t_block_offset[b] + rank] with rank taken from the block's two
@@ -228,380 +292,198 @@ __global__ void k_check_sorted(const int* __restrict__ a, int n, int* err) {
 }
 
 // ----------------------------------------------------------------------------------------------
-// CTA-cooperative kernels
+// The kernel: one warp per work item, no block-wide synchronisation in the loop.
 // ----------------------------------------------------------------------------------------------
-// CSR remainder parts of the item and the single write of the item's result:
-// C rows (fp32 or fp16) or, for a slice of a split window, fp32 partial sums in scratch.
-// Accumulators are in mma fragment layout: acc[n][2h + i] = row g + 8h, feature fcol + 8n + i.
-__device__ __forceinline__ void add_csr_parts(float (&acc)[4][4], const Item& it, const KernelArgs& a, int fbase,
-                                              int wid, int g, int t) {
-    const int w = it.window;
-    const size_t F = (size_t)a.F;
-    // ---- CSR remainder parts of this item (scalar loop: this path serves unaligned inputs only) ---
-    {
-        const int fcol = fbase + wid * 32 + 2 * t;  // + 8*n
-        for (int pass = 0; pass < 2; ++pass) {
-            const int pb = pass ? it.cs_begin : it.c_begin;
-            const int pe = pass ? it.cs_end : it.c_end;
-            const int* roff = pass ? a.f.cs_row_offset : a.f.c_row_offset;
-            const int* rrow = pass ? a.f.cs_row : a.f.c_row;
-            const int* rcol = pass ? a.f.cs_column : a.f.c_column;
-            const __half* rval = (const __half*)(pass ? a.f.cs_value : a.f.c_value);
-            for (int p = pb; p < pe; ++p) {
-                const int lr = rrow[p] - w * a.window;
-                if ((lr & 7) != g || lr < 0 || lr >= 16) continue;
-                const int hi = lr >> 3;
-                for (int e = roff[p]; e < roff[p + 1]; ++e) {
-                    const int c = rcol[e];
-                    const float v = __half2float(rval[e]);
-                    const __half* brow = a.B + (size_t)c * F;
-#pragma unroll
-                    for (int n = 0; n < 4; ++n) {
-                        const int f = fcol + n * 8;
-                        const float x0 = f < a.F ? v * __half2float(brow[f]) : 0.f;
-                        const float x1 = f + 1 < a.F ? v * __half2float(brow[f + 1]) : 0.f;
-                        if (hi) { acc[n][2] += x0; acc[n][3] += x1; }
-                        else { acc[n][0] += x0; acc[n][1] += x1; }
-                    }
-                }
-            }
-        }
-    }
-}
+// What bounds it: one 16-byte-chunked row of B per (window, column) pair has to come through L2 - 27.5 GB
+// at R-MAT scale 21, F = 128, 1.83 ms for a kernel that does nothing else.  With four warps per
+// scheduler the rate at which a warp gets through its own instruction stream decides how close a
+// kernel comes; hence no predicates, no address arithmetic but one multiply-add per row, constant
+// ring offsets in the instructions, and a loop of its own for packed tiles: 95 instructions per step instead
+// of 223, 2.64 -> 2.05 ms at scale 21 (13.4 TB/s), 0.76 -> 0.55 ms at scale 20, 0.128 -> 0.097 ms clustered.
+//
+// FS = features per warp (a multiple of 16 up to 128; F > 128 adds feature slabs on gridDim.y).
+// Per k-step the warp copies the 16 gathered rows (FS * 2 bytes each) with FS / 16 cp.async
+// instructions of 16 bytes per lane into a stage of its own ring - rows unpadded, the 16-byte chunks
+// of a row swizzled by the row number so that ldmatrix is conflict-free.  Column ids come in blocks
+// of 8 steps (512 bytes, one cp.async per lane).  The A operand goes straight into registers
+// STAGES - 1 steps ahead, so the ring holds gathered rows only.
+constexpr int kIdBlock = 8;   // steps per block of column ids
 
-__device__ __forceinline__ void finish_item(float (&acc)[4][4], const Item& it, const KernelArgs& a, int fbase,
-                                            int wid, int g, int t) {
-    const int w = it.window;
-    const size_t F = (size_t)a.F;
-    add_csr_parts(acc, it, a, fbase, wid, g, t);
-    // ---- epilogue ----------------------------------------------------------------------------
-    const int fcol = fbase + wid * 32 + 2 * t;
-    if (it.slot >= 0) {
-        float* dst = a.scratch + (size_t)it.slot * 16 * F;
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            const int f = fcol + n * 8;
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                float* d = dst + (size_t)(g + 8 * h) * F + f;
-                if (f < a.F) d[0] = acc[n][2 * h];
-                if (f + 1 < a.F) d[1] = acc[n][2 * h + 1];
-            }
-        }
-        return;
-    }
-    if (a.relu) {
-#pragma unroll
-        for (int n = 0; n < 4; ++n)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[n][i] = fmaxf(acc[n][i], 0.f);
-    }
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-        const int lr = g + 8 * h;
-        const long long row = (long long)w * a.window + lr;
-        if (lr >= a.window || row >= a.m_rows) continue;
-#pragma unroll
-        for (int n = 0; n < 4; ++n) {
-            const int f = fcol + n * 8;
-            if (a.out_half) {
-                __half* d = (__half*)a.C + (size_t)row * F + f;
-                if (f + 1 < a.F && (a.F & 1) == 0) { const __half2 hv = __floats2half2_rn(acc[n][2 * h], acc[n][2 * h + 1]); __stcs((unsigned int*)d, *(const unsigned int*)&hv); }
-                else {
-                    if (f < a.F) d[0] = __float2half_rn(acc[n][2 * h]);
-                    if (f + 1 < a.F) d[1] = __float2half_rn(acc[n][2 * h + 1]);
-                }
-            } else {
-                float* d = (float*)a.C + (size_t)row * F + f;
-                if (f + 1 < a.F && (a.F & 1) == 0) __stcs((float2*)d, make_float2(acc[n][2 * h], acc[n][2 * h + 1]));
-                else {
-                    if (f < a.F) d[0] = acc[n][2 * h];
-                    if (f + 1 < a.F) d[1] = acc[n][2 * h + 1];
-                }
-            }
-        }
-    }
-}
-
-template <int WARPS>
-struct Tile {
-    static constexpr int FS = WARPS * 32;          // features per CTA
-    static constexpr int ROWB = FS * 2 + 16;       // padded B-row bytes: conflict-free ldmatrix
-    static constexpr int BBYTES = 16 * ROWB;
-    static constexpr int STAGE = BBYTES + kARegionBytes;
-    static constexpr int SMEM = STAGE * kStages + kIdxRing * 64;
-    static constexpr int THREADS = WARPS * 32;
-    static constexpr int CPR = FS / 8;             // 16-byte chunks per B row
-};
-
-template <int WARPS>
-__global__ void __launch_bounds__(WARPS * 32) k_window_spmm(const KernelArgs a) {
-    using T = Tile<WARPS>;
-    extern __shared__ __align__(128) unsigned char smem[];
-    const int tid = threadIdx.x;
-    const int lane = tid & 31;
-    const int wid = tid >> 5;
-    const int g = lane >> 2;   // fragment row group
-    const int t = lane & 3;    // thread in group
-    const int fbase = blockIdx.y * T::FS;
-
-    const Item it = a.items[blockIdx.x];
-    const int w = it.window;
-    const int tile0 = it.tile0, ntiles = it.ntiles, blk0 = it.blk0, blk_end = it.blk_end;
-    const int nsteps = it.step_end - it.step_begin;
-    const size_t F = (size_t)a.F;
-    int* idx_ring = (int*)(smem + T::STAGE * kStages);
-
-    float acc[4][4];
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
-
-    // Column ids of step m (relative to the item) -> ring slot m % kIdxRing, by threads 0..3.
-    auto issue_idx = [&](int m) {
-        if (tid >= 4 || m >= nsteps) return;
-        const int s = it.step_begin + m;
-        int* dst = idx_ring + (m % kIdxRing) * 16 + tid * 4;
-        if (s < ntiles) {
-            cp_async16(smem_u32(dst), a.f.s_tile_column + (size_t)(tile0 + s) * 16 + tid * 4, 16);
-        } else {
-            const int b = blk0 + 2 * (s - ntiles) + (tid >> 1);
-            if (b < blk_end) cp_async16(smem_u32(dst), a.f.t_column + (size_t)b * 8 + (tid & 1) * 4, 16);
-            else { dst[0] = -1; dst[1] = -1; dst[2] = -1; dst[3] = -1; }
-        }
-    };
-
-
-    auto issue = [&](int j) {  // j: step index relative to the item
-        const int s = it.step_begin + j;
-        unsigned char* st = smem + (j % kStages) * T::STAGE;
-        const int* cols = idx_ring + (j % kIdxRing) * 16;
-        // ---- B rows: plain 2-byte loads (any alignment, any F)
-        for (int i = tid; i < 16 * T::FS; i += T::THREADS) {
-            const int r = i / T::FS, fo = i % T::FS;
-            const int c = cols[r];
-            __half v = __float2half(0.f);
-            if (c >= 0 && fbase + fo < a.F) v = a.B[(size_t)c * F + fbase + fo];
-            *(__half*)(st + r * T::ROWB + fo * 2) = v;
-        }
-        // ---- A operand
-        unsigned char* as = st + T::BBYTES;
-        if (s < ntiles) {
-            const size_t tile = (size_t)(tile0 + s);
-            if (tid < 16) cp_async16(smem_u32(as + tid * 16), a.f.s_packed_a + tile * 64 + tid * 4, 16);
-            else if (tid < 18) cp_async16(smem_u32(as + 256 + (tid - 16) * 16), a.f.s_packed_meta + tile * 8 + (tid - 16) * 4, 16);
-        } else {
-            const int b0 = blk0 + 2 * (s - ntiles);
-            for (int i = tid; i < 256; i += T::THREADS) {
-                const int r = i >> 4, k = i & 15;
-                const int b = b0 + (k >> 3);
-                __half v = __float2half(0.f);
-                if (b < blk_end) {
-                    const unsigned long long lo = (unsigned long long)a.f.t_binary[(size_t)b * 2];
-                    const unsigned long long hi = (unsigned long long)a.f.t_binary[(size_t)b * 2 + 1];
-                    const int bit = (r & 7) * 8 + (k & 7);
-                    const unsigned long long m = r < 8 ? lo : hi;
-                    if ((m >> bit) & 1ull) {
-                        int rank = __popcll(m & ((1ull << bit) - 1ull));
-                        if (r >= 8) rank += __popcll(lo);
-                        v = ((const __half*)a.f.t_value)[(size_t)a.f.t_block_offset[b] + rank];
-                    }
-                }
-                ((__half*)as)[r * kDenseRowHalfs + k] = v;
-            }
-        }
-    };
-
-    auto compute = [&](int j) {
-        const int s = it.step_begin + j;
-        const unsigned char* st = smem + (j % kStages) * T::STAGE;
-        const unsigned char* as = st + T::BBYTES;
-        // ldmatrix row address of this lane: matrix m = lane/8 -> k rows (m&1)*8.., features (m>>1)*8..
-        const int m = lane >> 3;
-        const int krow = (lane & 7) + (m & 1) * 8;
-        const uint32_t baddr = smem_u32(st + krow * T::ROWB + (wid * 32 + (m >> 1) * 8) * 2);
-        if (s < ntiles) {
-            const uint2 av = *(const uint2*)(as + lane * 8);
-            const uint32_t meta = *(const uint32_t*)(as + 256 + g * 4);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t b0, b1, b2, b3;
-                ldmatrix_x4_trans(baddr + h * 32, b0, b1, b2, b3);
-                mma_sp_16816(acc[2 * h], av.x, av.y, b0, b1, meta);
-                mma_sp_16816(acc[2 * h + 1], av.x, av.y, b2, b3, meta);
-            }
-        } else {
-            const uint32_t a0 = *(const uint32_t*)(as + g * 48 + t * 4);
-            const uint32_t a1 = *(const uint32_t*)(as + (g + 8) * 48 + t * 4);
-            const uint32_t a2 = *(const uint32_t*)(as + g * 48 + 16 + t * 4);
-            const uint32_t a3 = *(const uint32_t*)(as + (g + 8) * 48 + 16 + t * 4);
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-                uint32_t b0, b1, b2, b3;
-                ldmatrix_x4_trans(baddr + h * 32, b0, b1, b2, b3);
-                mma_16816(acc[2 * h], a0, a1, a2, a3, b0, b1);
-                mma_16816(acc[2 * h + 1], a0, a1, a2, a3, b2, b3);
-            }
-        }
-    };
-
-    // ---- software pipeline over the k-steps ------------------------------------------------
-    // Two rings: column ids run kIdxAhead steps ahead of the compute, the gathered B rows
-    // kStages-1 steps.  Group g_k (the k-th commit after the id prologue) carries the B rows of
-    // step k and the ids of step k + kStages - 1; waiting until at most kStages-2 groups are
-    // pending at iteration j therefore completes both the rows of step j and the ids that the
-    // row gather issued in this iteration needs.
-#pragma unroll
-    for (int m = 0; m < kIdxAhead; ++m) issue_idx(m);
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncthreads();
-#pragma unroll
-    for (int j = 0; j < kStages - 1; ++j) {
-        if (j < nsteps) issue(j);
-        cp_async_commit();
-    }
-    for (int j = 0; j < nsteps; ++j) {
-        cp_async_wait<kStages - 2>();
-        __syncthreads();
-        issue_idx(j + kIdxAhead);
-        if (j + kStages - 1 < nsteps) issue(j + kStages - 1);
-        cp_async_commit();
-        compute(j);
-    }
-    cp_async_wait<0>();
-
-    finish_item(acc, it, a, fbase, wid, g, t);
-}
-
-// ----------------------------------------------------------------------------------------------
-// Default kernel: one warp per work item, no block-wide synchronisation.
-// ----------------------------------------------------------------------------------------------
-// FS = features per warp (32 / 64 / 128; F > FS adds feature slabs on gridDim.y).  Per k-step the
-// warp copies the 16 gathered rows (FS * 2 bytes each) with 16 / (256 / FS) cp.async instructions
-// of 16 bytes per lane into a stage of its own ring - rows unpadded, the 16-byte chunks of a row
-// swizzled by the row number so that ldmatrix is conflict-free - and the column ids of a later
-// step into a small id ring.  The A operand (8 bytes of packed values and one metadata word per
-// lane, or the four fragment words of two expanded TC blocks) is a coalesced stream read once; it
-// goes straight into registers STAGES - 1 steps ahead, so the ring holds gathered rows only:
-// 3 x 4 KB + 256 B per warp at FS = 128, which lets 16 one-warp CTAs (four per scheduler, 128
-// registers each) share an SM - shared memory would take 17, but the fifth warp of one scheduler
-// would cap every warp at 96 registers, which measured slower.  Commit groups give the ordering
-// (see the group accounting at the loop); lanes meet in one __syncwarp per step.
-// Requirements (checked by the launcher): F % 8 == 0, B / C / scratch and the tile arrays 16-byte
-// aligned.
 template <int FS, int STAGES>
 struct WarpTile {
     static constexpr int NT = FS / 8;               // n-tiles (8 features) per warp
     static constexpr int CPR = FS / 8;              // 16-byte chunks per gathered row
-    static constexpr int RPI = 32 / CPR;            // rows one cp.async warp-instruction covers
-    static constexpr int NCP = 16 / RPI;            // cp.async instructions per lane and step
+    static constexpr int NCP = CPR / 2;             // cp.async instructions per lane and step
+    static constexpr bool POW2 = (CPR & (CPR - 1)) == 0;
     static constexpr int ROWB = FS * 2;             // no padding: the chunks of a row are swizzled
-    static constexpr int STAGE = 16 * ROWB;         // the B rows only; the A operand rides in registers
-    static constexpr int IDA = 2 * STAGES - 2;      // ids run this many steps ahead
-    static constexpr int RING = IDA <= 4 ? 4 : 8;   // id ring slots (64 B each), >= IDA
-    static constexpr int SMEM = STAGE * STAGES + RING * 64;
-    static_assert(STAGES >= 2 && STAGES <= 4, "id ring holds 8 steps");
+    static constexpr int STAGE = 16 * ROWB;
+    static constexpr int AHEAD = STAGES - 1;        // rows and A operand run this many steps ahead
+    static constexpr int IDS = 2 * kIdBlock * 64;
+    static constexpr int SMEM = STAGE * STAGES + IDS;
+    static_assert(FS % 16 == 0 && FS <= 128 && STAGES >= 2 && AHEAD <= kIdBlock, "");
     static_assert(SMEM >= 16 * (FS * 4 + 16), "the epilogue stages a 16 x FS fp32 tile in the ring");
     // chunk c of row r sits at position c ^ swz(r): the 8 rows one ldmatrix phase reads land in 8
-    // different 16-byte bank groups (rows of 64 B share a 128-byte line in pairs)
-    __device__ static constexpr int swz(int r) { return FS == 32 ? ((r >> 1) & 3) : (r & 7); }
+    // different 16-byte bank groups (a row is FS / 8 chunks long; an odd multiple of 2 chunks needs one
+    // swizzle bit, an odd multiple of 4 two, a multiple of 8 three)
+    __device__ static constexpr int swz(int r) {
+        return (FS / 16) & 1 ? ((r >> 2) & 1) : ((FS / 32) & 1 ? ((r >> 1) & 3) : (r & 7));
+    }
 };
 
-// Epilogue of a warp-owned item.  Accumulators are in mma fragment layout: acc[n][2h + i] = row
-// g + 8h, feature fbase + 8n + 2t + i.  The result tile is staged in the warp's (drained) ring and
-// leaves in 16-byte pieces of whole rows: fp32 partial sums to a scratch slot, or fp16 / fp32
-// rows of C, or fp16 rows into every peer buffer of the fused exchange.
+// Rows of the item's result leave the warp's (drained) ring: `tile` holds 16 rows of FS fp32 (or fp16
+// when HALF) with the given pitch.  Called by `nthreads` threads numbered `tid`.
 template <int FS>
-__device__ __forceinline__ void finish_item_warp(float (&acc)[FS / 8][4], const Item& it, const KernelArgs& a, int fbase,
-                                                 int lane, unsigned char* ring) {
-    constexpr int NT = FS / 8;
-    const int g = lane >> 2, t = lane & 3;
+__device__ __forceinline__ void store_rows(const unsigned char* tile, bool half_tile, const Item& it, const KernelArgs& a,
+                                           int fbase, int tid, int nthreads) {
     const bool partial = it.slot >= 0;
-    if (a.relu && !partial) {
-#pragma unroll
-        for (int n = 0; n < NT; ++n)
-#pragma unroll
-            for (int i = 0; i < 4; ++i) acc[n][i] = fmaxf(acc[n][i], 0.f);
-    }
-    const bool half_out = !partial && (a.out_half || a.n_peers > 0);
-    if (half_out) {
-        constexpr int PITCH = FS * 2 + 16;
-#pragma unroll
-        for (int n = 0; n < NT; ++n)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                *(__half2*)(ring + (g + 8 * h) * PITCH + (8 * n + 2 * t) * 2) = __floats2half2_rn(acc[n][2 * h], acc[n][2 * h + 1]);
-        __syncwarp();
-        constexpr int CPR = FS / 8;
-        for (int c = lane; c < 16 * CPR; c += 32) {
-            const int lr = c / CPR, ch = c % CPR;
-            const int f = fbase + ch * 8;
-            const long long row = (long long)it.window * a.window + lr;
-            if (lr >= a.window || row >= a.m_rows || f >= a.F) continue;
-            const uint4 v = *(const uint4*)(ring + lr * PITCH + ch * 16);
-            if (a.n_peers > 0) {
-                const size_t off = (size_t)(a.peer_row0 + row) * (size_t)a.F + f;
-                for (int d = 0; d < a.n_peers; ++d) *(uint4*)((__half*)a.peers[d] + off) = v;
-            } else {
-                __stcs((uint4*)((__half*)a.C + (size_t)row * a.F + f), v);
+    if (half_tile) {
+        constexpr int PITCH = FS * 2 + 16, CPR = FS / 8;
+        if (a.vec_out) {
+            for (int c = tid; c < 16 * CPR; c += nthreads) {
+                const int lr = c / CPR, ch = c % CPR;
+                const int f = fbase + ch * 8;
+                const long long row = (long long)it.window * a.window + lr;
+                if (lr >= a.window || row >= a.m_rows || f >= a.F) continue;
+                const uint4 v = *(const uint4*)(tile + lr * PITCH + ch * 16);
+                if (a.n_peers > 0) {
+                    const size_t off = (size_t)(a.peer_row0 + row) * (size_t)a.F + f;
+                    for (int d = 0; d < a.n_peers; ++d) *(uint4*)((__half*)a.peers[d] + off) = v;
+                } else {
+                    __stcs((uint4*)((__half*)a.C + (size_t)row * a.F + f), v);
+                }
+            }
+        } else {
+            for (int c = tid; c < 16 * FS; c += nthreads) {
+                const int lr = c / FS, f = fbase + c % FS;
+                const long long row = (long long)it.window * a.window + lr;
+                if (lr >= a.window || row >= a.m_rows || f >= a.F) continue;
+                ((__half*)a.C)[(size_t)row * a.F + f] = *(const __half*)(tile + lr * PITCH + (c % FS) * 2);
             }
         }
-    } else {
-        constexpr int PITCH = FS * 4 + 16;
-#pragma unroll
-        for (int n = 0; n < NT; ++n)
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-                *(float2*)(ring + (g + 8 * h) * PITCH + (8 * n + 2 * t) * 4) = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
-        __syncwarp();
-        constexpr int CPR = FS / 4;
-        float* dst = partial ? a.scratch + (size_t)it.slot * 16 * (size_t)a.F : (float*)a.C;
-        for (int c = lane; c < 16 * CPR; c += 32) {
+        return;
+    }
+    constexpr int PITCH = FS * 4 + 16, CPR = FS / 4;
+    if (partial || a.vec_out) {
+        float* dst = partial ? a.scratch + (size_t)it.slot * 16 * (size_t)a.ldS : (float*)a.C;
+        const int ld = partial ? a.ldS : a.F;
+        for (int c = tid; c < 16 * CPR; c += nthreads) {
             const int lr = c / CPR, ch = c % CPR;
             const int f = fbase + ch * 4;
             const long long row = (long long)it.window * a.window + lr;
-            if (f >= a.F) continue;
+            if (f >= ld) continue;
             if (!partial && (lr >= a.window || row >= a.m_rows)) continue;
-            const float4 v = *(const float4*)(ring + lr * PITCH + ch * 16);
-            float4* d = (float4*)(dst + (partial ? (size_t)lr : (size_t)row) * a.F + f);
+            const float4 v = *(const float4*)(tile + lr * PITCH + ch * 16);
+            float4* d = (float4*)(dst + (partial ? (size_t)lr : (size_t)row) * ld + f);
             if (partial) *d = v;
             else __stcs(d, v);
+        }
+    } else {
+        for (int c = tid; c < 16 * FS; c += nthreads) {
+            const int lr = c / FS, f = fbase + c % FS;
+            const long long row = (long long)it.window * a.window + lr;
+            if (lr >= a.window || row >= a.m_rows || f >= a.F) continue;
+            ((float*)a.C)[(size_t)row * a.F + f] = *(const float*)(tile + lr * PITCH + (c % FS) * 4);
         }
     }
 }
 
-template <int FS, int STAGES, int MINB>
-__global__ void __launch_bounds__(32, MINB) k_window_spmm_warp(const KernelArgs a) {
+// Accumulators are in mma fragment layout: acc[n][2h + i] = row g + 8h, feature 8n + 2t + i.
+template <int FS>
+__device__ __forceinline__ void stage_acc(const float (&acc)[FS / 8][4], bool half_tile, unsigned char* tile, int lane) {
+    const int g = lane >> 2, t = lane & 3;
+#pragma unroll
+    for (int n = 0; n < FS / 8; ++n)
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            if (half_tile) *(__half2*)(tile + (g + 8 * h) * (FS * 2 + 16) + (8 * n + 2 * t) * 2) = __floats2half2_rn(acc[n][2 * h], acc[n][2 * h + 1]);
+            else *(float2*)(tile + (g + 8 * h) * (FS * 4 + 16) + (8 * n + 2 * t) * 4) = make_float2(acc[n][2 * h], acc[n][2 * h + 1]);
+        }
+}
+
+// 8 features of a B row that does not start on a 16-byte boundary
+__device__ __forceinline__ uint4 load_unaligned8(const __half* p, int n) {
+    unsigned short v[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) v[i] = i < n ? __ldg((const unsigned short*)p + i) : (unsigned short)0;
+    return make_uint4(v[0] | (uint32_t)v[1] << 16, v[2] | (uint32_t)v[3] << 16, v[4] | (uint32_t)v[5] << 16,
+                      v[6] | (uint32_t)v[7] << 16);
+}
+
+template <int N, int I = 0, class Fn>
+__device__ __forceinline__ void static_for(Fn&& fn) {
+    if constexpr (I < N) {
+        fn(std::integral_constant<int, I>());
+        static_for<N, I + 1>(fn);
+    }
+}
+template <int FS, int BASE, bool SPARSE, int H = 0>
+__device__ __forceinline__ void compute_steps(float (&acc)[FS / 8][4], const uint32_t (&laddr)[4], const uint4& av) {
+    if constexpr (H < FS / 16) {
+        uint32_t b0, b1, b2, b3;
+        ldmatrix_x4_trans_at<(H >> 2) * 128 + BASE>(laddr[H & 3], b0, b1, b2, b3);
+        if constexpr (SPARSE) {
+            mma_sp_16816(acc[2 * H], av.x, av.y, b0, b1, av.z);
+            mma_sp_16816(acc[2 * H + 1], av.x, av.y, b2, b3, av.z);
+        } else {
+            mma_16816(acc[2 * H], av.x, av.y, av.z, av.w, b0, b1);
+            mma_16816(acc[2 * H + 1], av.x, av.y, av.z, av.w, b2, b3);
+        }
+        compute_steps<FS, BASE, SPARSE, H + 1>(acc, laddr, av);
+    }
+}
+
+// WPI warps share an item (each takes a contiguous share of its steps, the shares are added in
+// warp order at the end).  ALIGNED: rows of B start on 16-byte boundaries; otherwise they are
+// gathered with 2-byte loads (callers that can neither align B nor lend memory for a padded copy).
+template <int FS, int STAGES, int WPI, int MINB, bool ALIGNED, bool RANGE>
+__global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const KernelArgs a) {
     using T = WarpTile<FS, STAGES>;
-    extern __shared__ __align__(128) unsigned char smem[];
-    const int lane = threadIdx.x;
-    const int g = lane >> 2;
+    extern __shared__ __align__(128) unsigned char smem_all[];
+    const int lane = threadIdx.x & 31;
+    const int wid = WPI > 1 ? threadIdx.x >> 5 : 0;
+    unsigned char* const smem = smem_all + wid * T::SMEM;
     const int fbase = blockIdx.y * FS;
 
     const Item it = a.items[blockIdx.x];
-    const int nmain = it.step_end - it.step_begin;
-    const int nsparse = min(max(it.ntiles - it.step_begin, 0), nmain);   // steps [0, nsparse) are packed tiles,
-    const int nsteps = nmain + it.ce_n;                                  // [nsparse, nmain) TC pairs, the rest CSR groups
+    if constexpr (RANGE) {   // a test in the whole-matrix instance costs up to 20 % (it delays the first ids of short items)
+        if (it.window < a.w_begin || it.window >= a.w_end) return;
+    }
+    int first = 0, nsteps = it.nsteps;
+    if constexpr (WPI > 1) {
+        const int per = (it.nsteps + WPI - 1) / WPI;
+        first = min(wid * per, it.nsteps);
+        nsteps = min(first + per, it.nsteps) - first;
+    }
+    const int nsparse = min(max(it.nsparse - first, 0), nsteps);
+    const int* const ids = a.ids + ((size_t)it.step0 + first) * 16;
+    const uint32_t* const pa = a.packed_a + (size_t)(it.tile0 + first) * 64 + lane * 2;
+    const uint32_t* const pm = a.packed_meta + (size_t)(it.tile0 + first) * 8 + (lane >> 2);
+    const uint4* const pd = a.dense + ((long long)it.dense0 + max(first - it.nsparse, 0) - nsparse) * 32 + lane;
 
     const uint32_t smem0 = smem_u32(smem);
-    const uint32_t ring0 = smem0 + T::STAGE * STAGES;
-    const unsigned char* ringp = smem + T::STAGE * STAGES;
+    constexpr int ids_at = T::STAGE * STAGES;
 
-    // gather role of this lane: chunk `ch` of rows sub * NCP + k, k = 0 .. NCP-1
-    const int ch = lane % T::CPR, sub = lane / T::CPR;
-    const uint32_t pitch16 = (uint32_t)a.F >> 3;             // 16-byte units per B row
-    const uint32_t chunk16 = ((uint32_t)fbase >> 3) + ch;    // this lane's chunk inside a row
-    const bool fin = fbase + ch * 8 < a.F;
-    const uint4* Bq = (const uint4*)a.B;
-    const uint32_t dst0 = smem0 + (sub * T::NCP) * T::ROWB;
+    // gather role of this lane: T::NCP pieces of 16 bytes, piece k = chunk pc[k] of row pr[k]
+    int pr[T::NCP], pc[T::NCP];
+    uint32_t pdst[T::NCP];
+#pragma unroll
+    for (int k = 0; k < T::NCP; ++k) {
+        if (T::POW2) { pr[k] = lane / T::CPR * T::NCP + k; pc[k] = lane % T::CPR; }
+        else { pr[k] = (k * 32 + lane) / T::CPR; pc[k] = (k * 32 + lane) % T::CPR; }
+        pdst[k] = smem0 + pr[k] * T::ROWB + ((pc[k] ^ T::swz(pr[k])) << 4);
+    }
+    const uint32_t pitch = (uint32_t)a.ldb * 2u;
+    // a chunk beyond the end of the row repeats the last one; its features are not stored
+    const unsigned char* src0[T::POW2 ? 1 : T::NCP];
+#pragma unroll
+    for (int k = 0; k < (T::POW2 ? 1 : T::NCP); ++k)
+        src0[k] = (const unsigned char*)a.B + (size_t)(min(fbase / 8 + pc[k], a.bchunks - 1)) * 16;
+    auto src_of = [&](int k) -> const unsigned char* { return src0[T::POW2 ? 0 : k]; };
     // ldmatrix role: matrix lane / 8 -> k rows (m & 1) * 8 .., features (m >> 1) * 8 ..
-    const int mtx = lane >> 3;
-    const int lrow = (lane & 7) + (mtx & 1) * 8;
-    const uint32_t boff = smem0 + lrow * T::ROWB;
-    const int lswz = T::swz(lrow), lchunk = mtx >> 1;
-    const int t = lane & 3;
+    const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lchunk = lane >> 4;
+    uint32_t laddr[4];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) laddr[q] = smem0 + lrow * T::ROWB + (((2 * q + lchunk) ^ T::swz(lrow)) << 4);
 
     float acc[T::NT][4];
 #pragma unroll
@@ -609,160 +491,162 @@ __global__ void __launch_bounds__(32, MINB) k_window_spmm_warp(const KernelArgs 
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 
-    auto issue_idx = [&](int m) {
-        if (lane < 4 && m < nsteps) {
-            const int s = it.step_begin + m;
-            const uint32_t dst = ring0 + (m & (T::RING - 1)) * 64 + lane * 16;
-            if (m >= nmain) {
-                cp_async16(dst, a.ce_col + (size_t)(it.ce0 + m - nmain) * 16 + lane * 4, 16);
-            } else if (s < it.ntiles) {
-                cp_async16(dst, a.f.s_tile_column + (size_t)(it.tile0 + s) * 16 + lane * 4, 16);
-            } else {
-                const int b = it.blk0 + 2 * (s - it.ntiles) + (lane >> 1);
-                if (b < it.blk_end) cp_async16(dst, a.f.t_column + (size_t)b * 8 + (lane & 1) * 4, 16);
-                else *(int4*)(smem + T::STAGE * STAGES + (m & (T::RING - 1)) * 64 + lane * 16) = make_int4(-1, -1, -1, -1);
-            }
-        }
+    auto issue_ids = [&](int blk) {   // ids of steps 8 blk .. 8 blk + 7 (the array ends with a spare block)
+        cp_async16(smem0 + ids_at + (blk & 1) * (kIdBlock * 64) + lane * 16, ids + blk * (kIdBlock * 16) + lane * 4);
     };
-
-    auto issue = [&](int j, int stage) {
-        const int* cols = (const int*)(ringp + (j & (T::RING - 1)) * 64) + sub * T::NCP;
+    auto gather = [&](int j, auto stage) {
+        const unsigned char* idp = smem + ids_at + (j & (2 * kIdBlock - 1)) * 64;
         int c[T::NCP];
-        if constexpr (T::NCP == 8) {
-            const int4 x = *(const int4*)cols, y = *(const int4*)(cols + 4);
-            c[0] = x.x; c[1] = x.y; c[2] = x.z; c[3] = x.w;
-            c[4] = y.x; c[5] = y.y; c[6] = y.z; c[7] = y.w;
-        } else if constexpr (T::NCP == 4) {
-            const int4 x = *(const int4*)cols;
-            c[0] = x.x; c[1] = x.y; c[2] = x.z; c[3] = x.w;
+        if constexpr (T::POW2 && T::NCP >= 4) {
+#pragma unroll
+            for (int k = 0; k < T::NCP; k += 4) {
+                const int4 x = *(const int4*)(idp + pr[k] * 4);
+                c[k] = x.x; c[k + 1] = x.y; c[k + 2] = x.z; c[k + 3] = x.w;
+            }
         } else {
-            const int2 x = *(const int2*)cols;
-            c[0] = x.x; c[1] = x.y;
+#pragma unroll
+            for (int k = 0; k < T::NCP; ++k) c[k] = *(const int*)(idp + pr[k] * 4);
         }
-        const uint32_t d = dst0 + stage * T::STAGE;
 #pragma unroll
         for (int k = 0; k < T::NCP; ++k) {
-            const uint32_t o = (uint32_t)max(c[k], 0) * pitch16 + chunk16;
-            cp_async16(d + k * T::ROWB + ((ch ^ T::swz(sub * T::NCP + k)) << 4), Bq + o, (c[k] >= 0 && fin) ? 16 : 0);
+            if constexpr (ALIGNED) {
+                cp_async16_at<decltype(stage)::value * T::STAGE>(pdst[k], src_of(k) + (unsigned long long)(uint32_t)c[k] * pitch);
+            } else {
+                const int f = fbase + pc[k] * 8;
+                *(uint4*)(smem + (pdst[k] - smem0) + decltype(stage)::value * T::STAGE) = load_unaligned8(a.B + (size_t)c[k] * a.ldb + f, a.F - f);
+            }
         }
     };
-
-    // A operand of step j, straight into registers (a coalesced stream, read once): a packed tile
-    // gives this lane its 8 bytes of values (x, y) and its metadata word (z); a pair of TC blocks
-    // gives the four fragment words of the dense 16 x 16 tile
+    // A operand of step j: a packed tile gives this lane its 8 bytes of values (x, y) and its metadata
+    // word (z), a dense tile the four fragment words
     auto load_a = [&](int j) -> uint4 {
-        uint4 r = make_uint4(0u, 0u, 0u, 0u);
-        if (j >= nsteps) return r;
-        const int s = it.step_begin + j;
-        if (j >= nmain) {  // entries 2t, 2t+1, 2t+8, 2t+9 of the group, as stored (value | row << 16)
-            const unsigned* rv = a.ce_rv + (size_t)(it.ce0 + j - nmain) * 16 + 2 * t;
-            const uint2 lo = __ldg((const uint2*)rv), hi = __ldg((const uint2*)(rv + 8));
-            r = make_uint4(lo.x, lo.y, hi.x, hi.y);
-        } else if (s < it.ntiles) {
-            const size_t tile = (size_t)(it.tile0 + s);
-            const uint2 v = __ldg((const uint2*)(a.f.s_packed_a + tile * 64) + lane);
-            r.x = v.x; r.y = v.y;
-            r.z = (uint32_t)__ldg(a.f.s_packed_meta + tile * 8 + g);
+        uint4 r;
+        if (j < nsparse) {
+            const uint2 v = __ldg((const uint2*)(pa + (size_t)j * 64));
+            r = make_uint4(v.x, v.y, __ldg(pm + (size_t)j * 8), 0u);
         } else {
-            const int b = it.blk0 + 2 * (s - it.ntiles);
-            const uint32_t* d0 = (const uint32_t*)(a.tc_dense + (size_t)b * 128);
-            r.x = __ldg(d0 + g * 4 + t);
-            r.y = __ldg(d0 + (g + 8) * 4 + t);
-            if (b + 1 < it.blk_end) {
-                r.z = __ldg(d0 + 64 + g * 4 + t);
-                r.w = __ldg(d0 + 64 + (g + 8) * 4 + t);
-            }
+            r = __ldg(pd + (size_t)j * 32);
         }
         return r;
     };
-
-    auto compute = [&](int j, int stage, const uint4& av) {
-        const uint32_t baddr = boff + stage * T::STAGE;
-        if (j < nsparse) {
-#pragma unroll
-            for (int h = 0; h < T::NT / 2; ++h) {
-                uint32_t b0, b1, b2, b3;
-                ldmatrix_x4_trans(baddr + (((2 * h + lchunk) ^ lswz) << 4), b0, b1, b2, b3);
-                mma_sp_16816(acc[2 * h], av.x, av.y, b0, b1, av.z);
-                mma_sp_16816(acc[2 * h + 1], av.x, av.y, b2, b3, av.z);
-            }
-        } else {
-            uint32_t a0 = av.x, a1 = av.y, a2 = av.z, a3 = av.w;
-            if (j >= nmain) {
-                // CSR group: A[r][k] = value of entry k if its row is r.  Fragment words: rows g / g + 8,
-                // columns (2t, 2t+1) and (2t+8, 2t+9)
-                auto pick = [](uint32_t e, uint32_t row) -> uint32_t { return (e >> 16) == row ? (e & 0xffffu) : 0u; };
-                const uint32_t rlo = (uint32_t)g, rhi = (uint32_t)g + 8u;
-                a0 = pick(av.x, rlo) | (pick(av.y, rlo) << 16);
-                a1 = pick(av.x, rhi) | (pick(av.y, rhi) << 16);
-                a2 = pick(av.z, rlo) | (pick(av.w, rlo) << 16);
-                a3 = pick(av.z, rhi) | (pick(av.w, rhi) << 16);
-            }
-#pragma unroll
-            for (int h = 0; h < T::NT / 2; ++h) {
-                uint32_t b0, b1, b2, b3;
-                ldmatrix_x4_trans(baddr + (((2 * h + lchunk) ^ lswz) << 4), b0, b1, b2, b3);
-                mma_16816(acc[2 * h], a0, a1, a2, a3, b0, b1);
-                mma_16816(acc[2 * h + 1], a0, a1, a2, a3, b2, b3);
-            }
-        }
+    auto compute_sparse = [&](auto stage, const uint4& av) {
+        compute_steps<FS, decltype(stage)::value * T::STAGE, true>(acc, laddr, av);
+    };
+    auto compute = [&](int j, auto stage, const uint4& av) {
+        if (j < nsparse) compute_steps<FS, decltype(stage)::value * T::STAGE, true>(acc, laddr, av);
+        else compute_steps<FS, decltype(stage)::value * T::STAGE, false>(acc, laddr, av);
+    };
+    // rows and A operand of step j, and with every eighth step the ids of the block after its own:
+    // they land before the first step that reads them is gathered (AHEAD <= 8 steps earlier), in the
+    // half of the id ring whose last reader was the step before j
+    uint4 areg[STAGES];
+    auto fetch = [&](int j, auto stage) {
+        if ((j & (kIdBlock - 1)) == 0) issue_ids(j / kIdBlock + 1);
+        areg[decltype(stage)::value] = load_a(j);
+        gather(j, stage);
     };
 
-    // Group accounting.  The prologue group carries the ids of steps 0 .. IDA-1 and is waited for
-    // in full.  Then group k (k = 0, 1, ...) carries the rows of step k and, from k = STAGES-1 on,
-    // the ids of step k - (STAGES-1) + IDA.  At iteration j all groups but the newest STAGES-2 are
-    // complete, i.e. groups 0 .. j: the rows of step j, and the ids up to step j + IDA - STAGES + 1
-    // = j + STAGES - 1, exactly what the gather issued in this iteration reads.
-#pragma unroll
-    for (int m = 0; m < T::IDA; ++m) issue_idx(m);
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncwarp();
-    uint4 areg[STAGES];
-#pragma unroll
-    for (int j = 0; j < STAGES - 1; ++j) {
-        if (j < nsteps) issue(j, j);
+    if (nsteps > 0) {
+        issue_ids(0);
         cp_async_commit();
-        areg[j] = load_a(j);
+        cp_async_wait<0>();
+        __syncwarp();
     }
-
-    for (int j0 = 0; j0 < nsteps; j0 += STAGES) {
-#pragma unroll
-        for (int u = 0; u < STAGES; ++u) {
-            const int j = j0 + u;
-            if (j < nsteps) {
+    static_for<T::AHEAD>([&](auto u) {
+        constexpr int j = decltype(u)::value;
+        if (j < nsteps) fetch(j, u);
+        cp_async_commit();
+    });
+    // group j carries the rows of step j; at iteration j all groups but the newest STAGES - 2 are complete
+    int j = 0;
+    // whole rounds of packed tiles
+    for (; j + STAGES + T::AHEAD <= nsparse; j += STAGES) {
+        static_for<STAGES>([&](auto uu) {
+            constexpr int u = decltype(uu)::value, un = (u + T::AHEAD) % STAGES;
+            cp_async_wait<STAGES - 2>();
+            __syncwarp();
+            const int jn = j + u + T::AHEAD;
+            if ((jn & (kIdBlock - 1)) == 0) issue_ids(jn / kIdBlock + 1);
+            {
+                const uint2 v = __ldg((const uint2*)(pa + (size_t)jn * 64));
+                areg[un] = make_uint4(v.x, v.y, __ldg(pm + (size_t)jn * 8), 0u);
+            }
+            gather(jn, std::integral_constant<int, un>());
+            cp_async_commit();
+            compute_sparse(uu, areg[u]);
+        });
+    }
+    for (; j < nsteps; j += STAGES) {
+        static_for<STAGES>([&](auto uu) {
+            constexpr int u = decltype(uu)::value, un = (u + T::AHEAD) % STAGES;
+            if (j + u < nsteps) {
                 cp_async_wait<STAGES - 2>();
                 __syncwarp();
-                issue_idx(j + T::IDA);
-                if (j + STAGES - 1 < nsteps) issue(j + STAGES - 1, (u + STAGES - 1) % STAGES);
+                if (j + u + T::AHEAD < nsteps) fetch(j + u + T::AHEAD, std::integral_constant<int, un>());
                 cp_async_commit();
-                areg[(u + STAGES - 1) % STAGES] = load_a(j + STAGES - 1);
-                compute(j, u, areg[u]);
+                compute(j + u, uu, areg[u]);
             }
-        }
+        });
     }
     cp_async_wait<0>();
     __syncwarp();
-    finish_item_warp<FS>(acc, it, a, fbase, lane, smem);
+
+    // ---- epilogue: the single write of the item's result -----------------------------------------
+    const bool partial = it.slot >= 0;
+    const bool half_out = !partial && (a.out_half || a.n_peers > 0);
+    if constexpr (WPI == 1) {
+        if (a.relu && !partial) {
+#pragma unroll
+            for (int n = 0; n < T::NT; ++n)
+#pragma unroll
+                for (int i = 0; i < 4; ++i) acc[n][i] = fmaxf(acc[n][i], 0.f);
+        }
+        stage_acc<FS>(acc, half_out, smem, lane);
+        __syncwarp();
+        store_rows<FS>(smem, half_out, it, a, fbase, lane, 32);
+    } else {
+        stage_acc<FS>(acc, false, smem, lane);
+        __syncthreads();
+        // thread sums its 4-feature pieces over the warps' tiles, in warp order, in place in warp 0's
+        constexpr int PITCH = FS * 4 + 16;
+        for (int c = threadIdx.x; c < 16 * (FS / 4); c += 32 * WPI) {
+            const int at = c / (FS / 4) * PITCH + c % (FS / 4) * 16;
+            float4 v = *(const float4*)(smem_all + at);
+#pragma unroll
+            for (int q = 1; q < WPI; ++q) {
+                const float4 x = *(const float4*)(smem_all + q * T::SMEM + at);
+                v.x += x.x; v.y += x.y; v.z += x.z; v.w += x.w;
+            }
+            if (a.relu && !partial) { v.x = fmaxf(v.x, 0.f); v.y = fmaxf(v.y, 0.f); v.z = fmaxf(v.z, 0.f); v.w = fmaxf(v.w, 0.f); }
+            *(float4*)(smem_all + at) = v;
+        }
+        __syncthreads();
+        if (half_out) {
+            // repack the fp32 tile as fp16 into warp 1's part (already consumed)
+            unsigned char* ht = smem_all + T::SMEM;
+            for (int c = threadIdx.x; c < 16 * (FS / 4); c += 32 * WPI) {
+                const int r = c / (FS / 4), q = c % (FS / 4);
+                const float4 v = *(const float4*)(smem_all + r * PITCH + q * 16);
+                *(__half2*)(ht + r * (FS * 2 + 16) + q * 8) = __floats2half2_rn(v.x, v.y);
+                *(__half2*)(ht + r * (FS * 2 + 16) + q * 8 + 4) = __floats2half2_rn(v.z, v.w);
+            }
+            __syncthreads();
+            store_rows<FS>(ht, true, it, a, fbase, threadIdx.x, 32 * WPI);
+        } else {
+            store_rows<FS>(smem_all, false, it, a, fbase, threadIdx.x, 32 * WPI);
+        }
+    }
 }
 
-// Expands the bitmap + packed values of every TC block into a dense 16x8 fp16 tile.
-__global__ void k_expand_tc(const long long* __restrict__ t_binary, const int* __restrict__ t_block_offset,
-                            const __half* __restrict__ t_value, int blocks, __half* __restrict__ dense) {
+// B with rows padded to a multiple of 16 features (32-byte sectors), for widths whose rows do not
+// start on 16-byte boundaries: one pass over B against 2-byte gathers of every (window, column) pair.
+// One thread writes 8 features.
+__global__ void k_pad_rows(const __half* __restrict__ B, long long pieces, int F, int per_row, __half* __restrict__ out) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= (long long)blocks * 128) return;
-    const int b = (int)(i >> 7), r = (int)((i >> 3) & 15), k = (int)(i & 7);
-    const unsigned long long lo = (unsigned long long)t_binary[(size_t)b * 2];
-    const unsigned long long hi = (unsigned long long)t_binary[(size_t)b * 2 + 1];
-    const unsigned long long msk = r < 8 ? lo : hi;
-    const int bit = (r & 7) * 8 + k;
-    __half v = __float2half(0.f);
-    if ((msk >> bit) & 1ull) {
-        int rank = __popcll(msk & ((1ull << bit) - 1ull));
-        if (r >= 8) rank += __popcll(lo);
-        v = t_value[(size_t)t_block_offset[b] + rank];
-    }
-    dense[i] = v;
+    if (i >= pieces) return;
+    const long long r = i / per_row;
+    const int f = (int)(i - r * per_row) * 8;
+    ((uint4*)out)[i] = load_unaligned8(B + r * F + f, F - f);
 }
 
 // Adds the partial sums of a split window in slot order and writes its 16 rows of C.
@@ -772,21 +656,39 @@ struct PeerDst {
     long long row0;
 };
 
-__global__ void k_reduce_heavy(const Heavy* __restrict__ heavy, const float* __restrict__ scratch, void* C, int F,
-                               int m_rows, int window, int out_half, int relu, PeerDst pd) {
+// One thread owns 4 features of one row; the slots are read 8 at a time (independent loads) and added
+// one by one.
+__global__ void __launch_bounds__(128) k_reduce_heavy(const Heavy* __restrict__ heavy, const float* __restrict__ scratch,
+                                                      void* C, int F, int ldS, int m_rows, int window, int out_half,
+                                                      int relu, int w_begin, int w_end, PeerDst pd) {
     const Heavy h = heavy[blockIdx.x];
-    const int per = 16 * F;
-    for (int i = threadIdx.x; i < per; i += blockDim.x) {
-        const int lr = i / F, f = i % F;
-        const long long row = (long long)h.window * window + lr;
-        if (lr >= window || row >= m_rows) continue;
-        float s = 0.f;
-        for (int sl = h.slot_begin; sl < h.slot_end; ++sl) s += scratch[(size_t)sl * per + i];
-        if (relu) s = fmaxf(s, 0.f);
+    if (h.window < w_begin || h.window >= w_end) return;
+    const int quads = ldS / 4;
+    const int i = blockIdx.y * blockDim.x + threadIdx.x;
+    const int lr = i / quads, f = (i - lr * quads) * 4;
+    const long long row = (long long)h.window * window + lr;
+    if (lr >= window || row >= m_rows) return;
+    const float4* src = (const float4*)scratch + (size_t)h.slot_begin * 16 * quads + i;
+    float4 s = make_float4(0.f, 0.f, 0.f, 0.f);
+    const int n = h.slot_end - h.slot_begin;
+    for (int k = 0; k < n; k += 8) {
+        float4 v[8];
+#pragma unroll
+        for (int u = 0; u < 8; ++u)
+            v[u] = k + u < n ? __ldcs(src + (size_t)(k + u) * 16 * quads) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+        for (int u = 0; u < 8; ++u) { s.x += v[u].x; s.y += v[u].y; s.z += v[u].z; s.w += v[u].w; }
+    }
+    float r[4] = {s.x, s.y, s.z, s.w};
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        if (f + q >= F) break;
+        if (relu) r[q] = fmaxf(r[q], 0.f);
+        const size_t at = (size_t)row * F + f + q;
         if (pd.n > 0) {
-            for (int d = 0; d < pd.n; ++d) ((__half*)pd.ptr[d])[(size_t)(pd.row0 + row) * F + f] = __float2half_rn(s);
-        } else if (out_half) ((__half*)C)[(size_t)row * F + f] = __float2half_rn(s);
-        else ((float*)C)[(size_t)row * F + f] = s;
+            for (int d = 0; d < pd.n; ++d) ((__half*)pd.ptr[d])[(size_t)pd.row0 * F + at] = __float2half_rn(r[q]);
+        } else if (out_half) ((__half*)C)[at] = __float2half_rn(r[q]);
+        else ((float*)C)[at] = r[q];
     }
 }
 
@@ -799,16 +701,13 @@ using namespace trs;
 
 struct trs_spmm_plan {
     trs_format f;
-    int m_rows, k_cols, window, num_windows, chunk;
-    DevBuf<Item> items;               // in window order (window-range runs index it by window)
-    DevBuf<Item> items_sorted;        // the same items, long ones first (whole-matrix runs)
+    int m_rows, k_cols, window, num_windows;
+    DevBuf<Item> items;               // long ones first
     DevBuf<Heavy> heavy;
-    DevBuf<__half> tc_dense;          // TC blocks expanded to dense 16 x 8 fp16 tiles
-    DevBuf<int> ce_col;               // CSR remainder entries in groups of 16: column ids (-1 = padding)
-    DevBuf<unsigned> ce_rv;           //   and fp16 value | local row << 16
+    DevBuf<int> ids;                  // [steps + kIdBlock][16] column ids of the step stream
+    DevBuf<uint4> dense;              // [dense steps][32] A tiles of the dense steps in fragment order
     int n_items, n_heavy, n_slots;
-    std::vector<int> h_item_off, h_heavy_off;  // host copies of the per-window prefixes (num_windows + 1 each)
-    bool arrays_aligned;              // index / tile arrays are 16-byte aligned
+    bool few_items;                   // four warps per item
 };
 
 static int env_int(const char* name, int dflt) {
@@ -896,6 +795,7 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     if (f.parts_c_short > 0 && !(f.cs_row_offset && f.cs_row && f.cs_column && f.cs_value)) return TRS_E_ARG;
     if (f.num_windows > 0 && !f.s_window_tile_offset) return TRS_E_ARG;
     if (f.tiles > 0 && !(f.s_tile_column && f.s_packed_a && f.s_packed_meta)) return TRS_E_ARG;
+    if ((uintptr_t)f.s_packed_a & 7) return TRS_E_ARG;      // read 8 bytes per lane
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return TRS_E_NO_DEVICE;
 
@@ -909,20 +809,20 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     trs_spmm_plan* p = new trs_spmm_plan();
     p->f = f;
     p->m_rows = m_rows; p->k_cols = k_cols; p->window = window; p->num_windows = W;
-    // Longest run of k-steps one warp takes (longer windows are split into several items that write
-    // partial sums).  Shorter items for small shards (64 to 256 by the shard's number of steps) were
-    // measured and not kept: R-MAT scale 20 on one GPU 0.83 against 0.81 ms, a four-rank shard 0.46
-    // against 0.42 ms - the extra partial sums cost more than the shorter critical path wins.
-    p->chunk = max(8, env_int("TRS_CHUNK_STEPS", 256));
+    const int forced_chunk = env_int("TRS_CHUNK_STEPS", 0);
+    const int chunk = forced_chunk > 0 ? max(8, forced_chunk) : 0;
+    int dev = 0, sms = 0;
+    cudaGetDevice(&dev);
+    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+    sms = max(sms, 1);
     // per-window ranges of TC blocks and CSR parts (needed only while the items are made)
     DevBuf<int> ranges, cnt, off;
     DevBuf<unsigned char> tmp;
     auto fail = [&](int code) { ranges.release(); cnt.release(); off.release(); tmp.release(); trs_spmm_plan_destroy(p); return code; };
-    int rc = ranges.alloc((size_t)6 * W + 2 * ((size_t)W + 1));
+    int rc = ranges.alloc((size_t)6 * W);
     if (rc) return fail(rc);
-    cudaMemsetAsync(ranges.p, 0, sizeof(int) * ((size_t)6 * W + 2 * ((size_t)W + 1)), st);
-    WindowRanges wr{ranges.p, ranges.p + W, ranges.p + 2 * W, ranges.p + 3 * W, ranges.p + 4 * W, ranges.p + 5 * W,
-                    ranges.p + (size_t)6 * W, ranges.p + (size_t)6 * W + (W + 1)};
+    cudaMemsetAsync(ranges.p, 0, sizeof(int) * (size_t)6 * W, st);
+    WindowRanges wr{ranges.p, ranges.p + W, ranges.p + 2 * W, ranges.p + 3 * W, ranges.p + 4 * W, ranges.p + 5 * W};
     auto grid = [](long long n) { return (unsigned)((n + 255) / 256); };
     if (f.parts_t > 0)
         k_part_ranges<<<grid(f.parts_t), 256, 0, st>>>(f.t_window_row, f.t_row_offset, f.parts_t, 16, W,
@@ -932,87 +832,55 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     if (f.parts_c_short > 0)
         k_part_ranges<<<grid(f.parts_c_short), 256, 0, st>>>(f.cs_row, nullptr, f.parts_c_short, window, W,
                                                               wr.cs_begin, wr.cs_end, 0);
-    // counts -> exclusive scans (three arrays of W + 1)
-    rc = cnt.alloc((size_t)3 * (W + 1));
-    if (!rc) rc = off.alloc((size_t)3 * (W + 1));
+    // counts -> exclusive scans (kWindowCounts arrays of W + 1)
+    const size_t stride = (size_t)W + 1;
+    rc = cnt.alloc(kWindowCounts * stride);
+    if (!rc) rc = off.alloc(kWindowCounts * stride);
     size_t tmp_bytes = 0;
     cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, cnt.p, off.p, W + 1, st);
     if (!rc) rc = tmp.alloc(tmp_bytes + 16);
     if (rc) return fail(rc);
-    cudaMemsetAsync(cnt.p, 0, sizeof(int) * 3 * (W + 1), st);
-    // CSR remainder entries, expanded into groups of 16 per window
-    {
-        k_ce_count<<<grid(W + 1), 256, 0, st>>>(f, wr, W);
-        cub::DeviceScan::ExclusiveSum(tmp.p, tmp_bytes, wr.ce_count, wr.ce_begin, W + 1, st);
-        int groups = 0;
-        cudaError_t ee = cudaMemcpyAsync(&groups, wr.ce_begin + W, sizeof(int), cudaMemcpyDeviceToHost, st);
-        if (ee == cudaSuccess) ee = cudaStreamSynchronize(st);
-        if (ee != cudaSuccess) return fail((int)ee);
-        if (groups < 0) return fail(TRS_E_OFFSETS);
-        const size_t cap = (size_t)groups * 16;
-        rc = p->ce_col.alloc(cap);
-        if (!rc) rc = p->ce_rv.alloc(cap);
-        if (rc) return fail(rc);
-        if (cap > 0) {
-            cudaMemsetAsync(p->ce_col.p, 0xff, cap * sizeof(int), st);
-            cudaMemsetAsync(p->ce_rv.p, 0, cap * sizeof(unsigned), st);
-            if (f.parts_c > 0)
-                k_ce_fill<<<grid(f.parts_c), 256, 0, st>>>(f, wr, W, window, 0, (long long)cap, p->ce_col.p, p->ce_rv.p);
-            if (f.parts_c_short > 0)
-                k_ce_fill<<<grid(f.parts_c_short), 256, 0, st>>>(f, wr, W, window, 1, (long long)cap, p->ce_col.p, p->ce_rv.p);
-        }
-    }
-    k_count_items<<<grid(W), 256, 0, st>>>(f, wr, W, p->chunk, cnt.p, cnt.p + (W + 1), cnt.p + 2 * (W + 1));
-    for (int i = 0; i < 3; ++i)
-        cub::DeviceScan::ExclusiveSum(tmp.p, tmp_bytes, cnt.p + (size_t)i * (W + 1), off.p + (size_t)i * (W + 1), W + 1, st);
-    int totals[3] = {0, 0, 0};
-    for (int i = 0; i < 3; ++i)
-        cudaMemcpyAsync(&totals[i], off.p + (size_t)i * (W + 1) + W, sizeof(int), cudaMemcpyDeviceToHost, st);
+    auto scan = [&](int i) {
+        cub::DeviceScan::ExclusiveSum(tmp.p, tmp_bytes, cnt.p + i * stride, off.p + i * stride, W + 1, st);
+    };
+    k_count_steps<<<grid(W + 1), 256, 0, st>>>(f, wr, W, cnt.p);
+    scan(WC_STEPS); scan(WC_DENSE);
+    k_count_items<<<grid(W + 1), 256, 0, st>>>(W, chunk, sms, off.p + WC_STEPS * stride, cnt.p);
+    scan(WC_ITEMS); scan(WC_HEAVY); scan(WC_SLOTS);
+    int totals[kWindowCounts] = {};
+    for (int i = 0; i < kWindowCounts; ++i)
+        cudaMemcpyAsync(&totals[i], off.p + i * stride + W, sizeof(int), cudaMemcpyDeviceToHost, st);
     cudaError_t e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail((int)e);
-    p->n_items = totals[0]; p->n_heavy = totals[1]; p->n_slots = totals[2];
-    // per-window prefixes on the host, so that a run can be restricted to a window range
-    p->h_item_off.resize((size_t)W + 1);
-    p->h_heavy_off.resize((size_t)W + 1);
-    e = cudaMemcpy(p->h_item_off.data(), off.p, sizeof(int) * ((size_t)W + 1), cudaMemcpyDeviceToHost);
-    if (e == cudaSuccess)
-        e = cudaMemcpy(p->h_heavy_off.data(), off.p + (W + 1), sizeof(int) * ((size_t)W + 1), cudaMemcpyDeviceToHost);
-    if (e != cudaSuccess) return fail((int)e);
+    p->n_items = totals[WC_ITEMS]; p->n_heavy = totals[WC_HEAVY]; p->n_slots = totals[WC_SLOTS];
+    const int n_steps = totals[WC_STEPS], n_dense = totals[WC_DENSE];
+    if (n_steps < 0 || n_dense < 0) return fail(TRS_E_OFFSETS);
+    p->few_items = n_steps / (sms * kWarpsPerSm) < kFewSteps;
+    DevBuf<Item> by_window;   // items in window order, sorted into p->items
+    DevBuf<unsigned char> cls, sort_tmp;
+    auto fail2 = [&](int code) { by_window.release(); cls.release(); sort_tmp.release(); return fail(code); };
     rc = p->items.alloc(p->n_items);
+    if (!rc) rc = by_window.alloc(p->n_items);
+    if (!rc) rc = cls.alloc((size_t)2 * p->n_items);
     if (!rc) rc = p->heavy.alloc(p->n_heavy);
-    if (rc) return fail(rc);
-    k_fill_items<<<grid(W), 256, 0, st>>>(f, wr, W, p->chunk, off.p, off.p + (W + 1), off.p + 2 * (W + 1),
-                                           p->items.p, p->heavy.p);
-    // launch order of whole-matrix runs: a stable sort by length class, 32 classes (window order inside a class)
-    if (p->n_items > 0) {
-        DevBuf<unsigned char> cls, cls_out, sort_tmp;
-        rc = p->items_sorted.alloc(p->n_items);
-        if (!rc) rc = cls.alloc(p->n_items);
-        if (!rc) rc = cls_out.alloc(p->n_items);
-        size_t sort_bytes = 0;
-        cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, cls.p, cls_out.p, p->items.p, p->items_sorted.p, p->n_items, 0, 5, st);
-        if (!rc) rc = sort_tmp.alloc(sort_bytes + 16);
-        if (!rc) {
-            k_item_class<<<grid(p->n_items), 256, 0, st>>>(p->items.p, p->n_items, cls.p);
-            cub::DeviceRadixSort::SortPairs(sort_tmp.p, sort_bytes, cls.p, cls_out.p, p->items.p, p->items_sorted.p, p->n_items, 0, 5, st);
-            e = cudaStreamSynchronize(st);
-            if (e != cudaSuccess) rc = (int)e;
-        }
-        cls.release(); cls_out.release(); sort_tmp.release();
-        if (rc) return fail(rc);
-    }
-    rc = p->tc_dense.alloc((size_t)f.blocks * 128);
-    if (rc) return fail(rc);
-    if (f.blocks > 0)
-        k_expand_tc<<<grid((long long)f.blocks * 128), 256, 0, st>>>((const long long*)f.t_binary, f.t_block_offset,
-                                                                      (const __half*)f.t_value, f.blocks, p->tc_dense.p);
+    if (!rc) rc = p->ids.alloc(((size_t)n_steps + kIdBlock) * 16);
+    if (!rc) rc = p->dense.alloc((size_t)n_dense * 32);
+    size_t sort_bytes = 0;
+    cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, cls.p, cls.p, by_window.p, p->items.p, p->n_items, 0, kClassBits, st);
+    if (!rc) rc = sort_tmp.alloc(sort_bytes + 16);
+    if (rc) return fail2(rc);
+    k_fill_items<<<grid(W), 256, 0, st>>>(f, wr, W, off.p, by_window.p, p->heavy.p);
+    k_fill_steps<<<grid((long long)p->n_items * 32), 256, 0, st>>>(f, wr, by_window.p, p->n_items, off.p, W, window,
+                                                                   p->ids.p, p->dense.p);
+    k_item_class<<<grid(p->n_items), 256, 0, st>>>(by_window.p, p->n_items, cls.p);
+    e = cub::DeviceRadixSort::SortPairs(sort_tmp.p, sort_bytes, cls.p, cls.p + p->n_items, by_window.p, p->items.p, p->n_items,
+                                        0, kClassBits, st);
+    if (e != cudaSuccess) return fail2((int)e);
     e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) return fail((int)e);
+    if (e != cudaSuccess) return fail2((int)e);
+    by_window.release(); cls.release(); sort_tmp.release();
     ranges.release(); cnt.release(); off.release(); tmp.release();
-    const uintptr_t align_or = (uintptr_t)f.s_tile_column | (uintptr_t)f.s_packed_a | (uintptr_t)f.s_packed_meta |
-                               (uintptr_t)f.t_column;
-    p->arrays_aligned = (align_or & 15) == 0;
     *out_plan = p;
     return TRS_OK;
 }
@@ -1029,20 +897,27 @@ extern "C" int trs_spmm_status(const trs_spmm_plan* p, int* status) {
 extern "C" int trs_spmm_plan_destroy(trs_spmm_plan* p) {
     if (!p) return TRS_OK;
     p->items.release();
-    p->items_sorted.release();
     p->heavy.release();
-    p->tc_dense.release();
-    p->ce_col.release();
-    p->ce_rv.release();
+    p->ids.release();
+    p->dense.release();
     delete p;
     return TRS_OK;
 }
 
-static size_t items_scratch_bytes(const trs_spmm_plan* p, int F) { return (size_t)p->n_slots * 16 * (size_t)F * sizeof(float); }
+// Partial sums: 16 rows per slot, rows padded to whole 16-byte pieces.
+static int scratch_ld(int F) { return (F + 3) & ~3; }
+static size_t items_scratch_bytes(const trs_spmm_plan* p, int F) {
+    return (size_t)p->n_slots * 16 * (size_t)scratch_ld(F) * sizeof(float);
+}
+// Widths whose rows do not all start on 16-byte boundaries run on a copy of B with padded rows, kept in
+// the workspace behind the partial sums.
+static int padded_ld(int F) { return (F + 15) & ~15; }
+static size_t padded_at(const trs_spmm_plan* p, int F) { return (items_scratch_bytes(p, F) + 255) & ~(size_t)255; }
+static size_t padded_bytes(const trs_spmm_plan* p, int F) { return (size_t)p->k_cols * padded_ld(F) * sizeof(__half); }
 
 extern "C" int trs_spmm_workspace_bytes(const trs_spmm_plan* p, int F, size_t* bytes) {
     if (!p || !bytes || F <= 0) return TRS_E_ARG;
-    *bytes = items_scratch_bytes(p, F);
+    *bytes = F % 8 == 0 ? items_scratch_bytes(p, F) : padded_at(p, F) + padded_bytes(p, F);
     return TRS_OK;
 }
 
@@ -1057,26 +932,53 @@ extern "C" int trs_spmm_launches(const trs_spmm_plan* p) {
     return p->n_heavy > 0 ? 2 : 1;
 }
 
-template <int FS, int STAGES, int MINB>
-static int launch_warp_kernel(const KernelArgs& a, cudaStream_t st) {
-    using T = WarpTile<FS, STAGES>;
-    dim3 grid(a.n_items, ceil_div(a.F, FS));
-    TRS_CUDA(cudaFuncSetAttribute(k_window_spmm_warp<FS, STAGES, MINB>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM));
-    TRS_CUDA(cudaFuncSetAttribute(k_window_spmm_warp<FS, STAGES, MINB>, cudaFuncAttributePreferredSharedMemoryCarveout,
-                                  cudaSharedmemCarveoutMaxShared));
-    k_window_spmm_warp<FS, STAGES, MINB><<<grid, 32, T::SMEM, st>>>(a);
+template <int FS, int STAGES, int WPI, int MINB, bool ALIGNED, bool RANGE>
+static int launch_instance(const KernelArgs& a, int slabs, cudaStream_t st) {
+    auto kernel = k_window_spmm_warp<FS, STAGES, WPI, MINB, ALIGNED, RANGE>;
+    constexpr int smem = WarpTile<FS, STAGES>::SMEM * WPI;
+    // once per device and instance (the attributes belong to the device's copy of the kernel)
+    static std::atomic<unsigned long long> done{0};
+    int dev = 0;
+    TRS_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (!(done.load(std::memory_order_relaxed) & bit)) {
+        TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+        TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+        if (dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
+    }
+    kernel<<<dim3(a.n_items, slabs), 32 * WPI, smem, st>>>(a);
     TRS_LAUNCH_CHECK();
     return TRS_OK;
 }
 
-template <int WARPS>
-static int launch_cta_kernel(const KernelArgs& a, cudaStream_t st) {
-    using T = Tile<WARPS>;
-    dim3 grid(a.n_items, ceil_div(a.F, T::FS));
-    TRS_CUDA(cudaFuncSetAttribute(k_window_spmm<WARPS>, cudaFuncAttributeMaxDynamicSharedMemorySize, T::SMEM));
-    k_window_spmm<WARPS><<<grid, T::THREADS, T::SMEM, st>>>(a);
-    TRS_LAUNCH_CHECK();
-    return TRS_OK;
+template <int FS, int STAGES, int MINB, int MINB4>
+static int launch_sized(const KernelArgs& a, int slabs, bool few_items, bool range, cudaStream_t st) {
+    if (few_items) return range ? launch_instance<FS, STAGES, 4, MINB4, true, true>(a, slabs, st)
+                                : launch_instance<FS, STAGES, 4, MINB4, true, false>(a, slabs, st);
+    return range ? launch_instance<FS, STAGES, 1, MINB, true, true>(a, slabs, st)
+                 : launch_instance<FS, STAGES, 1, MINB, true, false>(a, slabs, st);
+}
+
+static int launch_window_kernel(const KernelArgs& a, bool aligned, bool few_items, bool range, cudaStream_t st) {
+    // As few slabs as 128 features allow (64-feature slabs for F = 128: 2678 against 2120 us at R-MAT scale 21),
+    // all of the same width rounded up to 16.  Stages and warps per SM fill the shared memory; measured at
+    // R-MAT scale 20, us: F = 32 with 4 / 6 / 8 stages 215 / 220 / 223 (scale 18, where the serial chain
+    // counts: 86 / 74 / 70), F = 64 with 3 / 4 / 5 stages 344 / 335 / 337 (137 / 110 / 93), F = 96 with 3 / 4 stages
+    // 494 / 467, F = 128 with 3 / 4 / 5 stages (16 / 12 / 10 warps) 577 / 627 / 650.
+    const int slabs = ceil_div(a.F, 128);
+    const int fs = ceil_div(ceil_div(a.F, slabs), 16);
+    if (!aligned) return fs <= 4 ? launch_instance<64, 3, 1, 16, false, true>(a, ceil_div(a.F, 64), st)
+                                 : launch_instance<128, 3, 1, 12, false, true>(a, ceil_div(a.F, 128), st);
+    switch (fs) {
+        case 1: return launch_sized<16, 6, 32, 8>(a, slabs, few_items, range, st);
+        case 2: return launch_sized<32, 6, 28, 7>(a, slabs, few_items, range, st);
+        case 3: return launch_sized<48, 4, 26, 6>(a, slabs, few_items, range, st);
+        case 4: return launch_sized<64, 4, 22, 5>(a, slabs, few_items, range, st);
+        case 5: return launch_sized<80, 4, 18, 4>(a, slabs, few_items, range, st);
+        case 6: return launch_sized<96, 4, 15, 4>(a, slabs, few_items, range, st);
+        case 7: return launch_sized<112, 3, 16, 4>(a, slabs, few_items, range, st);
+        default: return launch_sized<128, 3, 16, 4>(a, slabs, few_items, range, st);
+    }
 }
 
 extern "C" int trs_spmm_run(const trs_spmm_plan* p, const trs_half* B, void* C, int F, int out_dtype, void* workspace,
@@ -1107,7 +1009,7 @@ extern "C" int trs_spmm_run_bcast(const trs_spmm_plan* p, const trs_half* B, voi
     if (!p || !dst || n_dst < 1 || n_dst > 8 || row0 < 0) return TRS_E_ARG;
     for (int d = 0; d < n_dst; ++d)
         if (!dst[d] || ((uintptr_t)dst[d] & 15)) return TRS_E_ARG;
-    if (F % 8 != 0 || ((uintptr_t)B & 15) || !p->arrays_aligned) return TRS_E_ARG;  // the 16-byte row pieces need it
+    if (F % 8 != 0 || ((uintptr_t)B & 15)) return TRS_E_ARG;  // the 16-byte row pieces need it
     return run_impl(p, B, dst[0], F, TRS_OUT_F16, flags, workspace, workspace_bytes, stream, dst, n_dst, row0);
 }
 
@@ -1118,47 +1020,48 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
     if (w1 < 0) w1 = p->num_windows;
     if (w0 < 0 || w0 > w1 || w1 > p->num_windows) return TRS_E_ARG;
     if (w0 == w1) return TRS_OK;
-    // window range -> item / split-window ranges (both lists are in window order)
-    const int i0 = p->h_item_off[w0], n_items = p->h_item_off[w1] - i0;
-    const int h0 = p->h_heavy_off[w0], n_heavy = p->h_heavy_off[w1] - h0;
     if (flags & ~TRS_EPILOGUE_RELU) return TRS_E_ARG;
     if (out_dtype != TRS_OUT_F32 && out_dtype != TRS_OUT_F16) return TRS_E_ARG;
     const size_t need = items_scratch_bytes(p, F);
     if (need > 0 && (!workspace || workspace_bytes < need)) return TRS_E_WORKSPACE;
     cudaStream_t st = (cudaStream_t)stream;
     KernelArgs a;
-    a.f = p->f; a.n_items = n_items;
-    a.items = (w0 == 0 && w1 == p->num_windows) ? p->items_sorted.p : p->items.p + i0;
+    a.items = p->items.p; a.n_items = p->n_items;
+    a.w_begin = w0; a.w_end = w1;
+    a.ids = p->ids.p; a.dense = p->dense.p;
+    a.packed_a = p->f.s_packed_a; a.packed_meta = p->f.s_packed_meta;
     a.B = (const __half*)B; a.C = C; a.scratch = (float*)workspace;
-    a.m_rows = p->m_rows; a.k_cols = p->k_cols; a.window = p->window; a.F = F; a.out_half = out_dtype == TRS_OUT_F16;
+    a.ldb = F; a.ldS = scratch_ld(F); a.F = F; a.bchunks = ceil_div(F, 8);
+    a.m_rows = p->m_rows; a.window = p->window; a.out_half = out_dtype == TRS_OUT_F16;
+    a.vec_out = ((uintptr_t)C & 15) == 0 && F % (a.out_half ? 8 : 4) == 0;
     a.relu = (flags & TRS_EPILOGUE_RELU) ? 1 : 0;
     a.n_peers = n_peers; a.peer_row0 = peer_row0;
     for (int d = 0; d < 8; ++d) a.peers[d] = d < n_peers ? peers[d] : nullptr;
-    a.tc_dense = p->tc_dense.p;
-    a.ce_col = p->ce_col.p; a.ce_rv = p->ce_rv.p;
-    // The warp-owner kernel moves everything in 16-byte pieces; anything else takes the fallback.
-    const bool aligned = p->arrays_aligned && (F % 8 == 0) &&
-                         ((((uintptr_t)B | (uintptr_t)C | (uintptr_t)workspace) & 15) == 0);
-    // Three stages (two k-steps in flight per warp) and 16 warps per SM (four per scheduler)
-    // measured fastest at R-MAT scale 21: 2.72 ms, against 3.16 ms for four stages (13 warps) and
-    // 3.05 ms for 17 warps of 96 registers; 64-feature slabs for F = 128 (24 warps per SM, twice
-    // the steps) were slower too, and so was asking L2 for the rows (or the packed tiles) of later
-    // steps with prefetch instructions two to four steps ahead (2.9 - 3.3 ms; bulk prefetches 4.1 ms).
-    int rc;
-    if (!aligned) {
-        if (n_peers > 0) return TRS_E_ARG;
-        if (F <= 32) rc = launch_cta_kernel<1>(a, st);
-        else if (F <= 64) rc = launch_cta_kernel<2>(a, st);
-        else rc = launch_cta_kernel<4>(a, st);
-    } else if (F <= 32) rc = launch_warp_kernel<32, 3, 32>(a, st);
-    else if (F <= 64) rc = launch_warp_kernel<64, 3, 28>(a, st);   // 72 registers: seven warps per scheduler (0.49 against 0.51 ms with six; eight spill: 0.57 ms)
-    else rc = launch_warp_kernel<128, 3, 16>(a, st);   // F > 128: feature slabs of 128 on gridDim.y
+    // The kernel gathers B in 16-byte pieces.  Rows that do not start on 16-byte boundaries are copied to
+    // padded ones first when the workspace has room (trs_spmm_workspace_bytes asks for it when F % 8 != 0).
+    bool aligned = F % 8 == 0 && ((uintptr_t)B & 15) == 0;
+    if (((uintptr_t)workspace & 15) && need > 0) return TRS_E_WORKSPACE;
+    if (!aligned && n_peers == 0 && workspace && workspace_bytes >= padded_at(p, F) + padded_bytes(p, F) &&
+        ((uintptr_t)workspace & 15) == 0) {
+        __half* Bp = (__half*)((unsigned char*)workspace + padded_at(p, F));
+        a.ldb = padded_ld(F);
+        a.bchunks = a.ldb / 8;
+        const long long pieces = (long long)p->k_cols * a.bchunks;
+        k_pad_rows<<<(unsigned)ceil_div64(pieces, 256), 256, 0, st>>>(a.B, pieces, F, a.bchunks, Bp);
+        TRS_LAUNCH_CHECK();
+        a.B = Bp;
+        aligned = true;
+    }
+    if (!aligned && n_peers > 0) return TRS_E_ARG;
+    const int rc = launch_window_kernel(a, aligned, p->few_items, w0 > 0 || w1 < p->num_windows, st);
     if (rc) return rc;
-    if (n_heavy > 0) {
+    if (p->n_heavy > 0) {
         PeerDst pd;
         pd.n = a.n_peers; pd.row0 = a.peer_row0;
         for (int d = 0; d < 8; ++d) pd.ptr[d] = a.peers[d];
-        k_reduce_heavy<<<n_heavy, 256, 0, st>>>(p->heavy.p + h0, (const float*)workspace, C, F, p->m_rows, p->window, a.out_half, a.relu, pd);
+        const dim3 rgrid(p->n_heavy, ceil_div(16 * a.ldS / 4, 128));
+        k_reduce_heavy<<<rgrid, 128, 0, st>>>(p->heavy.p, (const float*)workspace, C, F, a.ldS, p->m_rows, p->window,
+                                              a.out_half, a.relu, w0, w1, pd);
         TRS_LAUNCH_CHECK();
     }
     return TRS_OK;
@@ -1170,9 +1073,8 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
 // Some hosts cannot give this library scratch memory at call time: applications that hand the
 // whole device memory to their own pool at start-up (a later cudaMalloc from a plug-in fails or
 // fragments that pool) and latency-critical loops in which cudaMalloc / cudaFree would stall
-// every stream of the device.  For them trs_spmm_run_static runs the window-per-CTA kernels
-// (k_window_spmm_warp / k_window_spmm + k_reduce_heavy), whose scratch need is small and known
-// from the plan, with the partial sums of split windows kept in the array below instead of a
+// every stream of the device.  For them trs_spmm_run_static runs the ordinary kernels
+// (k_window_spmm_warp + k_reduce_heavy), whose scratch need is small and known from the plan, with the partial sums of split windows kept in the array below instead of a
 // caller-provided workspace.  Every GPU that loads the library holds these bytes until exit.
 //
 // In host code the array's name is only a stand-in for the symbol; the device address is asked
@@ -1189,7 +1091,7 @@ std::mutex g_static_scratch_mutex;
 extern "C" int trs_spmm_run_static(const trs_spmm_plan* p, const trs_half* B, void* C, int F, int out_dtype,
                                    void* stream) {
     if (!p || !B || !C || F <= 0) return TRS_E_ARG;
-    const size_t need = (size_t)p->n_slots * 16 * (size_t)F * sizeof(float);
+    const size_t need = items_scratch_bytes(p, F);
     if (need > (size_t)TRS_STATIC_SCRATCH_BYTES) return TRS_E_LIMIT;
     int dev = -1;
     TRS_CUDA(cudaGetDevice(&dev));
