@@ -86,6 +86,9 @@ typedef struct trs_timing {
 const char* trs_strerror(int code);
 int trs_version(void);
 int trs_device_count(void);
+/* The library keeps up to 4 GiB of freed device memory per GPU for its next calls (temporaries, the buffers of
+ * the host-buffer entries); this returns what the current device's pool holds to the driver. */
+int trs_pool_trim(void);
 
 /* ---- SpMM: plan over device-resident format arrays ---------------------------------------
  * Replaces the device half of spmm_forward_fp16_tcu_cuda_sptc_mma_parallel_online
@@ -246,6 +249,15 @@ typedef struct trs_builder trs_builder; /* opaque; owns the output arrays on the
 int trs_build_create(const int32_t* rowptr, const int32_t* col, const float* values, int n_rows,
                      const trs_build_config* cfg, void* stream, trs_builder** out);
 int trs_build_destroy(trs_builder* b);
+/* The same build with the 29 arrays in memory the caller hands out while the build runs: `alloc` is
+ * called once per non-empty array, from the calling thread, with its number in the reference's
+ * return order and its size, and returns device memory usable on `stream` (NULL fails the build).  Only
+ * temporaries come from the library's pool.  The caller keeps ownership; trs_build_destroy frees
+ * the small host object. */
+typedef void* (*trs_build_alloc)(void* ctx, int array, size_t bytes);
+int trs_build_create_into(const int32_t* rowptr, const int32_t* col, const float* values, int n_rows,
+                          const trs_build_config* cfg, trs_build_alloc alloc, void* ctx, void* stream,
+                          trs_builder** out);
 /* The same build with every byte of device memory owned by the caller (the reference allocates
  * its outputs itself, block_online.cpp:844-870; a host that pools its device memory cannot let a
  * plug-in call cudaMalloc): trs_build_query gives an upper bound of the arena one build needs from

@@ -1,0 +1,50 @@
+"""Windows at the borders of the builder's matching tiers (a warp, a block, a block with the units outside shared
+memory), with long runs of equal units and with mixed ones, and key widths on both sides of 32 bits."""
+import pytest
+import torch
+
+from oracle import oracle as O
+from trspmm import build_format
+
+pytestmark = pytest.mark.gpu
+
+
+def _window(n_units, mixed, n_cols, seed):
+    """One 16-row window with 2 * n_units distinct columns; `mixed`: counts 1 to 5, otherwise 1 for nearly all."""
+    g = torch.Generator().manual_seed(seed)
+    d = 2 * n_units - seed % 2
+    cols = torch.randperm(n_cols, generator=g)[:d].sort().values
+    count = torch.randint(1, 6, (d,), generator=g) if mixed else 1 + (torch.rand(d, generator=g) < 0.001).long()
+    rows = torch.rand(d, 16, generator=g).argsort(dim=1)
+    keep = torch.arange(16)[None, :] < count[:, None]
+    r, c = rows[keep], cols[:, None].expand(-1, 16)[keep]
+    order = torch.argsort(r * n_cols + c)
+    r, c = r[order], c[order]
+    rowptr = torch.zeros(17, dtype=torch.int64)
+    rowptr[1:] = torch.cumsum(torch.bincount(r, minlength=16), 0)
+    return rowptr.to(torch.int32), c.to(torch.int32), torch.randn(c.numel(), generator=g)
+
+
+def _check(rp, col, val, **kw):
+    want, info = O.build_format(rp, col, val, **kw)
+    fmt, stats = build_format(rp.cuda(), col.cuda(), val.cuda(), **kw)
+    for name, a, b in zip(O.FORMAT_NAMES, fmt.arrays(), want):
+        assert torch.equal(a.cpu(), b), name
+    assert stats["dropped_nnz"] == info["dropped_nnz"]
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("units", [1, 16, 17, 31, 33, 64, 1023, 2048, 2049, 14336, 14337])
+def test_tier_borders(units, mixed):
+    _check(*_window(units, mixed, 1 << 20, units))
+
+
+def test_units_beyond_shared_memory():
+    _check(*_window(53000, True, 1 << 20, 1))
+
+
+@pytest.mark.parametrize("bits", [14, 22])   # one window: under 32 key bits; with 40001 windows 30 and 38
+def test_key_widths(bits):
+    rp, col, val = _window(40, True, 1 << bits, 3)
+    for empty_rows in (0, 16 * 40000):
+        _check(torch.cat([rp, rp[-1:].expand(empty_rows)]), col, val)

@@ -2,6 +2,7 @@
 // CPU result out; mGCN_online.cpp:760-1138) on top of the device-resident plan API.
 #include <string.h>
 
+#include <mutex>
 #include <vector>
 
 #include "trs_common.cuh"
@@ -33,6 +34,60 @@ extern "C" int trs_device_count(void) {
     int n = 0;
     if (cudaGetDeviceCount(&n) != cudaSuccess) return 0;
     return n;
+}
+
+namespace trs {
+
+namespace {
+constexpr int kPoolDevices = 64;
+cudaMemPool_t g_pool[kPoolDevices] = {};
+std::mutex g_pool_mutex;
+
+int device_pool(cudaMemPool_t* out) {
+    int dev = 0;
+    TRS_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= kPoolDevices) return TRS_E_LIMIT;
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    if (!g_pool[dev]) {
+        cudaMemPoolProps props;
+        memset(&props, 0, sizeof(props));
+        props.allocType = cudaMemAllocationTypePinned;
+        props.location.type = cudaMemLocationTypeDevice;
+        props.location.id = dev;
+        cudaMemPool_t pool = nullptr;
+        TRS_CUDA(cudaMemPoolCreate(&pool, &props));
+        unsigned long long keep = kPoolKeepBytes;
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+        g_pool[dev] = pool;
+    }
+    *out = g_pool[dev];
+    return TRS_OK;
+}
+}  // namespace
+
+int pool_alloc(void** p, size_t bytes, cudaStream_t st) {
+    *p = nullptr;
+    cudaMemPool_t pool;
+    const int rc = device_pool(&pool);
+    if (rc) return rc;
+    const cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, st);
+    if (e != cudaSuccess) { *p = nullptr; cudaGetLastError(); }
+    return (int)e;
+}
+
+void pool_free(void* p, cudaStream_t st) {
+    if (p) cudaFreeAsync(p, st);
+}
+
+}  // namespace trs
+
+// Returns the memory the library's pool of the current device holds for later calls to the driver.
+extern "C" int trs_pool_trim(void) {
+    int dev = 0;
+    TRS_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lock(trs::g_pool_mutex);
+    if (dev >= 0 && dev < trs::kPoolDevices && trs::g_pool[dev]) TRS_CUDA(cudaMemPoolTrimTo(trs::g_pool[dev], 0));
+    return TRS_OK;
 }
 
 namespace {

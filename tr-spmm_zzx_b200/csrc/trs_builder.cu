@@ -4,34 +4,37 @@
 // windows serially on one CPU thread with hash maps and an O(U^2) unit graph.  Here every stage
 // is a data-parallel pass over device arrays:
 //
-//   1. key = (window, column, local row) per entry, radix sort      -> per-window column lists
+//   1. key = (window, column) per entry, stable radix sort          -> per-window column lists
 //      (the reference's col_info map, block_online.cpp:589-603)
 //   2. run heads -> one record per (window, column): count, 16-bit row mask, first entry
 //   3. stable sort by (window, 16 - count): the (count desc, column asc) order both funnels
 //      use (block_online.cpp:226-230, 281-285)
 //   4. TC funnel: leading columns with count >= density in chunks of 8, kept when
-//      nnz/(window*8) >= tc_min_util (block_online.cpp:215-253)
+//      nnz/(window*8) >= tc_min_util (block_online.cpp:215-253).  Counts descend, so the kept chunks
+//      are the first ones and everything that follows is arithmetic on three numbers per window.
 //   5. units = consecutive pairs of the remaining columns (the first-fit of
 //      block_online.cpp:287-326 always takes the next column because its bit test cannot fail)
 //   6. matching (block_online.cpp:332-392): the unit graph is complete, so degrees are all
-//      equal, the node order is libstdc++ std::sort of unit nnz (emulated step for step, see
-//      trs_stdsort.cuh) and the partner of a node is the lowest-index unmatched other unit
+//      equal, the node order is libstdc++ std::sort of unit nnz (emulated, see trs_stdsort.cuh)
+//      and the partner of a node is the lowest-index unmatched other unit
 //   7. group emission, per-row (value, position) slots with the reference's "first two kept,
-//      the rest dropped" rule (block_online.cpp:629-703)
+//      the rest dropped" rule (block_online.cpp:629-703), and the 16x16 mma.sp tile of four groups
+//      (block_online.cpp:190-210, 796-841), all by one warp per tile
 //   8. TC blocks, bitmaps, values, parts (block_online.cpp:444-540)
 //   9. CUDA-core row parts from the columns of an unmatched sparse unit (block_online.cpp:397-439,
 //      706-733)
-//  10. 16x16 mma.sp tile packing (block_online.cpp:796-841; trs_pack.cu)
 //
 // Input contract: canonical CSR (columns strictly ascending inside a row), window in 1..16.
 #include <cub/device/device_radix_sort.cuh>
-#include <cub/device/device_reduce.cuh>
 #include <cub/device/device_scan.cuh>
+#include <cub/device/device_select.cuh>
+#include <thrust/iterator/counting_iterator.h>
 
 #include <stdlib.h>
 #include <string.h>
 
 #include <algorithm>
+#include <mutex>
 #include <vector>
 
 #include "trs_common.cuh"
@@ -49,280 +52,561 @@ struct BuildCfg {
 };
 
 // ---------------------------------------------------------------------------------------------
-// stage kernels
+// 0. the sizes and the row pointers: one pass, one read-back
 // ---------------------------------------------------------------------------------------------
-__global__ void kb_mark_rows(const int* __restrict__ rowptr, int n_rows, int* __restrict__ rowid, int* err) {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_rows) return;
-    const int b = rowptr[r], e = rowptr[r + 1];
-    if (e < b) { atomicOr(err, 1); return; }
-    if (e > b) rowid[b] = r;
-}
-
-struct MaxOp {
-    __device__ __forceinline__ int operator()(int a, int b) const { return a > b ? a : b; }
+struct InputInfo {
+    int first, last;  // rowptr[0], rowptr[n_rows]
+    int max_col;
+    int err;          // 1: decreasing row pointer, 2: columns negative, not ascending or repeated
 };
 
-__global__ void kb_make_keys(const int* __restrict__ col, const int* __restrict__ rowid, long long nnz, int window,
-                             int col_bits, u64* __restrict__ keys, int* __restrict__ edge, int* err) {
-    long long e = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= nnz) return;
-    const int r = rowid[e], c = col[e];
-    if (c < 0) atomicOr(err, 2);
-    if (e + 1 < nnz && rowid[e + 1] == r && col[e + 1] <= c) atomicOr(err, 2);  // not canonical
-    const int w = r / window, lr = r - w * window;
-    keys[e] = ((u64)w << (col_bits + 4)) | ((u64)(unsigned)c << 4) | (u64)lr;
-    edge[e] = (int)e;
+__global__ void kb_input_info(const int* __restrict__ rowptr, const int* __restrict__ col, int n_rows,
+                              InputInfo* __restrict__ info) {
+    const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
+    const int first = rowptr[0], nnz = rowptr[n_rows];
+    if (t0 == 0) { info->first = first; info->last = nnz; }
+    bool bad = false;
+    for (long long r = t0; r < n_rows; r += step) bad |= rowptr[r + 1] < rowptr[r];
+    if (bad) atomicOr(&info->err, 1);
+    if (first != 0 || !col) return;
+    int m = -1;
+    for (long long e = t0; e < nnz; e += step) m = max(m, col[e]);
+    m = __reduce_max_sync(0xffffffffu, m);
+    if ((threadIdx.x & 31) == 0 && m > info->max_col) atomicMax(&info->max_col, m);
 }
 
-__global__ void kb_heads(const u64* __restrict__ keys, long long nnz, int* __restrict__ head) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nnz) return;
-    head[i] = (i == 0 || (keys[i] >> 4) != (keys[i - 1] >> 4)) ? 1 : 0;
+// ---------------------------------------------------------------------------------------------
+// 1. keys.  The payload of an entry is (entry << 4 | local row) while entries fit 28 bits: the sort
+// is stable and entries come in row order, so the rows of a column stay ascending without sorting
+// by them.  Longer inputs carry the entry alone and look its row up.
+// ---------------------------------------------------------------------------------------------
+constexpr int kKeyItems = 8;
+
+template <class Key, bool PACKED>
+__global__ void __launch_bounds__(256) kb_make_keys(const int* __restrict__ rowptr, const int* __restrict__ col, int n_rows,
+                                                    int nnz, int window, int col_bits, Key* __restrict__ keys,
+                                                    unsigned* __restrict__ ent, InputInfo* __restrict__ info) {
+    // rows of this CTA's entries
+    __shared__ int s_lo, s_hi;
+    const long long e0 = (long long)blockIdx.x * (256 * kKeyItems);
+    const long long e1 = min(e0 + 256 * kKeyItems, (long long)nnz);
+    if (threadIdx.x < 2) {
+        const long long e = threadIdx.x ? e1 - 1 : e0;
+        int lo = 0, hi = n_rows;  // largest r with rowptr[r] <= e
+        while (hi - lo > 1) {
+            const int mid = lo + (hi - lo) / 2;
+            if (rowptr[mid] <= e) lo = mid; else hi = mid;
+        }
+        if (threadIdx.x) s_hi = lo; else s_lo = lo;
+    }
+    __syncthreads();
+    const int rlo = s_lo, rhi = s_hi + 1;
+    bool bad = false;
+#pragma unroll
+    for (int i = 0; i < kKeyItems; ++i) {
+        const long long e = e0 + i * 256 + threadIdx.x;
+        if (e >= e1) break;
+        int lo = rlo, hi = rhi;
+        while (hi - lo > 1) {
+            const int mid = lo + (hi - lo) / 2;
+            if (rowptr[mid] <= e) lo = mid; else hi = mid;
+        }
+        const int c = col[e];
+        bad |= c < 0 || (e + 1 < rowptr[lo + 1] && col[e + 1] <= c);
+        const int w = lo / window;
+        keys[e] = ((Key)w << col_bits) | (Key)(unsigned)c;
+        ent[e] = PACKED ? ((unsigned)e << 4) | (unsigned)(lo - w * window) : (unsigned)e;
+    }
+    if (bad) atomicOr(&info->err, 2);
 }
 
-// wc_id (inclusive scan of heads) -> start position of every (window, column) record
-__global__ void kb_wcol_start(const int* __restrict__ head, const int* __restrict__ wc_incl, long long nnz,
-                              int* __restrict__ wc_start) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nnz) return;
-    if (head[i]) wc_start[wc_incl[i] - 1] = (int)i;
-}
+// 2. first entry of every (window, column) record
+template <class Key>
+struct IsHead {
+    const Key* keys;
+    __device__ __forceinline__ bool operator()(int i) const { return i == 0 || keys[i] != keys[i - 1]; }
+};
 
-__global__ void kb_wcol_info(const u64* __restrict__ keys, const int* __restrict__ wc_start, int D, int col_bits,
-                             int density, int skip_tc, int* __restrict__ wc_win, int* __restrict__ wc_col,
-                             unsigned char* __restrict__ wc_count, unsigned short* __restrict__ wc_mask,
-                             int* __restrict__ win_ncol, int* __restrict__ win_ncand, unsigned* __restrict__ key2) {
-    int j = blockIdx.x * blockDim.x + threadIdx.x;
+struct __align__(16) Record {   // one (window, column): its first sorted entry, the rows it has, the first value
+    int col, start;
+    unsigned mask;
+    float value;
+};
+
+template <class Key, bool PACKED>
+__global__ void kb_records(const Key* __restrict__ keys, const unsigned* __restrict__ ent, const int* __restrict__ rowptr,
+                           const float* __restrict__ val, int n_rows, int window, const int* __restrict__ wc_start, int D,
+                           int nnz, int col_bits, Record* __restrict__ record, unsigned* __restrict__ key2, int* __restrict__ ord) {
+    const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= D) return;
-    const int b = wc_start[j], e = wc_start[j + 1];
-    const u64 k0 = keys[b];
+    const int b = wc_start[j], e = j + 1 < D ? wc_start[j + 1] : nnz;
+    const Key k = keys[b];
+    const int w = (int)(k >> col_bits);
     unsigned mask = 0;
-    for (int i = b; i < e; ++i) mask |= 1u << (unsigned)(keys[i] & 15);
-    const int w = (int)(k0 >> (col_bits + 4));
-    const int count = e - b;
-    wc_win[j] = w;
-    wc_col[j] = (int)((k0 >> 4) & ((1ull << col_bits) - 1ull));
-    wc_count[j] = (unsigned char)count;
-    wc_mask[j] = (unsigned short)mask;
-    // per-window counters, one atomic per warp and window (hub windows hold 10^5+ records)
-    const unsigned active = __activemask();
-    const unsigned peers = __match_any_sync(active, w);
-    const bool cand = !skip_tc && count >= density;
-    const unsigned cand_peers = __ballot_sync(active, cand) & peers;
-    if ((threadIdx.x & 31) == __ffs(peers) - 1) {
-        atomicAdd(&win_ncol[w], __popc(peers));
-        if (cand_peers) atomicAdd(&win_ncand[w], __popc(cand_peers));
+    for (int i = b; i < e; ++i) {
+        const unsigned v = ent[i];
+        int lr = (int)(v & 15u);
+        if (!PACKED) {
+            lr = 0;
+            for (int r = 1; r < window && w * window + r < n_rows; ++r) lr += rowptr[w * window + r] <= (int)v;
+        }
+        mask |= 1u << lr;
     }
-    key2[j] = ((unsigned)w << 4) | (unsigned)(16 - count);
+    record[j] = Record{(int)(k & (((Key)1 << col_bits) - 1)), b, mask, val[PACKED ? ent[b] >> 4 : ent[b]]};
+    key2[j] = ((unsigned)w << 4) | (unsigned)(16 - (e - b));
+    ord[j] = j;
 }
 
-// Position p of the (count desc, col asc) order: TC membership of the column there.
-__global__ void kb_tc_select(const int* __restrict__ ord, const int* __restrict__ wc_win,
-                             const unsigned char* __restrict__ wc_count, const int* __restrict__ wc_begin,
-                             const int* __restrict__ win_ncand, int D, int window, float tc_min_util,
-                             int* __restrict__ not_tc, int* __restrict__ lead) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= D) return;
-    const int j = ord[p];
-    const int w = wc_win[j];
-    const int wb = wc_begin[w];
-    const int o = p - wb;
-    const int ncand = win_ncand[w];
-    int is_tc = 0, is_lead = 0;
-    if (o < ncand) {
-        const int cs = wb + (o / 8) * 8;
-        const int ce = min(cs + 8, wb + ncand);
-        int real_nnz = 0;
-        for (int q = cs; q < ce; ++q) real_nnz += wc_count[ord[q]];
-        const float util = __fdiv_rn((float)real_nnz, (float)(window * 8));
-        if (!(util < tc_min_util)) { is_tc = 1; is_lead = (o % 8 == 0); }
+// ---------------------------------------------------------------------------------------------
+// 3. - 5. per window: records, TC columns, units, pair slots, TC blocks, TC parts
+// ---------------------------------------------------------------------------------------------
+struct Win {          // prefixes over windows (W + 1 of them) after the scan
+    int blocks, units, slots, parts;
+};
+struct WinSum {
+    __host__ __device__ __forceinline__ Win operator()(const Win& a, const Win& b) const {
+        return Win{a.blocks + b.blocks, a.units + b.units, a.slots + b.slots, a.parts + b.parts};
     }
-    not_tc[p] = !is_tc;
-    lead[p] = is_lead;
-}
-
-__global__ void kb_compact(const int* __restrict__ ord, const int* __restrict__ not_tc, const int* __restrict__ lead,
-                           const int* __restrict__ s_idx, const int* __restrict__ b_idx, const int* __restrict__ wc_win,
-                           const int* __restrict__ wc_begin, const int* __restrict__ win_ncand, int D,
-                           int* __restrict__ cand, int* __restrict__ blk_pos, int* __restrict__ blk_len) {
-    int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= D) return;
-    if (not_tc[p]) cand[s_idx[p]] = ord[p];
-    if (lead[p]) {
-        const int w = wc_win[ord[p]];
-        const int end = wc_begin[w] + win_ncand[w];
-        const int b = b_idx[p];
-        blk_pos[b] = p;
-        blk_len[b] = min(8, end - p);
-    }
-}
-
-// per window: candidate range, units, pair slots, block range
-__global__ void kb_window_counts(const int* __restrict__ wc_begin, const int* __restrict__ s_idx,
-                                 const int* __restrict__ b_idx, int W, int part_t, int* __restrict__ win_cb,
-                                 int* __restrict__ win_U, int* __restrict__ win_slots, int* __restrict__ win_bb,
-                                 int* __restrict__ win_parts) {
-    int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= W) return;
-    const int pb = wc_begin[w], pe = wc_begin[w + 1];
-    const int cb = s_idx[pb], ns = s_idx[pe] - cb;
-    const int U = (ns + 1) / 2;
-    win_cb[w] = cb;
-    win_U[w] = U;
-    win_slots[w] = (U + 1) / 2;
-    const int bb = b_idx[pb], nb = b_idx[pe] - bb;
-    win_bb[w] = bb;
-    win_parts[w] = nb == 0 ? 0 : (nb <= part_t ? 1 : (nb + part_t - 1) / part_t);
-}
-
-// unit nnz: one thread per sparse-route candidate, even local index writes its unit
-__global__ void kb_unit_nnz(const int* __restrict__ cand, int S, const int* __restrict__ wc_win,
-                            const unsigned char* __restrict__ wc_count, const int* __restrict__ win_cb,
-                            const int* __restrict__ win_ub, const int* __restrict__ win_cb_next_unused,
-                            const int* __restrict__ win_U, unsigned char* __restrict__ unit_nnz) {
-    int s = blockIdx.x * blockDim.x + threadIdx.x;
-    if (s >= S) return;
-    const int j = cand[s];
-    const int w = wc_win[j];
-    const int ls = s - win_cb[w];
-    if (ls & 1) return;
-    int nnz = wc_count[j];
-    // the partner is the next candidate if it belongs to the same window
-    if (s + 1 < S && wc_win[cand[s + 1]] == w) nnz += wc_count[cand[s + 1]];
-    unit_nnz[win_ub[w] + (ls >> 1)] = (unsigned char)nnz;
-}
-
-struct UnitLess {
-    const unsigned char* nnz;
-    __host__ __device__ bool operator()(int a, int b) const { return nnz[a] > nnz[b]; }
+};
+struct WindowView {
+    const int* rec;    // [W + 1] first record of the window
+    const int* tc;     // [W] TC columns: records [rec, rec + tc) in (count desc, column asc) order
+    const Win* pre;    // [W + 1]
 };
 
-// Matching of one window's units by one thread.  pair_a/pair_b get the groups in emission
-// order: matched pairs in greedy order, then the unmatched unit (if it is kept).
-__global__ void kb_match(const int* __restrict__ win_U, const int* __restrict__ win_ub,
-                         const int* __restrict__ win_pb, int W, int unit_min_nnz,
-                         const unsigned char* __restrict__ unit_nnz, int* __restrict__ order_buf,
-                         unsigned char* __restrict__ matched_buf, int* __restrict__ pair_a, int* __restrict__ pair_b,
-                         int* __restrict__ win_G, int* __restrict__ win_cuda_unit, const int* __restrict__ sel,
-                         int n_sel) {
-    int t = blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= n_sel) return;
-    const int w = sel ? sel[t] : t;
-    const int U = win_U[w];
-    int G = 0, cuda_unit = -1;
-    if (U > 0) {
-        const unsigned char* nnz = unit_nnz + win_ub[w];
-        int* order = order_buf + win_ub[w];
-        unsigned char* matched = matched_buf + win_ub[w];
-        for (int i = 0; i < U; ++i) { order[i] = i; matched[i] = 0; }
-        StdSort<UnitLess> sorter(order, UnitLess{nnz});
-        sorter.sort(U);
-        int* pa = pair_a + win_pb[w];
-        int* pb = pair_b + win_pb[w];
-        int lowest = 0;
-        for (int k = 0; k < U; ++k) {
-            const int idx = order[k];
-            if (matched[idx]) continue;
-            while (lowest < U && matched[lowest]) ++lowest;
-            int partner = lowest;
-            if (partner == idx) {
-                ++partner;
-                while (partner < U && matched[partner]) ++partner;
+constexpr int kWarpUnits = 2048;    // matching: windows up to here get a warp each,
+constexpr int kBlockUnits = 14336;  // up to here a block with 56 KB for the units, beyond a whole SM's memory
+constexpr int kSmemUnits = 52224;
+
+struct MatchCounts {
+    int n_block, n_huge;
+    int max_warp, max_huge;   // units of the largest window of the warp and of the last tier
+};
+
+__global__ void kb_windows(const int* __restrict__ wc_start, const unsigned* __restrict__ key2, const int* __restrict__ rowptr,
+                           int n_rows, int D, int W, BuildCfg cfg, int* __restrict__ rec, int* __restrict__ tc,
+                           Win* __restrict__ win, int* __restrict__ sel_block, int* __restrict__ sel_huge,
+                           MatchCounts* __restrict__ mc) {
+    const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w > W) return;
+    auto first_record = [&](int x) -> int {  // records of windows < x: the first one starts where the window's entries do
+        if (x >= W) return D;
+        const int e = rowptr[x * cfg.window];
+        int lo = 0, hi = D;
+        while (lo < hi) {
+            const int mid = lo + (hi - lo) / 2;
+            if (wc_start[mid] < e) lo = mid + 1; else hi = mid;
+        }
+        return lo;
+    };
+    const int b = first_record(w);
+    rec[w] = b;
+    if (w == W) { win[W] = Win{0, 0, 0, 0}; return; }
+    const int n = first_record(w + 1) - b;
+    auto count = [&](int o) -> int { return 16 - (int)(key2[b + o] & 15u); };  // o-th largest column
+    int cand = 0;
+    if (!cfg.skip_tc) {
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int mid = lo + (hi - lo) / 2;
+            if (count(mid) >= cfg.density) lo = mid + 1; else hi = mid;
+        }
+        cand = lo;
+    }
+    int lo = 0, hi = (cand + 7) / 8;  // chunks kept
+    while (lo < hi) {
+        const int mid = lo + (hi - lo) / 2;
+        int nnz = 0;
+        for (int o = mid * 8; o < min(mid * 8 + 8, cand); ++o) nnz += count(o);
+        const float util = __fdiv_rn((float)nnz, (float)(cfg.window * 8));
+        if (!(util < cfg.tc_min_util)) lo = mid + 1; else hi = mid;
+    }
+    const int t = min(lo * 8, cand);
+    const int units = (n - t + 1) / 2;
+    tc[w] = t;
+    win[w] = Win{lo, units, (units + 1) / 2, lo == 0 ? 0 : (lo + cfg.part_t - 1) / cfg.part_t};
+    if (units > kBlockUnits) { sel_huge[atomicAdd(&mc->n_huge, 1)] = w; atomicMax(&mc->max_huge, units); }
+    else if (units > kWarpUnits) sel_block[atomicAdd(&mc->n_block, 1)] = w;
+    else if (units > mc->max_warp) atomicMax(&mc->max_warp, units);
+}
+
+__device__ __forceinline__ int find_window(const int* __restrict__ prefix, int W, int x) {
+    // largest w in [0, W) with prefix[w] <= x   (prefix non-decreasing, prefix[W] > x)
+    int lo = 0, hi = W;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (prefix[mid] <= x) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// ---------------------------------------------------------------------------------------------
+// 6. matching of a window's units
+// ---------------------------------------------------------------------------------------------
+// A unit is one word: nnz << 26 | index, so that the sort touches one array (in shared memory for
+// all but enormous windows: every step of the sort and of the greedy pass is a dependent access, and
+// from L2 each cost ten times as much).  The order of equal keys is libstdc++'s, reproduced as follows.
+//   * Partition (Hoare, unguarded): the k-th element >= pivot from the left swaps with the k-th element
+//     <= pivot from the right while the former lies left of the latter; the cut is
+//     min(next left stopper, last swapped right position).  A warp finds the stoppers 32 at a time.
+//   * A range of equal keys - most of a hub window - is not sorted at all: there each partition moves
+//     the middle element to the front and reverses the rest, so every position can be traced back
+//     through the log2(n / 16) levels on its own.
+//   * Ranges of at most 16 are finished by one lane each (insertion sort), 32 at a time.
+// The result goes to order_out as unit indices.
+constexpr unsigned kUnitBits = 26;
+constexpr unsigned kUnitMask = (1u << kUnitBits) - 1u;
+
+struct UnitWordLess {
+    __host__ __device__ bool operator()(int a, int b) const { return ((unsigned)a >> kUnitBits) > ((unsigned)b >> kUnitBits); }
+};
+__device__ __forceinline__ unsigned unit_key(int word) { return (unsigned)word >> kUnitBits; }
+
+// Where the element that introsort leaves at position p of a range of n > 16 equal keys came from.
+__device__ __forceinline__ int equal_range_source(int n, int p) {
+    int f[28], l[28], levels = 0;
+    int lo = 0, hi = n;
+    while (hi - lo > 16) {
+        f[levels] = lo; l[levels] = hi; ++levels;
+        const int cut = lo + 1 + (hi - lo - 1) / 2;
+        if (p < cut) hi = cut; else lo = cut;
+    }
+    int s = p;
+    for (int i = levels - 1; i >= 0; --i) {
+        const int mid = f[i] + (l[i] - f[i]) / 2;
+        if (s == f[i]) s = mid;
+        else {
+            s = f[i] + l[i] - s;
+            if (s == mid) s = f[i];
+        }
+    }
+    return s;
+}
+__device__ __forceinline__ int equal_range_depth(int n) {  // partitions on the longest path
+    int d = 0;
+    for (; n > 16; ++d) n = max(1 + (n - 1) / 2, n - 1 - (n - 1) / 2);
+    return d;
+}
+
+// One warp partitions [first, last) of a as introsort does (median of three to the front included);
+// `sl` / `sr`: 32 ints of shared memory each.
+__device__ __forceinline__ int warp_partition(int* a, int first, int last, int* sl, int* sr, int lane) {
+    if (lane == 0) {
+        StdSort<UnitWordLess> S(a, UnitWordLess());
+        S.move_median_to_first(first, first + 1, first + (last - first) / 2, last - 1);
+    }
+    __syncwarp();
+    const unsigned pv = unit_key(a[first]);
+    const unsigned lt = (1u << lane) - 1u;
+    int lb = first + 1 - 32, rb = last - 1 + 32;  // the blocks start at lb (upwards) and rb (downwards)
+    unsigned lm = 0, rm = 0;                       // stoppers of the blocks not used yet
+    int last_r = 0x7fffffff;                       // right position of the last swap
+    while (true) {
+        while (lm == 0) {
+            lb += 32;
+            if (lb >= last) break;
+            const int i = lb + lane;
+            lm = __ballot_sync(0xffffffffu, i < last && unit_key(a[i]) <= pv);
+        }
+        while (rm == 0) {
+            rb -= 32;
+            if (rb <= first) break;
+            const int i = rb - lane;
+            rm = __ballot_sync(0xffffffffu, i > first && unit_key(a[i]) >= pv);
+        }
+        if (lm == 0 || rm == 0) break;
+        const int t = min(__popc(lm), __popc(rm));
+        if ((lm >> lane) & 1u) sl[__popc(lm & lt)] = lb + lane;
+        if ((rm >> lane) & 1u) sr[__popc(rm & lt)] = rb - lane;
+        __syncwarp();
+        int pl = 0, pr = 0;
+        bool ok = false;
+        if (lane < t) {
+            pl = sl[lane]; pr = sr[lane];
+            ok = pl < pr;
+        }
+        const int n_ok = __popc(__ballot_sync(0xffffffffu, ok));
+        if (ok) { const int x = a[pl]; a[pl] = a[pr]; a[pr] = x; }
+        if (n_ok > 0) last_r = __shfl_sync(0xffffffffu, pr, n_ok - 1);
+        __syncwarp();
+        if (n_ok < t) return min(sl[n_ok], last_r);  // sl[n_ok]: the next left stopper
+        // drop the t lowest bits of both masks
+        const bool keep_l = ((lm >> lane) & 1u) && __popc(lm & lt) >= t;
+        const bool keep_r = ((rm >> lane) & 1u) && __popc(rm & lt) >= t;
+        lm = __ballot_sync(0xffffffffu, keep_l);
+        rm = __ballot_sync(0xffffffffu, keep_r);
+    }
+    const int next_l = lm ? lb + __ffs(lm) - 1 : 0x7fffffff;
+    return min(next_l, last_r);
+}
+
+struct SortRange {
+    int first, last, depth;
+};
+
+// Introsort of a[first0, last0) by one warp; unit indices to out[first0, last0).
+// `stack`: 40 ranges, `sl`, `sr`: 32 ints, all in shared memory and this warp's own.
+__device__ void warp_introsort(int* a, int* __restrict__ out, int first0, int last0, int depth0, SortRange* stack, int* sl,
+                               int* sr, int lane) {
+    int sp = 0;
+    int first = first0, last = last0, depth = depth0;
+    int pend_first = 0, pend_last = 0, n_pend = 0;  // lane k holds the k-th finished leaf
+    StdSort<UnitWordLess> S(a, UnitWordLess());
+    auto flush = [&]() {
+        __syncwarp();
+        if (lane < n_pend && pend_last - pend_first > 1) S.insertion_range(pend_first, pend_last);
+        for (int i = pend_first; lane < n_pend && i < pend_last; ++i) out[i] = a[i] & (int)kUnitMask;
+        n_pend = 0;
+        __syncwarp();
+    };
+    while (true) {
+        const int n = last - first;
+        bool done = false;
+        if (n <= 16) {
+            if (n > 0) {
+                if (lane == n_pend) { pend_first = first; pend_last = last; }
+                if (++n_pend == 32) flush();
             }
-            if (partner >= U) continue;  // idx stays unmatched
-            matched[idx] = 1;
-            matched[partner] = 1;
-            pa[G] = idx;
-            pb[G] = partner;
+            done = true;
+        } else {
+            const unsigned k0 = unit_key(a[first]);
+            bool equal = false;
+            if (n > 32 && k0 == unit_key(a[last - 1]) && k0 == unit_key(a[first + n / 2]) && depth >= equal_range_depth(n)) {
+                equal = true;
+                for (int i = first + lane; i - lane < last; i += 32)
+                    if (__ballot_sync(0xffffffffu, i < last && unit_key(a[i]) != k0)) { equal = false; break; }
+            }
+            if (equal) {
+                for (int i = lane; i < n; i += 32) out[first + i] = a[first + equal_range_source(n, i)] & (int)kUnitMask;
+                done = true;
+            } else if (depth == 0) {
+                if (lane == 0) S.heap_sort(first, n);
+                __syncwarp();
+                for (int i = first + lane; i < last; i += 32) out[i] = a[i] & (int)kUnitMask;
+                done = true;
+            }
+        }
+        if (done) {
+            if (sp == 0) break;
+            --sp;
+            __syncwarp();
+            first = stack[sp].first; last = stack[sp].last; depth = stack[sp].depth;
+            continue;
+        }
+        const int cut = warp_partition(a, first, last, sl, sr, lane);
+        --depth;
+        // the longer part waits, so that the stack stays short
+        const bool right_first = last - cut < cut - first;
+        if (lane == 0) stack[sp] = right_first ? SortRange{first, cut, depth} : SortRange{cut, last, depth};
+        ++sp;
+        __syncwarp();
+        if (right_first) first = cut; else last = cut;
+    }
+    flush();
+}
+
+// Greedy pass over the sorted order (block_online.cpp:365-386) by one warp.  The next unmatched unit of the
+// order is paired with the lowest unmatched unit, again and again.  Two windows of 32 are open at a
+// time: entries of the order (`alive`: still unmatched) and the bitmask word of the lowest unmatched units
+// (`cur`).  While no alive entry lies in that word the two are independent, and the k-th alive entry
+// simply gets the k-th free bit; otherwise one pair is made and the windows are looked at again.  Pair by
+// pair a warp needs 390 cycles each (a thread 320), which was 80 % of a hub window's matching.
+// `freem`: a bit per unmatched unit, `sl`: 32 ints of shared memory.  Returns the number of pairs; *left: the
+// unit that stays alone (-1: none).
+__device__ __forceinline__ int warp_greedy(int U, unsigned* freem, const int* order, int* __restrict__ pa, int* __restrict__ pb,
+                                           int* sl, int lane, int* left) {
+    const int words = (U + 31) / 32;
+    const unsigned lt = (1u << lane) - 1u;
+    int wpos = 0, G = 0;
+    unsigned cur = U > 0 ? freem[0] : 0u;
+    *left = -1;
+    auto advance = [&]() {   // to the next word with an unmatched unit; cur = 0: there is none
+        __syncwarp();
+        for (wpos += 1; wpos < words; wpos += 32) {
+            const unsigned f = wpos + lane < words ? freem[wpos + lane] : 0u;
+            const unsigned some = __ballot_sync(0xffffffffu, f != 0);
+            if (!some) continue;
+            const int at = __ffs(some) - 1;
+            wpos += at;
+            cur = __shfl_sync(0xffffffffu, f, at);
+            return;
+        }
+    };
+    int next = lane < U ? order[lane] : -1;
+    for (int k0 = 0; k0 < U; k0 += 32) {
+        const int idx = next;
+        next = k0 + 32 + lane < U ? order[k0 + 32 + lane] : -1;
+        __syncwarp();
+        const int word = idx >> 5;
+        unsigned f = 0;   // units in words before wpos are all matched
+        if (idx >= 0 && word >= wpos) f = word == wpos ? cur : freem[word];
+        unsigned alive = __ballot_sync(0xffffffffu, (f >> (idx & 31)) & 1u);
+        while (alive) {
+            if (cur == 0) advance();
+            const bool mine = (alive >> lane) & 1u;
+            if (__ballot_sync(0xffffffffu, mine && word == wpos) == 0) {
+                const int t = min(__popc(alive), __popc(cur));
+                const int ra = __popc(alive & lt), rb = __popc(cur & lt);
+                const bool bit = (cur >> lane) & 1u;
+                if (bit) sl[rb] = lane;
+                __syncwarp();
+                if (mine && ra < t) {
+                    pa[G + ra] = idx;
+                    pb[G + ra] = wpos * 32 + sl[ra];
+                    atomicAnd(freem + word, ~(1u << (idx & 31)));
+                }
+                G += t;
+                alive = __ballot_sync(0xffffffffu, mine && ra >= t);
+                cur = __ballot_sync(0xffffffffu, bit && rb >= t);
+                continue;
+            }
+            const int i = __ffs(alive) - 1;
+            alive &= alive - 1;
+            const int x = __shfl_sync(0xffffffffu, idx, i);
+            const unsigned keep = ~(1u << (x & 31));
+            if ((x >> 5) == wpos) cur &= keep;
+            else if (lane == 0) atomicAnd(freem + (x >> 5), keep);
+            if (cur == 0) advance();
+            if (cur == 0) { *left = x; return G; }
+            const int y = wpos * 32 + __ffs(cur) - 1;
+            cur &= cur - 1;
+            alive &= ~__ballot_sync(0xffffffffu, idx == y);
+            if (lane == 0) { pa[G] = x; pb[G] = y; }
             ++G;
         }
-        if (U & 1) {  // exactly one unit is left over
-            int left = 0;
-            while (matched[left]) ++left;
-            if ((int)nnz[left] >= unit_min_nnz) { pa[G] = left; pb[G] = -1; ++G; }
-            else cuda_unit = left;
-        }
     }
-    win_G[w] = G;
-    win_cuda_unit[w] = cuda_unit;
+    return G;
 }
 
-// ---------------------------------------------------------------------------------------------
-// Matching of a HEAVY window (tens of thousands to millions of units, the hub windows of a
-// power-law graph) by one thread block.  Same result as kb_match, different execution:
-//   * the std::sort emulation runs its partitions cooperatively.  An unguarded Hoare partition
-//     swaps the k-th element >= pivot from the left with the k-th element <= pivot from the
-//     right while the former lies left of the latter; with rank(i) = how many such elements
-//     precede i, every thread can decide locally whether its element takes part and where its
-//     partner is.  K swaps happen, the cut is min(position of the (K+1)-th left stopper, position
-//     of the K-th right stopper) — checked against libstdc++ on the host, see tests;
-//   * ranges of at most kParRange elements are finished by single threads with the sequential
-//     emulation (introsort loop + the insertion pass restricted to the range);
-//   * the greedy pass stays sequential (each step depends on all earlier ones) but runs out of
-//     shared memory: a bitmask of matched units and tiles of the sorted order.
-// ---------------------------------------------------------------------------------------------
-constexpr int kMediumUnits = 96;    // above: one warp per window
-constexpr int kHeavyUnits = 2048;    // above: one 256-thread block per window
-constexpr int kOrderTile = 2048;
+struct MatchOut {
+    int* order;       // [units] scratch: sorted unit indices
+    int* pair_a;      // [slots] groups in emission order: matched pairs, then the unmatched unit if it is kept
+    int* pair_b;
+    int* groups;      // [W + 1]
+    int* tiles;       // [W + 1]
+    int* cuda_unit;   // [W] unmatched unit that goes to the CUDA cores, -1: none
+};
 
-__global__ void kb_split_windows(const int* __restrict__ win_U, int W, int* __restrict__ light, int* __restrict__ medium,
-                                 int* __restrict__ heavy, int* __restrict__ counters /* n_light, n_medium, n_heavy, max U */) {
-    int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= W) return;
-    const int U = win_U[w];
-    if (U > kHeavyUnits) heavy[atomicAdd(&counters[2], 1)] = w;
-    else if (U > kMediumUnits) medium[atomicAdd(&counters[1], 1)] = w;
-    else light[atomicAdd(&counters[0], 1)] = w;
-    atomicMax(&counters[3], U);
+__device__ __forceinline__ int unit_word(const unsigned* __restrict__ key2, int rec0, int ncol, int u) {
+    int nnz = 16 - (int)(key2[rec0 + 2 * u] & 15u);
+    if (2 * u + 1 < ncol) nnz += 16 - (int)(key2[rec0 + 2 * u + 1] & 15u);
+    return (int)(((unsigned)nnz << kUnitBits) | (unsigned)u);
 }
 
-template <int kHeavyThreads, int kParRange>
-__global__ void __launch_bounds__(kHeavyThreads) kb_match_coop(
-    const int* __restrict__ win_U, const int* __restrict__ win_ub, const int* __restrict__ win_pb, int unit_min_nnz,
-    const unsigned char* __restrict__ unit_nnz, int* __restrict__ order_buf, unsigned char* __restrict__ matched_buf,
-    int* __restrict__ pair_a, int* __restrict__ pair_b, int* __restrict__ win_G, int* __restrict__ win_cuda_unit,
-    const int* __restrict__ sel, int mask_words_cap) {
-    extern __shared__ unsigned int dyn[];   // [mask_words_cap] matched bitmask, then [kOrderTile] order tile
-    __shared__ int s_stack[64][3];
-    __shared__ int s_small[kHeavyThreads][3];
-    __shared__ int s_scan[kHeavyThreads];
-    __shared__ int s_sp, s_nsmall, s_K, s_lnext, s_cur[3], s_G, s_cuda;
-    const int tid = threadIdx.x;
+__device__ __forceinline__ void match_finish(int w, int G, int left, int left_nnz, int unit_min_nnz, const MatchOut& o, int slot0) {
+    int cuda = -1;
+    if (left >= 0) {
+        if (left_nnz >= unit_min_nnz) { o.pair_a[slot0 + G] = left; o.pair_b[slot0 + G] = -1; ++G; }
+        else cuda = left;
+    }
+    o.groups[w] = G;
+    o.tiles[w] = (G + 3) / 4;
+    o.cuda_unit[w] = cuda;
+}
+
+constexpr int kMatchWarps = 4;
+struct MatchWarpSmem {
+    SortRange stack[40];
+    int sl[32], sr[32];
+};
+
+// Windows of at most `max_units` units, one warp each.  Dynamic shared memory: per warp max_units words
+// and the bitmask.
+__global__ void __launch_bounds__(32 * kMatchWarps) kb_match_warp(WindowView v, int W, const unsigned* __restrict__ key2,
+                                                                  int unit_min_nnz, int max_units, MatchOut o) {
+    extern __shared__ int dyn[];
+    __shared__ MatchWarpSmem s_warp[kMatchWarps];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int w = blockIdx.x * kMatchWarps + wid;
+    if (w > W) return;
+    if (w == W) { if (lane == 0) { o.groups[W] = 0; o.tiles[W] = 0; } return; }
+    const Win p0 = v.pre[w];
+    const int U = v.pre[w + 1].units - p0.units;
+    if (U > max_units) return;
+    const int rec0 = v.rec[w] + v.tc[w], ncol = v.rec[w + 1] - rec0;
+    int* a = dyn + wid * (max_units + (max_units + 31) / 32);
+    unsigned* freem = (unsigned*)(a + max_units);
+    int* order = o.order + p0.units;
+    for (int i = lane; i < U; i += 32) a[i] = unit_word(key2, rec0, ncol, i);
+    for (int i = lane; i < (U + 31) / 32; i += 32) freem[i] = U - 32 * i >= 32 ? 0xffffffffu : (1u << (U - 32 * i)) - 1u;
+    __syncwarp();
+    MatchWarpSmem& m = s_warp[wid];
+    // units come in descending order already: an insertion sort of at most 16 of them moves nothing
+    if (U > 16) {
+        warp_introsort(a, order, 0, U, 2 * StdSort<UnitWordLess>::floor_log2(U), m.stack, m.sl, m.sr, lane);
+    } else if (lane < U) {
+        order[lane] = lane;
+    }
+    __syncwarp();   // `order` is read back by the lanes of the warp that wrote it
+    int left;
+    const int G = warp_greedy(U, freem, order, o.pair_a + p0.slots, o.pair_b + p0.slots, m.sl, lane, &left);
+    if (lane == 0) match_finish(w, G, left, left >= 0 ? (int)unit_key(unit_word(key2, rec0, ncol, left)) : 0, unit_min_nnz, o, p0.slots);
+}
+
+// Hub windows, one block each: long ranges are partitioned or traced by the whole block, ranges of
+// at most kWarpRange units are left to single warps.  The words live in dynamic shared memory when
+// they fit (smem_units), in `words_global` otherwise; the bitmask takes the same memory afterwards
+// (or `mask_global`).
+constexpr int kBlockThreads = 256, kWarpRange = 1024, kMaxRanges = 256;
+
+__global__ void __launch_bounds__(kBlockThreads) kb_match_block(WindowView v, const unsigned* __restrict__ key2, int unit_min_nnz,
+                                                                int smem_units, int* __restrict__ words_global,
+                                                                unsigned* __restrict__ mask_global, const int* __restrict__ sel,
+                                                                MatchOut o) {
+    extern __shared__ int dyn[];
+    __shared__ MatchWarpSmem s_warp[kBlockThreads / 32];
+    __shared__ SortRange s_stack[64], s_small[kMaxRanges];
+    __shared__ int s_scan[kBlockThreads / 32];
+    __shared__ int s_sp, s_nsmall, s_take, s_lnext;
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
     const int w = sel[blockIdx.x];
-    const int U = win_U[w];
-    const unsigned char* nnz = unit_nnz + win_ub[w];
-    int* order = order_buf + win_ub[w];
-    int* swapL = pair_a + win_pb[w];   // scratch during the sort, pair list afterwards
-    int* swapR = pair_b + win_pb[w];
-    for (int i = tid; i < U; i += kHeavyThreads) order[i] = i;
+    const Win p0 = v.pre[w];
+    const int U = v.pre[w + 1].units - p0.units;
+    const int rec0 = v.rec[w] + v.tc[w], ncol = v.rec[w + 1] - rec0;
+    const bool in_smem = U <= smem_units;
+    int* a = in_smem ? dyn : words_global + p0.units;
+    int* order = o.order + p0.units;
+    int* swapL = o.pair_a + p0.slots;   // scratch during the sort, pair list afterwards
+    int* swapR = o.pair_b + p0.slots;
+    for (int i = tid; i < U; i += kBlockThreads) a[i] = unit_word(key2, rec0, ncol, i);
     if (tid == 0) {
-        s_stack[0][0] = 0; s_stack[0][1] = U; s_stack[0][2] = 2 * StdSort<UnitLess>::floor_log2(U);
+        s_stack[0] = SortRange{0, U, 2 * StdSort<UnitWordLess>::floor_log2(U)};
         s_sp = 1; s_nsmall = 0;
     }
     __syncthreads();
-    StdSort<UnitLess> S(order, UnitLess{nnz});
+    StdSort<UnitWordLess> S(a, UnitWordLess());
 
-    auto block_excl_scan = [&](int v, int& total) -> int {  // exclusive scan over threads (in order)
-        s_scan[tid] = v;
-        __syncthreads();
-        for (int off = 1; off < kHeavyThreads; off <<= 1) {
-            const int t = tid >= off ? s_scan[tid - off] : 0;
-            __syncthreads();
-            s_scan[tid] += t;
-            __syncthreads();
+    auto block_excl_scan = [&](int x, int& total) -> int {
+        int incl = x;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += y;
         }
-        total = s_scan[kHeavyThreads - 1];
-        const int ex = s_scan[tid] - v;
+        if (lane == 31) s_scan[wid] = incl;
         __syncthreads();
-        return ex;
+        int before = 0;
+        total = 0;
+#pragma unroll
+        for (int q = 0; q < kBlockThreads / 32; ++q) {
+            if (q < wid) before += s_scan[q];
+            total += s_scan[q];
+        }
+        __syncthreads();
+        return before + incl - x;
     };
-    auto run_small = [&]() {  // every thread finishes one small range
+    auto run_small = [&]() {   // the warps take the waiting ranges one after the other
         __syncthreads();
-        if (tid < s_nsmall) {
-            const int f = s_small[tid][0], l = s_small[tid][1], d = s_small[tid][2];
-            if (d < 0) S.heap_sort(f, l - f);
-            else { S.introsort_range(f, l, d); S.insertion_range(f, l); }
+        if (tid == 0) s_take = 0;
+        __syncthreads();
+        const int n = s_nsmall;
+        while (true) {
+            int q = 0;
+            if (lane == 0) q = atomicAdd(&s_take, 1);
+            q = __shfl_sync(0xffffffffu, q, 0);
+            if (q >= n) break;
+            const SortRange r = s_small[q];
+            warp_introsort(a, order, r.first, r.last, r.depth, s_warp[wid].stack, s_warp[wid].sl, s_warp[wid].sr, lane);
         }
         __syncthreads();
         if (tid == 0) s_nsmall = 0;
@@ -331,40 +615,45 @@ __global__ void __launch_bounds__(kHeavyThreads) kb_match_coop(
 
     while (true) {
         __syncthreads();
-        const int sp_now = s_sp;   // read by everyone before thread 0 pops
+        const int sp = s_sp;
+        if (sp == 0) break;
+        const SortRange r = s_stack[sp - 1];
         __syncthreads();
-        if (sp_now == 0) break;
-        if (tid == 0) {
-            --s_sp;
-            s_cur[0] = s_stack[s_sp][0]; s_cur[1] = s_stack[s_sp][1]; s_cur[2] = s_stack[s_sp][2];
-        }
-        __syncthreads();
-        const int first = s_cur[0], last = s_cur[1];
-        int depth = s_cur[2];
-        if (last - first <= kParRange || depth == 0) {
-            if (last - first > 1) {
-                if (tid == 0) {
-                    s_small[s_nsmall][0] = first; s_small[s_nsmall][1] = last;
-                    s_small[s_nsmall][2] = (last - first > kParRange) ? -1 : depth;   // -1: depth exhausted -> heap sort
-                    ++s_nsmall;
-                }
-                __syncthreads();
-                if (s_nsmall == kHeavyThreads) run_small();
-            }
+        const int first = r.first, last = r.last, n = last - first;
+        if (n <= kWarpRange) {
+            if (tid == 0) { s_small[s_nsmall++] = r; s_sp = sp - 1; }
+            __syncthreads();
+            if (s_nsmall == kMaxRanges) run_small();
             continue;
         }
-        --depth;
-        if (tid == 0) S.move_median_to_first(first, first + 1, first + (last - first) / 2, last - 1);
+        const unsigned k0 = unit_key(a[first]);
+        const bool maybe_equal = k0 == unit_key(a[last - 1]) && k0 == unit_key(a[first + n / 2]) && r.depth >= equal_range_depth(n);
+        __syncthreads();   // everyone has looked before anything moves
+        if (maybe_equal) {
+            int differ = 0;
+            for (int i = first + tid; i < last; i += kBlockThreads) differ |= unit_key(a[i]) != k0;
+            if (!__syncthreads_or(differ)) {
+                for (int i = tid; i < n; i += kBlockThreads) order[first + i] = a[first + equal_range_source(n, i)] & (int)kUnitMask;
+                if (tid == 0) s_sp = sp - 1;
+                continue;
+            }
+        }
+        if (r.depth == 0) {
+            if (tid == 0) { S.heap_sort(first, n); s_sp = sp - 1; }
+            __syncthreads();
+            for (int i = first + tid; i < last; i += kBlockThreads) order[i] = a[i] & (int)kUnitMask;
+            continue;
+        }
+        if (tid == 0) S.move_median_to_first(first, first + 1, first + n / 2, last - 1);
         __syncthreads();
-        const int pvk = nnz[order[first]];
-        const int lo = first + 1, n = last - lo;
-        const int chunk = (n + kHeavyThreads - 1) / kHeavyThreads;
+        const unsigned pvk = unit_key(a[first]);
+        const int lo = first + 1, m = last - lo;
+        const int chunk = (m + kBlockThreads - 1) / kBlockThreads;
         const int cb = min(lo + tid * chunk, last), ce = min(cb + chunk, last);
-        // pass 1: stoppers per chunk.  left stopper: key <= pivot key (not less than the pivot in
-        // the descending order); right stopper: key >= pivot key
+        // pass 1: stoppers per chunk (left: key <= pivot, right: key >= pivot)
         int cL = 0, cR = 0;
         for (int i = cb; i < ce; ++i) {
-            const int k = nnz[order[i]];
+            const unsigned k = unit_key(a[i]);
             cL += (k <= pvk);
             cR += (k >= pvk);
         }
@@ -375,7 +664,7 @@ __global__ void __launch_bounds__(kHeavyThreads) kb_match_coop(
         // pass 2a: which left stoppers swap; K = their number
         int lrank = baseL, rem = cR, myswaps = 0;
         for (int i = cb; i < ce; ++i) {
-            const int k = nnz[order[i]];
+            const unsigned k = unit_key(a[i]);
             int right_of_i = baseRright + rem;
             if (k >= pvk) { right_of_i -= 1; rem -= 1; }
             if (k <= pvk) {
@@ -390,7 +679,7 @@ __global__ void __launch_bounds__(kHeavyThreads) kb_match_coop(
         // pass 2b: the partners on the right, and the (K+1)-th left stopper
         lrank = baseL; rem = cR;
         for (int i = cb; i < ce; ++i) {
-            const int k = nnz[order[i]];
+            const unsigned k = unit_key(a[i]);
             if (k >= pvk) {
                 const int rrank = baseRright + rem;   // rank from the right, 1-based
                 if (rrank <= K) swapR[rrank - 1] = i;
@@ -402,347 +691,38 @@ __global__ void __launch_bounds__(kHeavyThreads) kb_match_coop(
             }
         }
         __syncthreads();
-        const int cut = min(s_lnext, K >= 1 ? swapR[K - 1] : 0x7fffffff);
-        __syncthreads();
-        for (int k = tid; k < K; k += kHeavyThreads) {
-            const int a = swapL[k], b = swapR[k];
-            const int t = order[a]; order[a] = order[b]; order[b] = t;
-        }
-        __syncthreads();
         if (tid == 0) {
-            s_stack[s_sp][0] = cut; s_stack[s_sp][1] = last; s_stack[s_sp][2] = depth; ++s_sp;
-            s_stack[s_sp][0] = first; s_stack[s_sp][1] = cut; s_stack[s_sp][2] = depth; ++s_sp;
+            const int cut = min(s_lnext, K >= 1 ? swapR[K - 1] : 0x7fffffff);
+            s_stack[sp - 1] = SortRange{cut, last, r.depth - 1};
+            s_stack[sp] = SortRange{first, cut, r.depth - 1};
+            s_sp = sp + 1;
+        }
+        for (int k = tid; k < K; k += kBlockThreads) {
+            const int x = swapL[k], y = swapR[k];
+            const int t = a[x]; a[x] = a[y]; a[y] = t;
         }
     }
     run_small();
 
-    // ---- greedy pass (block_online.cpp:365-386), thread 0 over shared-memory tiles --------------
+    // the bitmask: in shared memory up to 32 * smem_units units
     const int words = (U + 31) / 32;
-    const bool in_smem = words <= mask_words_cap;
-    unsigned int* mask = dyn;
-    int* tile = (int*)(dyn + mask_words_cap);
-    unsigned char* matched = matched_buf + win_ub[w];
-    if (in_smem) { for (int i = tid; i < words; i += kHeavyThreads) mask[i] = 0u; }
-    else { for (int i = tid; i < U; i += kHeavyThreads) matched[i] = 0; }
-    if (tid == 0) { s_G = 0; s_cuda = -1; s_cur[0] = 0; }
+    unsigned* gmask = mask_global + p0.units / 32 + w;
+    const bool mask_in_smem = words <= smem_units;
+    for (int i = tid; i < words; i += kBlockThreads) {
+        const unsigned all = U - 32 * i >= 32 ? 0xffffffffu : (1u << (U - 32 * i)) - 1u;
+        if (mask_in_smem) dyn[i] = (int)all; else gmask[i] = all;
+    }
     __syncthreads();
-    auto is_set = [&](int i) -> bool { return in_smem ? ((mask[i >> 5] >> (i & 31)) & 1u) != 0 : matched[i] != 0; };
-    auto set_bit = [&](int i) { if (in_smem) mask[i >> 5] |= 1u << (i & 31); else matched[i] = 1; };
-    for (int k0 = 0; k0 < U; k0 += kOrderTile) {
-        const int len = min(kOrderTile, U - k0);
-        for (int i = tid; i < len; i += kHeavyThreads) tile[i] = order[k0 + i];
-        __syncthreads();
-        if (tid == 0) {
-            int G = s_G, lowest = s_cur[0];
-            for (int k = 0; k < len; ++k) {
-                const int idx = tile[k];
-                if (is_set(idx)) continue;
-                while (lowest < U && is_set(lowest)) ++lowest;
-                int partner = lowest;
-                if (partner == idx) {
-                    ++partner;
-                    while (partner < U && is_set(partner)) ++partner;
-                }
-                if (partner >= U) continue;
-                set_bit(idx); set_bit(partner);
-                swapL[G] = idx; swapR[G] = partner;   // pair_a / pair_b of this window
-                ++G;
-            }
-            s_G = G; s_cur[0] = lowest;
-        }
-        __syncthreads();
-    }
-    if (tid == 0) {
-        int G = s_G;
-        if (U & 1) {
-            int left = 0;
-            while (is_set(left)) ++left;
-            if ((int)nnz[left] >= unit_min_nnz) { swapL[G] = left; swapR[G] = -1; ++G; }
-            else s_cuda = left;
-        }
-        win_G[w] = G;
-        win_cuda_unit[w] = s_cuda;
-    }
+    if (wid > 0) return;
+    int left;
+    const int G = mask_in_smem ? warp_greedy(U, (unsigned*)dyn, order, swapL, swapR, s_warp[0].sl, lane, &left)
+                               : warp_greedy(U, gmask, order, swapL, swapR, s_warp[0].sl, lane, &left);
+    if (lane == 0) match_finish(w, G, left, left >= 0 ? (int)unit_key(unit_word(key2, rec0, ncol, left)) : 0, unit_min_nnz, o, p0.slots);
 }
 
-__device__ __forceinline__ int find_window(const int* __restrict__ prefix, int W, int x) {
-    // largest w in [0, W) with prefix[w] <= x   (prefix non-decreasing, prefix[W] > x)
-    int lo = 0, hi = W;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if (prefix[mid] <= x) lo = mid; else hi = mid;
-    }
-    return lo;
-}
-
-// one thread per pair slot: the group's columns, sorted ascending
-__global__ void kb_emit_groups(const int* __restrict__ win_pb, const int* __restrict__ win_G,
-                               const int* __restrict__ s_offset, const int* __restrict__ win_cb,
-                               const int* __restrict__ win_U, const int* __restrict__ wc_begin,
-                               const int* __restrict__ s_idx, int W, int total_slots, const int* __restrict__ pair_a,
-                               const int* __restrict__ pair_b, const int* __restrict__ cand,
-                               const int* __restrict__ wc_col, int* __restrict__ s_column, int* __restrict__ s_window,
-                               int* __restrict__ grp_wcol) {
-    int q = blockIdx.x * blockDim.x + threadIdx.x;
-    if (q >= total_slots) return;
-    const int w = find_window(win_pb, W, q);
-    const int k = q - win_pb[w];
-    if (k >= win_G[w]) return;
-    const int g = s_offset[w] + k;
-    const int cb = win_cb[w];
-    const int ns = s_idx[wc_begin[w + 1]] - cb;
-    int ids[4], cols[4], n = 0;
-    const int ua = pair_a[q], ub = pair_b[q];
-    for (int side = 0; side < 2; ++side) {
-        const int u = side ? ub : ua;
-        if (u < 0) continue;
-        for (int i = 0; i < 2; ++i) {
-            const int ls = 2 * u + i;
-            if (ls < ns) { ids[n] = cand[cb + ls]; cols[n] = wc_col[ids[n]]; ++n; }
-        }
-    }
-    for (int i = 1; i < n; ++i) {  // insertion sort by column id
-        const int c = cols[i], id = ids[i];
-        int k2 = i - 1;
-        while (k2 >= 0 && cols[k2] > c) { cols[k2 + 1] = cols[k2]; ids[k2 + 1] = ids[k2]; --k2; }
-        cols[k2 + 1] = c; ids[k2 + 1] = id;
-    }
-    for (int p = 0; p < 4; ++p) {
-        s_column[(size_t)g * 4 + p] = p < n ? cols[p] : -1;
-        grp_wcol[(size_t)g * 4 + p] = p < n ? ids[p] : -1;
-    }
-    s_window[g] = w;
-}
-
-// one thread per (group, local row): mask byte and the first two (value, position) slots.
-// In strict mode the non-zeros beyond the second one (which the reference drops) are recorded in
-// `extra_key` / `extra_at` (key = row << 32 | column) so that they can join the row's CUDA-core part.
-__global__ void kb_emit_rows(const int* __restrict__ grp_wcol, long long total, int window,
-                             const unsigned short* __restrict__ wc_mask, const int* __restrict__ wc_start,
-                             const int* __restrict__ wc_col, const int* __restrict__ s_window,
-                             const int* __restrict__ edge, const float* __restrict__ val,
-                             unsigned char* __restrict__ s_mask, float* __restrict__ s_value,
-                             signed char* __restrict__ s_pos, unsigned long long* __restrict__ dropped,
-                             unsigned long long* __restrict__ extra_key, int* __restrict__ extra_at,
-                             unsigned long long* __restrict__ extra_count, int* __restrict__ row_extra, int write_arrays) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= total) return;
-    const long long g = i / window;
-    const int lr = (int)(i - g * window);
-    unsigned mask = 0;
-    int slots = 0;
-    float rv[2] = {0.f, 0.f};
-    int rp[2] = {-1, -1};
-    for (int p = 0; p < 4; ++p) {
-        const int j = grp_wcol[g * 4 + p];
-        if (j < 0) break;
-        const unsigned m = wc_mask[j];
-        if (!((m >> lr) & 1u)) continue;
-        mask |= 1u << p;
-        const int at = wc_start[j] + __popc(m & ((1u << lr) - 1u));
-        if (slots < 2) {
-            rv[slots] = val[edge[at]];
-            rp[slots] = p;
-        } else if (extra_key) {
-            const unsigned long long k = atomicAdd(extra_count, 1ull);
-            const long long row = (long long)s_window[g] * window + lr;
-            extra_key[k] = ((unsigned long long)row << 32) | (unsigned)wc_col[j];
-            extra_at[k] = at;
-            atomicAdd(&row_extra[row], 1);
-        }
-        ++slots;
-    }
-    if (!write_arrays) return;
-    if (slots > 2) atomicAdd(dropped, (unsigned long long)(slots - 2));
-    s_mask[i] = (unsigned char)mask;
-    s_value[i * 2] = rv[0];
-    s_value[i * 2 + 1] = rv[1];
-    s_pos[i * 2] = (signed char)rp[0];
-    s_pos[i * 2 + 1] = (signed char)rp[1];
-}
-
-// one thread per TC block: columns ascending, bitmaps, value count; records each column's slot
-__global__ void kb_tc_blocks(const int* __restrict__ blk_pos, const int* __restrict__ blk_len, int NB,
-                             const int* __restrict__ ord, const int* __restrict__ wc_col,
-                             const unsigned short* __restrict__ wc_mask, int* __restrict__ t_column,
-                             long long* __restrict__ t_binary, int* __restrict__ blk_nnz, int* __restrict__ wc_slot) {
-    int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= NB) return;
-    const int p0 = blk_pos[b], len = blk_len[b];
-    int ids[8], cols[8];
-    for (int i = 0; i < len; ++i) { ids[i] = ord[p0 + i]; cols[i] = wc_col[ids[i]]; }
-    for (int i = 1; i < len; ++i) {
-        const int c = cols[i], id = ids[i];
-        int k = i - 1;
-        while (k >= 0 && cols[k] > c) { cols[k + 1] = cols[k]; ids[k + 1] = ids[k]; --k; }
-        cols[k + 1] = c; ids[k + 1] = id;
-    }
-    u64 lo = 0, hi = 0;
-    for (int k = 0; k < 8; ++k) {
-        t_column[(size_t)b * 8 + k] = k < len ? cols[k] : -1;
-        if (k >= len) continue;
-        wc_slot[ids[k]] = b * 8 + k;
-        const unsigned m = wc_mask[ids[k]];
-        for (int r = 0; r < 8; ++r) {
-            if ((m >> r) & 1u) lo |= 1ull << (r * 8 + k);
-            if ((m >> (r + 8)) & 1u) hi |= 1ull << (r * 8 + k);
-        }
-    }
-    t_binary[(size_t)b * 2] = (long long)lo;
-    t_binary[(size_t)b * 2 + 1] = (long long)hi;
-    blk_nnz[b] = __popcll(lo) + __popcll(hi);
-}
-
-// one thread per sorted entry: entries of TC columns go to their slot of t_value
-__global__ void kb_tc_values(const u64* __restrict__ keys, const int* __restrict__ edge,
-                             const int* __restrict__ wc_incl, long long nnz, const int* __restrict__ wc_slot,
-                             const long long* __restrict__ t_binary, const int* __restrict__ t_block_offset,
-                             const float* __restrict__ val, float* __restrict__ t_value) {
-    long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nnz) return;
-    const int slot = wc_slot[wc_incl[i] - 1];
-    if (slot < 0) return;
-    const int b = slot >> 3, k = slot & 7;
-    const int lr = (int)(keys[i] & 15);
-    const u64 lo = (u64)t_binary[(size_t)b * 2], hi = (u64)t_binary[(size_t)b * 2 + 1];
-    const int bit = (lr & 7) * 8 + k;
-    int rank;
-    if (lr < 8) rank = __popcll(lo & ((1ull << bit) - 1ull));
-    else rank = __popcll(lo) + __popcll(hi & ((1ull << bit) - 1ull));
-    t_value[(size_t)t_block_offset[b] + rank] = val[edge[i]];
-}
-
-__global__ void kb_tc_parts(const int* __restrict__ wc_begin, const int* __restrict__ b_idx,
-                            const int* __restrict__ win_bb, const int* __restrict__ part_off,
-                            const int* __restrict__ win_cuda_unit, int W, int part_t, int* __restrict__ t_row_offset,
-                            int* __restrict__ t_window_row, int* __restrict__ t_atomic) {
-    int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w == 0) t_row_offset[0] = 0;
-    if (w >= W) return;
-    const int bb = win_bb[w];
-    const int nb = b_idx[wc_begin[w + 1]] - bb;
-    if (nb == 0) return;
-    const int p0 = part_off[w];
-    if (nb <= part_t) {
-        t_row_offset[p0 + 1] = bb + nb;
-        t_window_row[p0] = w * 16;
-        t_atomic[p0] = win_cuda_unit[w] >= 0 ? 1 : 0;
-        return;
-    }
-    const int np = (nb + part_t - 1) / part_t;
-    for (int q = 0; q < np; ++q) {
-        t_row_offset[p0 + q + 1] = bb + min((q + 1) * part_t, nb);
-        t_window_row[p0 + q] = w * 16;
-        t_atomic[p0 + q] = 1;
-    }
-}
-
-// CUDA-core leftovers: the (at most two) columns of the window's rejected unit.  Per row the
-// entries come in ascending column order = CSR order.
-struct CudaRow {
-    int n;
-    int cols[2];
-    int at[2];  // position in the sorted entry array
-};
-__device__ __forceinline__ CudaRow cuda_row(int r, int window, const int* win_cuda_unit, const int* win_cb,
-                                            const int* wc_begin, const int* s_idx, const int* cand, const int* wc_col,
-                                            const unsigned short* wc_mask, const int* wc_start) {
-    CudaRow out;
-    out.n = 0;
-    const int w = r / window, lr = r - w * window;
-    const int u = win_cuda_unit[w];
-    if (u < 0) return out;
-    const int cb = win_cb[w];
-    const int ns = s_idx[wc_begin[w + 1]] - cb;
-    for (int i = 0; i < 2; ++i) {
-        const int ls = 2 * u + i;
-        if (ls >= ns) break;
-        const int j = cand[cb + ls];
-        const unsigned m = wc_mask[j];
-        if (!((m >> lr) & 1u)) continue;
-        out.cols[out.n] = wc_col[j];
-        out.at[out.n] = wc_start[j] + __popc(m & ((1u << lr) - 1u));
-        ++out.n;
-    }
-    if (out.n == 2 && out.cols[0] > out.cols[1]) {
-        int t = out.cols[0]; out.cols[0] = out.cols[1]; out.cols[1] = t;
-        t = out.at[0]; out.at[0] = out.at[1]; out.at[1] = t;
-    }
-    return out;
-}
-
-// split rule of block_online.cpp:415-439 as (long parts, short parts, long nnz, short nnz)
-__device__ __forceinline__ void split_counts(int n, int part_c, int short_size, int& nl, int& ns, int& zl, int& zs) {
-    nl = ns = zl = zs = 0;
-    if (n <= 0) return;
-    if (n <= short_size) { ns = 1; zs = n; return; }
-    if (n <= part_c) { nl = 1; zl = n; return; }
-    nl = n / part_c;
-    zl = nl * part_c;
-    const int residue = n % part_c;
-    if (residue > 0) {
-        if (residue <= short_size) { ns = 1; zs = residue; }
-        else { nl += 1; zl += residue; }
-    }
-}
-
-__global__ void kb_cuda_count(int n_rows, int window, int part_c, int short_size, const int* win_cuda_unit,
-                              const int* win_cb, const int* wc_begin, const int* s_idx, const int* cand,
-                              const int* wc_col, const unsigned short* wc_mask, const int* wc_start,
-                              const int* __restrict__ row_extra, int* __restrict__ cnt /* 4 arrays of n_rows + 1 */) {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r >= n_rows) return;
-    const CudaRow cr = cuda_row(r, window, win_cuda_unit, win_cb, wc_begin, s_idx, cand, wc_col, wc_mask, wc_start);
-    int nl, ns, zl, zs;
-    split_counts(cr.n + (row_extra ? row_extra[r] : 0), part_c, short_size, nl, ns, zl, zs);
-    const size_t stride = (size_t)n_rows + 1;
-    cnt[r] = nl; cnt[stride + r] = ns; cnt[2 * stride + r] = zl; cnt[3 * stride + r] = zs;
-}
-
-// The row's leftover entries in ascending column order: the (at most two) entries of the window's
-// rejected unit merged with the row's strict-mode extras (sorted by column beforehand).
-__global__ void kb_cuda_fill(int n_rows, int window, int part_c, int short_size, const int* win_cuda_unit,
-                             const int* win_cb, const int* wc_begin, const int* s_idx, const int* b_idx,
-                             const int* cand, const int* wc_col, const unsigned short* wc_mask, const int* wc_start,
-                             const int* edge, const float* val, const int* __restrict__ off,
-                             const int* __restrict__ extra_off, const unsigned long long* __restrict__ extra_key,
-                             const int* __restrict__ extra_at,
-                             int* c_row_offset, int* c_row, int* c_atomic, int* c_column, float* c_value,
-                             int* cs_row_offset, int* cs_row, int* cs_atomic, int* cs_column, float* cs_value) {
-    int r = blockIdx.x * blockDim.x + threadIdx.x;
-    if (r == 0) { c_row_offset[0] = 0; cs_row_offset[0] = 0; }
-    if (r >= n_rows) return;
-    const CudaRow cr = cuda_row(r, window, win_cuda_unit, win_cb, wc_begin, s_idx, cand, wc_col, wc_mask, wc_start);
-    const int xb = extra_off ? extra_off[r] : 0, xe = extra_off ? extra_off[r + 1] : 0;
-    const int n = cr.n + (xe - xb);
-    if (n <= 0) return;
-    const int w = r / window;
-    const int base_atomic = (b_idx[wc_begin[w + 1]] - b_idx[wc_begin[w]]) > 0 ? 1 : 0;
-    const size_t stride = (size_t)n_rows + 1;
-    int pl = off[r], ps = off[stride + r], zl = off[2 * stride + r], zs = off[3 * stride + r];
-    int iu = 0, ix = xb;  // cursors of the two sorted sources
-    auto next = [&](int& c, float& v) {
-        const int xc = ix < xe ? (int)(extra_key[ix] & 0xffffffffull) : 0x7fffffff;
-        if (iu < cr.n && cr.cols[iu] < xc) { c = cr.cols[iu]; v = val[edge[cr.at[iu]]]; ++iu; }
-        else { c = xc; v = val[edge[extra_at[ix]]]; ++ix; }
-    };
-    auto put = [&](int atomic, int cnt, bool residue) {
-        for (int i = 0; i < cnt; ++i) {
-            int c; float v;
-            next(c, v);
-            if (residue) { cs_column[zs + i] = c; cs_value[zs + i] = v; }
-            else { c_column[zl + i] = c; c_value[zl + i] = v; }
-        }
-        if (residue) { zs += cnt; cs_row[ps] = r; cs_atomic[ps] = atomic; cs_row_offset[ps + 1] = zs; ++ps; }
-        else { zl += cnt; c_row[pl] = r; c_atomic[pl] = atomic; c_row_offset[pl + 1] = zl; ++pl; }
-    };
-    if (n <= short_size) { put(base_atomic, n, true); return; }
-    if (n <= part_c) { put(base_atomic, n, false); return; }
-    for (int i = 0; i < n / part_c; ++i) put(1, part_c, false);
-    const int residue = n % part_c;
-    if (residue > 0) put(1, residue, residue <= short_size);
-}
-
+// ---------------------------------------------------------------------------------------------
+// 7. groups and tiles
+// ---------------------------------------------------------------------------------------------
 __global__ void kb_tiles(const int* __restrict__ tile_off, const int* __restrict__ s_offset, int W, int T,
                          int* __restrict__ s_tile_window, int* __restrict__ s_tile_group) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -752,14 +732,443 @@ __global__ void kb_tiles(const int* __restrict__ tile_off, const int* __restrict
     s_tile_group[t] = s_offset[w] + 4 * (t - tile_off[w]);
 }
 
-__global__ void kb_win_tiles(const int* __restrict__ win_G, int W, int* __restrict__ win_T) {
-    int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w < W) win_T[w] = (win_G[w] + 3) / 4;
+struct RecordView {
+    const int* ord;               // records in (window, count desc, column asc) order
+    const Record* rec;            // by record id
+    const unsigned* ent;          // sorted entries
+    const float* val;             // CSR values
+    int packed;                   // entries are (entry << 4 | local row)
+    __device__ __forceinline__ int entry(int at) const { return (int)(packed ? ent[at] >> 4 : ent[at]); }
+    // value of the record's k-th entry (most records of a power-law graph have one)
+    __device__ __forceinline__ float value(int start, float first, int k) const { return k == 0 ? first : val[entry(start + k)]; }
+};
+
+struct GroupOut {
+    int* s_column;
+    unsigned char* s_mask;
+    float* s_value;
+    signed char* s_pos;
+    int* s_window;
+    int* s_tile_column;
+    uint32_t* packed_a;
+    uint32_t* packed_meta;
+};
+
+// Non-zeros beyond the second one of a row inside a group, which the reference drops: counted, and
+// in strict mode recorded (key = row << 32 | column) so that they can join the row's CUDA-core part.
+constexpr int kDropCounters = 64;
+struct ExtraOut {
+    u64* count; // strict: length of the list; otherwise kDropCounters counters, one per block number modulo
+    u64* key;
+    int* at;    // entry
+};
+
+// One warp per tile of four groups: lane (q, g) = (lane / 8, lane % 8) owns rows g and g + 8 of group q,
+// which are also the two rows of its word pair in the packed tile.  One pass writes the un-packed arrays
+// (196 bytes per group) and the tile (352 bytes); reading the un-packed arrays back to pack them, and an
+// atomic per dropped entry, were most of the 0.63 ms the separate kernels took on the clustered
+// graph (0.09 ms now).
+template <bool STRICT>
+__global__ void __launch_bounds__(256) kb_emit_tiles(WindowView v, RecordView r, const int* __restrict__ s_offset,
+                                                     const int* __restrict__ tile_window, const int* __restrict__ tile_group,
+                                                     int T, int window, const int* __restrict__ pair_a,
+                                                     const int* __restrict__ pair_b, GroupOut o, ExtraOut x) {
+    // strict mode: a warp's extras wait in shared memory for a common place in the list (a tile has at
+    // most 128; one atomic per tile on the one counter would be the slowest part)
+    constexpr int kWait = STRICT ? 256 : 1;
+    __shared__ u64 s_key[8][kWait];
+    __shared__ int s_at[8][kWait];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = lane >> 3, g = lane & 7;
+    int waiting = 0;
+    auto flush = [&]() {
+        __syncwarp();
+        u64 at = 0;
+        if (lane == 0) at = atomicAdd(x.count, (u64)waiting);
+        at = __shfl_sync(0xffffffffu, at, 0);
+        for (int i = lane; i < waiting; i += 32) { x.key[at + i] = s_key[wid][i]; x.at[at + i] = s_at[wid][i]; }
+        waiting = 0;
+        __syncwarp();
+    };
+    int dropped = 0;
+    for (int t = blockIdx.x * 8 + wid; t < T; t += gridDim.x * 8) {
+        const int w = tile_window[t];
+        const int gid = tile_group[t] + q;
+        const int off = s_offset[w];
+        const bool live = gid < s_offset[w + 1];
+        // the group's columns, ascending
+        float first[4];
+        int st[4], col[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
+        unsigned m[4] = {0u, 0u, 0u, 0u};
+        int n = 0;
+        if (live) {
+            const int slot = v.pre[w].slots + gid - off;
+            const int rec0 = v.rec[w] + v.tc[w], ncol = v.rec[w + 1] - rec0;
+            const int u[2] = {pair_a[slot], pair_b[slot]};
+#pragma unroll
+            for (int i = 0; i < 4; ++i) {
+                const int ls = 2 * u[i >> 1] + (i & 1);
+                if (u[i >> 1] >= 0 && ls < ncol) {
+                    const Record c = r.rec[r.ord[rec0 + ls]];
+                    col[i] = c.col; st[i] = c.start; m[i] = c.mask; first[i] = c.value;
+                    ++n;
+                }
+            }
+            auto order2 = [&](int a, int b) {
+                if (col[a] > col[b]) {
+                    int s = col[a]; col[a] = col[b]; col[b] = s;
+                    s = st[a]; st[a] = st[b]; st[b] = s;
+                    const unsigned t = m[a]; m[a] = m[b]; m[b] = t;
+                    const float f = first[a]; first[a] = first[b]; first[b] = f;
+                }
+            };
+            order2(0, 1); order2(2, 3); order2(0, 2); order2(1, 3); order2(1, 2);
+        }
+#pragma unroll
+        for (int p = 0; p < 4; ++p)
+            if (p >= n) col[p] = -1;
+        // the two kept entries of both rows: positions from bit arithmetic, then all loads side by side
+        // (a branch per position, with its dependent loads inside, took three times as long)
+        unsigned bits[2];
+        int pos[2][2], at[2][2];
+        float value[2][2];
+        bool load[2][2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int lr = g + 8 * h;
+            bits[h] = ((m[0] >> lr) & 1u) | (((m[1] >> lr) & 1u) << 1) | (((m[2] >> lr) & 1u) << 2) | (((m[3] >> lr) & 1u) << 3);
+            unsigned rest = bits[h];
+#pragma unroll
+            for (int i = 0; i < 2; ++i) {
+                const int p = rest ? __ffs(rest) - 1 : -1;
+                rest &= rest - 1;
+                pos[h][i] = p;
+                const unsigned mp = p == 0 ? m[0] : p == 1 ? m[1] : p == 2 ? m[2] : m[3];
+                const int k = __popc(mp & ((1u << lr) - 1u));
+                at[h][i] = (p == 0 ? st[0] : p == 1 ? st[1] : p == 2 ? st[2] : st[3]) + k;
+                value[h][i] = p < 0 ? 0.f : p == 0 ? first[0] : p == 1 ? first[1] : p == 2 ? first[2] : first[3];
+                load[h][i] = p >= 0 && k > 0;
+            }
+        }
+        int e[2][2];
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < 2; ++i) e[h][i] = load[h][i] ? r.entry(at[h][i]) : 0;
+#pragma unroll
+        for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int i = 0; i < 2; ++i)
+                if (load[h][i]) value[h][i] = r.val[e[h][i]];
+        uint32_t meta = 0, word[2];
+        int n_extra = 0, extra_at[4], extra_col[4], extra_row[4];
+#pragma unroll
+        for (int h = 0; h < 2; ++h) {
+            const int lr = g + 8 * h;
+            dropped += max(__popc(bits[h]) - 2, 0);
+            if constexpr (STRICT) {
+                unsigned rest = bits[h] & (bits[h] - 1);
+                rest &= rest - 1;
+#pragma unroll
+                for (int i = 0; i < 2; ++i) {   // the third and fourth entry
+                    if (rest) {
+                        const int p = __ffs(rest) - 1;
+                        rest &= rest - 1;
+                        const unsigned mp = p == 2 ? m[2] : m[3];   // never the first two positions
+                        extra_at[2 * h + i] = r.entry((p == 2 ? st[2] : st[3]) + __popc(mp & ((1u << lr) - 1u)));
+                        extra_col[2 * h + i] = p == 2 ? col[2] : col[3];
+                        extra_row[2 * h + i] = w * window + lr;
+                        n_extra |= 1 << (2 * h + i);
+                    }
+                }
+            }
+            if (live && lr < window) {
+                const size_t i = (size_t)gid * window + lr;
+                o.s_mask[i] = (unsigned char)bits[h];
+                *(float2*)(o.s_value + 2 * i) = make_float2(value[h][0], value[h][1]);
+                *(char2*)(o.s_pos + 2 * i) = make_char2((signed char)pos[h][0], (signed char)pos[h][1]);
+            }
+            // the tile's two kept positions p0 < p1 (a missing slot gets a position holding 0.0)
+            const int slots = __popc(bits[h]);
+            int p0 = 0, p1 = 1;
+            float w0 = 0.f, w1 = 0.f;
+            if (slots >= 2) { p0 = pos[h][0]; p1 = pos[h][1]; w0 = value[h][0]; w1 = value[h][1]; }
+            else if (slots == 1) {
+                if (pos[h][0] == 0) w0 = value[h][0];
+                else { p1 = pos[h][0]; w1 = value[h][0]; }
+            }
+            meta |= (uint32_t)(p0 | (p1 << 2)) << (q * 4 + 16 * h);
+            word[h] = (uint32_t)__half_as_ushort(__float2half_rn(w0)) | ((uint32_t)__half_as_ushort(__float2half_rn(w1)) << 16);
+        }
+        if constexpr (STRICT) {
+            int incl = __popc(n_extra);
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, incl, d);
+                if (lane >= d) incl += y;
+            }
+            int put = waiting + incl - __popc(n_extra);
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if ((n_extra >> i) & 1) {
+                    s_key[wid][put] = ((u64)(unsigned)extra_row[i] << 32) | (unsigned)extra_col[i];
+                    s_at[wid][put] = extra_at[i];
+                    ++put;
+                }
+            waiting += __shfl_sync(0xffffffffu, incl, 31);
+            if (waiting > 128) flush();
+        }
+        *(uint2*)(o.packed_a + (size_t)t * 64 + g * 8 + q * 2) = make_uint2(word[0], word[1]);
+        meta |= __shfl_xor_sync(0xffffffffu, meta, 8);
+        meta |= __shfl_xor_sync(0xffffffffu, meta, 16);
+        if (q == 0) o.packed_meta[(size_t)t * 8 + g] = meta;
+        if (g == 0) {
+            const int4 c = make_int4(col[0], col[1], col[2], col[3]);
+            *(int4*)(o.s_tile_column + (size_t)t * 16 + q * 4) = c;
+            if (live) {
+                *(int4*)(o.s_column + (size_t)gid * 4) = c;
+                o.s_window[gid] = w;
+            }
+        }
+    }
+    if constexpr (STRICT) {
+        if (waiting > 0) flush();
+        return;
+    }
+    dropped = __reduce_add_sync(0xffffffffu, dropped);
+    if (lane == 0 && dropped) atomicAdd(x.count + blockIdx.x % kDropCounters, (u64)dropped);
 }
 
-__global__ void kb_iota(int* __restrict__ p, int n) {
-    int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) p[i] = i;
+// ---------------------------------------------------------------------------------------------
+// 8. TC blocks
+// ---------------------------------------------------------------------------------------------
+__device__ __forceinline__ int find_block_window(const Win* __restrict__ pre, int W, int b) {
+    int lo = 0, hi = W;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (pre[mid].blocks <= b) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+// one thread per TC block: columns ascending, bitmaps, value count; the record of every slot for kb_tc_values
+__global__ void kb_tc_blocks(WindowView v, RecordView r, int W, int NB, int* __restrict__ t_column,
+                             long long* __restrict__ t_binary, int* __restrict__ blk_nnz, int* __restrict__ slot_rec) {
+    int b = blockIdx.x * blockDim.x + threadIdx.x;
+    if (b > NB) return;
+    if (b == NB) { blk_nnz[NB] = 0; return; }
+    const int w = find_block_window(v.pre, W, b);
+    const int o0 = 8 * (b - v.pre[w].blocks), len = min(8, v.tc[w] - o0);
+    const int p0 = v.rec[w] + o0;
+    int ids[8], cols[8];
+    for (int i = 0; i < len; ++i) { ids[i] = r.ord[p0 + i]; cols[i] = r.rec[ids[i]].col; }
+    for (int i = 1; i < len; ++i) {
+        const int c = cols[i], id = ids[i];
+        int k = i - 1;
+        while (k >= 0 && cols[k] > c) { cols[k + 1] = cols[k]; ids[k + 1] = ids[k]; --k; }
+        cols[k + 1] = c; ids[k + 1] = id;
+    }
+    u64 lo = 0, hi = 0;
+    for (int k = 0; k < 8; ++k) {
+        t_column[(size_t)b * 8 + k] = k < len ? cols[k] : -1;
+        slot_rec[(size_t)b * 8 + k] = k < len ? ids[k] : -1;
+        if (k >= len) continue;
+        const unsigned m = r.rec[ids[k]].mask;
+        for (int i = 0; i < 8; ++i) {
+            if ((m >> i) & 1u) lo |= 1ull << (i * 8 + k);
+            if ((m >> (i + 8)) & 1u) hi |= 1ull << (i * 8 + k);
+        }
+    }
+    t_binary[(size_t)b * 2] = (long long)lo;
+    t_binary[(size_t)b * 2 + 1] = (long long)hi;
+    blk_nnz[b] = __popcll(lo) + __popcll(hi);
+}
+
+// one thread per (block, slot, row): its value, in bitmap order
+__global__ void kb_tc_values(RecordView r, const int* __restrict__ slot_rec, int NB, const long long* __restrict__ t_binary,
+                             const int* __restrict__ t_block_offset, float* __restrict__ t_value) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= (long long)NB * 128) return;
+    const int b = (int)(i >> 7), lr = (int)(i >> 3) & 15, k = (int)(i & 7);
+    const int id = slot_rec[(size_t)b * 8 + k];
+    if (id < 0) return;
+    const Record c = r.rec[id];
+    if (!((c.mask >> lr) & 1u)) return;
+    const float value = r.value(c.start, c.value, __popc(c.mask & ((1u << lr) - 1u)));
+    const u64 lo = (u64)t_binary[(size_t)b * 2], hi = (u64)t_binary[(size_t)b * 2 + 1];
+    const int bit = (lr & 7) * 8 + k;
+    const u64 below = (1ull << bit) - 1ull;
+    const int rank = lr < 8 ? __popcll(lo & below) : __popcll(lo) + __popcll(hi & below);
+    t_value[(size_t)t_block_offset[b] + rank] = value;
+}
+
+__global__ void kb_tc_parts(WindowView v, const int* __restrict__ win_cuda_unit, int W, int part_t,
+                            int* __restrict__ t_row_offset, int* __restrict__ t_window_row, int* __restrict__ t_atomic) {
+    int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w == 0) t_row_offset[0] = 0;
+    if (w >= W) return;
+    const int bb = v.pre[w].blocks, nb = v.pre[w + 1].blocks - bb;
+    const int p0 = v.pre[w].parts, np = v.pre[w + 1].parts - p0;
+    for (int q = 0; q < np; ++q) {
+        t_row_offset[p0 + q + 1] = bb + min((q + 1) * part_t, nb);
+        t_window_row[p0 + q] = w * 16;
+        t_atomic[p0 + q] = np > 1 || win_cuda_unit[w] >= 0 ? 1 : 0;
+    }
+}
+
+// ---------------------------------------------------------------------------------------------
+// 9. CUDA-core leftovers: the (at most two) columns of the window's rejected unit.  Per row the
+// entries come in ascending column order = CSR order.
+// ---------------------------------------------------------------------------------------------
+struct CudaRow {
+    int n;
+    int cols[2];
+    int ent[2];
+};
+__device__ __forceinline__ CudaRow cuda_row(int row, int window, const int* __restrict__ win_cuda_unit, const WindowView& v,
+                                            const RecordView& r) {
+    CudaRow out;
+    out.n = 0;
+    const int w = row / window, lr = row - w * window;
+    const int u = win_cuda_unit[w];
+    if (u < 0) return out;
+    const int rec0 = v.rec[w] + v.tc[w], ncol = v.rec[w + 1] - rec0;
+    for (int i = 0; i < 2; ++i) {
+        const int ls = 2 * u + i;
+        if (ls >= ncol) break;
+        const Record c = r.rec[r.ord[rec0 + ls]];
+        if (!((c.mask >> lr) & 1u)) continue;
+        out.cols[out.n] = c.col;
+        out.ent[out.n] = r.entry(c.start + __popc(c.mask & ((1u << lr) - 1u)));
+        ++out.n;
+    }
+    if (out.n == 2 && out.cols[0] > out.cols[1]) {
+        int t = out.cols[0]; out.cols[0] = out.cols[1]; out.cols[1] = t;
+        t = out.ent[0]; out.ent[0] = out.ent[1]; out.ent[1] = t;
+    }
+    return out;
+}
+
+// Strict mode: the row's dropped entries in the list sorted by (row, column).
+struct Extras {
+    const u64* key;
+    const int* at;
+    int n;
+    __device__ __forceinline__ int first(int row) const {
+        int lo = 0, hi = n;
+        while (lo < hi) {
+            const int mid = lo + (hi - lo) / 2;
+            if ((long long)(key[mid] >> 32) < row) lo = mid + 1; else hi = mid;
+        }
+        return lo;
+    }
+};
+
+// split rule of block_online.cpp:415-439: long parts, short parts, long nnz, short nnz
+struct Parts {
+    int nl, ns, zl, zs;
+};
+struct PartsSum {
+    __host__ __device__ __forceinline__ Parts operator()(const Parts& a, const Parts& b) const {
+        return Parts{a.nl + b.nl, a.ns + b.ns, a.zl + b.zl, a.zs + b.zs};
+    }
+};
+__device__ __forceinline__ Parts split_counts(int n, int part_c, int short_size) {
+    if (n <= 0) return Parts{0, 0, 0, 0};
+    if (n <= short_size) return Parts{0, 1, 0, n};
+    if (n <= part_c) return Parts{1, 0, n, 0};
+    Parts p{n / part_c, 0, n / part_c * part_c, 0};
+    const int residue = n % part_c;
+    if (residue > 0) {
+        if (residue <= short_size) { p.ns = 1; p.zs = residue; }
+        else { p.nl += 1; p.zl += residue; }
+    }
+    return p;
+}
+
+__global__ void kb_cuda_count(int n_rows, int window, int part_c, int short_size, const int* __restrict__ win_cuda_unit,
+                              WindowView v, RecordView r, Extras x, Parts* __restrict__ cnt) {
+    int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row > n_rows) return;
+    int n = 0;
+    if (row < n_rows) {
+        n = cuda_row(row, window, win_cuda_unit, v, r).n;
+        if (x.n > 0) n += x.first(row + 1) - x.first(row);
+    }
+    cnt[row] = split_counts(n, part_c, short_size);
+}
+
+struct PartsOut {
+    int *c_row_offset, *c_row, *c_atomic, *c_column;
+    float* c_value;
+    int *cs_row_offset, *cs_row, *cs_atomic, *cs_column;
+    float* cs_value;
+    // entry i of a row's list: the long parts come first
+    __device__ __forceinline__ void put(const Parts& o, int row_long, int i, int col, float value) const {
+        if (i < row_long) { c_column[o.zl + i] = col; c_value[o.zl + i] = value; }
+        else { cs_column[o.zs + i - row_long] = col; cs_value[o.zs + i - row_long] = value; }
+    }
+};
+
+// A row's list is the (at most two) entries of the window's rejected unit merged with the row's strict-mode
+// extras, by column.  One thread per row writes its parts and the unit's entries, one per extra its place:
+// its rank among the row's extras plus the unit entries before it (a hub row has thousands).
+__global__ void kb_cuda_rows(int n_rows, int window, int part_c, int short_size, const int* __restrict__ win_cuda_unit,
+                             WindowView v, RecordView r, Extras x, const Parts* __restrict__ off, PartsOut po) {
+    int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (row == 0) { po.c_row_offset[0] = 0; po.cs_row_offset[0] = 0; }
+    if (row >= n_rows) return;
+    const Parts o = off[row], e = off[row + 1];
+    const int row_long = e.zl - o.zl, nl = e.nl - o.nl, n = row_long + e.zs - o.zs;
+    if (n <= 0) return;
+    const int w = row / window;
+    const int atomic = n > part_c ? 1 : (v.pre[w + 1].blocks > v.pre[w].blocks ? 1 : 0);
+    for (int i = 0; i < nl; ++i) {
+        po.c_row[o.nl + i] = row;
+        po.c_atomic[o.nl + i] = atomic;
+        po.c_row_offset[o.nl + i + 1] = o.zl + min((i + 1) * part_c, row_long);
+    }
+    if (e.ns > o.ns) {
+        po.cs_row[o.ns] = row;
+        po.cs_atomic[o.ns] = atomic;
+        po.cs_row_offset[o.ns + 1] = e.zs;
+    }
+    const CudaRow cr = cuda_row(row, window, win_cuda_unit, v, r);
+    if (cr.n == 0) return;
+    const int xb = x.n > 0 ? x.first(row) : 0, xe = x.n > 0 ? x.first(row + 1) : 0;
+    for (int i = 0; i < cr.n; ++i) {
+        int lo = xb, hi = xe;   // extras with a smaller column
+        while (lo < hi) {
+            const int mid = lo + (hi - lo) / 2;
+            if ((int)(x.key[mid] & 0xffffffffull) < cr.cols[i]) lo = mid + 1; else hi = mid;
+        }
+        po.put(o, row_long, i + lo - xb, cr.cols[i], r.val[cr.ent[i]]);
+    }
+}
+
+__global__ void kb_cuda_extras(int window, const int* __restrict__ win_cuda_unit, WindowView v, RecordView r, Extras x,
+                               const Parts* __restrict__ off, PartsOut po) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= x.n) return;
+    const int row = (int)(x.key[i] >> 32), c = (int)(x.key[i] & 0xffffffffull);
+    int rank = i - x.first(row);
+    const CudaRow cr = cuda_row(row, window, win_cuda_unit, v, r);
+    for (int k = 0; k < cr.n; ++k) rank += cr.cols[k] < c;
+    const Parts o = off[row];
+    po.put(o, off[row + 1].zl - o.zl, rank, c, r.val[x.at[i]]);
+}
+
+// sizes that the host needs after the matching, in one place
+struct Totals {
+    int groups, tiles, tc_nnz, pad;
+    Parts parts;
+};
+__global__ void kb_totals(const int* __restrict__ s_offset, const int* __restrict__ tile_off, int W,
+                          const int* __restrict__ blk_off, int NB, const Parts* __restrict__ part_off, int n_rows,
+                          Totals* __restrict__ t) {
+    t->groups = s_offset[W];
+    t->tiles = tile_off[W];
+    t->tc_nnz = blk_off[NB];
+    if (part_off) t->parts = part_off[n_rows];
 }
 
 __global__ void kb_to_half(const float* __restrict__ src, long long n, __half* __restrict__ dst) {
@@ -777,7 +1186,9 @@ using namespace trs;
 struct trs_builder {
     BuildCfg cfg;
     Arena arena_store;
-    Arena* arena = nullptr;   // set: outputs and scratch come from the caller's memory
+    Arena* arena = nullptr;            // set: outputs and scratch come from the caller's memory
+    trs_build_alloc alloc = nullptr;   // set: outputs come from the caller's allocator
+    void* alloc_ctx = nullptr;
     int n_rows = 0, W = 0;
     long long nnz = 0;
     // the 29 arrays, reference order (block_online.cpp:844-870)
@@ -799,6 +1210,15 @@ struct trs_builder {
     long long distinct_cols = 0, units = 0;
     float build_ms = 0.f;
 
+    // array `id` with `count` elements
+    template <class T>
+    int out(DevBuf<T>& buf, int id, size_t count) {
+        if (!alloc || count == 0) return buf.alloc_from(arena, count);
+        buf.n = count;
+        buf.owned = false;
+        buf.p = (T*)alloc(alloc_ctx, id, count * sizeof(T));
+        return buf.p ? 0 : (int)cudaErrorMemoryAllocation;
+    }
     void release() {
         t_row_offset.release(); t_block_offset.release(); t_column.release(); t_window_row.release();
         t_atomic.release(); t_value.release(); t_binary.release();
@@ -812,43 +1232,6 @@ struct trs_builder {
 
 namespace {
 
-struct Scratch {  // frees everything it handed out (or gives it back to the caller's arena)
-    Arena* arena = nullptr;
-    std::vector<void*> ptrs;
-    std::vector<size_t> bytes;
-    ~Scratch() {
-        for (size_t i = ptrs.size(); i-- > 0;)
-            if (ptrs[i]) {
-                if (arena) arena->give_back(ptrs[i], bytes[i]);
-                else cudaFree(ptrs[i]);
-            }
-    }
-    template <class T>
-    int get(size_t n, T** out) {
-        void* d = nullptr;
-        const size_t nb = (n ? n : 1) * sizeof(T);
-        if (arena) {
-            d = arena->take(nb);
-            if (!d) { *out = nullptr; return TRS_E_WORKSPACE; }
-        } else {
-            cudaError_t e = cudaMalloc(&d, nb);
-            if (e != cudaSuccess) { *out = nullptr; return (int)e; }
-        }
-        ptrs.push_back(d);
-        bytes.push_back(nb);
-        *out = (T*)d;
-        return 0;
-    }
-    void drop(void* p) {
-        for (size_t i = 0; i < ptrs.size(); ++i)
-            if (ptrs[i] == p) {
-                if (arena) arena->give_back(p, bytes[i]);
-                else cudaFree(p);
-                ptrs[i] = nullptr;
-            }
-    }
-};
-
 inline unsigned grid_for(long long n, int block = 256) { return (unsigned)((n + block - 1) / block); }
 
 int bits_for(long long max_value) {  // bits needed to store values in [0, max_value]
@@ -859,431 +1242,354 @@ int bits_for(long long max_value) {  // bits needed to store values in [0, max_v
 
 #define TRS_TRY(expr) do { int _rc = (expr); if (_rc) return _rc; } while (0)
 
+// CUB's temporary storage, kept between calls and grown when one needs more
 struct Cub {
-    Scratch& sc;
-    void* tmp = nullptr;
-    size_t cap = 0;
+    TempSpace& ts;
     cudaStream_t st;
-    Cub(Scratch& s, cudaStream_t stream) : sc(s), st(stream) {}
-    int reserve(size_t bytes) {
-        if (bytes <= cap) return 0;
-        if (tmp) sc.drop(tmp);
-        unsigned char* p;
-        TRS_TRY(sc.get<unsigned char>(bytes, &p));
-        tmp = p; cap = bytes;
+    unsigned char* tmp = nullptr;
+    size_t cap = 0;
+    Cub(TempSpace& t, cudaStream_t s) : ts(t), st(s) {}
+    template <class Call>
+    int run(Call&& call) {
+        size_t bytes = 0;
+        TRS_CUDA(call((void*)nullptr, bytes));
+        if (bytes > cap || !tmp) {
+            if (tmp) ts.drop(tmp, cap);
+            TRS_TRY(ts.get<unsigned char>(bytes, &tmp));
+            cap = bytes;
+        }
+        TRS_CUDA(call((void*)tmp, bytes));
         return 0;
+    }
+    template <class T, class Op>
+    int exclusive_scan(const T* in, T* out, Op op, T zero, long long n) {
+        return run([&](void* t, size_t& b) { return cub::DeviceScan::ExclusiveScan(t, b, in, out, op, zero, n, st); });
     }
     int exclusive_sum(const int* in, int* out, long long n) {
-        size_t bytes = 0;
-        TRS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, bytes, in, out, n, st));
-        TRS_TRY(reserve(bytes));
-        TRS_CUDA(cub::DeviceScan::ExclusiveSum(tmp, bytes, in, out, n, st));
-        return 0;
-    }
-    int inclusive_sum(const int* in, int* out, long long n) {
-        size_t bytes = 0;
-        TRS_CUDA(cub::DeviceScan::InclusiveSum(nullptr, bytes, in, out, n, st));
-        TRS_TRY(reserve(bytes));
-        TRS_CUDA(cub::DeviceScan::InclusiveSum(tmp, bytes, in, out, n, st));
-        return 0;
-    }
-    int inclusive_max(int* inout, long long n) {
-        size_t bytes = 0;
-        TRS_CUDA(cub::DeviceScan::InclusiveScan(nullptr, bytes, inout, inout, MaxOp(), n, st));
-        TRS_TRY(reserve(bytes));
-        TRS_CUDA(cub::DeviceScan::InclusiveScan(tmp, bytes, inout, inout, MaxOp(), n, st));
-        return 0;
-    }
-    int max_reduce(const int* in, int* out, long long n) {
-        size_t bytes = 0;
-        TRS_CUDA(cub::DeviceReduce::Max(nullptr, bytes, in, out, n, st));
-        TRS_TRY(reserve(bytes));
-        TRS_CUDA(cub::DeviceReduce::Max(tmp, bytes, in, out, n, st));
-        return 0;
+        return run([&](void* t, size_t& b) { return cub::DeviceScan::ExclusiveSum(t, b, in, out, n, st); });
     }
     template <class K, class V>
     int sort_pairs(K* k_in, K* k_out, V* v_in, V* v_out, long long n, int end_bit, K** k_res, V** v_res) {
         cub::DoubleBuffer<K> kb(k_in, k_out);
         cub::DoubleBuffer<V> vb(v_in, v_out);
-        size_t bytes = 0;
-        TRS_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, bytes, kb, vb, n, 0, end_bit, st));
-        TRS_TRY(reserve(bytes));
-        TRS_CUDA(cub::DeviceRadixSort::SortPairs(tmp, bytes, kb, vb, n, 0, end_bit, st));
+        TRS_TRY(run([&](void* t, size_t& b) { return cub::DeviceRadixSort::SortPairs(t, b, kb, vb, n, 0, end_bit, st); }));
         *k_res = kb.Current();
         *v_res = vb.Current();
         return 0;
     }
 };
 
-int read_int(const int* dev, cudaStream_t st, int* out) {
-    TRS_CUDA(cudaMemcpyAsync(out, dev, sizeof(int), cudaMemcpyDeviceToHost, st));
+template <class T>
+int read_back(const T* dev, T* host, cudaStream_t st) {
+    TRS_CUDA(cudaMemcpyAsync(host, dev, sizeof(T), cudaMemcpyDeviceToHost, st));
     TRS_CUDA(cudaStreamSynchronize(st));
+    return 0;
+}
+
+// Streams on which the hub tiers of the matching run beside the others (two per device, made once).
+int side_streams(cudaStream_t out[2]) {
+    static cudaStream_t made[64][2] = {};
+    static std::mutex m;
+    int dev = 0;
+    TRS_CUDA(cudaGetDevice(&dev));
+    if (dev < 0 || dev >= 64) return TRS_E_LIMIT;
+    std::lock_guard<std::mutex> lock(m);
+    for (int i = 0; i < 2; ++i) {
+        if (!made[dev][i]) TRS_CUDA(cudaStreamCreateWithFlags(&made[dev][i], cudaStreamNonBlocking));
+        out[i] = made[dev][i];
+    }
+    return 0;
+}
+struct Event {
+    cudaEvent_t e = nullptr;
+    int record(cudaStream_t st) {
+        if (!e) TRS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+        TRS_CUDA(cudaEventRecord(e, st));
+        return 0;
+    }
+    ~Event() { if (e) cudaEventDestroy(e); }
+};
+
+struct Records {   // stages 1 - 3
+    int D = 0;
+    int *start = nullptr, *ord = nullptr;
+    Record* rec = nullptr;
+    unsigned *ent = nullptr, *key2 = nullptr;
+};
+
+template <class Key, bool PACKED>
+int make_records(trs_builder* B, const int* rowptr, const int* col, const float* val, InputInfo* d_info, int* d_count, int col_bits, int w_bits,
+                 TempSpace& ts, Cub& cub_, cudaStream_t st, Records* R) {
+    const int nnz = (int)B->nnz, n = B->n_rows, window = B->cfg.window;
+    Key *keys_a, *keys_b, *keys;
+    unsigned *ent_a, *ent_b;
+    TRS_TRY(ts.get(nnz, &keys_a));
+    TRS_TRY(ts.get(nnz, &keys_b));
+    TRS_TRY(ts.get(nnz, &ent_a));
+    TRS_TRY(ts.get(nnz, &ent_b));
+    kb_make_keys<Key, PACKED><<<grid_for(nnz, 256 * kKeyItems), 256, 0, st>>>(rowptr, col, n, nnz, window, col_bits, keys_a, ent_a, d_info);
+    TRS_LAUNCH_CHECK();
+    TRS_TRY(cub_.sort_pairs(keys_a, keys_b, ent_a, ent_b, (long long)nnz, col_bits + w_bits, &keys, &R->ent));
+    ts.drop(R->ent == ent_a ? ent_b : ent_a, nnz);
+    // first entries, into the key buffer that is free now
+    int* start = (int*)(keys == keys_a ? keys_b : keys_a);
+    IsHead<Key> is_head{keys};
+    TRS_TRY(cub_.run([&](void* t, size_t& b) {
+        return cub::DeviceSelect::If(t, b, thrust::counting_iterator<int>(0), start, d_count, nnz, is_head, st);
+    }));
+    int D = 0;
+    InputInfo info;
+    TRS_CUDA(cudaMemcpyAsync(&info, d_info, sizeof(info), cudaMemcpyDeviceToHost, st));
+    TRS_TRY(read_back(d_count, &D, st));
+    if (info.err & 2) return TRS_E_NOT_CANONICAL;
+    R->D = D;
+    unsigned *key2_a, *key2_b;
+    int *ord_a, *ord_b;
+    TRS_TRY(ts.get(D, &R->rec));
+    TRS_TRY(ts.get(D, &key2_a));
+    TRS_TRY(ts.get(D, &key2_b));
+    TRS_TRY(ts.get(D, &ord_a));
+    TRS_TRY(ts.get(D, &ord_b));
+    kb_records<Key, PACKED><<<grid_for(D), 256, 0, st>>>(keys, R->ent, rowptr, val, n, window, start, D, nnz, col_bits, R->rec,
+                                                        key2_a, ord_a);
+    TRS_LAUNCH_CHECK();
+    R->start = start;
+    ts.drop(keys, nnz);
+    TRS_TRY(cub_.sort_pairs(key2_a, key2_b, ord_a, ord_b, (long long)D, 4 + w_bits, &R->key2, &R->ord));  // stable
+    ts.drop(R->key2 == key2_a ? key2_b : key2_a, D);
+    ts.drop(R->ord == ord_a ? ord_b : ord_a, D);
+    return 0;
+}
+
+int empty_outputs(trs_builder* B, cudaStream_t st) {
+    TRS_TRY(B->out(B->s_offset, 22, (size_t)B->W + 1));
+    TRS_TRY(B->out(B->s_window_tile_offset, 28, (size_t)B->W + 1));
+    TRS_TRY(B->out(B->t_row_offset, 0, 1));
+    TRS_TRY(B->out(B->t_block_offset, 1, 1));
+    TRS_TRY(B->out(B->c_row_offset, 7, 1));
+    TRS_TRY(B->out(B->cs_row_offset, 12, 1));
+    TRS_CUDA(cudaMemsetAsync(B->s_offset.p, 0, sizeof(int) * ((size_t)B->W + 1), st));
+    TRS_CUDA(cudaMemsetAsync(B->s_window_tile_offset.p, 0, sizeof(int) * ((size_t)B->W + 1), st));
+    for (DevBuf<int>* b : {&B->t_row_offset, &B->t_block_offset, &B->c_row_offset, &B->cs_row_offset})
+        TRS_CUDA(cudaMemsetAsync(b->p, 0, sizeof(int), st));
     return 0;
 }
 
 int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val, cudaStream_t st) {
     const BuildCfg& cfg = B->cfg;
-    const int n = B->n_rows, window = cfg.window;
-    const int W = B->W;
-    Scratch sc;
-    sc.arena = B->arena;
-    Cub cub_(sc, st);
-    int* d_err;
-    TRS_TRY(sc.get<int>(4, &d_err));
-    TRS_CUDA(cudaMemsetAsync(d_err, 0, 4 * sizeof(int), st));
+    const int n = B->n_rows, window = cfg.window, W = B->W;
+    int dev = 0, sms = 1;
+    TRS_CUDA(cudaGetDevice(&dev));
+    TRS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    TempSpace ts;
+    ts.arena = B->arena;
+    ts.st = st;
+    Cub cub_(ts, st);
 
-    int first = 0, last = 0;
-    TRS_CUDA(cudaMemcpyAsync(&first, rowptr, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TRS_TRY(read_int(rowptr + n, st, &last));
-    if (first != 0 || last < 0) return TRS_E_OFFSETS;
-    const long long nnz = last;
-    B->nnz = nnz;
-
-    // outputs that exist even for an empty matrix
-    TRS_TRY(B->s_offset.alloc_from(B->arena, (size_t)W + 1));
-    TRS_TRY(B->s_window_tile_offset.alloc_from(B->arena, (size_t)W + 1));
-    TRS_TRY(B->t_row_offset.alloc_from(B->arena, 1));
-    TRS_TRY(B->t_block_offset.alloc_from(B->arena, 1));
-    TRS_TRY(B->c_row_offset.alloc_from(B->arena, 1));
-    TRS_TRY(B->cs_row_offset.alloc_from(B->arena, 1));
-    TRS_CUDA(cudaMemsetAsync(B->s_offset.p, 0, sizeof(int) * (W + 1), st));
-    TRS_CUDA(cudaMemsetAsync(B->s_window_tile_offset.p, 0, sizeof(int) * (W + 1), st));
-    TRS_CUDA(cudaMemsetAsync(B->t_row_offset.p, 0, sizeof(int), st));
-    TRS_CUDA(cudaMemsetAsync(B->t_block_offset.p, 0, sizeof(int), st));
-    TRS_CUDA(cudaMemsetAsync(B->c_row_offset.p, 0, sizeof(int), st));
-    TRS_CUDA(cudaMemsetAsync(B->cs_row_offset.p, 0, sizeof(int), st));
-    if (nnz == 0) {
-        int h = 0;
-        kb_mark_rows<<<grid_for(n), 256, 0, st>>>(rowptr, n, d_err, d_err);  // only the monotonicity check fires
-        TRS_TRY(read_int(d_err, st, &h));
-        return (h & 1) ? TRS_E_OFFSETS : TRS_OK;
-    }
-
-    // ---- 1. row ids, keys, sort ----------------------------------------------------------------
-    int* rowid;
-    TRS_TRY(sc.get<int>(nnz, &rowid));
-    TRS_CUDA(cudaMemsetAsync(rowid, 0, sizeof(int) * nnz, st));
-    kb_mark_rows<<<grid_for(n), 256, 0, st>>>(rowptr, n, rowid, d_err);
+    // ---- sizes of the input ---------------------------------------------------------------------
+    struct Head { InputInfo info; MatchCounts mc; Totals tot; int count; u64 dropped[kDropCounters]; };
+    Head* d_head;
+    TRS_TRY(ts.get(1, &d_head));
+    TRS_CUDA(cudaMemsetAsync(d_head, 0, sizeof(Head), st));
+    kb_input_info<<<2 * sms, 512, 0, st>>>(rowptr, col, n, &d_head->info);
     TRS_LAUNCH_CHECK();
-    {
-        int h = 0;
-        TRS_TRY(read_int(d_err, st, &h));
-        if (h & 1) return TRS_E_OFFSETS;  // a decreasing row pointer would also corrupt the scatter above
-    }
-    TRS_TRY(cub_.inclusive_max(rowid, nnz));
-    int* d_max;
-    TRS_TRY(sc.get<int>(1, &d_max));
-    TRS_TRY(cub_.max_reduce(col, d_max, nnz));
-    int max_col = 0;
-    TRS_TRY(read_int(d_max, st, &max_col));
-    if (max_col < 0) return TRS_E_NOT_CANONICAL;
-    const int col_bits = bits_for(max_col);
-    const int w_bits = bits_for(W > 0 ? W - 1 : 0);
+    InputInfo info;
+    TRS_TRY(read_back(&d_head->info, &info, st));
+    if (info.first != 0 || info.last < 0 || (info.err & 1)) return TRS_E_OFFSETS;
+    const long long nnz = B->nnz = info.last;
+    if (nnz == 0) return empty_outputs(B, st);
+    ts.chunk_bytes = std::max((size_t)16 << 20, (size_t)nnz * 24);
 
-    u64 *keys_a, *keys_b, *keys;
-    int *edge_a, *edge_b, *edge;
-    TRS_TRY(sc.get<u64>(nnz, &keys_a));
-    TRS_TRY(sc.get<u64>(nnz, &keys_b));
-    TRS_TRY(sc.get<int>(nnz, &edge_a));
-    TRS_TRY(sc.get<int>(nnz, &edge_b));
-    kb_make_keys<<<grid_for(nnz), 256, 0, st>>>(col, rowid, nnz, window, col_bits, keys_a, edge_a, d_err);
-    TRS_LAUNCH_CHECK();
-    TRS_TRY(cub_.sort_pairs(keys_a, keys_b, edge_a, edge_b, nnz, 4 + col_bits + w_bits, &keys, &edge));
-    {
-        int h = 0;
-        TRS_TRY(read_int(d_err, st, &h));
-        if (h & 2) return TRS_E_NOT_CANONICAL;
-    }
-    sc.drop(rowid);
-    sc.drop(keys == keys_a ? (void*)keys_b : (void*)keys_a);
-    sc.drop(edge == edge_a ? (void*)edge_b : (void*)edge_a);
-
-    // ---- 2. one record per (window, column) ----------------------------------------------------
-    int *head, *wc_incl;
-    TRS_TRY(sc.get<int>(nnz, &head));
-    TRS_TRY(sc.get<int>(nnz, &wc_incl));
-    kb_heads<<<grid_for(nnz), 256, 0, st>>>(keys, nnz, head);
-    TRS_LAUNCH_CHECK();
-    TRS_TRY(cub_.inclusive_sum(head, wc_incl, nnz));
-    int D = 0;
-    TRS_TRY(read_int(wc_incl + (nnz - 1), st, &D));
+    // ---- 1. - 3. columns of every window in (count desc, column asc) order ---------------------------
+    const int col_bits = bits_for(info.max_col), w_bits = bits_for(W > 0 ? W - 1 : 0);
+    const bool packed = nnz < (1ll << 28);
+    Records R;
+    if (col_bits + w_bits <= 32)
+        TRS_TRY(packed ? (make_records<unsigned, true>(B, rowptr, col, val, &d_head->info, &d_head->count, col_bits, w_bits, ts, cub_, st, &R))
+                       : (make_records<unsigned, false>(B, rowptr, col, val, &d_head->info, &d_head->count, col_bits, w_bits, ts, cub_, st, &R)));
+    else
+        TRS_TRY(packed ? (make_records<u64, true>(B, rowptr, col, val, &d_head->info, &d_head->count, col_bits, w_bits, ts, cub_, st, &R))
+                       : (make_records<u64, false>(B, rowptr, col, val, &d_head->info, &d_head->count, col_bits, w_bits, ts, cub_, st, &R)));
+    const int D = R.D;
     B->distinct_cols = D;
-    int *wc_start, *wc_win, *wc_col, *win_ncol, *win_ncand, *wc_begin;
-    unsigned char* wc_count;
-    unsigned short* wc_mask;
-    unsigned *key2_a, *key2_b, *key2;
-    int *ord_a, *ord_b, *ord;
-    TRS_TRY(sc.get<int>((size_t)D + 1, &wc_start));
-    TRS_TRY(sc.get<int>(D, &wc_win));
-    TRS_TRY(sc.get<int>(D, &wc_col));
-    TRS_TRY(sc.get<unsigned char>(D, &wc_count));
-    TRS_TRY(sc.get<unsigned short>(D, &wc_mask));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_ncol));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_ncand));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &wc_begin));
-    TRS_TRY(sc.get<unsigned>(D, &key2_a));
-    TRS_TRY(sc.get<unsigned>(D, &key2_b));
-    TRS_TRY(sc.get<int>(D, &ord_a));
-    TRS_TRY(sc.get<int>(D, &ord_b));
-    TRS_CUDA(cudaMemsetAsync(win_ncol, 0, sizeof(int) * (W + 1), st));
-    TRS_CUDA(cudaMemsetAsync(win_ncand, 0, sizeof(int) * (W + 1), st));
-    kb_wcol_start<<<grid_for(nnz), 256, 0, st>>>(head, wc_incl, nnz, wc_start);
-    const int nnz_i = (int)nnz;
-    TRS_CUDA(cudaMemcpyAsync(wc_start + D, &nnz_i, sizeof(int), cudaMemcpyHostToDevice, st));
-    kb_wcol_info<<<grid_for(D), 256, 0, st>>>(keys, wc_start, D, col_bits, cfg.density, cfg.skip_tc, wc_win, wc_col,
-                                               wc_count, wc_mask, win_ncol, win_ncand, key2_a);
-    TRS_LAUNCH_CHECK();
-    TRS_TRY(cub_.exclusive_sum(win_ncol, wc_begin, W + 1));
-    sc.drop(head);
+    const RecordView rv{R.ord, R.rec, R.ent, val, packed ? 1 : 0};
 
-    // ---- 3. (count desc, col asc) order inside each window ---------------------------------------
-    kb_iota<<<grid_for(D), 256, 0, st>>>(ord_a, D);
+    // ---- 4., 5. TC columns, units, sizes per window ---------------------------------------------
+    int *rec, *tc, *sel_block, *sel_huge;
+    Win *win, *pre;
+    TRS_TRY(ts.get((size_t)W + 1, &rec));
+    TRS_TRY(ts.get((size_t)W + 1, &tc));
+    TRS_TRY(ts.get((size_t)W + 1, &win));
+    TRS_TRY(ts.get((size_t)W + 1, &pre));
+    TRS_TRY(ts.get((size_t)W + 1, &sel_block));
+    TRS_TRY(ts.get((size_t)W + 1, &sel_huge));
+    kb_windows<<<grid_for(W + 1, 128), 128, 0, st>>>(R.start, R.key2, rowptr, n, D, W, cfg, rec, tc, win, sel_block, sel_huge, &d_head->mc);
     TRS_LAUNCH_CHECK();
-    TRS_TRY(cub_.sort_pairs(key2_a, key2_b, ord_a, ord_b, (long long)D, 4 + w_bits, &key2, &ord));  // LSD radix: stable
-
-    // ---- 4. TC funnel ----------------------------------------------------------------------------
-    int *not_tc, *lead, *s_idx, *b_idx;
-    TRS_TRY(sc.get<int>((size_t)D + 1, &not_tc));
-    TRS_TRY(sc.get<int>((size_t)D + 1, &lead));
-    TRS_TRY(sc.get<int>((size_t)D + 1, &s_idx));
-    TRS_TRY(sc.get<int>((size_t)D + 1, &b_idx));
-    TRS_CUDA(cudaMemsetAsync(not_tc + D, 0, sizeof(int), st));
-    TRS_CUDA(cudaMemsetAsync(lead + D, 0, sizeof(int), st));
-    kb_tc_select<<<grid_for(D), 256, 0, st>>>(ord, wc_win, wc_count, wc_begin, win_ncand, D, window, cfg.tc_min_util,
-                                               not_tc, lead);
-    TRS_LAUNCH_CHECK();
-    TRS_TRY(cub_.exclusive_sum(not_tc, s_idx, (long long)D + 1));
-    TRS_TRY(cub_.exclusive_sum(lead, b_idx, (long long)D + 1));
-    int S = 0, NB = 0;
-    TRS_CUDA(cudaMemcpyAsync(&S, s_idx + D, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TRS_TRY(read_int(b_idx + D, st, &NB));
-    int *cand, *blk_pos, *blk_len;
-    TRS_TRY(sc.get<int>(S, &cand));
-    TRS_TRY(sc.get<int>(NB, &blk_pos));
-    TRS_TRY(sc.get<int>(NB, &blk_len));
-    kb_compact<<<grid_for(D), 256, 0, st>>>(ord, not_tc, lead, s_idx, b_idx, wc_win, wc_begin, win_ncand, D, cand,
-                                             blk_pos, blk_len);
-    TRS_LAUNCH_CHECK();
-
-    // ---- 5. units ---------------------------------------------------------------------------------
-    int *win_cb, *win_U, *win_slots, *win_bb, *win_parts, *win_ub, *win_pb, *part_off;
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_cb));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_U));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_slots));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_bb));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_parts));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_ub));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_pb));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &part_off));
-    TRS_CUDA(cudaMemsetAsync(win_U + W, 0, sizeof(int), st));
-    TRS_CUDA(cudaMemsetAsync(win_slots + W, 0, sizeof(int), st));
-    TRS_CUDA(cudaMemsetAsync(win_parts + W, 0, sizeof(int), st));
-    kb_window_counts<<<grid_for(W), 256, 0, st>>>(wc_begin, s_idx, b_idx, W, cfg.part_t, win_cb, win_U, win_slots,
-                                                   win_bb, win_parts);
-    TRS_LAUNCH_CHECK();
-    TRS_TRY(cub_.exclusive_sum(win_U, win_ub, W + 1));
-    TRS_TRY(cub_.exclusive_sum(win_slots, win_pb, W + 1));
-    TRS_TRY(cub_.exclusive_sum(win_parts, part_off, W + 1));
-    int TU = 0, TS = 0, NP = 0;
-    TRS_CUDA(cudaMemcpyAsync(&TU, win_ub + W, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TRS_CUDA(cudaMemcpyAsync(&TS, win_pb + W, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TRS_TRY(read_int(part_off + W, st, &NP));
+    TRS_TRY(cub_.exclusive_scan(win, pre, WinSum(), Win{0, 0, 0, 0}, W + 1));
+    const WindowView v{rec, tc, pre};
+    Win total;
+    MatchCounts mc;
+    TRS_CUDA(cudaMemcpyAsync(&mc, &d_head->mc, sizeof(mc), cudaMemcpyDeviceToHost, st));
+    TRS_TRY(read_back(pre + W, &total, st));
+    const int NB = total.blocks, NP = total.parts, TU = total.units, TS = total.slots;
     B->units = TU;
-    unsigned char *unit_nnz, *matched;
-    int *order_buf, *pair_a, *pair_b, *win_G, *win_cuda_unit;
-    TRS_TRY(sc.get<unsigned char>(TU, &unit_nnz));
-    TRS_TRY(sc.get<unsigned char>(TU, &matched));
-    TRS_TRY(sc.get<int>(TU, &order_buf));
-    TRS_TRY(sc.get<int>(TS, &pair_a));
-    TRS_TRY(sc.get<int>(TS, &pair_b));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_G));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_cuda_unit));
-    TRS_CUDA(cudaMemsetAsync(win_G + W, 0, sizeof(int), st));
-    if (S > 0) {
-        kb_unit_nnz<<<grid_for(S), 256, 0, st>>>(cand, S, wc_win, wc_count, win_cb, win_ub, nullptr, win_U, unit_nnz);
-        TRS_LAUNCH_CHECK();
-    }
 
-    // ---- 6. matching -----------------------------------------------------------------------------
-    // small windows: one thread each; medium: one warp each; heavy (hubs): one 256-thread block each
-    int *sel_light, *sel_medium, *sel_heavy, *sel_cnt;
-    TRS_TRY(sc.get<int>((size_t)W + 1, &sel_light));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &sel_medium));
-    TRS_TRY(sc.get<int>((size_t)W + 1, &sel_heavy));
-    TRS_TRY(sc.get<int>(4, &sel_cnt));
-    TRS_CUDA(cudaMemsetAsync(sel_cnt, 0, 4 * sizeof(int), st));
-    kb_split_windows<<<grid_for(W), 256, 0, st>>>(win_U, W, sel_light, sel_medium, sel_heavy, sel_cnt);
-    TRS_LAUNCH_CHECK();
-    int h_cnt[4] = {0, 0, 0, 0};
-    TRS_CUDA(cudaMemcpyAsync(h_cnt, sel_cnt, 4 * sizeof(int), cudaMemcpyDeviceToHost, st));
-    TRS_CUDA(cudaStreamSynchronize(st));
-    if (h_cnt[0] > 0) {
-        kb_match<<<grid_for(h_cnt[0], 64), 64, 0, st>>>(win_U, win_ub, win_pb, W, cfg.unit_min_nnz, unit_nnz, order_buf,
-                                                          matched, pair_a, pair_b, win_G, win_cuda_unit, sel_light, h_cnt[0]);
-        TRS_LAUNCH_CHECK();
+    // ---- 6. matching ------------------------------------------------------------------------------
+    MatchOut mo;
+    TRS_TRY(ts.get(TU, &mo.order));
+    TRS_TRY(ts.get(TS, &mo.pair_a));
+    TRS_TRY(ts.get(TS, &mo.pair_b));
+    TRS_TRY(ts.get((size_t)W + 1, &mo.groups));
+    TRS_TRY(ts.get((size_t)W + 1, &mo.tiles));
+    TRS_TRY(ts.get((size_t)W + 1, &mo.cuda_unit));
+    if (mc.max_huge >= (int)kUnitMask) return TRS_E_LIMIT;
+    // one long chain per hub window: the tiers run side by side
+    cudaStream_t side[2] = {st, st};
+    Event ready, done[2];
+    if (mc.n_huge + mc.n_block > 0) {
+        TRS_TRY(side_streams(side));
+        TRS_TRY(ready.record(st));
+        TRS_CUDA(cudaFuncSetAttribute(kb_match_block, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemUnits * 4));
     }
-    if (h_cnt[1] > 0) {
-        const int cap_words = (kHeavyUnits + 31) / 32;
-        const size_t smem = (size_t)cap_words * 4 + (size_t)kOrderTile * 4;
-        kb_match_coop<32, 64><<<h_cnt[1], 32, smem, st>>>(win_U, win_ub, win_pb, cfg.unit_min_nnz, unit_nnz, order_buf, matched,
-                                                          pair_a, pair_b, win_G, win_cuda_unit, sel_medium, cap_words);
-        TRS_LAUNCH_CHECK();
-    }
-    if (h_cnt[2] > 0) {
-        // shared memory: bitmask of matched units (as many words as fit) + one tile of the order
-        const int max_words = (h_cnt[3] + 31) / 32;
-        const int cap_words = std::min(max_words, (200 * 1024 - kOrderTile * 4) / 4);
-        const size_t smem = (size_t)cap_words * 4 + (size_t)kOrderTile * 4;
-        TRS_CUDA(cudaFuncSetAttribute(kb_match_coop<256, 1024>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        kb_match_coop<256, 1024><<<h_cnt[2], 256, smem, st>>>(win_U, win_ub, win_pb, cfg.unit_min_nnz, unit_nnz, order_buf,
-                                                              matched, pair_a, pair_b, win_G, win_cuda_unit, sel_heavy,
-                                                              cap_words);
-        TRS_LAUNCH_CHECK();
-    }
-    TRS_TRY(cub_.exclusive_sum(win_G, B->s_offset.p, W + 1));
-    int G = 0;
-    TRS_TRY(read_int(B->s_offset.p + W, st, &G));
-
-    // ---- 7. groups ---------------------------------------------------------------------------------
-    int* grp_wcol;
-    TRS_TRY(sc.get<int>((size_t)G * 4, &grp_wcol));
-    TRS_TRY(B->s_column.alloc_from(B->arena, (size_t)G * 4));
-    TRS_TRY(B->s_window.alloc_from(B->arena, G));
-    TRS_TRY(B->s_mask.alloc_from(B->arena, (size_t)G * window));
-    TRS_TRY(B->s_value.alloc_from(B->arena, (size_t)G * window * 2));
-    TRS_TRY(B->s_pos.alloc_from(B->arena, (size_t)G * window * 2));
-    unsigned long long* d_dropped;
-    TRS_TRY(sc.get<unsigned long long>(1, &d_dropped));
-    TRS_CUDA(cudaMemsetAsync(d_dropped, 0, sizeof(unsigned long long), st));
-    if (G > 0) {
-        kb_emit_groups<<<grid_for(TS), 256, 0, st>>>(win_pb, win_G, B->s_offset.p, win_cb, win_U, wc_begin, s_idx, W, TS,
-                                                      pair_a, pair_b, cand, wc_col, B->s_column.p, B->s_window.p, grp_wcol);
-        TRS_LAUNCH_CHECK();
-        kb_emit_rows<<<grid_for((long long)G * window), 256, 0, st>>>(grp_wcol, (long long)G * window, window, wc_mask,
-                                                                       wc_start, wc_col, B->s_window.p, edge, val,
-                                                                       B->s_mask.p, B->s_value.p, B->s_pos.p, d_dropped,
-                                                                       nullptr, nullptr, nullptr, nullptr, 1);
-        TRS_LAUNCH_CHECK();
-    }
-    // strict mode: collect what was dropped, ordered by (row, column)
-    int* row_extra = nullptr;
-    int* extra_off = nullptr;
-    unsigned long long* extra_key = nullptr;
-    int* extra_at = nullptr;
-    if (cfg.strict && G > 0) {
-        unsigned long long h_dropped = 0;
-        TRS_CUDA(cudaMemcpyAsync(&h_dropped, d_dropped, sizeof(h_dropped), cudaMemcpyDeviceToHost, st));
-        TRS_CUDA(cudaStreamSynchronize(st));
-        if (h_dropped > 0) {
-            unsigned long long *key_a, *key_b, *d_xcount;
-            int *at_a, *at_b;
-            TRS_TRY(sc.get<unsigned long long>(h_dropped, &key_a));
-            TRS_TRY(sc.get<unsigned long long>(h_dropped, &key_b));
-            TRS_TRY(sc.get<int>(h_dropped, &at_a));
-            TRS_TRY(sc.get<int>(h_dropped, &at_b));
-            TRS_TRY(sc.get<unsigned long long>(1, &d_xcount));
-            TRS_TRY(sc.get<int>((size_t)n + 1, &row_extra));
-            TRS_TRY(sc.get<int>((size_t)n + 1, &extra_off));
-            TRS_CUDA(cudaMemsetAsync(d_xcount, 0, sizeof(unsigned long long), st));
-            TRS_CUDA(cudaMemsetAsync(row_extra, 0, sizeof(int) * ((size_t)n + 1), st));
-            kb_emit_rows<<<grid_for((long long)G * window), 256, 0, st>>>(grp_wcol, (long long)G * window, window, wc_mask,
-                                                                           wc_start, wc_col, B->s_window.p, edge, val, nullptr,
-                                                                           nullptr, nullptr, nullptr, key_a, at_a, d_xcount,
-                                                                           row_extra, 0);
-            TRS_LAUNCH_CHECK();
-            TRS_TRY(cub_.sort_pairs(key_a, key_b, at_a, at_b, (long long)h_dropped, 32 + bits_for(n), &extra_key, &extra_at));
-            TRS_TRY(cub_.exclusive_sum(row_extra, extra_off, (long long)n + 1));
-            TRS_CUDA(cudaMemsetAsync(d_dropped, 0, sizeof(unsigned long long), st));   // nothing is lost in this mode
+    if (mc.n_huge > 0) {
+        const int smem_units = mc.max_huge <= kSmemUnits ? mc.max_huge : kSmemUnits;
+        int* words = nullptr;
+        unsigned* mask = nullptr;
+        if (mc.max_huge > kSmemUnits) {
+            TRS_TRY(ts.get(TU, &words));
+            TRS_TRY(ts.get((size_t)TU / 32 + W + 2, &mask));
         }
-    }
-
-    // ---- 8. TC blocks, values, parts ------------------------------------------------------------
-    int *blk_nnz, *wc_slot;
-    TRS_TRY(sc.get<int>((size_t)NB + 1, &blk_nnz));
-    TRS_TRY(sc.get<int>(D, &wc_slot));
-    TRS_CUDA(cudaMemsetAsync(wc_slot, 0xFF, sizeof(int) * (size_t)D, st));
-    TRS_CUDA(cudaMemsetAsync(blk_nnz + NB, 0, sizeof(int), st));
-    B->t_block_offset.release();
-    TRS_TRY(B->t_block_offset.alloc_from(B->arena, (size_t)NB + 1));
-    TRS_TRY(B->t_column.alloc_from(B->arena, (size_t)NB * 8));
-    TRS_TRY(B->t_binary.alloc_from(B->arena, (size_t)NB * 2));
-    int tc_nnz = 0;
-    if (NB > 0) {
-        kb_tc_blocks<<<grid_for(NB), 256, 0, st>>>(blk_pos, blk_len, NB, ord, wc_col, wc_mask, B->t_column.p, B->t_binary.p,
-                                                    blk_nnz, wc_slot);
+        TRS_CUDA(cudaStreamWaitEvent(side[0], ready.e, 0));
+        kb_match_block<<<mc.n_huge, kBlockThreads, (size_t)smem_units * 4, side[0]>>>(v, R.key2, cfg.unit_min_nnz, smem_units, words, mask,
+                                                                                 sel_huge, mo);
         TRS_LAUNCH_CHECK();
     }
+    if (mc.n_block > 0) {
+        TRS_CUDA(cudaStreamWaitEvent(side[1], ready.e, 0));
+        kb_match_block<<<mc.n_block, kBlockThreads, (size_t)kBlockUnits * 4, side[1]>>>(v, R.key2, cfg.unit_min_nnz, kBlockUnits, nullptr,
+                                                                                   nullptr, sel_block, mo);
+        TRS_LAUNCH_CHECK();
+    }
+    {
+        const int units = std::max(32, (mc.max_warp + 31) & ~31);
+        const size_t smem = (size_t)kMatchWarps * (units + units / 32) * 4;
+        kb_match_warp<<<grid_for(W + 1, kMatchWarps), 32 * kMatchWarps, smem, st>>>(v, W, R.key2, cfg.unit_min_nnz, units, mo);
+        TRS_LAUNCH_CHECK();
+    }
+    if (mc.n_huge > 0) { TRS_TRY(done[0].record(side[0])); TRS_CUDA(cudaStreamWaitEvent(st, done[0].e, 0)); }
+    if (mc.n_block > 0) { TRS_TRY(done[1].record(side[1])); TRS_CUDA(cudaStreamWaitEvent(st, done[1].e, 0)); }
+    TRS_TRY(B->out(B->s_offset, 22, (size_t)W + 1));
+    TRS_TRY(B->out(B->s_window_tile_offset, 28, (size_t)W + 1));
+    TRS_TRY(cub_.exclusive_sum(mo.groups, B->s_offset.p, W + 1));
+    TRS_TRY(cub_.exclusive_sum(mo.tiles, B->s_window_tile_offset.p, W + 1));
+
+    // ---- 8. TC blocks (their values need the block offsets) --------------------------------------
+    int *blk_nnz, *slot_rec;
+    TRS_TRY(ts.get((size_t)NB + 1, &blk_nnz));
+    TRS_TRY(ts.get((size_t)NB * 8, &slot_rec));
+    TRS_TRY(B->out(B->t_block_offset, 1, (size_t)NB + 1));
+    TRS_TRY(B->out(B->t_column, 2, (size_t)NB * 8));
+    TRS_TRY(B->out(B->t_binary, 6, (size_t)NB * 2));
+    kb_tc_blocks<<<grid_for(NB + 1, 128), 128, 0, st>>>(v, rv, W, NB, B->t_column.p, B->t_binary.p, blk_nnz, slot_rec);
+    TRS_LAUNCH_CHECK();
     TRS_TRY(cub_.exclusive_sum(blk_nnz, B->t_block_offset.p, (long long)NB + 1));
-    TRS_TRY(read_int(B->t_block_offset.p + NB, st, &tc_nnz));
-    TRS_TRY(B->t_value.alloc_from(B->arena, tc_nnz));
+    TRS_TRY(B->out(B->t_row_offset, 0, (size_t)NP + 1));
+    TRS_TRY(B->out(B->t_window_row, 4, NP));
+    TRS_TRY(B->out(B->t_atomic, 5, NP));
+    kb_tc_parts<<<grid_for(W), 256, 0, st>>>(v, mo.cuda_unit, W, cfg.part_t, B->t_row_offset.p, B->t_window_row.p, B->t_atomic.p);
+    TRS_LAUNCH_CHECK();
+
+    // ---- 9. CUDA-core parts: counted now, or in strict mode when the dropped entries are known ------
+    Parts *cnt, *off;
+    TRS_TRY(ts.get((size_t)n + 1, &cnt));
+    TRS_TRY(ts.get((size_t)n + 1, &off));
+    Extras x{nullptr, nullptr, 0};
+    auto count_parts = [&]() -> int {
+        kb_cuda_count<<<grid_for(n + 1), 256, 0, st>>>(n, window, cfg.part_c, cfg.short_size, mo.cuda_unit, v, rv, x, cnt);
+        TRS_LAUNCH_CHECK();
+        return cub_.exclusive_scan(cnt, off, PartsSum(), Parts{0, 0, 0, 0}, (long long)n + 1);
+    };
+    if (!cfg.strict) TRS_TRY(count_parts());
+    kb_totals<<<1, 1, 0, st>>>(B->s_offset.p, B->s_window_tile_offset.p, W, B->t_block_offset.p, NB, cfg.strict ? nullptr : off, n,
+                               &d_head->tot);
+    TRS_LAUNCH_CHECK();
+    Totals tot;
+    TRS_TRY(read_back(&d_head->tot, &tot, st));
+    const int G = tot.groups, T = tot.tiles;
+
+    TRS_TRY(B->out(B->t_value, 3, tot.tc_nnz));
     if (NB > 0) {
-        kb_tc_values<<<grid_for(nnz), 256, 0, st>>>(keys, edge, wc_incl, nnz, wc_slot, B->t_binary.p, B->t_block_offset.p,
-                                                     val, B->t_value.p);
+        kb_tc_values<<<grid_for((long long)NB * 128), 256, 0, st>>>(rv, slot_rec, NB, B->t_binary.p, B->t_block_offset.p, B->t_value.p);
         TRS_LAUNCH_CHECK();
     }
-    B->t_row_offset.release();
-    TRS_TRY(B->t_row_offset.alloc_from(B->arena, (size_t)NP + 1));
-    TRS_TRY(B->t_window_row.alloc_from(B->arena, NP));
-    TRS_TRY(B->t_atomic.alloc_from(B->arena, NP));
-    kb_tc_parts<<<grid_for(W), 256, 0, st>>>(wc_begin, b_idx, win_bb, part_off, win_cuda_unit, W, cfg.part_t,
-                                              B->t_row_offset.p, B->t_window_row.p, B->t_atomic.p);
-    TRS_LAUNCH_CHECK();
 
-    // ---- 9. CUDA-core row parts ---------------------------------------------------------------
-    int *cnt4, *off4;
-    const size_t stride = (size_t)n + 1;
-    TRS_TRY(sc.get<int>(4 * stride, &cnt4));
-    TRS_TRY(sc.get<int>(4 * stride, &off4));
-    TRS_CUDA(cudaMemsetAsync(cnt4, 0, sizeof(int) * 4 * stride, st));
-    kb_cuda_count<<<grid_for(n), 256, 0, st>>>(n, window, cfg.part_c, cfg.short_size, win_cuda_unit, win_cb, wc_begin, s_idx,
-                                                cand, wc_col, wc_mask, wc_start, row_extra, cnt4);
-    TRS_LAUNCH_CHECK();
-    int tot[4] = {0, 0, 0, 0};
-    for (int i = 0; i < 4; ++i) {
-        TRS_TRY(cub_.exclusive_sum(cnt4 + i * stride, off4 + i * stride, (long long)stride));
-        TRS_CUDA(cudaMemcpyAsync(&tot[i], off4 + i * stride + n, sizeof(int), cudaMemcpyDeviceToHost, st));
+    // ---- 7. groups and tiles ------------------------------------------------------------------------
+    TRS_TRY(B->out(B->s_column, 17, (size_t)G * 4));
+    TRS_TRY(B->out(B->s_mask, 18, (size_t)G * window));
+    TRS_TRY(B->out(B->s_value, 19, (size_t)G * window * 2));
+    TRS_TRY(B->out(B->s_pos, 20, (size_t)G * window * 2));
+    TRS_TRY(B->out(B->s_window, 21, G));
+    TRS_TRY(B->out(B->s_tile_window, 23, T));
+    TRS_TRY(B->out(B->s_tile_group, 24, T));
+    TRS_TRY(B->out(B->s_tile_column, 25, (size_t)T * 16));
+    TRS_TRY(B->out(B->s_packed_a, 26, (size_t)T * 64));
+    TRS_TRY(B->out(B->s_packed_meta, 27, (size_t)T * 8));
+    u64 *xkey_a = nullptr, *xkey_b = nullptr;
+    int *xat_a = nullptr, *xat_b = nullptr;
+    if (cfg.strict) {   // at least two of a row's entries in a group are kept, so at most half are dropped
+        TRS_TRY(ts.get((size_t)nnz / 2 + 1, &xkey_a));
+        TRS_TRY(ts.get((size_t)nnz / 2 + 1, &xat_a));
     }
-    TRS_CUDA(cudaStreamSynchronize(st));
-    B->c_row_offset.release(); B->cs_row_offset.release();
-    TRS_TRY(B->c_row_offset.alloc_from(B->arena, (size_t)tot[0] + 1));
-    TRS_TRY(B->c_row.alloc_from(B->arena, tot[0]));
-    TRS_TRY(B->c_atomic.alloc_from(B->arena, tot[0]));
-    TRS_TRY(B->c_column.alloc_from(B->arena, tot[2]));
-    TRS_TRY(B->c_value.alloc_from(B->arena, tot[2]));
-    TRS_TRY(B->cs_row_offset.alloc_from(B->arena, (size_t)tot[1] + 1));
-    TRS_TRY(B->cs_row.alloc_from(B->arena, tot[1]));
-    TRS_TRY(B->cs_atomic.alloc_from(B->arena, tot[1]));
-    TRS_TRY(B->cs_column.alloc_from(B->arena, tot[3]));
-    TRS_TRY(B->cs_value.alloc_from(B->arena, tot[3]));
-    kb_cuda_fill<<<grid_for(n), 256, 0, st>>>(n, window, cfg.part_c, cfg.short_size, win_cuda_unit, win_cb, wc_begin, s_idx,
-                                               b_idx, cand, wc_col, wc_mask, wc_start, edge, val, off4, extra_off, extra_key,
-                                               extra_at, B->c_row_offset.p,
-                                               B->c_row.p, B->c_atomic.p, B->c_column.p, B->c_value.p, B->cs_row_offset.p,
-                                               B->cs_row.p, B->cs_atomic.p, B->cs_column.p, B->cs_value.p);
-    TRS_LAUNCH_CHECK();
-
-    // ---- 10. tiles -----------------------------------------------------------------------------------
-    int* win_T;
-    TRS_TRY(sc.get<int>((size_t)W + 1, &win_T));
-    TRS_CUDA(cudaMemsetAsync(win_T + W, 0, sizeof(int), st));
-    kb_win_tiles<<<grid_for(W), 256, 0, st>>>(win_G, W, win_T);
-    TRS_TRY(cub_.exclusive_sum(win_T, B->s_window_tile_offset.p, W + 1));
-    int T = 0;
-    TRS_TRY(read_int(B->s_window_tile_offset.p + W, st, &T));
-    TRS_TRY(B->s_tile_window.alloc_from(B->arena, T));
-    TRS_TRY(B->s_tile_group.alloc_from(B->arena, T));
-    TRS_TRY(B->s_tile_column.alloc_from(B->arena, (size_t)T * 16));
-    TRS_TRY(B->s_packed_a.alloc_from(B->arena, (size_t)T * 64));
-    TRS_TRY(B->s_packed_meta.alloc_from(B->arena, (size_t)T * 8));
     if (T > 0) {
-        kb_tiles<<<grid_for(T), 256, 0, st>>>(B->s_window_tile_offset.p, B->s_offset.p, W, T, B->s_tile_window.p,
-                                               B->s_tile_group.p);
+        kb_tiles<<<grid_for(T), 256, 0, st>>>(B->s_window_tile_offset.p, B->s_offset.p, W, T, B->s_tile_window.p, B->s_tile_group.p);
         TRS_LAUNCH_CHECK();
-        TRS_TRY(pack_tiles(B->s_column.p, B->s_value.p, (const int8_t*)B->s_pos.p, B->s_offset.p, B->s_tile_window.p,
-                           B->s_tile_group.p, T, window, B->s_tile_column.p, B->s_packed_a.p, B->s_packed_meta.p, st));
+        const GroupOut go{B->s_column.p, B->s_mask.p, B->s_value.p, B->s_pos.p, B->s_window.p, B->s_tile_column.p,
+                          B->s_packed_a.p, B->s_packed_meta.p};
+        const ExtraOut xo{d_head->dropped, xkey_a, xat_a};
+        auto emit = cfg.strict ? kb_emit_tiles<true> : kb_emit_tiles<false>;
+        // strict mode collects a warp's extras over many tiles; otherwise a tile per warp hides most latency
+        emit<<<cfg.strict ? std::min(grid_for(T, 8), (unsigned)sms * 8u) : grid_for(T, 8), 256, 0, st>>>(v, rv, B->s_offset.p, B->s_tile_window.p, B->s_tile_group.p,
+                                                                           T, window, mo.pair_a, mo.pair_b, go, xo);
+        TRS_LAUNCH_CHECK();
     }
-    TRS_CUDA(cudaMemcpyAsync(&B->dropped, d_dropped, sizeof(unsigned long long), cudaMemcpyDeviceToHost, st));
-    TRS_CUDA(cudaStreamSynchronize(st));
+    if (cfg.strict) {
+        u64 n_extra = 0;
+        TRS_TRY(read_back(d_head->dropped, &n_extra, st));
+        if (n_extra > 0) {
+            u64* key;
+            int* at;
+            TRS_TRY(ts.get(n_extra, &xkey_b));
+            TRS_TRY(ts.get(n_extra, &xat_b));
+            TRS_TRY(cub_.sort_pairs(xkey_a, xkey_b, xat_a, xat_b, (long long)n_extra, 32 + bits_for(n), &key, &at));
+            x = Extras{key, at, (int)n_extra};
+        }
+        TRS_TRY(count_parts());
+        TRS_TRY(read_back(off + n, &tot.parts, st));
+    }
+    const Parts& p = tot.parts;
+    TRS_TRY(B->out(B->c_row_offset, 7, (size_t)p.nl + 1));
+    TRS_TRY(B->out(B->c_row, 8, p.nl));
+    TRS_TRY(B->out(B->c_atomic, 9, p.nl));
+    TRS_TRY(B->out(B->c_column, 10, p.zl));
+    TRS_TRY(B->out(B->c_value, 11, p.zl));
+    TRS_TRY(B->out(B->cs_row_offset, 12, (size_t)p.ns + 1));
+    TRS_TRY(B->out(B->cs_row, 13, p.ns));
+    TRS_TRY(B->out(B->cs_atomic, 14, p.ns));
+    TRS_TRY(B->out(B->cs_column, 15, p.zs));
+    TRS_TRY(B->out(B->cs_value, 16, p.zs));
+    const PartsOut po{B->c_row_offset.p, B->c_row.p, B->c_atomic.p, B->c_column.p, B->c_value.p,
+                      B->cs_row_offset.p, B->cs_row.p, B->cs_atomic.p, B->cs_column.p, B->cs_value.p};
+    kb_cuda_rows<<<grid_for(n), 256, 0, st>>>(n, window, cfg.part_c, cfg.short_size, mo.cuda_unit, v, rv, x, off, po);
+    TRS_LAUNCH_CHECK();
+    if (x.n > 0) {
+        kb_cuda_extras<<<grid_for(x.n), 256, 0, st>>>(window, mo.cuda_unit, v, rv, x, off, po);
+        TRS_LAUNCH_CHECK();
+    }
+    Head head;
+    TRS_TRY(read_back(d_head, &head, st));
+    B->dropped = 0;
+    if (!cfg.strict)   // nothing is lost in strict mode
+        for (u64 d : head.dropped) B->dropped += d;
     TRS_LAUNCH_CHECK();
     return TRS_OK;
 }
@@ -1324,8 +1630,8 @@ const void* array_ptr(const trs_builder* B, int id, size_t* elem) {
 }  // namespace
 
 static int build_impl(const int32_t* rowptr, const int32_t* col, const float* values, int n_rows,
-                      const trs_build_config* cfg, void* arena, size_t arena_bytes, bool use_arena, void* stream,
-                      trs_builder** out) {
+                      const trs_build_config* cfg, void* arena, size_t arena_bytes, bool use_arena, trs_build_alloc alloc,
+                      void* ctx, void* stream, trs_builder** out) {
     if (!rowptr || !cfg || !out || n_rows <= 0) return TRS_E_ARG;
     *out = nullptr;
     if (cfg->window <= 0 || cfg->window > 16) return TRS_E_WINDOW;
@@ -1339,6 +1645,8 @@ static int build_impl(const int32_t* rowptr, const int32_t* col, const float* va
         B->arena_store.cap = arena_bytes;
         B->arena = &B->arena_store;
     }
+    B->alloc = alloc;
+    B->alloc_ctx = ctx;
     B->cfg = BuildCfg{cfg->part_t, cfg->part_c, cfg->short_size, cfg->density, cfg->window, cfg->tc_min_util,
                       cfg->skip_tc, cfg->unit_min_nnz, cfg->strict ? 1 : 0};
     B->n_rows = n_rows;
@@ -1361,7 +1669,14 @@ static int build_impl(const int32_t* rowptr, const int32_t* col, const float* va
 
 extern "C" int trs_build_create(const int32_t* rowptr, const int32_t* col, const float* values, int n_rows,
                                 const trs_build_config* cfg, void* stream, trs_builder** out) {
-    return build_impl(rowptr, col, values, n_rows, cfg, nullptr, 0, false, stream, out);
+    return build_impl(rowptr, col, values, n_rows, cfg, nullptr, 0, false, nullptr, nullptr, stream, out);
+}
+
+extern "C" int trs_build_create_into(const int32_t* rowptr, const int32_t* col, const float* values, int n_rows,
+                                     const trs_build_config* cfg, trs_build_alloc alloc, void* ctx, void* stream,
+                                     trs_builder** out) {
+    if (!alloc) return TRS_E_ARG;
+    return build_impl(rowptr, col, values, n_rows, cfg, nullptr, 0, false, alloc, ctx, stream, out);
 }
 
 // Upper bound of the device memory one build can need (outputs + temporaries), from the sizes
@@ -1390,7 +1705,7 @@ extern "C" int trs_build_query(int n_rows, long long nnz, const trs_build_config
 extern "C" int trs_build_fill(const int32_t* rowptr, const int32_t* col, const float* values, int n_rows,
                               const trs_build_config* cfg, void* arena, size_t arena_bytes, void* stream,
                               trs_builder** out) {
-    return build_impl(rowptr, col, values, n_rows, cfg, arena, arena_bytes, true, stream, out);
+    return build_impl(rowptr, col, values, n_rows, cfg, arena, arena_bytes, true, nullptr, nullptr, stream, out);
 }
 
 extern "C" int trs_build_arena_used(const trs_builder* B, size_t* bytes) {
@@ -1471,6 +1786,13 @@ extern "C" int trs_build_format(trs_builder* B, trs_format* out, void* stream) {
     out->num_windows = B->W; out->tiles = (int)B->s_tile_window.n;
     return TRS_OK;
 }
+
+namespace {
+struct UnitLess {
+    const unsigned char* nnz;
+    __host__ __device__ bool operator()(int a, int b) const { return nnz[a] > nnz[b]; }
+};
+}  // namespace
 
 // Host-side run of the std::sort emulation (the same code the matching kernel runs), so that
 // it can be checked against libstdc++ without a GPU.

@@ -60,6 +60,58 @@ struct Arena {
     }
 };
 
+// Device memory from the library's stream-ordered pool (one per device, trs_api.cu).  A cudaMalloc /
+// cudaFree pair costs 80 - 400 us here and stops the device; the pool gives memory that an earlier call
+// freed back in about a microsecond.  It keeps at most kPoolKeepBytes between calls (trs_pool_trim returns that
+// too), may be used from any thread, and hands memory freed on one stream to another only after the
+// free has been reached on the first.
+constexpr size_t kPoolKeepBytes = (size_t)4 << 30;
+int pool_alloc(void** p, size_t bytes, cudaStream_t st);
+void pool_free(void* p, cudaStream_t st);
+
+// Temporaries of one call: blocks cut out of the caller's arena, or out of chunks from the pool.
+struct TempSpace {
+    Arena* arena = nullptr;
+    cudaStream_t st = nullptr;
+    size_t chunk_bytes = (size_t)16 << 20;
+    static constexpr int kMaxChunks = 32;
+    Arena chunk[kMaxChunks];
+    int n_chunks = 0;
+    int take(size_t bytes, void** out) {
+        *out = nullptr;
+        if (arena) { *out = arena->take(bytes); return *out ? 0 : TRS_E_WORKSPACE; }
+        for (int i = n_chunks; i-- > 0;)
+            if ((*out = chunk[i].take(bytes))) return 0;
+        if (n_chunks == kMaxChunks) return (int)cudaErrorMemoryAllocation;
+        Arena& c = chunk[n_chunks];
+        c = Arena();
+        c.cap = (bytes > chunk_bytes ? bytes : chunk_bytes) + 256;
+        const int rc = pool_alloc((void**)&c.base, c.cap, st);
+        if (rc) return rc;
+        ++n_chunks;
+        *out = c.take(bytes);
+        return *out ? 0 : (int)cudaErrorMemoryAllocation;
+    }
+    template <class T>
+    int get(size_t n, T** out) {
+        void* d;
+        const int rc = take((n ? n : 1) * sizeof(T), &d);
+        *out = (T*)d;
+        return rc;
+    }
+    // gives a block back early, so that later requests can use it
+    template <class T>
+    void drop(T* p, size_t n) {
+        const size_t bytes = (n ? n : 1) * sizeof(T);
+        if (arena) { arena->give_back(p, bytes); return; }
+        for (int i = 0; i < n_chunks; ++i)
+            if ((unsigned char*)p >= chunk[i].base && (unsigned char*)p < chunk[i].base + chunk[i].cap) chunk[i].give_back(p, bytes);
+    }
+    ~TempSpace() {
+        for (int i = 0; i < n_chunks; ++i) pool_free(chunk[i].base, st);
+    }
+};
+
 // Simple owning device buffer for plan-lifetime index arrays; with an arena the memory is the
 // caller's and release() only forgets it.
 template <class T>

@@ -51,6 +51,8 @@ class TrsTiming(C.Structure):
                 ("total_ms", "tc_ms", "cuda_long_ms", "cuda_short_ms", "sptc_ms", "h2d_ms", "d2h_ms")]
 
 
+BuildAlloc = C.CFUNCTYPE(C.c_void_p, C.c_void_p, C.c_int, C.c_size_t)   # trs_build_alloc
+
 _LIB = None
 
 
@@ -112,6 +114,10 @@ def load():
     for name in ("trs_sddmm_plan_create", "trs_sddmm_plan_run", "trs_sddmm_plan_info", "trs_sddmm_plan_destroy"):
         getattr(lib, name).restype = i32
     lib.trs_build_create.argtypes = [vp, vp, vp, i32, C.POINTER(TrsBuildConfig), vp, C.POINTER(vp)]
+    lib.trs_pool_trim.argtypes = []
+    lib.trs_pool_trim.restype = i32
+    lib.trs_build_create_into.argtypes = [vp, vp, vp, i32, C.POINTER(TrsBuildConfig), BuildAlloc, vp, vp, C.POINTER(vp)]
+    lib.trs_build_create_into.restype = i32
     lib.trs_build_fill.argtypes = [vp, vp, vp, i32, C.POINTER(TrsBuildConfig), vp, sz, vp, C.POINTER(vp)]
     lib.trs_build_fill.restype = i32
     lib.trs_build_query.argtypes = [i32, C.c_longlong, C.POINTER(TrsBuildConfig), C.POINTER(sz)]

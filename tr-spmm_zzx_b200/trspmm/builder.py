@@ -79,6 +79,7 @@ def build_format(rowptr: torch.Tensor, col: torch.Tensor, val: torch.Tensor, par
                               int(e_min if unit_min_nnz is None else unit_min_nnz), int(bool(strict)))
     lib = _lib.load()
     handle = C.c_void_p()
+    arrays = [None] * len(FORMAT_NAMES)
     if arena is not None:
         if arena.device != dev or arena.dtype != torch.uint8 or not arena.is_contiguous():
             raise ValueError("arena must be a contiguous uint8 tensor on the inputs' device")
@@ -86,38 +87,46 @@ def build_format(rowptr: torch.Tensor, col: torch.Tensor, val: torch.Tensor, par
         skip = (-base) % 256                      # the library wants a 256-byte aligned start
         if arena.numel() <= skip:
             raise ValueError("arena too small")
+    failed = []
+
+    def hand_out(_ctx, i, n_bytes):               # the arrays are torch tensors from the start: nothing is copied
+        try:
+            dt = _DTYPES.get(FORMAT_NAMES[i], torch.int32)
+            arrays[i] = torch.empty(n_bytes // dt.itemsize, dtype=dt, device=dev)
+            return arrays[i].data_ptr()
+        except Exception as e:                    # an exception cannot cross the C frames
+            failed.append(e)
+            return None
+
     arena_used = 0
     with torch.cuda.device(dev):
         stream = _lib.current_stream_ptr(dev)
         args = (rowptr.data_ptr(), col.data_ptr() if col.numel() else None, val.data_ptr() if val.numel() else None,
                 rowptr.numel() - 1, C.byref(cfg))
         if arena is None:
-            _lib.check(lib.trs_build_create(*args, stream, C.byref(handle)))
+            rc = lib.trs_build_create_into(*args, _lib.BuildAlloc(hand_out), None, stream, C.byref(handle))
+            if failed:
+                raise failed[0]
+            _lib.check(rc)
         else:
             _lib.check(lib.trs_build_fill(*args, base + skip, arena.numel() - skip, stream, C.byref(handle)))
         try:
-            sizes = (C.c_longlong * len(FORMAT_NAMES))()
-            _lib.check(lib.trs_build_sizes(handle, sizes))
             stats = _lib.TrsBuildStats()
             _lib.check(lib.trs_build_stats(handle, C.byref(stats)))
-            arrays = []
-            for i, name in enumerate(FORMAT_NAMES):
-                dt = _DTYPES.get(name, torch.int32)
-                n_el = int(sizes[i])
-                if arena is None:
-                    t = torch.empty(n_el, dtype=dt, device=dev)
-                    if n_el:
-                        _lib.check(lib.trs_build_copy(handle, i, t.data_ptr(), 0, stream))
-                elif n_el:
-                    off = int(lib.trs_build_array(handle, i)) - base
-                    t = arena[off:off + n_el * torch.empty(0, dtype=dt).element_size()].view(dt)
-                else:
-                    t = torch.empty(0, dtype=dt, device=dev)
-                arrays.append(t.view(_shape(name, n_el, window)))
             if arena is not None:
+                sizes = (C.c_longlong * len(FORMAT_NAMES))()
+                _lib.check(lib.trs_build_sizes(handle, sizes))
+                for i, name in enumerate(FORMAT_NAMES):
+                    if sizes[i]:
+                        dt = _DTYPES.get(name, torch.int32)
+                        off = int(lib.trs_build_array(handle, i)) - base
+                        arrays[i] = arena[off:off + sizes[i] * dt.itemsize].view(dt)
                 used = C.c_size_t()
                 _lib.check(lib.trs_build_arena_used(handle, C.byref(used)))
                 arena_used = used.value + skip
+            for i, name in enumerate(FORMAT_NAMES):
+                t = arrays[i] if arrays[i] is not None else torch.empty(0, dtype=_DTYPES.get(name, torch.int32), device=dev)
+                arrays[i] = t.view(_shape(name, t.numel(), window))
             torch.cuda.current_stream(dev).synchronize()
         finally:
             lib.trs_build_destroy(handle)
