@@ -87,8 +87,14 @@ const char* trs_strerror(int code);
 int trs_version(void);
 int trs_device_count(void);
 /* The library keeps up to 4 GiB of freed device memory per GPU for its next calls (temporaries, the buffers of
- * the host-buffer entries); this returns what the current device's pool holds to the driver. */
+ * the host-buffer entries) and 32 MiB of pinned host memory for copies from and to pageable memory; this
+ * returns what the current device's pool holds, and the pinned memory, to the driver. */
 int trs_pool_trim(void);
+/* Copies n device arrays into host memory of any kind (pageable memory through the pinned ring, several threads
+ * filling it); ordered after the work on `stream`, complete on return. */
+int trs_copy_to_host(int n, void* const* host, const void* const* dev, const size_t* bytes, void* stream);
+/* The other direction: returns when the host arrays have been read; the copies are then queued on `stream`. */
+int trs_copy_to_device(int n, const void* const* host, void* const* dev, const size_t* bytes, void* stream);
 
 /* ---- SpMM: plan over device-resident format arrays ---------------------------------------
  * Replaces the device half of spmm_forward_fp16_tcu_cuda_sptc_mma_parallel_online

@@ -1,0 +1,42 @@
+"""Copies between pageable host arrays and the device: sizes around a chunk and around the whole pinned ring, many
+arrays in one call, two threads at once."""
+import threading
+
+import pytest
+import torch
+
+from trspmm import _lib
+
+pytestmark = pytest.mark.gpu
+MB = 1 << 20
+
+
+@pytest.mark.parametrize("sizes", [[1], [MB // 2 - 1], [MB - 1], [MB], [MB + 1], [31 * MB + 7], [32 * MB], [33 * MB + 1], [80 * MB + 5],
+                                   [0, 3, 5 * MB + 1, 0, MB, 17, 2 * MB - 1]])
+def test_round_trip(sizes):
+    dev = torch.device("cuda", 0)
+    g = torch.Generator().manual_seed(sum(sizes))
+    host = [torch.randint(0, 256, (n,), generator=g, dtype=torch.uint8) for n in sizes]
+    up = _lib.copy_to_device(host, dev)
+    for a, b in zip(up, host):
+        assert torch.equal(a, b.cuda())
+    for a, b in zip(_lib.copy_to_host(up, dev), host):
+        assert torch.equal(a, b)
+
+
+def test_two_threads():
+    dev = torch.device("cuda", 0)
+    data = [torch.arange(9 * MB + i, dtype=torch.int32) for i in range(2)]
+    bad = []
+
+    def go(i):
+        for _ in range(5):
+            if not torch.equal(_lib.copy_to_host(_lib.copy_to_device([data[i]], dev), dev)[0], data[i]):
+                bad.append(i)
+
+    threads = [threading.Thread(target=go, args=(i,)) for i in range(2)]
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not bad
+    assert _lib.load().trs_pool_trim() == 0
+    assert torch.equal(_lib.copy_to_host([data[0].cuda()], dev)[0], data[0])   # the ring comes back after a trim

@@ -13,6 +13,7 @@ import time
 
 import torch
 
+from trspmm import _lib
 from trspmm.builder import build_format
 
 __all__ = ["block_sptc_2to4_online"]
@@ -31,9 +32,12 @@ def block_sptc_2to4_online(row1, column1, values1, partSize_t, partSize_c, short
     t0 = time.perf_counter()
     on_cpu = not row1.is_cuda
     dev = torch.device("cuda", torch.cuda.current_device()) if on_cpu else row1.device
-    fmt, _ = build_format(row1.to(dev), column1.to(dev), values1.to(dev), int(partSize_t), int(partSize_c),
-                          int(shortSize), int(density), int(window), float(tc_min_util))
+    csr = [t.contiguous() for t in (row1, column1, values1)]
+    if on_cpu and not (column1.is_cuda or values1.is_cuda):
+        csr = _lib.copy_to_device(csr, dev)
+    fmt, _ = build_format(*(t.to(dev) for t in csr), int(partSize_t), int(partSize_c), int(shortSize), int(density),
+                          int(window), float(tc_min_util))
     arrays = fmt.arrays()
     if on_cpu:
-        arrays = [a.cpu() for a in arrays]
+        arrays = _lib.copy_to_host(arrays, dev)
     return arrays + [torch.tensor(time.perf_counter() - t0, dtype=torch.float32)]

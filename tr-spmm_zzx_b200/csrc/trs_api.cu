@@ -81,8 +81,9 @@ void pool_free(void* p, cudaStream_t st) {
 
 }  // namespace trs
 
-// Returns the memory the library's pool of the current device holds for later calls to the driver.
+// Returns to the driver what the library holds for later calls: the current device's pool, the pinned ring.
 extern "C" int trs_pool_trim(void) {
+    trs::release_host_ring();
     int dev = 0;
     TRS_CUDA(cudaGetDevice(&dev));
     std::lock_guard<std::mutex> lock(trs::g_pool_mutex);
@@ -92,38 +93,59 @@ extern "C" int trs_pool_trim(void) {
 
 namespace {
 
-// Owns the device copies made for one host-format upload.
+// Owns the device copies made for one host-format upload.  Arrays are first noted (put / raw), then get their
+// places in one block from the pool and are filled in one go (commit).
 struct Upload {
-    std::vector<void*> ptrs;
-    ~Upload() { for (void* p : ptrs) cudaFree(p); }
+    struct Part { const void* host; size_t bytes; void** dev; };
+    std::vector<Part> parts;
+    std::vector<void*> blocks;
+    cudaStream_t st = nullptr;
+    int device = 0;
+    ~Upload() {
+        if (blocks.empty()) return;
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev != device) cudaSetDevice(device);
+        cudaDeviceSynchronize();   // whatever still uses them, on any stream
+        for (void* p : blocks) pool_free(p, nullptr);
+        if (dev != device) cudaSetDevice(dev);
+    }
     template <class T>
     int put(const T* host, size_t n, const T** dev) {
         *dev = nullptr;
         if (n == 0) return 0;
         if (!host) return TRS_E_ARG;
-        void* d = nullptr;
-        cudaError_t e = cudaMalloc(&d, n * sizeof(T));
-        if (e != cudaSuccess) return (int)e;
-        ptrs.push_back(d);
-        e = cudaMemcpy(d, host, n * sizeof(T), cudaMemcpyHostToDevice);
-        if (e != cudaSuccess) return (int)e;
-        *dev = (const T*)d;
+        parts.push_back(Part{host, n * sizeof(T), (void**)dev});
         return 0;
-    }
-    void drop(void* d) {
-        for (void*& p : ptrs)
-            if (p && p == d) { cudaFree(d); p = nullptr; }
     }
     template <class T>
-    int raw(size_t n, T** dev) {
+    void raw(size_t n, T** dev) {
         *dev = nullptr;
-        if (n == 0) return 0;
-        void* d = nullptr;
-        cudaError_t e = cudaMalloc(&d, n * sizeof(T));
-        if (e != cudaSuccess) return (int)e;
-        ptrs.push_back(d);
-        *dev = (T*)d;
-        return 0;
+        if (n) parts.push_back(Part{nullptr, n * sizeof(T), (void**)dev});
+    }
+    int commit() {
+        size_t total = 0;
+        for (const Part& p : parts) total += (p.bytes + 255) & ~(size_t)255;
+        if (total == 0) return 0;
+        TRS_CUDA(cudaGetDevice(&device));
+        void* block;
+        int rc = pool_alloc(&block, total, st);
+        if (rc) return rc;
+        blocks.push_back(block);
+        std::vector<HostSegment> seg;
+        unsigned char* at = (unsigned char*)block;
+        for (const Part& p : parts) {
+            *p.dev = at;
+            if (p.host) seg.push_back(HostSegment{(void*)p.host, at, p.bytes});
+            at += (p.bytes + 255) & ~(size_t)255;
+        }
+        parts.clear();
+        return copy_to_device(seg.data(), (int)seg.size(), st);
+    }
+    template <class T>
+    int now(size_t n, T** dev) {   // one array by itself
+        raw(n, dev);
+        return commit();
     }
 };
 
@@ -214,6 +236,7 @@ struct EventPair {
 // chunk go back to the host while the next chunk is computed.
 constexpr int kSlots = 2;
 constexpr int kMaxChunks = 16;
+constexpr int kSlabDim = 64;   // features per slab of the blocking call
 
 struct ResidentSlot {
     trs_half* d_rhs = nullptr;
@@ -242,9 +265,11 @@ namespace {
 int slot_init(trs_resident* h, int i) {
     ResidentSlot& s = h->slot[i];
     if (s.d_rhs) return TRS_OK;
-    int rc = h->up.raw<trs_half>((size_t)h->k_cols * h->max_dim, &s.d_rhs);
-    if (!rc) rc = h->up.raw<unsigned char>((size_t)h->m_rows * h->max_dim * sizeof(float), (unsigned char**)&s.d_out);
+    h->up.raw<trs_half>((size_t)h->k_cols * h->max_dim, &s.d_rhs);
+    h->up.raw<unsigned char>((size_t)h->m_rows * h->max_dim * sizeof(float), (unsigned char**)&s.d_out);
+    const int rc = h->up.commit();
     if (rc) return rc;
+    TRS_CUDA(cudaStreamSynchronize(h->up.st));   // the pool's memory is ordered after this stream only
     TRS_CUDA(cudaEventCreateWithFlags(&s.in_done, cudaEventDisableTiming));
     TRS_CUDA(cudaEventCreateWithFlags(&s.k_done, cudaEventDisableTiming));
     TRS_CUDA(cudaEventCreateWithFlags(&s.out_done, cudaEventDisableTiming));
@@ -256,7 +281,7 @@ int resident_finish_create(trs_resident* h, int mOri, int kOri, int window, int 
     h->m_rows = mOri; h->k_cols = kOri; h->max_dim = max_dimN; h->window = window;
     int rc = trs_spmm_plan_create(&h->dev, mOri, kOri, window, 1, nullptr, &h->plan);
     if (!rc) rc = trs_spmm_workspace_bytes(h->plan, max_dimN, &h->ws_bytes);
-    if (!rc) rc = h->up.raw<unsigned char>(h->ws_bytes, (unsigned char**)&h->d_ws);
+    if (!rc) rc = h->up.now<unsigned char>(h->ws_bytes, (unsigned char**)&h->d_ws);
     if (!rc) rc = slot_init(h, 0);  // the second slot is allocated by the first overlapping submit
     if (rc) return rc;
     h->num_windows = trs_spmm_num_windows(h->plan);
@@ -277,8 +302,6 @@ int resident_chunks(const trs_resident* h, size_t out_bytes) {
     return k;
 }
 
-// Enqueue one call on the three streams; returns without waiting.  `timed` records the six
-// timing events of the synchronous entry.
 int resident_drain(trs_resident* h) {
     cudaError_t e1 = cudaStreamSynchronize(h->s_in);
     cudaError_t e2 = cudaStreamSynchronize(h->stream);
@@ -297,14 +320,61 @@ int resident_workspace(trs_resident* h, int dimN) {
     if (rc || need <= h->ws_bytes) return rc;
     rc = resident_drain(h);
     if (rc) return rc;
-    void* grown = nullptr;
-    rc = h->up.raw<unsigned char>(need, (unsigned char**)&grown);
+    void* grown = nullptr;   // the old one stays with the handle until it is destroyed
+    rc = h->up.now<unsigned char>(need, (unsigned char**)&grown);
+    if (!rc) rc = (int)cudaStreamSynchronize(h->up.st);
     if (rc) return rc;
-    h->up.drop(h->d_ws);
     h->d_ws = grown;
     h->ws_bytes = need;
     return TRS_OK;
 }
+
+// The blocking call in feature slabs: while the input copy of slab s + 1 runs, slab s is multiplied and copied
+// back - the only overlap of the two directions that one call has.  A slab's rows are cut out of the host
+// rows by 2-D copies: 128-byte pieces move at 51 GB/s (64-byte ones at 35 - 41, whole rows at 55), so
+// slabs have 64 features.  R-MAT 18, F = 128: 2.74 -> 2.1 ms.
+int resident_slabs(int dimN, size_t in_bytes) { return dimN >= 2 * kSlabDim && in_bytes >= ((size_t)8 << 20) ? dimN / kSlabDim : 1; }
+
+int resident_enqueue_slabs(trs_resident* h, const trs_half* rhs_host, void* out_host, int dimN, int out_dtype, int slabs, bool timed) {
+    ResidentSlot& s = h->slot[h->seq % kSlots];
+    int rc = slot_init(h, (int)(h->seq % kSlots));
+    const int last_dim = dimN - kSlabDim * (slabs - 1);
+    if (!rc) rc = resident_workspace(h, last_dim);
+    if (rc) return rc;
+    const size_t elt = out_dtype == TRS_OUT_F16 ? 2 : 4;
+    TRS_CUDA(cudaStreamWaitEvent(h->s_in, s.k_done, 0));
+    TRS_CUDA(cudaStreamWaitEvent(h->stream, s.out_done, 0));
+    if (timed) cudaEventRecord(h->t_ev[0], h->s_in);
+    for (int i = 0; i < slabs; ++i) {
+        const int d0 = i * kSlabDim, d = i + 1 < slabs ? kSlabDim : last_dim;
+        trs_half* in = s.d_rhs + (size_t)h->k_cols * d0;
+        unsigned char* out = (unsigned char*)s.d_out + (size_t)h->m_rows * d0 * elt;
+        TRS_CUDA(cudaMemcpy2DAsync(in, d * sizeof(trs_half), rhs_host + d0, dimN * sizeof(trs_half), d * sizeof(trs_half),
+                                   h->k_cols, cudaMemcpyHostToDevice, h->s_in));
+        TRS_CUDA(cudaEventRecord(s.in_done, h->s_in));
+        TRS_CUDA(cudaStreamWaitEvent(h->stream, s.in_done, 0));
+        if (timed && i == 0) cudaEventRecord(h->t_ev[2], h->stream);
+        rc = trs_spmm_run(h->plan, in, out, d, out_dtype, h->d_ws, h->ws_bytes, h->stream);
+        if (rc) return rc;
+        TRS_CUDA(cudaEventRecord(s.chunk_done[0], h->stream));
+        TRS_CUDA(cudaStreamWaitEvent(h->s_out, s.chunk_done[0], 0));
+        if (timed && i == 0) cudaEventRecord(h->t_ev[4], h->s_out);
+        TRS_CUDA(cudaMemcpy2DAsync((unsigned char*)out_host + d0 * elt, dimN * elt, out, d * elt, d * elt, h->m_rows,
+                                   cudaMemcpyDeviceToHost, h->s_out));
+    }
+    if (timed) {
+        cudaEventRecord(h->t_ev[1], h->s_in);
+        cudaEventRecord(h->t_ev[3], h->stream);
+        cudaEventRecord(h->t_ev[5], h->s_out);
+    }
+    TRS_CUDA(cudaEventRecord(s.k_done, h->stream));
+    TRS_CUDA(cudaEventRecord(s.out_done, h->s_out));
+    ++h->seq;
+    return TRS_OK;
+}
+
+// Enqueue one call on the three streams; returns without waiting.  `timed` records the six
+// timing events of the synchronous entry.
 
 int resident_enqueue(trs_resident* h, const trs_half* rhs_host, void* out_host, int dimN, int out_dtype, bool timed) {
     const int si = (int)(h->seq % kSlots);
@@ -367,6 +437,7 @@ extern "C" int trs_resident_create(const trs_format* host_format, int mOri, int 
     if (trs_device_count() == 0) return TRS_E_NO_DEVICE;
     trs_resident* h = new trs_resident();
     int rc = upload_format(*host_format, h->up, &h->dev);
+    if (!rc) rc = h->up.commit();
     if (!rc) rc = resident_finish_create(h, mOri, kOri, window, max_dimN);
     if (rc) { trs_resident_destroy(h); return rc; }
     *out = h;
@@ -414,7 +485,9 @@ extern "C" int trs_resident_forward(trs_resident* h, const trs_half* rhs_host, v
     int rc = resident_check_args(h, rhs_host, out_host, dimN, out_dtype);
     if (rc) return rc;
     if (timing) memset(timing, 0, sizeof(*timing));
-    rc = resident_enqueue(h, rhs_host, out_host, dimN, out_dtype, timing != nullptr);
+    const int slabs = resident_slabs(dimN, (size_t)h->k_cols * dimN * sizeof(trs_half));
+    rc = slabs > 1 ? resident_enqueue_slabs(h, rhs_host, out_host, dimN, out_dtype, slabs, timing != nullptr)
+                   : resident_enqueue(h, rhs_host, out_host, dimN, out_dtype, timing != nullptr);
     const int drc = resident_drain(h);
     if (!rc) rc = drc;
     if (!rc && h->pending_rc) { rc = h->pending_rc; }
@@ -449,36 +522,42 @@ extern "C" int trs_spmm_forward_host(const trs_format* host_format, const trs_ha
     if (!host_format || !rhs_host || !out_host) return TRS_E_ARG;
     if (dimN <= 0 || mOri <= 0 || kOri <= 0 || epoches <= 0) return TRS_E_ARG;
     if (window <= 0 || window > 16) return TRS_E_WINDOW;
-    trs_resident* h = nullptr;
-    int rc = trs_resident_create(host_format, mOri, kOri, window, dimN, &h);
+    if (trs_device_count() == 0) return TRS_E_NO_DEVICE;
+    // everything in two blocks of the pool (inputs and result; the plan's own), on the thread's stream
+    cudaStream_t st = cudaStreamPerThread;
+    Upload up;
+    up.st = st;
+    trs_format dev;
+    const trs_half* d_rhs = nullptr;
+    float* d_out = nullptr;
+    int rc = upload_format(*host_format, up, &dev);
+    if (!rc) rc = up.put(rhs_host, (size_t)kOri * dimN, &d_rhs);
     if (rc) return rc;
-    trs_timing t1;
-    memset(&t1, 0, sizeof(t1));
-    EventPair ev;
-    rc = ev.init();
-    if (!rc) {
-        cudaError_t e = cudaMemcpyAsync(h->slot[0].d_rhs, rhs_host, (size_t)kOri * dimN * sizeof(trs_half), cudaMemcpyHostToDevice, h->stream);
-        if (e != cudaSuccess) rc = (int)e;
-    }
+    up.raw((size_t)mOri * dimN, &d_out);
+    if ((rc = up.commit())) return rc;
+    struct PlanOwner {
+        trs_spmm_plan* p = nullptr;
+        ~PlanOwner() { trs_spmm_plan_destroy(p); }
+    } plan;
+    if ((rc = trs_spmm_plan_create(&dev, mOri, kOri, window, 1, st, &plan.p))) return rc;
+    size_t ws_bytes = 0;
+    unsigned char* ws = nullptr;
+    if ((rc = trs_spmm_workspace_bytes(plan.p, dimN, &ws_bytes))) return rc;
+    if ((rc = up.now(ws_bytes, &ws))) return rc;
     // one untimed run, then `epoches` timed ones (mGCNkernel_online.cu:1604-1687 warms up and
     // averages over epoches the same way); C is fully rewritten by every run
-    if (!rc) rc = trs_spmm_run(h->plan, h->slot[0].d_rhs, h->slot[0].d_out, dimN, TRS_OUT_F32, h->d_ws, h->ws_bytes, h->stream);
-    if (!rc) {
-        cudaEventRecord(ev.a, h->stream);
-        for (int i = 0; i < epoches && !rc; ++i)
-            rc = trs_spmm_run(h->plan, h->slot[0].d_rhs, h->slot[0].d_out, dimN, TRS_OUT_F32, h->d_ws, h->ws_bytes, h->stream);
-        cudaEventRecord(ev.b, h->stream);
-    }
-    if (!rc) {
-        cudaError_t e = cudaMemcpyAsync(out_host, h->slot[0].d_out, (size_t)mOri * dimN * sizeof(float), cudaMemcpyDeviceToHost, h->stream);
-        if (e == cudaSuccess) e = cudaStreamSynchronize(h->stream);
-        if (e != cudaSuccess) rc = (int)e;
-    }
+    EventPair ev;
+    rc = ev.init();
+    if (!rc) rc = trs_spmm_run(plan.p, d_rhs, d_out, dimN, TRS_OUT_F32, ws, ws_bytes, st);
+    if (!rc) cudaEventRecord(ev.a, st);
+    for (int i = 0; i < epoches && !rc; ++i) rc = trs_spmm_run(plan.p, d_rhs, d_out, dimN, TRS_OUT_F32, ws, ws_bytes, st);
+    if (!rc) cudaEventRecord(ev.b, st);
+    const HostSegment back{out_host, d_out, (size_t)mOri * dimN * sizeof(float)};
+    if (!rc) rc = copy_to_host(&back, 1, st);
     if (!rc && timing) {
         memset(timing, 0, sizeof(*timing));
         timing->total_ms = ev.ms() / (float)epoches;
     }
-    trs_resident_destroy(h);
     return rc;
 }
 
@@ -520,6 +599,7 @@ extern "C" int trs_sptc_unpacked_forward_host(const int32_t* s_column, const flo
     }
     const int tiles = (int)tile_window.size();
     Upload up;
+    up.st = cudaStreamPerThread;
     const int *d_col, *d_off, *d_tw, *d_tg; const float* d_val; const int8_t* d_pos;
     int rc;
     if ((rc = up.put(s_column, (size_t)groups * 4, &d_col))) return rc;
@@ -529,11 +609,12 @@ extern "C" int trs_sptc_unpacked_forward_host(const int32_t* s_column, const flo
     if ((rc = up.put(tile_window.data(), tile_window.size(), &d_tw))) return rc;
     if ((rc = up.put(tile_group.data(), tile_group.size(), &d_tg))) return rc;
     int* d_tcol; uint32_t *d_pa, *d_pm;
-    if ((rc = up.raw<int>((size_t)tiles * 16, &d_tcol))) return rc;
-    if ((rc = up.raw<uint32_t>((size_t)tiles * 64, &d_pa))) return rc;
-    if ((rc = up.raw<uint32_t>((size_t)tiles * 8, &d_pm))) return rc;
-    if ((rc = trs::pack_tiles(d_col, d_val, d_pos, d_off, d_tw, d_tg, tiles, window, d_tcol, d_pa, d_pm, nullptr))) return rc;
-    TRS_CUDA(cudaDeviceSynchronize());
+    up.raw((size_t)tiles * 16, &d_tcol);
+    up.raw((size_t)tiles * 64, &d_pa);
+    up.raw((size_t)tiles * 8, &d_pm);
+    if ((rc = up.commit())) return rc;
+    if ((rc = trs::pack_tiles(d_col, d_val, d_pos, d_off, d_tw, d_tg, tiles, window, d_tcol, d_pa, d_pm, up.st))) return rc;
+    TRS_CUDA(cudaStreamSynchronize(up.st));
     // download the packed tiles and go through the common host path (keeps one code path)
     std::vector<int> h_tcol((size_t)tiles * 16);
     std::vector<uint32_t> h_pa((size_t)tiles * 64), h_pm((size_t)tiles * 8);

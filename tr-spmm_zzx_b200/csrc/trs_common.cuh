@@ -239,6 +239,17 @@ __device__ __forceinline__ void bulk_g2s(uint32_t dst, const void* src, uint32_t
                  : "memory");
 }
 
+// trs_hostcopy.cu: pageable host memory <-> device, ordered after the work on `st`.  copy_to_host returns when
+// the host memory is written, copy_to_device when it has been read (the copies are then queued on `st`).
+struct HostSegment {
+    void* host;
+    void* dev;
+    size_t bytes;
+};
+int copy_to_host(const HostSegment* seg, int n, cudaStream_t st);
+int copy_to_device(const HostSegment* seg, int n, cudaStream_t st);
+void release_host_ring();
+
 // trs_pack.cu
 int pack_tiles(const int* s_column, const float* s_value, const int8_t* s_pos, const int* s_offset,
                const int* tile_window, const int* tile_group, long long tiles, int window, int* s_tile_column,

@@ -702,10 +702,12 @@ using namespace trs;
 struct trs_spmm_plan {
     trs_format f;
     int m_rows, k_cols, window, num_windows;
-    DevBuf<Item> items;               // long ones first
-    DevBuf<Heavy> heavy;
-    DevBuf<int> ids;                  // [steps + kIdBlock][16] column ids of the step stream
-    DevBuf<uint4> dense;              // [dense steps][32] A tiles of the dense steps in fragment order
+    int device = 0;
+    void* block = nullptr;   // the arrays below
+    Item* items = nullptr;   // long ones first
+    Heavy* heavy = nullptr;
+    int* ids = nullptr;      // [steps + kIdBlock][16] column ids of the step stream
+    uint4* dense = nullptr;  // [dense steps][32] A tiles of the dense steps in fragment order
     int n_items, n_heavy, n_slots;
     bool few_items;                   // four warps per item
 };
@@ -715,11 +717,40 @@ static int env_int(const char* name, int dflt) {
     return v ? atoi(v) : dflt;
 }
 
-static int validate_on_device(const trs_format& f, int m_rows, int k_cols, int window, int num_windows,
-                              cudaStream_t st) {
-    int* d_err = nullptr;
-    TRS_CUDA(cudaMalloc(&d_err, sizeof(int)));
-    cudaMemsetAsync(d_err, 0, sizeof(int), st);
+// What the plan reads back while it is made.
+struct PlanInfo {
+    int err;                      // V_* bits
+    int c_entries, cs_entries;    // last prefix entries of the CSR parts
+    int totals[kWindowCounts];
+};
+
+__global__ void k_plan_lasts(trs_format f, PlanInfo* info) {
+    if (f.parts_c > 0) info->c_entries = f.c_row_offset[f.parts_c];
+    if (f.parts_c_short > 0) info->cs_entries = f.cs_row_offset[f.parts_c_short];
+}
+__global__ void k_plan_totals(const int* __restrict__ off, int num_windows, PlanInfo* info) {
+    const size_t stride = (size_t)num_windows + 1;
+    if (threadIdx.x < kWindowCounts) info->totals[threadIdx.x] = off[threadIdx.x * stride + num_windows];
+}
+
+static int verdict(int err) {
+    if (err & V_OFFSETS) return TRS_E_OFFSETS;
+    if (err & V_SHAPE) return TRS_E_SHAPE;
+    if (err & V_COLUMN) return TRS_E_COLUMN;
+    if (err & V_ROW) return TRS_E_ROW;
+    return TRS_OK;
+}
+
+static int read_info(const PlanInfo* dev, PlanInfo* host, cudaStream_t st) {
+    TRS_CUDA(cudaMemcpyAsync(host, dev, sizeof(*host), cudaMemcpyDeviceToHost, st));
+    TRS_CUDA(cudaStreamSynchronize(st));
+    return TRS_OK;
+}
+
+// Queues the checks of the format arrays; the ones that size their reads by prefix entries wait for the verdict
+// on the prefixes.  Bits end up in info->err, which the caller reads with the plan's totals.
+static int validate_on_device(const trs_format& f, int m_rows, int k_cols, int num_windows, PlanInfo* info, cudaStream_t st) {
+    int* d_err = &info->err;
     auto grid = [](long long n) { return (unsigned)((n + 255) / 256); };
     if (f.parts_t > 0) {
         k_check_prefix<<<grid(f.parts_t + 1), 256, 0, st>>>(f.t_row_offset, f.parts_t + 1, f.blocks, d_err);
@@ -737,42 +768,20 @@ static int validate_on_device(const trs_format& f, int m_rows, int k_cols, int w
         k_check_range<<<grid(n), 256, 0, st>>>(row, n, 0, m_rows, V_ROW, d_err);
         k_check_sorted<<<grid(n), 256, 0, st>>>(row, n, d_err);
     }
-    // The checks below size their reads by prefix entries, so the verdict on the prefixes comes first.
-    {
-        int h_pre = 0;
-        cudaError_t e1 = cudaMemcpyAsync(&h_pre, d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
-        if (e1 == cudaSuccess) e1 = cudaStreamSynchronize(st);
-        if (e1 != cudaSuccess) { cudaFree(d_err); return (int)e1; }
-        if (h_pre & V_OFFSETS) { cudaFree(d_err); return TRS_E_OFFSETS; }
-        if (h_pre & V_SHAPE) { cudaFree(d_err); return TRS_E_SHAPE; }
-    }
-    if (f.blocks > 0)
-        k_check_tc_popcount<<<grid(f.blocks), 256, 0, st>>>((const long long*)f.t_binary, f.t_block_offset, f.blocks, d_err);
-    // column ids of the CSR parts: their count is the last prefix entry, which lives on the device
-    for (int pass = 0; pass < 2; ++pass) {
-        const int n = pass ? f.parts_c_short : f.parts_c;
-        if (n <= 0) continue;
-        int last = 0;
-        cudaError_t e2 = cudaMemcpyAsync(&last, (pass ? f.cs_row_offset : f.c_row_offset) + n, sizeof(int), cudaMemcpyDeviceToHost, st);
-        if (e2 == cudaSuccess) e2 = cudaStreamSynchronize(st);
-        if (e2 != cudaSuccess) { cudaFree(d_err); return (int)e2; }
-        if (last > 0)
-            k_check_range<<<grid(last), 256, 0, st>>>(pass ? f.cs_column : f.c_column, last, 0, k_cols, V_COLUMN, d_err);
-    }
     if (f.num_windows > 0) {
         k_check_prefix<<<grid(f.num_windows + 1), 256, 0, st>>>(f.s_window_tile_offset, f.num_windows + 1, f.tiles, d_err);
         if (f.tiles > 0)
             k_check_range<<<grid((long long)f.tiles * 16), 256, 0, st>>>(f.s_tile_column, (long long)f.tiles * 16, -1, k_cols, V_COLUMN, d_err);
     }
-    int h_err = 0;
-    cudaError_t e = cudaMemcpyAsync(&h_err, d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
-    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
-    cudaFree(d_err);
-    if (e != cudaSuccess) return (int)e;
-    if (h_err & V_OFFSETS) return TRS_E_OFFSETS;
-    if (h_err & V_SHAPE) return TRS_E_SHAPE;
-    if (h_err & V_COLUMN) return TRS_E_COLUMN;
-    if (h_err & V_ROW) return TRS_E_ROW;
+    k_plan_lasts<<<1, 1, 0, st>>>(f, info);
+    PlanInfo h;
+    const int rc = read_info(info, &h, st);
+    if (rc) return rc;
+    if (h.err & (V_OFFSETS | V_SHAPE)) return verdict(h.err);
+    if (f.blocks > 0)
+        k_check_tc_popcount<<<grid(f.blocks), 256, 0, st>>>((const long long*)f.t_binary, f.t_block_offset, f.blocks, d_err);
+    if (h.c_entries > 0) k_check_range<<<grid(h.c_entries), 256, 0, st>>>(f.c_column, h.c_entries, 0, k_cols, V_COLUMN, d_err);
+    if (h.cs_entries > 0) k_check_range<<<grid(h.cs_entries), 256, 0, st>>>(f.cs_column, h.cs_entries, 0, k_cols, V_COLUMN, d_err);
     return TRS_OK;
 }
 
@@ -801,28 +810,28 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
 
     cudaStream_t st = (cudaStream_t)stream;
     const int W = max(ceil_div(m_rows, window), f.num_windows);
-    if (validate) {
-        int rc = validate_on_device(f, m_rows, k_cols, window, W, st);
-        if (rc != TRS_OK) return rc;
-    }
+    TempSpace ts;
+    ts.st = st;
+    const size_t stride = (size_t)W + 1;
+    ts.chunk_bytes = ((size_t)6 + 2 * kWindowCounts) * stride * sizeof(int) + ((size_t)1 << 20);
+    PlanInfo* d_info;
+    int *ranges, *cnt, *off;
+    int rc = ts.get(1, &d_info);
+    if (!rc) rc = ts.get((size_t)6 * W, &ranges);
+    if (!rc) rc = ts.get(kWindowCounts * stride, &cnt);
+    if (!rc) rc = ts.get(kWindowCounts * stride, &off);
+    if (rc) return rc;
+    TRS_CUDA(cudaMemsetAsync(d_info, 0, sizeof(PlanInfo), st));
+    if (validate && (rc = validate_on_device(f, m_rows, k_cols, W, d_info, st))) return rc;
 
-    trs_spmm_plan* p = new trs_spmm_plan();
-    p->f = f;
-    p->m_rows = m_rows; p->k_cols = k_cols; p->window = window; p->num_windows = W;
     const int forced_chunk = env_int("TRS_CHUNK_STEPS", 0);
     const int chunk = forced_chunk > 0 ? max(8, forced_chunk) : 0;
     int dev = 0, sms = 0;
-    cudaGetDevice(&dev);
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-    sms = max(sms, 1);
-    // per-window ranges of TC blocks and CSR parts (needed only while the items are made)
-    DevBuf<int> ranges, cnt, off;
-    DevBuf<unsigned char> tmp;
-    auto fail = [&](int code) { ranges.release(); cnt.release(); off.release(); tmp.release(); trs_spmm_plan_destroy(p); return code; };
-    int rc = ranges.alloc((size_t)6 * W);
-    if (rc) return fail(rc);
-    cudaMemsetAsync(ranges.p, 0, sizeof(int) * (size_t)6 * W, st);
-    WindowRanges wr{ranges.p, ranges.p + W, ranges.p + 2 * W, ranges.p + 3 * W, ranges.p + 4 * W, ranges.p + 5 * W};
+    TRS_CUDA(cudaGetDevice(&dev));
+    TRS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+    // per-window ranges of TC blocks and CSR parts
+    TRS_CUDA(cudaMemsetAsync(ranges, 0, sizeof(int) * (size_t)6 * W, st));
+    WindowRanges wr{ranges, ranges + W, ranges + 2 * W, ranges + 3 * W, ranges + 4 * W, ranges + 5 * W};
     auto grid = [](long long n) { return (unsigned)((n + 255) / 256); };
     if (f.parts_t > 0)
         k_part_ranges<<<grid(f.parts_t), 256, 0, st>>>(f.t_window_row, f.t_row_offset, f.parts_t, 16, W,
@@ -833,54 +842,62 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
         k_part_ranges<<<grid(f.parts_c_short), 256, 0, st>>>(f.cs_row, nullptr, f.parts_c_short, window, W,
                                                               wr.cs_begin, wr.cs_end, 0);
     // counts -> exclusive scans (kWindowCounts arrays of W + 1)
-    const size_t stride = (size_t)W + 1;
-    rc = cnt.alloc(kWindowCounts * stride);
-    if (!rc) rc = off.alloc(kWindowCounts * stride);
     size_t tmp_bytes = 0;
-    cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, cnt.p, off.p, W + 1, st);
-    if (!rc) rc = tmp.alloc(tmp_bytes + 16);
-    if (rc) return fail(rc);
-    auto scan = [&](int i) {
-        cub::DeviceScan::ExclusiveSum(tmp.p, tmp_bytes, cnt.p + i * stride, off.p + i * stride, W + 1, st);
-    };
-    k_count_steps<<<grid(W + 1), 256, 0, st>>>(f, wr, W, cnt.p);
-    scan(WC_STEPS); scan(WC_DENSE);
-    k_count_items<<<grid(W + 1), 256, 0, st>>>(W, chunk, sms, off.p + WC_STEPS * stride, cnt.p);
-    scan(WC_ITEMS); scan(WC_HEAVY); scan(WC_SLOTS);
-    int totals[kWindowCounts] = {};
-    for (int i = 0; i < kWindowCounts; ++i)
-        cudaMemcpyAsync(&totals[i], off.p + i * stride + W, sizeof(int), cudaMemcpyDeviceToHost, st);
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return fail((int)e);
-    p->n_items = totals[WC_ITEMS]; p->n_heavy = totals[WC_HEAVY]; p->n_slots = totals[WC_SLOTS];
-    const int n_steps = totals[WC_STEPS], n_dense = totals[WC_DENSE];
-    if (n_steps < 0 || n_dense < 0) return fail(TRS_E_OFFSETS);
+    unsigned char* tmp;
+    TRS_CUDA(cub::DeviceScan::ExclusiveSum(nullptr, tmp_bytes, cnt, off, W + 1, st));
+    if ((rc = ts.get(tmp_bytes + 16, &tmp))) return rc;
+    auto scan = [&](int i) { return cub::DeviceScan::ExclusiveSum(tmp, tmp_bytes, cnt + i * stride, off + i * stride, W + 1, st); };
+    k_count_steps<<<grid(W + 1), 256, 0, st>>>(f, wr, W, cnt);
+    TRS_CUDA(scan(WC_STEPS));
+    TRS_CUDA(scan(WC_DENSE));
+    k_count_items<<<grid(W + 1), 256, 0, st>>>(W, chunk, sms, off + WC_STEPS * stride, cnt);
+    TRS_CUDA(scan(WC_ITEMS));
+    TRS_CUDA(scan(WC_HEAVY));
+    TRS_CUDA(scan(WC_SLOTS));
+    k_plan_totals<<<1, 32, 0, st>>>(off, W, d_info);
+    PlanInfo info;
+    if ((rc = read_info(d_info, &info, st))) return rc;
+    if ((rc = verdict(info.err))) return rc;
+    const int n_items = info.totals[WC_ITEMS], n_heavy = info.totals[WC_HEAVY];
+    const int n_steps = info.totals[WC_STEPS], n_dense = info.totals[WC_DENSE];
+    if (n_steps < 0 || n_dense < 0 || n_items < 0) return TRS_E_OFFSETS;
+
+    // the plan's own memory, one block
+    trs_spmm_plan* p = new trs_spmm_plan();
+    p->f = f;
+    p->m_rows = m_rows; p->k_cols = k_cols; p->window = window; p->num_windows = W; p->device = dev;
+    p->n_items = n_items; p->n_heavy = n_heavy; p->n_slots = info.totals[WC_SLOTS];
     p->few_items = n_steps / (sms * kWarpsPerSm) < kFewSteps;
-    DevBuf<Item> by_window;   // items in window order, sorted into p->items
-    DevBuf<unsigned char> cls, sort_tmp;
-    auto fail2 = [&](int code) { by_window.release(); cls.release(); sort_tmp.release(); return fail(code); };
-    rc = p->items.alloc(p->n_items);
-    if (!rc) rc = by_window.alloc(p->n_items);
-    if (!rc) rc = cls.alloc((size_t)2 * p->n_items);
-    if (!rc) rc = p->heavy.alloc(p->n_heavy);
-    if (!rc) rc = p->ids.alloc(((size_t)n_steps + kIdBlock) * 16);
-    if (!rc) rc = p->dense.alloc((size_t)n_dense * 32);
+    const size_t ids_bytes = ((size_t)n_steps + kIdBlock) * 64, dense_bytes = (size_t)n_dense * 512;
+    const size_t items_bytes = (size_t)n_items * sizeof(Item), heavy_bytes = (size_t)n_heavy * sizeof(Heavy);
+    auto fail = [&](int code) { trs_spmm_plan_destroy(p); return code; };
+    if ((rc = pool_alloc(&p->block, ids_bytes + dense_bytes + items_bytes + heavy_bytes, st))) return fail(rc);
+    unsigned char* at = (unsigned char*)p->block;
+    p->ids = (int*)at; at += ids_bytes;
+    p->dense = (uint4*)at; at += dense_bytes;
+    p->items = (Item*)at; at += items_bytes;
+    p->heavy = (Heavy*)at;
+
+    Item* by_window;   // items in window order, sorted into p->items
+    unsigned char *cls, *sort_tmp;
     size_t sort_bytes = 0;
-    cub::DeviceRadixSort::SortPairs(nullptr, sort_bytes, cls.p, cls.p, by_window.p, p->items.p, p->n_items, 0, kClassBits, st);
-    if (!rc) rc = sort_tmp.alloc(sort_bytes + 16);
-    if (rc) return fail2(rc);
-    k_fill_items<<<grid(W), 256, 0, st>>>(f, wr, W, off.p, by_window.p, p->heavy.p);
-    k_fill_steps<<<grid((long long)p->n_items * 32), 256, 0, st>>>(f, wr, by_window.p, p->n_items, off.p, W, window,
-                                                                   p->ids.p, p->dense.p);
-    k_item_class<<<grid(p->n_items), 256, 0, st>>>(by_window.p, p->n_items, cls.p);
-    e = cub::DeviceRadixSort::SortPairs(sort_tmp.p, sort_bytes, cls.p, cls.p + p->n_items, by_window.p, p->items.p, p->n_items,
-                                        0, kClassBits, st);
-    if (e != cudaSuccess) return fail2((int)e);
-    e = cudaStreamSynchronize(st);
+    rc = ts.get(n_items, &by_window);
+    if (!rc) rc = ts.get((size_t)2 * n_items, &cls);
+    if (rc) return fail(rc);
+    auto sort = [&](void* t) {
+        return cub::DeviceRadixSort::SortPairs(t, sort_bytes, cls, cls + n_items, by_window, p->items, n_items, 0, kClassBits, st);
+    };
+    cudaError_t e = sort(nullptr);
+    if (e == cudaSuccess && (rc = ts.get(sort_bytes + 16, &sort_tmp))) return fail(rc);
+    if (e == cudaSuccess) {
+        k_fill_items<<<grid(W), 256, 0, st>>>(f, wr, W, off, by_window, p->heavy);
+        k_fill_steps<<<grid((long long)n_items * 32), 256, 0, st>>>(f, wr, by_window, n_items, off, W, window, p->ids, p->dense);
+        k_item_class<<<grid(n_items), 256, 0, st>>>(by_window, n_items, cls);
+        e = sort(sort_tmp);
+    }
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaGetLastError();
-    if (e != cudaSuccess) return fail2((int)e);
-    by_window.release(); cls.release(); sort_tmp.release();
-    ranges.release(); cnt.release(); off.release(); tmp.release();
+    if (e != cudaSuccess) return fail((int)e);
     *out_plan = p;
     return TRS_OK;
 }
@@ -896,10 +913,15 @@ extern "C" int trs_spmm_status(const trs_spmm_plan* p, int* status) {
 
 extern "C" int trs_spmm_plan_destroy(trs_spmm_plan* p) {
     if (!p) return TRS_OK;
-    p->items.release();
-    p->heavy.release();
-    p->ids.release();
-    p->dense.release();
+    if (p->block) {
+        // kernels on any stream may still read the plan: wait as cudaFree would
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev != p->device) cudaSetDevice(p->device);
+        cudaDeviceSynchronize();
+        pool_free(p->block, nullptr);
+        if (dev != p->device) cudaSetDevice(dev);
+    }
     delete p;
     return TRS_OK;
 }
@@ -1026,9 +1048,9 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
     if (need > 0 && (!workspace || workspace_bytes < need)) return TRS_E_WORKSPACE;
     cudaStream_t st = (cudaStream_t)stream;
     KernelArgs a;
-    a.items = p->items.p; a.n_items = p->n_items;
+    a.items = p->items; a.n_items = p->n_items;
     a.w_begin = w0; a.w_end = w1;
-    a.ids = p->ids.p; a.dense = p->dense.p;
+    a.ids = p->ids; a.dense = p->dense;
     a.packed_a = p->f.s_packed_a; a.packed_meta = p->f.s_packed_meta;
     a.B = (const __half*)B; a.C = C; a.scratch = (float*)workspace;
     a.ldb = F; a.ldS = scratch_ld(F); a.F = F; a.bchunks = ceil_div(F, 8);
@@ -1060,7 +1082,7 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
         pd.n = a.n_peers; pd.row0 = a.peer_row0;
         for (int d = 0; d < 8; ++d) pd.ptr[d] = a.peers[d];
         const dim3 rgrid(p->n_heavy, ceil_div(16 * a.ldS / 4, 128));
-        k_reduce_heavy<<<rgrid, 128, 0, st>>>(p->heavy.p, (const float*)workspace, C, F, a.ldS, p->m_rows, p->window,
+        k_reduce_heavy<<<rgrid, 128, 0, st>>>(p->heavy, (const float*)workspace, C, F, a.ldS, p->m_rows, p->window,
                                               a.out_half, a.relu, w0, w1, pd);
         TRS_LAUNCH_CHECK();
     }

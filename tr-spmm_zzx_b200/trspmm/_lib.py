@@ -114,6 +114,10 @@ def load():
     for name in ("trs_sddmm_plan_create", "trs_sddmm_plan_run", "trs_sddmm_plan_info", "trs_sddmm_plan_destroy"):
         getattr(lib, name).restype = i32
     lib.trs_build_create.argtypes = [vp, vp, vp, i32, C.POINTER(TrsBuildConfig), vp, C.POINTER(vp)]
+    lib.trs_copy_to_host.argtypes = [i32, C.POINTER(vp), C.POINTER(vp), C.POINTER(sz), vp]
+    lib.trs_copy_to_host.restype = i32
+    lib.trs_copy_to_device.argtypes = [i32, C.POINTER(vp), C.POINTER(vp), C.POINTER(sz), vp]
+    lib.trs_copy_to_device.restype = i32
     lib.trs_pool_trim.argtypes = []
     lib.trs_pool_trim.restype = i32
     lib.trs_build_create_into.argtypes = [vp, vp, vp, i32, C.POINTER(TrsBuildConfig), BuildAlloc, vp, vp, C.POINTER(vp)]
@@ -145,6 +149,31 @@ def load():
 def check(code: int):
     if code != 0:
         raise TrsError(code, load().trs_strerror(code).decode())
+
+
+def _copy(entry, host, dev, device):
+    n = len(host)
+    check(entry(n, (C.c_void_p * n)(*[t.data_ptr() for t in host]), (C.c_void_p * n)(*[t.data_ptr() for t in dev]),
+                (C.c_size_t * n)(*[t.numel() * t.element_size() for t in host]), current_stream_ptr(device)))
+
+
+def copy_to_host(tensors, device):
+    """CPU copies of contiguous CUDA tensors of one device (trs_copy_to_host): all of them in one go, after the work on the
+    current stream."""
+    import torch
+    out = [torch.empty(t.shape, dtype=t.dtype) for t in tensors]
+    with torch.cuda.device(device):
+        _copy(load().trs_copy_to_host, out, tensors, device)
+    return out
+
+
+def copy_to_device(tensors, device):
+    """Copies of contiguous CPU tensors on `device` (trs_copy_to_device), ordered on the current stream."""
+    import torch
+    out = [torch.empty(t.shape, dtype=t.dtype, device=device) for t in tensors]
+    with torch.cuda.device(device):
+        _copy(load().trs_copy_to_device, tensors, out, device)
+    return out
 
 
 def current_stream_ptr(device) -> int:
