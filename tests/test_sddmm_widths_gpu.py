@@ -1,0 +1,36 @@
+"""SDDMM at widths around the kernels' 32-feature chunks (planned: up to 256 in registers; entry-parallel beyond), rows
+off 16-byte boundaries, and patterns with long runs of empty rows."""
+import pytest
+import torch
+
+from oracle import oracle as O
+from trspmm import SddmmPlan, graphs, sddmm
+
+pytestmark = pytest.mark.gpu
+
+
+def _pattern(kind):
+    if kind == "rmat":
+        return graphs.rmat_graph(10, 12, seed=4)[:2]
+    g = torch.Generator().manual_seed(6)                       # 5000 rows, a few of them with entries
+    rows = torch.randint(0, 40, (3000,), generator=g) * 123
+    return graphs.coo_to_csr(rows, torch.randint(0, 700, (3000,), generator=g), 5000, 700)[:2]
+
+
+@pytest.mark.parametrize("kind", ["rmat", "gaps"])
+@pytest.mark.parametrize("K", [1, 8, 31, 32, 33, 48, 72, 96, 100, 127, 128, 136, 160, 192, 200, 224, 256, 264, 300])
+def test_widths(kind, K):
+    rp, col = _pattern(kind)
+    n, m = rp.numel() - 1, 1024 if kind == "rmat" else 700
+    g = torch.Generator().manual_seed(K)
+    X, Y = torch.randn(n, K, generator=g).half(), torch.randn(m, K, generator=g).half()
+    ref = O.sddmm_csr(rp, col, X, Y).float()
+    scale = float(ref.abs().max())
+    rp, col, X, Y = rp.cuda(), col.cuda(), X.cuda(), Y.cuda()
+    plan = SddmmPlan(rp, col, m)
+    for run in (lambda out: sddmm(rp, col, X, Y, out=out), lambda out: plan.run(X, Y, out=out)):
+        out = run(torch.full((col.numel(),), float("nan"), dtype=torch.float16, device="cuda")).float().cpu()
+        assert float((out - ref).abs().max()) <= 2e-3 * scale
+    base = torch.empty(n * K + 8, dtype=torch.float16, device="cuda")   # X one element off its boundary
+    Xo = base[1:1 + n * K].view(n, K).copy_(X)
+    assert torch.equal(plan.run(Xo, Y), plan.run(X, Y)) and torch.equal(sddmm(rp, col, Xo, Y), sddmm(rp, col, X, Y))

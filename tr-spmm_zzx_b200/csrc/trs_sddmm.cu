@@ -3,153 +3,155 @@
 // The reference has no SDDMM operator; the definition is fixed by the benchmark
 // configuration (X, Y dense fp16, fp32 accumulate, fp16 result in CSR order).
 //
-// Work is split by ENTRY, not by row, so power-law rows cost nothing extra: a warp takes a run
-// of consecutive entries, an 8-lane group takes one entry at a time and reads the 128-byte
-// slices of X[row] and Y[col] with one 16-byte load per lane, multiplies in fp32 and reduces
-// with three shuffles.  The row of an entry is found once per warp by binary search in the row
-// pointers and then advanced linearly.
+// Both kernels below contract on the tensor cores (mma m16n8k16, fp32 accumulate) over the feature
+// dimension, which is contiguous in both operands, so fragments are filled by plain 16-byte pieces:
+// lane (g, t) takes bytes [64 c + 16 t, +16) of its row for every 32-feature chunk c - the same feature
+// positions on both sides, which is all the MMA needs (the order of k inside a chunk is free).
+// Rows that do not start on 16-byte boundaries are copied to padded ones first.
 #include <stdlib.h>
 #include <string.h>
 
 #include <cub/cub.cuh>
 
+#include <algorithm>
+#include <atomic>
+#include <mutex>
+#include <vector>
+
 #include "trs_common.cuh"
 
 namespace trs {
 
-constexpr int kEntriesPerWarp = 512;
+// ----------------------------------------------------------------------------------------------
+// Entry-parallel SDDMM (patterns used once)
+// ----------------------------------------------------------------------------------------------
+// Work is split by ENTRY, not by row, so power-law rows cost nothing extra.  Eight consecutive entries, of
+// whatever rows, are one MMA: row g of A is the X row of entry g, column g of B its Y row, and the
+// diagonal of the product is the result (lane 4 g + g / 2 holds it).  That wastes the other products but replaces
+// conversions, FMAs and shuffles, which were 19 warp instructions per entry at K = 64, by 2 loads and 2 MMAs per
+// 32 features and 8 entries; what is left is the gather of one Y row per entry through L2.
+// Uniform 50 021 rows x 17 entries, K = 96: 112 -> 24 us.
+//
+// Inputs are not validated by a pass of their own on this entry (trs_sddmm_plan_create does that for
+// planned patterns), so the kernel bounds what it dereferences: rows stop at the last one, and an
+// entry whose column lies outside [0, n_cols) reads row 0 of Y and is written as NaN.
+constexpr int kEntryWarps = 8, kEntryCtas = 5;   // warps per CTA, CTAs per SM
 
-__device__ __forceinline__ float dot8(const uint4& x, const uint4& y) {
-    const __half2* xh = reinterpret_cast<const __half2*>(&x);
-    const __half2* yh = reinterpret_cast<const __half2*>(&y);
-    float s = 0.f;
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const float2 a = __half22float2(xh[i]);
-        const float2 b = __half22float2(yh[i]);
-        s = fmaf(a.x, b.x, s);
-        s = fmaf(a.y, b.y, s);
+// Largest r in [0, n) with a[r] <= x (a ascending, a[0] <= x), by the whole warp: 32 probes per round.
+__device__ __forceinline__ int warp_find(const int* __restrict__ a, int n, int x, int lane) {
+    int lo = 0, len = n;   // the answer is in [lo, lo + len)
+    while (len > 1) {
+        const int step = (len + 31) / 32;
+        const int at = lo + lane * step;
+        const unsigned le = __ballot_sync(0xffffffffu, lane * step < len && a[at] <= x);
+        const int k = 31 - __clz(le | 1u);
+        lo += k * step;
+        len = min(step, len - k * step);
     }
-    return s;
+    return lo;
 }
 
-constexpr int kUnroll = 8;  // entries in flight per 8-lane group
-
-template <bool VEC>
-__global__ void __launch_bounds__(256) k_sddmm(const int* __restrict__ rowptr, const int* __restrict__ col,
-                                               const __half* __restrict__ X, const __half* __restrict__ Y,
-                                               __half* __restrict__ out, int n_rows, int n_cols, long long nnz, int K) {
-    // Inputs are not validated by a pass of their own on this entry (trs_sddmm_plan_create does
-    // that for planned patterns), so the kernel bounds what it dereferences: the row walk stops at
-    // the last row, and an entry whose column lies outside [0, n_cols) reads row 0 of Y and is
-    // written as NaN instead of gathering out of range.
-    const int lane = threadIdx.x & 31;
-    const int sub = lane >> 3, sl = lane & 7;
-    const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
-    const long long e0 = warp * kEntriesPerWarp;
-    if (e0 >= nnz) return;
-    const long long e1 = min(e0 + (long long)kEntriesPerWarp, nnz);
-    // row containing e0: largest r with rowptr[r] <= e0
-    int lo = 0, hi = n_rows;
-    while (hi - lo > 1) {
-        const int mid = (lo + hi) >> 1;
-        if ((long long)rowptr[mid] <= e0) lo = mid; else hi = mid;
-    }
-    int row = lo;
-    if (VEC && K == 64) {
-        // fast path: one 16-byte slice of X[row] and Y[col] per lane.  The Y slices of kUnroll
-        // entries are requested before any is consumed, so an 8-lane group keeps kUnroll random
-        // 128-byte rows in flight; X[row] changes rarely and is (re)read at use (an L1 hit).
-        int xrow = -1;
-        uint4 xv = make_uint4(0, 0, 0, 0);
-        for (long long eb = e0; eb < e1; eb += 4 * kUnroll) {
-            uint4 yv[kUnroll];
-            int rows[kUnroll];
-            unsigned bad = 0;
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-                const long long e = eb + sub + 4 * u;
-                rows[u] = -1;
-                yv[u] = make_uint4(0, 0, 0, 0);
-                if (e < e1) {
-                    while (row + 1 < n_rows && (long long)rowptr[row + 1] <= e) ++row;
-                    rows[u] = row;
-                    int c = col[e];
-                    if ((unsigned)c >= (unsigned)n_cols) { c = 0; bad |= 1u << u; }
-                    yv[u] = __ldg(reinterpret_cast<const uint4*>(Y + (size_t)c * 64) + sl);
-                }
-            }
-#pragma unroll
-            for (int u = 0; u < kUnroll; ++u) {
-                if (rows[u] >= 0 && rows[u] != xrow) {
-                    xrow = rows[u];
-                    xv = __ldg(reinterpret_cast<const uint4*>(X + (size_t)xrow * 64) + sl);
-                }
-                float s = dot8(xv, yv[u]);
-                s += __shfl_xor_sync(0xffffffffu, s, 1);
-                s += __shfl_xor_sync(0xffffffffu, s, 2);
-                s += __shfl_xor_sync(0xffffffffu, s, 4);
-                if (rows[u] >= 0 && sl == 0) out[eb + sub + 4 * u] = (bad >> u) & 1u ? __ushort_as_half((unsigned short)0x7e00) : __float2half_rn(s);
-            }
-        }
-        return;
-    }
-    for (long long eb = e0; eb < e1; eb += 4) {
-        const long long e = eb + sub;
-        const bool live = e < e1;
-        float s = 0.f;
-        bool bad = false;
-        if (live) {
-            while (row + 1 < n_rows && (long long)rowptr[row + 1] <= e) ++row;
+template <int KCH>   // 32-feature chunks per pass (K > 32 KCH loops)
+__global__ void __launch_bounds__(32 * kEntryWarps, kEntryCtas) k_sddmm(const int* __restrict__ rowptr, const int* __restrict__ col,
+                                                            const __half* __restrict__ X, const __half* __restrict__ Y,
+                                                            __half* __restrict__ out, int n_rows, int n_cols, int K, int ld) {
+    const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+    const int nnz = rowptr[0] == 0 ? rowptr[n_rows] : 0;   // anything else is an error the caller reports
+    const int pieces = (K + 7) / 8, ld16 = ld / 8;
+    // a warp's share of the entries, in chunks of 32 to 256
+    const int per_warp = min(max((nnz / (int)(gridDim.x * kEntryWarps) + 31) & ~31, 32), 256);
+    for (long long warp = (long long)blockIdx.x * kEntryWarps + (threadIdx.x >> 5);; warp += (long long)gridDim.x * kEntryWarps) {
+        const long long first = warp * per_warp;
+        if (first >= nnz) return;
+        const int e_end = (int)min(first + per_warp, (long long)nnz);
+        int row = warp_find(rowptr, n_rows, (int)first, lane);   // row of the chunk's first entry
+        for (int e0 = (int)first; e0 < e_end; e0 += 32) {
+            // columns and rows of 32 entries, one per lane
+            const int e = min(e0 + lane, e_end - 1);
+            const int bound = row + 1 + lane < n_rows ? rowptr[row + 1 + lane] : 0x7fffffff;
             int c = col[e];
-            if ((unsigned)c >= (unsigned)n_cols) { c = 0; bad = true; }
-            const __half* xr = X + (size_t)row * K;
-            const __half* yr = Y + (size_t)c * K;
-            if (VEC) {
-                for (int k = sl * 8; k < K; k += 64) {
-                    const uint4 xv = __ldg(reinterpret_cast<const uint4*>(xr + k));
-                    const uint4 yv = __ldg(reinterpret_cast<const uint4*>(yr + k));
-                    s += dot8(xv, yv);
+            const bool bad = (unsigned)c >= (unsigned)n_cols;
+            if (bad) c = 0;
+            int r = 0;   // how many of the next 32 rows start at or before e
+#pragma unroll
+            for (int s = 16; s; s >>= 1)
+                if (__shfl_sync(0xffffffffu, bound, r + s - 1) <= e) r += s;
+            r += __shfl_sync(0xffffffffu, bound, 31) <= e ? 1 : 0;
+            r += row;
+            if (__any_sync(0xffffffffu, r - row > 31)) {   // many empty rows in between
+                int lo = 0, hi = n_rows;
+                while (hi - lo > 1) {
+                    const int mid = (lo + hi) >> 1;
+                    if (rowptr[mid] <= e) lo = mid; else hi = mid;
                 }
-            } else {
-                for (int k = sl; k < K; k += 8) s = fmaf(__half2float(xr[k]), __half2float(yr[k]), s);
+                r = lo;
+            }
+            row = __shfl_sync(0xffffffffu, r, 31);
+            const unsigned bad_mask = __ballot_sync(0xffffffffu, bad);
+#pragma unroll
+            for (int b = 0; b < 4; ++b) {
+                if (e0 + 8 * b >= e_end) break;
+                const uint4* x = (const uint4*)X + (size_t)__shfl_sync(0xffffffffu, r, 8 * b + g) * ld16 + t;
+                const uint4* y = (const uint4*)Y + (size_t)__shfl_sync(0xffffffffu, c, 8 * b + g) * ld16 + t;
+                float d[4] = {0.f, 0.f, 0.f, 0.f};
+                for (int p0 = 0; p0 < pieces; p0 += 4 * KCH) {
+                    uint4 xv[KCH], yv[KCH];
+#pragma unroll
+                    for (int ch = 0; ch < KCH; ++ch) {
+                        const bool in = p0 + 4 * ch + t < pieces;
+                        xv[ch] = in ? __ldg(x + p0 + 4 * ch) : make_uint4(0, 0, 0, 0);
+                        yv[ch] = in ? __ldg(y + p0 + 4 * ch) : make_uint4(0, 0, 0, 0);
+                    }
+#pragma unroll
+                    for (int ch = 0; ch < KCH; ++ch) {
+                        mma_16816(d, xv[ch].x, 0u, xv[ch].y, 0u, yv[ch].x, yv[ch].y);
+                        mma_16816(d, xv[ch].z, 0u, xv[ch].w, 0u, yv[ch].z, yv[ch].w);
+                    }
+                }
+                const int i = 8 * b + g;
+                if (t == (g >> 1) && e0 + i < e_end) {
+                    const float v = (g & 1) ? d[1] : d[0];
+                    out[e0 + i] = (bad_mask >> i) & 1u ? __ushort_as_half((unsigned short)0x7e00) : __float2half_rn(v);
+                }
             }
         }
-        s += __shfl_xor_sync(0xffffffffu, s, 1);
-        s += __shfl_xor_sync(0xffffffffu, s, 2);
-        s += __shfl_xor_sync(0xffffffffu, s, 4);
-        if (live && sl == 0) out[e] = bad ? __ushort_as_half((unsigned short)0x7e00) : __float2half_rn(s);
     }
+}
+
+// Rows of `K` halfs copied to rows of `ld` halfs (a multiple of 8, zero-filled): one thread per 16 bytes.
+__global__ void k_sddmm_pad(const __half* __restrict__ src, long long pieces, int K, int per_row, __half* __restrict__ dst) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= pieces) return;
+    const long long r = i / per_row;
+    const int k = (int)(i - r * per_row) * 8;
+    const unsigned short* s = (const unsigned short*)src + r * K + k;
+    unsigned short v[8];
+#pragma unroll
+    for (int j = 0; j < 8; ++j) v[j] = k + j < K ? s[j] : (unsigned short)0;
+    ((uint4*)dst)[i] = make_uint4(v[0] | (uint32_t)v[1] << 16, v[2] | (uint32_t)v[3] << 16, v[4] | (uint32_t)v[5] << 16,
+                                  v[6] | (uint32_t)v[7] << 16);
+}
+
+__global__ void k_sddmm_ends(const int* __restrict__ rowptr, int n_rows, int* __restrict__ ends) {
+    ends[0] = rowptr[0];
+    ends[1] = rowptr[n_rows];
 }
 
 // ----------------------------------------------------------------------------------------------
 // Planned, tensor-core SDDMM
 // ----------------------------------------------------------------------------------------------
-// The entry-parallel kernel above gathers one Y row per ENTRY and spends ~19 warp instructions
-// per entry on conversions, FMAs and shuffles.  With a plan over the pattern the work is done per
-// (16-row window, column) PAIR instead: the distinct columns of a window, ascending, are cut into
-// blocks of 8; for a block one warp multiplies the window's X tile (16 x K) with the 8 gathered
-// Y rows on the tensor cores (mma m16n8k16, fp32 accumulate) and stores only the dot products
-// the pattern has.  The contraction runs over the feature dimension, which is contiguous in
-// both operands, so the fragments are filled by plain 16-byte loads: lane (g, t) reads bytes
-// [64 c + 16 t, +16) of X[row g], X[row g + 8] and Y[col g] for every 32-feature chunk c — the
-// same feature positions on both sides, which is all the MMA needs (the order of the k index
-// inside a chunk is free).
-//
-// Block record (128 bytes, one cache line): 8 column ids (-1 = unused slot), a 16 x 8 bitmap of
-// the entries present (bit 8 r + n), the window id, and for each of the 16 rows the CSR index of
-// its first entry inside the block.  Columns ascend inside a CSR row and a block holds a
-// contiguous run of the window's sorted distinct columns, so the entries of a row inside a block
-// are consecutive in CSR order: entry (r, n) = start[r] + popcount(rowbits(r) below bit n).
+// With a plan over the pattern the work is done per (16-row window, column) PAIR: the distinct columns of a window,
+// ascending, are cut into quads of 32 (four MMA blocks of 8).  A quad has a header, 32 column ids (unused slots of its last
+// block repeat the first column) and the list of its entries in CSR order: (CSR index - first one of the window) << 9 |
+// row << 5 | column.  That holds windows of up to 2^23 entries; a pattern with a larger one runs the entry-parallel kernel.
 // The pattern must be canonical CSR (columns ascending and unique per row).
-struct SddmmBlock {
-    int col[8];
-    unsigned bits[4];
+constexpr int kPosBits = 9;   // row (4) and column (5) of an entry inside its quad
+struct __align__(16) SddmmQuad {
     int window;
-    int pad[3];
-    int start[16];
+    int first;           // CSR index of the window's first entry
+    int entries_blocks;  // entries << 3 | blocks of 8 columns in use
+    int list;            // first entry in the list
 };
-static_assert(sizeof(SddmmBlock) == 128, "one cache line per block");
 
 __device__ __forceinline__ int row_of_entry(const int* __restrict__ rowptr, int n_rows, long long e) {
     int lo = 0, hi = n_rows;  // largest r with rowptr[r] <= e
@@ -184,7 +186,7 @@ __global__ void ksp_heads(const unsigned long long* __restrict__ key, long long 
 // first_pair[w] = number of distinct (window, column) pairs in windows < w, for w in [0, W]
 __global__ void ksp_window_pairs(const unsigned long long* __restrict__ key, const int* __restrict__ pair_idx,
                                  long long nnz, int total_pairs, int W, int* __restrict__ first_pair,
-                                 int* __restrict__ blocks_of) {
+                                 int* __restrict__ quads_of, int* __restrict__ n_blocks) {
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (w > W) return;
     auto lower = [&](int win) -> int {  // pairs before the first sorted entry of window >= win
@@ -197,168 +199,239 @@ __global__ void ksp_window_pairs(const unsigned long long* __restrict__ key, con
     };
     const int mine = lower(w);
     first_pair[w] = mine;
-    if (w < W) blocks_of[w] = (lower(w + 1) - mine + 7) >> 3;
-}
-
-__global__ void ksp_init_blocks(SddmmBlock* __restrict__ blk, long long n) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;  // one int of a record per thread
-    if (i >= n * 32) return;
-    const int f = (int)(i & 31);
-    int v = 0;
-    if (f < 8) v = -1;
-    else if (f >= 16) v = 0x7fffffff;
-    ((int*)blk)[i] = v;
-}
-
-__global__ void ksp_fill(const unsigned long long* __restrict__ key, const int* __restrict__ ent,
-                         const int* __restrict__ pair_idx, const int* __restrict__ head,
-                         const int* __restrict__ first_pair, const int* __restrict__ blk_off,
-                         const int* __restrict__ rowptr, int n_rows, long long nnz, SddmmBlock* __restrict__ blk) {
-    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nnz) return;
-    const unsigned long long k = key[i];
-    const int w = (int)(k >> 32);
-    const int local = pair_idx[i] - first_pair[w];
-    SddmmBlock* b = blk + (size_t)blk_off[w] + (local >> 3);
-    const int n = local & 7;
-    const int e = ent[i];
-    const int r = row_of_entry(rowptr, n_rows, e) - (w << 4);
-    atomicOr(&b->bits[r >> 2], 1u << (((r & 3) << 3) + n));
-    atomicMin(&b->start[r], e);
-    if (head[i]) {
-        b->col[n] = (int)(unsigned)k;
-        if (n == 0) b->window = w;
+    if (w < W) {
+        const int n = lower(w + 1) - mine;
+        quads_of[w] = (n + 31) >> 5;
+        if (n > 0) atomicAdd(n_blocks, (n + 7) >> 3);
+    } else {
+        quads_of[w] = 0;
     }
 }
 
-constexpr int kSddmmBlocksPerWarp = 48;
+// Column ids, and where a quad's entries begin among the sorted ones (they are contiguous).
+__global__ void ksp_columns(const unsigned long long* __restrict__ key, const int* __restrict__ pair_idx,
+                            const int* __restrict__ head, const int* __restrict__ first_pair, const int* __restrict__ quad_off,
+                            long long nnz, int* __restrict__ ids, int* __restrict__ begin) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= nnz || !head[i]) return;
+    const unsigned long long k = key[i];
+    const int w = (int)(k >> 32);
+    const int local = pair_idx[i] - first_pair[w];
+    const size_t q = (size_t)quad_off[w] + (local >> 5);
+    ids[q * 32 + (local & 31)] = (int)(unsigned)k;
+    if ((local & 31) == 0) begin[q] = (int)i;
+}
 
-// One warp walks kSddmmBlocksPerWarp consecutive blocks, one block at a time, with both dependent
-// loads of a block taken off the warp's critical path: the
-// 128-byte records run kRecAhead blocks ahead and the 8 gathered Y rows kRowAhead blocks ahead,
-// all as 16-byte cp.async copies into the warp's own rings in shared memory (one commit group per
-// block, lanes meet in one __syncwarp per block, no block-wide barrier).  The odd Y rows land with
-// the two 64-byte halves of every 128 bytes swapped (chunk c at position c ^ 4): a 16-byte access
-// is served eight lanes at a time, those are the lanes (g, t) of two consecutive rows g with four
-// chunks each, and the swap puts the two rows into different halves of the 128-byte bank line, so
-// the copies and the fragment reads - lane (g, t) takes chunks 4 ch + t of row g - are
-// conflict-free without padding (rows of 64 bytes already alternate halves).  Holding the rows in
-// registers instead (plain 16-byte loads two blocks ahead, no shared-memory round trip) measured
-// slower: 0.127 against 0.109 ms on the clustered pattern.
-constexpr int kRecRing = 8, kRecAhead = 6, kRowAhead = 3, kRowStages = 4;
+// One warp per quad: header, repeated columns, and the entries in CSR order, placed by row masks.
+__global__ void ksp_quads(const unsigned long long* __restrict__ key, const int* __restrict__ ent, const int* __restrict__ pair_idx,
+                          const int* __restrict__ first_pair, const int* __restrict__ begin, const int* __restrict__ rowptr,
+                          int n_rows, int nnz, int n_quads, SddmmQuad* __restrict__ quads, int* __restrict__ ids,
+                          unsigned* __restrict__ list, int* __restrict__ err) {
+    __shared__ unsigned s_mask[8][16];
+    __shared__ int s_before[8][16];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int q = blockIdx.x * 8 + wid;
+    if (q >= n_quads) return;
+    const int b = begin[q], e = q + 1 < n_quads ? begin[q + 1] : nnz;
+    const int w = (int)(key[b] >> 32), pair0 = pair_idx[b];
+    const int cols = pair_idx[e - 1] - pair0 + 1;
+    const int e0 = rowptr[w * 16];
+    if (lane < 16) s_mask[wid][lane] = 0u;
+    __syncwarp();
+    auto place = [&](int i, int& r, int& n) {
+        const int x = ent[i];
+        n = pair_idx[i] - pair0;
+        r = 0;
+        for (int k = 1; k < 16 && w * 16 + k < n_rows; ++k) r += rowptr[w * 16 + k] <= x;
+    };
+    for (int i = b + lane; i < e; i += 32) {
+        int r, n;
+        place(i, r, n);
+        atomicOr(&s_mask[wid][r], 1u << n);
+    }
+    __syncwarp();
+    int count = lane < 16 ? __popc(s_mask[wid][lane]) : 0, incl = count;
+#pragma unroll
+    for (int d = 1; d < 16; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, incl, d);
+        if (lane >= d) incl += y;
+    }
+    if (lane < 16) s_before[wid][lane] = incl - count;
+    __syncwarp();
+    for (int i = b + lane; i < e; i += 32) {
+        int r, n;
+        place(i, r, n);
+        const int rel = ent[i] - e0;
+        if (rel >= 1 << (32 - kPosBits)) atomicOr(err, 4);
+        list[b + s_before[wid][r] + __popc(s_mask[wid][r] & ((1u << n) - 1u))] = ((unsigned)rel << kPosBits) | (unsigned)(r << 5 | n);
+    }
+    const int blocks = (cols + 7) / 8;
+    if (lane >= cols && lane < blocks * 8) ids[(size_t)q * 32 + lane] = ids[(size_t)q * 32];
+    if (lane == 0) quads[q] = SddmmQuad{w, e0, (e - b) << 3 | blocks, b};
+}
+
+// One warp walks a contiguous range of quads, one block of 8 columns at a time: the window's X tile (16 x K) sits
+// in registers as A fragments, the 8 gathered Y rows are the B fragments.  Column ids (one per lane) and
+// headers come from memory two quads ahead, the Y rows kRowAhead blocks ahead as 16-byte cp.async copies into the
+// warp's ring; a lane copies exactly the pieces it reads back, so no lane waits for another.  (The odd Y rows land with
+// the two 64-byte halves of every 128 bytes swapped: chunk c at position c ^ 4.  A 16-byte access is served eight lanes
+// at a time - two consecutive rows g with four chunks each - and the swap puts the two rows into different halves of the
+// 128-byte bank line.)  The 16 x 32 products of a quad are rounded to fp16 into a small tile, and its list of
+// entries - in CSR order, so that neighbours in the list are mostly neighbours in `out` - says which of them go where.
+//
+// What bounds it: instruction issue and the LSU pipe.  With a bitmap per block and four predicated 2-byte stores per
+// lane a block took 99 instructions and, on a power-law pattern, 9 to 16 scattered store sectors one at a time;
+// with lists it is about 35, and what is left is the L2 gather (38 us of the clustered pattern's 0.57 GB at K = 64).
+constexpr int kRowAhead = 3, kRowStages = 4;
+constexpr int kTilePitch = 80;    // bytes per row of the 16 x 32 fp16 tile: the quad's stores hit 32 different banks
+constexpr int kListAhead = 3;     // entries of the list that a lane holds from the start of the quad
 
 template <int KCH>
 struct SddmmRing {
-    static constexpr int ROWB = KCH * 64;                 // bytes of a Y row (K halfs)
+    static constexpr int ROWB = KCH * 64;                 // bytes of a Y row in the ring
     static constexpr int CPR = KCH * 4;                   // 16-byte chunks per row
+    static constexpr bool SWAP = CPR % 8 == 0;            // rows of 64 (mod 128) bytes alternate halves by themselves
     static constexpr int STAGE = 8 * ROWB;
-    static constexpr int WARP_SMEM = kRecRing * 128 + kRowStages * STAGE;
+    static constexpr int WARP_SMEM = kRowStages * STAGE + 16 * kTilePitch;
     static constexpr int SMEM = 4 * WARP_SMEM;
+    // per SM: shared memory and registers (K = 64 with 8 CTAs of 64 registers spills: 85 against 81 us, clustered)
+    static constexpr int CTAS = KCH == 1 ? 8 : KCH == 2 ? 7 : KCH <= 4 ? 5 : KCH <= 6 ? 4 : 3;
 };
 
-template <int KCH, int MINB>
-__global__ void __launch_bounds__(128, MINB) k_sddmm_tc_ring(const SddmmBlock* __restrict__ blk, long long n_blocks,
-                                                             const __half* __restrict__ X, const __half* __restrict__ Y,
-                                                             __half* __restrict__ out, int n_rows, int blocks_per_warp) {
+template <int N, int I = 0, class Fn>
+__device__ __forceinline__ void sddmm_for(Fn&& fn) {
+    if constexpr (I < N) {
+        fn(std::integral_constant<int, I>());
+        sddmm_for<N, I + 1>(fn);
+    }
+}
+
+template <int OFFSET, int FROM>
+__device__ __forceinline__ void cp_async16_to(uint32_t dst, const void* src) {
+    asm volatile("cp.async.cg.shared.global [%0+%2], [%1+%3], 16;\n" ::"r"(dst), "l"(src), "n"(OFFSET), "n"(FROM));
+}
+
+// TAIL: K is not a multiple of 32; the chunks past the end of a row are zero on both sides.
+template <int KCH, bool TAIL>
+__global__ void __launch_bounds__(128, SddmmRing<KCH>::CTAS) k_sddmm_tc_ring(
+    const SddmmQuad* __restrict__ quads, const int* __restrict__ ids, const unsigned* __restrict__ list, int n_quads,
+    const __half* __restrict__ X, const __half* __restrict__ Y, __half* __restrict__ out, int n_rows, int pieces, int ld16,
+    int quads_per_warp) {
     using R = SddmmRing<KCH>;
     extern __shared__ __align__(128) unsigned char smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int g = lane >> 2, t = lane & 3;
-    const long long warp = (long long)blockIdx.x * (blockDim.x >> 5) + wid;
-    const long long b0 = warp * blocks_per_warp;
-    if (b0 >= n_blocks) return;
-    const int nb = (int)(min(b0 + (long long)blocks_per_warp, n_blocks) - b0);
-    unsigned char* recs = smem + wid * R::WARP_SMEM;
-    unsigned char* rows = recs + kRecRing * 128;
-    const uint32_t recs0 = smem_u32(recs), rows0 = smem_u32(rows);
-    constexpr int ROW16 = KCH * 4;
-    const uint4* Xq = (const uint4*)X + t;
-    const uint4* Yq = (const uint4*)Y;
+    const int q0 = (blockIdx.x * 4 + wid) * quads_per_warp;
+    if (q0 >= n_quads) return;
+    const int nq = min(quads_per_warp, n_quads - q0);
+    unsigned char* const ring = smem + wid * R::WARP_SMEM;
+    unsigned char* const tile = ring + kRowStages * R::STAGE;
+    const uint32_t rows0 = smem_u32(ring);
+    const unsigned char* Xq = (const unsigned char*)(X + 8 * t);
+    const unsigned char* Yq = (const unsigned char*)(Y + 8 * t);
+    const uint32_t pitch = (uint32_t)ld16 * 16u;
+    const uint32_t swap = R::SWAP ? (uint32_t)(g & 1) * 64u : 0u;
+    const uint32_t row_at = rows0 + g * R::ROWB + t * 16;
+    const uint32_t at_even = row_at + swap, at_odd = row_at + (swap ^ 64u);
+    quads += q0;
+    ids += (size_t)q0 * 32 + lane;
 
-    // `slot` / `stage` arguments are the ring positions of block j, passed separately so that they are
-    // compile-time constants inside the unrolled loop below
-    auto issue_rec = [&](int j, int slot) {   // record of block j -> record ring (8 lanes x 16 B)
-        if (j < nb && lane < 8) cp_async16(recs0 + slot * 128 + lane * 16, (const uint4*)(blk + b0 + j) + lane, 16);
+    auto load_ids = [&](int q) { return q < nq ? __ldg(ids + (size_t)q * 32) : 0; };
+    auto load_head = [&](int q) { return q < nq ? __ldg((const int4*)(quads + q)) : make_int4(0, 0, 0, 0); };
+    auto issue_rows = [&](int c, auto stage) {
+        constexpr int S = decltype(stage)::value * R::STAGE;
+        const unsigned char* src = Yq + (unsigned long long)(uint32_t)c * pitch;
+        sddmm_for<KCH>([&](auto ii) {
+            constexpr int i = decltype(ii)::value;
+            const uint32_t at = R::SWAP ? ((i & 1) ? at_odd : at_even) : row_at;
+            constexpr int off = S + (R::SWAP ? (i / 2) * 128 : i * 64);
+            if constexpr (!TAIL) cp_async16_to<off, i * 64>(at, src);
+            else cp_async16(at + off, 4 * i + t < pieces ? src + i * 64 : src, 4 * i + t < pieces ? 16 : 0);
+        });
     };
-    // Y rows of block j (its record is in the ring): lane copies chunks (lane & 3) + 4 i of row lane >> 2
-    auto issue_rows = [&](int j, int slot, int stage) {
-        if (j >= nb) return;
-        const int c = *(const int*)(recs + slot * 128 + g * 4);
-        const uint4* src = Yq + (size_t)max(c, 0) * ROW16;
-        const uint32_t dst = rows0 + stage * R::STAGE + g * R::ROWB;
-#pragma unroll
-        for (int i = 0; i < KCH; ++i) {
-            const int chunk = t + 4 * i;
-            cp_async16(dst + ((chunk ^ ((g & 1) << 2)) & (R::CPR - 1)) * 16, src + chunk, c >= 0 ? 16 : 0);
-        }
-    };
-    // group accounting: prologue = records 0 .. kRecAhead-1 (waited for), then one group per block j
-    // holding the rows of block j + kRowAhead and the record of block j + kRecAhead; the rows of
-    // blocks 0 .. kRowAhead-1 are kRowAhead groups of their own.  At iteration j all but the newest
-    // kRowAhead-1 groups are complete: the rows of block j and the record of block j + kRowAhead.
-#pragma unroll
-    for (int j = 0; j < kRecAhead; ++j) issue_rec(j, j);
-    cp_async_commit();
-    cp_async_wait<0>();
-    __syncwarp();
-#pragma unroll
-    for (int j = 0; j < kRowAhead; ++j) {
-        issue_rows(j, j, j);
+    // blocks of 8 columns in a quad; z: entries << 3 | blocks
+    auto blocks_of = [](const int4& h) { return h.z & 7; };
+
+    int id = load_ids(0), id1 = load_ids(1);
+    int4 head = load_head(0), head1 = load_head(1);
+    sddmm_for<kRowAhead>([&](auto u) {
+        constexpr int b = decltype(u)::value;
+        if (b < blocks_of(head)) issue_rows(__shfl_sync(0xffffffffu, id, 8 * b + g), u);
         cp_async_commit();
-    }
-
+    });
     int cur_w = -1;
     uint4 xa[KCH], xb[KCH];
 #pragma unroll
     for (int c = 0; c < KCH; ++c) xa[c] = xb[c] = make_uint4(0, 0, 0, 0);
-    static_assert(kRecRing == 8 && kRowStages == 4, "the loop is unrolled by the record ring");
-    for (int j0 = 0; j0 < nb; j0 += kRecRing) {
+
+    for (int q = 0; q < nq; ++q) {
+        const int id2 = load_ids(q + 2);
+        const int4 head2 = load_head(q + 2);
+        const int nb = blocks_of(head), nb1 = blocks_of(head1), n_ent = head.z >> 3;
+        const unsigned* entries = list + (unsigned)head.w;
+        unsigned ent[kListAhead];
 #pragma unroll
-        for (int u = 0; u < kRecRing; ++u) {
-            const int j = j0 + u;
-            if (j >= nb) break;
-            cp_async_wait<kRowAhead - 1>();
-            __syncwarp();
-            issue_rec(j + kRecAhead, (u + kRecAhead) & (kRecRing - 1));
-            issue_rows(j + kRowAhead, (u + kRowAhead) & (kRecRing - 1), (u + kRowAhead) & (kRowStages - 1));
-            cp_async_commit();
-            const unsigned char* rec = recs + u * 128;
-            const int w = *(const int*)(rec + 48);
-            const unsigned wa = *(const unsigned*)(rec + 32 + (g >> 2) * 4), wb = *(const unsigned*)(rec + 32 + ((g >> 2) + 2) * 4);
-            if (w != cur_w) {  // warp-uniform
-                cur_w = w;
-                const int ra = min(w * 16 + g, n_rows - 1), rb = min(w * 16 + g + 8, n_rows - 1);
-#pragma unroll
-                for (int ch = 0; ch < KCH; ++ch) {
-                    xa[ch] = __ldg(Xq + (size_t)ra * ROW16 + ch * 4);
-                    xb[ch] = __ldg(Xq + (size_t)rb * ROW16 + ch * 4);
-                }
-            }
-            const unsigned char* yrow = rows + (u & (kRowStages - 1)) * R::STAGE + g * R::ROWB;
-            float d[4] = {0.f, 0.f, 0.f, 0.f};
+        for (int i = 0; i < kListAhead; ++i) ent[i] = 32 * i + lane < n_ent ? __ldg(entries + 32 * i + lane) : 0u;
+        if (head.x != cur_w) {  // warp-uniform
+            cur_w = head.x;
+            const unsigned char* ra = Xq + (size_t)min(cur_w * 16 + g, n_rows - 1) * pitch;
+            const unsigned char* rb = Xq + (size_t)min(cur_w * 16 + g + 8, n_rows - 1) * pitch;
 #pragma unroll
             for (int ch = 0; ch < KCH; ++ch) {
-                const uint4 y = *(const uint4*)(yrow + (((4 * ch + t) ^ ((g & 1) << 2)) & (R::CPR - 1)) * 16);
-                mma_16816(d, xa[ch].x, xb[ch].x, xa[ch].y, xb[ch].y, y.x, y.y);
-                mma_16816(d, xa[ch].z, xb[ch].z, xa[ch].w, xb[ch].w, y.z, y.w);
-            }
-            const unsigned ba = (wa >> ((g & 3) << 3)) & 0xffu, bbits = (wb >> ((g & 3) << 3)) & 0xffu;
-            const int n0 = 2 * t;
-            if ((ba >> n0) & 3u) {
-                const int s = *(const int*)(rec + 64 + g * 4) + __popc(ba & ((1u << n0) - 1u));
-                if ((ba >> n0) & 1u) out[s] = __float2half_rn(d[0]);
-                if ((ba >> n0) & 2u) out[s + ((ba >> n0) & 1u)] = __float2half_rn(d[1]);
-            }
-            if ((bbits >> n0) & 3u) {
-                const int s = *(const int*)(rec + 64 + (g + 8) * 4) + __popc(bbits & ((1u << n0) - 1u));
-                if ((bbits >> n0) & 1u) out[s] = __float2half_rn(d[2]);
-                if ((bbits >> n0) & 2u) out[s + ((bbits >> n0) & 1u)] = __float2half_rn(d[3]);
+                if (!TAIL || 4 * ch + t < pieces) {
+                    xa[ch] = __ldg((const uint4*)(ra + ch * 64));
+                    xb[ch] = __ldg((const uint4*)(rb + ch * 64));
+                }
             }
         }
+        // group 4 q + b carries the rows of block b; all but the newest kRowAhead - 1 groups are complete
+        const bool full = nb == 4 && nb1 == 4;
+        auto blocks = [&](auto all) {
+        sddmm_for<4>([&](auto uu) {
+            constexpr bool ALL = decltype(all)::value;
+            constexpr int b = decltype(uu)::value, bn = (b + kRowAhead) & 3;
+            cp_async_wait<kRowAhead - 1>();
+            if constexpr (b + kRowAhead < 4) {
+                if (ALL || bn < nb) issue_rows(__shfl_sync(0xffffffffu, id, 8 * bn + g), std::integral_constant<int, bn>());
+            } else {
+                if (ALL || bn < nb1) issue_rows(__shfl_sync(0xffffffffu, id1, 8 * bn + g), std::integral_constant<int, bn>());
+            }
+            cp_async_commit();
+            if (ALL || b < nb) {
+                float d[4] = {0.f, 0.f, 0.f, 0.f}, d2[4] = {0.f, 0.f, 0.f, 0.f};   // two chains
+                sddmm_for<KCH>([&](auto ii) {
+                    constexpr int i = decltype(ii)::value;
+                    constexpr int off = b * R::STAGE + (R::SWAP ? (i / 2) * 128 : i * 64);
+                    uint4 y;
+                    const uint32_t at = R::SWAP ? ((i & 1) ? at_odd : at_even) : row_at;
+                    asm volatile("ld.shared.v4.u32 {%0,%1,%2,%3}, [%4+%5];" : "=r"(y.x), "=r"(y.y), "=r"(y.z), "=r"(y.w) : "r"(at), "n"(off));
+                    mma_16816(d, xa[i].x, xb[i].x, xa[i].y, xb[i].y, y.x, y.y);
+                    mma_16816(d2, xa[i].z, xb[i].z, xa[i].w, xb[i].w, y.z, y.w);
+                });
+#pragma unroll
+                for (int i = 0; i < 4; ++i) d[i] += d2[i];
+                *(__half2*)(tile + g * kTilePitch + b * 16 + t * 4) = __floats2half2_rn(d[0], d[1]);
+                *(__half2*)(tile + (g + 8) * kTilePitch + b * 16 + t * 4) = __floats2half2_rn(d[2], d[3]);
+            }
+        });
+        };
+        if (full) blocks(std::true_type()); else blocks(std::false_type());
+        __syncwarp();
+        __half* const o = out + (unsigned)head.y;
+        auto put = [&](unsigned e) {
+            const unsigned pos = e & ((1u << kPosBits) - 1u);
+            o[e >> kPosBits] = *(const __half*)(tile + (pos >> 5) * kTilePitch + (pos & 31u) * 2);
+        };
+#pragma unroll
+        for (int i = 0; i < kListAhead; ++i)
+            if (32 * i + lane < n_ent) put(ent[i]);
+        for (int i = 32 * kListAhead + lane; i < n_ent; i += 32) put(__ldg(entries + i));
+        __syncwarp();
+        id = id1; id1 = id2;
+        head = head1; head1 = head2;
     }
     cp_async_wait<0>();
 }
-
 
 }  // namespace trs
 
@@ -367,12 +440,18 @@ struct trs_sddmm_plan {
     const int32_t* col = nullptr;
     int n_rows = 0, n_cols = 0;
     long long nnz = 0, n_blocks = 0, n_pairs = 0;
-    trs::DevBuf<trs::SddmmBlock> blocks;
+    int n_quads = 0;
+    bool wide = false;   // a window with too many entries for the lists
+    trs::DevBuf<trs::SddmmQuad> quads;
+    trs::DevBuf<int> ids;         // [quads][32]
+    trs::DevBuf<unsigned> list;   // [nnz]
 };
 
 extern "C" int trs_sddmm_plan_destroy(trs_sddmm_plan* p) {
     if (!p) return TRS_OK;
-    p->blocks.release();
+    p->quads.release();
+    p->ids.release();
+    p->list.release();
     delete p;
     return TRS_OK;
 }
@@ -398,85 +477,84 @@ extern "C" int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, 
     if (nnz == 0) { *out = p; return TRS_OK; }
 
     const int W = (n_rows + 15) / 16;
-    DevBuf<unsigned long long> key_a, key_b;
-    DevBuf<int> ent_a, ent_b, head, pair_idx, first_pair, blocks_of, blk_off;
-    DevBuf<unsigned char> tmp;
-    auto cleanup = [&]() {
-        key_a.release(); key_b.release(); ent_a.release(); ent_b.release(); head.release(); pair_idx.release();
-        first_pair.release(); blocks_of.release(); blk_off.release(); tmp.release();
-    };
-    auto fail = [&](int code) { cleanup(); trs_sddmm_plan_destroy(p); return code; };
-    int rc = key_a.alloc(nnz);
-    if (!rc) rc = key_b.alloc(nnz);
-    if (!rc) rc = ent_a.alloc(nnz);
-    if (!rc) rc = ent_b.alloc(nnz);
-    if (!rc) rc = head.alloc(nnz);
-    if (!rc) rc = pair_idx.alloc(nnz);
-    if (!rc) rc = first_pair.alloc((size_t)W + 1);
-    if (!rc) rc = blocks_of.alloc((size_t)W + 1);
-    if (!rc) rc = blk_off.alloc((size_t)W + 1);
+    TempSpace ts;
+    ts.st = st;
+    ts.chunk_bytes = (size_t)nnz * 38 + ((size_t)W + 1) * 12 + ((size_t)8 << 20);
+    unsigned long long *key_a, *key_b;
+    int *ent_a, *ent_b, *head, *pair_idx, *first_pair, *quads_of, *quad_off, *begin, *d_err;
+    auto fail = [&](int code) { trs_sddmm_plan_destroy(p); return code; };
+    int rc = ts.get(nnz, &key_a);
+    if (!rc) rc = ts.get(nnz, &key_b);
+    if (!rc) rc = ts.get(nnz, &ent_a);
+    if (!rc) rc = ts.get(nnz, &ent_b);
+    if (!rc) rc = ts.get(nnz, &head);
+    if (!rc) rc = ts.get(nnz, &pair_idx);
+    if (!rc) rc = ts.get((size_t)W + 1, &first_pair);
+    if (!rc) rc = ts.get((size_t)W + 1, &quads_of);
+    if (!rc) rc = ts.get((size_t)W + 1, &quad_off);
+    if (!rc) rc = ts.get(nnz, &begin);
+    if (!rc) rc = ts.get(2, &d_err);   // error bits, number of 8-column blocks
     if (rc) return fail(rc);
     auto grid = [](long long n) { return (unsigned)((n + 255) / 256); };
-    DevBuf<int> d_err;
-    rc = d_err.alloc(1);
-    if (rc) return fail(rc);
-    cudaMemsetAsync(d_err.p, 0, sizeof(int), st);
-    ksp_keys<<<grid(nnz), 256, 0, st>>>(rowptr, col, n_rows, n_cols, nnz, key_a.p, ent_a.p, d_err.p);
+    cudaMemsetAsync(d_err, 0, 2 * sizeof(int), st);
+    ksp_keys<<<grid(nnz), 256, 0, st>>>(rowptr, col, n_rows, n_cols, nnz, key_a, ent_a, d_err);
     {
         int herr = 0;
-        cudaError_t ee = cudaMemcpyAsync(&herr, d_err.p, sizeof(int), cudaMemcpyDeviceToHost, st);
+        cudaError_t ee = cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
         if (ee == cudaSuccess) ee = cudaStreamSynchronize(st);
-        d_err.release();
         if (ee != cudaSuccess) return fail((int)ee);
         if (herr & 1) return fail(TRS_E_COLUMN);
         if (herr & 2) return fail(TRS_E_NOT_CANONICAL);
     }
     int wbits = 1;
     while ((1ll << wbits) < W) ++wbits;
-    cub::DoubleBuffer<unsigned long long> kb(key_a.p, key_b.p);
-    cub::DoubleBuffer<int> vb(ent_a.p, ent_b.p);
+    cub::DoubleBuffer<unsigned long long> kb(key_a, key_b);
+    cub::DoubleBuffer<int> vb(ent_a, ent_b);
     size_t bytes = 0, bytes2 = 0, bytes3 = 0;
     cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, bytes, kb, vb, (int)nnz, 0, 32 + wbits, st);
-    if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(nullptr, bytes2, head.p, pair_idx.p, (int)nnz, st);
-    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, bytes3, blocks_of.p, blk_off.p, W + 1, st);
+    if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(nullptr, bytes2, head, pair_idx, (int)nnz, st);
+    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, bytes3, quads_of, quad_off, W + 1, st);
     if (e != cudaSuccess) return fail((int)e);
-    if (bytes2 > bytes) bytes = bytes2;
-    if (bytes3 > bytes) bytes = bytes3;
-    rc = tmp.alloc(bytes + 16);
-    if (rc) return fail(rc);
-    e = cub::DeviceRadixSort::SortPairs(tmp.p, bytes, kb, vb, (int)nnz, 0, 32 + wbits, st);
+    bytes = std::max(bytes, std::max(bytes2, bytes3));
+    unsigned char* tmp;
+    if ((rc = ts.get(bytes + 16, &tmp))) return fail(rc);
+    e = cub::DeviceRadixSort::SortPairs(tmp, bytes, kb, vb, (int)nnz, 0, 32 + wbits, st);
     if (e != cudaSuccess) return fail((int)e);
     const unsigned long long* key = kb.Current();
     const int* ent = vb.Current();
-    ksp_heads<<<grid(nnz), 256, 0, st>>>(key, nnz, head.p);
-    e = cub::DeviceScan::InclusiveSum(tmp.p, bytes, head.p, pair_idx.p, (int)nnz, st);  // pair id + 1
+    ksp_heads<<<grid(nnz), 256, 0, st>>>(key, nnz, head);
+    e = cub::DeviceScan::InclusiveSum(tmp, bytes, head, pair_idx, (int)nnz, st);  // pair id + 1
     if (e != cudaSuccess) return fail((int)e);
     int total_pairs = 0;
-    e = cudaMemcpyAsync(&total_pairs, pair_idx.p + (nnz - 1), sizeof(int), cudaMemcpyDeviceToHost, st);
+    e = cudaMemcpyAsync(&total_pairs, pair_idx + (nnz - 1), sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail((int)e);
-    // pair_idx holds inclusive sums: pair id of sorted entry i = pair_idx[i] - 1.  ksp_window_pairs
-    // and ksp_fill only use differences against first_pair, which is taken from the same array.
-    e = cudaMemsetAsync(blocks_of.p, 0, sizeof(int) * ((size_t)W + 1), st);
+    // pair_idx holds inclusive sums: pair id of sorted entry i = pair_idx[i] - 1.  Only differences against
+    // first_pair, which is taken from the same array, are used.
+    ksp_window_pairs<<<grid(W + 1), 256, 0, st>>>(key, pair_idx, nnz, total_pairs + 1, W, first_pair, quads_of, d_err + 1);
+    e = cub::DeviceScan::ExclusiveSum(tmp, bytes, quads_of, quad_off, W + 1, st);
     if (e != cudaSuccess) return fail((int)e);
-    ksp_window_pairs<<<grid(W + 1), 256, 0, st>>>(key, pair_idx.p, nnz, total_pairs + 1, W, first_pair.p, blocks_of.p);
-    e = cub::DeviceScan::ExclusiveSum(tmp.p, bytes, blocks_of.p, blk_off.p, W + 1, st);
-    if (e != cudaSuccess) return fail((int)e);
-    int n_blocks = 0;
-    e = cudaMemcpyAsync(&n_blocks, blk_off.p + W, sizeof(int), cudaMemcpyDeviceToHost, st);
+    int n_quads = 0, n_blocks = 0;
+    e = cudaMemcpyAsync(&n_quads, quad_off + W, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaMemcpyAsync(&n_blocks, d_err + 1, sizeof(int), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e != cudaSuccess) return fail((int)e);
+    p->n_quads = n_quads;
     p->n_blocks = n_blocks;
     p->n_pairs = total_pairs;
-    rc = p->blocks.alloc((size_t)n_blocks);
+    rc = p->quads.alloc((size_t)n_quads);
+    if (!rc) rc = p->ids.alloc((size_t)n_quads * 32);
+    if (!rc) rc = p->list.alloc((size_t)nnz);
     if (rc) return fail(rc);
-    ksp_init_blocks<<<grid((long long)n_blocks * 32), 256, 0, st>>>(p->blocks.p, n_blocks);
-    ksp_fill<<<grid(nnz), 256, 0, st>>>(key, ent, pair_idx.p, head.p, first_pair.p, blk_off.p, rowptr, n_rows, nnz,
-                                       p->blocks.p);
-    e = cudaStreamSynchronize(st);
+    ksp_columns<<<grid(nnz), 256, 0, st>>>(key, pair_idx, head, first_pair, quad_off, nnz, p->ids.p, begin);
+    ksp_quads<<<(unsigned)ceil_div(n_quads, 8), 256, 0, st>>>(key, ent, pair_idx, first_pair, begin, rowptr, n_rows, (int)nnz, n_quads,
+                                                              p->quads.p, p->ids.p, p->list.p, d_err);
+    int herr = 0;
+    e = cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
+    if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return fail((int)e);
-    cleanup();
+    p->wide = (herr & 4) != 0;
     *out = p;
     return TRS_OK;
 }
@@ -488,33 +566,136 @@ extern "C" int trs_sddmm_plan_info(const trs_sddmm_plan* p, long long* n_pairs, 
     return TRS_OK;
 }
 
-extern "C" int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_half* X, const trs_half* Y, trs_half* out,
-                         int n_rows, int n_cols, int K, void* stream);
+namespace {
+
+using namespace trs;
+
+// X and Y as the kernels want them: rows on 16-byte boundaries, `ld` halfs apart.  Otherwise padded copies in
+// pool memory, given back to the pool behind the kernel.
+struct Operands {
+    const __half *X = nullptr, *Y = nullptr;
+    int ld = 0;
+    void* copy = nullptr;
+    cudaStream_t st = nullptr;
+    int prepare(const trs_half* x, const trs_half* y, int n_rows, int n_cols, int K, cudaStream_t stream) {
+        st = stream;
+        X = (const __half*)x; Y = (const __half*)y; ld = K;
+        if (K % 8 == 0 && (((uintptr_t)x | (uintptr_t)y) & 15) == 0) return TRS_OK;
+        ld = (K + 15) & ~15;   // whole 32-byte sectors
+        const int per_row = ld / 8;
+        const int rc = pool_alloc(&copy, ((size_t)n_rows + n_cols) * ld * sizeof(__half), st);
+        if (rc) return rc;
+        __half* xp = (__half*)copy;
+        __half* yp = xp + (size_t)n_rows * ld;
+        k_sddmm_pad<<<(unsigned)ceil_div64((long long)n_rows * per_row, 256), 256, 0, st>>>(X, (long long)n_rows * per_row, K, per_row, xp);
+        k_sddmm_pad<<<(unsigned)ceil_div64((long long)n_cols * per_row, 256), 256, 0, st>>>(Y, (long long)n_cols * per_row, K, per_row, yp);
+        TRS_LAUNCH_CHECK();
+        X = xp; Y = yp;
+        return TRS_OK;
+    }
+    ~Operands() { pool_free(copy, st); }
+};
+
+int sm_count() {
+    static std::atomic<int> cached[64];
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) return 1;
+    int n = cached[dev].load(std::memory_order_relaxed);
+    if (n == 0) {
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev);
+        cached[dev].store(n, std::memory_order_relaxed);
+    }
+    return n > 0 ? n : 1;
+}
+
+int launch_entries(const int32_t* rowptr, const int32_t* col, const Operands& o, trs_half* out, int n_rows, int n_cols, int K,
+                   cudaStream_t st) {
+    const int grid = sm_count() * kEntryCtas;   // one wave
+    auto go = [&](auto kernel) { kernel<<<grid, 32 * kEntryWarps, 0, st>>>(rowptr, col, o.X, o.Y, (__half*)out, n_rows, n_cols, K, o.ld); };
+    if (K <= 32) go(k_sddmm<1>);
+    else if (K <= 64) go(k_sddmm<2>);
+    else if (K <= 96) go(k_sddmm<3>);
+    else go(k_sddmm<4>);
+    TRS_LAUNCH_CHECK();
+    return TRS_OK;
+}
+
+template <int KCH, bool TAIL>
+int launch_ring(const trs_sddmm_plan* p, const Operands& o, trs_half* out, int K, cudaStream_t st) {
+    using R = SddmmRing<KCH>;
+    auto kernel = k_sddmm_tc_ring<KCH, TAIL>;
+    static std::atomic<unsigned long long> done{0};   // per device
+    int dev = 0;
+    TRS_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (!(done.load(std::memory_order_relaxed) & bit)) {
+        TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM));
+        if (dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
+    }
+    // one wave of warps with equal shares (48 blocks a warp left the last of 2.4 waves nearly empty)
+    const int per_warp = ceil_div(p->n_quads, sm_count() * R::CTAS * 4);
+    kernel<<<ceil_div(ceil_div(p->n_quads, per_warp), 4), 128, R::SMEM, st>>>(p->quads.p, p->ids.p, p->list.p, p->n_quads, o.X, o.Y,
+                                                                             (__half*)out, p->n_rows, (K + 7) / 8, o.ld / 8, per_warp);
+    TRS_LAUNCH_CHECK();
+    return TRS_OK;
+}
+
+template <int KCH>
+int launch_ring_k(const trs_sddmm_plan* p, const Operands& o, trs_half* out, int K, cudaStream_t st) {
+    return K == 32 * KCH ? launch_ring<KCH, false>(p, o, out, K, st) : launch_ring<KCH, true>(p, o, out, K, st);
+}
+
+// Two ints the device writes and the host reads (pinned, mapped), with the event that says they are there.  Taken for one
+// call, kept for the next ones: as many exist as calls ever ran at the same time.
+struct EndsWord {
+    int* p = nullptr;
+    cudaEvent_t ready = nullptr;
+    int device = 0;
+};
+std::mutex g_ends_mutex;
+std::vector<EndsWord> g_ends;
+
+int take_ends(EndsWord* w) {
+    int dev = 0;
+    TRS_CUDA(cudaGetDevice(&dev));
+    {
+        std::lock_guard<std::mutex> lock(g_ends_mutex);
+        for (size_t i = g_ends.size(); i-- > 0;)
+            if (g_ends[i].device == dev) {
+                *w = g_ends[i];
+                g_ends.erase(g_ends.begin() + i);
+                return TRS_OK;
+            }
+    }
+    w->device = dev;
+    TRS_CUDA(cudaHostAlloc((void**)&w->p, 2 * sizeof(int), cudaHostAllocPortable | cudaHostAllocMapped));
+    TRS_CUDA(cudaEventCreateWithFlags(&w->ready, cudaEventDisableTiming));
+    return TRS_OK;
+}
+
+}  // namespace
 
 extern "C" int trs_sddmm_plan_run(const trs_sddmm_plan* p, const trs_half* X, const trs_half* Y, trs_half* out, int K,
                                   void* stream) {
     if (!p || !X || !Y || K <= 0) return TRS_E_ARG;
     if (p->nnz == 0) return TRS_OK;
     if (!out) return TRS_E_ARG;
-    const bool tc = (K == 32 || K == 64 || K == 128) && (((uintptr_t)X & 15) == 0) && (((uintptr_t)Y & 15) == 0);
-    if (!tc) return trs_sddmm(p->rowptr, p->col, X, Y, out, p->n_rows, p->n_cols, K, stream);
     cudaStream_t st = (cudaStream_t)stream;
-    const int bpw = trs::kSddmmBlocksPerWarp;
-    const long long warps = trs::ceil_div64(p->n_blocks, bpw);
-    const unsigned grid = (unsigned)trs::ceil_div64(warps, 4);
-    const __half *x = (const __half*)X, *y = (const __half*)Y;
-    auto launch = [&](auto kernel, int smem) -> int {
-        TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-        kernel<<<grid, 128, smem, st>>>(p->blocks.p, p->n_blocks, x, y, (__half*)out, p->n_rows, bpw);
-        return TRS_OK;
-    };
-    int rc;
-    if (K == 32) rc = launch(trs::k_sddmm_tc_ring<1, 8>, trs::SddmmRing<1>::SMEM);
-    else if (K == 64) rc = launch(trs::k_sddmm_tc_ring<2, 8>, trs::SddmmRing<2>::SMEM);
-    else rc = launch(trs::k_sddmm_tc_ring<4, 5>, trs::SddmmRing<4>::SMEM);
+    Operands o;
+    const int rc = o.prepare(X, Y, p->n_rows, p->n_cols, K, st);
     if (rc) return rc;
-    TRS_LAUNCH_CHECK();
-    return TRS_OK;
+    switch (p->wide ? 0 : (K + 31) / 32) {
+        case 1: return launch_ring_k<1>(p, o, out, K, st);
+        case 2: return launch_ring_k<2>(p, o, out, K, st);
+        case 3: return launch_ring_k<3>(p, o, out, K, st);
+        case 4: return launch_ring_k<4>(p, o, out, K, st);
+        case 5: return launch_ring_k<5>(p, o, out, K, st);
+        case 6: return launch_ring_k<6>(p, o, out, K, st);
+        case 7: return launch_ring_k<7>(p, o, out, K, st);
+        case 8: return launch_ring_k<8>(p, o, out, K, st);
+        default: break;   // a window's X tile no longer fits the registers
+    }
+    return launch_entries(p->rowptr, p->col, o, out, p->n_rows, p->n_cols, K, st);
 }
 
 extern "C" int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_half* X, const trs_half* Y, trs_half* out,
@@ -523,21 +704,29 @@ extern "C" int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_ha
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return TRS_E_NO_DEVICE;
     cudaStream_t st = (cudaStream_t)stream;
-    int ends[2] = {0, 0};
-    TRS_CUDA(cudaMemcpyAsync(&ends[0], rowptr, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TRS_CUDA(cudaMemcpyAsync(&ends[1], rowptr + n_rows, sizeof(int), cudaMemcpyDeviceToHost, st));
-    TRS_CUDA(cudaStreamSynchronize(st));
-    if (ends[0] != 0 || ends[1] < 0) return TRS_E_OFFSETS;
-    const long long nnz = ends[1];
-    if (nnz == 0) return TRS_OK;
-    if (!col || !out) return TRS_E_ARG;
-    const long long warps = trs::ceil_div64(nnz, trs::kEntriesPerWarp);
-    const unsigned blocks = (unsigned)trs::ceil_div64(warps, 8);
-    const bool vec = (K % 8 == 0) && (((uintptr_t)X & 15) == 0) && (((uintptr_t)Y & 15) == 0);
-    if (vec)
-        trs::k_sddmm<true><<<blocks, 256, 0, st>>>(rowptr, col, (const __half*)X, (const __half*)Y, (__half*)out, n_rows, n_cols, nnz, K);
-    else
-        trs::k_sddmm<false><<<blocks, 256, 0, st>>>(rowptr, col, (const __half*)X, (const __half*)Y, (__half*)out, n_rows, n_cols, nnz, K);
-    TRS_LAUNCH_CHECK();
+    // The ends of rowptr decide whether this is an error, and only the device has them.  They are fetched by a kernel
+    // of their own and waited for after the product is queued (it looks at them itself): the host waits for
+    // earlier work of the stream, the device for nobody.
+    EndsWord ends;
+    int rc = take_ends(&ends);
+    if (rc) return rc;
+    Operands o;
+    k_sddmm_ends<<<1, 1, 0, st>>>(rowptr, n_rows, ends.p);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaEventRecord(ends.ready, st);
+    if (e == cudaSuccess && col && out) {
+        rc = o.prepare(X, Y, n_rows, n_cols, K, st);
+        if (!rc) rc = launch_entries(rowptr, col, o, out, n_rows, n_cols, K, st);
+    }
+    if (e == cudaSuccess) e = cudaEventSynchronize(ends.ready);
+    const int first = ends.p[0], last = ends.p[1];
+    {
+        std::lock_guard<std::mutex> lock(g_ends_mutex);
+        g_ends.push_back(ends);
+    }
+    if (e != cudaSuccess) return (int)e;
+    if (rc) return rc;
+    if (first != 0 || last < 0) return TRS_E_OFFSETS;
+    if (last > 0 && (!col || !out)) return TRS_E_ARG;
     return TRS_OK;
 }
