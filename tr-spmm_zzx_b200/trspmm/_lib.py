@@ -179,3 +179,17 @@ def copy_to_device(tensors, device):
 def current_stream_ptr(device) -> int:
     import torch
     return torch.cuda.current_stream(device).cuda_stream
+
+
+def launch(index: int, entry, *args):
+    """entry(*args, current stream of device `index`), with that device current.  The device guard and the stream object
+    of torch.cuda cost 3.7 us a call, as much as a small product takes on the GPU; both are skipped when the device
+    is current already, which it is in all but multi-device programs."""
+    import torch
+    if torch._C._cuda_getDevice() == index:
+        code = entry(*args, torch._C._cuda_getCurrentRawStream(index))
+    else:
+        with torch.cuda.device(index):
+            code = entry(*args, torch._C._cuda_getCurrentRawStream(index))
+    if code:
+        check(code)

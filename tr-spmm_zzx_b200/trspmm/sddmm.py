@@ -15,16 +15,16 @@ def sddmm(rowptr: torch.Tensor, col: torch.Tensor, X: torch.Tensor, Y: torch.Ten
     dev = X.device
     if dev.type != "cuda":
         raise ValueError("sddmm needs CUDA tensors (there is no CPU fallback)")
+    index = X.get_device()
     for t, dt in ((rowptr, torch.int32), (col, torch.int32), (X, torch.float16), (Y, torch.float16)):
-        if t.dtype != dt or t.device != dev or not t.is_contiguous():
+        if t.dtype is not dt or t.get_device() != index or not t.is_contiguous():
             raise ValueError("rowptr/col must be int32, X/Y fp16, all contiguous on one CUDA device")
     if X.dim() != 2 or Y.dim() != 2 or X.shape[1] != Y.shape[1] or rowptr.numel() - 1 != X.shape[0]:
         raise ValueError("X must be [n_rows, K], Y [n_cols, K]")
     if out is None:
-        out = torch.empty(col.numel(), dtype=torch.float16, device=dev)
-    with torch.cuda.device(dev):
-        _lib.check(lib.trs_sddmm(rowptr.data_ptr(), col.data_ptr(), X.data_ptr(), Y.data_ptr(), out.data_ptr(),
-                                 X.shape[0], Y.shape[0], X.shape[1], _lib.current_stream_ptr(dev)))
+        out = torch.empty_like(col, dtype=torch.float16)
+    _lib.launch(index, lib.trs_sddmm, rowptr.data_ptr(), col.data_ptr(), X.data_ptr(), Y.data_ptr(), out.data_ptr(),
+                X.shape[0], Y.shape[0], X.shape[1])
     return out
 
 
@@ -42,7 +42,7 @@ class SddmmPlan:
         for t in (rowptr, col):
             if t.dtype != torch.int32 or t.device != dev or not t.is_contiguous():
                 raise ValueError("rowptr/col must be contiguous int32 tensors on one CUDA device")
-        self.rowptr, self.col, self.device = rowptr, col, dev
+        self.rowptr, self.col, self.device, self._index = rowptr, col, dev, rowptr.get_device()
         self.n_rows, self.n_cols = rowptr.numel() - 1, int(n_cols)
         self._handle = C.c_void_p()
         with torch.cuda.device(dev):
@@ -54,17 +54,16 @@ class SddmmPlan:
 
     def run(self, X: torch.Tensor, Y: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
         for t in (X, Y):
-            if t.dtype != torch.float16 or t.device != self.device or not t.is_contiguous() or t.dim() != 2:
+            if t.dtype is not torch.float16 or t.get_device() != self._index or not t.is_contiguous() or t.dim() != 2:
                 raise ValueError("X/Y must be contiguous fp16 matrices on the plan's device")
         if X.shape[0] != self.n_rows or Y.shape[0] != self.n_cols or X.shape[1] != Y.shape[1]:
             raise ValueError("X must be [n_rows, K], Y [n_cols, K]")
         if out is None:
-            out = torch.empty(self.col.numel(), dtype=torch.float16, device=self.device)
+            out = torch.empty_like(self.col, dtype=torch.float16)
         elif out.dtype != torch.float16 or out.numel() != self.col.numel() or not out.is_contiguous():
             raise ValueError("out must be a contiguous fp16 vector with one element per entry")
-        with torch.cuda.device(self.device):
-            _lib.check(self.lib.trs_sddmm_plan_run(self._handle, X.data_ptr(), Y.data_ptr(), out.data_ptr(),
-                                                   X.shape[1], _lib.current_stream_ptr(self.device)))
+        _lib.launch(self._index, self.lib.trs_sddmm_plan_run, self._handle, X.data_ptr(), Y.data_ptr(), out.data_ptr(),
+                    X.shape[1])
         return out
 
     def close(self):

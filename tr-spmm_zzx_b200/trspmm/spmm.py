@@ -32,6 +32,7 @@ class SpmmPlan:
         self.fmt = fmt.half_values().contiguous()
         self.m_rows, self.k_cols, self.window = int(m_rows), int(k_cols), int(window)
         self.device = self.fmt.device
+        self._index = self.device.index
         self._handle = C.c_void_p()
         self._ws = {}
         with torch.cuda.device(self.device):
@@ -65,16 +66,17 @@ class SpmmPlan:
     def _check_B(self, B: torch.Tensor) -> int:
         """Every entry that hands B to a kernel goes through this: a short or strided B would become
         an out-of-range gather on the device."""
-        if B.device != self.device or B.dtype != torch.float16 or B.dim() != 2 or not B.is_contiguous():
+        if B.dtype is not torch.float16 or B.get_device() != self._index or B.dim() != 2 or not B.is_contiguous():
             raise ValueError("B must be a contiguous fp16 [k_cols, F] tensor on the plan's device")
-        if B.shape[0] != self.k_cols:
-            raise ValueError(f"B has {B.shape[0]} rows, the plan expects {self.k_cols}")
-        if B.shape[1] <= 0:
+        rows, F = B.shape
+        if rows != self.k_cols:
+            raise ValueError(f"B has {rows} rows, the plan expects {self.k_cols}")
+        if F <= 0:
             raise ValueError("B needs at least one feature column")
-        return B.shape[1]
+        return F
 
     def _check_out(self, out: torch.Tensor, F: int):
-        if out.shape != (self.m_rows, F) or not out.is_contiguous() or out.device != self.device:
+        if out.shape != (self.m_rows, F) or not out.is_contiguous() or out.get_device() != self._index:
             raise ValueError("out must be a contiguous [m_rows, F] tensor on the plan's device")
         _out_code(out.dtype)
 
@@ -85,18 +87,23 @@ class SpmmPlan:
             self._ws[F] = ws
         return ws
 
+    def _new_out(self, B: torch.Tensor, F: int, dtype) -> torch.Tensor:
+        if dtype is torch.float16 and self.m_rows == self.k_cols:
+            return torch.empty_like(B)   # half the time of an empty() with a shape and a device
+        return B.new_empty((self.m_rows, F), dtype=dtype)
+
     def run(self, B: torch.Tensor, out: torch.Tensor | None = None, out_dtype=torch.float16,
             relu: bool = False) -> torch.Tensor:
         F = self._check_B(B)
         if out is None:
-            out = torch.empty((self.m_rows, F), dtype=out_dtype, device=self.device)
+            code = _out_code(out_dtype)
+            out = self._new_out(B, F, out_dtype)
         else:
             self._check_out(out, F)
+            code = _out_code(out.dtype)
         ws = self._workspace(F)
-        with torch.cuda.device(self.device):
-            _lib.check(self.lib.trs_spmm_run_ex(self._handle, B.data_ptr(), out.data_ptr(), F, _out_code(out.dtype),
-                                                1 if relu else 0, ws.data_ptr(), ws.numel(),
-                                                _lib.current_stream_ptr(self.device)))
+        _lib.launch(self._index, self.lib.trs_spmm_run_ex, self._handle, B.data_ptr(), out.data_ptr(), F, code,
+                    1 if relu else 0, ws.data_ptr(), ws.numel())
         return out
 
     @property
@@ -126,10 +133,8 @@ class SpmmPlan:
             raise ValueError("1 to 8 destination buffers and a non-negative row offset")
         ws = self._workspace(F)
         arr = (C.c_void_p * len(dst_ptrs))(*[int(p) for p in dst_ptrs])
-        with torch.cuda.device(self.device):
-            _lib.check(self.lib.trs_spmm_run_bcast(self._handle, B.data_ptr(), arr, len(dst_ptrs), int(row0), F,
-                                                   1 if relu else 0, ws.data_ptr(), ws.numel(),
-                                                   _lib.current_stream_ptr(self.device)))
+        _lib.launch(self._index, self.lib.trs_spmm_run_bcast, self._handle, B.data_ptr(), arr, len(dst_ptrs), int(row0), F,
+                    1 if relu else 0, ws.data_ptr(), ws.numel())
 
     def run_static(self, B: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         """trs_spmm_run_static: the same product with the partial sums of split windows kept in
@@ -139,9 +144,8 @@ class SpmmPlan:
         TrsError(-10) when the plan needs more scratch than the fixed array holds.  Calls on one
         device share the array, so do not let two of them overlap on the GPU."""
         self._check_out(out, self._check_B(B))
-        with torch.cuda.device(self.device):
-            _lib.check(self.lib.trs_spmm_run_static(self._handle, B.data_ptr(), out.data_ptr(), B.shape[1],
-                                                    _out_code(out.dtype), _lib.current_stream_ptr(self.device)))
+        _lib.launch(self._index, self.lib.trs_spmm_run_static, self._handle, B.data_ptr(), out.data_ptr(), B.shape[1],
+                    _out_code(out.dtype))
         return out
 
     def close(self):
