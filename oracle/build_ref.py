@@ -85,10 +85,10 @@ def build_all(verbose: bool = True) -> dict:
     """Build whatever can be built; returns {module: path or reason}."""
     root = _ref_root()
     report: dict = {}
-    if not root.exists():
+    block = root / "TR-source" / "Block"
+    if not block.is_dir():  # absent, or an empty mount point
         return {"skipped": f"reference tree {root} not present"}
     OUT.mkdir(exist_ok=True)
-    block = root / "TR-source" / "Block"
     jobs = [
         ("Libra5BlockOnline", block / "block_online.cpp", build_torch_ext),
         ("matching_utils", block / "block_matching_window_para_dr.cpp", build_pybind_ext),
