@@ -14,7 +14,7 @@ import os
 
 import torch
 
-from trspmm import _lib
+from trspmm import _hostpool, _lib
 from trspmm.format import FORMAT_NAMES, Format
 
 __all__ = [
@@ -141,7 +141,7 @@ def forward_fp16_tcu_cuda_sptc_mma_parallel_online(
 
 def _run_host(fmt, rhs, dimN, mOri, kOri, window, epoches, six):
     lib = _lib.load()
-    out = torch.empty((mOri, dimN), dtype=torch.float32)
+    out = _hostpool.empty((mOri, dimN), torch.float32)
     timing = _lib.TrsTiming()
     cf = fmt.c_struct()
     _lib.check(lib.trs_spmm_forward_host(C.byref(cf), rhs.data_ptr(), out.data_ptr(), dimN, mOri, kOri, window,
@@ -195,7 +195,7 @@ def _unpacked(s_column, s_value, s_pos, s_window, s_offsets, rhs_matrix, window,
     groups = s_column.size(0)
     _check(s_value.numel() == groups * window * 2, "s_value must have shape [groups, window, 2]")
     _check(s_pos.numel() == groups * window * 2, "s_pos must have shape [groups, window, 2]")
-    out = torch.empty((mOri, dimN), dtype=torch.float32)
+    out = _hostpool.empty((mOri, dimN), torch.float32)
     timing = _lib.TrsTiming()
     nw = 0
     if s_offsets is not None:

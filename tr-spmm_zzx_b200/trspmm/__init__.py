@@ -5,7 +5,7 @@ this package binds it with ctypes and uses torch only for device memory and stre
 no CPU fallback: every operator raises when the library or a CUDA device is missing.
 """
 from . import graphs  # noqa: F401
-from ._lib import TrsError, lib_path, load  # noqa: F401
+from ._lib import TrsError, lib_path, load, release_cached_memory  # noqa: F401
 from .format import FORMAT_NAMES, Format  # noqa: F401
 from .spmm import SpmmPlan, spmm_forward_host, ResidentSpmm  # noqa: F401
 from .sddmm import sddmm, SddmmPlan  # noqa: F401

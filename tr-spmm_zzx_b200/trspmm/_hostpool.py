@@ -1,0 +1,62 @@
+"""Host memory of large results that came and went, kept for the next ones.
+
+The reference's calling convention returns a new CPU tensor per call.  For a result of tens of megabytes the page
+faults of fresh memory cost more than the copy from the device (33 MB: 1.7 against 0.6 ms), and the C library gives
+such blocks back to the system every time.  Blocks handed out here return to a list when the last tensor
+over them is gone; at most KEEP_BYTES wait there, the oldest go first, release() lets all of them go.
+"""
+from __future__ import annotations
+
+import math
+import mmap
+import threading
+import weakref
+
+import numpy as np
+import torch
+
+MIN_BYTES = 1 << 20      # below, the C library reuses memory itself
+KEEP_BYTES = 256 << 20
+_BLOCK = 2 << 20         # large pages
+
+_lock = threading.RLock()   # re-entrant: a collection inside take() may give blocks back
+_idle: list = []            # oldest first
+
+
+def _give_back(block):
+    with _lock:
+        _idle.append(block)
+        waiting = sum(len(b) for b in _idle)
+        while waiting > KEEP_BYTES:
+            waiting -= len(_idle.pop(0))
+
+
+def _take(n: int):
+    with _lock:
+        fits = [i for i, b in enumerate(_idle) if n <= len(b) <= n + n // 4 + _BLOCK]
+        if fits:
+            return _idle.pop(min(fits, key=lambda i: len(_idle[i])))
+    block = mmap.mmap(-1, -(-n // _BLOCK) * _BLOCK)
+    if hasattr(mmap, "MADV_HUGEPAGE"):
+        try:
+            block.madvise(mmap.MADV_HUGEPAGE)
+        except OSError:   # a kernel without large pages
+            pass
+    return block
+
+
+def empty(shape, dtype: torch.dtype) -> torch.Tensor:
+    """An uninitialised CPU tensor."""
+    count = math.prod(shape)
+    n = count * dtype.itemsize
+    if n < MIN_BYTES or n > KEEP_BYTES:
+        return torch.empty(shape, dtype=dtype)
+    block = _take(n)
+    owner = np.frombuffer(block, dtype=np.uint8, count=n)   # lives as long as the tensor's storage
+    weakref.finalize(owner, _give_back, block).atexit = False
+    return torch.from_numpy(owner).view(dtype).view(shape)
+
+
+def release():
+    with _lock:
+        _idle.clear()

@@ -161,10 +161,19 @@ def copy_to_host(tensors, device):
     """CPU copies of contiguous CUDA tensors of one device (trs_copy_to_host): all of them in one go, after the work on the
     current stream."""
     import torch
-    out = [torch.empty(t.shape, dtype=t.dtype) for t in tensors]
+    from . import _hostpool
+    out = [_hostpool.empty(t.shape, t.dtype) for t in tensors]
     with torch.cuda.device(device):
         _copy(load().trs_copy_to_host, out, tensors, device)
     return out
+
+
+def release_cached_memory():
+    """Gives back what is kept between calls: the current device's pool and the pinned ring of the library, the
+    idle result buffers on the host."""
+    from . import _hostpool
+    _hostpool.release()
+    check(load().trs_pool_trim())
 
 
 def copy_to_device(tensors, device):

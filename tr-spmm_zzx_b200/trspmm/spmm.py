@@ -5,7 +5,7 @@ import ctypes as C
 
 import torch
 
-from . import _lib
+from . import _hostpool, _lib
 from .format import Format
 
 OUT_F32, OUT_F16 = 0, 1
@@ -173,7 +173,7 @@ def spmm_forward_host(fmt: Format, rhs: torch.Tensor, dimN: int, mOri: int, kOri
     lib = _lib.load()
     f = _cpu_format(fmt)
     rhs = rhs.contiguous()
-    out = torch.empty((mOri, dimN), dtype=torch.float32)
+    out = _hostpool.empty((mOri, dimN), torch.float32)
     timing = _lib.TrsTiming()
     cf = f.c_struct()
     _lib.check(lib.trs_spmm_forward_host(C.byref(cf), rhs.data_ptr(), out.data_ptr(), dimN, mOri, kOri, window,
