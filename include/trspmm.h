@@ -345,6 +345,9 @@ int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, int n_rows,
                           void* stream, trs_sddmm_plan** out);
 int trs_sddmm_plan_run(const trs_sddmm_plan* plan, const trs_half* X, const trs_half* Y,
                        trs_half* out, int K, void* stream);
+/* The same with the result in fp32 (TRS_OUT_F32: the fp16 values widened) or fp16. */
+int trs_sddmm_plan_run_ex(const trs_sddmm_plan* plan, const trs_half* X, const trs_half* Y, void* out, int K,
+                          int out_dtype, void* stream);
 /* distinct (window, column) pairs and 8-column blocks of the plan */
 int trs_sddmm_plan_info(const trs_sddmm_plan* plan, long long* n_pairs, long long* n_blocks);
 int trs_sddmm_plan_destroy(trs_sddmm_plan* plan);

@@ -31,6 +31,7 @@ def test_widths(kind, K):
     for run in (lambda out: sddmm(rp, col, X, Y, out=out), lambda out: plan.run(X, Y, out=out)):
         out = run(torch.full((col.numel(),), float("nan"), dtype=torch.float16, device="cuda")).float().cpu()
         assert float((out - ref).abs().max()) <= 2e-3 * scale
+    assert torch.equal(plan.run(X, Y, out_dtype=torch.float32), plan.run(X, Y).float())
     base = torch.empty(n * K + 8, dtype=torch.float16, device="cuda")   # X one element off its boundary
     Xo = base[1:1 + n * K].view(n, K).copy_(X)
     assert torch.equal(plan.run(Xo, Y), plan.run(X, Y)) and torch.equal(sddmm(rp, col, Xo, Y), sddmm(rp, col, X, Y))

@@ -51,10 +51,17 @@ __device__ __forceinline__ int warp_find(const int* __restrict__ a, int n, int x
     return lo;
 }
 
+// Results are fp16 values; callers that go on in fp32 (the gradient of fp32 edge weights) take them widened.
+__device__ __forceinline__ void store_result(void* out, int f32, long long i, __half v) {
+    if (f32) ((float*)out)[i] = __half2float(v);
+    else ((__half*)out)[i] = v;
+}
+
 template <int KCH>   // 32-feature chunks per pass (K > 32 KCH loops)
 __global__ void __launch_bounds__(32 * kEntryWarps, kEntryCtas) k_sddmm(const int* __restrict__ rowptr, const int* __restrict__ col,
                                                             const __half* __restrict__ X, const __half* __restrict__ Y,
-                                                            __half* __restrict__ out, int n_rows, int n_cols, int K, int ld) {
+                                                            void* __restrict__ out, int out_f32, int n_rows, int n_cols, int K,
+                                                            int ld) {
     const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
     const int nnz = rowptr[0] == 0 ? rowptr[n_rows] : 0;   // anything else is an error the caller reports
     const int pieces = (K + 7) / 8, ld16 = ld / 8;
@@ -111,7 +118,7 @@ __global__ void __launch_bounds__(32 * kEntryWarps, kEntryCtas) k_sddmm(const in
                 const int i = 8 * b + g;
                 if (t == (g >> 1) && e0 + i < e_end) {
                     const float v = (g & 1) ? d[1] : d[0];
-                    out[e0 + i] = (bad_mask >> i) & 1u ? __ushort_as_half((unsigned short)0x7e00) : __float2half_rn(v);
+                    store_result(out, out_f32, e0 + i, (bad_mask >> i) & 1u ? __ushort_as_half((unsigned short)0x7e00) : __float2half_rn(v));
                 }
             }
         }
@@ -315,8 +322,8 @@ __device__ __forceinline__ void cp_async16_to(uint32_t dst, const void* src) {
 template <int KCH, bool TAIL>
 __global__ void __launch_bounds__(128, SddmmRing<KCH>::CTAS) k_sddmm_tc_ring(
     const SddmmQuad* __restrict__ quads, const int* __restrict__ ids, const unsigned* __restrict__ list, int n_quads,
-    const __half* __restrict__ X, const __half* __restrict__ Y, __half* __restrict__ out, int n_rows, int pieces, int ld16,
-    int quads_per_warp) {
+    const __half* __restrict__ X, const __half* __restrict__ Y, void* __restrict__ out, int out_f32, int n_rows, int pieces,
+    int ld16, int quads_per_warp) {
     using R = SddmmRing<KCH>;
     extern __shared__ __align__(128) unsigned char smem[];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -417,10 +424,10 @@ __global__ void __launch_bounds__(128, SddmmRing<KCH>::CTAS) k_sddmm_tc_ring(
         };
         if (full) blocks(std::true_type()); else blocks(std::false_type());
         __syncwarp();
-        __half* const o = out + (unsigned)head.y;
+        const long long o = (unsigned)head.y;
         auto put = [&](unsigned e) {
             const unsigned pos = e & ((1u << kPosBits) - 1u);
-            o[e >> kPosBits] = *(const __half*)(tile + (pos >> 5) * kTilePitch + (pos & 31u) * 2);
+            store_result(out, out_f32, o + (e >> kPosBits), *(const __half*)(tile + (pos >> 5) * kTilePitch + (pos & 31u) * 2));
         };
 #pragma unroll
         for (int i = 0; i < kListAhead; ++i)
@@ -608,10 +615,10 @@ int sm_count() {
     return n > 0 ? n : 1;
 }
 
-int launch_entries(const int32_t* rowptr, const int32_t* col, const Operands& o, trs_half* out, int n_rows, int n_cols, int K,
-                   cudaStream_t st) {
+int launch_entries(const int32_t* rowptr, const int32_t* col, const Operands& o, void* out, int out_f32, int n_rows, int n_cols,
+                   int K, cudaStream_t st) {
     const int grid = sm_count() * kEntryCtas;   // one wave
-    auto go = [&](auto kernel) { kernel<<<grid, 32 * kEntryWarps, 0, st>>>(rowptr, col, o.X, o.Y, (__half*)out, n_rows, n_cols, K, o.ld); };
+    auto go = [&](auto kernel) { kernel<<<grid, 32 * kEntryWarps, 0, st>>>(rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K, o.ld); };
     if (K <= 32) go(k_sddmm<1>);
     else if (K <= 64) go(k_sddmm<2>);
     else if (K <= 96) go(k_sddmm<3>);
@@ -621,7 +628,7 @@ int launch_entries(const int32_t* rowptr, const int32_t* col, const Operands& o,
 }
 
 template <int KCH, bool TAIL>
-int launch_ring(const trs_sddmm_plan* p, const Operands& o, trs_half* out, int K, cudaStream_t st) {
+int launch_ring(const trs_sddmm_plan* p, const Operands& o, void* out, int out_f32, int K, cudaStream_t st) {
     using R = SddmmRing<KCH>;
     auto kernel = k_sddmm_tc_ring<KCH, TAIL>;
     static std::atomic<unsigned long long> done{0};   // per device
@@ -635,14 +642,14 @@ int launch_ring(const trs_sddmm_plan* p, const Operands& o, trs_half* out, int K
     // one wave of warps with equal shares (48 blocks a warp left the last of 2.4 waves nearly empty)
     const int per_warp = ceil_div(p->n_quads, sm_count() * R::CTAS * 4);
     kernel<<<ceil_div(ceil_div(p->n_quads, per_warp), 4), 128, R::SMEM, st>>>(p->quads.p, p->ids.p, p->list.p, p->n_quads, o.X, o.Y,
-                                                                             (__half*)out, p->n_rows, (K + 7) / 8, o.ld / 8, per_warp);
+                                                                             out, out_f32, p->n_rows, (K + 7) / 8, o.ld / 8, per_warp);
     TRS_LAUNCH_CHECK();
     return TRS_OK;
 }
 
 template <int KCH>
-int launch_ring_k(const trs_sddmm_plan* p, const Operands& o, trs_half* out, int K, cudaStream_t st) {
-    return K == 32 * KCH ? launch_ring<KCH, false>(p, o, out, K, st) : launch_ring<KCH, true>(p, o, out, K, st);
+int launch_ring_k(const trs_sddmm_plan* p, const Operands& o, void* out, int out_f32, int K, cudaStream_t st) {
+    return K == 32 * KCH ? launch_ring<KCH, false>(p, o, out, out_f32, K, st) : launch_ring<KCH, true>(p, o, out, out_f32, K, st);
 }
 
 // Two ints the device writes and the host reads (pinned, mapped), with the event that says they are there.  Taken for one
@@ -677,7 +684,14 @@ int take_ends(EndsWord* w) {
 
 extern "C" int trs_sddmm_plan_run(const trs_sddmm_plan* p, const trs_half* X, const trs_half* Y, trs_half* out, int K,
                                   void* stream) {
+    return trs_sddmm_plan_run_ex(p, X, Y, out, K, TRS_OUT_F16, stream);
+}
+
+extern "C" int trs_sddmm_plan_run_ex(const trs_sddmm_plan* p, const trs_half* X, const trs_half* Y, void* out, int K,
+                                     int out_dtype, void* stream) {
     if (!p || !X || !Y || K <= 0) return TRS_E_ARG;
+    if (out_dtype != TRS_OUT_F32 && out_dtype != TRS_OUT_F16) return TRS_E_ARG;
+    const int out_f32 = out_dtype == TRS_OUT_F32;
     if (p->nnz == 0) return TRS_OK;
     if (!out) return TRS_E_ARG;
     cudaStream_t st = (cudaStream_t)stream;
@@ -685,17 +699,17 @@ extern "C" int trs_sddmm_plan_run(const trs_sddmm_plan* p, const trs_half* X, co
     const int rc = o.prepare(X, Y, p->n_rows, p->n_cols, K, st);
     if (rc) return rc;
     switch (p->wide ? 0 : (K + 31) / 32) {
-        case 1: return launch_ring_k<1>(p, o, out, K, st);
-        case 2: return launch_ring_k<2>(p, o, out, K, st);
-        case 3: return launch_ring_k<3>(p, o, out, K, st);
-        case 4: return launch_ring_k<4>(p, o, out, K, st);
-        case 5: return launch_ring_k<5>(p, o, out, K, st);
-        case 6: return launch_ring_k<6>(p, o, out, K, st);
-        case 7: return launch_ring_k<7>(p, o, out, K, st);
-        case 8: return launch_ring_k<8>(p, o, out, K, st);
+        case 1: return launch_ring_k<1>(p, o, out, out_f32, K, st);
+        case 2: return launch_ring_k<2>(p, o, out, out_f32, K, st);
+        case 3: return launch_ring_k<3>(p, o, out, out_f32, K, st);
+        case 4: return launch_ring_k<4>(p, o, out, out_f32, K, st);
+        case 5: return launch_ring_k<5>(p, o, out, out_f32, K, st);
+        case 6: return launch_ring_k<6>(p, o, out, out_f32, K, st);
+        case 7: return launch_ring_k<7>(p, o, out, out_f32, K, st);
+        case 8: return launch_ring_k<8>(p, o, out, out_f32, K, st);
         default: break;   // a window's X tile no longer fits the registers
     }
-    return launch_entries(p->rowptr, p->col, o, out, p->n_rows, p->n_cols, K, st);
+    return launch_entries(p->rowptr, p->col, o, out, out_f32, p->n_rows, p->n_cols, K, st);
 }
 
 extern "C" int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_half* X, const trs_half* Y, trs_half* out,
@@ -716,7 +730,7 @@ extern "C" int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_ha
     if (e == cudaSuccess) e = cudaEventRecord(ends.ready, st);
     if (e == cudaSuccess && col && out) {
         rc = o.prepare(X, Y, n_rows, n_cols, K, st);
-        if (!rc) rc = launch_entries(rowptr, col, o, out, n_rows, n_cols, K, st);
+        if (!rc) rc = launch_entries(rowptr, col, o, out, 0, n_rows, n_cols, K, st);
     }
     if (e == cudaSuccess) e = cudaEventSynchronize(ends.ready);
     const int first = ends.p[0], last = ends.p[1];

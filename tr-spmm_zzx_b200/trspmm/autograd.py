@@ -46,7 +46,7 @@ class _SpmmFn(torch.autograd.Function):
         dB = op.plan_t.run(dC, out_dtype=torch.float16) if ctx.needs_input_grad[2] else None
         dval = None
         if ctx.values_need_grad:
-            dval = op.sddmm_plan().run(dC, B.contiguous()).float()
+            dval = op.sddmm_plan().run(dC, B.contiguous(), out_dtype=torch.float32)
         return None, dval, dB
 
 

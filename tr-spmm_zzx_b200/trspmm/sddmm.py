@@ -52,18 +52,22 @@ class SddmmPlan:
         _lib.check(self.lib.trs_sddmm_plan_info(self._handle, C.byref(pairs), C.byref(blocks)))
         self.n_pairs, self.n_blocks = pairs.value, blocks.value
 
-    def run(self, X: torch.Tensor, Y: torch.Tensor, out: torch.Tensor | None = None) -> torch.Tensor:
+    def run(self, X: torch.Tensor, Y: torch.Tensor, out: torch.Tensor | None = None,
+            out_dtype=torch.float16) -> torch.Tensor:
+        """One fp16 value per entry, in CSR order; out_dtype=torch.float32 returns the same values widened."""
         for t in (X, Y):
             if t.dtype is not torch.float16 or t.get_device() != self._index or not t.is_contiguous() or t.dim() != 2:
                 raise ValueError("X/Y must be contiguous fp16 matrices on the plan's device")
         if X.shape[0] != self.n_rows or Y.shape[0] != self.n_cols or X.shape[1] != Y.shape[1]:
             raise ValueError("X must be [n_rows, K], Y [n_cols, K]")
         if out is None:
-            out = torch.empty_like(self.col, dtype=torch.float16)
+            if out_dtype is not torch.float16 and out_dtype is not torch.float32:
+                raise TypeError("output dtype must be torch.float32 or torch.float16")
+            out = torch.empty_like(self.col, dtype=out_dtype)
         elif out.dtype != torch.float16 or out.numel() != self.col.numel() or not out.is_contiguous():
             raise ValueError("out must be a contiguous fp16 vector with one element per entry")
-        _lib.launch(self._index, self.lib.trs_sddmm_plan_run, self._handle, X.data_ptr(), Y.data_ptr(), out.data_ptr(),
-                    X.shape[1])
+        _lib.launch(self._index, self.lib.trs_sddmm_plan_run_ex, self._handle, X.data_ptr(), Y.data_ptr(), out.data_ptr(),
+                    X.shape[1], 0 if out.dtype is torch.float32 else 1)
         return out
 
     def close(self):
