@@ -180,16 +180,19 @@ struct Copier {
         start(list, true);
         const int total = (int)list.size();
         cudaError_t e = cudaSuccess;
-        int issued = 0;
-        for (int i = 0; i < total && e == cudaSuccess; ++i) {
-            for (; issued < total && issued < i + kSlots && e == cudaSuccess; ++issued) {
+        // Chunks go out as slots come free, arrived ones go to the workers at once, and neither waits for the other: with the
+        // next arrival held back until a slot was free the workers took turns, 48 MB in 2.46 ms instead of 1.25.
+        for (int issued = 0, arrived = 0; arrived < total && e == cudaSuccess;) {
+            if (issued < total && issued == arrived && issued >= kSlots) wait_done(done[issued - kSlots]);
+            while (issued < total && e == cudaSuccess && (issued < kSlots || done[issued - kSlots].load(std::memory_order_acquire))) {
                 const int s = issued % kSlots;
-                if (issued >= kSlots) wait_done(done[issued - kSlots]);
                 e = cudaMemcpyAsync(ring + (size_t)s * kChunk, list[issued].dev, list[issued].bytes, cudaMemcpyDeviceToHost, st);
                 if (e == cudaSuccess) e = cudaEventRecord(ev[s], st);
+                ++issued;
+                if (arrived < issued - 4) break;   // look at the arrivals in between
             }
-            if (e == cudaSuccess) e = cudaEventSynchronize(ev[i % kSlots]);
-            if (e == cudaSuccess) allowed.store(i + 1, std::memory_order_release);
+            if (e == cudaSuccess) e = cudaEventSynchronize(ev[arrived % kSlots]);
+            if (e == cudaSuccess) allowed.store(++arrived, std::memory_order_release);
         }
         if (e != cudaSuccess) { abandon(); return (int)e; }
         for (int i = 0; i < total; ++i) wait_done(done[i]);
