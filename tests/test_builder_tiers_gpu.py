@@ -48,3 +48,23 @@ def test_key_widths(bits):
     rp, col, val = _window(40, True, 1 << bits, 3)
     for empty_rows in (0, 16 * 40000):
         _check(torch.cat([rp, rp[-1:].expand(empty_rows)]), col, val)
+
+
+@pytest.mark.parametrize("window", [16, 5])
+@pytest.mark.parametrize("entries", [1, 63, 255, 256, 257, 1023, 1024, 1025, 4095, 4096, 4097, 9000])
+def test_sort_class_borders(entries, window):
+    """A window with exactly that many entries between small and empty ones: sorted by a CTA of the class, or (beyond 4096)
+    by the device-wide passes; columns shared by many rows and columns of one row."""
+    g = torch.Generator().manual_seed(entries)
+    n_cols = max(2 * entries // window, 3 * window)
+    rows = torch.arange(entries) % window + window                       # the second window
+    cols = torch.empty(entries, dtype=torch.int64)
+    for r in range(window):
+        at = rows == window + r
+        cols[at] = torch.randperm(n_cols, generator=g)[:int(at.sum())]
+    rows = torch.cat([rows, torch.tensor([0, 3 * window, 4 * window + 1])])
+    cols = torch.cat([cols, torch.tensor([n_cols - 1, 0, 5])])
+    order = torch.argsort(rows * n_cols + cols)
+    rowptr = torch.zeros(6 * window + 1, dtype=torch.int64)
+    rowptr[1:] = torch.cumsum(torch.bincount(rows, minlength=6 * window), 0)
+    _check(rowptr.to(torch.int32), cols[order].to(torch.int32), torch.randn(entries + 3, generator=g), window=window)

@@ -4,10 +4,11 @@
 // windows serially on one CPU thread with hash maps and an O(U^2) unit graph.  Here every stage
 // is a data-parallel pass over device arrays:
 //
-//   1. key = (window, column) per entry, stable radix sort          -> per-window column lists
+//   1. windows by size: a CTA per window sorts its entries by column in shared memory (hub windows:
+//      device-wide sorts)                                          -> per-window column lists
 //      (the reference's col_info map, block_online.cpp:589-603)
-//   2. run heads -> one record per (window, column): count, 16-bit row mask, first entry
-//   3. stable sort by (window, 16 - count): the (count desc, column asc) order both funnels
+//   2. runs of equal columns -> one record per (window, column): count, 16-bit row mask, first entry
+//   3. stable sort by 16 - count: the (count desc, column asc) order both funnels
 //      use (block_online.cpp:226-230, 281-285)
 //   4. TC funnel: leading columns with count >= density in chunks of 8, kept when
 //      nnz/(window*8) >= tc_min_util (block_online.cpp:215-253).  Counts descend, so the kept chunks
@@ -25,6 +26,7 @@
 //      706-733)
 //
 // Input contract: canonical CSR (columns strictly ascending inside a row), window in 1..16.
+#include <cub/block/block_radix_sort.cuh>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_select.cuh>
@@ -52,113 +54,338 @@ struct BuildCfg {
 };
 
 // ---------------------------------------------------------------------------------------------
-// 0. the sizes and the row pointers: one pass, one read-back
+// 0. the sizes, the row pointers and the windows by size: one pass, one read-back
 // ---------------------------------------------------------------------------------------------
+// Size classes of windows by number of entries: sorted by one CTA in shared memory up to sort_cap(2), by
+// device-wide passes over all larger ones together beyond (hub windows).
+constexpr int kSortClasses = 3;
+__host__ __device__ constexpr int sort_cap(int c) { return 256 << (2 * c); }   // 256, 1024, 4096
+
 struct InputInfo {
     int first, last;  // rowptr[0], rowptr[n_rows]
     int max_col;
     int err;          // 1: decreasing row pointer, 2: columns negative, not ascending or repeated
+    int windows[kSortClasses + 1];   // windows per class, hubs last
+    int pad;
+    u64 hub_entries;
 };
 
-__global__ void kb_input_info(const int* __restrict__ rowptr, const int* __restrict__ col, int n_rows,
-                              InputInfo* __restrict__ info) {
+__global__ void kb_input_info(const int* __restrict__ rowptr, const int* __restrict__ col, int n_rows, int window, int W,
+                              int* __restrict__ sel /* [kSortClasses + 1][W] */, InputInfo* __restrict__ info) {
     const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
     const int first = rowptr[0], nnz = rowptr[n_rows];
     if (t0 == 0) { info->first = first; info->last = nnz; }
     bool bad = false;
     for (long long r = t0; r < n_rows; r += step) bad |= rowptr[r + 1] < rowptr[r];
     if (bad) atomicOr(&info->err, 1);
+    const int lane = threadIdx.x & 31;
+    for (long long w0 = t0 - lane; w0 < W; w0 += step) {   // whole warps
+        const long long w = w0 + lane;
+        long long n = 0;
+        if (w < W) n = (long long)rowptr[min((w + 1) * window, (long long)n_rows)] - rowptr[w * window];
+        int c = kSortClasses + 1;   // empty: no class
+        if (n > 0) {
+            c = kSortClasses;
+            for (int i = kSortClasses - 1; i >= 0; --i)
+                if (n <= sort_cap(i)) c = i;
+        }
+        for (int i = 0; i <= kSortClasses; ++i) {
+            const unsigned in = __ballot_sync(0xffffffffu, c == i);
+            if (!in) continue;
+            int at = 0;
+            if (lane == 0) at = atomicAdd(&info->windows[i], __popc(in));
+            at = __shfl_sync(0xffffffffu, at, 0);
+            if (c == i) sel[(size_t)i * W + at + __popc(in & ((1u << lane) - 1u))] = (int)w;
+        }
+        if (c == kSortClasses) atomicAdd(&info->hub_entries, (u64)n);
+    }
     if (first != 0 || !col) return;
     int m = -1;
     for (long long e = t0; e < nnz; e += step) m = max(m, col[e]);
     m = __reduce_max_sync(0xffffffffu, m);
-    if ((threadIdx.x & 31) == 0 && m > info->max_col) atomicMax(&info->max_col, m);
+    if (lane == 0 && m > info->max_col) atomicMax(&info->max_col, m);
 }
 
 // ---------------------------------------------------------------------------------------------
-// 1. keys.  The payload of an entry is (entry << 4 | local row) while entries fit 28 bits: the sort
-// is stable and entries come in row order, so the rows of a column stay ascending without sorting
-// by them.  Longer inputs carry the entry alone and look its row up.
+// 1. - 3. the columns of every window
 // ---------------------------------------------------------------------------------------------
-constexpr int kKeyItems = 8;
-
-template <class Key, bool PACKED>
-__global__ void __launch_bounds__(256) kb_make_keys(const int* __restrict__ rowptr, const int* __restrict__ col, int n_rows,
-                                                    int nnz, int window, int col_bits, Key* __restrict__ keys,
-                                                    unsigned* __restrict__ ent, InputInfo* __restrict__ info) {
-    // rows of this CTA's entries
-    __shared__ int s_lo, s_hi;
-    const long long e0 = (long long)blockIdx.x * (256 * kKeyItems);
-    const long long e1 = min(e0 + 256 * kKeyItems, (long long)nnz);
-    if (threadIdx.x < 2) {
-        const long long e = threadIdx.x ? e1 - 1 : e0;
-        int lo = 0, hi = n_rows;  // largest r with rowptr[r] <= e
-        while (hi - lo > 1) {
-            const int mid = lo + (hi - lo) / 2;
-            if (rowptr[mid] <= e) lo = mid; else hi = mid;
-        }
-        if (threadIdx.x) s_hi = lo; else s_lo = lo;
-    }
-    __syncthreads();
-    const int rlo = s_lo, rhi = s_hi + 1;
-    bool bad = false;
-#pragma unroll
-    for (int i = 0; i < kKeyItems; ++i) {
-        const long long e = e0 + i * 256 + threadIdx.x;
-        if (e >= e1) break;
-        int lo = rlo, hi = rhi;
-        while (hi - lo > 1) {
-            const int mid = lo + (hi - lo) / 2;
-            if (rowptr[mid] <= e) lo = mid; else hi = mid;
-        }
-        const int c = col[e];
-        bad |= c < 0 || (e + 1 < rowptr[lo + 1] && col[e + 1] <= c);
-        const int w = lo / window;
-        keys[e] = ((Key)w << col_bits) | (Key)(unsigned)c;
-        ent[e] = PACKED ? ((unsigned)e << 4) | (unsigned)(lo - w * window) : (unsigned)e;
-    }
-    if (bad) atomicOr(&info->err, 2);
-}
-
-// 2. first entry of every (window, column) record
-template <class Key>
-struct IsHead {
-    const Key* keys;
-    __device__ __forceinline__ bool operator()(int i) const { return i == 0 || keys[i] != keys[i - 1]; }
-};
-
+// The entries of a window are contiguous in the input, so a window's part of every array below starts at
+// the index of its first entry, and no global position has to be found.  What comes out, per window:
+//   rec    one record per column, in (count desc, column asc) order
+//   cnt    their counts
+//   sval   the values in (column, row) order; record r's are sval[r.start .. r.start + count)
+//   ncol   how many records
 struct __align__(16) Record {   // one (window, column): its first sorted entry, the rows it has, the first value
     int col, start;
     unsigned mask;
     float value;
 };
 
-template <class Key, bool PACKED>
-__global__ void kb_records(const Key* __restrict__ keys, const unsigned* __restrict__ ent, const int* __restrict__ rowptr,
-                           const float* __restrict__ val, int n_rows, int window, const int* __restrict__ wc_start, int D,
-                           int nnz, int col_bits, Record* __restrict__ record, unsigned* __restrict__ key2, int* __restrict__ ord) {
+struct WindowOut {
+    Record* rec;
+    unsigned char* cnt;
+    float* sval;
+    int* ncol;
+};
+
+// One CTA per window of at most T * I entries.  A stable block sort by column (entries come in row order, so the rows
+// of a column stay ascending) and one by count, everything in between in shared memory: 12 bytes read and 4 + 17
+// per column written per entry.  Device-wide sorts of (window, column) keys with their key, head and record passes
+// moved ten times that and took 0.69 of the 1.30 ms of a build of the clustered graph; this takes 0.26 ms.  Its bound is
+// the shared-memory pipe and issue, in the digit passes: 5-bit and 6-bit digits, 64 and 256 threads with the same
+// number of entries measured 275 to 322 us against 262.
+template <int T, int I, int RB>
+struct WindowSort {
+    static constexpr int N = T * I, CHUNKS = N / 32;
+    using Sort = cub::BlockRadixSort<unsigned, T, I, unsigned short, RB>;
+    struct Smem {
+        union {
+            typename Sort::TempStorage sort;
+            unsigned short place[16 * CHUNKS];   // records of a count in a chunk of 32, then where they go
+        };
+        alignas(16) unsigned key[N];
+        unsigned short idx[N];     // local row << 12 | place in the window
+        unsigned short start[N];   // of the records
+        unsigned mask[N / 2];      // of the records, two in a word
+        int chunk[CHUNKS];         // records that begin in a chunk of 32 entries, then before it
+        int bound[17];             // first entry of every row
+        int warp_sum[T / 32];
+    };
+};
+
+template <int T, int I, int RB>
+__global__ void __launch_bounds__(T) kb_sort_window(const int* __restrict__ rowptr, const int* __restrict__ col,
+                                                    const float* __restrict__ val, int n_rows, int window, int col_bits,
+                                                    const int* __restrict__ sel, WindowOut out, InputInfo* __restrict__ info) {
+    using S = WindowSort<T, I, RB>;
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    typename S::Smem& s = *reinterpret_cast<typename S::Smem*>(smem_raw);
+    static_assert(S::N <= 4096, "the place in the window takes 12 bits");
+    const int tid = threadIdx.x, lane = tid & 31;
+    const int w = sel[blockIdx.x];
+    if (tid < 17) s.bound[tid] = rowptr[min((long long)w * window + min(tid, window), (long long)n_rows)];
+    __syncthreads();
+    const int base = s.bound[0], n = s.bound[16] - base;
+    const unsigned pad = (unsigned)((1ull << col_bits) - 1ull);   // padding stays last: it comes last and the sort is stable
+    for (int i = tid; i < S::N; i += T) s.key[i] = i < n ? (unsigned)col[base + i] : pad;
+    for (int i = tid; i < S::N / 2; i += T) s.mask[i] = 0u;
+    __syncthreads();
+    unsigned key[I];
+    unsigned short idx[I];
+    {
+        const int i0 = tid * I;
+#pragma unroll
+        for (int k = 0; k < I; k += 4) {
+            const uint4 x = *(const uint4*)(s.key + i0 + k);
+            key[k] = x.x; key[k + 1] = x.y; key[k + 2] = x.z; key[k + 3] = x.w;
+        }
+        const unsigned next = i0 + I < S::N ? s.key[i0 + I] : pad;
+        int row = 0;
+#pragma unroll
+        for (int d = 8; d; d >>= 1)
+            if (row + d < window && s.bound[row + d] - base <= i0) row += d;
+        int row_end = s.bound[row + 1] - base;
+        bool bad = false;
+#pragma unroll
+        for (int k = 0; k < I; ++k) {
+            const int i = i0 + k;
+            while (i >= row_end && row + 1 < window) row_end = s.bound[++row + 1] - base;
+            idx[k] = (unsigned short)(row << 12 | i);
+            if (i < n) bad |= key[k] > pad || (i + 1 < row_end && (k + 1 < I ? key[k + 1 < I ? k + 1 : k] : next) <= key[k]);
+        }
+        if (bad) atomicOr(&info->err, 2);
+    }
+    __syncthreads();
+    typename S::Sort(s.sort).SortBlockedToStriped(key, idx, 0, col_bits);
+    // sorted entry k * T + tid is this thread's k-th: a warp holds chunks of 32 neighbours
+#pragma unroll
+    for (int k = 0; k < I; ++k) {
+        s.key[k * T + tid] = key[k];
+        s.idx[k * T + tid] = idx[k];
+    }
+    __syncthreads();
+    // records begin where the column changes
+    unsigned heads[I];
+#pragma unroll
+    for (int k = 0; k < I; ++k) {
+        const int i = k * T + tid;
+        heads[k] = __ballot_sync(0xffffffffu, i < n && (i == 0 || s.key[i > 0 ? i - 1 : 0] != key[k]));
+        if (lane == 0) s.chunk[i >> 5] = __popc(heads[k]);
+    }
+    __syncthreads();
+    if (tid < 32) {
+        int before = 0;
+        for (int c0 = 0; c0 < S::CHUNKS; c0 += 32) {
+            const int x = c0 + lane < S::CHUNKS ? s.chunk[c0 + lane] : 0;
+            int sum = x;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const int y = __shfl_up_sync(0xffffffffu, sum, d);
+                if (lane >= d) sum += y;
+            }
+            if (c0 + lane < S::CHUNKS) s.chunk[c0 + lane] = before + sum - x;
+            before += __shfl_sync(0xffffffffu, sum, 31);
+        }
+        if (lane == 0) s.warp_sum[0] = before;
+    }
+    __syncthreads();
+    const int D = s.warp_sum[0];
+#pragma unroll
+    for (int k = 0; k < I; ++k) {
+        const int i = k * T + tid;
+        if (i - lane >= n) break;
+        const unsigned upto = heads[k] & (0xffffffffu >> (31 - lane));
+        const int r = s.chunk[i >> 5] + __popc(upto) - 1, seg = upto ? 31 - __clz(upto) : 0;   // no head yet: a record goes on
+        unsigned m = i < n ? 1u << (idx[k] >> 12) : 0u;
+#pragma unroll
+        for (int d = 1; d < 16; d <<= 1) {   // at most 16 entries share a column
+            const unsigned y = __shfl_up_sync(0xffffffffu, m, d);
+            if (lane - d >= seg) m |= y;
+        }
+        if (i < n) {
+            if ((heads[k] >> lane) & 1u) s.start[r] = (unsigned short)i;
+            if (lane == 31 || i + 1 == n || ((heads[k] >> (lane + 1)) & 1u)) atomicOr(&s.mask[r >> 1], m << (16 * (r & 1)));
+        }
+    }
+    for (int i = tid; i < n; i += T) out.sval[base + i] = val[base + (s.idx[i] & 0xfff)];
+    __syncthreads();
+    const unsigned short* const masks = (const unsigned short*)s.mask;
+    const int chunks = (D + 31) / 32, cells = 16 * chunks;
+    for (int i = tid; i < cells; i += T) s.place[i] = 0;   // the sort's memory: its last readers are barriers back
+    __syncthreads();
+    // (count desc, column asc): records keep their order inside a count, so a record's place is the number of records of
+    // larger counts, of its count in earlier chunks of 32, and of its count before it in its own chunk
+    const unsigned lt = (1u << lane) - 1u;
+    for (int c = tid >> 5; c < chunks; c += T / 32) {
+        const int q = c * 32 + lane;
+        const int k = q < D ? 16 - __popc((unsigned)masks[q]) : 16;
+        const unsigned same = __match_any_sync(0xffffffffu, k);
+        if (k < 16 && (same & lt) == 0) s.place[k * chunks + c] = (unsigned short)__popc(same);
+    }
+    __syncthreads();
+    int before = 0;   // exclusive sums over the cells, T at a time
+    for (int c0 = 0; c0 < cells; c0 += T) {
+        const int i = c0 + tid, x = i < cells ? s.place[i] : 0;
+        int sum = x;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, sum, d);
+            if (lane >= d) sum += y;
+        }
+        if (lane == 31) s.warp_sum[tid >> 5] = sum;
+        __syncthreads();
+        int at = before + sum - x;
+#pragma unroll
+        for (int q = 0; q < T / 32; ++q) {
+            if (q < (tid >> 5)) at += s.warp_sum[q];
+            before += s.warp_sum[q];
+        }
+        if (i < cells) s.place[i] = (unsigned short)at;
+        __syncthreads();
+    }
+    for (int c = tid >> 5; c < chunks; c += T / 32) {
+        const int q = c * 32 + lane;
+        const int k = q < D ? 16 - __popc((unsigned)masks[q]) : 16;
+        const unsigned same = __match_any_sync(0xffffffffu, k);
+        if (k == 16) continue;
+        const int st = s.start[q];
+        const size_t o = (size_t)base + s.place[k * chunks + c] + __popc(same & lt);
+        out.rec[o] = Record{(int)s.key[st], base + st, masks[q], val[base + (s.idx[st] & 0xfff)]};
+        out.cnt[o] = (unsigned char)(16 - k);
+    }
+    if (tid == 0) out.ncol[w] = D;
+}
+
+// Hub windows: the same through device-wide sorts, keys (hub << col_bits | column), payload the place in the window.
+struct HubView {
+    const int* sel;   // [H] windows
+    const int* off;   // [H + 1] first entry in the compact arrays
+    int n;
+};
+__device__ __forceinline__ int find_hub(const HubView& h, int x) {
+    int lo = 0, hi = h.n;
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (h.off[mid] <= x) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+// local row of an entry: rows of the window that start at or before it
+__device__ __forceinline__ int local_row(const int* __restrict__ rowptr, int n_rows, int w, int window, int e) {
+    int lo = 0, hi = min(window, n_rows - w * window);
+    while (hi - lo > 1) {
+        const int mid = (lo + hi) >> 1;
+        if (rowptr[w * window + mid] <= e) lo = mid; else hi = mid;
+    }
+    return lo;
+}
+
+__global__ void kb_hub_sizes(const int* __restrict__ rowptr, int n_rows, int window, const int* __restrict__ sel, int H,
+                             int* __restrict__ size) {
+    const int h = blockIdx.x * blockDim.x + threadIdx.x;
+    if (h > H) return;
+    size[h] = h < H ? rowptr[min((long long)(sel[h] + 1) * window, (long long)n_rows)] - rowptr[(size_t)sel[h] * window] : 0;
+}
+
+template <class Key>
+__global__ void kb_hub_keys(const int* __restrict__ rowptr, const int* __restrict__ col, int n_rows, int window, HubView hub, int E,
+                            int col_bits, Key* __restrict__ keys, int* __restrict__ place, InputInfo* __restrict__ info) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= E) return;
+    const int h = find_hub(hub, x), w = hub.sel[h];
+    const int at = x - hub.off[h], e = rowptr[(size_t)w * window] + at;
+    const int c = col[e], r = w * window + local_row(rowptr, n_rows, w, window, e);
+    if (c < 0 || (e + 1 < rowptr[r + 1] && col[e + 1] <= c)) atomicOr(&info->err, 2);
+    keys[x] = ((Key)h << col_bits) | (Key)(unsigned)max(c, 0);
+    place[x] = at;
+}
+
+template <class Key>
+struct IsHead {
+    const Key* keys;
+    __device__ __forceinline__ bool operator()(int i) const { return i == 0 || keys[i] != keys[i - 1]; }
+};
+
+template <class Key>
+__global__ void kb_hub_records(const Key* __restrict__ keys, const int* __restrict__ place, const int* __restrict__ rowptr,
+                               const float* __restrict__ val, int n_rows, int window, HubView hub, const int* __restrict__ start,
+                               int D, int E, int col_bits, Record* __restrict__ record, unsigned* __restrict__ key2,
+                               int* __restrict__ ord, int* __restrict__ first_rec) {
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= D) return;
-    const int b = wc_start[j], e = j + 1 < D ? wc_start[j + 1] : nnz;
-    const Key k = keys[b];
-    const int w = (int)(k >> col_bits);
+    const int b = start[j], e = j + 1 < D ? start[j + 1] : E;
+    const int h = (int)(keys[b] >> col_bits), w = hub.sel[h];
+    const int base = rowptr[(size_t)w * window];
     unsigned mask = 0;
-    for (int i = b; i < e; ++i) {
-        const unsigned v = ent[i];
-        int lr = (int)(v & 15u);
-        if (!PACKED) {
-            lr = 0;
-            for (int r = 1; r < window && w * window + r < n_rows; ++r) lr += rowptr[w * window + r] <= (int)v;
-        }
-        mask |= 1u << lr;
-    }
-    record[j] = Record{(int)(k & (((Key)1 << col_bits) - 1)), b, mask, val[PACKED ? ent[b] >> 4 : ent[b]]};
-    key2[j] = ((unsigned)w << 4) | (unsigned)(16 - (e - b));
+    for (int i = b; i < e; ++i) mask |= 1u << local_row(rowptr, n_rows, w, window, base + place[i]);
+    record[j] = Record{(int)(keys[b] & (((Key)1 << col_bits) - 1)), base + b - hub.off[h], mask, val[base + place[b]]};
+    key2[j] = ((unsigned)h << 4) | (unsigned)(16 - (e - b));
     ord[j] = j;
+    if (b == hub.off[h]) first_rec[h] = j;
+}
+
+__global__ void kb_hub_place(const unsigned* __restrict__ key2, const int* __restrict__ ord, const Record* __restrict__ record, int D,
+                             const int* __restrict__ rowptr, int window, HubView hub, const int* __restrict__ first_rec, WindowOut out) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= D) return;
+    const unsigned k = key2[p];
+    const int h = (int)(k >> 4), w = hub.sel[h], o = p - first_rec[h];
+    const size_t at = (size_t)rowptr[(size_t)w * window] + o;
+    out.rec[at] = record[ord[p]];
+    out.cnt[at] = (unsigned char)(16u - (k & 15u));
+    if (p + 1 == D || (key2[p + 1] >> 4) != (unsigned)h) out.ncol[w] = o + 1;
+}
+
+__global__ void kb_hub_values(const int* __restrict__ place, const int* __restrict__ rowptr, const float* __restrict__ val, int window,
+                              HubView hub, int E, float* __restrict__ sval) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= E) return;
+    const int h = find_hub(hub, x), base = rowptr[(size_t)hub.sel[h] * window];
+    sval[base + x - hub.off[h]] = val[base + place[x]];
 }
 
 // ---------------------------------------------------------------------------------------------
-// 3. - 5. per window: records, TC columns, units, pair slots, TC blocks, TC parts
+// 4., 5. per window: TC columns, units, pair slots, TC blocks, TC parts
 // ---------------------------------------------------------------------------------------------
 struct Win {          // prefixes over windows (W + 1 of them) after the scan
     int blocks, units, slots, parts;
@@ -169,7 +396,8 @@ struct WinSum {
     }
 };
 struct WindowView {
-    const int* rec;    // [W + 1] first record of the window
+    const int* rec;    // [W] first record of the window
+    const int* end;    // [W] behind its last one
     const int* tc;     // [W] TC columns: records [rec, rec + tc) in (count desc, column asc) order
     const Win* pre;    // [W + 1]
 };
@@ -181,29 +409,23 @@ constexpr int kSmemUnits = 52224;
 struct MatchCounts {
     int n_block, n_huge;
     int max_warp, max_huge;   // units of the largest window of the warp and of the last tier
+    u64 records;
 };
 
-__global__ void kb_windows(const int* __restrict__ wc_start, const unsigned* __restrict__ key2, const int* __restrict__ rowptr,
-                           int n_rows, int D, int W, BuildCfg cfg, int* __restrict__ rec, int* __restrict__ tc,
+__global__ void kb_windows(const int* __restrict__ rowptr, const int* __restrict__ ncol, const unsigned char* __restrict__ cnt,
+                           int W, BuildCfg cfg, int* __restrict__ rec, int* __restrict__ end, int* __restrict__ tc,
                            Win* __restrict__ win, int* __restrict__ sel_block, int* __restrict__ sel_huge,
                            MatchCounts* __restrict__ mc) {
     const int w = blockIdx.x * blockDim.x + threadIdx.x;
+    const int n = w < W ? ncol[w] : 0;
+    const int sum = __reduce_add_sync(0xffffffffu, n);
+    if ((threadIdx.x & 31) == 0 && sum) atomicAdd(&mc->records, (u64)sum);
     if (w > W) return;
-    auto first_record = [&](int x) -> int {  // records of windows < x: the first one starts where the window's entries do
-        if (x >= W) return D;
-        const int e = rowptr[x * cfg.window];
-        int lo = 0, hi = D;
-        while (lo < hi) {
-            const int mid = lo + (hi - lo) / 2;
-            if (wc_start[mid] < e) lo = mid + 1; else hi = mid;
-        }
-        return lo;
-    };
-    const int b = first_record(w);
-    rec[w] = b;
     if (w == W) { win[W] = Win{0, 0, 0, 0}; return; }
-    const int n = first_record(w + 1) - b;
-    auto count = [&](int o) -> int { return 16 - (int)(key2[b + o] & 15u); };  // o-th largest column
+    const int b = rowptr[(size_t)w * cfg.window];
+    rec[w] = b;
+    end[w] = b + n;
+    auto count = [&](int o) -> int { return cnt[b + o]; };  // o-th largest column
     int cand = 0;
     if (!cfg.skip_tc) {
         int lo = 0, hi = n;
@@ -487,9 +709,9 @@ struct MatchOut {
     int* cuda_unit;   // [W] unmatched unit that goes to the CUDA cores, -1: none
 };
 
-__device__ __forceinline__ int unit_word(const unsigned* __restrict__ key2, int rec0, int ncol, int u) {
-    int nnz = 16 - (int)(key2[rec0 + 2 * u] & 15u);
-    if (2 * u + 1 < ncol) nnz += 16 - (int)(key2[rec0 + 2 * u + 1] & 15u);
+__device__ __forceinline__ int unit_word(const unsigned char* __restrict__ cnt, int rec0, int ncol, int u) {
+    int nnz = cnt[rec0 + 2 * u];
+    if (2 * u + 1 < ncol) nnz += cnt[rec0 + 2 * u + 1];
     return (int)(((unsigned)nnz << kUnitBits) | (unsigned)u);
 }
 
@@ -512,7 +734,7 @@ struct MatchWarpSmem {
 
 // Windows of at most `max_units` units, one warp each.  Dynamic shared memory: per warp max_units words
 // and the bitmask.
-__global__ void __launch_bounds__(32 * kMatchWarps) kb_match_warp(WindowView v, int W, const unsigned* __restrict__ key2,
+__global__ void __launch_bounds__(32 * kMatchWarps) kb_match_warp(WindowView v, int W, const unsigned char* __restrict__ cnt,
                                                                   int unit_min_nnz, int max_units, MatchOut o) {
     extern __shared__ int dyn[];
     __shared__ MatchWarpSmem s_warp[kMatchWarps];
@@ -523,11 +745,11 @@ __global__ void __launch_bounds__(32 * kMatchWarps) kb_match_warp(WindowView v, 
     const Win p0 = v.pre[w];
     const int U = v.pre[w + 1].units - p0.units;
     if (U > max_units) return;
-    const int rec0 = v.rec[w] + v.tc[w], ncol = v.rec[w + 1] - rec0;
+    const int rec0 = v.rec[w] + v.tc[w], ncol = v.end[w] - rec0;
     int* a = dyn + wid * (max_units + (max_units + 31) / 32);
     unsigned* freem = (unsigned*)(a + max_units);
     int* order = o.order + p0.units;
-    for (int i = lane; i < U; i += 32) a[i] = unit_word(key2, rec0, ncol, i);
+    for (int i = lane; i < U; i += 32) a[i] = unit_word(cnt, rec0, ncol, i);
     for (int i = lane; i < (U + 31) / 32; i += 32) freem[i] = U - 32 * i >= 32 ? 0xffffffffu : (1u << (U - 32 * i)) - 1u;
     __syncwarp();
     MatchWarpSmem& m = s_warp[wid];
@@ -540,7 +762,7 @@ __global__ void __launch_bounds__(32 * kMatchWarps) kb_match_warp(WindowView v, 
     __syncwarp();   // `order` is read back by the lanes of the warp that wrote it
     int left;
     const int G = warp_greedy(U, freem, order, o.pair_a + p0.slots, o.pair_b + p0.slots, m.sl, lane, &left);
-    if (lane == 0) match_finish(w, G, left, left >= 0 ? (int)unit_key(unit_word(key2, rec0, ncol, left)) : 0, unit_min_nnz, o, p0.slots);
+    if (lane == 0) match_finish(w, G, left, left >= 0 ? (int)unit_key(unit_word(cnt, rec0, ncol, left)) : 0, unit_min_nnz, o, p0.slots);
 }
 
 // Hub windows, one block each: long ranges are partitioned or traced by the whole block, ranges of
@@ -549,7 +771,7 @@ __global__ void __launch_bounds__(32 * kMatchWarps) kb_match_warp(WindowView v, 
 // (or `mask_global`).
 constexpr int kBlockThreads = 256, kWarpRange = 1024, kMaxRanges = 256;
 
-__global__ void __launch_bounds__(kBlockThreads) kb_match_block(WindowView v, const unsigned* __restrict__ key2, int unit_min_nnz,
+__global__ void __launch_bounds__(kBlockThreads) kb_match_block(WindowView v, const unsigned char* __restrict__ cnt, int unit_min_nnz,
                                                                 int smem_units, int* __restrict__ words_global,
                                                                 unsigned* __restrict__ mask_global, const int* __restrict__ sel,
                                                                 MatchOut o) {
@@ -562,13 +784,13 @@ __global__ void __launch_bounds__(kBlockThreads) kb_match_block(WindowView v, co
     const int w = sel[blockIdx.x];
     const Win p0 = v.pre[w];
     const int U = v.pre[w + 1].units - p0.units;
-    const int rec0 = v.rec[w] + v.tc[w], ncol = v.rec[w + 1] - rec0;
+    const int rec0 = v.rec[w] + v.tc[w], ncol = v.end[w] - rec0;
     const bool in_smem = U <= smem_units;
     int* a = in_smem ? dyn : words_global + p0.units;
     int* order = o.order + p0.units;
     int* swapL = o.pair_a + p0.slots;   // scratch during the sort, pair list afterwards
     int* swapR = o.pair_b + p0.slots;
-    for (int i = tid; i < U; i += kBlockThreads) a[i] = unit_word(key2, rec0, ncol, i);
+    for (int i = tid; i < U; i += kBlockThreads) a[i] = unit_word(cnt, rec0, ncol, i);
     if (tid == 0) {
         s_stack[0] = SortRange{0, U, 2 * StdSort<UnitWordLess>::floor_log2(U)};
         s_sp = 1; s_nsmall = 0;
@@ -717,7 +939,7 @@ __global__ void __launch_bounds__(kBlockThreads) kb_match_block(WindowView v, co
     int left;
     const int G = mask_in_smem ? warp_greedy(U, (unsigned*)dyn, order, swapL, swapR, s_warp[0].sl, lane, &left)
                                : warp_greedy(U, gmask, order, swapL, swapR, s_warp[0].sl, lane, &left);
-    if (lane == 0) match_finish(w, G, left, left >= 0 ? (int)unit_key(unit_word(key2, rec0, ncol, left)) : 0, unit_min_nnz, o, p0.slots);
+    if (lane == 0) match_finish(w, G, left, left >= 0 ? (int)unit_key(unit_word(cnt, rec0, ncol, left)) : 0, unit_min_nnz, o, p0.slots);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -733,14 +955,10 @@ __global__ void kb_tiles(const int* __restrict__ tile_off, const int* __restrict
 }
 
 struct RecordView {
-    const int* ord;               // records in (window, count desc, column asc) order
-    const Record* rec;            // by record id
-    const unsigned* ent;          // sorted entries
-    const float* val;             // CSR values
-    int packed;                   // entries are (entry << 4 | local row)
-    __device__ __forceinline__ int entry(int at) const { return (int)(packed ? ent[at] >> 4 : ent[at]); }
+    const Record* rec;
+    const float* sval;
     // value of the record's k-th entry (most records of a power-law graph have one)
-    __device__ __forceinline__ float value(int start, float first, int k) const { return k == 0 ? first : val[entry(start + k)]; }
+    __device__ __forceinline__ float value(int start, float first, int k) const { return k == 0 ? first : sval[start + k]; }
 };
 
 struct GroupOut {
@@ -760,14 +978,22 @@ constexpr int kDropCounters = 64;
 struct ExtraOut {
     u64* count; // strict: length of the list; otherwise kDropCounters counters, one per block number modulo
     u64* key;
-    int* at;    // entry
+    int* at;    // place in sval
 };
 
 // One warp per tile of four groups: lane (q, g) = (lane / 8, lane % 8) owns rows g and g + 8 of group q,
 // which are also the two rows of its word pair in the packed tile.  One pass writes the un-packed arrays
-// (196 bytes per group) and the tile (352 bytes); reading the un-packed arrays back to pack them, and an
-// atomic per dropped entry, were most of the 0.63 ms the separate kernels took on the clustered
-// graph (0.09 ms now).
+// (196 bytes per group) and the tile (352 bytes).  What bounds it is instruction issue: the four records of a group
+// are loaded by one lane each, ranked by column with three shuffles and read back from shared memory by
+// position; the positions of a row's first two entries, and the tile's metadata for them, come from tables
+// indexed by the row's occupancy pattern.  With all four records in every lane's registers, sorted by a network
+// and picked by selects, a tile took 590 instructions instead of 320 (clustered graph: 270 against 159 us).
+constexpr unsigned kFirstPos = 0x12131210u;          // 2 bits per pattern: position of the first entry
+constexpr unsigned kSecondPos = 0x6b7c6840u;         // of the second
+constexpr u64 kTilePos = 0x498e4dcc49884444ull;      // 4 bits: p0 | p1 << 2, the tile's two kept positions p0 < p1 (a
+                                                     // missing entry gets a position holding 0.0)
+constexpr unsigned kLoneLater = 0x114u;              // patterns with one entry, not in position 0: it is the second kept one
+
 template <bool STRICT>
 __global__ void __launch_bounds__(256) kb_emit_tiles(WindowView v, RecordView r, const int* __restrict__ s_offset,
                                                      const int* __restrict__ tile_window, const int* __restrict__ tile_group,
@@ -778,6 +1004,7 @@ __global__ void __launch_bounds__(256) kb_emit_tiles(WindowView v, RecordView r,
     constexpr int kWait = STRICT ? 256 : 1;
     __shared__ u64 s_key[8][kWait];
     __shared__ int s_at[8][kWait];
+    __shared__ Record s_rec[8][4][4];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, q = lane >> 3, g = lane & 7;
     int waiting = 0;
     auto flush = [&]() {
@@ -793,113 +1020,59 @@ __global__ void __launch_bounds__(256) kb_emit_tiles(WindowView v, RecordView r,
     for (int t = blockIdx.x * 8 + wid; t < T; t += gridDim.x * 8) {
         const int w = tile_window[t];
         const int gid = tile_group[t] + q;
-        const int off = s_offset[w];
         const bool live = gid < s_offset[w + 1];
-        // the group's columns, ascending
-        float first[4];
-        int st[4], col[4] = {0x7fffffff, 0x7fffffff, 0x7fffffff, 0x7fffffff};
-        unsigned m[4] = {0u, 0u, 0u, 0u};
-        int n = 0;
-        if (live) {
-            const int slot = v.pre[w].slots + gid - off;
-            const int rec0 = v.rec[w] + v.tc[w], ncol = v.rec[w + 1] - rec0;
-            const int u[2] = {pair_a[slot], pair_b[slot]};
-#pragma unroll
-            for (int i = 0; i < 4; ++i) {
-                const int ls = 2 * u[i >> 1] + (i & 1);
-                if (u[i >> 1] >= 0 && ls < ncol) {
-                    const Record c = r.rec[r.ord[rec0 + ls]];
-                    col[i] = c.col; st[i] = c.start; m[i] = c.mask; first[i] = c.value;
-                    ++n;
-                }
-            }
-            auto order2 = [&](int a, int b) {
-                if (col[a] > col[b]) {
-                    int s = col[a]; col[a] = col[b]; col[b] = s;
-                    s = st[a]; st[a] = st[b]; st[b] = s;
-                    const unsigned t = m[a]; m[a] = m[b]; m[b] = t;
-                    const float f = first[a]; first[a] = first[b]; first[b] = f;
-                }
-            };
-            order2(0, 1); order2(2, 3); order2(0, 2); order2(1, 3); order2(1, 2);
+        // the group's columns, ascending: lane g < 4 brings column g
+        Record c{0x7fffffff, 0, 0u, 0.f};
+        if (live && g < 4) {
+            const int slot = v.pre[w].slots + gid - s_offset[w];
+            const int rec0 = v.rec[w] + v.tc[w], ncol = v.end[w] - rec0;
+            const int u = (g < 2 ? pair_a : pair_b)[slot], ls = 2 * u + (g & 1);
+            if (u >= 0 && ls < ncol) c = r.rec[rec0 + ls];
         }
+        int rank = 0;
 #pragma unroll
-        for (int p = 0; p < 4; ++p)
-            if (p >= n) col[p] = -1;
-        // the two kept entries of both rows: positions from bit arithmetic, then all loads side by side
-        // (a branch per position, with its dependent loads inside, took three times as long)
-        unsigned bits[2];
-        int pos[2][2], at[2][2];
-        float value[2][2];
-        bool load[2][2];
-#pragma unroll
-        for (int h = 0; h < 2; ++h) {
-            const int lr = g + 8 * h;
-            bits[h] = ((m[0] >> lr) & 1u) | (((m[1] >> lr) & 1u) << 1) | (((m[2] >> lr) & 1u) << 2) | (((m[3] >> lr) & 1u) << 3);
-            unsigned rest = bits[h];
-#pragma unroll
-            for (int i = 0; i < 2; ++i) {
-                const int p = rest ? __ffs(rest) - 1 : -1;
-                rest &= rest - 1;
-                pos[h][i] = p;
-                const unsigned mp = p == 0 ? m[0] : p == 1 ? m[1] : p == 2 ? m[2] : m[3];
-                const int k = __popc(mp & ((1u << lr) - 1u));
-                at[h][i] = (p == 0 ? st[0] : p == 1 ? st[1] : p == 2 ? st[2] : st[3]) + k;
-                value[h][i] = p < 0 ? 0.f : p == 0 ? first[0] : p == 1 ? first[1] : p == 2 ? first[2] : first[3];
-                load[h][i] = p >= 0 && k > 0;
-            }
+        for (int i = 1; i < 4; ++i) {
+            const int other = __shfl_xor_sync(0xffffffffu, c.col, i);
+            rank += other < c.col || (other == c.col && (g ^ i) < g);
         }
-        int e[2][2];
+        if (g < 4) {
+            if (c.mask == 0u) c.col = -1;
+            s_rec[wid][q][rank] = c;
+        }
+        __syncwarp();
+        const Record* const group = s_rec[wid][q];
+        // occupancy of rows g (low byte) and g + 8
+        unsigned both = 0;
 #pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int i = 0; i < 2; ++i) e[h][i] = load[h][i] ? r.entry(at[h][i]) : 0;
-#pragma unroll
-        for (int h = 0; h < 2; ++h)
-#pragma unroll
-            for (int i = 0; i < 2; ++i)
-                if (load[h][i]) value[h][i] = r.val[e[h][i]];
+        for (int p = 0; p < 4; ++p) both |= ((group[p].mask >> g) & 0x101u) << p;
         uint32_t meta = 0, word[2];
-        int n_extra = 0, extra_at[4], extra_col[4], extra_row[4];
+        int n_extra = 0;
 #pragma unroll
         for (int h = 0; h < 2; ++h) {
             const int lr = g + 8 * h;
-            dropped += max(__popc(bits[h]) - 2, 0);
-            if constexpr (STRICT) {
-                unsigned rest = bits[h] & (bits[h] - 1);
-                rest &= rest - 1;
-#pragma unroll
-                for (int i = 0; i < 2; ++i) {   // the third and fourth entry
-                    if (rest) {
-                        const int p = __ffs(rest) - 1;
-                        rest &= rest - 1;
-                        const unsigned mp = p == 2 ? m[2] : m[3];   // never the first two positions
-                        extra_at[2 * h + i] = r.entry((p == 2 ? st[2] : st[3]) + __popc(mp & ((1u << lr) - 1u)));
-                        extra_col[2 * h + i] = p == 2 ? col[2] : col[3];
-                        extra_row[2 * h + i] = w * window + lr;
-                        n_extra |= 1 << (2 * h + i);
-                    }
-                }
-            }
+            const unsigned bits = (both >> (8 * h)) & 15u, below = (1u << lr) - 1u;
+            const int slots = __popc(bits);
+            dropped += max(slots - 2, 0);
+            const int p0 = (kFirstPos >> (2 * bits)) & 3, p1 = (kSecondPos >> (2 * bits)) & 3;
+            const Record a = group[p0], b = group[p1];
+            const int ka = __popc(a.mask & below), kb = __popc(b.mask & below);
+            float va = slots > 0 ? a.value : 0.f, vb = slots > 1 ? b.value : 0.f;
+            if (slots > 0 && ka) va = r.sval[a.start + ka];
+            if (slots > 1 && kb) vb = r.sval[b.start + kb];
+            if constexpr (STRICT) n_extra |= (int)(((bits & (bits - 1u)) & ((bits & (bits - 1u)) - 1u)) >> 2) << (2 * h);
             if (live && lr < window) {
                 const size_t i = (size_t)gid * window + lr;
-                o.s_mask[i] = (unsigned char)bits[h];
-                *(float2*)(o.s_value + 2 * i) = make_float2(value[h][0], value[h][1]);
-                *(char2*)(o.s_pos + 2 * i) = make_char2((signed char)pos[h][0], (signed char)pos[h][1]);
+                o.s_mask[i] = (unsigned char)bits;
+                *(float2*)(o.s_value + 2 * i) = make_float2(va, vb);
+                *(char2*)(o.s_pos + 2 * i) = make_char2((signed char)(slots > 0 ? p0 : -1), (signed char)(slots > 1 ? p1 : -1));
             }
-            // the tile's two kept positions p0 < p1 (a missing slot gets a position holding 0.0)
-            const int slots = __popc(bits[h]);
-            int p0 = 0, p1 = 1;
-            float w0 = 0.f, w1 = 0.f;
-            if (slots >= 2) { p0 = pos[h][0]; p1 = pos[h][1]; w0 = value[h][0]; w1 = value[h][1]; }
-            else if (slots == 1) {
-                if (pos[h][0] == 0) w0 = value[h][0];
-                else { p1 = pos[h][0]; w1 = value[h][0]; }
-            }
-            meta |= (uint32_t)(p0 | (p1 << 2)) << (q * 4 + 16 * h);
-            word[h] = (uint32_t)__half_as_ushort(__float2half_rn(w0)) | ((uint32_t)__half_as_ushort(__float2half_rn(w1)) << 16);
+            meta |= (uint32_t)((kTilePos >> (4 * bits)) & 15u) << (q * 4 + 16 * h);
+            if ((kLoneLater >> bits) & 1u) { vb = va; va = 0.f; }
+            const __half2 pair = __floats2half2_rn(va, vb);
+            word[h] = *(const uint32_t*)&pair;
         }
         if constexpr (STRICT) {
+            // n_extra: bit 2 h + i says that row g + 8 h has a third or fourth entry, in position 2 + i
             int incl = __popc(n_extra);
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
@@ -910,8 +1083,10 @@ __global__ void __launch_bounds__(256) kb_emit_tiles(WindowView v, RecordView r,
 #pragma unroll
             for (int i = 0; i < 4; ++i)
                 if ((n_extra >> i) & 1) {
-                    s_key[wid][put] = ((u64)(unsigned)extra_row[i] << 32) | (unsigned)extra_col[i];
-                    s_at[wid][put] = extra_at[i];
+                    const int lr = g + 8 * (i >> 1);
+                    const Record e = group[2 + (i & 1)];
+                    s_key[wid][put] = ((u64)(unsigned)(w * window + lr) << 32) | (unsigned)e.col;
+                    s_at[wid][put] = e.start + __popc(e.mask & ((1u << lr) - 1u));
                     ++put;
                 }
             waiting += __shfl_sync(0xffffffffu, incl, 31);
@@ -922,13 +1097,14 @@ __global__ void __launch_bounds__(256) kb_emit_tiles(WindowView v, RecordView r,
         meta |= __shfl_xor_sync(0xffffffffu, meta, 16);
         if (q == 0) o.packed_meta[(size_t)t * 8 + g] = meta;
         if (g == 0) {
-            const int4 c = make_int4(col[0], col[1], col[2], col[3]);
-            *(int4*)(o.s_tile_column + (size_t)t * 16 + q * 4) = c;
+            const int4 cols = make_int4(group[0].col, group[1].col, group[2].col, group[3].col);
+            *(int4*)(o.s_tile_column + (size_t)t * 16 + q * 4) = cols;
             if (live) {
-                *(int4*)(o.s_column + (size_t)gid * 4) = c;
+                *(int4*)(o.s_column + (size_t)gid * 4) = cols;
                 o.s_window[gid] = w;
             }
         }
+        __syncwarp();   // the records are overwritten by the next tile's
     }
     if constexpr (STRICT) {
         if (waiting > 0) flush();
@@ -960,7 +1136,7 @@ __global__ void kb_tc_blocks(WindowView v, RecordView r, int W, int NB, int* __r
     const int o0 = 8 * (b - v.pre[w].blocks), len = min(8, v.tc[w] - o0);
     const int p0 = v.rec[w] + o0;
     int ids[8], cols[8];
-    for (int i = 0; i < len; ++i) { ids[i] = r.ord[p0 + i]; cols[i] = r.rec[ids[i]].col; }
+    for (int i = 0; i < len; ++i) { ids[i] = p0 + i; cols[i] = r.rec[p0 + i].col; }
     for (int i = 1; i < len; ++i) {
         const int c = cols[i], id = ids[i];
         int k = i - 1;
@@ -1022,7 +1198,7 @@ __global__ void kb_tc_parts(WindowView v, const int* __restrict__ win_cuda_unit,
 struct CudaRow {
     int n;
     int cols[2];
-    int ent[2];
+    int at[2];   // places in sval
 };
 __device__ __forceinline__ CudaRow cuda_row(int row, int window, const int* __restrict__ win_cuda_unit, const WindowView& v,
                                             const RecordView& r) {
@@ -1031,19 +1207,19 @@ __device__ __forceinline__ CudaRow cuda_row(int row, int window, const int* __re
     const int w = row / window, lr = row - w * window;
     const int u = win_cuda_unit[w];
     if (u < 0) return out;
-    const int rec0 = v.rec[w] + v.tc[w], ncol = v.rec[w + 1] - rec0;
+    const int rec0 = v.rec[w] + v.tc[w], ncol = v.end[w] - rec0;
     for (int i = 0; i < 2; ++i) {
         const int ls = 2 * u + i;
         if (ls >= ncol) break;
-        const Record c = r.rec[r.ord[rec0 + ls]];
+        const Record c = r.rec[rec0 + ls];
         if (!((c.mask >> lr) & 1u)) continue;
         out.cols[out.n] = c.col;
-        out.ent[out.n] = r.entry(c.start + __popc(c.mask & ((1u << lr) - 1u)));
+        out.at[out.n] = c.start + __popc(c.mask & ((1u << lr) - 1u));
         ++out.n;
     }
     if (out.n == 2 && out.cols[0] > out.cols[1]) {
         int t = out.cols[0]; out.cols[0] = out.cols[1]; out.cols[1] = t;
-        t = out.ent[0]; out.ent[0] = out.ent[1]; out.ent[1] = t;
+        t = out.at[0]; out.at[0] = out.at[1]; out.at[1] = t;
     }
     return out;
 }
@@ -1141,7 +1317,7 @@ __global__ void kb_cuda_rows(int n_rows, int window, int part_c, int short_size,
             const int mid = lo + (hi - lo) / 2;
             if ((int)(x.key[mid] & 0xffffffffull) < cr.cols[i]) lo = mid + 1; else hi = mid;
         }
-        po.put(o, row_long, i + lo - xb, cr.cols[i], r.val[cr.ent[i]]);
+        po.put(o, row_long, i + lo - xb, cr.cols[i], r.sval[cr.at[i]]);
     }
 }
 
@@ -1154,7 +1330,7 @@ __global__ void kb_cuda_extras(int window, const int* __restrict__ win_cuda_unit
     const CudaRow cr = cuda_row(row, window, win_cuda_unit, v, r);
     for (int k = 0; k < cr.n; ++k) rank += cr.cols[k] < c;
     const Parts o = off[row];
-    po.put(o, off[row + 1].zl - o.zl, rank, c, r.val[x.at[i]]);
+    po.put(o, off[row + 1].zl - o.zl, rank, c, r.sval[x.at[i]]);
 }
 
 // sizes that the host needs after the matching, in one place
@@ -1279,6 +1455,27 @@ struct Cub {
     }
 };
 
+// Pinned memory for the few words a build reads back; as many blocks exist as builds ever ran at the same time.
+struct Mirror {
+    static constexpr size_t kBytes = 2048;
+    unsigned char* p = nullptr;
+    static std::mutex& lock() { static std::mutex m; return m; }
+    static std::vector<unsigned char*>& idle() { static std::vector<unsigned char*> v; return v; }
+    int take() {
+        {
+            std::lock_guard<std::mutex> g(lock());
+            if (!idle().empty()) { p = idle().back(); idle().pop_back(); return 0; }
+        }
+        TRS_CUDA(cudaHostAlloc((void**)&p, kBytes, cudaHostAllocPortable));
+        return 0;
+    }
+    ~Mirror() {
+        if (!p) return;
+        std::lock_guard<std::mutex> g(lock());
+        idle().push_back(p);
+    }
+};
+
 template <class T>
 int read_back(const T* dev, T* host, cudaStream_t st) {
     TRS_CUDA(cudaMemcpyAsync(host, dev, sizeof(T), cudaMemcpyDeviceToHost, st));
@@ -1311,53 +1508,89 @@ struct Event {
 };
 
 struct Records {   // stages 1 - 3
-    int D = 0;
-    int *start = nullptr, *ord = nullptr;
-    Record* rec = nullptr;
-    unsigned *ent = nullptr, *key2 = nullptr;
+    WindowOut w{};
+    int* sel = nullptr;   // [kSortClasses + 1][W]
 };
 
-template <class Key, bool PACKED>
-int make_records(trs_builder* B, const int* rowptr, const int* col, const float* val, InputInfo* d_info, int* d_count, int col_bits, int w_bits,
-                 TempSpace& ts, Cub& cub_, cudaStream_t st, Records* R) {
-    const int nnz = (int)B->nnz, n = B->n_rows, window = B->cfg.window;
-    Key *keys_a, *keys_b, *keys;
-    unsigned *ent_a, *ent_b;
-    TRS_TRY(ts.get(nnz, &keys_a));
-    TRS_TRY(ts.get(nnz, &keys_b));
-    TRS_TRY(ts.get(nnz, &ent_a));
-    TRS_TRY(ts.get(nnz, &ent_b));
-    kb_make_keys<Key, PACKED><<<grid_for(nnz, 256 * kKeyItems), 256, 0, st>>>(rowptr, col, n, nnz, window, col_bits, keys_a, ent_a, d_info);
+template <int T, int I, int RB>
+int sort_class(int c, const InputInfo& info, const int* rowptr, const int* col, const float* val, const trs_builder* B, int col_bits,
+               const Records& R, InputInfo* d_info, cudaStream_t st) {
+    if (info.windows[c] == 0) return 0;
+    constexpr int smem = (int)sizeof(typename WindowSort<T, I, RB>::Smem);
+    auto kernel = kb_sort_window<T, I, RB>;
+    if (smem > 48 * 1024) TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    kernel<<<info.windows[c], T, smem, st>>>(rowptr, col, val, B->n_rows, B->cfg.window, col_bits, R.sel + (size_t)c * B->W, R.w, d_info);
     TRS_LAUNCH_CHECK();
-    TRS_TRY(cub_.sort_pairs(keys_a, keys_b, ent_a, ent_b, (long long)nnz, col_bits + w_bits, &keys, &R->ent));
-    ts.drop(R->ent == ent_a ? ent_b : ent_a, nnz);
+    return 0;
+}
+
+template <class Key>
+int sort_hubs(trs_builder* B, const int* rowptr, const int* col, const float* val, const InputInfo& info, InputInfo* d_info,
+              int* d_count, int col_bits, TempSpace& ts, Cub& cub_, cudaStream_t st, const Records& R) {
+    const int H = info.windows[kSortClasses], E = (int)info.hub_entries, n = B->n_rows, window = B->cfg.window;
+    const int h_bits = bits_for(H - 1);
+    const int* sel = R.sel + (size_t)kSortClasses * B->W;
+    int *size, *off, *first_rec, *place_a, *place_b, *place;
+    Key *keys_a, *keys_b, *keys;
+    TRS_TRY(ts.get((size_t)H + 1, &size));
+    TRS_TRY(ts.get((size_t)H + 1, &off));
+    TRS_TRY(ts.get((size_t)H, &first_rec));
+    TRS_TRY(ts.get(E, &keys_a));
+    TRS_TRY(ts.get(E, &keys_b));
+    TRS_TRY(ts.get(E, &place_a));
+    TRS_TRY(ts.get(E, &place_b));
+    kb_hub_sizes<<<grid_for(H + 1), 256, 0, st>>>(rowptr, n, window, sel, H, size);
+    TRS_LAUNCH_CHECK();
+    TRS_TRY(cub_.exclusive_sum(size, off, H + 1));
+    const HubView hub{sel, off, H};
+    kb_hub_keys<Key><<<grid_for(E), 256, 0, st>>>(rowptr, col, n, window, hub, E, col_bits, keys_a, place_a, d_info);
+    TRS_LAUNCH_CHECK();
+    TRS_TRY(cub_.sort_pairs(keys_a, keys_b, place_a, place_b, (long long)E, col_bits + h_bits, &keys, &place));
     // first entries, into the key buffer that is free now
     int* start = (int*)(keys == keys_a ? keys_b : keys_a);
     IsHead<Key> is_head{keys};
     TRS_TRY(cub_.run([&](void* t, size_t& b) {
-        return cub::DeviceSelect::If(t, b, thrust::counting_iterator<int>(0), start, d_count, nnz, is_head, st);
+        return cub::DeviceSelect::If(t, b, thrust::counting_iterator<int>(0), start, d_count, E, is_head, st);
     }));
     int D = 0;
-    InputInfo info;
-    TRS_CUDA(cudaMemcpyAsync(&info, d_info, sizeof(info), cudaMemcpyDeviceToHost, st));
     TRS_TRY(read_back(d_count, &D, st));
-    if (info.err & 2) return TRS_E_NOT_CANONICAL;
-    R->D = D;
-    unsigned *key2_a, *key2_b;
-    int *ord_a, *ord_b;
-    TRS_TRY(ts.get(D, &R->rec));
+    Record* record;
+    unsigned *key2_a, *key2_b, *key2;
+    int *ord_a, *ord_b, *ord;
+    TRS_TRY(ts.get(D, &record));
     TRS_TRY(ts.get(D, &key2_a));
     TRS_TRY(ts.get(D, &key2_b));
     TRS_TRY(ts.get(D, &ord_a));
     TRS_TRY(ts.get(D, &ord_b));
-    kb_records<Key, PACKED><<<grid_for(D), 256, 0, st>>>(keys, R->ent, rowptr, val, n, window, start, D, nnz, col_bits, R->rec,
-                                                        key2_a, ord_a);
+    kb_hub_records<Key><<<grid_for(D), 256, 0, st>>>(keys, place, rowptr, val, n, window, hub, start, D, E, col_bits, record, key2_a, ord_a, first_rec);
     TRS_LAUNCH_CHECK();
-    R->start = start;
-    ts.drop(keys, nnz);
-    TRS_TRY(cub_.sort_pairs(key2_a, key2_b, ord_a, ord_b, (long long)D, 4 + w_bits, &R->key2, &R->ord));  // stable
-    ts.drop(R->key2 == key2_a ? key2_b : key2_a, D);
-    ts.drop(R->ord == ord_a ? ord_b : ord_a, D);
+    TRS_TRY(cub_.sort_pairs(key2_a, key2_b, ord_a, ord_b, (long long)D, 4 + h_bits, &key2, &ord));  // stable
+    kb_hub_place<<<grid_for(D), 256, 0, st>>>(key2, ord, record, D, rowptr, window, hub, first_rec, R.w);
+    TRS_LAUNCH_CHECK();
+    kb_hub_values<<<grid_for(E), 256, 0, st>>>(place, rowptr, val, window, hub, E, R.w.sval);
+    TRS_LAUNCH_CHECK();
+    ts.drop(ord_b, D); ts.drop(ord_a, D); ts.drop(key2_b, D); ts.drop(key2_a, D); ts.drop(record, D);
+    ts.drop(place_b, E); ts.drop(place_a, E); ts.drop(keys_b, E); ts.drop(keys_a, E);
+    return 0;
+}
+
+int make_records(trs_builder* B, const int* rowptr, const int* col, const float* val, const InputInfo& info, InputInfo* d_info,
+                 int* d_count, TempSpace& ts, Cub& cub_, cudaStream_t st, Records* R) {
+    const int col_bits = bits_for(info.max_col), W = B->W;
+    const size_t nnz = (size_t)B->nnz;
+    TRS_TRY(ts.get(nnz, &R->w.rec));
+    TRS_TRY(ts.get(nnz, &R->w.sval));
+    TRS_TRY(ts.get(nnz, &R->w.cnt));
+    TRS_TRY(ts.get((size_t)W, &R->w.ncol));
+    TRS_CUDA(cudaMemsetAsync(R->w.ncol, 0, sizeof(int) * (size_t)W, st));
+    if (info.windows[kSortClasses] > 0) {
+        const int h_bits = bits_for(info.windows[kSortClasses] - 1);
+        TRS_TRY(col_bits + h_bits <= 32 ? sort_hubs<unsigned>(B, rowptr, col, val, info, d_info, d_count, col_bits, ts, cub_, st, *R)
+                                        : sort_hubs<u64>(B, rowptr, col, val, info, d_info, d_count, col_bits, ts, cub_, st, *R));
+    }
+    TRS_TRY((sort_class<512, 8, 4>(2, info, rowptr, col, val, B, col_bits, *R, d_info, st)));
+    TRS_TRY((sort_class<128, 8, 4>(1, info, rowptr, col, val, B, col_bits, *R, d_info, st)));
+    TRS_TRY((sort_class<64, 4, 4>(0, info, rowptr, col, val, B, col_bits, *R, d_info, st)));
     return 0;
 }
 
@@ -1388,49 +1621,50 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
 
     // ---- sizes of the input ---------------------------------------------------------------------
     struct Head { InputInfo info; MatchCounts mc; Totals tot; int count; u64 dropped[kDropCounters]; };
+    struct Back { Head head; Win total; Parts parts; };   // what the host sees of it
+    static_assert(sizeof(Back) <= Mirror::kBytes, "");
+    Mirror mirror;
+    TRS_TRY(mirror.take());
+    Back* const back = (Back*)mirror.p;
     Head* d_head;
     TRS_TRY(ts.get(1, &d_head));
     TRS_CUDA(cudaMemsetAsync(d_head, 0, sizeof(Head), st));
-    kb_input_info<<<2 * sms, 512, 0, st>>>(rowptr, col, n, &d_head->info);
+    Records R;
+    TRS_TRY(ts.get((size_t)(kSortClasses + 1) * W, &R.sel));
+    kb_input_info<<<2 * sms, 512, 0, st>>>(rowptr, col, n, window, W, R.sel, &d_head->info);
     TRS_LAUNCH_CHECK();
-    InputInfo info;
-    TRS_TRY(read_back(&d_head->info, &info, st));
+    auto sync_head = [&]() { return read_back(d_head, &back->head, st); };
+    TRS_TRY(sync_head());
+    const InputInfo info = back->head.info;
     if (info.first != 0 || info.last < 0 || (info.err & 1)) return TRS_E_OFFSETS;
     const long long nnz = B->nnz = info.last;
     if (nnz == 0) return empty_outputs(B, st);
     ts.chunk_bytes = std::max((size_t)16 << 20, (size_t)nnz * 24);
 
-    // ---- 1. - 3. columns of every window in (count desc, column asc) order ---------------------------
-    const int col_bits = bits_for(info.max_col), w_bits = bits_for(W > 0 ? W - 1 : 0);
-    const bool packed = nnz < (1ll << 28);
-    Records R;
-    if (col_bits + w_bits <= 32)
-        TRS_TRY(packed ? (make_records<unsigned, true>(B, rowptr, col, val, &d_head->info, &d_head->count, col_bits, w_bits, ts, cub_, st, &R))
-                       : (make_records<unsigned, false>(B, rowptr, col, val, &d_head->info, &d_head->count, col_bits, w_bits, ts, cub_, st, &R)));
-    else
-        TRS_TRY(packed ? (make_records<u64, true>(B, rowptr, col, val, &d_head->info, &d_head->count, col_bits, w_bits, ts, cub_, st, &R))
-                       : (make_records<u64, false>(B, rowptr, col, val, &d_head->info, &d_head->count, col_bits, w_bits, ts, cub_, st, &R)));
-    const int D = R.D;
-    B->distinct_cols = D;
-    const RecordView rv{R.ord, R.rec, R.ent, val, packed ? 1 : 0};
+    // ---- 1. - 3. columns of every window in (count desc, col asc) order ---------------------------
+    TRS_TRY(make_records(B, rowptr, col, val, info, &d_head->info, &d_head->count, ts, cub_, st, &R));
+    const RecordView rv{R.w.rec, R.w.sval};
 
     // ---- 4., 5. TC columns, units, sizes per window ---------------------------------------------
-    int *rec, *tc, *sel_block, *sel_huge;
+    int *rec, *end, *tc, *sel_block, *sel_huge;
     Win *win, *pre;
     TRS_TRY(ts.get((size_t)W + 1, &rec));
+    TRS_TRY(ts.get((size_t)W + 1, &end));
     TRS_TRY(ts.get((size_t)W + 1, &tc));
     TRS_TRY(ts.get((size_t)W + 1, &win));
     TRS_TRY(ts.get((size_t)W + 1, &pre));
     TRS_TRY(ts.get((size_t)W + 1, &sel_block));
     TRS_TRY(ts.get((size_t)W + 1, &sel_huge));
-    kb_windows<<<grid_for(W + 1, 128), 128, 0, st>>>(R.start, R.key2, rowptr, n, D, W, cfg, rec, tc, win, sel_block, sel_huge, &d_head->mc);
+    kb_windows<<<grid_for(W + 1, 128), 128, 0, st>>>(rowptr, R.w.ncol, R.w.cnt, W, cfg, rec, end, tc, win, sel_block, sel_huge, &d_head->mc);
     TRS_LAUNCH_CHECK();
     TRS_TRY(cub_.exclusive_scan(win, pre, WinSum(), Win{0, 0, 0, 0}, W + 1));
-    const WindowView v{rec, tc, pre};
-    Win total;
-    MatchCounts mc;
-    TRS_CUDA(cudaMemcpyAsync(&mc, &d_head->mc, sizeof(mc), cudaMemcpyDeviceToHost, st));
-    TRS_TRY(read_back(pre + W, &total, st));
+    const WindowView v{rec, end, tc, pre};
+    TRS_CUDA(cudaMemcpyAsync(&back->total, pre + W, sizeof(Win), cudaMemcpyDeviceToHost, st));
+    TRS_TRY(sync_head());
+    if (back->head.info.err & 2) return TRS_E_NOT_CANONICAL;
+    const Win total = back->total;
+    const MatchCounts mc = back->head.mc;
+    B->distinct_cols = (long long)mc.records;
     const int NB = total.blocks, NP = total.parts, TU = total.units, TS = total.slots;
     B->units = TU;
 
@@ -1460,20 +1694,20 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
             TRS_TRY(ts.get((size_t)TU / 32 + W + 2, &mask));
         }
         TRS_CUDA(cudaStreamWaitEvent(side[0], ready.e, 0));
-        kb_match_block<<<mc.n_huge, kBlockThreads, (size_t)smem_units * 4, side[0]>>>(v, R.key2, cfg.unit_min_nnz, smem_units, words, mask,
+        kb_match_block<<<mc.n_huge, kBlockThreads, (size_t)smem_units * 4, side[0]>>>(v, R.w.cnt, cfg.unit_min_nnz, smem_units, words, mask,
                                                                                  sel_huge, mo);
         TRS_LAUNCH_CHECK();
     }
     if (mc.n_block > 0) {
         TRS_CUDA(cudaStreamWaitEvent(side[1], ready.e, 0));
-        kb_match_block<<<mc.n_block, kBlockThreads, (size_t)kBlockUnits * 4, side[1]>>>(v, R.key2, cfg.unit_min_nnz, kBlockUnits, nullptr,
+        kb_match_block<<<mc.n_block, kBlockThreads, (size_t)kBlockUnits * 4, side[1]>>>(v, R.w.cnt, cfg.unit_min_nnz, kBlockUnits, nullptr,
                                                                                    nullptr, sel_block, mo);
         TRS_LAUNCH_CHECK();
     }
     {
         const int units = std::max(32, (mc.max_warp + 31) & ~31);
         const size_t smem = (size_t)kMatchWarps * (units + units / 32) * 4;
-        kb_match_warp<<<grid_for(W + 1, kMatchWarps), 32 * kMatchWarps, smem, st>>>(v, W, R.key2, cfg.unit_min_nnz, units, mo);
+        kb_match_warp<<<grid_for(W + 1, kMatchWarps), 32 * kMatchWarps, smem, st>>>(v, W, R.w.cnt, cfg.unit_min_nnz, units, mo);
         TRS_LAUNCH_CHECK();
     }
     if (mc.n_huge > 0) { TRS_TRY(done[0].record(side[0])); TRS_CUDA(cudaStreamWaitEvent(st, done[0].e, 0)); }
@@ -1513,8 +1747,8 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     kb_totals<<<1, 1, 0, st>>>(B->s_offset.p, B->s_window_tile_offset.p, W, B->t_block_offset.p, NB, cfg.strict ? nullptr : off, n,
                                &d_head->tot);
     TRS_LAUNCH_CHECK();
-    Totals tot;
-    TRS_TRY(read_back(&d_head->tot, &tot, st));
+    TRS_TRY(sync_head());
+    Totals tot = back->head.tot;
     const int G = tot.groups, T = tot.tiles;
 
     TRS_TRY(B->out(B->t_value, 3, tot.tc_nnz));
@@ -1553,8 +1787,8 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
         TRS_LAUNCH_CHECK();
     }
     if (cfg.strict) {
-        u64 n_extra = 0;
-        TRS_TRY(read_back(d_head->dropped, &n_extra, st));
+        TRS_TRY(sync_head());
+        const u64 n_extra = back->head.dropped[0];
         if (n_extra > 0) {
             u64* key;
             int* at;
@@ -1564,7 +1798,8 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
             x = Extras{key, at, (int)n_extra};
         }
         TRS_TRY(count_parts());
-        TRS_TRY(read_back(off + n, &tot.parts, st));
+        TRS_TRY(read_back(off + n, &back->parts, st));
+        tot.parts = back->parts;
     }
     const Parts& p = tot.parts;
     TRS_TRY(B->out(B->c_row_offset, 7, (size_t)p.nl + 1));
@@ -1585,11 +1820,10 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
         kb_cuda_extras<<<grid_for(x.n), 256, 0, st>>>(window, mo.cuda_unit, v, rv, x, off, po);
         TRS_LAUNCH_CHECK();
     }
-    Head head;
-    TRS_TRY(read_back(d_head, &head, st));
+    TRS_TRY(sync_head());
     B->dropped = 0;
     if (!cfg.strict)   // nothing is lost in strict mode
-        for (u64 d : head.dropped) B->dropped += d;
+        for (u64 d : back->head.dropped) B->dropped += d;
     TRS_LAUNCH_CHECK();
     return TRS_OK;
 }

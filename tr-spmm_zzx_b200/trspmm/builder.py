@@ -33,6 +33,10 @@ def _shape(name: str, n: int, window: int):
     return (n,)
 
 
+_ARRAY_DTYPES = [_DTYPES.get(n, torch.int32) for n in FORMAT_NAMES]
+_SHAPED = [(i, n) for i, n in enumerate(FORMAT_NAMES) if _shape(n, 0, 1) != (0,)]   # arrays of more than one dimension
+
+
 def env_switches():
     """The two environment switches the reference's builder reads at call time
     (block_online.cpp:564-567)."""
@@ -91,16 +95,16 @@ def build_format(rowptr: torch.Tensor, col: torch.Tensor, val: torch.Tensor, par
 
     def hand_out(_ctx, i, n_bytes):               # the arrays are torch tensors from the start: nothing is copied
         try:
-            dt = _DTYPES.get(FORMAT_NAMES[i], torch.int32)
-            arrays[i] = torch.empty(n_bytes // dt.itemsize, dtype=dt, device=dev)
-            return arrays[i].data_ptr()
+            dt = _ARRAY_DTYPES[i]
+            t = arrays[i] = torch.empty(n_bytes // dt.itemsize, dtype=dt, device=dev)
+            return t.data_ptr()
         except Exception as e:                    # an exception cannot cross the C frames
             failed.append(e)
             return None
 
     arena_used = 0
     with torch.cuda.device(dev):
-        stream = _lib.current_stream_ptr(dev)
+        stream = _lib.current_stream_ptr(dev)   # both entries return when the build is complete on it
         args = (rowptr.data_ptr(), col.data_ptr() if col.numel() else None, val.data_ptr() if val.numel() else None,
                 rowptr.numel() - 1, C.byref(cfg))
         if arena is None:
@@ -124,10 +128,11 @@ def build_format(rowptr: torch.Tensor, col: torch.Tensor, val: torch.Tensor, par
                 used = C.c_size_t()
                 _lib.check(lib.trs_build_arena_used(handle, C.byref(used)))
                 arena_used = used.value + skip
-            for i, name in enumerate(FORMAT_NAMES):
-                t = arrays[i] if arrays[i] is not None else torch.empty(0, dtype=_DTYPES.get(name, torch.int32), device=dev)
-                arrays[i] = t.view(_shape(name, t.numel(), window))
-            torch.cuda.current_stream(dev).synchronize()
+            for i, t in enumerate(arrays):
+                if t is None:
+                    arrays[i] = torch.empty(0, dtype=_ARRAY_DTYPES[i], device=dev)
+            for i, name in _SHAPED:
+                arrays[i] = arrays[i].view(_shape(name, arrays[i].numel(), window))
         finally:
             lib.trs_build_destroy(handle)
     info = {n: getattr(stats, n) for n, _ in stats._fields_}
