@@ -30,12 +30,18 @@ namespace trs {
 // diagonal of the product is the result (lane 4 g + g / 2 holds it).  That wastes the other products but replaces
 // conversions, FMAs and shuffles, which were 19 warp instructions per entry at K = 64, by 2 loads and 2 MMAs per
 // 32 features and 8 entries; what is left is the gather of one Y row per entry through L2.
-// Uniform 50 021 rows x 17 entries, K = 96: 112 -> 24 us.
+// Uniform 50 021 rows x 17 entries, K = 96: 112 -> 27 us with every step's loads behind the one before, 22 us with the next
+// step's ids loaded ahead and no branch between the batches of a step.
 //
 // Inputs are not validated by a pass of their own on this entry (trs_sddmm_plan_create does that for
 // planned patterns), so the kernel bounds what it dereferences: rows stop at the last one, and an
 // entry whose column lies outside [0, n_cols) reads row 0 of Y and is written as NaN.
-constexpr int kEntryWarps = 8, kEntryCtas = 5;   // warps per CTA, CTAs per SM
+constexpr int kEntryWarps = 8;   // warps per CTA
+// CTAs per SM, and batches of 8 entries whose loads the compiler may put side by side: narrow rows want warps, wide ones
+// registers.  R-MAT 20, us, 5 CTAs x 4 batches against 4 x 2: K = 32 446 / 511, K = 64 579 / 619, K = 96 793 / 739, K = 128 1055 /
+// 983, K = 256 3088 / 2217.
+__host__ __device__ constexpr int entry_ctas(int kch) { return kch <= 2 ? 5 : 4; }
+__host__ __device__ constexpr int entry_batches(int kch) { return kch <= 2 ? 4 : 2; }
 
 // Largest r in [0, n) with a[r] <= x (a ascending, a[0] <= x), by the whole warp: 32 probes per round.
 __device__ __forceinline__ int warp_find(const int* __restrict__ a, int n, int x, int lane) {
@@ -57,8 +63,9 @@ __device__ __forceinline__ void store_result(void* out, int f32, long long i, __
     else ((__half*)out)[i] = v;
 }
 
-template <int KCH>   // 32-feature chunks per pass (K > 32 KCH loops)
-__global__ void __launch_bounds__(32 * kEntryWarps, kEntryCtas) k_sddmm(const int* __restrict__ rowptr, const int* __restrict__ col,
+// KCH: 32-feature chunks per pass; FULL: one pass, all of it (otherwise K is looped over and its end tested)
+template <int KCH, bool FULL>
+__global__ void __launch_bounds__(32 * kEntryWarps, entry_ctas(KCH)) k_sddmm(const int* __restrict__ rowptr, const int* __restrict__ col,
                                                             const __half* __restrict__ X, const __half* __restrict__ Y,
                                                             void* __restrict__ out, int out_f32, int n_rows, int n_cols, int K,
                                                             int ld) {
@@ -72,11 +79,15 @@ __global__ void __launch_bounds__(32 * kEntryWarps, kEntryCtas) k_sddmm(const in
         if (first >= nnz) return;
         const int e_end = (int)min(first + per_warp, (long long)nnz);
         int row = warp_find(rowptr, n_rows, (int)first, lane);   // row of the chunk's first entry
+        // columns and row ends of the next 32 entries are loaded while the present ones are multiplied
+        auto load_col = [&](int e0) { return col[min(e0 + lane, e_end - 1)]; };
+        auto load_bound = [&]() { return row + 1 + lane < n_rows ? rowptr[row + 1 + lane] : 0x7fffffff; };
+        int c_next = load_col((int)first), bound_next = load_bound();
         for (int e0 = (int)first; e0 < e_end; e0 += 32) {
             // columns and rows of 32 entries, one per lane
             const int e = min(e0 + lane, e_end - 1);
-            const int bound = row + 1 + lane < n_rows ? rowptr[row + 1 + lane] : 0x7fffffff;
-            int c = col[e];
+            const int bound = bound_next;
+            int c = c_next;
             const bool bad = (unsigned)c >= (unsigned)n_cols;
             if (bad) c = 0;
             int r = 0;   // how many of the next 32 rows start at or before e
@@ -95,17 +106,21 @@ __global__ void __launch_bounds__(32 * kEntryWarps, kEntryCtas) k_sddmm(const in
             }
             row = __shfl_sync(0xffffffffu, r, 31);
             const unsigned bad_mask = __ballot_sync(0xffffffffu, bad);
-#pragma unroll
+            if (e0 + 32 < e_end) {
+                c_next = load_col(e0 + 32);
+                bound_next = load_bound();
+            }
+            // entries past the end repeat the last one and are not stored
+#pragma unroll entry_batches(KCH)
             for (int b = 0; b < 4; ++b) {
-                if (e0 + 8 * b >= e_end) break;
                 const uint4* x = (const uint4*)X + (size_t)__shfl_sync(0xffffffffu, r, 8 * b + g) * ld16 + t;
                 const uint4* y = (const uint4*)Y + (size_t)__shfl_sync(0xffffffffu, c, 8 * b + g) * ld16 + t;
                 float d[4] = {0.f, 0.f, 0.f, 0.f};
-                for (int p0 = 0; p0 < pieces; p0 += 4 * KCH) {
+                for (int p0 = 0; p0 < (FULL ? 1 : pieces); p0 += 4 * KCH) {
                     uint4 xv[KCH], yv[KCH];
 #pragma unroll
                     for (int ch = 0; ch < KCH; ++ch) {
-                        const bool in = p0 + 4 * ch + t < pieces;
+                        const bool in = FULL || p0 + 4 * ch + t < pieces;
                         xv[ch] = in ? __ldg(x + p0 + 4 * ch) : make_uint4(0, 0, 0, 0);
                         yv[ch] = in ? __ldg(y + p0 + 4 * ch) : make_uint4(0, 0, 0, 0);
                     }
@@ -319,10 +334,10 @@ __device__ __forceinline__ void cp_async16_to(uint32_t dst, const void* src) {
 }
 
 // TAIL: K is not a multiple of 32; the chunks past the end of a row are zero on both sides.
-template <int KCH, bool TAIL>
+template <int KCH, bool TAIL, bool F32>
 __global__ void __launch_bounds__(128, SddmmRing<KCH>::CTAS) k_sddmm_tc_ring(
     const SddmmQuad* __restrict__ quads, const int* __restrict__ ids, const unsigned* __restrict__ list, int n_quads,
-    const __half* __restrict__ X, const __half* __restrict__ Y, void* __restrict__ out, int out_f32, int n_rows, int pieces,
+    const __half* __restrict__ X, const __half* __restrict__ Y, void* __restrict__ out, int n_rows, int pieces,
     int ld16, int quads_per_warp) {
     using R = SddmmRing<KCH>;
     extern __shared__ __align__(128) unsigned char smem[];
@@ -427,7 +442,7 @@ __global__ void __launch_bounds__(128, SddmmRing<KCH>::CTAS) k_sddmm_tc_ring(
         const long long o = (unsigned)head.y;
         auto put = [&](unsigned e) {
             const unsigned pos = e & ((1u << kPosBits) - 1u);
-            store_result(out, out_f32, o + (e >> kPosBits), *(const __half*)(tile + (pos >> 5) * kTilePitch + (pos & 31u) * 2));
+            store_result(out, F32, o + (e >> kPosBits), *(const __half*)(tile + (pos >> 5) * kTilePitch + (pos & 31u) * 2));
         };
 #pragma unroll
         for (int i = 0; i < kListAhead; ++i)
@@ -617,20 +632,23 @@ int sm_count() {
 
 int launch_entries(const int32_t* rowptr, const int32_t* col, const Operands& o, void* out, int out_f32, int n_rows, int n_cols,
                    int K, cudaStream_t st) {
-    const int grid = sm_count() * kEntryCtas;   // one wave
-    auto go = [&](auto kernel) { kernel<<<grid, 32 * kEntryWarps, 0, st>>>(rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K, o.ld); };
-    if (K <= 32) go(k_sddmm<1>);
-    else if (K <= 64) go(k_sddmm<2>);
-    else if (K <= 96) go(k_sddmm<3>);
-    else go(k_sddmm<4>);
+    auto go = [&](auto kernel, int ctas) { kernel<<<sm_count() * ctas, 32 * kEntryWarps, 0, st>>>(rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K, o.ld); };
+    if (K == 32) go(k_sddmm<1, true>, entry_ctas(1));
+    else if (K < 32) go(k_sddmm<1, false>, entry_ctas(1));
+    else if (K == 64) go(k_sddmm<2, true>, entry_ctas(2));
+    else if (K < 64) go(k_sddmm<2, false>, entry_ctas(2));
+    else if (K == 96) go(k_sddmm<3, true>, entry_ctas(3));
+    else if (K < 96) go(k_sddmm<3, false>, entry_ctas(3));
+    else if (K == 128) go(k_sddmm<4, true>, entry_ctas(4));
+    else go(k_sddmm<4, false>, entry_ctas(4));
     TRS_LAUNCH_CHECK();
     return TRS_OK;
 }
 
-template <int KCH, bool TAIL>
-int launch_ring(const trs_sddmm_plan* p, const Operands& o, void* out, int out_f32, int K, cudaStream_t st) {
+template <int KCH, bool TAIL, bool F32>
+int launch_ring(const trs_sddmm_plan* p, const Operands& o, void* out, int K, cudaStream_t st) {
     using R = SddmmRing<KCH>;
-    auto kernel = k_sddmm_tc_ring<KCH, TAIL>;
+    auto kernel = k_sddmm_tc_ring<KCH, TAIL, F32>;
     static std::atomic<unsigned long long> done{0};   // per device
     int dev = 0;
     TRS_CUDA(cudaGetDevice(&dev));
@@ -642,14 +660,15 @@ int launch_ring(const trs_sddmm_plan* p, const Operands& o, void* out, int out_f
     // one wave of warps with equal shares (48 blocks a warp left the last of 2.4 waves nearly empty)
     const int per_warp = ceil_div(p->n_quads, sm_count() * R::CTAS * 4);
     kernel<<<ceil_div(ceil_div(p->n_quads, per_warp), 4), 128, R::SMEM, st>>>(p->quads.p, p->ids.p, p->list.p, p->n_quads, o.X, o.Y,
-                                                                             out, out_f32, p->n_rows, (K + 7) / 8, o.ld / 8, per_warp);
+                                                                             out, p->n_rows, (K + 7) / 8, o.ld / 8, per_warp);
     TRS_LAUNCH_CHECK();
     return TRS_OK;
 }
 
 template <int KCH>
 int launch_ring_k(const trs_sddmm_plan* p, const Operands& o, void* out, int out_f32, int K, cudaStream_t st) {
-    return K == 32 * KCH ? launch_ring<KCH, false>(p, o, out, out_f32, K, st) : launch_ring<KCH, true>(p, o, out, out_f32, K, st);
+    if (out_f32) return K == 32 * KCH ? launch_ring<KCH, false, true>(p, o, out, K, st) : launch_ring<KCH, true, true>(p, o, out, K, st);
+    return K == 32 * KCH ? launch_ring<KCH, false, false>(p, o, out, K, st) : launch_ring<KCH, true, false>(p, o, out, K, st);
 }
 
 // Two ints the device writes and the host reads (pinned, mapped), with the event that says they are there.  Taken for one
