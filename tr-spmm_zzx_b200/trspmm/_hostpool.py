@@ -19,6 +19,8 @@ MIN_BYTES = 1 << 20      # below, the C library reuses memory itself
 KEEP_BYTES = 256 << 20
 _BLOCK = 2 << 20         # large pages
 
+_adapted = False
+
 _lock = threading.RLock()   # re-entrant: a collection inside take() may give blocks back
 _idle: list = []            # oldest first
 
@@ -51,6 +53,13 @@ def empty(shape, dtype: torch.dtype) -> torch.Tensor:
     n = count * dtype.itemsize
     if n < MIN_BYTES or n > KEEP_BYTES:
         return torch.empty(shape, dtype=dtype)
+    global _adapted
+    if not _adapted:
+        # The C library takes blocks up to the largest one freed so far (32 MB at most) from its heap, larger ones from the
+        # system each time.  Results used to raise that mark; without them a program's own arrays of a few
+        # megabytes would fault their pages in anew on every allocation.
+        _adapted = True
+        torch.empty(31 << 20, dtype=torch.uint8)
     block = _take(n)
     owner = np.frombuffer(block, dtype=np.uint8, count=n)   # lives as long as the tensor's storage
     weakref.finalize(owner, _give_back, block).atexit = False
