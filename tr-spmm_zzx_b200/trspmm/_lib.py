@@ -4,6 +4,8 @@ from __future__ import annotations
 import ctypes as C
 from pathlib import Path
 
+import torch
+
 PKG_ROOT = Path(__file__).resolve().parents[1]
 
 
@@ -161,7 +163,6 @@ def _copy(entry, host, dev, device):
 def copy_to_host(tensors, device):
     """CPU copies of contiguous CUDA tensors of one device (trs_copy_to_host): all of them in one go, after the work on the
     current stream."""
-    import torch
     from . import _hostpool
     out = [_hostpool.empty(t.shape, t.dtype) for t in tensors]
     with torch.cuda.device(device):
@@ -179,7 +180,6 @@ def release_cached_memory():
 
 def copy_to_device(tensors, device):
     """Copies of contiguous CPU tensors on `device` (trs_copy_to_device), ordered on the current stream."""
-    import torch
     out = [torch.empty(t.shape, dtype=t.dtype, device=device) for t in tensors]
     with torch.cuda.device(device):
         _copy(load().trs_copy_to_device, tensors, out, device)
@@ -187,19 +187,20 @@ def copy_to_device(tensors, device):
 
 
 def current_stream_ptr(device) -> int:
-    import torch
     return torch.cuda.current_stream(device).cuda_stream
+
+
+_get_device, _raw_stream = getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
 
 
 def launch(index: int, entry, *args):
     """entry(*args, current stream of device `index`), with that device current.  The device guard and the stream object
     of torch.cuda cost 3.7 us a call, as much as a small product takes on the GPU; both are skipped when the device
     is current already, which it is in all but multi-device programs."""
-    import torch
-    if torch._C._cuda_getDevice() == index:
-        code = entry(*args, torch._C._cuda_getCurrentRawStream(index))
+    if _get_device() == index:
+        code = entry(*args, _raw_stream(index))
     else:
         with torch.cuda.device(index):
-            code = entry(*args, torch._C._cuda_getCurrentRawStream(index))
+            code = entry(*args, _raw_stream(index))
     if code:
         check(code)

@@ -80,12 +80,13 @@ class SpmmPlan:
             raise ValueError("out must be a contiguous [m_rows, F] tensor on the plan's device")
         _out_code(out.dtype)
 
-    def _workspace(self, F: int) -> torch.Tensor:
+    def _workspace(self, F: int):
+        """(address, bytes) of the scratch memory kept for feature width F."""
         ws = self._ws.get(F)
         if ws is None:
-            ws = torch.empty(max(self.workspace_bytes(F), 16), dtype=torch.uint8, device=self.device)
-            self._ws[F] = ws
-        return ws
+            t = torch.empty(max(self.workspace_bytes(F), 16), dtype=torch.uint8, device=self.device)
+            ws = self._ws[F] = (t.data_ptr(), t.numel(), t)
+        return ws[0], ws[1]
 
     def _new_out(self, B: torch.Tensor, F: int, dtype) -> torch.Tensor:
         if dtype is torch.float16 and self.m_rows == self.k_cols:
@@ -101,9 +102,9 @@ class SpmmPlan:
         else:
             self._check_out(out, F)
             code = _out_code(out.dtype)
-        ws = self._workspace(F)
+        ws, ws_bytes = self._workspace(F)
         _lib.launch(self._index, self.lib.trs_spmm_run_ex, self._handle, B.data_ptr(), out.data_ptr(), F, code,
-                    1 if relu else 0, ws.data_ptr(), ws.numel())
+                    1 if relu else 0, ws, ws_bytes)
         return out
 
     @property
@@ -116,10 +117,10 @@ class SpmmPlan:
         only those rows of `out` are written."""
         F = self._check_B(B)
         self._check_out(out, F)
-        ws = self._workspace(F)
+        ws, ws_bytes = self._workspace(F)
         with torch.cuda.device(self.device):
             _lib.check(self.lib.trs_spmm_run_windows(self._handle, B.data_ptr(), out.data_ptr(), F, _out_code(out.dtype),
-                                                     1 if relu else 0, ws.data_ptr(), ws.numel(),
+                                                     1 if relu else 0, ws, ws_bytes,
                                                      _lib.current_stream_ptr(self.device), int(window_begin),
                                                      int(window_end)))
         return out
@@ -131,10 +132,10 @@ class SpmmPlan:
         F = self._check_B(B)
         if not 1 <= len(dst_ptrs) <= 8 or row0 < 0:
             raise ValueError("1 to 8 destination buffers and a non-negative row offset")
-        ws = self._workspace(F)
+        ws, ws_bytes = self._workspace(F)
         arr = (C.c_void_p * len(dst_ptrs))(*[int(p) for p in dst_ptrs])
         _lib.launch(self._index, self.lib.trs_spmm_run_bcast, self._handle, B.data_ptr(), arr, len(dst_ptrs), int(row0), F,
-                    1 if relu else 0, ws.data_ptr(), ws.numel())
+                    1 if relu else 0, ws, ws_bytes)
 
     def run_static(self, B: torch.Tensor, out: torch.Tensor) -> torch.Tensor:
         """trs_spmm_run_static: the same product with the partial sums of split windows kept in
