@@ -90,9 +90,12 @@ int trs_device_count(void);
  * the host-buffer entries) and 32 MiB of pinned host memory for copies from and to pageable memory; this
  * returns what the current device's pool holds, and the pinned memory, to the driver. */
 int trs_pool_trim(void);
-/* Copies n device arrays into host memory of any kind (pageable memory through the pinned ring, several threads
- * filling it); ordered after the work on `stream`, complete on return. */
+/* Copies n device arrays into host memory of any kind (page-locked memory directly, pageable memory through the
+ * pinned ring, several threads filling it); ordered after the work on `stream`, complete on return. */
 int trs_copy_to_host(int n, void* const* host, const void* const* dev, const size_t* bytes, void* stream);
+/* Page-locks host memory of the caller, so that copies from and to it need no staging, and releases it again. */
+int trs_host_register(void* host, size_t bytes);
+int trs_host_unregister(void* host);
 /* The other direction: returns when the host arrays have been read; the copies are then queued on `stream`. */
 int trs_copy_to_device(int n, const void* const* host, void* const* dev, const size_t* bytes, void* stream);
 

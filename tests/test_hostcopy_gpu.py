@@ -24,6 +24,23 @@ def test_round_trip(sizes):
         assert torch.equal(a, b)
 
 
+def test_results_in_reused_blocks():
+    """A result block is page-locked on its second use and copied into directly, beside arrays that are staged."""
+    from trspmm import _hostpool
+    dev = torch.device("cuda", 0)
+    _hostpool.release()
+    src = [torch.arange(n, dtype=torch.int32, device=dev) for n in (3 * MB, 100, MB // 8, 2 * MB + 3)]
+    locked = []
+    for k in range(4):
+        got = _lib.copy_to_host([s + k for s in src], dev)
+        for a, b in zip(got, src):
+            assert torch.equal(a, (b + k).cpu())
+        locked.append(got[0].is_pinned())
+        del got, a
+    assert not locked[0] and locked[-1]
+    _hostpool.release()
+
+
 def test_two_threads():
     dev = torch.device("cuda", 0)
     data = [torch.arange(9 * MB + i, dtype=torch.int32) for i in range(2)]

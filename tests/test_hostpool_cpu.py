@@ -35,5 +35,5 @@ def test_waiting_memory_is_bounded(monkeypatch):
     monkeypatch.setattr(_hostpool, "KEEP_BYTES", 8 << 20)
     held = [_hostpool.empty((1 << 20,), torch.float32) for _ in range(4)]
     held.clear()
-    assert sum(len(b) for b in _hostpool._idle) <= 8 << 20
+    assert sum(b.bytes for b in _hostpool._idle) <= 8 << 20
     assert _hostpool.empty((3 << 20,), torch.float32).numel() == 3 << 20   # beyond the bound: ordinary memory

@@ -12,6 +12,7 @@ from __future__ import annotations
 import ctypes as C
 import os
 
+import numpy as np
 import torch
 
 from trspmm import _hostpool, _lib
@@ -108,11 +109,12 @@ def forward_fp16_tcu_cuda_sptc_mma_parallel_online(
     groups = s_column.size(0)
     _check(s_value.size(0) == groups, "s_value group count mismatch")
     _check(s_pos.size(0) == groups, "s_pos group count mismatch")
-    _check(int(s_offsets[0]) == 0, "s_offsets must start with 0")
-    _check(int(s_offsets[-1]) == groups, "s_offsets end must equal group count")
-    per_window = s_offsets[1:] - s_offsets[:-1]
-    _check(bool((per_window >= 0).all()), "s_offsets must be non-decreasing")
-    num_tiles = int(((per_window + 3) // 4).sum())
+    offsets = s_offsets.numpy()
+    _check(offsets[0] == 0, "s_offsets must start with 0")
+    _check(offsets[-1] == groups, "s_offsets end must equal group count")
+    per_window = np.diff(offsets)
+    _check(per_window.size == 0 or per_window.min() >= 0, "s_offsets must be non-decreasing")
+    num_tiles = int(((per_window + 3) >> 2).sum())
     packed = s_tile_window.size(0)
     _check(s_tile_column.size(0) == packed, "s_tile_column tile count mismatch")
     _check(s_packed_a.size(0) == packed, "s_packed_a tile count mismatch")

@@ -3,6 +3,8 @@
 #include <string.h>
 
 #include <mutex>
+#include <system_error>
+#include <thread>
 #include <vector>
 
 #include "trs_common.cuh"
@@ -146,6 +148,67 @@ struct Upload {
     int now(size_t n, T** dev) {   // one array by itself
         raw(n, dev);
         return commit();
+    }
+};
+
+// A stream and an event for work beside the caller's, kept between calls: as many exist as were ever in use at once.
+struct SideStream {
+    cudaStream_t st = nullptr;
+    cudaEvent_t ready = nullptr;
+    int device = 0;
+};
+std::mutex g_side_mutex;
+std::vector<SideStream> g_side;
+
+int take_side(SideStream* s) {
+    int device = 0;
+    TRS_CUDA(cudaGetDevice(&device));
+    {
+        std::lock_guard<std::mutex> lock(g_side_mutex);
+        for (size_t i = g_side.size(); i-- > 0;)
+            if (g_side[i].device == device) {
+                *s = g_side[i];
+                g_side.erase(g_side.begin() + i);
+                return TRS_OK;
+            }
+    }
+    s->device = device;
+    TRS_CUDA(cudaEventCreateWithFlags(&s->ready, cudaEventDisableTiming));
+    TRS_CUDA(cudaStreamCreateWithFlags(&s->st, cudaStreamNonBlocking));
+    return TRS_OK;
+}
+
+// Makes a plan on a thread and a stream of its own, behind what `after` holds so far.
+class PlanThread {
+    std::thread t_;
+    SideStream side_;
+    int rc_ = TRS_OK;
+
+public:
+    int start(const trs_format& dev, int m_rows, int k_cols, int window, cudaStream_t after, trs_spmm_plan** out) {
+        const int rc = take_side(&side_);
+        if (rc) return rc;
+        TRS_CUDA(cudaEventRecord(side_.ready, after));
+        TRS_CUDA(cudaStreamWaitEvent(side_.st, side_.ready, 0));
+        try {
+            t_ = std::thread([=] {
+                const cudaError_t e = cudaSetDevice(side_.device);
+                rc_ = e != cudaSuccess ? (int)e : trs_spmm_plan_create(&dev, m_rows, k_cols, window, 1, side_.st, out);
+            });
+        } catch (const std::system_error&) {   // no thread to be had: the caller makes the plan itself
+        }
+        return TRS_OK;
+    }
+    bool started() const { return t_.joinable(); }
+    int join() {
+        if (t_.joinable()) t_.join();
+        return rc_;
+    }
+    ~PlanThread() {
+        join();
+        if (!side_.st) return;
+        std::lock_guard<std::mutex> lock(g_side_mutex);
+        g_side.push_back(side_);
     }
 };
 
@@ -528,18 +591,27 @@ extern "C" int trs_spmm_forward_host(const trs_format* host_format, const trs_ha
     Upload up;
     up.st = st;
     trs_format dev;
-    const trs_half* d_rhs = nullptr;
+    trs_half* d_rhs = nullptr;
     float* d_out = nullptr;
     int rc = upload_format(*host_format, up, &dev);
-    if (!rc) rc = up.put(rhs_host, (size_t)kOri * dimN, &d_rhs);
     if (rc) return rc;
+    const size_t rhs_bytes = (size_t)kOri * dimN * sizeof(trs_half);
+    up.raw((size_t)kOri * dimN, &d_rhs);
     up.raw((size_t)mOri * dimN, &d_out);
     if ((rc = up.commit())) return rc;
     struct PlanOwner {
         trs_spmm_plan* p = nullptr;
         ~PlanOwner() { trs_spmm_plan_destroy(p); }
     } plan;
-    if ((rc = trs_spmm_plan_create(&dev, mOri, kOri, window, 1, st, &plan.p))) return rc;
+    // the plan needs the format only: it is made (some twenty small kernels and two read-backs) while the dense operand goes up
+    {
+        PlanThread maker;
+        if (rhs_bytes >= ((size_t)2 << 20)) rc = maker.start(dev, mOri, kOri, window, st, &plan.p);
+        const HostSegment in{(void*)rhs_host, d_rhs, rhs_bytes};
+        if (!rc) rc = copy_to_device(&in, 1, st);
+        const int plan_rc = maker.started() ? maker.join() : (rc ? rc : trs_spmm_plan_create(&dev, mOri, kOri, window, 1, st, &plan.p));
+        if (rc || plan_rc) return rc ? rc : plan_rc;
+    }
     size_t ws_bytes = 0;
     unsigned char* ws = nullptr;
     if ((rc = trs_spmm_workspace_bytes(plan.p, dimN, &ws_bytes))) return rc;

@@ -12,6 +12,7 @@
 #include <emmintrin.h>
 #endif
 
+#include <algorithm>
 #include <atomic>
 #include <condition_variable>
 #include <mutex>
@@ -24,6 +25,7 @@ namespace trs {
 namespace {
 
 constexpr size_t kChunk = (size_t)1 << 20;
+constexpr size_t kSmallChunk = (size_t)256 << 10, kRamp = (size_t)2 << 20;
 constexpr int kSlots = 32;
 constexpr int kMaxWorkers = 8;
 constexpr size_t kStageFrom = (size_t)512 << 10;  // below, the driver's own path is as fast
@@ -244,7 +246,33 @@ int plain(const HostSegment* seg, int n, bool to_host, cudaStream_t st) {
     return 0;
 }
 
-int staged(const HostSegment* seg, int n, bool to_host, cudaStream_t st) {
+bool page_locked(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
+    return a.type == cudaMemoryTypeHost;
+}
+
+int staged(const HostSegment* all, int n_all, bool to_host, cudaStream_t st) {
+    // Page-locked arrays need no staging: the copy engine takes them directly (57 GB/s; through the ring host memory
+    // is crossed three times and 36 - 38 GB/s are left).  Downloads wait for them at the end.
+    std::vector<HostSegment> rest;
+    bool direct = false;
+    for (int i = 0; i < n_all; ++i) {
+        if (all[i].bytes >= kStageFrom && page_locked(all[i].host)) {
+            if (to_host) TRS_CUDA(cudaMemcpyAsync(all[i].host, all[i].dev, all[i].bytes, cudaMemcpyDeviceToHost, st));
+            else TRS_CUDA(cudaMemcpyAsync(all[i].dev, all[i].host, all[i].bytes, cudaMemcpyHostToDevice, st));
+            direct = true;
+        } else {
+            rest.push_back(all[i]);
+        }
+    }
+    struct Wait {   // the host memory is the caller's again when this returns
+        cudaStream_t st;
+        bool on;
+        ~Wait() { if (on) cudaStreamSynchronize(st); }
+    } wait{st, direct};
+    const HostSegment* seg = rest.data();
+    const int n = (int)rest.size();
     size_t total = 0;
     for (int i = 0; i < n; ++i) total += seg[i].bytes;
     Copier& c = copier();
@@ -254,12 +282,22 @@ int staged(const HostSegment* seg, int n, bool to_host, cudaStream_t st) {
     if (rc) return rc;
     if (to_host)
         for (int i = 0; i < n; ++i) ask_for_large_pages(seg[i]);
+    // Chunks of 1 MiB, but small ones where nothing else runs beside them: at the start of an upload (the copy engine waits for
+    // the first chunk to be filled) and at the end of a download (the call waits for the last one to be emptied); a
+    // download also leaves its small arrays for the end.
+    std::vector<HostSegment> order(seg, seg + n);
+    if (to_host) std::stable_sort(order.begin(), order.end(), [](const HostSegment& x, const HostSegment& y) { return x.bytes > y.bytes; });
     std::vector<Chunk> list;
-    list.reserve(total / kChunk + n + 1);
-    for (int i = 0; i < n; ++i)
-        for (size_t o = 0; o < seg[i].bytes; o += kChunk)
-            list.push_back(Chunk{(unsigned char*)seg[i].host + o, (unsigned char*)seg[i].dev + o,
-                                 seg[i].bytes - o < kChunk ? seg[i].bytes - o : kChunk});
+    list.reserve(total / kChunk + n + 2 * kRamp / kSmallChunk);
+    size_t before = 0;
+    for (const HostSegment& g : order)
+        for (size_t o = 0; o < g.bytes;) {
+            const size_t most = (to_host ? total - before <= kRamp : before < kRamp) ? kSmallChunk : kChunk;
+            const size_t bytes = g.bytes - o < most ? g.bytes - o : most;
+            list.push_back(Chunk{(unsigned char*)g.host + o, (unsigned char*)g.dev + o, bytes});
+            o += bytes;
+            before += bytes;
+        }
     return to_host ? c.down(list, st) : c.up(list, st);
 }
 
@@ -287,6 +325,20 @@ static int segments(int n, void* const* host, void* const* dev, const size_t* by
         seg->push_back(trs::HostSegment{host[i], dev[i], bytes[i]});
     }
     return TRS_OK;
+}
+
+extern "C" int trs_host_register(void* host, size_t bytes) {
+    if (!host || !bytes) return TRS_E_ARG;
+    const cudaError_t e = cudaHostRegister(host, bytes, cudaHostRegisterPortable);
+    if (e != cudaSuccess) cudaGetLastError();
+    return (int)e;
+}
+
+extern "C" int trs_host_unregister(void* host) {
+    if (!host) return TRS_E_ARG;
+    const cudaError_t e = cudaHostUnregister(host);
+    if (e != cudaSuccess) cudaGetLastError();
+    return (int)e;
 }
 
 extern "C" int trs_copy_to_host(int n, void* const* host, const void* const* dev, const size_t* bytes, void* stream) {

@@ -121,6 +121,10 @@ def load():
     lib.trs_copy_to_host.restype = i32
     lib.trs_copy_to_device.argtypes = [i32, C.POINTER(vp), C.POINTER(vp), C.POINTER(sz), vp]
     lib.trs_copy_to_device.restype = i32
+    lib.trs_host_register.argtypes = [vp, sz]
+    lib.trs_host_register.restype = i32
+    lib.trs_host_unregister.argtypes = [vp]
+    lib.trs_host_unregister.restype = i32
     lib.trs_pool_trim.argtypes = []
     lib.trs_pool_trim.restype = i32
     lib.trs_build_create_into.argtypes = [vp, vp, vp, i32, C.POINTER(TrsBuildConfig), BuildAlloc, vp, vp, C.POINTER(vp)]
