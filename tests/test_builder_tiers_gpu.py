@@ -51,9 +51,9 @@ def test_key_widths(bits):
 
 
 @pytest.mark.parametrize("window", [16, 5])
-@pytest.mark.parametrize("entries", [1, 63, 255, 256, 257, 1023, 1024, 1025, 4095, 4096, 4097, 9000])
+@pytest.mark.parametrize("entries", [1, 63, 255, 256, 257, 1023, 1024, 1025, 4095, 4096, 4097, 8191, 8192, 8193, 9000, 20000])
 def test_sort_class_borders(entries, window):
-    """A window with exactly that many entries between small and empty ones: sorted by a CTA of the class, or (beyond 4096)
+    """A window with exactly that many entries between small and empty ones: sorted by a CTA of the class, or (beyond 8192)
     by the device-wide passes; columns shared by many rows and columns of one row."""
     g = torch.Generator().manual_seed(entries)
     n_cols = max(2 * entries // window, 3 * window)

@@ -26,7 +26,6 @@
 //      706-733)
 //
 // Input contract: canonical CSR (columns strictly ascending inside a row), window in 1..16.
-#include <cub/block/block_radix_sort.cuh>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_select.cuh>
@@ -56,10 +55,10 @@ struct BuildCfg {
 // ---------------------------------------------------------------------------------------------
 // 0. the sizes, the row pointers and the windows by size: one pass, one read-back
 // ---------------------------------------------------------------------------------------------
-// Size classes of windows by number of entries: sorted by one CTA in shared memory up to sort_cap(2), by
+// Size classes of windows by number of entries: sorted by one CTA in shared memory up to the last sort_cap, by
 // device-wide passes over all larger ones together beyond (hub windows).
-constexpr int kSortClasses = 3;
-__host__ __device__ constexpr int sort_cap(int c) { return 256 << (2 * c); }   // 256, 1024, 4096
+constexpr int kSortClasses = 4;
+__host__ __device__ constexpr int sort_cap(int c) { return c == 0 ? 256 : c == 1 ? 1024 : c == 2 ? 4096 : 8192; }
 
 struct InputInfo {
     int first, last;  // rowptr[0], rowptr[n_rows]
@@ -128,169 +127,200 @@ struct WindowOut {
     int* ncol;
 };
 
-// One CTA per window of at most T * I entries.  A stable block sort by column (entries come in row order, so the rows
-// of a column stay ascending) and one by count, everything in between in shared memory: 12 bytes read and 4 + 17
-// per column written per entry.  Device-wide sorts of (window, column) keys with their key, head and record passes
-// moved ten times that and took 0.69 of the 1.30 ms of a build of the clustered graph; this takes 0.26 ms.  Its bound is
-// the shared-memory pipe and issue, in the digit passes: 5-bit and 6-bit digits, 64 and 256 threads with the same
-// number of entries measured 275 to 322 us against 262.
-template <int T, int I, int RB>
+// One CTA per window of at most CAP entries, everything in shared memory; 12 bytes read and 4 + 17 per column written
+// per entry.  The rows of a window are sorted already, so four rounds merge them two by two: a thread finds where its
+// outputs begin by binary search along the diagonal (merge path) and then takes them one by one.  A record's place in the
+// (count desc, column asc) order is counted, not sorted.
+//
+// What bounds it: issue and the shared-memory pipe.  Device-wide sorts of (window, column) keys with their key, head and
+// record passes moved ten times the bytes: 0.69 of the 1.30 ms of a build of the clustered graph.  A radix sort of the block
+// instead of the merge took 262 us there whatever its digits, a merge with a binary search per entry and round 305; this
+// takes 201 (windows of 780 entries), and 32 in place of 53 on windows of 510.
+template <int T, int CAP, class Key>
 struct WindowSort {
-    static constexpr int N = T * I, CHUNKS = N / 32;
-    using Sort = cub::BlockRadixSort<unsigned, T, I, unsigned short, RB>;
+    static constexpr int PB = CAP <= 256 ? 8 : CAP <= 1024 ? 10 : CAP <= 4096 ? 12 : 13;   // bits of a place in the window
+    static_assert(CAP <= 1 << PB, "");
     struct Smem {
-        union {
-            typename Sort::TempStorage sort;
-            unsigned short place[16 * CHUNKS];   // records of a count in a chunk of 32, then where they go
-        };
-        alignas(16) unsigned key[N];
-        unsigned short idx[N];     // local row << 12 | place in the window
-        unsigned short start[N];   // of the records
-        unsigned mask[N / 2];      // of the records, two in a word
-        int chunk[CHUNKS];         // records that begin in a chunk of 32 entries, then before it
-        int bound[17];             // first entry of every row
-        int warp_sum[T / 32];
+        Key key[2][CAP];           // column << PB | place in the window
+        unsigned char row[CAP];    // row whose entries begin at or before a position
+        unsigned short start[CAP]; // of the records
+        unsigned mask[CAP / 2];    // of the records, two in a word
+        unsigned heads[CAP / 32];  // entries where the column changes
+        int chunk[CAP / 32];       // records that begin in a chunk of 32 entries, then before it
+        int bound[17];             // first entry of every row, from the window's first
+        int warp_sum[32];
     };
 };
 
-template <int T, int I, int RB>
+template <int T, int CAP, class Key>
 __global__ void __launch_bounds__(T) kb_sort_window(const int* __restrict__ rowptr, const int* __restrict__ col,
-                                                    const float* __restrict__ val, int n_rows, int window, int col_bits,
+                                                    const float* __restrict__ val, int n_rows, int window,
                                                     const int* __restrict__ sel, WindowOut out, InputInfo* __restrict__ info) {
-    using S = WindowSort<T, I, RB>;
+    using S = WindowSort<T, CAP, Key>;
+    constexpr int PB = S::PB;
+    constexpr unsigned kPlace = (1u << PB) - 1u;
     extern __shared__ __align__(16) unsigned char smem_raw[];
     typename S::Smem& s = *reinterpret_cast<typename S::Smem*>(smem_raw);
-    static_assert(S::N <= 4096, "the place in the window takes 12 bits");
-    const int tid = threadIdx.x, lane = tid & 31;
+    unsigned short* const cells = reinterpret_cast<unsigned short*>(s.key[1]);   // free after the merge; 16 per chunk of records
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    const unsigned lt = (1u << lane) - 1u;
     const int w = sel[blockIdx.x];
-    if (tid < 17) s.bound[tid] = rowptr[min((long long)w * window + min(tid, window), (long long)n_rows)];
+    const int base = rowptr[(size_t)w * window];
+    if (tid < 17) s.bound[tid] = rowptr[min((long long)w * window + min(tid, window), (long long)n_rows)] - base;
     __syncthreads();
-    const int base = s.bound[0], n = s.bound[16] - base;
-    const unsigned pad = (unsigned)((1ull << col_bits) - 1ull);   // padding stays last: it comes last and the sort is stable
-    for (int i = tid; i < S::N; i += T) s.key[i] = i < n ? (unsigned)col[base + i] : pad;
-    for (int i = tid; i < S::N / 2; i += T) s.mask[i] = 0u;
-    __syncthreads();
-    unsigned key[I];
-    unsigned short idx[I];
-    {
-        const int i0 = tid * I;
-#pragma unroll
-        for (int k = 0; k < I; k += 4) {
-            const uint4 x = *(const uint4*)(s.key + i0 + k);
-            key[k] = x.x; key[k + 1] = x.y; key[k + 2] = x.z; key[k + 3] = x.w;
-        }
-        const unsigned next = i0 + I < S::N ? s.key[i0 + I] : pad;
+    const int n = s.bound[16];
+    bool bad = false;
+    for (int i = tid; i < n; i += T) {
+        const int c = col[base + i];
         int row = 0;
 #pragma unroll
         for (int d = 8; d; d >>= 1)
-            if (row + d < window && s.bound[row + d] - base <= i0) row += d;
-        int row_end = s.bound[row + 1] - base;
-        bool bad = false;
+            if (row + d < window && s.bound[row + d] <= i) row += d;
+        s.key[0][i] = (Key)(unsigned)c << PB | (Key)(unsigned)i;
+        s.row[i] = (unsigned char)row;
+        bad |= c < 0 || (i + 1 < s.bound[row + 1] && col[base + i + 1] <= c);
+    }
+    for (int i = tid; i < (n + 1) / 2; i += T) s.mask[i] = 0u;
+    if (__syncthreads_or(bad)) {   // nothing below holds for unsorted rows
+        if (tid == 0) atomicOr(&info->err, 2);
+        return;
+    }
+    // outputs per thread and round; odd, so that the threads' stores fall into different banks
+    const int per = ((n + T - 1) / T) | 1, o0 = tid * per, o1 = min(o0 + per, n);
+    constexpr Key kNone = ~(Key)0;
 #pragma unroll
-        for (int k = 0; k < I; ++k) {
-            const int i = i0 + k;
-            while (i >= row_end && row + 1 < window) row_end = s.bound[++row + 1] - base;
-            idx[k] = (unsigned short)(row << 12 | i);
-            if (i < n) bad |= key[k] > pad || (i + 1 < row_end && (k + 1 < I ? key[k + 1 < I ? k + 1 : k] : next) <= key[k]);
+    for (int L = 0; L < 4; ++L) {
+        const Key* const src = s.key[L & 1];
+        Key* const dst = s.key[1 - (L & 1)];
+        if (o0 < n) {
+            int pair = s.row[o0] >> (L + 1);
+            int s0 = s.bound[pair << (L + 1)], s1 = s.bound[(2 * pair + 1) << L], s2 = s.bound[(pair + 1) << (L + 1)];
+            // how many of the pair's first o0 - s0 outputs come from its first run
+            const int d = o0 - s0;
+            int lo = max(0, d - (s2 - s1)), hi = min(d, s1 - s0);
+            while (lo < hi) {
+                const int mid = (lo + hi) >> 1;
+                if (src[s0 + mid] < src[s1 + d - 1 - mid]) lo = mid + 1; else hi = mid;
+            }
+            int i = s0 + lo, j = s1 + d - lo;
+            Key a = i < s1 ? src[i] : kNone, b = j < s2 ? src[j] : kNone;
+            for (int p = o0;;) {
+                const bool first = a < b;
+                dst[p] = first ? a : b;
+                if (++p == o1) break;
+                if (p == s2) {   // on to the next pair that has entries
+                    do {
+                        ++pair;
+                        s0 = s2;
+                        s1 = s.bound[(2 * pair + 1) << L];
+                        s2 = s.bound[(pair + 1) << (L + 1)];
+                    } while (s2 == s0);
+                    i = s0; j = s1;
+                    a = i < s1 ? src[i] : kNone;
+                    b = j < s2 ? src[j] : kNone;
+                } else if (first) {
+                    ++i;
+                    a = i < s1 ? src[i] : kNone;
+                } else {
+                    ++j;
+                    b = j < s2 ? src[j] : kNone;
+                }
+            }
         }
-        if (bad) atomicOr(&info->err, 2);
+        __syncthreads();
     }
-    __syncthreads();
-    typename S::Sort(s.sort).SortBlockedToStriped(key, idx, 0, col_bits);
-    // sorted entry k * T + tid is this thread's k-th: a warp holds chunks of 32 neighbours
-#pragma unroll
-    for (int k = 0; k < I; ++k) {
-        s.key[k * T + tid] = key[k];
-        s.idx[k * T + tid] = idx[k];
-    }
-    __syncthreads();
+    const Key* const key = s.key[0];
     // records begin where the column changes
-    unsigned heads[I];
-#pragma unroll
-    for (int k = 0; k < I; ++k) {
-        const int i = k * T + tid;
-        heads[k] = __ballot_sync(0xffffffffu, i < n && (i == 0 || s.key[i > 0 ? i - 1 : 0] != key[k]));
-        if (lane == 0) s.chunk[i >> 5] = __popc(heads[k]);
+    const int chunks = (n + 31) / 32;
+    for (int c = wid; c < chunks; c += T / 32) {
+        const int i = c * 32 + lane;
+        const bool head = i < n && (i == 0 || (key[i] >> PB) != (key[i > 0 ? i - 1 : 0] >> PB));
+        const unsigned heads = __ballot_sync(0xffffffffu, head);
+        if (lane == 0) {
+            s.heads[c] = heads;
+            s.chunk[c] = __popc(heads);
+        }
     }
     __syncthreads();
     if (tid < 32) {
         int before = 0;
-        for (int c0 = 0; c0 < S::CHUNKS; c0 += 32) {
-            const int x = c0 + lane < S::CHUNKS ? s.chunk[c0 + lane] : 0;
+        for (int c0 = 0; c0 < chunks; c0 += 32) {
+            const int x = c0 + lane < chunks ? s.chunk[c0 + lane] : 0;
             int sum = x;
 #pragma unroll
             for (int d = 1; d < 32; d <<= 1) {
                 const int y = __shfl_up_sync(0xffffffffu, sum, d);
                 if (lane >= d) sum += y;
             }
-            if (c0 + lane < S::CHUNKS) s.chunk[c0 + lane] = before + sum - x;
+            if (c0 + lane < chunks) s.chunk[c0 + lane] = before + sum - x;
             before += __shfl_sync(0xffffffffu, sum, 31);
         }
         if (lane == 0) s.warp_sum[0] = before;
     }
     __syncthreads();
     const int D = s.warp_sum[0];
-#pragma unroll
-    for (int k = 0; k < I; ++k) {
-        const int i = k * T + tid;
-        if (i - lane >= n) break;
-        const unsigned upto = heads[k] & (0xffffffffu >> (31 - lane));
-        const int r = s.chunk[i >> 5] + __popc(upto) - 1, seg = upto ? 31 - __clz(upto) : 0;   // no head yet: a record goes on
-        unsigned m = i < n ? 1u << (idx[k] >> 12) : 0u;
+    for (int c = wid; c < chunks; c += T / 32) {
+        const int i = c * 32 + lane;
+        const unsigned heads = s.heads[c], upto = heads & (0xffffffffu >> (31 - lane));
+        const int r = s.chunk[c] + __popc(upto) - 1, seg = upto ? 31 - __clz(upto) : 0;   // no head yet: a record goes on
+        unsigned m = 0u;
+        if (i < n) {
+            const unsigned place = (unsigned)key[i] & kPlace;
+            out.sval[base + i] = val[base + place];
+            m = 1u << s.row[place];
+        }
 #pragma unroll
         for (int d = 1; d < 16; d <<= 1) {   // at most 16 entries share a column
             const unsigned y = __shfl_up_sync(0xffffffffu, m, d);
             if (lane - d >= seg) m |= y;
         }
         if (i < n) {
-            if ((heads[k] >> lane) & 1u) s.start[r] = (unsigned short)i;
-            if (lane == 31 || i + 1 == n || ((heads[k] >> (lane + 1)) & 1u)) atomicOr(&s.mask[r >> 1], m << (16 * (r & 1)));
+            if ((heads >> lane) & 1u) s.start[r] = (unsigned short)i;
+            if (lane == 31 || i + 1 == n || ((heads >> (lane + 1)) & 1u)) atomicOr(&s.mask[r >> 1], m << (16 * (r & 1)));
         }
     }
-    for (int i = tid; i < n; i += T) out.sval[base + i] = val[base + (s.idx[i] & 0xfff)];
-    __syncthreads();
-    const unsigned short* const masks = (const unsigned short*)s.mask;
-    const int chunks = (D + 31) / 32, cells = 16 * chunks;
-    for (int i = tid; i < cells; i += T) s.place[i] = 0;   // the sort's memory: its last readers are barriers back
-    __syncthreads();
     // (count desc, column asc): records keep their order inside a count, so a record's place is the number of records of
     // larger counts, of its count in earlier chunks of 32, and of its count before it in its own chunk
-    const unsigned lt = (1u << lane) - 1u;
-    for (int c = tid >> 5; c < chunks; c += T / 32) {
+    const unsigned short* const masks = (const unsigned short*)s.mask;
+    const int rchunks = (D + 31) / 32, ncells = 16 * rchunks;
+    for (int i = tid; i < ncells; i += T) cells[i] = 0;
+    __syncthreads();
+    for (int c = wid; c < rchunks; c += T / 32) {
         const int q = c * 32 + lane;
         const int k = q < D ? 16 - __popc((unsigned)masks[q]) : 16;
         const unsigned same = __match_any_sync(0xffffffffu, k);
-        if (k < 16 && (same & lt) == 0) s.place[k * chunks + c] = (unsigned short)__popc(same);
+        if (k < 16 && (same & lt) == 0) cells[k * rchunks + c] = (unsigned short)__popc(same);
     }
     __syncthreads();
     int before = 0;   // exclusive sums over the cells, T at a time
-    for (int c0 = 0; c0 < cells; c0 += T) {
-        const int i = c0 + tid, x = i < cells ? s.place[i] : 0;
+    for (int c0 = 0; c0 < ncells; c0 += T) {
+        const int i = c0 + tid, x = i < ncells ? cells[i] : 0;
         int sum = x;
 #pragma unroll
         for (int d = 1; d < 32; d <<= 1) {
             const int y = __shfl_up_sync(0xffffffffu, sum, d);
             if (lane >= d) sum += y;
         }
-        if (lane == 31) s.warp_sum[tid >> 5] = sum;
+        if (lane == 31) s.warp_sum[wid] = sum;
         __syncthreads();
         int at = before + sum - x;
 #pragma unroll
         for (int q = 0; q < T / 32; ++q) {
-            if (q < (tid >> 5)) at += s.warp_sum[q];
+            if (q < wid) at += s.warp_sum[q];
             before += s.warp_sum[q];
         }
-        if (i < cells) s.place[i] = (unsigned short)at;
+        if (i < ncells) cells[i] = (unsigned short)at;
         __syncthreads();
     }
-    for (int c = tid >> 5; c < chunks; c += T / 32) {
+    for (int c = wid; c < rchunks; c += T / 32) {
         const int q = c * 32 + lane;
         const int k = q < D ? 16 - __popc((unsigned)masks[q]) : 16;
         const unsigned same = __match_any_sync(0xffffffffu, k);
         if (k == 16) continue;
         const int st = s.start[q];
-        const size_t o = (size_t)base + s.place[k * chunks + c] + __popc(same & lt);
-        out.rec[o] = Record{(int)s.key[st], base + st, masks[q], val[base + (s.idx[st] & 0xfff)]};
+        const Key first = key[st];
+        const size_t o = (size_t)base + cells[k * rchunks + c] + __popc(same & lt);
+        out.rec[o] = Record{(int)(first >> PB), base + st, masks[q], val[base + ((unsigned)first & kPlace)]};
         out.cnt[o] = (unsigned char)(16 - k);
     }
     if (tid == 0) out.ncol[w] = D;
@@ -1512,16 +1542,23 @@ struct Records {   // stages 1 - 3
     int* sel = nullptr;   // [kSortClasses + 1][W]
 };
 
-template <int T, int I, int RB>
-int sort_class(int c, const InputInfo& info, const int* rowptr, const int* col, const float* val, const trs_builder* B, int col_bits,
-               const Records& R, InputInfo* d_info, cudaStream_t st) {
-    if (info.windows[c] == 0) return 0;
-    constexpr int smem = (int)sizeof(typename WindowSort<T, I, RB>::Smem);
-    auto kernel = kb_sort_window<T, I, RB>;
+template <int T, class Key, int C>
+int sort_class_as(const InputInfo& info, const int* rowptr, const int* col, const float* val, const trs_builder* B, const Records& R,
+                  InputInfo* d_info, cudaStream_t st) {
+    constexpr int CAP = sort_cap(C), smem = (int)sizeof(typename WindowSort<T, CAP, Key>::Smem);
+    auto kernel = kb_sort_window<T, CAP, Key>;
     if (smem > 48 * 1024) TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    kernel<<<info.windows[c], T, smem, st>>>(rowptr, col, val, B->n_rows, B->cfg.window, col_bits, R.sel + (size_t)c * B->W, R.w, d_info);
+    kernel<<<info.windows[C], T, smem, st>>>(rowptr, col, val, B->n_rows, B->cfg.window, R.sel + (size_t)C * B->W, R.w, d_info);
     TRS_LAUNCH_CHECK();
     return 0;
+}
+template <int T, int C>
+int sort_class(const InputInfo& info, const int* rowptr, const int* col, const float* val, const trs_builder* B, int col_bits,
+               const Records& R, InputInfo* d_info, cudaStream_t st) {
+    if (info.windows[C] == 0) return 0;
+    return col_bits + WindowSort<T, sort_cap(C), unsigned>::PB <= 32
+               ? sort_class_as<T, unsigned, C>(info, rowptr, col, val, B, R, d_info, st)
+               : sort_class_as<T, u64, C>(info, rowptr, col, val, B, R, d_info, st);
 }
 
 template <class Key>
@@ -1588,9 +1625,10 @@ int make_records(trs_builder* B, const int* rowptr, const int* col, const float*
         TRS_TRY(col_bits + h_bits <= 32 ? sort_hubs<unsigned>(B, rowptr, col, val, info, d_info, d_count, col_bits, ts, cub_, st, *R)
                                         : sort_hubs<u64>(B, rowptr, col, val, info, d_info, d_count, col_bits, ts, cub_, st, *R));
     }
-    TRS_TRY((sort_class<512, 8, 4>(2, info, rowptr, col, val, B, col_bits, *R, d_info, st)));
-    TRS_TRY((sort_class<128, 8, 4>(1, info, rowptr, col, val, B, col_bits, *R, d_info, st)));
-    TRS_TRY((sort_class<64, 4, 4>(0, info, rowptr, col, val, B, col_bits, *R, d_info, st)));
+    TRS_TRY((sort_class<1024, 3>(info, rowptr, col, val, B, col_bits, *R, d_info, st)));
+    TRS_TRY((sort_class<512, 2>(info, rowptr, col, val, B, col_bits, *R, d_info, st)));
+    TRS_TRY((sort_class<128, 1>(info, rowptr, col, val, B, col_bits, *R, d_info, st)));
+    TRS_TRY((sort_class<64, 0>(info, rowptr, col, val, B, col_bits, *R, d_info, st)));
     return 0;
 }
 
