@@ -1363,18 +1363,12 @@ __global__ void kb_cuda_extras(int window, const int* __restrict__ win_cuda_unit
     po.put(o, off[row + 1].zl - o.zl, rank, c, r.sval[x.at[i]]);
 }
 
-// sizes that the host needs after the matching, in one place
-struct Totals {
-    int groups, tiles, tc_nnz, pad;
-    Parts parts;
-};
-__global__ void kb_totals(const int* __restrict__ s_offset, const int* __restrict__ tile_off, int W,
-                          const int* __restrict__ blk_off, int NB, const Parts* __restrict__ part_off, int n_rows,
-                          Totals* __restrict__ t) {
-    t->groups = s_offset[W];
-    t->tiles = tile_off[W];
-    t->tc_nnz = blk_off[NB];
-    if (part_off) t->parts = part_off[n_rows];
+// Two runs of words into pinned host memory: a copy of a few words took 3.4 us behind a gap of up to 8 on the copy
+// engine, this takes 2 behind 1.
+__global__ void kb_publish(const int* __restrict__ a, int na, int* __restrict__ host_a, const int* __restrict__ b, int nb,
+                           int* __restrict__ host_b) {
+    for (int i = threadIdx.x; i < na; i += blockDim.x) host_a[i] = a[i];
+    for (int i = threadIdx.x; i < nb; i += blockDim.x) host_b[i] = b[i];
 }
 
 __global__ void kb_to_half(const float* __restrict__ src, long long n, __half* __restrict__ dst) {
@@ -1489,9 +1483,12 @@ struct Cub {
 struct Mirror {
     static constexpr size_t kBytes = 2048;
     unsigned char* p = nullptr;
+    cudaStream_t st = nullptr;
+    bool pending = true;   // a kernel on `st` may still write here
     static std::mutex& lock() { static std::mutex m; return m; }
     static std::vector<unsigned char*>& idle() { static std::vector<unsigned char*> v; return v; }
-    int take() {
+    int take(cudaStream_t stream) {
+        st = stream;
         {
             std::lock_guard<std::mutex> g(lock());
             if (!idle().empty()) { p = idle().back(); idle().pop_back(); return 0; }
@@ -1501,14 +1498,28 @@ struct Mirror {
     }
     ~Mirror() {
         if (!p) return;
+        if (pending) cudaStreamSynchronize(st);
         std::lock_guard<std::mutex> g(lock());
         idle().push_back(p);
     }
 };
 
+// what a build reads back, from the device into a Mirror; the host may look after an event or a synchronisation behind it
+template <class A, class B>
+int publish(const A* a, A* host_a, const B* b, B* host_b, cudaStream_t st) {
+    kb_publish<<<1, 128, 0, st>>>((const int*)a, (int)(sizeof(A) / 4), (int*)host_a, (const int*)b, (int)(sizeof(B) / 4), (int*)host_b);
+    TRS_LAUNCH_CHECK();
+    return 0;
+}
+template <class T>
+int publish(const T* dev, T* host, cudaStream_t st) {
+    kb_publish<<<1, 128, 0, st>>>((const int*)dev, (int)(sizeof(T) / 4), (int*)host, nullptr, 0, nullptr);
+    TRS_LAUNCH_CHECK();
+    return 0;
+}
 template <class T>
 int read_back(const T* dev, T* host, cudaStream_t st) {
-    TRS_CUDA(cudaMemcpyAsync(host, dev, sizeof(T), cudaMemcpyDeviceToHost, st));
+    TRS_TRY(publish(dev, host, st));
     TRS_CUDA(cudaStreamSynchronize(st));
     return 0;
 }
@@ -1532,6 +1543,10 @@ struct Event {
     int record(cudaStream_t st) {
         if (!e) TRS_CUDA(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
         TRS_CUDA(cudaEventRecord(e, st));
+        return 0;
+    }
+    int wait() const {
+        TRS_CUDA(cudaEventSynchronize(e));
         return 0;
     }
     ~Event() { if (e) cudaEventDestroy(e); }
@@ -1561,9 +1576,10 @@ int sort_class(const InputInfo& info, const int* rowptr, const int* col, const f
                : sort_class_as<T, u64, C>(info, rowptr, col, val, B, R, d_info, st);
 }
 
-template <class Key>
+// `meanwhile` queues what does not depend on the hub windows
+template <class Key, class Other>
 int sort_hubs(trs_builder* B, const int* rowptr, const int* col, const float* val, const InputInfo& info, InputInfo* d_info,
-              int* d_count, int col_bits, TempSpace& ts, Cub& cub_, cudaStream_t st, const Records& R) {
+              int* d_count, int* h_count, int col_bits, TempSpace& ts, Cub& cub_, cudaStream_t st, const Records& R, Other&& meanwhile) {
     const int H = info.windows[kSortClasses], E = (int)info.hub_entries, n = B->n_rows, window = B->cfg.window;
     const int h_bits = bits_for(H - 1);
     const int* sel = R.sel + (size_t)kSortClasses * B->W;
@@ -1589,8 +1605,10 @@ int sort_hubs(trs_builder* B, const int* rowptr, const int* col, const float* va
     TRS_TRY(cub_.run([&](void* t, size_t& b) {
         return cub::DeviceSelect::If(t, b, thrust::counting_iterator<int>(0), start, d_count, E, is_head, st);
     }));
-    int D = 0;
-    TRS_TRY(read_back(d_count, &D, st));
+    TRS_TRY(publish(d_count, h_count, st));
+    TRS_TRY(meanwhile());
+    TRS_CUDA(cudaStreamSynchronize(st));
+    const int D = *h_count;
     Record* record;
     unsigned *key2_a, *key2_b, *key2;
     int *ord_a, *ord_b, *ord;
@@ -1611,8 +1629,11 @@ int sort_hubs(trs_builder* B, const int* rowptr, const int* col, const float* va
     return 0;
 }
 
+// The hub windows are a chain of small launches with a read-back in it (R-MAT 15: 160 us) and the classes keep the chip
+// half busy one after the other (R-MAT 18: 180 us): with more than one of them in a graph, two other streams take the
+// classes beside the chain (whole build of R-MAT 15 662 -> 541 us, of R-MAT 18 1470 -> 1338, with the sizes read back by kernels).
 int make_records(trs_builder* B, const int* rowptr, const int* col, const float* val, const InputInfo& info, InputInfo* d_info,
-                 int* d_count, TempSpace& ts, Cub& cub_, cudaStream_t st, Records* R) {
+                 int* d_count, int* h_count, TempSpace& ts, Cub& cub_, cudaStream_t st, Records* R) {
     const int col_bits = bits_for(info.max_col), W = B->W;
     const size_t nnz = (size_t)B->nnz;
     TRS_TRY(ts.get(nnz, &R->w.rec));
@@ -1620,16 +1641,36 @@ int make_records(trs_builder* B, const int* rowptr, const int* col, const float*
     TRS_TRY(ts.get(nnz, &R->w.cnt));
     TRS_TRY(ts.get((size_t)W, &R->w.ncol));
     TRS_CUDA(cudaMemsetAsync(R->w.ncol, 0, sizeof(int) * (size_t)W, st));
+    int parts = 0;
+    for (int c = 0; c <= kSortClasses; ++c) parts += info.windows[c] > 0;
+    const bool fork = parts > 1;
+    cudaStream_t side[2] = {st, st};
+    Event ready, done[2];
+    if (fork) {
+        TRS_TRY(side_streams(side));
+        TRS_TRY(ready.record(st));
+        for (cudaStream_t s : side) TRS_CUDA(cudaStreamWaitEvent(s, ready.e, 0));
+    }
+    auto classes = [&]() -> int {
+        TRS_TRY((sort_class<1024, 3>(info, rowptr, col, val, B, col_bits, *R, d_info, side[0])));
+        TRS_TRY((sort_class<512, 2>(info, rowptr, col, val, B, col_bits, *R, d_info, side[1])));
+        TRS_TRY((sort_class<128, 1>(info, rowptr, col, val, B, col_bits, *R, d_info, side[0])));
+        return sort_class<64, 0>(info, rowptr, col, val, B, col_bits, *R, d_info, side[1]);
+    };
+    int rc = 0;
     if (info.windows[kSortClasses] > 0) {
         const int h_bits = bits_for(info.windows[kSortClasses] - 1);
-        TRS_TRY(col_bits + h_bits <= 32 ? sort_hubs<unsigned>(B, rowptr, col, val, info, d_info, d_count, col_bits, ts, cub_, st, *R)
-                                        : sort_hubs<u64>(B, rowptr, col, val, info, d_info, d_count, col_bits, ts, cub_, st, *R));
+        rc = col_bits + h_bits <= 32 ? sort_hubs<unsigned>(B, rowptr, col, val, info, d_info, d_count, h_count, col_bits, ts, cub_, st, *R, classes)
+                                     : sort_hubs<u64>(B, rowptr, col, val, info, d_info, d_count, h_count, col_bits, ts, cub_, st, *R, classes);
+    } else {
+        rc = classes();
     }
-    TRS_TRY((sort_class<1024, 3>(info, rowptr, col, val, B, col_bits, *R, d_info, st)));
-    TRS_TRY((sort_class<512, 2>(info, rowptr, col, val, B, col_bits, *R, d_info, st)));
-    TRS_TRY((sort_class<128, 1>(info, rowptr, col, val, B, col_bits, *R, d_info, st)));
-    TRS_TRY((sort_class<64, 0>(info, rowptr, col, val, B, col_bits, *R, d_info, st)));
-    return 0;
+    if (fork)
+        for (int i = 0; i < 2; ++i) {   // after an error too: what is freed next may still be in use
+            TRS_TRY(done[i].record(side[i]));
+            TRS_CUDA(cudaStreamWaitEvent(st, done[i].e, 0));
+        }
+    return rc;
 }
 
 int empty_outputs(trs_builder* B, cudaStream_t st) {
@@ -1658,29 +1699,29 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     Cub cub_(ts, st);
 
     // ---- sizes of the input ---------------------------------------------------------------------
-    struct Head { InputInfo info; MatchCounts mc; Totals tot; int count; u64 dropped[kDropCounters]; };
-    struct Back { Head head; Win total; Parts parts; };   // what the host sees of it
+    struct Counts { InputInfo info; MatchCounts mc; };
+    struct Head { Counts counts; u64 dropped[kDropCounters]; int hub_records, pad; };
+    struct Back { Head head; Win total; Parts parts; int groups, tiles, tc_nnz; };   // what the host sees of it
     static_assert(sizeof(Back) <= Mirror::kBytes, "");
     Mirror mirror;
-    TRS_TRY(mirror.take());
+    TRS_TRY(mirror.take(st));
     Back* const back = (Back*)mirror.p;
     Head* d_head;
     TRS_TRY(ts.get(1, &d_head));
     TRS_CUDA(cudaMemsetAsync(d_head, 0, sizeof(Head), st));
     Records R;
     TRS_TRY(ts.get((size_t)(kSortClasses + 1) * W, &R.sel));
-    kb_input_info<<<2 * sms, 512, 0, st>>>(rowptr, col, n, window, W, R.sel, &d_head->info);
+    kb_input_info<<<2 * sms, 512, 0, st>>>(rowptr, col, n, window, W, R.sel, &d_head->counts.info);
     TRS_LAUNCH_CHECK();
-    auto sync_head = [&]() { return read_back(d_head, &back->head, st); };
-    TRS_TRY(sync_head());
-    const InputInfo info = back->head.info;
+    TRS_TRY(read_back(&d_head->counts.info, &back->head.counts.info, st));
+    const InputInfo info = back->head.counts.info;
     if (info.first != 0 || info.last < 0 || (info.err & 1)) return TRS_E_OFFSETS;
     const long long nnz = B->nnz = info.last;
     if (nnz == 0) return empty_outputs(B, st);
-    ts.chunk_bytes = std::max((size_t)16 << 20, (size_t)nnz * 24);
+    ts.chunk_bytes = std::max((size_t)16 << 20, (size_t)nnz * 28);
 
     // ---- 1. - 3. columns of every window in (count desc, col asc) order ---------------------------
-    TRS_TRY(make_records(B, rowptr, col, val, info, &d_head->info, &d_head->count, ts, cub_, st, &R));
+    TRS_TRY(make_records(B, rowptr, col, val, info, &d_head->counts.info, &d_head->hub_records, &back->head.hub_records, ts, cub_, st, &R));
     const RecordView rv{R.w.rec, R.w.sval};
 
     // ---- 4., 5. TC columns, units, sizes per window ---------------------------------------------
@@ -1693,27 +1734,57 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     TRS_TRY(ts.get((size_t)W + 1, &pre));
     TRS_TRY(ts.get((size_t)W + 1, &sel_block));
     TRS_TRY(ts.get((size_t)W + 1, &sel_huge));
-    kb_windows<<<grid_for(W + 1, 128), 128, 0, st>>>(rowptr, R.w.ncol, R.w.cnt, W, cfg, rec, end, tc, win, sel_block, sel_huge, &d_head->mc);
+    kb_windows<<<grid_for(W + 1, 128), 128, 0, st>>>(rowptr, R.w.ncol, R.w.cnt, W, cfg, rec, end, tc, win, sel_block, sel_huge, &d_head->counts.mc);
     TRS_LAUNCH_CHECK();
     TRS_TRY(cub_.exclusive_scan(win, pre, WinSum(), Win{0, 0, 0, 0}, W + 1));
     const WindowView v{rec, end, tc, pre};
-    TRS_CUDA(cudaMemcpyAsync(&back->total, pre + W, sizeof(Win), cudaMemcpyDeviceToHost, st));
-    TRS_TRY(sync_head());
-    if (back->head.info.err & 2) return TRS_E_NOT_CANONICAL;
-    const Win total = back->total;
-    const MatchCounts mc = back->head.mc;
-    B->distinct_cols = (long long)mc.records;
-    const int NB = total.blocks, NP = total.parts, TU = total.units, TS = total.slots;
-    B->units = TU;
+    Event sized, grouped, counted;
+    TRS_TRY(publish(&d_head->counts, &back->head.counts, (const Win*)pre + W, &back->total, st));
+    TRS_TRY(sized.record(st));
 
     // ---- 6. matching ------------------------------------------------------------------------------
     MatchOut mo;
-    TRS_TRY(ts.get(TU, &mo.order));
-    TRS_TRY(ts.get(TS, &mo.pair_a));
-    TRS_TRY(ts.get(TS, &mo.pair_b));
-    TRS_TRY(ts.get((size_t)W + 1, &mo.groups));
-    TRS_TRY(ts.get((size_t)W + 1, &mo.tiles));
-    TRS_TRY(ts.get((size_t)W + 1, &mo.cuda_unit));
+    auto match_arrays = [&](size_t units, size_t slots) -> int {
+        TRS_TRY(ts.get(units, &mo.order));
+        TRS_TRY(ts.get(slots, &mo.pair_a));
+        TRS_TRY(ts.get(slots, &mo.pair_b));
+        TRS_TRY(ts.get((size_t)W + 1, &mo.groups));
+        TRS_TRY(ts.get((size_t)W + 1, &mo.tiles));
+        return ts.get((size_t)W + 1, &mo.cuda_unit);
+    };
+    auto match_warps = [&](int max_units) -> int {
+        const int units = std::max(32, (max_units + 31) & ~31);
+        const size_t smem = (size_t)kMatchWarps * (units + units / 32) * 4;
+        kb_match_warp<<<grid_for(W + 1, kMatchWarps), 32 * kMatchWarps, smem, st>>>(v, W, R.w.cnt, cfg.unit_min_nnz, units, mo);
+        TRS_LAUNCH_CHECK();
+        return 0;
+    };
+    // the sizes of the groups go to the host before the TC blocks are made, so that it lays out their arrays meanwhile
+    auto group_sizes = [&]() -> int {
+        TRS_TRY(B->out(B->s_offset, 22, (size_t)W + 1));
+        TRS_TRY(B->out(B->s_window_tile_offset, 28, (size_t)W + 1));
+        TRS_TRY(cub_.exclusive_sum(mo.groups, B->s_offset.p, W + 1));
+        TRS_TRY(cub_.exclusive_sum(mo.tiles, B->s_window_tile_offset.p, W + 1));
+        TRS_TRY(publish((const int*)B->s_offset.p + W, &back->groups, (const int*)B->s_window_tile_offset.p + W, &back->tiles, st));
+        return grouped.record(st);
+    };
+    // Without large windows the bounds are close enough to start before the sizes have come back (30 us of 870 on the
+    // clustered graph).  With them the words of every warp would take the shared memory of many.
+    const bool ahead = info.windows[2] == 0 && info.windows[3] == 0 && info.windows[kSortClasses] == 0;
+    static_assert(sort_cap(1) / 2 <= kWarpUnits, "");
+    if (ahead) {
+        TRS_TRY(match_arrays((size_t)nnz / 2 + W, (size_t)nnz / 4 + W));
+        TRS_TRY(match_warps(sort_cap(info.windows[1] > 0 ? 1 : 0) / 2));
+        TRS_TRY(group_sizes());
+    }
+    TRS_TRY(sized.wait());
+    if (back->head.counts.info.err & 2) return TRS_E_NOT_CANONICAL;
+    const Win total = back->total;
+    const MatchCounts mc = back->head.counts.mc;
+    B->distinct_cols = (long long)mc.records;
+    const int NB = total.blocks, NP = total.parts, TU = total.units, TS = total.slots;
+    B->units = TU;
+    if (!ahead) TRS_TRY(match_arrays(TU, TS));
     if (mc.max_huge >= (int)kUnitMask) return TRS_E_LIMIT;
     // one long chain per hub window: the tiers run side by side
     cudaStream_t side[2] = {st, st};
@@ -1742,18 +1813,7 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
                                                                                    nullptr, sel_block, mo);
         TRS_LAUNCH_CHECK();
     }
-    {
-        const int units = std::max(32, (mc.max_warp + 31) & ~31);
-        const size_t smem = (size_t)kMatchWarps * (units + units / 32) * 4;
-        kb_match_warp<<<grid_for(W + 1, kMatchWarps), 32 * kMatchWarps, smem, st>>>(v, W, R.w.cnt, cfg.unit_min_nnz, units, mo);
-        TRS_LAUNCH_CHECK();
-    }
-    if (mc.n_huge > 0) { TRS_TRY(done[0].record(side[0])); TRS_CUDA(cudaStreamWaitEvent(st, done[0].e, 0)); }
-    if (mc.n_block > 0) { TRS_TRY(done[1].record(side[1])); TRS_CUDA(cudaStreamWaitEvent(st, done[1].e, 0)); }
-    TRS_TRY(B->out(B->s_offset, 22, (size_t)W + 1));
-    TRS_TRY(B->out(B->s_window_tile_offset, 28, (size_t)W + 1));
-    TRS_TRY(cub_.exclusive_sum(mo.groups, B->s_offset.p, W + 1));
-    TRS_TRY(cub_.exclusive_sum(mo.tiles, B->s_window_tile_offset.p, W + 1));
+    if (!ahead) TRS_TRY(match_warps(mc.max_warp));
 
     // ---- 8. TC blocks (their values need the block offsets) --------------------------------------
     int *blk_nnz, *slot_rec;
@@ -1765,6 +1825,11 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     kb_tc_blocks<<<grid_for(NB + 1, 128), 128, 0, st>>>(v, rv, W, NB, B->t_column.p, B->t_binary.p, blk_nnz, slot_rec);
     TRS_LAUNCH_CHECK();
     TRS_TRY(cub_.exclusive_sum(blk_nnz, B->t_block_offset.p, (long long)NB + 1));
+    if (!ahead) {   // the hub windows are matched by now
+        if (mc.n_huge > 0) { TRS_TRY(done[0].record(side[0])); TRS_CUDA(cudaStreamWaitEvent(st, done[0].e, 0)); }
+        if (mc.n_block > 0) { TRS_TRY(done[1].record(side[1])); TRS_CUDA(cudaStreamWaitEvent(st, done[1].e, 0)); }
+        TRS_TRY(group_sizes());
+    }
     TRS_TRY(B->out(B->t_row_offset, 0, (size_t)NP + 1));
     TRS_TRY(B->out(B->t_window_row, 4, NP));
     TRS_TRY(B->out(B->t_atomic, 5, NP));
@@ -1782,20 +1847,16 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
         return cub_.exclusive_scan(cnt, off, PartsSum(), Parts{0, 0, 0, 0}, (long long)n + 1);
     };
     if (!cfg.strict) TRS_TRY(count_parts());
-    kb_totals<<<1, 1, 0, st>>>(B->s_offset.p, B->s_window_tile_offset.p, W, B->t_block_offset.p, NB, cfg.strict ? nullptr : off, n,
-                               &d_head->tot);
-    TRS_LAUNCH_CHECK();
-    TRS_TRY(sync_head());
-    Totals tot = back->head.tot;
-    const int G = tot.groups, T = tot.tiles;
-
-    TRS_TRY(B->out(B->t_value, 3, tot.tc_nnz));
-    if (NB > 0) {
-        kb_tc_values<<<grid_for((long long)NB * 128), 256, 0, st>>>(rv, slot_rec, NB, B->t_binary.p, B->t_block_offset.p, B->t_value.p);
-        TRS_LAUNCH_CHECK();
+    if (cfg.strict) {
+        TRS_TRY(publish((const int*)B->t_block_offset.p + NB, &back->tc_nnz, st));
+    } else {
+        TRS_TRY(publish((const int*)B->t_block_offset.p + NB, &back->tc_nnz, (const Parts*)off + n, &back->parts, st));
     }
+    TRS_TRY(counted.record(st));
 
     // ---- 7. groups and tiles ------------------------------------------------------------------------
+    TRS_TRY(grouped.wait());
+    const int G = back->groups, T = back->tiles;
     TRS_TRY(B->out(B->s_column, 17, (size_t)G * 4));
     TRS_TRY(B->out(B->s_mask, 18, (size_t)G * window));
     TRS_TRY(B->out(B->s_value, 19, (size_t)G * window * 2));
@@ -1824,8 +1885,14 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
                                                                            T, window, mo.pair_a, mo.pair_b, go, xo);
         TRS_LAUNCH_CHECK();
     }
+    TRS_TRY(counted.wait());
+    TRS_TRY(B->out(B->t_value, 3, back->tc_nnz));
+    if (NB > 0) {
+        kb_tc_values<<<grid_for((long long)NB * 128), 256, 0, st>>>(rv, slot_rec, NB, B->t_binary.p, B->t_block_offset.p, B->t_value.p);
+        TRS_LAUNCH_CHECK();
+    }
     if (cfg.strict) {
-        TRS_TRY(sync_head());
+        TRS_TRY(read_back(&d_head->dropped, &back->head.dropped, st));
         const u64 n_extra = back->head.dropped[0];
         if (n_extra > 0) {
             u64* key;
@@ -1836,10 +1903,9 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
             x = Extras{key, at, (int)n_extra};
         }
         TRS_TRY(count_parts());
-        TRS_TRY(read_back(off + n, &back->parts, st));
-        tot.parts = back->parts;
+        TRS_TRY(read_back((const Parts*)off + n, &back->parts, st));
     }
-    const Parts& p = tot.parts;
+    const Parts p = back->parts;
     TRS_TRY(B->out(B->c_row_offset, 7, (size_t)p.nl + 1));
     TRS_TRY(B->out(B->c_row, 8, p.nl));
     TRS_TRY(B->out(B->c_atomic, 9, p.nl));
@@ -1858,7 +1924,8 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
         kb_cuda_extras<<<grid_for(x.n), 256, 0, st>>>(window, mo.cuda_unit, v, rv, x, off, po);
         TRS_LAUNCH_CHECK();
     }
-    TRS_TRY(sync_head());
+    TRS_TRY(read_back(&d_head->dropped, &back->head.dropped, st));
+    mirror.pending = false;
     B->dropped = 0;
     if (!cfg.strict)   // nothing is lost in strict mode
         for (u64 d : back->head.dropped) B->dropped += d;
