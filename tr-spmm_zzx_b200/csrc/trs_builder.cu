@@ -975,13 +975,21 @@ __global__ void __launch_bounds__(kBlockThreads) kb_match_block(WindowView v, co
 // ---------------------------------------------------------------------------------------------
 // 7. groups and tiles
 // ---------------------------------------------------------------------------------------------
-__global__ void kb_tiles(const int* __restrict__ tile_off, const int* __restrict__ s_offset, int W, int T,
-                         int* __restrict__ s_tile_window, int* __restrict__ s_tile_group) {
+struct __align__(16) TileSource {   // where a tile's columns come from
+    int slot;    // of its first group in the pair lists
+    int rec;     // first record of the window that is in a unit
+    int ncol;    // how many of them
+    int groups;  // of the tile, 1 .. 4
+};
+__global__ void kb_tiles(const int* __restrict__ tile_off, const int* __restrict__ s_offset, WindowView v, int W, int T,
+                         int* __restrict__ s_tile_window, int* __restrict__ s_tile_group, TileSource* __restrict__ source) {
     int t = blockIdx.x * blockDim.x + threadIdx.x;
     if (t >= T) return;
-    const int w = find_window(tile_off, W, t);
+    const int w = find_window(tile_off, W, t), first = 4 * (t - tile_off[w]);
     s_tile_window[t] = w;
-    s_tile_group[t] = s_offset[w] + 4 * (t - tile_off[w]);
+    s_tile_group[t] = s_offset[w] + first;
+    const int rec = v.rec[w] + v.tc[w];
+    source[t] = TileSource{v.pre[w].slots + first, rec, v.end[w] - rec, min(4, s_offset[w + 1] - s_offset[w] - first)};
 }
 
 struct RecordView {
@@ -1013,7 +1021,10 @@ struct ExtraOut {
 
 // One warp per tile of four groups: lane (q, g) = (lane / 8, lane % 8) owns rows g and g + 8 of group q,
 // which are also the two rows of its word pair in the packed tile.  One pass writes the un-packed arrays
-// (196 bytes per group) and the tile (352 bytes).  What bounds it is instruction issue: the four records of a group
+// (196 bytes per group) and the tile (352 bytes).  A record is the end of a chain of three loads of up to a thousand
+// cycles each: with a tile per warp they were two thirds of its time (clustered graph: 159 us), so a warp works on many
+// tiles and has the source of the tile after the next, the units of the next and its records under way (106 us).  Few
+// instructions matter too: the four records of a group
 // are loaded by one lane each, ranked by column with three shuffles and read back from shared memory by
 // position; the positions of a row's first two entries, and the tile's metadata for them, come from tables
 // indexed by the row's occupancy pattern.  With all four records in every lane's registers, sorted by a network
@@ -1025,7 +1036,7 @@ constexpr u64 kTilePos = 0x498e4dcc49884444ull;      // 4 bits: p0 | p1 << 2, th
 constexpr unsigned kLoneLater = 0x114u;              // patterns with one entry, not in position 0: it is the second kept one
 
 template <bool STRICT>
-__global__ void __launch_bounds__(256) kb_emit_tiles(WindowView v, RecordView r, const int* __restrict__ s_offset,
+__global__ void __launch_bounds__(256) kb_emit_tiles(const TileSource* __restrict__ source, RecordView r,
                                                      const int* __restrict__ tile_window, const int* __restrict__ tile_group,
                                                      int T, int window, const int* __restrict__ pair_a,
                                                      const int* __restrict__ pair_b, GroupOut o, ExtraOut x) {
@@ -1047,18 +1058,27 @@ __global__ void __launch_bounds__(256) kb_emit_tiles(WindowView v, RecordView r,
         __syncwarp();
     };
     int dropped = 0;
-    for (int t = blockIdx.x * 8 + wid; t < T; t += gridDim.x * 8) {
-        const int w = tile_window[t];
-        const int gid = tile_group[t] + q;
-        const bool live = gid < s_offset[w + 1];
-        // the group's columns, ascending: lane g < 4 brings column g
-        Record c{0x7fffffff, 0, 0u, 0.f};
-        if (live && g < 4) {
-            const int slot = v.pre[w].slots + gid - s_offset[w];
-            const int rec0 = v.rec[w] + v.tc[w], ncol = v.end[w] - rec0;
-            const int u = (g < 2 ? pair_a : pair_b)[slot], ls = 2 * u + (g & 1);
-            if (u >= 0 && ls < ncol) c = r.rec[rec0 + ls];
-        }
+    const int step = gridDim.x * 8;
+    auto source_of = [&](int t) -> int4 { return t < T ? __ldg((const int4*)source + t) : make_int4(0, 0, 0, 0); };
+    // lane g < 4 brings one of its group's columns
+    auto unit_of = [&](const int4& at) -> int { return g < 4 && q < at.w ? (g < 2 ? pair_a : pair_b)[at.x + q] : -1; };
+    auto record_of = [&](const int4& at, int u) -> Record {
+        const int ls = 2 * u + (g & 1);
+        return u >= 0 && ls < at.z ? r.rec[at.y + ls] : Record{0x7fffffff, 0, 0u, 0.f};
+    };
+    int t = blockIdx.x * 8 + wid;
+    int4 at0 = source_of(t), at1 = source_of(t + step), at2 = source_of(t + 2 * step);
+    Record next = record_of(at0, unit_of(at0));
+    int u1 = unit_of(at1);
+    for (; t < T; t += step) {
+        const int w = tile_window[t], gid = tile_group[t] + q;
+        const bool live = q < at0.w;
+        Record c = next;
+        next = record_of(at1, u1);
+        u1 = unit_of(at2);
+        at0 = at1;
+        at1 = at2;
+        at2 = source_of(t + 3 * step);
         int rank = 0;
 #pragma unroll
         for (int i = 1; i < 4; ++i) {
@@ -1874,15 +1894,16 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
         TRS_TRY(ts.get((size_t)nnz / 2 + 1, &xat_a));
     }
     if (T > 0) {
-        kb_tiles<<<grid_for(T), 256, 0, st>>>(B->s_window_tile_offset.p, B->s_offset.p, W, T, B->s_tile_window.p, B->s_tile_group.p);
+        TileSource* source;
+        TRS_TRY(ts.get(T, &source));
+        kb_tiles<<<grid_for(T), 256, 0, st>>>(B->s_window_tile_offset.p, B->s_offset.p, v, W, T, B->s_tile_window.p, B->s_tile_group.p, source);
         TRS_LAUNCH_CHECK();
         const GroupOut go{B->s_column.p, B->s_mask.p, B->s_value.p, B->s_pos.p, B->s_window.p, B->s_tile_column.p,
                           B->s_packed_a.p, B->s_packed_meta.p};
         const ExtraOut xo{d_head->dropped, xkey_a, xat_a};
         auto emit = cfg.strict ? kb_emit_tiles<true> : kb_emit_tiles<false>;
-        // strict mode collects a warp's extras over many tiles; otherwise a tile per warp hides most latency
-        emit<<<cfg.strict ? std::min(grid_for(T, 8), (unsigned)sms * 8u) : grid_for(T, 8), 256, 0, st>>>(v, rv, B->s_offset.p, B->s_tile_window.p, B->s_tile_group.p,
-                                                                           T, window, mo.pair_a, mo.pair_b, go, xo);
+        emit<<<std::min(grid_for(T, 8), (unsigned)sms * 8u), 256, 0, st>>>(source, rv, B->s_tile_window.p, B->s_tile_group.p, T, window,
+                                                                           mo.pair_a, mo.pair_b, go, xo);
         TRS_LAUNCH_CHECK();
     }
     TRS_TRY(counted.wait());
