@@ -68,3 +68,15 @@ def test_sort_class_borders(entries, window):
     rowptr = torch.zeros(6 * window + 1, dtype=torch.int64)
     rowptr[1:] = torch.cumsum(torch.bincount(rows, minlength=6 * window), 0)
     _check(rowptr.to(torch.int32), cols[order].to(torch.int32), torch.randn(entries + 3, generator=g), window=window)
+
+
+@pytest.mark.parametrize("rows", [1, 255, 256, 257, 512, 1025])
+def test_part_block_borders(rows):
+    """Rows on both sides of the blocks that count the CUDA-core parts; windows with a unit that is not kept."""
+    g = torch.Generator().manual_seed(rows)
+    hit = torch.rand(rows, 90, generator=g) < 0.06
+    hit[:, :3] |= torch.rand(rows, 3, generator=g) < 0.5
+    rowptr = torch.zeros(rows + 1, dtype=torch.int64)
+    rowptr[1:] = torch.cumsum(hit.sum(1), 0)
+    col = hit.nonzero()[:, 1]
+    _check(rowptr.to(torch.int32), col.to(torch.int32), torch.randn(col.numel(), generator=g), window=7, unit_min_nnz=4)

@@ -29,6 +29,9 @@
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <cub/device/device_select.cuh>
+#include <thrust/iterator/transform_iterator.h>
+#include <thrust/iterator/transform_output_iterator.h>
+#include <thrust/iterator/zip_iterator.h>
 #include <thrust/iterator/counting_iterator.h>
 
 #include <stdlib.h>
@@ -70,7 +73,8 @@ struct InputInfo {
 };
 
 __global__ void kb_input_info(const int* __restrict__ rowptr, const int* __restrict__ col, int n_rows, int window, int W,
-                              int* __restrict__ sel /* [kSortClasses + 1][W] */, InputInfo* __restrict__ info) {
+                              int* __restrict__ sel /* [kSortClasses + 1][W] */, int* __restrict__ ncol /* [W], cleared */,
+                              InputInfo* __restrict__ info) {
     const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
     const int first = rowptr[0], nnz = rowptr[n_rows];
     if (t0 == 0) { info->first = first; info->last = nnz; }
@@ -81,7 +85,10 @@ __global__ void kb_input_info(const int* __restrict__ rowptr, const int* __restr
     for (long long w0 = t0 - lane; w0 < W; w0 += step) {   // whole warps
         const long long w = w0 + lane;
         long long n = 0;
-        if (w < W) n = (long long)rowptr[min((w + 1) * window, (long long)n_rows)] - rowptr[w * window];
+        if (w < W) {
+            n = (long long)rowptr[min((w + 1) * window, (long long)n_rows)] - rowptr[w * window];
+            ncol[w] = 0;
+        }
         int c = kSortClasses + 1;   // empty: no class
         if (n > 0) {
             c = kSortClasses;
@@ -735,7 +742,6 @@ struct MatchOut {
     int* pair_a;      // [slots] groups in emission order: matched pairs, then the unmatched unit if it is kept
     int* pair_b;
     int* groups;      // [W + 1]
-    int* tiles;       // [W + 1]
     int* cuda_unit;   // [W] unmatched unit that goes to the CUDA cores, -1: none
 };
 
@@ -752,7 +758,6 @@ __device__ __forceinline__ void match_finish(int w, int G, int left, int left_nn
         else cuda = left;
     }
     o.groups[w] = G;
-    o.tiles[w] = (G + 3) / 4;
     o.cuda_unit[w] = cuda;
 }
 
@@ -771,7 +776,7 @@ __global__ void __launch_bounds__(32 * kMatchWarps) kb_match_warp(WindowView v, 
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     const int w = blockIdx.x * kMatchWarps + wid;
     if (w > W) return;
-    if (w == W) { if (lane == 0) { o.groups[W] = 0; o.tiles[W] = 0; } return; }
+    if (w == W) { if (lane == 0) { o.groups[W] = 0; } return; }
     const Win p0 = v.pre[w];
     const int U = v.pre[w + 1].units - p0.units;
     if (U > max_units) return;
@@ -975,6 +980,21 @@ __global__ void __launch_bounds__(kBlockThreads) kb_match_block(WindowView v, co
 // ---------------------------------------------------------------------------------------------
 // 7. groups and tiles
 // ---------------------------------------------------------------------------------------------
+struct __align__(8) GroupsTiles {   // of a window, scanned together
+    int groups, tiles;
+};
+struct GroupsTilesSum {
+    __host__ __device__ __forceinline__ GroupsTiles operator()(const GroupsTiles& a, const GroupsTiles& b) const {
+        return GroupsTiles{a.groups + b.groups, a.tiles + b.tiles};
+    }
+};
+struct WithTiles {
+    __host__ __device__ __forceinline__ GroupsTiles operator()(int groups) const { return GroupsTiles{groups, (groups + 3) / 4}; }
+};
+struct ToTuple {
+    __host__ __device__ __forceinline__ thrust::tuple<int, int> operator()(const GroupsTiles& g) const { return {g.groups, g.tiles}; }
+};
+
 struct __align__(16) TileSource {   // where a tile's columns come from
     int slot;    // of its first group in the pair lists
     int rec;     // first record of the window that is in a unit
@@ -1311,16 +1331,46 @@ __device__ __forceinline__ Parts split_counts(int n, int part_c, int short_size)
     return p;
 }
 
-__global__ void kb_cuda_count(int n_rows, int window, int part_c, int short_size, const int* __restrict__ win_cuda_unit,
-                              WindowView v, RecordView r, Extras x, Parts* __restrict__ cnt) {
-    int row = blockIdx.x * blockDim.x + threadIdx.x;
-    if (row > n_rows) return;
+// Where a row's parts begin: the sum over the rows before it in its block of kPartRows rows, and over the blocks before.
+// A device-wide scan of all rows' 16-byte counts took 18 us behind 4 for the counts (262144 rows), the blocks' sums 5.
+constexpr int kPartRows = 256;
+struct PartsAt {
+    const Parts* inside;   // [n_rows + 1]
+    const Parts* before;   // [blocks + 1], the last one: all
+    __device__ __forceinline__ Parts operator[](int row) const { return PartsSum()(inside[row], before[row / kPartRows]); }
+};
+__global__ void __launch_bounds__(kPartRows) kb_cuda_count(int n_rows, int window, int part_c, int short_size,
+                                                           const int* __restrict__ win_cuda_unit, WindowView v, RecordView r, Extras x,
+                                                           Parts* __restrict__ inside, Parts* __restrict__ block) {
+    __shared__ Parts s_warp[kPartRows / 32];
+    const int row = blockIdx.x * kPartRows + threadIdx.x, lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
     int n = 0;
     if (row < n_rows) {
         n = cuda_row(row, window, win_cuda_unit, v, r).n;
         if (x.n > 0) n += x.first(row + 1) - x.first(row);
     }
-    cnt[row] = split_counts(n, part_c, short_size);
+    const Parts own = split_counts(n, part_c, short_size);
+    Parts incl = own;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const Parts y{__shfl_up_sync(0xffffffffu, incl.nl, d), __shfl_up_sync(0xffffffffu, incl.ns, d),
+                      __shfl_up_sync(0xffffffffu, incl.zl, d), __shfl_up_sync(0xffffffffu, incl.zs, d)};
+        if (lane >= d) incl = PartsSum()(incl, y);
+    }
+    if (lane == 31) s_warp[wid] = incl;
+    __syncthreads();
+    Parts before{0, 0, 0, 0}, all{0, 0, 0, 0};
+    for (int q = 0; q < kPartRows / 32; ++q) {
+        if (q == wid) before = all;
+        all = PartsSum()(all, s_warp[q]);
+    }
+    if (row <= n_rows)
+        inside[row] = Parts{before.nl + incl.nl - own.nl, before.ns + incl.ns - own.ns, before.zl + incl.zl - own.zl,
+                            before.zs + incl.zs - own.zs};
+    if (threadIdx.x == 0) {
+        block[blockIdx.x] = all;
+        if (blockIdx.x + 1 == gridDim.x) block[gridDim.x] = Parts{0, 0, 0, 0};
+    }
 }
 
 struct PartsOut {
@@ -1339,7 +1389,7 @@ struct PartsOut {
 // extras, by column.  One thread per row writes its parts and the unit's entries, one per extra its place:
 // its rank among the row's extras plus the unit entries before it (a hub row has thousands).
 __global__ void kb_cuda_rows(int n_rows, int window, int part_c, int short_size, const int* __restrict__ win_cuda_unit,
-                             WindowView v, RecordView r, Extras x, const Parts* __restrict__ off, PartsOut po) {
+                             WindowView v, RecordView r, Extras x, PartsAt off, PartsOut po) {
     int row = blockIdx.x * blockDim.x + threadIdx.x;
     if (row == 0) { po.c_row_offset[0] = 0; po.cs_row_offset[0] = 0; }
     if (row >= n_rows) return;
@@ -1372,7 +1422,7 @@ __global__ void kb_cuda_rows(int n_rows, int window, int part_c, int short_size,
 }
 
 __global__ void kb_cuda_extras(int window, const int* __restrict__ win_cuda_unit, WindowView v, RecordView r, Extras x,
-                               const Parts* __restrict__ off, PartsOut po) {
+                               PartsAt off, PartsOut po) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= x.n) return;
     const int row = (int)(x.key[i] >> 32), c = (int)(x.key[i] & 0xffffffffull);
@@ -1481,8 +1531,8 @@ struct Cub {
         TRS_CUDA(call((void*)tmp, bytes));
         return 0;
     }
-    template <class T, class Op>
-    int exclusive_scan(const T* in, T* out, Op op, T zero, long long n) {
+    template <class In, class Out, class T, class Op>
+    int exclusive_scan(In in, Out out, Op op, T zero, long long n) {
         return run([&](void* t, size_t& b) { return cub::DeviceScan::ExclusiveScan(t, b, in, out, op, zero, n, st); });
     }
     int exclusive_sum(const int* in, int* out, long long n) {
@@ -1545,6 +1595,16 @@ int read_back(const T* dev, T* host, cudaStream_t st) {
 }
 
 // Streams on which the hub tiers of the matching run beside the others (two per device, made once).
+// Work on the side streams that the caller's stream has not been made to wait for: a call that fails in between waits
+// here, before the memory goes back.
+struct SideWork {
+    cudaStream_t s[2] = {nullptr, nullptr};
+    bool open = false;
+    ~SideWork() {
+        if (open)
+            for (cudaStream_t x : s) cudaStreamSynchronize(x);
+    }
+};
 int side_streams(cudaStream_t out[2]) {
     static cudaStream_t made[64][2] = {};
     static std::mutex m;
@@ -1659,8 +1719,6 @@ int make_records(trs_builder* B, const int* rowptr, const int* col, const float*
     TRS_TRY(ts.get(nnz, &R->w.rec));
     TRS_TRY(ts.get(nnz, &R->w.sval));
     TRS_TRY(ts.get(nnz, &R->w.cnt));
-    TRS_TRY(ts.get((size_t)W, &R->w.ncol));
-    TRS_CUDA(cudaMemsetAsync(R->w.ncol, 0, sizeof(int) * (size_t)W, st));
     int parts = 0;
     for (int c = 0; c <= kSortClasses; ++c) parts += info.windows[c] > 0;
     const bool fork = parts > 1;
@@ -1731,7 +1789,8 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     TRS_CUDA(cudaMemsetAsync(d_head, 0, sizeof(Head), st));
     Records R;
     TRS_TRY(ts.get((size_t)(kSortClasses + 1) * W, &R.sel));
-    kb_input_info<<<2 * sms, 512, 0, st>>>(rowptr, col, n, window, W, R.sel, &d_head->counts.info);
+    TRS_TRY(ts.get((size_t)W, &R.w.ncol));
+    kb_input_info<<<2 * sms, 512, 0, st>>>(rowptr, col, n, window, W, R.sel, R.w.ncol, &d_head->counts.info);
     TRS_LAUNCH_CHECK();
     TRS_TRY(read_back(&d_head->counts.info, &back->head.counts.info, st));
     const InputInfo info = back->head.counts.info;
@@ -1769,7 +1828,6 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
         TRS_TRY(ts.get(slots, &mo.pair_a));
         TRS_TRY(ts.get(slots, &mo.pair_b));
         TRS_TRY(ts.get((size_t)W + 1, &mo.groups));
-        TRS_TRY(ts.get((size_t)W + 1, &mo.tiles));
         return ts.get((size_t)W + 1, &mo.cuda_unit);
     };
     auto match_warps = [&](int max_units) -> int {
@@ -1783,8 +1841,10 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     auto group_sizes = [&]() -> int {
         TRS_TRY(B->out(B->s_offset, 22, (size_t)W + 1));
         TRS_TRY(B->out(B->s_window_tile_offset, 28, (size_t)W + 1));
-        TRS_TRY(cub_.exclusive_sum(mo.groups, B->s_offset.p, W + 1));
-        TRS_TRY(cub_.exclusive_sum(mo.tiles, B->s_window_tile_offset.p, W + 1));
+        const auto both = thrust::make_transform_iterator((const int*)mo.groups, WithTiles());
+        const auto out = thrust::make_transform_output_iterator(
+            thrust::make_zip_iterator(thrust::make_tuple(B->s_offset.p, B->s_window_tile_offset.p)), ToTuple());
+        TRS_TRY(cub_.exclusive_scan(both, out, GroupsTilesSum(), GroupsTiles{0, 0}, W + 1));
         TRS_TRY(publish((const int*)B->s_offset.p + W, &back->groups, (const int*)B->s_window_tile_offset.p + W, &back->tiles, st));
         return grouped.record(st);
     };
@@ -1807,12 +1867,14 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     if (!ahead) TRS_TRY(match_arrays(TU, TS));
     if (mc.max_huge >= (int)kUnitMask) return TRS_E_LIMIT;
     // one long chain per hub window: the tiers run side by side
-    cudaStream_t side[2] = {st, st};
+    SideWork work;
+    cudaStream_t* const side = work.s;
+    TRS_TRY(side_streams(side));
     Event ready, done[2];
     if (mc.n_huge + mc.n_block > 0) {
-        TRS_TRY(side_streams(side));
         TRS_TRY(ready.record(st));
         TRS_CUDA(cudaFuncSetAttribute(kb_match_block, cudaFuncAttributeMaxDynamicSharedMemorySize, kSmemUnits * 4));
+        work.open = true;
     }
     if (mc.n_huge > 0) {
         const int smem_units = mc.max_huge <= kSmemUnits ? mc.max_huge : kSmemUnits;
@@ -1848,6 +1910,7 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     if (!ahead) {   // the hub windows are matched by now
         if (mc.n_huge > 0) { TRS_TRY(done[0].record(side[0])); TRS_CUDA(cudaStreamWaitEvent(st, done[0].e, 0)); }
         if (mc.n_block > 0) { TRS_TRY(done[1].record(side[1])); TRS_CUDA(cudaStreamWaitEvent(st, done[1].e, 0)); }
+        work.open = false;
         TRS_TRY(group_sizes());
     }
     TRS_TRY(B->out(B->t_row_offset, 0, (size_t)NP + 1));
@@ -1857,20 +1920,23 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     TRS_LAUNCH_CHECK();
 
     // ---- 9. CUDA-core parts: counted now, or in strict mode when the dropped entries are known ------
-    Parts *cnt, *off;
-    TRS_TRY(ts.get((size_t)n + 1, &cnt));
-    TRS_TRY(ts.get((size_t)n + 1, &off));
+    Parts *inside, *block, *before;
+    const unsigned part_blocks = grid_for((long long)n + 1, kPartRows);
+    TRS_TRY(ts.get((size_t)n + 1, &inside));
+    TRS_TRY(ts.get((size_t)part_blocks + 1, &block));
+    TRS_TRY(ts.get((size_t)part_blocks + 1, &before));
+    const PartsAt off{inside, before};
     Extras x{nullptr, nullptr, 0};
     auto count_parts = [&]() -> int {
-        kb_cuda_count<<<grid_for(n + 1), 256, 0, st>>>(n, window, cfg.part_c, cfg.short_size, mo.cuda_unit, v, rv, x, cnt);
+        kb_cuda_count<<<part_blocks, kPartRows, 0, st>>>(n, window, cfg.part_c, cfg.short_size, mo.cuda_unit, v, rv, x, inside, block);
         TRS_LAUNCH_CHECK();
-        return cub_.exclusive_scan(cnt, off, PartsSum(), Parts{0, 0, 0, 0}, (long long)n + 1);
+        return cub_.exclusive_scan(block, before, PartsSum(), Parts{0, 0, 0, 0}, (long long)part_blocks + 1);
     };
     if (!cfg.strict) TRS_TRY(count_parts());
     if (cfg.strict) {
         TRS_TRY(publish((const int*)B->t_block_offset.p + NB, &back->tc_nnz, st));
     } else {
-        TRS_TRY(publish((const int*)B->t_block_offset.p + NB, &back->tc_nnz, (const Parts*)off + n, &back->parts, st));
+        TRS_TRY(publish((const int*)B->t_block_offset.p + NB, &back->tc_nnz, (const Parts*)before + part_blocks, &back->parts, st));
     }
     TRS_TRY(counted.record(st));
 
@@ -1902,15 +1968,25 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
                           B->s_packed_a.p, B->s_packed_meta.p};
         const ExtraOut xo{d_head->dropped, xkey_a, xat_a};
         auto emit = cfg.strict ? kb_emit_tiles<true> : kb_emit_tiles<false>;
-        emit<<<std::min(grid_for(T, 8), (unsigned)sms * 8u), 256, 0, st>>>(source, rv, B->s_tile_window.p, B->s_tile_group.p, T, window,
+        // as many blocks as are resident
+        emit<<<std::min(grid_for(T, 8), (unsigned)sms * 4u), 256, 0, st>>>(source, rv, B->s_tile_window.p, B->s_tile_group.p, T, window,
                                                                            mo.pair_a, mo.pair_b, go, xo);
         TRS_LAUNCH_CHECK();
     }
+    // the values of the TC blocks fill the last wave of the tiles
     TRS_TRY(counted.wait());
     TRS_TRY(B->out(B->t_value, 3, back->tc_nnz));
+    Event valued;
     if (NB > 0) {
-        kb_tc_values<<<grid_for((long long)NB * 128), 256, 0, st>>>(rv, slot_rec, NB, B->t_binary.p, B->t_block_offset.p, B->t_value.p);
+        work.open = true;
+        TRS_CUDA(cudaStreamWaitEvent(side[0], counted.e, 0));
+        kb_tc_values<<<grid_for((long long)NB * 128), 256, 0, side[0]>>>(rv, slot_rec, NB, B->t_binary.p, B->t_block_offset.p, B->t_value.p);
         TRS_LAUNCH_CHECK();
+        TRS_TRY(valued.record(side[0]));
+    }
+    if (NB > 0) {
+        TRS_CUDA(cudaStreamWaitEvent(st, valued.e, 0));
+        work.open = false;
     }
     if (cfg.strict) {
         TRS_TRY(read_back(&d_head->dropped, &back->head.dropped, st));
@@ -1924,7 +2000,7 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
             x = Extras{key, at, (int)n_extra};
         }
         TRS_TRY(count_parts());
-        TRS_TRY(read_back((const Parts*)off + n, &back->parts, st));
+        TRS_TRY(read_back((const Parts*)before + part_blocks, &back->parts, st));
     }
     const Parts p = back->parts;
     TRS_TRY(B->out(B->c_row_offset, 7, (size_t)p.nl + 1));
