@@ -521,23 +521,14 @@ struct UnitWordLess {
 };
 __device__ __forceinline__ unsigned unit_key(int word) { return (unsigned)word >> kUnitBits; }
 
-// Where the element that introsort leaves at position p of a range of n > 16 equal keys came from.
-__device__ __forceinline__ int equal_range_source(int n, int p) {
-    int f[28], l[28], levels = 0;
-    int lo = 0, hi = n;
-    while (hi - lo > 16) {
-        f[levels] = lo; l[levels] = hi; ++levels;
-        const int cut = lo + 1 + (hi - lo - 1) / 2;
-        if (p < cut) hi = cut; else lo = cut;
-    }
-    int s = p;
-    for (int i = levels - 1; i >= 0; --i) {
-        const int mid = f[i] + (l[i] - f[i]) / 2;
-        if (s == f[i]) s = mid;
-        else {
-            s = f[i] + l[i] - s;
-            if (s == mid) s = f[i];
-        }
+// Where introsort puts the element at position s of a range of n > 16 equal keys: every partition brings the middle one to
+// the front and reverses the rest.
+__device__ __forceinline__ int equal_range_target(int n, int s) {
+    int f = 0, l = n;
+    while (l - f > 16) {
+        const int mid = f + (l - f) / 2, cut = f + 1 + (l - f - 1) / 2;
+        s = s == mid ? f : f + l - (s == f ? mid : s);
+        if (s < cut) l = cut; else f = cut;
     }
     return s;
 }
@@ -550,12 +541,15 @@ __device__ __forceinline__ int equal_range_depth(int n) {  // partitions on the 
 // One warp partitions [first, last) of a as introsort does (median of three to the front included);
 // `sl` / `sr`: 32 ints of shared memory each.
 __device__ __forceinline__ int warp_partition(int* a, int first, int last, int* sl, int* sr, int lane) {
-    if (lane == 0) {
-        StdSort<UnitWordLess> S(a, UnitWordLess());
-        S.move_median_to_first(first, first + 1, first + (last - first) / 2, last - 1);
-    }
+    const int mid = first + (last - first) / 2;
+    const int vf = a[first], va = a[first + 1], vb = a[mid], vc = a[last - 1];
+    const unsigned ka = unit_key(va), kb = unit_key(vb), kc = unit_key(vc);
+    const int median = ka > kb ? (kb > kc ? mid : ka > kc ? last - 1 : first + 1) : (ka > kc ? first + 1 : kb > kc ? last - 1 : mid);
+    const int vm = median == first + 1 ? va : median == mid ? vb : vc;
     __syncwarp();
-    const unsigned pv = unit_key(a[first]);
+    if (lane == 0) { a[first] = vm; a[median] = vf; }
+    __syncwarp();
+    const unsigned pv = unit_key(vm);
     const unsigned lt = (1u << lane) - 1u;
     int lb = first + 1 - 32, rb = last - 1 + 32;  // the blocks start at lb (upwards) and rb (downwards)
     unsigned lm = 0, rm = 0;                       // stoppers of the blocks not used yet
@@ -603,40 +597,82 @@ struct SortRange {
     int first, last, depth;
 };
 
+// Introsort of a[first, first + n), n <= 32, by one warp, an element per lane; unit indices to out[first ..).  The stoppers
+// of a partition and their partners are counted in ballots.  What is left below 17 elements the library insertion-sorts,
+// which is stable and never crosses a cut, so the whole range ends up stably sorted: an element's place is the number of
+// larger keys and of equal ones before it, from one ballot per bit.  In shared memory a partition takes some 700 cycles
+// whatever its length, and most are of this length (matching of the clustered graph 130 -> 100 us with the pairs below).
+__device__ void warp_sort_lanes(int* a, int* __restrict__ out, int first, int n, int depth, int* sl, int* sr, int lane) {
+    int v = lane < n ? a[first + lane] : 0;
+    const unsigned lt = (1u << lane) - 1u, gt = ~lt << 1;
+    for (int f = 0, l = n; l - f > 16;) {
+        if (depth == 0) {
+            if (lane < n) a[first + lane] = v;
+            __syncwarp();
+            if (lane == 0) StdSort<UnitWordLess>(a, UnitWordLess()).heap_sort(first + f, l - f);
+            __syncwarp();
+            if (lane < n) v = a[first + lane];
+            break;
+        }
+        --depth;
+        const int pa = f + 1, pb = f + (l - f) / 2, pc = l - 1;
+        const unsigned ka = unit_key(__shfl_sync(0xffffffffu, v, pa)), kb = unit_key(__shfl_sync(0xffffffffu, v, pb)),
+                       kc = unit_key(__shfl_sync(0xffffffffu, v, pc));
+        const int median = ka > kb ? (kb > kc ? pb : ka > kc ? pc : pa) : (ka > kc ? pa : kb > kc ? pc : pb);
+        const int vf = __shfl_sync(0xffffffffu, v, f), vm = __shfl_sync(0xffffffffu, v, median);
+        if (lane == f) v = vm;
+        if (lane == median) v = vf;
+        const unsigned key = unit_key(v), pivot = unit_key(vm);
+        const bool in = lane > f && lane < l, is_l = in && key <= pivot, is_r = in && key >= pivot;
+        const unsigned lm = __ballot_sync(0xffffffffu, is_l), rm = __ballot_sync(0xffffffffu, is_r);
+        const int rl = __popc(lm & lt), rr = __popc(rm & gt);   // ranks, from the left and from the right
+        const int swaps = __popc(__ballot_sync(0xffffffffu, is_l && rr > rl));
+        const bool swap_l = is_l && rl < swaps, swap_r = is_r && rr < swaps;
+        if (swap_l) sl[rl] = lane;
+        if (swap_r) sr[rr] = lane;
+        __syncwarp();
+        const int partner = swap_l ? sr[rl] : swap_r ? sl[rr] : lane;
+        v = __shfl_sync(0xffffffffu, v, partner);
+        const unsigned next_l = __ballot_sync(0xffffffffu, is_l && rl >= swaps), last_r = __ballot_sync(0xffffffffu, swap_r);
+        const int cut = min(next_l ? __ffs(next_l) - 1 : 32, last_r ? __ffs(last_r) - 1 : 32);
+        if (l - cut > cut - f) f = cut; else l = cut;   // at most one side has more than 16
+    }
+    const unsigned key = unit_key(v);
+    unsigned eq = n < 32 ? (1u << n) - 1u : 0xffffffffu, larger = 0;
+#pragma unroll
+    for (int b = 31 - kUnitBits; b >= 0; --b) {
+        const bool one = (key >> b) & 1u;
+        const unsigned ones = __ballot_sync(0xffffffffu, one);
+        if (!one) larger |= eq & ones;
+        eq &= one ? ones : ~ones;
+    }
+    if (lane < n) out[first + __popc(larger) + __popc(eq & lt)] = v & (int)kUnitMask;
+    __syncwarp();
+}
+
 // Introsort of a[first0, last0) by one warp; unit indices to out[first0, last0).
 // `stack`: 40 ranges, `sl`, `sr`: 32 ints, all in shared memory and this warp's own.
 __device__ void warp_introsort(int* a, int* __restrict__ out, int first0, int last0, int depth0, SortRange* stack, int* sl,
                                int* sr, int lane) {
     int sp = 0;
     int first = first0, last = last0, depth = depth0;
-    int pend_first = 0, pend_last = 0, n_pend = 0;  // lane k holds the k-th finished leaf
     StdSort<UnitWordLess> S(a, UnitWordLess());
-    auto flush = [&]() {
-        __syncwarp();
-        if (lane < n_pend && pend_last - pend_first > 1) S.insertion_range(pend_first, pend_last);
-        for (int i = pend_first; lane < n_pend && i < pend_last; ++i) out[i] = a[i] & (int)kUnitMask;
-        n_pend = 0;
-        __syncwarp();
-    };
     while (true) {
         const int n = last - first;
         bool done = false;
-        if (n <= 16) {
-            if (n > 0) {
-                if (lane == n_pend) { pend_first = first; pend_last = last; }
-                if (++n_pend == 32) flush();
-            }
+        if (n <= 32) {
+            warp_sort_lanes(a, out, first, n, depth, sl, sr, lane);
             done = true;
         } else {
             const unsigned k0 = unit_key(a[first]);
             bool equal = false;
-            if (n > 32 && k0 == unit_key(a[last - 1]) && k0 == unit_key(a[first + n / 2]) && depth >= equal_range_depth(n)) {
+            if (k0 == unit_key(a[last - 1]) && k0 == unit_key(a[first + n / 2]) && depth >= equal_range_depth(n)) {
                 equal = true;
                 for (int i = first + lane; i - lane < last; i += 32)
                     if (__ballot_sync(0xffffffffu, i < last && unit_key(a[i]) != k0)) { equal = false; break; }
             }
             if (equal) {
-                for (int i = lane; i < n; i += 32) out[first + i] = a[first + equal_range_source(n, i)] & (int)kUnitMask;
+                for (int i = lane; i < n; i += 32) out[first + equal_range_target(n, i)] = a[first + i] & (int)kUnitMask;
                 done = true;
             } else if (depth == 0) {
                 if (lane == 0) S.heap_sort(first, n);
@@ -661,7 +697,6 @@ __device__ void warp_introsort(int* a, int* __restrict__ out, int first0, int la
         __syncwarp();
         if (right_first) first = cut; else last = cut;
     }
-    flush();
 }
 
 // Greedy pass over the sorted order (block_online.cpp:365-386) by one warp.  The next unmatched unit of the
@@ -719,19 +754,48 @@ __device__ __forceinline__ int warp_greedy(int U, unsigned* freem, const int* or
                 cur = __ballot_sync(0xffffffffu, bit && rb >= t);
                 continue;
             }
-            const int i = __ffs(alive) - 1;
-            alive &= alive - 1;
-            const int x = __shfl_sync(0xffffffffu, idx, i);
-            const unsigned keep = ~(1u << (x & 31));
-            if ((x >> 5) == wpos) cur &= keep;
-            else if (lane == 0) atomicAnd(freem + (x >> 5), keep);
-            if (cur == 0) advance();
-            if (cur == 0) { *left = x; return G; }
-            const int y = wpos * 32 + __ffs(cur) - 1;
-            cur &= cur - 1;
-            alive &= ~__ballot_sync(0xffffffffu, idx == y);
-            if (lane == 0) { pa[G] = x; pb[G] = y; }
-            ++G;
+            // units of the lowest free word are among the next alive ones: pair by pair, in registers (80 cycles a pair; with
+            // the free words updated in shared memory 390).  Lane i knows which bit of the word its unit is, lane b which
+            // alive unit bit b is; lane p keeps the p-th pair.
+            const unsigned drop_bit = mine && word == wpos ? 1u << (idx & 31) : 0u;
+            sl[lane] = -1;
+            __syncwarp();
+            if (drop_bit) sl[idx & 31] = lane;
+            __syncwarp();
+            const int at = sl[lane];
+            const unsigned drop_lane = at >= 0 ? 1u << at : 0u;
+            int px = 0, py = 0, n = 0;
+            bool waits = false;   // the last unit taken from the order finds its partner in a later word
+            while (alive) {
+                const int i = __ffs(alive) - 1;
+                alive &= alive - 1;
+                cur &= ~__shfl_sync(0xffffffffu, drop_bit, i);
+                if (lane == n) px = i;
+                if (cur == 0) { waits = true; break; }
+                const int y = __ffs(cur) - 1;
+                cur &= cur - 1;
+                alive &= ~__shfl_sync(0xffffffffu, drop_lane, y);
+                if (lane == n) py = y;
+                ++n;
+                if (cur == 0) break;
+            }
+            const int x = __shfl_sync(0xffffffffu, idx, px);
+            if (lane < n + waits) {
+                if ((x >> 5) != wpos) atomicAnd(freem + (x >> 5), ~(1u << (x & 31)));
+                pa[G + lane] = x;
+                if (lane < n) pb[G + lane] = wpos * 32 + py;
+            }
+            G += n;
+            if (waits) {
+                advance();
+                const int alone = __shfl_sync(0xffffffffu, x, n);
+                if (cur == 0) { *left = alone; return G; }
+                const int y = wpos * 32 + __ffs(cur) - 1;
+                cur &= cur - 1;
+                alive &= ~__ballot_sync(0xffffffffu, idx == y);
+                if (lane == 0) pb[G] = y;
+                ++G;
+            }
         }
     }
     return G;
@@ -804,7 +868,7 @@ __global__ void __launch_bounds__(32 * kMatchWarps) kb_match_warp(WindowView v, 
 // at most kWarpRange units are left to single warps.  The words live in dynamic shared memory when
 // they fit (smem_units), in `words_global` otherwise; the bitmask takes the same memory afterwards
 // (or `mask_global`).
-constexpr int kBlockThreads = 256, kWarpRange = 1024, kMaxRanges = 256;
+constexpr int kBlockThreads = 512, kWarpRange = 1024, kMaxRanges = 256;
 
 __global__ void __launch_bounds__(kBlockThreads) kb_match_block(WindowView v, const unsigned char* __restrict__ cnt, int unit_min_nnz,
                                                                 int smem_units, int* __restrict__ words_global,
@@ -890,7 +954,7 @@ __global__ void __launch_bounds__(kBlockThreads) kb_match_block(WindowView v, co
             int differ = 0;
             for (int i = first + tid; i < last; i += kBlockThreads) differ |= unit_key(a[i]) != k0;
             if (!__syncthreads_or(differ)) {
-                for (int i = tid; i < n; i += kBlockThreads) order[first + i] = a[first + equal_range_source(n, i)] & (int)kUnitMask;
+                for (int i = tid; i < n; i += kBlockThreads) order[first + equal_range_target(n, i)] = a[first + i] & (int)kUnitMask;
                 if (tid == 0) s_sp = sp - 1;
                 continue;
             }
@@ -905,7 +969,7 @@ __global__ void __launch_bounds__(kBlockThreads) kb_match_block(WindowView v, co
         __syncthreads();
         const unsigned pvk = unit_key(a[first]);
         const int lo = first + 1, m = last - lo;
-        const int chunk = (m + kBlockThreads - 1) / kBlockThreads;
+        const int chunk = ((m + kBlockThreads - 1) / kBlockThreads) | 1;   // odd: the threads read from different banks
         const int cb = min(lo + tid * chunk, last), ce = min(cb + chunk, last);
         // pass 1: stoppers per chunk (left: key <= pivot, right: key >= pivot)
         int cL = 0, cR = 0;
@@ -954,9 +1018,17 @@ __global__ void __launch_bounds__(kBlockThreads) kb_match_block(WindowView v, co
             s_stack[sp] = SortRange{first, cut, r.depth - 1};
             s_sp = sp + 1;
         }
-        for (int k = tid; k < K; k += kBlockThreads) {
-            const int x = swapL[k], y = swapR[k];
-            const int t = a[x]; a[x] = a[y]; a[y] = t;
+        for (int k0 = tid; k0 < K; k0 += 4 * kBlockThreads) {   // four pairs' loads under way
+            int x[4], y[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int k = k0 + j * kBlockThreads;
+                x[j] = k < K ? swapL[k] : -1;
+                y[j] = k < K ? swapR[k] : -1;
+            }
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+                if (x[j] >= 0) { const int t = a[x[j]]; a[x[j]] = a[y[j]]; a[y[j]] = t; }
         }
     }
     run_small();
