@@ -703,8 +703,7 @@ __device__ void warp_introsort(int* a, int* __restrict__ out, int first0, int la
 // order is paired with the lowest unmatched unit, again and again.  Two windows of 32 are open at a
 // time: entries of the order (`alive`: still unmatched) and the bitmask word of the lowest unmatched units
 // (`cur`).  While no alive entry lies in that word the two are independent, and the k-th alive entry
-// simply gets the k-th free bit; otherwise one pair is made and the windows are looked at again.  Pair by
-// pair a warp needs 390 cycles each (a thread 320), which was 80 % of a hub window's matching.
+// simply gets the k-th free bit; otherwise the pairs are made one by one until the word or the entries are used up.
 // `freem`: a bit per unmatched unit, `sl`: 32 ints of shared memory.  Returns the number of pairs; *left: the
 // unit that stays alone (-1: none).
 __device__ __forceinline__ int warp_greedy(int U, unsigned* freem, const int* order, int* __restrict__ pa, int* __restrict__ pb,
