@@ -23,7 +23,7 @@ def _case():
 
 
 @pytest.mark.parametrize("chunk", ["256", "8"])
-@pytest.mark.parametrize("F", [1, 7, 8, 15, 16, 17, 31, 47, 48, 56, 72, 80, 95, 96, 112, 127, 128, 129, 136, 200, 257])
+@pytest.mark.parametrize("F", [1, 7, 8, 15, 16, 17, 24, 31, 40, 47, 48, 56, 72, 80, 95, 96, 112, 120, 127, 128, 129, 136, 200, 257])
 def test_widths(F, chunk, monkeypatch):
     monkeypatch.setenv("TRS_CHUNK_STEPS", chunk)
     arrays, n = _case()

@@ -435,7 +435,7 @@ __device__ __forceinline__ void compute_steps(float (&acc)[FS / 8][4], const uin
 // WPI warps share an item (each takes a contiguous share of its steps, the shares are added in
 // warp order at the end).  ALIGNED: rows of B start on 16-byte boundaries; otherwise they are
 // gathered with 2-byte loads (callers that can neither align B nor lend memory for a padded copy).
-template <int FS, int STAGES, int WPI, int MINB, bool ALIGNED, bool RANGE>
+template <int FS, int STAGES, int WPI, int MINB, bool ALIGNED, bool RANGE, bool RAGGED>
 __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const KernelArgs a) {
     using T = WarpTile<FS, STAGES>;
     extern __shared__ __align__(128) unsigned char smem_all[];
@@ -473,11 +473,14 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
         pdst[k] = smem0 + pr[k] * T::ROWB + ((pc[k] ^ T::swz(pr[k])) << 4);
     }
     const uint32_t pitch = (uint32_t)a.ldb * 2u;
-    // a chunk beyond the end of the row repeats the last one; its features are not stored
+    // A chunk beyond the end of the row repeats the last one, or, RAGGED, is not copied; its features are not stored
     const unsigned char* src0[T::POW2 ? 1 : T::NCP];
+    bool in_row[T::POW2 ? 1 : T::NCP];
 #pragma unroll
-    for (int k = 0; k < (T::POW2 ? 1 : T::NCP); ++k)
+    for (int k = 0; k < (T::POW2 ? 1 : T::NCP); ++k) {
+        in_row[k] = !RAGGED || fbase / 8 + pc[k] < a.bchunks;
         src0[k] = (const unsigned char*)a.B + (size_t)(min(fbase / 8 + pc[k], a.bchunks - 1)) * 16;
+    }
     auto src_of = [&](int k) -> const unsigned char* { return src0[T::POW2 ? 0 : k]; };
     // ldmatrix role: matrix lane / 8 -> k rows (m & 1) * 8 .., features (m >> 1) * 8 ..
     const int lrow = (lane & 7) + ((lane >> 3) & 1) * 8, lchunk = lane >> 4;
@@ -510,7 +513,8 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
 #pragma unroll
         for (int k = 0; k < T::NCP; ++k) {
             if constexpr (ALIGNED) {
-                cp_async16_at<decltype(stage)::value * T::STAGE>(pdst[k], src_of(k) + (unsigned long long)(uint32_t)c[k] * pitch);
+                if (in_row[T::POW2 ? 0 : k])
+                    cp_async16_at<decltype(stage)::value * T::STAGE>(pdst[k], src_of(k) + (unsigned long long)(uint32_t)c[k] * pitch);
             } else {
                 const int f = fbase + pc[k] * 8;
                 *(uint4*)(smem + (pdst[k] - smem0) + decltype(stage)::value * T::STAGE) = load_unaligned8(a.B + (size_t)c[k] * a.ldb + f, a.F - f);
@@ -954,9 +958,9 @@ extern "C" int trs_spmm_launches(const trs_spmm_plan* p) {
     return p->n_heavy > 0 ? 2 : 1;
 }
 
-template <int FS, int STAGES, int WPI, int MINB, bool ALIGNED, bool RANGE>
+template <int FS, int STAGES, int WPI, int MINB, bool ALIGNED, bool RANGE, bool RAGGED>
 static int launch_instance(const KernelArgs& a, int slabs, cudaStream_t st) {
-    auto kernel = k_window_spmm_warp<FS, STAGES, WPI, MINB, ALIGNED, RANGE>;
+    auto kernel = k_window_spmm_warp<FS, STAGES, WPI, MINB, ALIGNED, RANGE, RAGGED>;
     constexpr int smem = WarpTile<FS, STAGES>::SMEM * WPI;
     // once per device and instance (the attributes belong to the device's copy of the kernel)
     static std::atomic<unsigned long long> done{0};
@@ -973,12 +977,21 @@ static int launch_instance(const KernelArgs& a, int slabs, cudaStream_t st) {
     return TRS_OK;
 }
 
+template <int FS, int STAGES, int MINB, int MINB4, bool RAGGED>
+static int launch_items(const KernelArgs& a, int slabs, bool few_items, bool range, cudaStream_t st) {
+    if (few_items) return range ? launch_instance<FS, STAGES, 4, MINB4, true, true, RAGGED>(a, slabs, st)
+                                : launch_instance<FS, STAGES, 4, MINB4, true, false, RAGGED>(a, slabs, st);
+    return range ? launch_instance<FS, STAGES, 1, MINB, true, true, RAGGED>(a, slabs, st)
+                 : launch_instance<FS, STAGES, 1, MINB, true, false, RAGGED>(a, slabs, st);
+}
+// Rows of an odd number of 16-byte chunks in one slab leave out the chunk that is not there: two lanes that ask for one
+// piece cost as much as two pieces (F = 24 / 40 / 56 / 120 on a clustered graph of 377920 rows 103 / 134 / 130 / 214 us, without
+// 78 / 105 / 114 / 199).  The test takes up to a tenth where every chunk is there (F = 64 97 against 110), and gives as
+// much as it takes with several slabs.
 template <int FS, int STAGES, int MINB, int MINB4>
 static int launch_sized(const KernelArgs& a, int slabs, bool few_items, bool range, cudaStream_t st) {
-    if (few_items) return range ? launch_instance<FS, STAGES, 4, MINB4, true, true>(a, slabs, st)
-                                : launch_instance<FS, STAGES, 4, MINB4, true, false>(a, slabs, st);
-    return range ? launch_instance<FS, STAGES, 1, MINB, true, true>(a, slabs, st)
-                 : launch_instance<FS, STAGES, 1, MINB, true, false>(a, slabs, st);
+    return slabs == 1 && a.bchunks < FS / 8 ? launch_items<FS, STAGES, MINB, MINB4, true>(a, slabs, few_items, range, st)
+                                            : launch_items<FS, STAGES, MINB, MINB4, false>(a, slabs, few_items, range, st);
 }
 
 static int launch_window_kernel(const KernelArgs& a, bool aligned, bool few_items, bool range, cudaStream_t st) {
@@ -989,8 +1002,8 @@ static int launch_window_kernel(const KernelArgs& a, bool aligned, bool few_item
     // 494 / 467, F = 128 with 3 / 4 / 5 stages (16 / 12 / 10 warps) 577 / 627 / 650.
     const int slabs = ceil_div(a.F, 128);
     const int fs = ceil_div(ceil_div(a.F, slabs), 16);
-    if (!aligned) return fs <= 4 ? launch_instance<64, 3, 1, 16, false, true>(a, ceil_div(a.F, 64), st)
-                                 : launch_instance<128, 3, 1, 12, false, true>(a, ceil_div(a.F, 128), st);
+    if (!aligned) return fs <= 4 ? launch_instance<64, 3, 1, 16, false, true, false>(a, ceil_div(a.F, 64), st)
+                                 : launch_instance<128, 3, 1, 12, false, true, false>(a, ceil_div(a.F, 128), st);
     switch (fs) {
         case 1: return launch_sized<16, 6, 32, 8>(a, slabs, few_items, range, st);
         case 2: return launch_sized<32, 6, 28, 7>(a, slabs, few_items, range, st);
