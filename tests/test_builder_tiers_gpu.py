@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
-from trspmm import build_format
+from trspmm import TrsError, build_format
 
 pytestmark = pytest.mark.gpu
 
@@ -80,3 +80,14 @@ def test_part_block_borders(rows):
     rowptr[1:] = torch.cumsum(hit.sum(1), 0)
     col = hit.nonzero()[:, 1]
     _check(rowptr.to(torch.int32), col.to(torch.int32), torch.randn(col.numel(), generator=g), window=7, unit_min_nnz=4)
+
+
+@pytest.mark.parametrize("entries", [12, 600])
+def test_repeated_columns_are_refused(entries):
+    """A column repeated in every row, in a window sorted by a CTA and in a hub window: more entries of one column than the
+    window has rows must not get as far as the records."""
+    rp = torch.arange(17, dtype=torch.int32) * entries
+    col = torch.full((16 * entries,), 5, dtype=torch.int32)
+    with pytest.raises(TrsError) as e:
+        build_format(rp.cuda(), col.cuda(), torch.ones(16 * entries).cuda())
+    assert e.value.code == -8

@@ -1703,6 +1703,9 @@ struct Event {
     ~Event() { if (e) cudaEventDestroy(e); }
 };
 
+struct HubBack {   // what the host sees of the hub windows before their records are made
+    int records, err;
+};
 struct Records {   // stages 1 - 3
     WindowOut w{};
     int* sel = nullptr;   // [kSortClasses + 1][W]
@@ -1730,7 +1733,7 @@ int sort_class(const InputInfo& info, const int* rowptr, const int* col, const f
 // `meanwhile` queues what does not depend on the hub windows
 template <class Key, class Other>
 int sort_hubs(trs_builder* B, const int* rowptr, const int* col, const float* val, const InputInfo& info, InputInfo* d_info,
-              int* d_count, int* h_count, int col_bits, TempSpace& ts, Cub& cub_, cudaStream_t st, const Records& R, Other&& meanwhile) {
+              int* d_count, HubBack* back, int col_bits, TempSpace& ts, Cub& cub_, cudaStream_t st, const Records& R, Other&& meanwhile) {
     const int H = info.windows[kSortClasses], E = (int)info.hub_entries, n = B->n_rows, window = B->cfg.window;
     const int h_bits = bits_for(H - 1);
     const int* sel = R.sel + (size_t)kSortClasses * B->W;
@@ -1756,10 +1759,11 @@ int sort_hubs(trs_builder* B, const int* rowptr, const int* col, const float* va
     TRS_TRY(cub_.run([&](void* t, size_t& b) {
         return cub::DeviceSelect::If(t, b, thrust::counting_iterator<int>(0), start, d_count, E, is_head, st);
     }));
-    TRS_TRY(publish(d_count, h_count, st));
+    TRS_TRY(publish((const int*)d_count, &back->records, (const int*)&d_info->err, &back->err, st));
     TRS_TRY(meanwhile());
     TRS_CUDA(cudaStreamSynchronize(st));
-    const int D = *h_count;
+    if (back->err & 2) return TRS_E_NOT_CANONICAL;   // a repeated column may have more entries than a record counts
+    const int D = back->records;
     Record* record;
     unsigned *key2_a, *key2_b, *key2;
     int *ord_a, *ord_b, *ord;
@@ -1784,7 +1788,7 @@ int sort_hubs(trs_builder* B, const int* rowptr, const int* col, const float* va
 // half busy one after the other (R-MAT 18: 180 us): with more than one of them in a graph, two other streams take the
 // classes beside the chain (whole build of R-MAT 15 662 -> 541 us, of R-MAT 18 1470 -> 1338, with the sizes read back by kernels).
 int make_records(trs_builder* B, const int* rowptr, const int* col, const float* val, const InputInfo& info, InputInfo* d_info,
-                 int* d_count, int* h_count, TempSpace& ts, Cub& cub_, cudaStream_t st, Records* R) {
+                 int* d_count, HubBack* back, TempSpace& ts, Cub& cub_, cudaStream_t st, Records* R) {
     const int col_bits = bits_for(info.max_col), W = B->W;
     const size_t nnz = (size_t)B->nnz;
     TRS_TRY(ts.get(nnz, &R->w.rec));
@@ -1809,8 +1813,8 @@ int make_records(trs_builder* B, const int* rowptr, const int* col, const float*
     int rc = 0;
     if (info.windows[kSortClasses] > 0) {
         const int h_bits = bits_for(info.windows[kSortClasses] - 1);
-        rc = col_bits + h_bits <= 32 ? sort_hubs<unsigned>(B, rowptr, col, val, info, d_info, d_count, h_count, col_bits, ts, cub_, st, *R, classes)
-                                     : sort_hubs<u64>(B, rowptr, col, val, info, d_info, d_count, h_count, col_bits, ts, cub_, st, *R, classes);
+        rc = col_bits + h_bits <= 32 ? sort_hubs<unsigned>(B, rowptr, col, val, info, d_info, d_count, back, col_bits, ts, cub_, st, *R, classes)
+                                     : sort_hubs<u64>(B, rowptr, col, val, info, d_info, d_count, back, col_bits, ts, cub_, st, *R, classes);
     } else {
         rc = classes();
     }
@@ -1850,7 +1854,7 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     // ---- sizes of the input ---------------------------------------------------------------------
     struct Counts { InputInfo info; MatchCounts mc; };
     struct Head { Counts counts; u64 dropped[kDropCounters]; int hub_records, pad; };
-    struct Back { Head head; Win total; Parts parts; int groups, tiles, tc_nnz; };   // what the host sees of it
+    struct Back { Head head; HubBack hub; Win total; Parts parts; int groups, tiles, tc_nnz; };   // what the host sees of it
     static_assert(sizeof(Back) <= Mirror::kBytes, "");
     Mirror mirror;
     TRS_TRY(mirror.take(st));
@@ -1871,7 +1875,7 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     ts.chunk_bytes = std::max((size_t)16 << 20, (size_t)nnz * 28);
 
     // ---- 1. - 3. columns of every window in (count desc, col asc) order ---------------------------
-    TRS_TRY(make_records(B, rowptr, col, val, info, &d_head->counts.info, &d_head->hub_records, &back->head.hub_records, ts, cub_, st, &R));
+    TRS_TRY(make_records(B, rowptr, col, val, info, &d_head->counts.info, &d_head->hub_records, &back->hub, ts, cub_, st, &R));
     const RecordView rv{R.w.rec, R.w.sval};
 
     // ---- 4., 5. TC columns, units, sizes per window ---------------------------------------------
