@@ -91,3 +91,10 @@ def test_repeated_columns_are_refused(entries):
     with pytest.raises(TrsError) as e:
         build_format(rp.cuda(), col.cuda(), torch.ones(16 * entries).cuda())
     assert e.value.code == -8
+
+
+def test_entries_without_arrays_are_refused():
+    empty = torch.zeros(0, dtype=torch.int32).cuda()
+    with pytest.raises(TrsError) as e:
+        build_format(torch.arange(17, dtype=torch.int32).cuda(), empty, empty.float())
+    assert e.value.code == -1

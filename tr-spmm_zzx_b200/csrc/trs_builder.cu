@@ -1872,6 +1872,7 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     if (info.first != 0 || info.last < 0 || (info.err & 1)) return TRS_E_OFFSETS;
     const long long nnz = B->nnz = info.last;
     if (nnz == 0) return empty_outputs(B, st);
+    if (!col || !val) return TRS_E_ARG;
     ts.chunk_bytes = std::max((size_t)16 << 20, (size_t)nnz * 28);
 
     // ---- 1. - 3. columns of every window in (count desc, col asc) order ---------------------------
