@@ -25,20 +25,45 @@ def test_round_trip(sizes):
 
 
 def test_results_in_reused_blocks():
-    """A result block is page-locked on its second use and copied into directly, beside arrays that are staged."""
+    """Result blocks are used again and stay ordinary memory, beside small arrays that are not pooled."""
     from trspmm import _hostpool
     dev = torch.device("cuda", 0)
     _hostpool.release()
     src = [torch.arange(n, dtype=torch.int32, device=dev) for n in (3 * MB, 100, MB // 8, 2 * MB + 3)]
-    locked = []
     for k in range(4):
         got = _lib.copy_to_host([s + k for s in src], dev)
         for a, b in zip(got, src):
             assert torch.equal(a, (b + k).cpu())
-        locked.append(got[0].is_pinned())
+        assert not any(t.is_pinned() for t in got)
         del got, a
-    assert not locked[0] and locked[-1]
     _hostpool.release()
+
+
+def test_result_dropped_while_it_is_copied():
+    """A caller queues a copy of a result behind work on a stream of its own and drops the result: the next results
+    must not reach the copy."""
+    dev = torch.device("cuda", 0)
+    side, src, copies = torch.cuda.Stream(), torch.arange(4 * MB, dtype=torch.int32, device=dev), []
+    for k in range(6):
+        got = _lib.copy_to_host([src + k], dev)
+        with torch.cuda.stream(side):
+            torch.cuda._sleep(20_000_000)
+            copies.append(got[0].to(dev, non_blocking=True))
+        del got
+    torch.cuda.synchronize()
+    for k, c in enumerate(copies):
+        assert torch.equal(c, src + k)
+
+
+def test_page_locked_arrays():
+    """Arrays that the caller has page-locked, as torch does or through the library, beside pageable ones."""
+    dev, lib = torch.device("cuda", 0), _lib.load()
+    host = [torch.arange(n, dtype=torch.int32) for n in (MB, 2 * MB + 5, 100)]
+    host[0] = host[0].pin_memory()
+    _lib.check(lib.trs_host_register(host[1].data_ptr(), host[1].numel() * 4))
+    for a, b in zip(_lib.copy_to_device(host, dev), host):
+        assert torch.equal(a, b.cuda())
+    _lib.check(lib.trs_host_unregister(host[1].data_ptr()))
 
 
 def test_two_threads():

@@ -3,8 +3,10 @@
 The reference's calling convention returns a new CPU tensor per call.  For a result of tens of megabytes the page
 faults of fresh memory cost more than the copy from the device (33 MB: 1.7 against 0.6 ms), and the C library gives
 such blocks back to the system every time.  Blocks handed out here return to a list when the last tensor
-over them is gone; at most KEEP_BYTES wait there, the oldest go first, release() lets all of them go.  A block that
-comes back into use is page-locked (a few milliseconds, once), after which the device copies into it directly.
+over them is gone; at most KEEP_BYTES wait there, the oldest go first, release() lets all of them go.
+
+They are never page-locked: a copy from page-locked memory may still be under way when the tensor is gone, and nothing
+would keep the block from the next result until then.
 """
 from __future__ import annotations
 
@@ -31,45 +33,26 @@ class _Block:
         self.bytes = -(-n // _BLOCK) * _BLOCK
         self.memory = mmap.mmap(-1, self.bytes)
         self.address = np.frombuffer(self.memory, dtype=np.uint8).ctypes.data
-        self.locked = None   # not tried yet
         if hasattr(mmap, "MADV_HUGEPAGE"):
             try:
                 self.memory.madvise(mmap.MADV_HUGEPAGE)
             except OSError:   # a kernel without large pages
                 pass
 
-    def lock(self):
-        if self.locked is None:
-            from . import _lib
-            self.locked = torch.cuda.is_initialized() and _lib.load().trs_host_register(self.address, self.bytes) == 0
-
-    def unlock(self):
-        if self.locked:
-            from . import _lib
-            _lib.load().trs_host_unregister(self.address)
-            self.locked = None
-
 
 def _give_back(block):
-    gone = []
     with _lock:
         _idle.append(block)
         waiting = sum(b.bytes for b in _idle)
         while waiting > KEEP_BYTES:
-            gone.append(_idle.pop(0))
-            waiting -= gone[-1].bytes
-    for b in gone:
-        b.unlock()
+            waiting -= _idle.pop(0).bytes
 
 
 def _take(n: int):
     with _lock:
         fits = [i for i, b in enumerate(_idle) if n <= b.bytes <= n + n // 4 + _BLOCK]
         block = _idle.pop(min(fits, key=lambda i: _idle[i].bytes)) if fits else None
-    if block is None:
-        return _Block(n)
-    block.lock()
-    return block
+    return _Block(n) if block is None else block
 
 
 def empty(shape, dtype: torch.dtype) -> torch.Tensor:
@@ -93,7 +76,4 @@ def empty(shape, dtype: torch.dtype) -> torch.Tensor:
 
 def release():
     with _lock:
-        gone = _idle[:]
         _idle.clear()
-    for b in gone:
-        b.unlock()
