@@ -93,3 +93,12 @@ def test_private_after_a_fork():
     b = _hostpool.empty((1 << 20,), torch.float32).fill_(3)
     os.write(to_child[1], b"w")
     assert os.waitstatus_to_exitcode(os.waitpid(pid, 0)[1]) == 0 and same and b.data_ptr() == at
+
+
+def test_allocates_what_it_returns(monkeypatch):
+    """The first result makes no allocation but its own: the heap's policy is the program's."""
+    sizes, empty = [], torch.empty
+    monkeypatch.setattr(torch, "empty", lambda *a, **k: sizes.append(a[0]) or empty(*a, **k))
+    monkeypatch.setattr(_hostpool, "_adapted", False, raising=False)
+    _hostpool.empty((1 << 20,), torch.float32)
+    assert sorted(sizes) == [0, 4 << 20]

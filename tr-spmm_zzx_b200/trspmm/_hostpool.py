@@ -20,7 +20,6 @@ import torch
 MIN_BYTES = 1 << 20      # below, the C library reuses memory itself
 KEEP_BYTES = 256 << 20
 
-_adapted = False
 _use_count = getattr(torch._C, "_storage_Use_Count", None)
 
 _lock = threading.Lock()
@@ -56,13 +55,6 @@ def empty(shape, dtype: torch.dtype) -> torch.Tensor:
     n = math.prod(shape) * dtype.itemsize
     if n < MIN_BYTES or n > KEEP_BYTES or _use_count is None:
         return torch.empty(shape, dtype=dtype, device="cpu")
-    global _adapted
-    if not _adapted:
-        # The C library takes blocks up to the largest one freed so far (32 MB at most) from its heap, larger ones from the
-        # system each time.  Results used to raise that mark; without them a program's own arrays of a few
-        # megabytes would fault their pages in anew on every allocation.
-        _adapted = True
-        torch.empty(31 << 20, dtype=torch.uint8)
     with _lock:
         block = _take(n)
         out = torch.empty(0, dtype=dtype, device="cpu").set_(block.storage, 0, shape)
