@@ -66,6 +66,17 @@ def test_page_locked_arrays():
     _lib.check(lib.trs_host_unregister(host[1].data_ptr()))
 
 
+@pytest.mark.parametrize("n", [100, MB // 8 - 1, MB // 8])
+def test_page_locked_array_written_after_the_upload(n):
+    """An upload has read its arrays when it returns, small page-locked ones behind earlier work too."""
+    dev = torch.device("cuda", 0)
+    host = torch.arange(n, dtype=torch.int32).pin_memory()
+    torch.cuda._sleep(50_000_000)
+    up = _lib.copy_to_device([host], dev)[0]
+    host.zero_()
+    assert torch.equal(up.cpu(), torch.arange(n, dtype=torch.int32))
+
+
 def test_two_threads():
     dev = torch.device("cuda", 0)
     data = [torch.arange(9 * MB + i, dtype=torch.int32) for i in range(2)]

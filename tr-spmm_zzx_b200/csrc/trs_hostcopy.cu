@@ -236,20 +236,23 @@ Copier& copier() {
     return *c;
 }
 
+// Memory that the copy engine reads or writes directly, after the call has returned if nothing waits for it.
+bool page_locked(const void* p) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
+    return a.type != cudaMemoryTypeUnregistered;
+}
+
 int plain(const HostSegment* seg, int n, bool to_host, cudaStream_t st) {
+    bool wait = to_host;
     for (int i = 0; i < n; ++i) {
         if (!seg[i].bytes) continue;
         if (to_host) TRS_CUDA(cudaMemcpyAsync(seg[i].host, seg[i].dev, seg[i].bytes, cudaMemcpyDeviceToHost, st));
         else TRS_CUDA(cudaMemcpyAsync(seg[i].dev, seg[i].host, seg[i].bytes, cudaMemcpyHostToDevice, st));
+        wait = wait || page_locked(seg[i].host);
     }
-    if (to_host) TRS_CUDA(cudaStreamSynchronize(st));
+    if (wait) TRS_CUDA(cudaStreamSynchronize(st));
     return 0;
-}
-
-bool page_locked(const void* p) {
-    cudaPointerAttributes a;
-    if (cudaPointerGetAttributes(&a, p) != cudaSuccess) { cudaGetLastError(); return false; }
-    return a.type == cudaMemoryTypeHost;
 }
 
 int staged(const HostSegment* all, int n_all, bool to_host, cudaStream_t st) {
