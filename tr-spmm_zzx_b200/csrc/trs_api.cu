@@ -126,8 +126,10 @@ struct Upload {
         if (n) parts.push_back(Part{nullptr, n * sizeof(T), (void**)dev});
     }
     int commit() {
+        std::vector<Part> noted;   // forgotten whatever happens: their `dev` may live on a caller's stack
+        noted.swap(parts);
         size_t total = 0;
-        for (const Part& p : parts) total += (p.bytes + 255) & ~(size_t)255;
+        for (const Part& p : noted) total += (p.bytes + 255) & ~(size_t)255;
         if (total == 0) return 0;
         TRS_CUDA(cudaGetDevice(&device));
         void* block;
@@ -136,12 +138,11 @@ struct Upload {
         blocks.push_back(block);
         std::vector<HostSegment> seg;
         unsigned char* at = (unsigned char*)block;
-        for (const Part& p : parts) {
+        for (const Part& p : noted) {
             *p.dev = at;
             if (p.host) seg.push_back(HostSegment{(void*)p.host, at, p.bytes});
             at += (p.bytes + 255) & ~(size_t)255;
         }
-        parts.clear();
         return copy_to_device(seg.data(), (int)seg.size(), st);
     }
     template <class T>
