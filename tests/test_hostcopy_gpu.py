@@ -1,5 +1,7 @@
 """Copies between pageable host arrays and the device: sizes around a chunk and around the whole pinned ring, many
 arrays in one call, two threads at once."""
+import subprocess
+import sys
 import threading
 
 import pytest
@@ -93,3 +95,32 @@ def test_two_threads():
     assert not bad
     assert _lib.load().trs_pool_trim() == 0
     assert torch.equal(_lib.copy_to_host([data[0].cuda()], dev)[0], data[0])   # the ring comes back after a trim
+
+
+def test_no_threads_to_be_had():
+    """Where the system gives no threads, copies and the host entries go without.  (A child process whose default thread
+    stack is larger than the address space.)"""
+    code = """
+import ctypes, sys
+sys.path[:0] = [%r, %r]
+import torch
+from trspmm import SpmmPlan, _lib, build_format, graphs, spmm_forward_host
+rp, col, val = graphs.uniform_graph(1 << 15, 8, seed=1, device="cuda")
+n = rp.numel() - 1
+fmt = build_format(rp, col, val)[0]
+B = torch.randn(n, 64).half()
+want = SpmmPlan(fmt, n, n).run(B.cuda(), out_dtype=torch.float32).cpu()
+host = fmt.half_values().to("cpu")
+torch.cuda.synchronize()
+libc, attr = ctypes.CDLL(None), ctypes.create_string_buffer(256)
+assert libc.pthread_attr_init(attr) == 0
+assert libc.pthread_attr_setstacksize(attr, ctypes.c_size_t(1 << 48)) == 0
+assert libc.pthread_setattr_default_np(attr) == 0
+data = torch.arange(3 << 20, dtype=torch.int32)
+dev = torch.device("cuda", 0)
+assert torch.equal(_lib.copy_to_host(_lib.copy_to_device([data], dev), dev)[0], data)
+assert torch.equal(spmm_forward_host(host, B, 64, n, n)[0], want)
+print("done")
+""" % (str(_lib.PKG_ROOT), str(_lib.PKG_ROOT.parent))
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300)
+    assert r.returncode == 0 and r.stdout.strip() == "done", r.stderr[-2000:]

@@ -493,7 +493,7 @@ int resident_check_args(trs_resident* h, const trs_half* rhs_host, void* out_hos
 }  // namespace
 
 extern "C" int trs_resident_create(const trs_format* host_format, int mOri, int kOri, int window, int max_dimN,
-                                   trs_resident** out) {
+                                   trs_resident** out) try {
     if (!host_format || !out || max_dimN <= 0) return TRS_E_ARG;
     *out = nullptr;
     if (mOri <= 0 || kOri <= 0) return TRS_E_ARG;
@@ -506,10 +506,10 @@ extern "C" int trs_resident_create(const trs_format* host_format, int mOri, int 
     if (rc) { trs_resident_destroy(h); return rc; }
     *out = h;
     return TRS_OK;
-}
+} TRS_CATCH
 
 extern "C" int trs_resident_create_device(const trs_format* dev_format, int mOri, int kOri, int window, int max_dimN,
-                                          trs_resident** out) {
+                                          trs_resident** out) try {
     if (!dev_format || !out || max_dimN <= 0) return TRS_E_ARG;
     *out = nullptr;
     if (mOri <= 0 || kOri <= 0) return TRS_E_ARG;
@@ -521,7 +521,7 @@ extern "C" int trs_resident_create_device(const trs_format* dev_format, int mOri
     if (rc) { trs_resident_destroy(h); return rc; }
     *out = h;
     return TRS_OK;
-}
+} TRS_CATCH
 
 extern "C" int trs_resident_destroy(trs_resident* h) {
     if (!h) return TRS_OK;
@@ -545,7 +545,7 @@ extern "C" int trs_resident_destroy(trs_resident* h) {
 }
 
 extern "C" int trs_resident_forward(trs_resident* h, const trs_half* rhs_host, void* out_host, int dimN, int out_dtype,
-                                    trs_timing* timing) {
+                                    trs_timing* timing) try {
     int rc = resident_check_args(h, rhs_host, out_host, dimN, out_dtype);
     if (rc) return rc;
     if (timing) memset(timing, 0, sizeof(*timing));
@@ -563,15 +563,15 @@ extern "C" int trs_resident_forward(trs_resident* h, const trs_half* rhs_host, v
         cudaEventElapsedTime(&timing->d2h_ms, h->t_ev[4], h->t_ev[5]);
     }
     return TRS_OK;
-}
+} TRS_CATCH
 
-extern "C" int trs_resident_submit(trs_resident* h, const trs_half* rhs_host, void* out_host, int dimN, int out_dtype) {
+extern "C" int trs_resident_submit(trs_resident* h, const trs_half* rhs_host, void* out_host, int dimN, int out_dtype) try {
     int rc = resident_check_args(h, rhs_host, out_host, dimN, out_dtype);
     if (rc) return rc;
     rc = resident_enqueue(h, rhs_host, out_host, dimN, out_dtype, false);
     if (rc && !h->pending_rc) h->pending_rc = rc;
     return rc;
-}
+} TRS_CATCH
 
 extern "C" int trs_resident_wait(trs_resident* h) {
     if (!h) return TRS_E_ARG;
@@ -582,7 +582,7 @@ extern "C" int trs_resident_wait(trs_resident* h) {
 }
 
 extern "C" int trs_spmm_forward_host(const trs_format* host_format, const trs_half* rhs_host, float* out_host, int dimN,
-                                     int mOri, int kOri, int window, int epoches, trs_timing* timing) {
+                                     int mOri, int kOri, int window, int epoches, trs_timing* timing) try {
     if (!host_format || !rhs_host || !out_host) return TRS_E_ARG;
     if (dimN <= 0 || mOri <= 0 || kOri <= 0 || epoches <= 0) return TRS_E_ARG;
     if (window <= 0 || window > 16) return TRS_E_WINDOW;
@@ -632,12 +632,12 @@ extern "C" int trs_spmm_forward_host(const trs_format* host_format, const trs_ha
         timing->total_ms = ev.ms() / (float)epoches;
     }
     return rc;
-}
+} TRS_CATCH
 
 extern "C" int trs_sptc_unpacked_forward_host(const int32_t* s_column, const float* s_value, const int8_t* s_pos,
                                               const int32_t* s_window, const int32_t* s_offsets, int groups,
                                               int num_windows, const trs_half* rhs_host, float* out_host, int window,
-                                              int dimN, int mOri, int kOri, int epoches, trs_timing* timing) {
+                                              int dimN, int mOri, int kOri, int epoches, trs_timing* timing) try {
     if (!rhs_host || !out_host || groups < 0) return TRS_E_ARG;
     if (dimN <= 0 || mOri <= 0 || kOri <= 0 || epoches <= 0) return TRS_E_ARG;
     if (window <= 0 || window > 16) return TRS_E_WINDOW;
@@ -705,4 +705,4 @@ extern "C" int trs_sptc_unpacked_forward_host(const int32_t* s_column, const flo
     f.num_windows = num_windows;
     f.tiles = tiles;
     return trs_spmm_forward_host(&f, rhs_host, out_host, dimN, mOri, kOri, window, epoches, timing);
-}
+} TRS_CATCH

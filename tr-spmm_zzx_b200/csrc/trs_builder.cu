@@ -2143,7 +2143,7 @@ const void* array_ptr(const trs_builder* B, int id, size_t* elem) {
 
 static int build_impl(const int32_t* rowptr, const int32_t* col, const float* values, int n_rows,
                       const trs_build_config* cfg, void* arena, size_t arena_bytes, bool use_arena, trs_build_alloc alloc,
-                      void* ctx, void* stream, trs_builder** out) {
+                      void* ctx, void* stream, trs_builder** out) try {
     if (!rowptr || !cfg || !out || n_rows <= 0) return TRS_E_ARG;
     *out = nullptr;
     if (cfg->window <= 0 || cfg->window > 16) return TRS_E_WINDOW;
@@ -2177,7 +2177,7 @@ static int build_impl(const int32_t* rowptr, const int32_t* col, const float* va
     fill_sizes(B);
     *out = B;
     return TRS_OK;
-}
+} TRS_CATCH
 
 extern "C" int trs_build_create(const int32_t* rowptr, const int32_t* col, const float* values, int n_rows,
                                 const trs_build_config* cfg, void* stream, trs_builder** out) {

@@ -6,6 +6,9 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <exception>
+#include <new>
+
 #include "trspmm.h"
 
 #define TRS_CUDA(expr)                                     \
@@ -19,6 +22,11 @@
         cudaError_t _e = cudaGetLastError();               \
         if (_e != cudaSuccess) return (int)_e;             \
     } while (0)
+
+// Ends a function-try-block of a C entry: no C++ exception crosses it.
+#define TRS_CATCH                                                                     \
+    catch (const std::bad_alloc&) { return (int)cudaErrorMemoryAllocation; }          \
+    catch (const std::exception&) { return (int)cudaErrorOperatingSystem; }
 
 namespace trs {
 

@@ -16,6 +16,7 @@
 #include <atomic>
 #include <condition_variable>
 #include <mutex>
+#include <system_error>
 #include <thread>
 #include <vector>
 
@@ -144,8 +145,10 @@ struct Copier {
         if (workers == 0) {
             const int hw = (int)std::thread::hardware_concurrency();
             const int want = hw >= 4 ? (hw / 2 < kMaxWorkers ? hw / 2 : kMaxWorkers) : 1;
-            for (int i = 0; i < want; ++i) std::thread([this] { worker_main(); }).detach();
-            workers = want;
+            try {
+                for (; workers < want; ++workers) std::thread([this] { worker_main(); }).detach();
+            } catch (const std::system_error&) {   // no more threads to be had: those that there are do the work
+            }
         }
         return drain();
     }
@@ -283,6 +286,7 @@ int staged(const HostSegment* all, int n_all, bool to_host, cudaStream_t st) {
     if (total < kStageFrom || !lock.try_lock()) return plain(seg, n, to_host, st);
     const int rc = c.prepare();
     if (rc) return rc;
+    if (c.workers == 0) return plain(seg, n, to_host, st);
     if (to_host)
         for (int i = 0; i < n; ++i) ask_for_large_pages(seg[i]);
     // Chunks of 1 MiB, but small ones where nothing else runs beside them: at the start of an upload (the copy engine waits for
@@ -344,14 +348,14 @@ extern "C" int trs_host_unregister(void* host) {
     return (int)e;
 }
 
-extern "C" int trs_copy_to_host(int n, void* const* host, const void* const* dev, const size_t* bytes, void* stream) {
+extern "C" int trs_copy_to_host(int n, void* const* host, const void* const* dev, const size_t* bytes, void* stream) try {
     std::vector<trs::HostSegment> seg;
     const int rc = segments(n, host, (void* const*)dev, bytes, &seg);
     return rc ? rc : trs::copy_to_host(seg.data(), (int)seg.size(), (cudaStream_t)stream);
-}
+} TRS_CATCH
 
-extern "C" int trs_copy_to_device(int n, const void* const* host, void* const* dev, const size_t* bytes, void* stream) {
+extern "C" int trs_copy_to_device(int n, const void* const* host, void* const* dev, const size_t* bytes, void* stream) try {
     std::vector<trs::HostSegment> seg;
     const int rc = segments(n, (void* const*)host, dev, bytes, &seg);
     return rc ? rc : trs::copy_to_device(seg.data(), (int)seg.size(), (cudaStream_t)stream);
-}
+} TRS_CATCH

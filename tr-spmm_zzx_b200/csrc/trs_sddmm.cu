@@ -479,7 +479,7 @@ extern "C" int trs_sddmm_plan_destroy(trs_sddmm_plan* p) {
 }
 
 extern "C" int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, int n_rows, int n_cols, void* stream,
-                                     trs_sddmm_plan** out) {
+                                     trs_sddmm_plan** out) try {
     using namespace trs;
     if (!out) return TRS_E_ARG;
     *out = nullptr;
@@ -579,7 +579,7 @@ extern "C" int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, 
     p->wide = (herr & 4) != 0;
     *out = p;
     return TRS_OK;
-}
+} TRS_CATCH
 
 extern "C" int trs_sddmm_plan_info(const trs_sddmm_plan* p, long long* n_pairs, long long* n_blocks) {
     if (!p) return TRS_E_ARG;
@@ -732,7 +732,7 @@ extern "C" int trs_sddmm_plan_run_ex(const trs_sddmm_plan* p, const trs_half* X,
 }
 
 extern "C" int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_half* X, const trs_half* Y, trs_half* out,
-                         int n_rows, int n_cols, int K, void* stream) {
+                         int n_rows, int n_cols, int K, void* stream) try {
     if (!rowptr || !X || !Y || n_rows <= 0 || n_cols <= 0 || K <= 0) return TRS_E_ARG;
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return TRS_E_NO_DEVICE;
@@ -762,4 +762,4 @@ extern "C" int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_ha
     if (first != 0 || last < 0) return TRS_E_OFFSETS;
     if (last > 0 && (!col || !out)) return TRS_E_ARG;
     return TRS_OK;
-}
+} TRS_CATCH

@@ -793,7 +793,7 @@ static int validate_on_device(const trs_format& f, int m_rows, int k_cols, int n
 // short column array cannot be over-read: the caller states the lengths implicitly through the
 // prefix arrays, exactly as the reference does (mGCN_online.cpp:982-1042 copies numel() items).
 extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, int k_cols, int window, int validate,
-                                    void* stream, trs_spmm_plan** out_plan) {
+                                    void* stream, trs_spmm_plan** out_plan) try {
     if (!dev_format || !out_plan) return TRS_E_ARG;
     *out_plan = nullptr;
     if (m_rows <= 0 || k_cols <= 0) return TRS_E_ARG;
@@ -904,7 +904,7 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     if (e != cudaSuccess) return fail((int)e);
     *out_plan = p;
     return TRS_OK;
-}
+} TRS_CATCH
 
 // No kernel of this library waits on a flag or a barrier that another warp or kernel sets (the
 // window kernels synchronise inside one warp or one CTA only), so there is no wait that could
