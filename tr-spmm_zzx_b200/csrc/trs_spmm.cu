@@ -64,7 +64,7 @@ struct KernelArgs {
     const Item* items;             // longest first
     int n_items;
     int w_begin, w_end;            // window range of this run (RANGE instances: items outside return at once)
-    const int* ids;                // [steps + kIdBlock][16] column ids of the step stream
+    const int* ids;                // [steps + kIdSpare][16] column ids of the step stream
     const uint32_t* packed_a;      // [tiles][64]
     const uint32_t* packed_meta;   // [tiles][8]
     const uint4* dense;            // [dense steps][32] A tiles in fragment order, one uint4 per lane
@@ -308,6 +308,9 @@ __global__ void k_check_sorted(const int* __restrict__ a, int n, int* err) {
 // of 8 steps (512 bytes, one cp.async per lane).  The A operand goes straight into registers
 // STAGES - 1 steps ahead, so the ring holds gathered rows only.
 constexpr int kIdBlock = 8;   // steps per block of column ids
+// Step j of an item, j a multiple of kIdBlock, asks for the ids of steps j + kIdBlock .. j + 2 kIdBlock - 1, whether the
+// item has them or not, so the array goes on that far behind the last step.
+constexpr int kIdSpare = 2 * kIdBlock;
 
 template <int FS, int STAGES>
 struct WarpTile {
@@ -494,7 +497,7 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
 #pragma unroll
         for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 
-    auto issue_ids = [&](int blk) {   // ids of steps 8 blk .. 8 blk + 7 (the array ends with a spare block)
+    auto issue_ids = [&](int blk) {   // ids of steps 8 blk .. 8 blk + 7
         cp_async16(smem0 + ids_at + (blk & 1) * (kIdBlock * 64) + lane * 16, ids + blk * (kIdBlock * 16) + lane * 4);
     };
     auto gather = [&](int j, auto stage) {
@@ -710,7 +713,7 @@ struct trs_spmm_plan {
     void* block = nullptr;   // the arrays below
     Item* items = nullptr;   // long ones first
     Heavy* heavy = nullptr;
-    int* ids = nullptr;      // [steps + kIdBlock][16] column ids of the step stream
+    int* ids = nullptr;      // [steps + kIdSpare][16] column ids of the step stream
     uint4* dense = nullptr;  // [dense steps][32] A tiles of the dense steps in fragment order
     int n_items, n_heavy, n_slots;
     bool few_items;                   // four warps per item
@@ -872,7 +875,7 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     p->m_rows = m_rows; p->k_cols = k_cols; p->window = window; p->num_windows = W; p->device = dev;
     p->n_items = n_items; p->n_heavy = n_heavy; p->n_slots = info.totals[WC_SLOTS];
     p->few_items = n_steps / (sms * kWarpsPerSm) < kFewSteps;
-    const size_t ids_bytes = ((size_t)n_steps + kIdBlock) * 64, dense_bytes = (size_t)n_dense * 512;
+    const size_t ids_bytes = ((size_t)n_steps + kIdSpare) * 64, dense_bytes = (size_t)n_dense * 512;
     const size_t items_bytes = (size_t)n_items * sizeof(Item), heavy_bytes = (size_t)n_heavy * sizeof(Heavy);
     auto fail = [&](int code) { trs_spmm_plan_destroy(p); return code; };
     if ((rc = pool_alloc(&p->block, ids_bytes + dense_bytes + items_bytes + heavy_bytes, st))) return fail(rc);
