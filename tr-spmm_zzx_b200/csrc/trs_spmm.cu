@@ -42,7 +42,7 @@ struct Item {        // 32 bytes: everything a warp needs to start
     int nsteps;
     int tile0;       // packed tile of step 0
     int dense0;      // dense tile of step nsparse
-    int pad;
+    int open;        // first packed step of the window, in the stream, with an open slot
 };
 
 struct Heavy {
@@ -169,17 +169,18 @@ __global__ void k_fill_items(trs_format f, WindowRanges wr, int num_windows, con
     for (int i = 0; i < n; ++i) {
         const int b = min(i * per, steps), e = min(b + per, steps);
         items[i0 + i] = Item{w, n > 1 ? slot0 + i : -1, step0 + b, min(max(tiles - b, 0), e - b), e - b, tile0 + b,
-                             dense0 + max(b - tiles, 0), 0};
+                             dense0 + max(b - tiles, 0), 0x7fffffff};
     }
     if (n > 1) heavy[heavy0] = Heavy{w, slot0, slot0 + n};
 }
 
-// The step stream, one warp per item.  An unused column slot of a step repeats the step's first
-// column (its A entries are zero), so that the gather needs no special case; a step without any
-// column takes column 0.
+// The step stream, one warp per item.  An unused column slot of a step repeats the step's first column, so that the gather
+// needs no special case.  Its A entries are zero, but zero times an infinity is not: where the multiplication looks at such
+// a slot - always in a dense tile, in a packed one if a row's metadata names it - the slot stays open (-1), and the
+// gather fills it with zeros.  `open[w]`: the window's first packed step with an open slot.
 __global__ void k_fill_steps(trs_format f, WindowRanges wr, const Item* __restrict__ items, int n_items,
                              const int* __restrict__ off, int num_windows, int window, int* __restrict__ ids,
-                             uint4* __restrict__ dense) {
+                             uint4* __restrict__ dense, int* __restrict__ open) {
     const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5;
     const int lane = threadIdx.x & 31;
     if (i >= n_items) return;
@@ -190,7 +191,19 @@ __global__ void k_fill_steps(trs_format f, WindowRanges wr, const Item* __restri
         if (lane < 16) c = f.s_tile_column[(size_t)(it.tile0 + j) * 16 + lane];
         const unsigned have = __ballot_sync(0xffffffffu, c >= 0);
         const int dup = have ? __shfl_sync(0xffffffffu, c, __ffs(have) - 1) : 0;
-        if (lane < 16) ids[((size_t)it.step0 + j) * 16 + lane] = c >= 0 ? c : dup;
+        bool is_open = false;
+        if (have != 0xffffu) {
+            unsigned used = 0;   // slots that a row's two positions per group name
+            if (lane < 8) {
+                const unsigned m = f.s_packed_meta[(size_t)(it.tile0 + j) * 8 + lane];
+#pragma unroll
+                for (int i = 0; i < 8; ++i)
+                    used |= ((1u << ((m >> (4 * i)) & 3u)) | (1u << ((m >> (4 * i + 2)) & 3u))) << (4 * (i & 3));
+            }
+            is_open = (__reduce_or_sync(0xffffffffu, used) & ~have) != 0;
+            if (is_open && lane == 0) atomicMin(open + w, it.step0 + j);
+        }
+        if (lane < 16) ids[((size_t)it.step0 + j) * 16 + lane] = c >= 0 ? c : is_open ? -1 : dup;
     }
     if (it.nsteps == it.nsparse) return;
     const WindowSteps ws = window_steps(f, wr, w);
@@ -246,9 +259,7 @@ __global__ void k_fill_steps(trs_format f, WindowRanges wr, const Item* __restri
                 if ((e1 >> 16) == row) a[q] |= e1 << 16;
             }
         }
-        const unsigned have = __ballot_sync(0xffffffffu, c >= 0);
-        const int dup = have ? __shfl_sync(0xffffffffu, c, __ffs(have) - 1) : 0;
-        if (lane < 16) ids[((size_t)it.step0 + j) * 16 + lane] = c >= 0 ? c : dup;
+        if (lane < 16) ids[((size_t)it.step0 + j) * 16 + lane] = c;
         dense[((size_t)it.dense0 + j - it.nsparse) * 32 + lane] = make_uint4(a[0], a[1], a[2], a[3]);
     }
 }
@@ -272,9 +283,11 @@ __global__ void k_check_range(const int* __restrict__ a, long long n, int lo, in
 // Launch-order class of an item: long items first, so that the last wave of the grid consists of
 // short ones.  Classes of 8 steps (four classes over the whole range measured 4 - 6 % slower).
 constexpr int kClassBits = 6;
-__global__ void k_item_class(const Item* __restrict__ items, int n, unsigned char* __restrict__ cls) {
+__global__ void k_item_class(Item* __restrict__ items, int n, const int* __restrict__ open, unsigned char* __restrict__ cls) {
     int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i < n) cls[i] = (unsigned char)(63 - min(items[i].nsteps / 8, 63));
+    if (i >= n) return;
+    cls[i] = (unsigned char)(63 - min(items[i].nsteps / 8, 63));
+    items[i].open = open[items[i].window];
 }
 
 // The TC kernels read t_value[t_block_offset[b] + rank] with rank taken from the block's two
@@ -458,6 +471,7 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
         nsteps = min(first + per, it.nsteps) - first;
     }
     const int nsparse = min(max(it.nsparse - first, 0), nsteps);
+    const int nclosed = min(max(it.open - it.step0 - first, 0), nsparse);   // packed tiles before the first with an open slot
     const int* const ids = a.ids + ((size_t)it.step0 + first) * 16;
     const uint32_t* const pa = a.packed_a + (size_t)(it.tile0 + first) * 64 + lane * 2;
     const uint32_t* const pm = a.packed_meta + (size_t)(it.tile0 + first) * 8 + (lane >> 2);
@@ -500,7 +514,8 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
     auto issue_ids = [&](int blk) {   // ids of steps 8 blk .. 8 blk + 7
         cp_async16(smem0 + ids_at + (blk & 1) * (kIdBlock * 64) + lane * 16, ids + blk * (kIdBlock * 16) + lane * 4);
     };
-    auto gather = [&](int j, auto stage) {
+    // `tested`: the step may have open slots
+    auto gather = [&](int j, auto stage, auto tested) {
         const unsigned char* idp = smem + ids_at + (j & (2 * kIdBlock - 1)) * 64;
         int c[T::NCP];
         if constexpr (T::POW2 && T::NCP >= 4) {
@@ -516,11 +531,15 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
 #pragma unroll
         for (int k = 0; k < T::NCP; ++k) {
             if constexpr (ALIGNED) {
-                if (in_row[T::POW2 ? 0 : k])
+                if (!in_row[T::POW2 ? 0 : k]) continue;
+                if constexpr (decltype(tested)::value)   // without a branch: 105 against 109 - 113 us with one (clustered, F = 128)
+                    cp_async16(pdst[k] + decltype(stage)::value * T::STAGE,
+                               src_of(k) + (unsigned long long)(uint32_t)max(c[k], 0) * pitch, (~c[k] >> 27) & 16);
+                else
                     cp_async16_at<decltype(stage)::value * T::STAGE>(pdst[k], src_of(k) + (unsigned long long)(uint32_t)c[k] * pitch);
             } else {
                 const int f = fbase + pc[k] * 8;
-                *(uint4*)(smem + (pdst[k] - smem0) + decltype(stage)::value * T::STAGE) = load_unaligned8(a.B + (size_t)c[k] * a.ldb + f, a.F - f);
+                *(uint4*)(smem + (pdst[k] - smem0) + decltype(stage)::value * T::STAGE) = load_unaligned8(a.B + (size_t)max(c[k], 0) * a.ldb + f, c[k] < 0 ? 0 : a.F - f);
             }
         }
     };
@@ -550,7 +569,7 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
     auto fetch = [&](int j, auto stage) {
         if ((j & (kIdBlock - 1)) == 0) issue_ids(j / kIdBlock + 1);
         areg[decltype(stage)::value] = load_a(j);
-        gather(j, stage);
+        gather(j, stage, std::true_type());
     };
 
     if (nsteps > 0) {
@@ -566,8 +585,8 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
     });
     // group j carries the rows of step j; at iteration j all groups but the newest STAGES - 2 are complete
     int j = 0;
-    // whole rounds of packed tiles
-    for (; j + STAGES + T::AHEAD <= nsparse; j += STAGES) {
+    // whole rounds of packed tiles without open slots
+    for (; j + STAGES + T::AHEAD <= nclosed; j += STAGES) {
         static_for<STAGES>([&](auto uu) {
             constexpr int u = decltype(uu)::value, un = (u + T::AHEAD) % STAGES;
             cp_async_wait<STAGES - 2>();
@@ -578,12 +597,26 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
                 const uint2 v = __ldg((const uint2*)(pa + (size_t)jn * 64));
                 areg[un] = make_uint4(v.x, v.y, __ldg(pm + (size_t)jn * 8), 0u);
             }
-            gather(jn, std::integral_constant<int, un>());
+            gather(jn, std::integral_constant<int, un>(), std::false_type());
             cp_async_commit();
             compute_sparse(uu, areg[u]);
         });
     }
     for (; j < nsteps; j += STAGES) {
+        if (j >= nsparse && j + STAGES + T::AHEAD <= nsteps) {   // a whole round of dense tiles
+            static_for<STAGES>([&](auto uu) {
+                constexpr int u = decltype(uu)::value, un = (u + T::AHEAD) % STAGES;
+                cp_async_wait<STAGES - 2>();
+                __syncwarp();
+                const int jn = j + u + T::AHEAD;
+                if ((jn & (kIdBlock - 1)) == 0) issue_ids(jn / kIdBlock + 1);
+                areg[un] = __ldg(pd + (size_t)jn * 32);
+                gather(jn, std::integral_constant<int, un>(), std::true_type());
+                cp_async_commit();
+                compute_steps<FS, u * T::STAGE, false>(acc, laddr, areg[u]);
+            });
+            continue;
+        }
         static_for<STAGES>([&](auto uu) {
             constexpr int u = decltype(uu)::value, un = (u + T::AHEAD) % STAGES;
             if (j + u < nsteps) {
@@ -886,20 +919,23 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     p->heavy = (Heavy*)at;
 
     Item* by_window;   // items in window order, sorted into p->items
+    int* open;
     unsigned char *cls, *sort_tmp;
     size_t sort_bytes = 0;
     rc = ts.get(n_items, &by_window);
     if (!rc) rc = ts.get((size_t)2 * n_items, &cls);
+    if (!rc) rc = ts.get((size_t)W, &open);
     if (rc) return fail(rc);
     auto sort = [&](void* t) {
         return cub::DeviceRadixSort::SortPairs(t, sort_bytes, cls, cls + n_items, by_window, p->items, n_items, 0, kClassBits, st);
     };
     cudaError_t e = sort(nullptr);
     if (e == cudaSuccess && (rc = ts.get(sort_bytes + 16, &sort_tmp))) return fail(rc);
+    if (e == cudaSuccess) e = cudaMemsetAsync(open, 0x7f, sizeof(int) * (size_t)W, st);
     if (e == cudaSuccess) {
         k_fill_items<<<grid(W), 256, 0, st>>>(f, wr, W, off, by_window, p->heavy);
-        k_fill_steps<<<grid((long long)n_items * 32), 256, 0, st>>>(f, wr, by_window, n_items, off, W, window, p->ids, p->dense);
-        k_item_class<<<grid(n_items), 256, 0, st>>>(by_window, n_items, cls);
+        k_fill_steps<<<grid((long long)n_items * 32), 256, 0, st>>>(f, wr, by_window, n_items, off, W, window, p->ids, p->dense, open);
+        k_item_class<<<grid(n_items), 256, 0, st>>>(by_window, n_items, open, cls);
         e = sort(sort_tmp);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
