@@ -38,6 +38,11 @@ def test_widths(F, chunk, monkeypatch):
     assert _err(r, torch.relu(ref)) <= MAX_ERR_F32
 
 
+@pytest.mark.parametrize("F", [104, 152, 168, 184, 208, 224, 232, 264, 320, 392])
+def test_slabs_that_rows_do_not_fill(F, monkeypatch):
+    test_widths(F, "8", monkeypatch)
+
+
 @pytest.mark.parametrize("F,offset", [(64, 4), (47, 1), (128, 2), (33, 0)])
 def test_no_room_for_a_padded_copy(F, offset):
     """B off a 16-byte boundary and a workspace that holds the partial sums only."""

@@ -1023,22 +1023,24 @@ static int launch_items(const KernelArgs& a, int slabs, bool few_items, bool ran
     return range ? launch_instance<FS, STAGES, 1, MINB, true, true, RAGGED>(a, slabs, st)
                  : launch_instance<FS, STAGES, 1, MINB, true, false, RAGGED>(a, slabs, st);
 }
-// Rows of an odd number of 16-byte chunks in one slab leave out the chunk that is not there: two lanes that ask for one
-// piece cost as much as two pieces (F = 24 / 40 / 56 / 120 on a clustered graph of 377920 rows 103 / 134 / 130 / 214 us, without
-// 78 / 105 / 114 / 199).  The test takes up to a tenth where every chunk is there (F = 64 97 against 110), and gives as
-// much as it takes with several slabs.
+// Rows that do not fill the slabs' 16-byte chunks leave out the chunks that are not there: two lanes that ask for one piece
+// cost as much as two pieces.  Clustered graph of 262144 rows, F = 136 / 168 / 200 / 232 / 264: 234 / 256 / 302 / 316 / 376
+// us with the last chunk repeated, 195 / 224 / 253 / 280 / 342 without; R-MAT 18 316 / 332 / 442 / 395 / 473 and 258 / 291 / 326 /
+// 355 / 441.  The test takes up to a tenth where every chunk is there (F = 64 97 against 110).
 template <int FS, int STAGES, int MINB, int MINB4>
 static int launch_sized(const KernelArgs& a, int slabs, bool few_items, bool range, cudaStream_t st) {
-    return slabs == 1 && a.bchunks < FS / 8 ? launch_items<FS, STAGES, MINB, MINB4, true>(a, slabs, few_items, range, st)
+    return a.bchunks < slabs * (FS / 8) ? launch_items<FS, STAGES, MINB, MINB4, true>(a, slabs, few_items, range, st)
                                             : launch_items<FS, STAGES, MINB, MINB4, false>(a, slabs, few_items, range, st);
 }
 
 static int launch_window_kernel(const KernelArgs& a, bool aligned, bool few_items, bool range, cudaStream_t st) {
     // As few slabs as 128 features allow (64-feature slabs for F = 128: 2678 against 2120 us at R-MAT scale 21),
-    // all of the same width rounded up to 16.  Stages and warps per SM fill the shared memory; measured at
-    // R-MAT scale 20, us: F = 32 with 4 / 6 / 8 stages 215 / 220 / 223 (scale 18, where the serial chain
-    // counts: 86 / 74 / 70), F = 64 with 3 / 4 / 5 stages 344 / 335 / 337 (137 / 110 / 93), F = 96 with 3 / 4 stages
-    // 494 / 467, F = 128 with 3 / 4 / 5 stages (16 / 12 / 10 warps) 577 / 627 / 650.
+    // all of the same width rounded up to 16.  There is no instance of 112: its seven pieces per lane lie in rows of
+    // their own, and F = 104 / 112 / 200 / 208 take 68 / 55 / 129 / 109 us there and 64 / 55 / 118 / 104 in the one of 128 without
+    // the missing chunks (uniform 131072; R-MAT 18 188 / 160 / 360 / 339 and 173 / 156 / 326 / 300).  Stages and warps per
+    // SM fill the shared memory; measured at R-MAT scale 20, us: F = 32 with 4 / 6 / 8 stages 215 / 220 / 223 (scale 18,
+    // where the serial chain counts: 86 / 74 / 70), F = 64 with 3 / 4 / 5 stages 344 / 335 / 337 (137 / 110 / 93), F = 96
+    // with 3 / 4 stages 494 / 467, F = 128 with 3 / 4 / 5 stages (16 / 12 / 10 warps) 577 / 627 / 650.
     const int slabs = ceil_div(a.F, 128);
     const int fs = ceil_div(ceil_div(a.F, slabs), 16);
     if (!aligned) return fs <= 4 ? launch_instance<64, 3, 1, 16, false, true, false>(a, ceil_div(a.F, 64), st)
@@ -1050,7 +1052,6 @@ static int launch_window_kernel(const KernelArgs& a, bool aligned, bool few_item
         case 4: return launch_sized<64, 4, 22, 5>(a, slabs, few_items, range, st);
         case 5: return launch_sized<80, 4, 18, 4>(a, slabs, few_items, range, st);
         case 6: return launch_sized<96, 4, 15, 4>(a, slabs, few_items, range, st);
-        case 7: return launch_sized<112, 3, 16, 4>(a, slabs, few_items, range, st);
         default: return launch_sized<128, 3, 16, 4>(a, slabs, few_items, range, st);
     }
 }
