@@ -25,6 +25,7 @@
 
 #include <string.h>
 
+#include <algorithm>
 #include <atomic>
 #include <type_traits>
 #include <mutex>
@@ -134,20 +135,39 @@ __global__ void k_count_steps(trs_format f, WindowRanges wr, int num_windows, in
 // done; below 32 steps the extra partial sums cost more than the shorter tail gives, above 512 nothing
 // is left to gain.  Measured best at R-MAT scale 14 / 16 / 17 / 18 / 19 / 20 / 21, F = 128: 32 / 48 / 96 / 192 / 256 / 384 / 512
 // steps; 256 for all of them took 57 / 66 / 118 / 148 / 277 / 589 / 2080 us against 21 / 43 / 74 / 143 / 277 / 554 / 2049.
-// A matrix with less than six steps per warp slot gives every item four warps instead (few_items).
+// With less than six steps per warp slot items get four warps each anyway (warps_per_item) and may be four times as long.
+// Windows of ordinary length are left whole, though: cutting nearly all of them in two doubles the time (uniform 24000, 32
+// entries per row, 33 steps per window, F = 32 / 128 / 512: 17 / 40 / 126 us in items of 17 steps, 10 / 20 / 58 whole).  A matrix
+// of few long windows needs the cuts to fill the GPU: below one window per four warp slots they stop at 128 steps.
 constexpr int kWarpsPerSm = 16, kFewSteps = 6;
-__host__ __device__ __forceinline__ int item_steps(int total_steps, int sms) {
+__host__ __device__ __forceinline__ int item_steps(int total_steps, int windows, int sms) {
     const int share = total_steps / (sms * kWarpsPerSm);
-    return share < kFewSteps ? 128 : min(max(share, 32), 512);
+    if (share < kFewSteps) return 128;
+    const int whole = min((int)(3ll * total_steps / (2 * windows)), 4 * windows < sms * kWarpsPerSm ? 128 : 512);
+    return min(max(max(share, 32), whole), 512);
 }
 
-__global__ void k_count_items(int num_windows, int chunk, int sms, const int* __restrict__ step_off, int* __restrict__ cnt) {
+// One warp per item or four.  A step of a lone warp takes about five times as long as the SM needs for one with its warps
+// all at work, a warp's start and end as long as twelve steps in the one sense and three in the other; an item of four
+// warps adds twenty (it ends with two barriers and a sum).  So, in steps of an SM, the time is the longer of its longest
+// item and of all its items.  R-MAT 13, F = 64 / 128 / 512, 1 -> 4 warps: 27 / 34 / 38 -> 14 / 18 / 31 us; uniform 8192, 32
+// entries per row, F = 128 / 256: 12.4 / 15.4 -> 11.2 / 18.5; uniform 32768, 4 entries per row, F = 64 / 256: 8.0 / 14.4 -> 11.0 / 28.7.
+static int warps_per_item(int items, long long steps, int longest, int slabs, int sms) {
+    const long long one = std::max(5ll * (longest + 12), slabs * (steps + 3ll * items) / sms);
+    const long long four = std::max(5ll * (longest / 4 + 12), slabs * (steps + 20ll * items) / sms);
+    return four < one ? 4 : 1;
+}
+
+__global__ void k_count_items(int num_windows, int chunk, int sms, const int* __restrict__ step_off, int* __restrict__ cnt,
+                              int* __restrict__ longest) {
     int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (chunk <= 0) chunk = item_steps(step_off[num_windows], num_windows, sms);
+    const int steps = w < num_windows ? step_off[w + 1] - step_off[w] : 0;
+    int items = w < num_windows ? max(1, (steps + chunk - 1) / chunk) : 0;
+    const int most = __reduce_max_sync(0xffffffffu, items > 0 ? (steps + items - 1) / items : 0);
+    if ((threadIdx.x & 31) == 0 && most > *longest) atomicMax(longest, most);
     if (w > num_windows) return;
     const size_t stride = (size_t)num_windows + 1;
-    if (chunk <= 0) chunk = item_steps(step_off[num_windows], sms);
-    int items = 0;
-    if (w < num_windows) items = max(1, (step_off[w + 1] - step_off[w] + chunk - 1) / chunk);
     cnt[WC_ITEMS * stride + w] = items;
     cnt[WC_HEAVY * stride + w] = items > 1 ? 1 : 0;
     cnt[WC_SLOTS * stride + w] = items > 1 ? items : 0;
@@ -749,7 +769,7 @@ struct trs_spmm_plan {
     int* ids = nullptr;      // [steps + kIdSpare][16] column ids of the step stream
     uint4* dense = nullptr;  // [dense steps][32] A tiles of the dense steps in fragment order
     int n_items, n_heavy, n_slots;
-    bool few_items;                   // four warps per item
+    int n_steps, longest, sms;        // of all items, of the longest one; SMs of the device
 };
 
 static int env_int(const char* name, int dflt) {
@@ -762,6 +782,7 @@ struct PlanInfo {
     int err;                      // V_* bits
     int c_entries, cs_entries;    // last prefix entries of the CSR parts
     int totals[kWindowCounts];
+    int longest;                  // steps of the longest item
 };
 
 __global__ void k_plan_lasts(trs_format f, PlanInfo* info) {
@@ -890,7 +911,7 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     k_count_steps<<<grid(W + 1), 256, 0, st>>>(f, wr, W, cnt);
     TRS_CUDA(scan(WC_STEPS));
     TRS_CUDA(scan(WC_DENSE));
-    k_count_items<<<grid(W + 1), 256, 0, st>>>(W, chunk, sms, off + WC_STEPS * stride, cnt);
+    k_count_items<<<grid(W + 1), 256, 0, st>>>(W, chunk, sms, off + WC_STEPS * stride, cnt, &d_info->longest);
     TRS_CUDA(scan(WC_ITEMS));
     TRS_CUDA(scan(WC_HEAVY));
     TRS_CUDA(scan(WC_SLOTS));
@@ -907,7 +928,7 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     p->f = f;
     p->m_rows = m_rows; p->k_cols = k_cols; p->window = window; p->num_windows = W; p->device = dev;
     p->n_items = n_items; p->n_heavy = n_heavy; p->n_slots = info.totals[WC_SLOTS];
-    p->few_items = n_steps / (sms * kWarpsPerSm) < kFewSteps;
+    p->n_steps = n_steps; p->longest = info.longest; p->sms = sms;
     const size_t ids_bytes = ((size_t)n_steps + kIdSpare) * 64, dense_bytes = (size_t)n_dense * 512;
     const size_t items_bytes = (size_t)n_items * sizeof(Item), heavy_bytes = (size_t)n_heavy * sizeof(Heavy);
     auto fail = [&](int code) { trs_spmm_plan_destroy(p); return code; };
@@ -1033,7 +1054,7 @@ static int launch_sized(const KernelArgs& a, int slabs, bool few_items, bool ran
                                             : launch_items<FS, STAGES, MINB, MINB4, false>(a, slabs, few_items, range, st);
 }
 
-static int launch_window_kernel(const KernelArgs& a, bool aligned, bool few_items, bool range, cudaStream_t st) {
+static int launch_window_kernel(const KernelArgs& a, bool aligned, const trs_spmm_plan* p, bool range, cudaStream_t st) {
     // As few slabs as 128 features allow (64-feature slabs for F = 128: 2678 against 2120 us at R-MAT scale 21),
     // all of the same width rounded up to 16.  There is no instance of 112: its seven pieces per lane lie in rows of
     // their own, and F = 104 / 112 / 200 / 208 take 68 / 55 / 129 / 109 us there and 64 / 55 / 118 / 104 in the one of 128 without
@@ -1045,6 +1066,8 @@ static int launch_window_kernel(const KernelArgs& a, bool aligned, bool few_item
     const int fs = ceil_div(ceil_div(a.F, slabs), 16);
     if (!aligned) return fs <= 4 ? launch_instance<64, 3, 1, 16, false, true, false>(a, ceil_div(a.F, 64), st)
                                  : launch_instance<128, 3, 1, 12, false, true, false>(a, ceil_div(a.F, 128), st);
+    // by the whole plan, so that the rows of a range of windows get the bits they get in a whole run
+    const bool few_items = warps_per_item(p->n_items, p->n_steps, p->longest, slabs, p->sms) == 4;
     switch (fs) {
         case 1: return launch_sized<16, 6, 32, 8>(a, slabs, few_items, range, st);
         case 2: return launch_sized<32, 6, 28, 7>(a, slabs, few_items, range, st);
@@ -1128,7 +1151,7 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
         aligned = true;
     }
     if (!aligned && n_peers > 0) return TRS_E_ARG;
-    const int rc = launch_window_kernel(a, aligned, p->few_items, w0 > 0 || w1 < p->num_windows, st);
+    const int rc = launch_window_kernel(a, aligned, p, w0 > 0 || w1 < p->num_windows, st);
     if (rc) return rc;
     if (p->n_heavy > 0) {
         PeerDst pd;
