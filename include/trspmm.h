@@ -109,8 +109,8 @@ int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, int k_cols, i
                          int validate, void* stream, trs_spmm_plan** out_plan);
 int trs_spmm_plan_destroy(trs_spmm_plan* plan);
 /* Scratch the run needs for feature width F: the partial sums of windows split across CTAs and, when
- * F % 8 != 0, room for a copy of B with padded rows.  (A workspace that holds the partial sums only,
- * trs_spmm_static_scratch_bytes, is accepted too: such widths are then gathered with 2-byte loads.) */
+ * F % 8 != 0, room for a copy of B with padded rows.  (A workspace of trs_spmm_static_scratch_bytes is
+ * accepted too: such widths are then gathered with 2-byte loads, and windows may be cut less finely.) */
 int trs_spmm_workspace_bytes(const trs_spmm_plan* plan, int F, size_t* bytes);
 /* C[m_rows, F] = A' * B[k_cols, F]; fp16 inputs, fp32 accumulate; C fully written (no memset
  * needed), fp32 or fp16 per out_dtype.  Asynchronous on `stream`; allocates nothing. */
@@ -157,7 +157,8 @@ int trs_spmm_status(const trs_spmm_plan* plan, int* status);
  * reference.  It runs the same kernels as trs_spmm_run, keeping the partial sums of split
  * windows in a fixed array inside the library (TRS_STATIC_SCRATCH_BYTES per GPU, held from
  * library load to process exit) and allocates nothing, on the host or the device.
- *   - returns TRS_E_LIMIT when the plan needs more scratch for this F than the array holds
+ *   - where the partial sums do not fit the array, windows are cut less finely, at 256 steps;
+ *     returns TRS_E_LIMIT when that needs more scratch for this F than the array holds too
  *     (trs_spmm_static_scratch_bytes tells the need); nothing is launched then;
  *   - the first call on each device looks up the array's device address; make that call before
  *     any stream capture starts on that device;

@@ -14,7 +14,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
-from trspmm import Format, SpmmPlan, TrsError, graphs
+from trspmm import Format, SpmmPlan, TrsError, build_format, graphs
 
 pytestmark = pytest.mark.gpu
 
@@ -57,3 +57,17 @@ def test_static_scratch_entry_refuses_oversized_plans(monkeypatch):
         plan.run_static(B, out)
     assert e.value.code == -10
     assert float(out.min()) == 3.0 and float(out.max()) == 3.0  # nothing was launched
+
+
+def test_static_entry_at_sizes_whose_windows_are_cut_finely():
+    """Matrices for which the ordinary entry cuts windows so finely that their partial sums exceed the fixed array."""
+    rp, col, val = graphs.rmat_graph(16, 16, seed=4, device="cuda")
+    n = rp.numel() - 1
+    plan = SpmmPlan(build_format(rp, col, val)[0], n, n)
+    for F in (128, 256):
+        assert plan.workspace_bytes(F) > 8 << 20 >= plan.static_scratch_bytes(F) > 0
+        B = torch.randn(n, F, generator=torch.Generator().manual_seed(F)).half().cuda()
+        want = plan.run(B, out_dtype=torch.float32)
+        got = plan.run_static(B, torch.full((n, F), float("nan"), device="cuda"))
+        assert O.scaled_max_error(got.cpu(), want.cpu()) <= MAX_ERR_F32
+        assert torch.equal(got, plan.run_static(B, torch.empty_like(got)))

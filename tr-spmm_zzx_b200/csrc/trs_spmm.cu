@@ -158,14 +158,35 @@ static int warps_per_item(int items, long long steps, int longest, int slabs, in
     return four < one ? 4 : 1;
 }
 
+// Where scratch for the partial sums is short (the fixed array of trs_spmm_run_static), windows are cut at 256 steps and no
+// earlier: a matrix below R-MAT scale 19 has several times the slots otherwise.
+constexpr int kCoarseSteps = 256;
+struct Cut {          // of all windows together
+    int items, heavy, slots;
+    int longest;      // steps of the longest item
+};
+__device__ __forceinline__ int cut_window(int steps, int chunk) { return max(1, (steps + chunk - 1) / chunk); }
+
 __global__ void k_count_items(int num_windows, int chunk, int sms, const int* __restrict__ step_off, int* __restrict__ cnt,
-                              int* __restrict__ longest) {
+                              int* __restrict__ longest, Cut* __restrict__ coarse) {
     int w = blockIdx.x * blockDim.x + threadIdx.x;
     if (chunk <= 0) chunk = item_steps(step_off[num_windows], num_windows, sms);
-    const int steps = w < num_windows ? step_off[w + 1] - step_off[w] : 0;
-    int items = w < num_windows ? max(1, (steps + chunk - 1) / chunk) : 0;
-    const int most = __reduce_max_sync(0xffffffffu, items > 0 ? (steps + items - 1) / items : 0);
-    if ((threadIdx.x & 31) == 0 && most > *longest) atomicMax(longest, most);
+    const bool live = w < num_windows;
+    const int steps = live ? step_off[w + 1] - step_off[w] : 0, lane = threadIdx.x & 31;
+    const int items = live ? cut_window(steps, chunk) : 0;
+    const int most = __reduce_max_sync(0xffffffffu, live ? (steps + items - 1) / items : 0);
+    if (lane == 0 && most > *longest) atomicMax(longest, most);
+    if (chunk < kCoarseSteps) {
+        const int n = live ? cut_window(steps, kCoarseSteps) : 0;
+        const int all = __reduce_add_sync(0xffffffffu, n), heavy = __popc(__ballot_sync(0xffffffffu, n > 1));
+        const int slots = __reduce_add_sync(0xffffffffu, n > 1 ? n : 0);
+        const int coarsest = __reduce_max_sync(0xffffffffu, live ? (steps + n - 1) / n : 0);
+        if (lane == 0) {
+            atomicAdd(&coarse->items, all);
+            if (heavy) { atomicAdd(&coarse->heavy, heavy); atomicAdd(&coarse->slots, slots); }
+            if (coarsest > coarse->longest) atomicMax(&coarse->longest, coarsest);
+        }
+    }
     if (w > num_windows) return;
     const size_t stride = (size_t)num_windows + 1;
     cnt[WC_ITEMS * stride + w] = items;
@@ -173,13 +194,10 @@ __global__ void k_count_items(int num_windows, int chunk, int sms, const int* __
     cnt[WC_SLOTS * stride + w] = items > 1 ? items : 0;
 }
 
-__global__ void k_fill_items(trs_format f, WindowRanges wr, int num_windows, const int* __restrict__ off,
-                             Item* __restrict__ items, Heavy* __restrict__ heavy) {
-    int w = blockIdx.x * blockDim.x + threadIdx.x;
-    if (w >= num_windows) return;
+// The items of window w: n of them from items[0], the slots from slot0 if there is more than one.
+__device__ __forceinline__ void fill_window(const trs_format& f, int w, int num_windows, const int* __restrict__ off, int n, int slot0,
+                                            int open, Item* __restrict__ items, Heavy* __restrict__ heavy) {
     const size_t stride = (size_t)num_windows + 1;
-    const int i0 = off[WC_ITEMS * stride + w], n = off[WC_ITEMS * stride + w + 1] - i0;
-    const int heavy0 = off[WC_HEAVY * stride + w], slot0 = off[WC_SLOTS * stride + w];
     const int step0 = off[WC_STEPS * stride + w], steps = off[WC_STEPS * stride + w + 1] - step0;
     const int dense0 = off[WC_DENSE * stride + w];
     const int tile0 = w < f.num_windows ? f.s_window_tile_offset[w] : 0;
@@ -188,10 +206,44 @@ __global__ void k_fill_items(trs_format f, WindowRanges wr, int num_windows, con
     const int per = (steps + n - 1) / n;
     for (int i = 0; i < n; ++i) {
         const int b = min(i * per, steps), e = min(b + per, steps);
-        items[i0 + i] = Item{w, n > 1 ? slot0 + i : -1, step0 + b, min(max(tiles - b, 0), e - b), e - b, tile0 + b,
-                             dense0 + max(b - tiles, 0), 0x7fffffff};
+        items[i] = Item{w, n > 1 ? slot0 + i : -1, step0 + b, min(max(tiles - b, 0), e - b), e - b, tile0 + b,
+                        dense0 + max(b - tiles, 0), open};
     }
-    if (n > 1) heavy[heavy0] = Heavy{w, slot0, slot0 + n};
+    if (n > 1) *heavy = Heavy{w, slot0, slot0 + n};
+}
+
+__global__ void k_fill_items(trs_format f, int num_windows, const int* __restrict__ off, Item* __restrict__ items,
+                             Heavy* __restrict__ heavy) {
+    int w = blockIdx.x * blockDim.x + threadIdx.x;
+    if (w >= num_windows) return;
+    const size_t stride = (size_t)num_windows + 1;
+    const int i0 = off[WC_ITEMS * stride + w];
+    fill_window(f, w, num_windows, off, off[WC_ITEMS * stride + w + 1] - i0, off[WC_SLOTS * stride + w], 0x7fffffff, items + i0,
+                heavy + off[WC_HEAVY * stride + w]);
+}
+
+// The coarse items, in no particular order (their windows' partial sums are still added in theirs).  `made`: cleared.
+__global__ void k_fill_coarse(trs_format f, int num_windows, const int* __restrict__ off, const int* __restrict__ open,
+                              Cut* __restrict__ made, Item* __restrict__ items, Heavy* __restrict__ heavy) {
+    const int w = blockIdx.x * blockDim.x + threadIdx.x, lane = threadIdx.x & 31;
+    const int* const step_off = off + WC_STEPS * ((size_t)num_windows + 1);
+    const int n = w < num_windows ? cut_window(step_off[w + 1] - step_off[w], kCoarseSteps) : 0, s = n > 1 ? n : 0;
+    int items_to = n, slots_to = s;   // up to this lane's
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, items_to, d), z = __shfl_up_sync(0xffffffffu, slots_to, d);
+        if (lane >= d) { items_to += y; slots_to += z; }
+    }
+    const unsigned split = __ballot_sync(0xffffffffu, n > 1);
+    int i0 = 0, slot0 = 0, h0 = 0;
+    if (lane == 31) {
+        i0 = atomicAdd(&made->items, items_to);
+        if (split) { slot0 = atomicAdd(&made->slots, slots_to); h0 = atomicAdd(&made->heavy, __popc(split)); }
+    }
+    i0 = __shfl_sync(0xffffffffu, i0, 31) + items_to - n;
+    slot0 = __shfl_sync(0xffffffffu, slot0, 31) + slots_to - s;
+    h0 = __shfl_sync(0xffffffffu, h0, 31) + __popc(split & ((1u << lane) - 1u));
+    if (n > 0) fill_window(f, w, num_windows, off, n, slot0, open[w], items + i0, heavy + h0);
 }
 
 // The step stream, one warp per item.  An unused column slot of a step repeats the step's first column, so that the gather
@@ -759,17 +811,22 @@ __global__ void __launch_bounds__(128) k_reduce_heavy(const Heavy* __restrict__ 
 // ----------------------------------------------------------------------------------------------
 using namespace trs;
 
+struct ItemSet {
+    Item* items = nullptr;   // long ones first
+    Heavy* heavy = nullptr;
+    int n_items = 0, n_heavy = 0, n_slots = 0;
+    int longest = 0;         // steps of the longest item
+};
+
 struct trs_spmm_plan {
     trs_format f;
     int m_rows, k_cols, window, num_windows;
     int device = 0;
     void* block = nullptr;   // the arrays below
-    Item* items = nullptr;   // long ones first
-    Heavy* heavy = nullptr;
+    ItemSet fine, coarse;    // the coarse one only where it needs fewer slots
     int* ids = nullptr;      // [steps + kIdSpare][16] column ids of the step stream
     uint4* dense = nullptr;  // [dense steps][32] A tiles of the dense steps in fragment order
-    int n_items, n_heavy, n_slots;
-    int n_steps, longest, sms;        // of all items, of the longest one; SMs of the device
+    int n_steps, sms;        // of all items; SMs of the device
 };
 
 static int env_int(const char* name, int dflt) {
@@ -783,6 +840,7 @@ struct PlanInfo {
     int c_entries, cs_entries;    // last prefix entries of the CSR parts
     int totals[kWindowCounts];
     int longest;                  // steps of the longest item
+    Cut coarse, made;
 };
 
 __global__ void k_plan_lasts(trs_format f, PlanInfo* info) {
@@ -911,7 +969,7 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     k_count_steps<<<grid(W + 1), 256, 0, st>>>(f, wr, W, cnt);
     TRS_CUDA(scan(WC_STEPS));
     TRS_CUDA(scan(WC_DENSE));
-    k_count_items<<<grid(W + 1), 256, 0, st>>>(W, chunk, sms, off + WC_STEPS * stride, cnt, &d_info->longest);
+    k_count_items<<<grid(W + 1), 256, 0, st>>>(W, chunk, sms, off + WC_STEPS * stride, cnt, &d_info->longest, &d_info->coarse);
     TRS_CUDA(scan(WC_ITEMS));
     TRS_CUDA(scan(WC_HEAVY));
     TRS_CUDA(scan(WC_SLOTS));
@@ -927,19 +985,25 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     trs_spmm_plan* p = new trs_spmm_plan();
     p->f = f;
     p->m_rows = m_rows; p->k_cols = k_cols; p->window = window; p->num_windows = W; p->device = dev;
-    p->n_items = n_items; p->n_heavy = n_heavy; p->n_slots = info.totals[WC_SLOTS];
-    p->n_steps = n_steps; p->longest = info.longest; p->sms = sms;
+    p->n_steps = n_steps; p->sms = sms;
+    ItemSet &fine = p->fine, &coarse = p->coarse;
+    fine.n_items = n_items; fine.n_heavy = n_heavy; fine.n_slots = info.totals[WC_SLOTS]; fine.longest = info.longest;
+    if (chunk == 0 && info.coarse.items > 0 && info.coarse.slots < fine.n_slots) {
+        coarse.n_items = info.coarse.items; coarse.n_heavy = info.coarse.heavy; coarse.n_slots = info.coarse.slots;
+        coarse.longest = info.coarse.longest;
+    }
     const size_t ids_bytes = ((size_t)n_steps + kIdSpare) * 64, dense_bytes = (size_t)n_dense * 512;
-    const size_t items_bytes = (size_t)n_items * sizeof(Item), heavy_bytes = (size_t)n_heavy * sizeof(Heavy);
+    const size_t items_bytes = ((size_t)n_items + coarse.n_items) * sizeof(Item);
+    const size_t heavy_bytes = ((size_t)n_heavy + coarse.n_heavy) * sizeof(Heavy);
     auto fail = [&](int code) { trs_spmm_plan_destroy(p); return code; };
     if ((rc = pool_alloc(&p->block, ids_bytes + dense_bytes + items_bytes + heavy_bytes, st))) return fail(rc);
     unsigned char* at = (unsigned char*)p->block;
     p->ids = (int*)at; at += ids_bytes;
     p->dense = (uint4*)at; at += dense_bytes;
-    p->items = (Item*)at; at += items_bytes;
-    p->heavy = (Heavy*)at;
+    fine.items = (Item*)at; coarse.items = fine.items + n_items; at += items_bytes;
+    fine.heavy = (Heavy*)at; coarse.heavy = fine.heavy + n_heavy;
 
-    Item* by_window;   // items in window order, sorted into p->items
+    Item* by_window;   // items in window order, sorted into fine.items
     int* open;
     unsigned char *cls, *sort_tmp;
     size_t sort_bytes = 0;
@@ -948,15 +1012,17 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     if (!rc) rc = ts.get((size_t)W, &open);
     if (rc) return fail(rc);
     auto sort = [&](void* t) {
-        return cub::DeviceRadixSort::SortPairs(t, sort_bytes, cls, cls + n_items, by_window, p->items, n_items, 0, kClassBits, st);
+        return cub::DeviceRadixSort::SortPairs(t, sort_bytes, cls, cls + n_items, by_window, fine.items, n_items, 0, kClassBits, st);
     };
     cudaError_t e = sort(nullptr);
     if (e == cudaSuccess && (rc = ts.get(sort_bytes + 16, &sort_tmp))) return fail(rc);
     if (e == cudaSuccess) e = cudaMemsetAsync(open, 0x7f, sizeof(int) * (size_t)W, st);
     if (e == cudaSuccess) {
-        k_fill_items<<<grid(W), 256, 0, st>>>(f, wr, W, off, by_window, p->heavy);
+        k_fill_items<<<grid(W), 256, 0, st>>>(f, W, off, by_window, fine.heavy);
         k_fill_steps<<<grid((long long)n_items * 32), 256, 0, st>>>(f, wr, by_window, n_items, off, W, window, p->ids, p->dense, open);
         k_item_class<<<grid(n_items), 256, 0, st>>>(by_window, n_items, open, cls);
+        if (coarse.n_items > 0)
+            k_fill_coarse<<<grid(W), 256, 0, st>>>(f, W, off, open, &d_info->made, coarse.items, coarse.heavy);
         e = sort(sort_tmp);
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -992,30 +1058,33 @@ extern "C" int trs_spmm_plan_destroy(trs_spmm_plan* p) {
 
 // Partial sums: 16 rows per slot, rows padded to whole 16-byte pieces.
 static int scratch_ld(int F) { return (F + 3) & ~3; }
-static size_t items_scratch_bytes(const trs_spmm_plan* p, int F) {
-    return (size_t)p->n_slots * 16 * (size_t)scratch_ld(F) * sizeof(float);
+static size_t set_scratch_bytes(const ItemSet& s, int F) { return (size_t)s.n_slots * 16 * (size_t)scratch_ld(F) * sizeof(float); }
+static size_t items_scratch_bytes(const trs_spmm_plan* p, int F) { return set_scratch_bytes(p->fine, F); }
+// The items a run with so much scratch takes: the fine ones, or the coarse ones where those need more than there is.
+static const ItemSet& items_for(const trs_spmm_plan* p, int F, size_t scratch_bytes) {
+    return p->coarse.n_items == 0 || items_scratch_bytes(p, F) <= scratch_bytes ? p->fine : p->coarse;
 }
 // Widths whose rows do not all start on 16-byte boundaries run on a copy of B with padded rows, kept in
 // the workspace behind the partial sums.
 static int padded_ld(int F) { return (F + 15) & ~15; }
-static size_t padded_at(const trs_spmm_plan* p, int F) { return (items_scratch_bytes(p, F) + 255) & ~(size_t)255; }
+static size_t padded_at(const ItemSet& s, int F) { return (set_scratch_bytes(s, F) + 255) & ~(size_t)255; }
 static size_t padded_bytes(const trs_spmm_plan* p, int F) { return (size_t)p->k_cols * padded_ld(F) * sizeof(__half); }
 
 extern "C" int trs_spmm_workspace_bytes(const trs_spmm_plan* p, int F, size_t* bytes) {
     if (!p || !bytes || F <= 0) return TRS_E_ARG;
-    *bytes = F % 8 == 0 ? items_scratch_bytes(p, F) : padded_at(p, F) + padded_bytes(p, F);
+    *bytes = F % 8 == 0 ? items_scratch_bytes(p, F) : padded_at(p->fine, F) + padded_bytes(p, F);
     return TRS_OK;
 }
 
 extern "C" int trs_spmm_static_scratch_bytes(const trs_spmm_plan* p, int F, size_t* bytes) {
     if (!p || !bytes || F <= 0) return TRS_E_ARG;
-    *bytes = items_scratch_bytes(p, F);
+    *bytes = set_scratch_bytes(items_for(p, F, TRS_STATIC_SCRATCH_BYTES), F);
     return TRS_OK;
 }
 
 extern "C" int trs_spmm_launches(const trs_spmm_plan* p) {
     if (!p) return 0;
-    return p->n_heavy > 0 ? 2 : 1;
+    return p->fine.n_heavy > 0 ? 2 : 1;
 }
 
 template <int FS, int STAGES, int WPI, int MINB, bool ALIGNED, bool RANGE, bool RAGGED>
@@ -1054,7 +1123,7 @@ static int launch_sized(const KernelArgs& a, int slabs, bool few_items, bool ran
                                             : launch_items<FS, STAGES, MINB, MINB4, false>(a, slabs, few_items, range, st);
 }
 
-static int launch_window_kernel(const KernelArgs& a, bool aligned, const trs_spmm_plan* p, bool range, cudaStream_t st) {
+static int launch_window_kernel(const KernelArgs& a, bool aligned, const trs_spmm_plan* p, const ItemSet& set, bool range, cudaStream_t st) {
     // As few slabs as 128 features allow (64-feature slabs for F = 128: 2678 against 2120 us at R-MAT scale 21),
     // all of the same width rounded up to 16.  There is no instance of 112: its seven pieces per lane lie in rows of
     // their own, and F = 104 / 112 / 200 / 208 take 68 / 55 / 129 / 109 us there and 64 / 55 / 118 / 104 in the one of 128 without
@@ -1067,7 +1136,7 @@ static int launch_window_kernel(const KernelArgs& a, bool aligned, const trs_spm
     if (!aligned) return fs <= 4 ? launch_instance<64, 3, 1, 16, false, true, false>(a, ceil_div(a.F, 64), st)
                                  : launch_instance<128, 3, 1, 12, false, true, false>(a, ceil_div(a.F, 128), st);
     // by the whole plan, so that the rows of a range of windows get the bits they get in a whole run
-    const bool few_items = warps_per_item(p->n_items, p->n_steps, p->longest, slabs, p->sms) == 4;
+    const bool few_items = warps_per_item(set.n_items, p->n_steps, set.longest, slabs, p->sms) == 4;
     switch (fs) {
         case 1: return launch_sized<16, 6, 32, 8>(a, slabs, few_items, range, st);
         case 2: return launch_sized<32, 6, 28, 7>(a, slabs, few_items, range, st);
@@ -1120,11 +1189,12 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
     if (w0 == w1) return TRS_OK;
     if (flags & ~TRS_EPILOGUE_RELU) return TRS_E_ARG;
     if (out_dtype != TRS_OUT_F32 && out_dtype != TRS_OUT_F16) return TRS_E_ARG;
-    const size_t need = items_scratch_bytes(p, F);
+    const ItemSet& set = items_for(p, F, workspace ? workspace_bytes : 0);
+    const size_t need = set_scratch_bytes(set, F);
     if (need > 0 && (!workspace || workspace_bytes < need)) return TRS_E_WORKSPACE;
     cudaStream_t st = (cudaStream_t)stream;
     KernelArgs a;
-    a.items = p->items; a.n_items = p->n_items;
+    a.items = set.items; a.n_items = set.n_items;
     a.w_begin = w0; a.w_end = w1;
     a.ids = p->ids; a.dense = p->dense;
     a.packed_a = p->f.s_packed_a; a.packed_meta = p->f.s_packed_meta;
@@ -1139,9 +1209,9 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
     // padded ones first when the workspace has room (trs_spmm_workspace_bytes asks for it when F % 8 != 0).
     bool aligned = F % 8 == 0 && ((uintptr_t)B & 15) == 0;
     if (((uintptr_t)workspace & 15) && need > 0) return TRS_E_WORKSPACE;
-    if (!aligned && n_peers == 0 && workspace && workspace_bytes >= padded_at(p, F) + padded_bytes(p, F) &&
+    if (!aligned && n_peers == 0 && workspace && workspace_bytes >= padded_at(set, F) + padded_bytes(p, F) &&
         ((uintptr_t)workspace & 15) == 0) {
-        __half* Bp = (__half*)((unsigned char*)workspace + padded_at(p, F));
+        __half* Bp = (__half*)((unsigned char*)workspace + padded_at(set, F));
         a.ldb = padded_ld(F);
         a.bchunks = a.ldb / 8;
         const long long pieces = (long long)p->k_cols * a.bchunks;
@@ -1151,14 +1221,14 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
         aligned = true;
     }
     if (!aligned && n_peers > 0) return TRS_E_ARG;
-    const int rc = launch_window_kernel(a, aligned, p, w0 > 0 || w1 < p->num_windows, st);
+    const int rc = launch_window_kernel(a, aligned, p, set, w0 > 0 || w1 < p->num_windows, st);
     if (rc) return rc;
-    if (p->n_heavy > 0) {
+    if (set.n_heavy > 0) {
         PeerDst pd;
         pd.n = a.n_peers; pd.row0 = a.peer_row0;
         for (int d = 0; d < 8; ++d) pd.ptr[d] = a.peers[d];
-        const dim3 rgrid(p->n_heavy, ceil_div(16 * a.ldS / 4, 128));
-        k_reduce_heavy<<<rgrid, 128, 0, st>>>(p->heavy, (const float*)workspace, C, F, a.ldS, p->m_rows, p->window,
+        const dim3 rgrid(set.n_heavy, ceil_div(16 * a.ldS / 4, 128));
+        k_reduce_heavy<<<rgrid, 128, 0, st>>>(set.heavy, (const float*)workspace, C, F, a.ldS, p->m_rows, p->window,
                                               a.out_half, a.relu, w0, w1, pd);
         TRS_LAUNCH_CHECK();
     }
@@ -1189,8 +1259,7 @@ std::mutex g_static_scratch_mutex;
 extern "C" int trs_spmm_run_static(const trs_spmm_plan* p, const trs_half* B, void* C, int F, int out_dtype,
                                    void* stream) {
     if (!p || !B || !C || F <= 0) return TRS_E_ARG;
-    const size_t need = items_scratch_bytes(p, F);
-    if (need > (size_t)TRS_STATIC_SCRATCH_BYTES) return TRS_E_LIMIT;
+    if (set_scratch_bytes(items_for(p, F, TRS_STATIC_SCRATCH_BYTES), F) > (size_t)TRS_STATIC_SCRATCH_BYTES) return TRS_E_LIMIT;
     int dev = -1;
     TRS_CUDA(cudaGetDevice(&dev));
     if (dev < 0 || dev >= kMaxDevices) return TRS_E_LIMIT;
