@@ -5,7 +5,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
-from trspmm import Format, SpmmPlan, _lib, graphs
+from trspmm import Format, SpmmPlan, _lib, build_format, graphs
 
 pytestmark = pytest.mark.gpu
 MAX_ERR_F32 = 2e-5
@@ -56,3 +56,29 @@ def test_no_room_for_a_padded_copy(F, offset):
     _lib.check(plan.lib.trs_spmm_run(plan._handle, B.data_ptr(), out.data_ptr(), F, 0, ws.data_ptr(), ws.numel(),
                                      _lib.current_stream_ptr(out.device)))
     assert _err(out, ref) <= MAX_ERR_F32
+
+
+@pytest.mark.parametrize("rows", [16, 1500, 16 * 1024, 16 * 1025 + 3, 16 * 5000])
+@pytest.mark.parametrize("F", [64, 47])
+def test_ranges_of_windows(rows, F):
+    """Ranges on both sides of the samples at which a plan knows where windows begin, with and without hub windows; every
+    one writes its own rows, with the bits of the whole run."""
+    for rp, col, val in (graphs.uniform_graph(rows, 5, seed=2, device="cuda"),
+                         graphs.coo_to_csr(torch.cat([torch.arange(rows), torch.zeros(9000, dtype=torch.long)]),
+                                           torch.cat([torch.arange(rows), torch.arange(9000)]), rows, max(rows, 9000))[:2] + (None,)):
+        rp, col = rp.cuda(), col.cuda()
+        val = torch.rand(col.numel(), device="cuda") if val is None else val
+        k = max(rows, 9000)
+        plan = SpmmPlan(build_format(rp, col, val)[0], rows, k)
+        W = plan.num_windows
+        B = torch.randn(k, F, generator=torch.Generator().manual_seed(F)).half().cuda()
+        want = plan.run(B, out_dtype=torch.float32)
+        out = torch.full_like(want, float("nan"))
+        cuts = sorted({0, 1, min(5, W), W // 2, W // 2 + 1 if W > 1 else W, W - 1, W} - {-1})
+        for w0, w1 in zip(cuts[:-1], cuts[1:]):
+            before = out.clone()
+            plan.run_windows(B, out, w0, w1)
+            mine = slice(16 * w0, min(16 * w1, rows))
+            before[mine] = want[mine]
+            assert torch.equal(torch.nan_to_num(out, nan=-7.0), torch.nan_to_num(before, nan=-7.0)), (w0, w1)
+        assert torch.equal(out, want)

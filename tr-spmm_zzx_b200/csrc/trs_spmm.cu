@@ -62,7 +62,7 @@ struct WindowRanges {
 };
 
 struct KernelArgs {
-    const Item* items;             // longest first
+    const Item* items;             // longest first, in window order for a range of windows
     int n_items;
     int w_begin, w_end;            // window range of this run (RANGE instances: items outside return at once)
     const int* ids;                // [steps + kIdSpare][16] column ids of the step stream
@@ -824,6 +824,10 @@ struct trs_spmm_plan {
     int device = 0;
     void* block = nullptr;   // the arrays below
     ItemSet fine, coarse;    // the coarse one only where it needs fewer slots
+    Item* by_window = nullptr;   // the fine items in window order, for runs of a range of windows
+    // first item, first split window and first step of every per_sample-th window
+    int per_sample = 1;
+    std::vector<int> item_at, heavy_at, step_at;
     int* ids = nullptr;      // [steps + kIdSpare][16] column ids of the step stream
     uint4* dense = nullptr;  // [dense steps][32] A tiles of the dense steps in fragment order
     int n_steps, sms;        // of all items; SMs of the device
@@ -847,9 +851,25 @@ __global__ void k_plan_lasts(trs_format f, PlanInfo* info) {
     if (f.parts_c > 0) info->c_entries = f.c_row_offset[f.parts_c];
     if (f.parts_c_short > 0) info->cs_entries = f.cs_row_offset[f.parts_c_short];
 }
-__global__ void k_plan_totals(const int* __restrict__ off, int num_windows, PlanInfo* info) {
+// Where every per_sample-th window begins, so that a run of a range of windows launches little more than its own items
+// (the windows in front of it and behind it up to a sample return at once); all of them would be a read-back of megabytes.
+constexpr int kSamples = 1024;
+struct PlanSamples {
+    int item[kSamples + 1], heavy[kSamples + 1], step[kSamples + 1];
+};
+struct PlanBack {
+    PlanInfo info;
+    PlanSamples at;
+};
+__global__ void k_plan_totals(const int* __restrict__ off, int num_windows, int per_sample, PlanBack* back) {
     const size_t stride = (size_t)num_windows + 1;
-    if (threadIdx.x < kWindowCounts) info->totals[threadIdx.x] = off[threadIdx.x * stride + num_windows];
+    if (threadIdx.x < kWindowCounts) back->info.totals[threadIdx.x] = off[threadIdx.x * stride + num_windows];
+    for (int i = threadIdx.x; i <= kSamples; i += blockDim.x) {
+        const long long w = min((long long)i * per_sample, (long long)num_windows);
+        back->at.item[i] = off[WC_ITEMS * stride + w];
+        back->at.heavy[i] = off[WC_HEAVY * stride + w];
+        back->at.step[i] = off[WC_STEPS * stride + w];
+    }
 }
 
 static int verdict(int err) {
@@ -860,7 +880,8 @@ static int verdict(int err) {
     return TRS_OK;
 }
 
-static int read_info(const PlanInfo* dev, PlanInfo* host, cudaStream_t st) {
+template <class T>
+static int read_info(const T* dev, T* host, cudaStream_t st) {
     TRS_CUDA(cudaMemcpyAsync(host, dev, sizeof(*host), cudaMemcpyDeviceToHost, st));
     TRS_CUDA(cudaStreamSynchronize(st));
     return TRS_OK;
@@ -933,9 +954,10 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     ts.st = st;
     const size_t stride = (size_t)W + 1;
     ts.chunk_bytes = ((size_t)6 + 2 * kWindowCounts) * stride * sizeof(int) + ((size_t)1 << 20);
-    PlanInfo* d_info;
+    PlanBack* d_back;
     int *ranges, *cnt, *off;
-    int rc = ts.get(1, &d_info);
+    int rc = ts.get(1, &d_back);
+    PlanInfo* const d_info = &d_back->info;
     if (!rc) rc = ts.get((size_t)6 * W, &ranges);
     if (!rc) rc = ts.get(kWindowCounts * stride, &cnt);
     if (!rc) rc = ts.get(kWindowCounts * stride, &off);
@@ -973,9 +995,11 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     TRS_CUDA(scan(WC_ITEMS));
     TRS_CUDA(scan(WC_HEAVY));
     TRS_CUDA(scan(WC_SLOTS));
-    k_plan_totals<<<1, 32, 0, st>>>(off, W, d_info);
-    PlanInfo info;
-    if ((rc = read_info(d_info, &info, st))) return rc;
+    const int per_sample = ceil_div(W, kSamples);
+    k_plan_totals<<<1, 256, 0, st>>>(off, W, per_sample, d_back);
+    PlanBack back;
+    if ((rc = read_info(d_back, &back, st))) return rc;
+    const PlanInfo& info = back.info;
     if ((rc = verdict(info.err))) return rc;
     const int n_items = info.totals[WC_ITEMS], n_heavy = info.totals[WC_HEAVY];
     const int n_steps = info.totals[WC_STEPS], n_dense = info.totals[WC_DENSE];
@@ -986,6 +1010,10 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     p->f = f;
     p->m_rows = m_rows; p->k_cols = k_cols; p->window = window; p->num_windows = W; p->device = dev;
     p->n_steps = n_steps; p->sms = sms;
+    p->per_sample = per_sample;
+    p->item_at.assign(back.at.item, back.at.item + kSamples + 1);
+    p->heavy_at.assign(back.at.heavy, back.at.heavy + kSamples + 1);
+    p->step_at.assign(back.at.step, back.at.step + kSamples + 1);
     ItemSet &fine = p->fine, &coarse = p->coarse;
     fine.n_items = n_items; fine.n_heavy = n_heavy; fine.n_slots = info.totals[WC_SLOTS]; fine.longest = info.longest;
     if (chunk == 0 && info.coarse.items > 0 && info.coarse.slots < fine.n_slots) {
@@ -993,22 +1021,21 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
         coarse.longest = info.coarse.longest;
     }
     const size_t ids_bytes = ((size_t)n_steps + kIdSpare) * 64, dense_bytes = (size_t)n_dense * 512;
-    const size_t items_bytes = ((size_t)n_items + coarse.n_items) * sizeof(Item);
+    const size_t items_bytes = ((size_t)2 * n_items + coarse.n_items) * sizeof(Item);
     const size_t heavy_bytes = ((size_t)n_heavy + coarse.n_heavy) * sizeof(Heavy);
     auto fail = [&](int code) { trs_spmm_plan_destroy(p); return code; };
     if ((rc = pool_alloc(&p->block, ids_bytes + dense_bytes + items_bytes + heavy_bytes, st))) return fail(rc);
     unsigned char* at = (unsigned char*)p->block;
     p->ids = (int*)at; at += ids_bytes;
     p->dense = (uint4*)at; at += dense_bytes;
-    fine.items = (Item*)at; coarse.items = fine.items + n_items; at += items_bytes;
+    p->by_window = (Item*)at; fine.items = p->by_window + n_items; coarse.items = fine.items + n_items; at += items_bytes;
     fine.heavy = (Heavy*)at; coarse.heavy = fine.heavy + n_heavy;
 
-    Item* by_window;   // items in window order, sorted into fine.items
+    Item* const by_window = p->by_window;
     int* open;
     unsigned char *cls, *sort_tmp;
     size_t sort_bytes = 0;
-    rc = ts.get(n_items, &by_window);
-    if (!rc) rc = ts.get((size_t)2 * n_items, &cls);
+    rc = ts.get((size_t)2 * n_items, &cls);
     if (!rc) rc = ts.get((size_t)W, &open);
     if (rc) return fail(rc);
     auto sort = [&](void* t) {
@@ -1195,6 +1222,17 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
     cudaStream_t st = (cudaStream_t)stream;
     KernelArgs a;
     a.items = set.items; a.n_items = set.n_items;
+    const Heavy* heavy = set.heavy;
+    int n_heavy = set.n_heavy;
+    const bool whole = w0 == 0 && w1 == p->num_windows;
+    if (!whole && &set == &p->fine) {
+        const int s0 = w0 / p->per_sample, s1 = ceil_div(w1, p->per_sample);
+        heavy += p->heavy_at[s0]; n_heavy = p->heavy_at[s1] - p->heavy_at[s0];
+        // a third of a matrix with hub windows still gains more from long items first than it loses by the items of others
+        // (halves of R-MAT 20, F = 128: 378 us, in window order 490; eighths 230 either way)
+        const int n = p->item_at[s1] - p->item_at[s0];
+        if (set.n_heavy == 0 || n < set.n_items / 3) { a.items = p->by_window + p->item_at[s0]; a.n_items = n; }
+    }
     a.w_begin = w0; a.w_end = w1;
     a.ids = p->ids; a.dense = p->dense;
     a.packed_a = p->f.s_packed_a; a.packed_meta = p->f.s_packed_meta;
@@ -1221,14 +1259,14 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
         aligned = true;
     }
     if (!aligned && n_peers > 0) return TRS_E_ARG;
-    const int rc = launch_window_kernel(a, aligned, p, set, w0 > 0 || w1 < p->num_windows, st);
+    const int rc = launch_window_kernel(a, aligned, p, set, !whole, st);
     if (rc) return rc;
-    if (set.n_heavy > 0) {
+    if (n_heavy > 0) {
         PeerDst pd;
         pd.n = a.n_peers; pd.row0 = a.peer_row0;
         for (int d = 0; d < 8; ++d) pd.ptr[d] = a.peers[d];
-        const dim3 rgrid(set.n_heavy, ceil_div(16 * a.ldS / 4, 128));
-        k_reduce_heavy<<<rgrid, 128, 0, st>>>(set.heavy, (const float*)workspace, C, F, a.ldS, p->m_rows, p->window,
+        const dim3 rgrid(n_heavy, ceil_div(16 * a.ldS / 4, 128));
+        k_reduce_heavy<<<rgrid, 128, 0, st>>>(heavy, (const float*)workspace, C, F, a.ldS, p->m_rows, p->window,
                                               a.out_half, a.relu, w0, w1, pd);
         TRS_LAUNCH_CHECK();
     }
