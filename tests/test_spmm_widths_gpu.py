@@ -82,3 +82,15 @@ def test_ranges_of_windows(rows, F):
             before[mine] = want[mine]
             assert torch.equal(torch.nan_to_num(out, nan=-7.0), torch.nan_to_num(before, nan=-7.0)), (w0, w1)
         assert torch.equal(out, want)
+
+
+def test_packed_values_off_their_boundary():
+    """Packed tiles that begin 4 bytes behind an 8-byte boundary."""
+    arrays, n = _case()
+    fmt = Format(arrays).to("cuda")
+    B = torch.randn(n, 64, generator=torch.Generator().manual_seed(2)).half().cuda()
+    want = SpmmPlan(fmt, n, n).run(B, out_dtype=torch.float32)
+    moved = torch.empty(fmt.s_packed_a.numel() + 1, dtype=fmt.s_packed_a.dtype, device="cuda")[1:].view(fmt.s_packed_a.shape)
+    fmt.s_packed_a = moved.copy_(fmt.s_packed_a)
+    assert moved.data_ptr() % 8 == 4
+    assert torch.equal(SpmmPlan(fmt, n, n).run(B, out_dtype=torch.float32), want)

@@ -944,7 +944,6 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     if (f.parts_c_short > 0 && !(f.cs_row_offset && f.cs_row && f.cs_column && f.cs_value)) return TRS_E_ARG;
     if (f.num_windows > 0 && !f.s_window_tile_offset) return TRS_E_ARG;
     if (f.tiles > 0 && !(f.s_tile_column && f.s_packed_a && f.s_packed_meta)) return TRS_E_ARG;
-    if ((uintptr_t)f.s_packed_a & 7) return TRS_E_ARG;      // read 8 bytes per lane
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return TRS_E_NO_DEVICE;
 
@@ -1023,11 +1022,18 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     const size_t ids_bytes = ((size_t)n_steps + kIdSpare) * 64, dense_bytes = (size_t)n_dense * 512;
     const size_t items_bytes = ((size_t)2 * n_items + coarse.n_items) * sizeof(Item);
     const size_t heavy_bytes = ((size_t)n_heavy + coarse.n_heavy) * sizeof(Heavy);
+    // the kernels read the packed values 8 bytes per lane; an array that does not allow that is copied
+    const size_t packed_bytes = ((uintptr_t)f.s_packed_a & 7) != 0 ? (size_t)f.tiles * 256 : 0;
     auto fail = [&](int code) { trs_spmm_plan_destroy(p); return code; };
-    if ((rc = pool_alloc(&p->block, ids_bytes + dense_bytes + items_bytes + heavy_bytes, st))) return fail(rc);
+    if ((rc = pool_alloc(&p->block, ids_bytes + dense_bytes + packed_bytes + items_bytes + heavy_bytes, st))) return fail(rc);
     unsigned char* at = (unsigned char*)p->block;
     p->ids = (int*)at; at += ids_bytes;
     p->dense = (uint4*)at; at += dense_bytes;
+    if (packed_bytes) {
+        const cudaError_t copied = cudaMemcpyAsync(at, f.s_packed_a, packed_bytes, cudaMemcpyDeviceToDevice, st);
+        if (copied != cudaSuccess) return fail((int)copied);
+        p->f.s_packed_a = (const uint32_t*)at; at += packed_bytes;
+    }
     p->by_window = (Item*)at; fine.items = p->by_window + n_items; coarse.items = fine.items + n_items; at += items_bytes;
     fine.heavy = (Heavy*)at; coarse.heavy = fine.heavy + n_heavy;
 
