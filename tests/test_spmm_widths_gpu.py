@@ -94,3 +94,34 @@ def test_packed_values_off_their_boundary():
     fmt.s_packed_a = moved.copy_(fmt.s_packed_a)
     assert moved.data_ptr() % 8 == 4
     assert torch.equal(SpmmPlan(fmt, n, n).run(B, out_dtype=torch.float32), want)
+
+
+def test_one_plan_on_two_streams():
+    """Widths whose rows are copied, no split windows: calls on several streams share nothing that is written."""
+    rp, col, val = graphs.uniform_graph(1 << 17, 8, seed=1, device="cuda")
+    n = rp.numel() - 1
+    plan = SpmmPlan(build_format(rp, col, val)[0], n, n)
+    assert plan.launches == 1
+    for F in (47, 31):
+        B = [torch.randn(n, F, generator=torch.Generator().manual_seed(i)).half().cuda() for i in range(3)]
+        want = [plan.run(b) for b in B]
+        streams = [torch.cuda.Stream() for _ in B]
+        torch.cuda.synchronize()
+        got = [[] for _ in B]
+        for _ in range(10):
+            for i, s in enumerate(streams):
+                with torch.cuda.stream(s):
+                    got[i].append(plan.run(B[i]))
+        torch.cuda.synchronize()
+        for i in range(len(B)):
+            assert all(torch.equal(g, want[i]) for g in got[i])
+
+
+def test_copies_of_B_do_not_pile_up():
+    arrays, n = _case()
+    plan = SpmmPlan(Format(arrays).to("cuda"), n, n)
+    B = torch.randn(n, 63, generator=torch.Generator().manual_seed(2)).half().cuda()
+    before = torch.cuda.memory_allocated()
+    for F in range(1, 63, 2):
+        plan.run(B[:, :F].contiguous())
+    assert torch.cuda.memory_allocated() == before

@@ -80,13 +80,18 @@ class SpmmPlan:
             raise ValueError("out must be a contiguous [m_rows, F] tensor on the plan's device")
         _out_code(out.dtype)
 
-    def _workspace(self, F: int):
-        """(address, bytes) of the scratch memory kept for feature width F."""
+    def _workspace(self, F: int, B: torch.Tensor):
+        """(address, bytes, owner) of scratch memory for feature width F.  Partial sums stay with the plan.  What holds a
+        copy of B belongs to one call: it is as large as B, and calls on other streams must not share it."""
         ws = self._ws.get(F)
         if ws is None:
-            t = torch.empty(max(self.workspace_bytes(F), 16), dtype=torch.uint8, device=self.device)
-            ws = self._ws[F] = (t.data_ptr(), t.numel(), t)
-        return ws[0], ws[1]
+            n = max(self.workspace_bytes(F), 16)
+            t = torch.empty(n, dtype=torch.uint8, device=self.device) if F % 8 == 0 else None
+            ws = self._ws[F] = (0 if t is None else t.data_ptr(), n, t)
+        if ws[2] is None:
+            t = B.new_empty((ws[1] + 1) // 2)
+            return t.data_ptr(), ws[1], t
+        return ws
 
     def _new_out(self, B: torch.Tensor, F: int, dtype) -> torch.Tensor:
         if dtype is torch.float16 and self.m_rows == self.k_cols:
@@ -102,7 +107,7 @@ class SpmmPlan:
         else:
             self._check_out(out, F)
             code = _out_code(out.dtype)
-        ws, ws_bytes = self._workspace(F)
+        ws, ws_bytes, _owner = self._workspace(F, B)
         _lib.launch(self._index, self.lib.trs_spmm_run_ex, self._handle, B.data_ptr(), out.data_ptr(), F, code,
                     1 if relu else 0, ws, ws_bytes)
         return out
@@ -117,7 +122,7 @@ class SpmmPlan:
         only those rows of `out` are written."""
         F = self._check_B(B)
         self._check_out(out, F)
-        ws, ws_bytes = self._workspace(F)
+        ws, ws_bytes, _owner = self._workspace(F, B)
         with torch.cuda.device(self.device):
             _lib.check(self.lib.trs_spmm_run_windows(self._handle, B.data_ptr(), out.data_ptr(), F, _out_code(out.dtype),
                                                      1 if relu else 0, ws, ws_bytes,
@@ -132,7 +137,7 @@ class SpmmPlan:
         F = self._check_B(B)
         if not 1 <= len(dst_ptrs) <= 8 or row0 < 0:
             raise ValueError("1 to 8 destination buffers and a non-negative row offset")
-        ws, ws_bytes = self._workspace(F)
+        ws, ws_bytes, _owner = self._workspace(F, B)
         arr = (C.c_void_p * len(dst_ptrs))(*[int(p) for p in dst_ptrs])
         _lib.launch(self._index, self.lib.trs_spmm_run_bcast, self._handle, B.data_ptr(), arr, len(dst_ptrs), int(row0), F,
                     1 if relu else 0, ws, ws_bytes)
