@@ -109,7 +109,7 @@ int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, int k_cols, i
                          int validate, void* stream, trs_spmm_plan** out_plan);
 int trs_spmm_plan_destroy(trs_spmm_plan* plan);
 /* Scratch the run needs for feature width F: the partial sums of windows split across CTAs and, when
- * F % 8 != 0, room for a copy of B with padded rows.  (A workspace of trs_spmm_static_scratch_bytes is
+ * F % 8 != 0 and the matrix is not nearly empty, room for a copy of B with padded rows.  (A workspace of trs_spmm_static_scratch_bytes is
  * accepted too: such widths are then gathered with 2-byte loads, and windows may be cut less finely.) */
 int trs_spmm_workspace_bytes(const trs_spmm_plan* plan, int F, size_t* bytes);
 /* C[m_rows, F] = A' * B[k_cols, F]; fp16 inputs, fp32 accumulate; C fully written (no memset

@@ -125,3 +125,23 @@ def test_copies_of_B_do_not_pile_up():
     for F in range(1, 63, 2):
         plan.run(B[:, :F].contiguous())
     assert torch.cuda.memory_allocated() == before
+
+
+@pytest.mark.parametrize("entries", [400, 6400, 64000])
+def test_nearly_empty_matrices(entries):
+    """Odd widths where a copy of B would cost more than the product, and ranges of windows on both sides of that."""
+    n, F = 1 << 16, 45
+    g = torch.Generator().manual_seed(entries)
+    rows = torch.cat([torch.randint(n, (entries // 2,), generator=g), torch.randint(n // 16, (entries // 2,), generator=g)])
+    rp, col = graphs.coo_to_csr(rows, torch.randint(n, (entries,), generator=g), n, n)[:2]
+    val = torch.rand(col.numel(), generator=g)
+    plan = SpmmPlan(build_format(rp.cuda(), col.cuda(), val.cuda(), strict=True)[0], n, n)
+    B = torch.randn(n, F, generator=g).half()
+    ref = O.spmm_csr(rp, col, val, B)
+    assert (plan.workspace_bytes(F) < n * F) == (entries < 64000)
+    out = plan.run(B.cuda(), out_dtype=torch.float32)
+    assert _err(out, ref) <= MAX_ERR_F32
+    parts = torch.empty_like(out)
+    for w0, w1 in ((0, 300), (300, 4000), (4000, n // 16)):
+        plan.run_windows(B.cuda(), parts, w0, w1)
+    assert torch.equal(parts, out)

@@ -418,7 +418,9 @@ int resident_enqueue_slabs(trs_resident* h, const trs_half* rhs_host, void* out_
         TRS_CUDA(cudaEventRecord(s.in_done, h->s_in));
         TRS_CUDA(cudaStreamWaitEvent(h->stream, s.in_done, 0));
         if (timed && i == 0) cudaEventRecord(h->t_ev[2], h->stream);
-        rc = trs_spmm_run(h->plan, in, out, d, out_dtype, h->d_ws, h->ws_bytes, h->stream);
+        SpmmHow how;
+        how.width = dimN;
+        rc = spmm_run(h->plan, in, out, d, out_dtype, h->d_ws, h->ws_bytes, h->stream, 0, h->num_windows, how);
         if (rc) return rc;
         TRS_CUDA(cudaEventRecord(s.chunk_done[0], h->stream));
         TRS_CUDA(cudaStreamWaitEvent(h->s_out, s.chunk_done[0], 0));
@@ -464,7 +466,9 @@ int resident_enqueue(trs_resident* h, const trs_half* rhs_host, void* out_host, 
         const int w0 = (int)((long long)h->num_windows * c / chunks);
         const int w1 = (int)((long long)h->num_windows * (c + 1) / chunks);
         if (w1 <= w0) continue;
-        rc = trs_spmm_run_windows(h->plan, s.d_rhs, s.d_out, dimN, out_dtype, 0, h->d_ws, h->ws_bytes, h->stream, w0, w1);
+        SpmmHow how;   // rows of B that need a copy get it once for all chunks
+        how.rows = c == 0 ? SpmmHow::FOR_ALL_RUNS : SpmmHow::COPIED;
+        rc = spmm_run(h->plan, s.d_rhs, s.d_out, dimN, out_dtype, h->d_ws, h->ws_bytes, h->stream, w0, w1, how);
         if (rc) return rc;
         TRS_CUDA(cudaEventRecord(s.chunk_done[c], h->stream));
         TRS_CUDA(cudaStreamWaitEvent(h->s_out, s.chunk_done[c], 0));

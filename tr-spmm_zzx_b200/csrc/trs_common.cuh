@@ -258,6 +258,16 @@ int copy_to_host(const HostSegment* seg, int n, cudaStream_t st);
 int copy_to_device(const HostSegment* seg, int n, cudaStream_t st);
 void release_host_ring();
 
+// trs_spmm.cu: trs_spmm_run_windows for callers that cut one product into several runs.
+struct SpmmHow {
+    int width = 0;   // the product's own width where `F` is a slab of it: what goes by the width goes by that
+    // Rows of B off 16-byte boundaries: copied to the workspace if the run pays for that, if all runs of the plan's windows
+    // together do, or already there from a run of the second kind.
+    enum Rows { FOR_THIS_RUN, FOR_ALL_RUNS, COPIED } rows = FOR_THIS_RUN;
+};
+int spmm_run(const trs_spmm_plan* p, const trs_half* B, void* C, int F, int out_dtype, void* workspace, size_t workspace_bytes,
+             cudaStream_t st, int w0, int w1, const SpmmHow& how);
+
 // trs_pack.cu
 int pack_tiles(const int* s_column, const float* s_value, const int8_t* s_pos, const int* s_offset,
                const int* tile_window, const int* tile_group, long long tiles, int window, int* s_tile_column,

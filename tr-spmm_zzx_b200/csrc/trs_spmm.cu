@@ -1101,11 +1101,14 @@ static const ItemSet& items_for(const trs_spmm_plan* p, int F, size_t scratch_by
 // the workspace behind the partial sums.
 static int padded_ld(int F) { return (F + 15) & ~15; }
 static size_t padded_at(const ItemSet& s, int F) { return (set_scratch_bytes(s, F) + 255) & ~(size_t)255; }
+// The copy takes 0.04 - 0.08 ns per row of B, 2-byte gathers 0.4 - 1 ns more per step than aligned ones, so it pays from
+// a step per ten rows on (a matrix of 1 M rows with 10000 entries, F = 100: 190 us with the copy, 100 without).
+static bool copy_pays(const trs_spmm_plan* p, long long steps) { return 10 * steps >= p->k_cols; }
 static size_t padded_bytes(const trs_spmm_plan* p, int F) { return (size_t)p->k_cols * padded_ld(F) * sizeof(__half); }
 
 extern "C" int trs_spmm_workspace_bytes(const trs_spmm_plan* p, int F, size_t* bytes) {
     if (!p || !bytes || F <= 0) return TRS_E_ARG;
-    *bytes = F % 8 == 0 ? items_scratch_bytes(p, F) : padded_at(p->fine, F) + padded_bytes(p, F);
+    *bytes = F % 8 == 0 || !copy_pays(p, p->n_steps) ? items_scratch_bytes(p, F) : padded_at(p->fine, F) + padded_bytes(p, F);
     return TRS_OK;
 }
 
@@ -1156,7 +1159,7 @@ static int launch_sized(const KernelArgs& a, int slabs, bool few_items, bool ran
                                             : launch_items<FS, STAGES, MINB, MINB4, false>(a, slabs, few_items, range, st);
 }
 
-static int launch_window_kernel(const KernelArgs& a, bool aligned, const trs_spmm_plan* p, const ItemSet& set, bool range, cudaStream_t st) {
+static int launch_window_kernel(const KernelArgs& a, bool aligned, const trs_spmm_plan* p, const ItemSet& set, int width, bool range, cudaStream_t st) {
     // As few slabs as 128 features allow (64-feature slabs for F = 128: 2678 against 2120 us at R-MAT scale 21),
     // all of the same width rounded up to 16.  There is no instance of 112: its seven pieces per lane lie in rows of
     // their own, and F = 104 / 112 / 200 / 208 take 68 / 55 / 129 / 109 us there and 64 / 55 / 118 / 104 in the one of 128 without
@@ -1166,10 +1169,14 @@ static int launch_window_kernel(const KernelArgs& a, bool aligned, const trs_spm
     // with 3 / 4 stages 494 / 467, F = 128 with 3 / 4 / 5 stages (16 / 12 / 10 warps) 577 / 627 / 650.
     const int slabs = ceil_div(a.F, 128);
     const int fs = ceil_div(ceil_div(a.F, slabs), 16);
-    if (!aligned) return fs <= 4 ? launch_instance<64, 3, 1, 16, false, true, false>(a, ceil_div(a.F, 64), st)
-                                 : launch_instance<128, 3, 1, 12, false, true, false>(a, ceil_div(a.F, 128), st);
-    // by the whole plan, so that the rows of a range of windows get the bits they get in a whole run
-    const bool few_items = warps_per_item(set.n_items, p->n_steps, set.longest, slabs, p->sms) == 4;
+    // by the whole plan and the whole width, so that a range of windows or a slab gets the bits it gets in a whole run
+    const bool few_items = warps_per_item(set.n_items, p->n_steps, set.longest, ceil_div(width, 128), p->sms) == 4;
+    if (!aligned) {
+        if (few_items) return fs <= 4 ? launch_instance<64, 3, 4, 4, false, true, false>(a, ceil_div(a.F, 64), st)
+                                      : launch_instance<128, 3, 4, 3, false, true, false>(a, ceil_div(a.F, 128), st);
+        return fs <= 4 ? launch_instance<64, 3, 1, 16, false, true, false>(a, ceil_div(a.F, 64), st)
+                       : launch_instance<128, 3, 1, 12, false, true, false>(a, ceil_div(a.F, 128), st);
+    }
     switch (fs) {
         case 1: return launch_sized<16, 6, 32, 8>(a, slabs, few_items, range, st);
         case 2: return launch_sized<32, 6, 28, 7>(a, slabs, few_items, range, st);
@@ -1188,7 +1195,7 @@ extern "C" int trs_spmm_run(const trs_spmm_plan* p, const trs_half* B, void* C, 
 
 static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, int out_dtype, int flags, void* workspace,
                     size_t workspace_bytes, void* stream, void* const* peers = nullptr, int n_peers = 0,
-                    long long peer_row0 = 0, int w0 = 0, int w1 = -1);
+                    long long peer_row0 = 0, int w0 = 0, int w1 = -1, const SpmmHow& how = SpmmHow());
 
 extern "C" int trs_spmm_run_ex(const trs_spmm_plan* p, const trs_half* B, void* C, int F, int out_dtype, int flags,
                                void* workspace, size_t workspace_bytes, void* stream) {
@@ -1200,6 +1207,11 @@ extern "C" int trs_spmm_run_windows(const trs_spmm_plan* p, const trs_half* B, v
                                     int window_end) {
     if (window_end < 0) return TRS_E_ARG;
     return run_impl(p, B, C, F, out_dtype, flags, workspace, workspace_bytes, stream, nullptr, 0, 0, window_begin, window_end);
+}
+
+int trs::spmm_run(const trs_spmm_plan* p, const trs_half* B, void* C, int F, int out_dtype, void* workspace, size_t workspace_bytes,
+                  cudaStream_t st, int w0, int w1, const SpmmHow& how) {
+    return run_impl(p, B, C, F, out_dtype, 0, workspace, workspace_bytes, st, nullptr, 0, 0, w0, w1, how);
 }
 
 extern "C" int trs_spmm_num_windows(const trs_spmm_plan* p) { return p ? p->num_windows : TRS_E_ARG; }
@@ -1215,7 +1227,7 @@ extern "C" int trs_spmm_run_bcast(const trs_spmm_plan* p, const trs_half* B, voi
 
 static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, int out_dtype, int flags, void* workspace,
                     size_t workspace_bytes, void* stream, void* const* peers, int n_peers, long long peer_row0, int w0,
-                    int w1) {
+                    int w1, const SpmmHow& how) {
     if (!p || !B || !C || F <= 0) return TRS_E_ARG;
     if (w1 < 0) w1 = p->num_windows;
     if (w0 < 0 || w0 > w1 || w1 > p->num_windows) return TRS_E_ARG;
@@ -1231,8 +1243,8 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
     const Heavy* heavy = set.heavy;
     int n_heavy = set.n_heavy;
     const bool whole = w0 == 0 && w1 == p->num_windows;
+    const int s0 = w0 / p->per_sample, s1 = ceil_div(w1, p->per_sample);
     if (!whole && &set == &p->fine) {
-        const int s0 = w0 / p->per_sample, s1 = ceil_div(w1, p->per_sample);
         heavy += p->heavy_at[s0]; n_heavy = p->heavy_at[s1] - p->heavy_at[s0];
         // a third of a matrix with hub windows still gains more from long items first than it loses by the items of others
         // (halves of R-MAT 20, F = 128: 378 us, in window order 490; eighths 230 either way)
@@ -1250,22 +1262,23 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
     a.n_peers = n_peers; a.peer_row0 = peer_row0;
     for (int d = 0; d < 8; ++d) a.peers[d] = d < n_peers ? peers[d] : nullptr;
     // The kernel gathers B in 16-byte pieces.  Rows that do not start on 16-byte boundaries are copied to
-    // padded ones first when the workspace has room (trs_spmm_workspace_bytes asks for it when F % 8 != 0).
+    // padded ones first when that pays and the workspace has room (trs_spmm_workspace_bytes asks for it).
     bool aligned = F % 8 == 0 && ((uintptr_t)B & 15) == 0;
     if (((uintptr_t)workspace & 15) && need > 0) return TRS_E_WORKSPACE;
-    if (!aligned && n_peers == 0 && workspace && workspace_bytes >= padded_at(set, F) + padded_bytes(p, F) &&
+    const bool pays = copy_pays(p, how.rows == SpmmHow::FOR_THIS_RUN && !whole ? p->step_at[s1] - p->step_at[s0] : p->n_steps);
+    if (!aligned && pays && n_peers == 0 && workspace && workspace_bytes >= padded_at(set, F) + padded_bytes(p, F) &&
         ((uintptr_t)workspace & 15) == 0) {
         __half* Bp = (__half*)((unsigned char*)workspace + padded_at(set, F));
         a.ldb = padded_ld(F);
         a.bchunks = a.ldb / 8;
         const long long pieces = (long long)p->k_cols * a.bchunks;
-        k_pad_rows<<<(unsigned)ceil_div64(pieces, 256), 256, 0, st>>>(a.B, pieces, F, a.bchunks, Bp);
+        if (how.rows != SpmmHow::COPIED) k_pad_rows<<<(unsigned)ceil_div64(pieces, 256), 256, 0, st>>>(a.B, pieces, F, a.bchunks, Bp);
         TRS_LAUNCH_CHECK();
         a.B = Bp;
         aligned = true;
     }
     if (!aligned && n_peers > 0) return TRS_E_ARG;
-    const int rc = launch_window_kernel(a, aligned, p, set, !whole, st);
+    const int rc = launch_window_kernel(a, aligned, p, set, how.width > 0 ? how.width : F, !whole, st);
     if (rc) return rc;
     if (n_heavy > 0) {
         PeerDst pd;
