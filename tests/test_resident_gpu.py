@@ -40,3 +40,20 @@ def test_call_after_one_that_found_no_memory():
     for F in (47, 128, 47):
         op.forward(B[F], out[F])
         assert torch.equal(out[F], want[F])
+
+
+@pytest.mark.parametrize("pinned", [(True, True), (False, False), (True, False), (False, True)])
+@pytest.mark.parametrize("F", [128, 130, 160, 200, 256])
+def test_kinds_of_host_memory(F, pinned):
+    """Blocking calls of a size that goes in slabs, on page-locked and pageable operands, and on rows off 64-byte boundaries."""
+    fmt, n = _case(1 << 16)
+    op, plan = ResidentSpmm(fmt, n, n, max_dimN=256), SpmmPlan(fmt, n, n)
+    B = torch.randn(n, F, generator=torch.Generator().manual_seed(F)).half()
+    for dtype in (torch.float32, torch.float16):
+        want = plan.run(B.cuda(), out_dtype=dtype).cpu()
+        for offset in (0, 2):
+            rhs, out = torch.empty(n * F + offset, dtype=torch.float16), torch.empty(n * F + offset, dtype=dtype)
+            rhs, out = rhs.pin_memory() if pinned[0] else rhs, out.pin_memory() if pinned[1] else out
+            rhs, out = rhs[offset:].view(n, F).copy_(B), out[offset:].view(n, F)
+            op.forward(rhs, out)
+            assert torch.equal(out, want)

@@ -394,16 +394,27 @@ int resident_workspace(trs_resident* h, int dimN) {
 }
 
 // The blocking call in feature slabs: while the input copy of slab s + 1 runs, slab s is multiplied and copied
-// back - the only overlap of the two directions that one call has.  A slab's rows are cut out of the host
-// rows by 2-D copies: 128-byte pieces move at 51 GB/s (64-byte ones at 35 - 41, whole rows at 55), so
-// slabs have 64 features.  R-MAT 18, F = 128: 2.74 -> 2.1 ms.
-int resident_slabs(int dimN, size_t in_bytes) { return dimN >= 2 * kSlabDim && in_bytes >= ((size_t)8 << 20) ? dimN / kSlabDim : 1; }
+// back - the only overlap of the two directions that one call has.  A slab's rows are cut out of the host rows by 2-D
+// copies, which wants page-locked memory (pageable rows go through the driver piece by piece: R-MAT 18, F = 256, 27 -> 36 ms) and
+// pieces of whole 64 bytes: 128-byte pieces move at 51 GB/s (64-byte ones at 35 - 41, whole rows at 55), so slabs
+// have 64 features, and widths that are no multiple of 32 lose more than they gain (R-MAT 18, F = 128 / 160 / 192 / 256 in
+// fp32 3.74 / 4.66 / 5.55 / 7.38 -> 3.45 / 4.36 / 4.78 / 6.17 ms; F = 130 / 136 / 200 / 232 3.87 / 4.02 / 5.84 / 6.74 -> 4.51 /
+// 4.37 / 6.21 / 6.90).
+bool in_pieces(const void* host) {
+    cudaPointerAttributes a;
+    if (((uintptr_t)host & 63) != 0) return false;
+    if (cudaPointerGetAttributes(&a, host) != cudaSuccess) { cudaGetLastError(); return false; }
+    return a.type == cudaMemoryTypeHost;
+}
+int resident_slabs(int dimN, size_t in_bytes, const void* in, const void* out) {
+    const bool slabs = dimN >= 2 * kSlabDim && dimN % 32 == 0 && in_bytes >= ((size_t)8 << 20) && in_pieces(in) && in_pieces(out);
+    return slabs ? dimN / kSlabDim : 1;
+}
 
 int resident_enqueue_slabs(trs_resident* h, const trs_half* rhs_host, void* out_host, int dimN, int out_dtype, int slabs, bool timed) {
     ResidentSlot& s = h->slot[h->seq % kSlots];
     int rc = slot_init(h, (int)(h->seq % kSlots));
     const int last_dim = dimN - kSlabDim * (slabs - 1);
-    if (!rc) rc = resident_workspace(h, last_dim);
     if (rc) return rc;
     const size_t elt = out_dtype == TRS_OUT_F16 ? 2 : 4;
     TRS_CUDA(cudaStreamWaitEvent(h->s_in, s.k_done, 0));
@@ -553,7 +564,7 @@ extern "C" int trs_resident_forward(trs_resident* h, const trs_half* rhs_host, v
     int rc = resident_check_args(h, rhs_host, out_host, dimN, out_dtype);
     if (rc) return rc;
     if (timing) memset(timing, 0, sizeof(*timing));
-    const int slabs = resident_slabs(dimN, (size_t)h->k_cols * dimN * sizeof(trs_half));
+    const int slabs = resident_slabs(dimN, (size_t)h->k_cols * dimN * sizeof(trs_half), rhs_host, out_host);
     rc = slabs > 1 ? resident_enqueue_slabs(h, rhs_host, out_host, dimN, out_dtype, slabs, timing != nullptr)
                    : resident_enqueue(h, rhs_host, out_host, dimN, out_dtype, timing != nullptr);
     const int drc = resident_drain(h);
