@@ -338,11 +338,11 @@ int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_half* X, cons
               trs_half* out, int n_rows, int n_cols, int K, void* stream);
 /* Planned SDDMM for a pattern that is used many times (training epochs): the plan groups the
  * entries by (16-row window, column), so that each distinct Y row of a window is gathered once
- * and the dot products run on the tensor cores (mma m16n8k16, fp32 accumulate) for K = 32, 64,
- * 128 with 16-byte aligned X / Y; other shapes run the entry-parallel kernel of trs_sddmm.  The
+ * and the dot products run on the tensor cores (mma m16n8k16, fp32 accumulate) for K up to 256; wider
+ * ones, and windows of more than 2^23 entries, run the entry-parallel kernel of trs_sddmm.  The
  * pattern must be canonical CSR (columns ascending and unique inside a row) and stay valid and
- * unchanged while the plan lives (checked at creation: TRS_E_COLUMN for a column outside
- * [0, n_cols), TRS_E_NOT_CANONICAL otherwise).  Results equal trs_sddmm's up to fp32 summation order.
+ * unchanged while the plan lives (checked at creation: TRS_E_OFFSETS for decreasing row pointers,
+ * TRS_E_COLUMN for a column outside [0, n_cols), TRS_E_NOT_CANONICAL otherwise).  Results equal trs_sddmm's up to fp32 summation order.
  * No counterpart in the reference. */
 typedef struct trs_sddmm_plan trs_sddmm_plan;
 int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, int n_rows, int n_cols,

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
-from trspmm import SddmmPlan, graphs, sddmm
+from trspmm import SddmmPlan, TrsError, graphs, sddmm
 
 pytestmark = pytest.mark.gpu
 
@@ -35,3 +35,11 @@ def test_widths(kind, K):
     base = torch.empty(n * K + 8, dtype=torch.float16, device="cuda")   # X one element off its boundary
     Xo = base[1:1 + n * K].view(n, K).copy_(X)
     assert torch.equal(plan.run(Xo, Y), plan.run(X, Y)) and torch.equal(sddmm(rp, col, Xo, Y), sddmm(rp, col, X, Y))
+
+
+def test_plan_refuses_decreasing_row_pointers():
+    rp = torch.tensor([0, 40, 20] + [60] * 30, dtype=torch.int32)
+    col = torch.arange(60, dtype=torch.int32)
+    with pytest.raises(TrsError) as e:
+        SddmmPlan(rp.cuda(), col.cuda(), 64)
+    assert e.value.code == -3

@@ -184,6 +184,12 @@ __device__ __forceinline__ int row_of_entry(const int* __restrict__ rowptr, int 
     return lo;
 }
 
+// err |= 8 for a decreasing row pointer: the lists place entries by them.
+__global__ void ksp_rows(const int* __restrict__ rowptr, int n_rows, int* __restrict__ err) {
+    const int r = blockIdx.x * blockDim.x + threadIdx.x;
+    if (r < n_rows && rowptr[r + 1] < rowptr[r]) atomicOr(err, 8);
+}
+
 // Also validates the pattern: err |= 1 for a column outside [0, n_cols), |= 2 for columns that are
 // not strictly ascending inside a row (the plan's entry addressing relies on canonical CSR).
 __global__ void ksp_keys(const int* __restrict__ rowptr, const int* __restrict__ col, int n_rows, int n_cols,
@@ -519,12 +525,14 @@ extern "C" int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, 
     if (rc) return fail(rc);
     auto grid = [](long long n) { return (unsigned)((n + 255) / 256); };
     cudaMemsetAsync(d_err, 0, 2 * sizeof(int), st);
+    ksp_rows<<<grid(n_rows), 256, 0, st>>>(rowptr, n_rows, d_err);
     ksp_keys<<<grid(nnz), 256, 0, st>>>(rowptr, col, n_rows, n_cols, nnz, key_a, ent_a, d_err);
     {
         int herr = 0;
         cudaError_t ee = cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
         if (ee == cudaSuccess) ee = cudaStreamSynchronize(st);
         if (ee != cudaSuccess) return fail((int)ee);
+        if (herr & 8) return fail(TRS_E_OFFSETS);
         if (herr & 1) return fail(TRS_E_COLUMN);
         if (herr & 2) return fail(TRS_E_NOT_CANONICAL);
     }
