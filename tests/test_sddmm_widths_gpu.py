@@ -43,3 +43,13 @@ def test_plan_refuses_decreasing_row_pointers():
     with pytest.raises(TrsError) as e:
         SddmmPlan(rp.cuda(), col.cuda(), 64)
     assert e.value.code == -3
+
+
+def test_results_are_vectors():
+    """Columns given as a matrix of one column, as COO files have them."""
+    rp, col = (t.cuda() for t in _pattern("rmat"))
+    X = torch.randn(1024, 32, generator=torch.Generator().manual_seed(1)).half().cuda()
+    for run in (lambda c: sddmm(rp, c, X, X), lambda c: SddmmPlan(rp, c, 1024).run(X, X),
+                lambda c: SddmmPlan(rp, c, 1024).run(X, X, out_dtype=torch.float32)):
+        assert run(col[:, None]).shape == (col.numel(),)
+        assert torch.equal(run(col[:, None]), run(col))

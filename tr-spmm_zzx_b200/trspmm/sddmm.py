@@ -9,6 +9,11 @@ import torch
 from . import _lib
 
 
+def _new_out(col: torch.Tensor, dtype: torch.dtype) -> torch.Tensor:
+    """One element per entry, a vector whatever the shape of `col` (empty_like takes half the time of an empty)."""
+    return torch.empty_like(col, dtype=dtype) if col.dim() == 1 else col.new_empty(col.numel(), dtype=dtype)
+
+
 def sddmm(rowptr: torch.Tensor, col: torch.Tensor, X: torch.Tensor, Y: torch.Tensor,
           out: torch.Tensor | None = None) -> torch.Tensor:
     lib = _lib.load()
@@ -22,7 +27,7 @@ def sddmm(rowptr: torch.Tensor, col: torch.Tensor, X: torch.Tensor, Y: torch.Ten
     if X.dim() != 2 or Y.dim() != 2 or X.shape[1] != Y.shape[1] or rowptr.numel() - 1 != X.shape[0]:
         raise ValueError("X must be [n_rows, K], Y [n_cols, K]")
     if out is None:
-        out = torch.empty_like(col, dtype=torch.float16)
+        out = _new_out(col, torch.float16)
     _lib.launch(index, lib.trs_sddmm, rowptr.data_ptr(), col.data_ptr(), X.data_ptr(), Y.data_ptr(), out.data_ptr(),
                 X.shape[0], Y.shape[0], X.shape[1])
     return out
@@ -63,7 +68,7 @@ class SddmmPlan:
         if out is None:
             if out_dtype is not torch.float16 and out_dtype is not torch.float32:
                 raise TypeError("output dtype must be torch.float32 or torch.float16")
-            out = torch.empty_like(self.col, dtype=out_dtype)
+            out = _new_out(self.col, out_dtype)
         elif out.dtype != torch.float16 or out.numel() != self.col.numel() or not out.is_contiguous():
             raise ValueError("out must be a contiguous fp16 vector with one element per entry")
         _lib.launch(self._index, self.lib.trs_sddmm_plan_run_ex, self._handle, X.data_ptr(), Y.data_ptr(), out.data_ptr(),
