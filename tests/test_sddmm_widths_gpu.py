@@ -53,3 +53,38 @@ def test_results_are_vectors():
                 lambda c: SddmmPlan(rp, c, 1024).run(X, X, out_dtype=torch.float32)):
         assert run(col[:, None]).shape == (col.numel(),)
         assert torch.equal(run(col[:, None]), run(col))
+
+
+@pytest.mark.parametrize("K", [32, 47, 64, 300])
+def test_under_capture(K):
+    """A plan's product can be captured at any width, with the copies that some of them make of X and Y."""
+    rp, col = (t.cuda() for t in _pattern("rmat"))
+    plan = SddmmPlan(rp, col, 1024)
+    g = torch.Generator().manual_seed(K)
+    X, Y = (torch.randn(1024, K, generator=g).half().cuda() for _ in range(2))
+    want = plan.run(X, Y)
+    out = torch.zeros_like(want)
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        plan.run(X, Y, out=out)
+    for scale in (1, 2, 4):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(out, want * scale)
+        X *= 2
+
+
+def test_as_many_entries_as_an_int_counts():
+    """2^31 - 1 entries: the last step of the entry-parallel kernel ends at the last one."""
+    n, K, nnz = 1 << 16, 8, 2 ** 31 - 1
+    if torch.cuda.mem_get_info()[0] < 20 << 30:
+        pytest.skip("needs 20 GB")
+    rp = torch.arange(n + 1, dtype=torch.int64) << 15
+    rp[-1] = nnz
+    col = torch.arange(nnz, dtype=torch.int32, device="cuda").bitwise_and_(1023)
+    g = torch.Generator().manual_seed(3)
+    X, Y = torch.randn(n, K, generator=g).half(), torch.randn(1024, K, generator=g).half()
+    out = sddmm(rp.to(torch.int32).cuda(), col, X.cuda(), Y.cuda())
+    at = torch.cat([torch.arange(nnz - 70, nnz), torch.arange(70), torch.randint(nnz, (1000,), generator=g)])
+    want = (X.float()[at >> 15] * Y.float()[at & 1023]).sum(1)
+    assert float((out[at.cuda()].float().cpu() - want).abs().max()) <= 2e-3 * float(want.abs().max())

@@ -80,12 +80,12 @@ __global__ void __launch_bounds__(32 * kEntryWarps, entry_ctas(KCH)) k_sddmm(con
         const int e_end = (int)min(first + per_warp, (long long)nnz);
         int row = warp_find(rowptr, n_rows, (int)first, lane);   // row of the chunk's first entry
         // columns and row ends of the next 32 entries are loaded while the present ones are multiplied
-        auto load_col = [&](int e0) { return col[min(e0 + lane, e_end - 1)]; };
+        auto load_col = [&](unsigned e0) { return col[min(e0 + lane, (unsigned)e_end - 1u)]; };
         auto load_bound = [&]() { return row + 1 + lane < n_rows ? rowptr[row + 1 + lane] : 0x7fffffff; };
-        int c_next = load_col((int)first), bound_next = load_bound();
-        for (int e0 = (int)first; e0 < e_end; e0 += 32) {
+        int c_next = load_col((unsigned)first), bound_next = load_bound();
+        for (unsigned e0 = (unsigned)first; e0 < (unsigned)e_end; e0 += 32) {   // unsigned: may step past 2^31 - 1
             // columns and rows of 32 entries, one per lane
-            const int e = min(e0 + lane, e_end - 1);
+            const int e = (int)min(e0 + lane, (unsigned)e_end - 1u);
             const int bound = bound_next;
             int c = c_next;
             const bool bad = (unsigned)c >= (unsigned)n_cols;
@@ -106,7 +106,7 @@ __global__ void __launch_bounds__(32 * kEntryWarps, entry_ctas(KCH)) k_sddmm(con
             }
             row = __shfl_sync(0xffffffffu, r, 31);
             const unsigned bad_mask = __ballot_sync(0xffffffffu, bad);
-            if (e0 + 32 < e_end) {
+            if (e0 + 32 < (unsigned)e_end) {
                 c_next = load_col(e0 + 32);
                 bound_next = load_bound();
             }
@@ -131,7 +131,7 @@ __global__ void __launch_bounds__(32 * kEntryWarps, entry_ctas(KCH)) k_sddmm(con
                     }
                 }
                 const int i = 8 * b + g;
-                if (t == (g >> 1) && e0 + i < e_end) {
+                if (t == (g >> 1) && e0 + i < (unsigned)e_end) {
                     const float v = (g & 1) ? d[1] : d[0];
                     store_result(out, out_f32, e0 + i, (bad_mask >> i) & 1u ? __ushort_as_half((unsigned short)0x7e00) : __float2half_rn(v));
                 }
