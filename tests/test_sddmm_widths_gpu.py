@@ -88,3 +88,50 @@ def test_as_many_entries_as_an_int_counts():
     at = torch.cat([torch.arange(nnz - 70, nnz), torch.arange(70), torch.randint(nnz, (1000,), generator=g)])
     want = (X.float()[at >> 15] * Y.float()[at & 1023]).sum(1)
     assert float((out[at.cuda()].float().cpu() - want).abs().max()) <= 2e-3 * float(want.abs().max())
+
+
+@pytest.mark.parametrize("K", [3, 47, 300])
+def test_no_memory_for_copies(K):
+    """Rows off 16-byte boundaries where the GPU has no room for padded copies of them."""
+    from trspmm import _lib
+    n = 1 << 21
+    rp, col = (t.cuda() for t in graphs.coo_to_csr(torch.arange(0, n, 5), torch.arange(0, n, 5).flip(0), n, n)[:2])
+    X, Y = (torch.randn(n, K, device="cuda", dtype=torch.float16) for _ in range(2))
+    plan = SddmmPlan(rp, col, n)
+    want = sddmm(rp, col, X, Y)
+    out = [torch.empty_like(want) for _ in range(2)]
+    torch.cuda.empty_cache()
+    _lib.check(_lib.load().trs_pool_trim())
+    hog = [torch.empty(torch.cuda.mem_get_info()[0] - (64 << 20), dtype=torch.uint8, device="cuda")]
+    while True:
+        try:
+            hog.append(torch.empty(4 << 20, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            break
+    try:
+        sddmm(rp, col, X, Y, out=out[0])
+        plan.run(X, Y, out=out[1])
+        torch.cuda.synchronize()
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    scale = float(want.abs().max())
+    for o in out:
+        assert float((o.float() - want.float()).abs().max()) <= 2e-3 * scale
+
+
+def test_windows_beyond_the_entry_lists():
+    """A window with more entries than the lists of a plan can place runs the entry-parallel kernel."""
+    n_cols, K = 600_000, 16
+    rp = torch.arange(33, dtype=torch.int32) * n_cols
+    rp[17:] = rp[16] + torch.arange(16, dtype=torch.int32)
+    col = torch.cat([torch.arange(n_cols, dtype=torch.int32).repeat(16), torch.arange(15, dtype=torch.int32)]).cuda()
+    rp = rp.cuda()
+    g = torch.Generator().manual_seed(7)
+    X, Y = torch.randn(32, K, generator=g).half().cuda(), torch.randn(n_cols, K, generator=g).half().cuda()
+    plan = SddmmPlan(rp, col, n_cols)
+    want = torch.cat([(X[:16].float() @ Y.float().T).flatten(), (X[17:].float() * Y[:15].float()).sum(1)])
+    for dtype in (torch.float16, torch.float32):
+        got = plan.run(X, Y, out_dtype=dtype).float()
+        assert float((got - want).abs().max()) <= 2e-3 * float(want.abs().max())
+    assert torch.equal(plan.run(X, Y), sddmm(rp, col, X, Y))

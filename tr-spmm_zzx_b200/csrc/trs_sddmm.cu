@@ -140,6 +140,25 @@ __global__ void __launch_bounds__(32 * kEntryWarps, entry_ctas(KCH)) k_sddmm(con
     }
 }
 
+// The same product on rows of any alignment, a warp per entry, where there is no memory for copies of X and Y.
+__global__ void __launch_bounds__(256) k_sddmm_plain(const int* __restrict__ rowptr, const int* __restrict__ col,
+                                                     const __half* __restrict__ X, const __half* __restrict__ Y,
+                                                     void* __restrict__ out, int out_f32, int n_rows, int n_cols, int K) {
+    const int lane = threadIdx.x & 31, nnz = rowptr[0] == 0 ? rowptr[n_rows] : 0;
+    const long long step = (long long)gridDim.x * 8;
+    for (long long e = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); e < nnz; e += step) {
+        const int row = warp_find(rowptr, n_rows, (int)e, lane);
+        const int c = col[e];
+        const bool bad = (unsigned)c >= (unsigned)n_cols;
+        const __half *x = X + (size_t)row * K, *y = Y + (size_t)(bad ? 0 : c) * K;
+        float s = 0.f;
+        for (int k = lane; k < K; k += 32) s = fmaf(__half2float(x[k]), __half2float(y[k]), s);
+#pragma unroll
+        for (int d = 16; d; d >>= 1) s += __shfl_xor_sync(0xffffffffu, s, d);
+        if (lane == 0) store_result(out, out_f32, e, bad ? __ushort_as_half((unsigned short)0x7e00) : __float2half_rn(s));
+    }
+}
+
 // Rows of `K` halfs copied to rows of `ld` halfs (a multiple of 8, zero-filled): one thread per 16 bytes.
 __global__ void k_sddmm_pad(const __half* __restrict__ src, long long pieces, int K, int per_row, __half* __restrict__ dst) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -601,7 +620,7 @@ namespace {
 using namespace trs;
 
 // X and Y as the kernels want them: rows on 16-byte boundaries, `ld` halfs apart.  Otherwise padded copies in
-// pool memory, given back to the pool behind the kernel.
+// pool memory, given back to the pool behind the kernel; ld = 0: there is no memory for them.
 struct Operands {
     const __half *X = nullptr, *Y = nullptr;
     int ld = 0;
@@ -614,6 +633,7 @@ struct Operands {
         ld = (K + 15) & ~15;   // whole 32-byte sectors
         const int per_row = ld / 8;
         const int rc = pool_alloc(&copy, ((size_t)n_rows + n_cols) * ld * sizeof(__half), st);
+        if (rc == (int)cudaErrorMemoryAllocation) { ld = 0; return TRS_OK; }
         if (rc) return rc;
         __half* xp = (__half*)copy;
         __half* yp = xp + (size_t)n_rows * ld;
@@ -640,6 +660,11 @@ int sm_count() {
 
 int launch_entries(const int32_t* rowptr, const int32_t* col, const Operands& o, void* out, int out_f32, int n_rows, int n_cols,
                    int K, cudaStream_t st) {
+    if (o.ld == 0) {
+        k_sddmm_plain<<<sm_count() * 8, 256, 0, st>>>(rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K);
+        TRS_LAUNCH_CHECK();
+        return TRS_OK;
+    }
     auto go = [&](auto kernel, int ctas) { kernel<<<sm_count() * ctas, 32 * kEntryWarps, 0, st>>>(rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K, o.ld); };
     if (K == 32) go(k_sddmm<1, true>, entry_ctas(1));
     else if (K < 32) go(k_sddmm<1, false>, entry_ctas(1));
@@ -725,7 +750,7 @@ extern "C" int trs_sddmm_plan_run_ex(const trs_sddmm_plan* p, const trs_half* X,
     Operands o;
     const int rc = o.prepare(X, Y, p->n_rows, p->n_cols, K, st);
     if (rc) return rc;
-    switch (p->wide ? 0 : (K + 31) / 32) {
+    switch (p->wide || o.ld == 0 ? 0 : (K + 31) / 32) {
         case 1: return launch_ring_k<1>(p, o, out, out_f32, K, st);
         case 2: return launch_ring_k<2>(p, o, out, out_f32, K, st);
         case 3: return launch_ring_k<3>(p, o, out, out_f32, K, st);
