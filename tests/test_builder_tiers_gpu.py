@@ -4,7 +4,7 @@ import pytest
 import torch
 
 from oracle import oracle as O
-from trspmm import TrsError, build_format
+from trspmm import TrsError, build_format, graphs
 
 pytestmark = pytest.mark.gpu
 
@@ -98,3 +98,34 @@ def test_entries_without_arrays_are_refused():
     with pytest.raises(TrsError) as e:
         build_format(torch.arange(17, dtype=torch.int32).cuda(), empty, empty.float())
     assert e.value.code == -1
+
+
+@pytest.mark.parametrize("error", [MemoryError, KeyboardInterrupt])
+@pytest.mark.parametrize("strict", [False, True])
+def test_array_that_cannot_be_had(error, strict, monkeypatch):
+    """Memory for the k-th array fails, while other streams are at work on the build or not: the caller's exception comes
+    out, and the next build is right."""
+    rp, col, val = (t.cuda() for t in graphs.rmat_graph(13, 16, seed=8))   # hub windows and all classes
+    want = build_format(rp, col, val, strict=strict)[0].arrays()
+    empty = torch.empty
+    for k in range(40):
+        calls = [0]
+
+        def failing(*a, **kw):
+            calls[0] += 1
+            if calls[0] == k + 1:
+                raise error("no room")
+            return empty(*a, **kw)
+
+        with monkeypatch.context() as m:
+            m.setattr(torch, "empty", failing)
+            try:
+                got = build_format(rp, col, val, strict=strict)[0].arrays()
+            except error:
+                got = None
+        if got is None:
+            got = build_format(rp, col, val, strict=strict)[0].arrays()
+        assert all(torch.equal(a, b) for a, b in zip(got, want)), k
+        if calls[0] <= k:
+            break
+    assert 10 < k < 40

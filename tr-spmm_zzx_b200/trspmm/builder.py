@@ -98,7 +98,7 @@ def build_format(rowptr: torch.Tensor, col: torch.Tensor, val: torch.Tensor, par
             dt = _ARRAY_DTYPES[i]
             t = arrays[i] = torch.empty(n_bytes // dt.itemsize, dtype=dt, device=dev)
             return t.data_ptr()
-        except Exception as e:                    # an exception cannot cross the C frames
+        except BaseException as e:                # nothing crosses the C frames, an interrupt least of all
             failed.append(e)
             return None
 
