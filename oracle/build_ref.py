@@ -14,7 +14,7 @@ with the system g++; no reference source is copied into this repository):
 The resulting modules are used (a) to pin the restatement in oracle/ against the
 real reference, (b) to generate the committed fixtures in tests/golden/ and
 (c) optionally as a timed CPU baseline.  When the reference tree is absent
-(e.g. on a GPU box) the script does nothing and reports that.
+the script does nothing and reports that.
 """
 from __future__ import annotations
 

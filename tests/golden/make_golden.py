@@ -1,7 +1,7 @@
 #!/usr/bin/env python3
 """Generate the committed fixtures from the reference's own compiled builder.
 
-Run in a container that has the reference tree (it cannot travel to a GPU box):
+Run where the reference tree is:
 
     python oracle/build_ref.py && python tests/golden/make_golden.py
 
