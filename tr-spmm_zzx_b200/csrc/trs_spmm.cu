@@ -637,11 +637,21 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
     // rows and A operand of step j, and with every eighth step the ids of the block after its own:
     // they land before the first step that reads them is gathered (AHEAD <= 8 steps earlier), in the
     // half of the id ring whose last reader was the step before j
+    // Outside the whole rounds, steps that have no open slots may be asked for instead of tested, a branch against two
+    // instructions per piece.  Seven graphs, against steps that are all taken as closed: F = 16 / 48 / 56 / 72 0.98 / 0.99 / 1.06 /
+    // 1.04 times tested, 0.97 / 0.93 / 1.00 / 0.97 asked for; F = 32 / 96 / 128 the other way round by 1 to 4 %.
+    constexpr bool kAsk = FS == 16 || FS == 48 || FS == 64 || FS == 80;
     uint4 areg[STAGES];
     auto fetch = [&](int j, auto stage) {
         if ((j & (kIdBlock - 1)) == 0) issue_ids(j / kIdBlock + 1);
-        areg[decltype(stage)::value] = load_a(j);
-        gather(j, stage, std::true_type());
+        if (kAsk && j < nclosed) {
+            const uint2 v = __ldg((const uint2*)(pa + (size_t)j * 64));
+            areg[decltype(stage)::value] = make_uint4(v.x, v.y, __ldg(pm + (size_t)j * 8), 0u);
+            gather(j, stage, std::false_type());
+        } else {
+            areg[decltype(stage)::value] = load_a(j);
+            gather(j, stage, std::true_type());
+        }
     };
 
     if (nsteps > 0) {
@@ -1166,7 +1176,7 @@ static int launch_window_kernel(const KernelArgs& a, bool aligned, const trs_spm
     // the missing chunks (uniform 131072; R-MAT 18 188 / 160 / 360 / 339 and 173 / 156 / 326 / 300).  Stages and warps per
     // SM fill the shared memory; measured at R-MAT scale 20, us: F = 32 with 4 / 6 / 8 stages 215 / 220 / 223 (scale 18,
     // where the serial chain counts: 86 / 74 / 70), F = 64 with 3 / 4 / 5 stages 344 / 335 / 337 (137 / 110 / 93), F = 96
-    // with 3 / 4 stages 494 / 467, F = 128 with 3 / 4 / 5 stages (16 / 12 / 10 warps) 577 / 627 / 650.
+    // with 3 / 4 stages 494 / 467, F = 80 with 18 / 16 warps (96 / 128 registers, the former spill) 3 % more / less, F = 128 with 3 / 4 / 5 stages (16 / 12 / 10 warps) 577 / 627 / 650.
     const int slabs = ceil_div(a.F, 128);
     const int fs = ceil_div(ceil_div(a.F, slabs), 16);
     // by the whole plan and the whole width, so that a range of windows or a slab gets the bits it gets in a whole run
@@ -1182,7 +1192,7 @@ static int launch_window_kernel(const KernelArgs& a, bool aligned, const trs_spm
         case 2: return launch_sized<32, 6, 28, 7>(a, slabs, few_items, range, st);
         case 3: return launch_sized<48, 4, 26, 6>(a, slabs, few_items, range, st);
         case 4: return launch_sized<64, 4, 22, 5>(a, slabs, few_items, range, st);
-        case 5: return launch_sized<80, 4, 18, 4>(a, slabs, few_items, range, st);
+        case 5: return launch_sized<80, 4, 16, 4>(a, slabs, few_items, range, st);
         case 6: return launch_sized<96, 4, 15, 4>(a, slabs, few_items, range, st);
         default: return launch_sized<128, 3, 16, 4>(a, slabs, few_items, range, st);
     }
