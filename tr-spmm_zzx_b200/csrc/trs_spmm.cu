@@ -1176,7 +1176,8 @@ static int launch_window_kernel(const KernelArgs& a, bool aligned, const trs_spm
     // the missing chunks (uniform 131072; R-MAT 18 188 / 160 / 360 / 339 and 173 / 156 / 326 / 300).  Stages and warps per
     // SM fill the shared memory; measured at R-MAT scale 20, us: F = 32 with 4 / 6 / 8 stages 215 / 220 / 223 (scale 18,
     // where the serial chain counts: 86 / 74 / 70), F = 64 with 3 / 4 / 5 stages 344 / 335 / 337 (137 / 110 / 93), F = 96
-    // with 3 / 4 stages 494 / 467, F = 80 with 18 / 16 warps (96 / 128 registers, the former spill) 3 % more / less, F = 128 with 3 / 4 / 5 stages (16 / 12 / 10 warps) 577 / 627 / 650.
+    // with 3 / 4 stages 494 / 467, F = 128 with 3 / 4 / 5 stages (16 / 12 / 10 warps) 577 / 627 / 650.  F = 80 with 18 warps
+    // (96 registers, some spilled) takes 3 % more than with 16.
     const int slabs = ceil_div(a.F, 128);
     const int fs = ceil_div(ceil_div(a.F, slabs), 16);
     // by the whole plan and the whole width, so that a range of windows or a slab gets the bits it gets in a whole run

@@ -195,6 +195,7 @@ def current_stream_ptr(device) -> int:
 
 
 _get_device, _raw_stream = getattr(torch._C, "_cuda_getDevice", None), getattr(torch._C, "_cuda_getCurrentRawStream", None)
+_capturing = getattr(torch._C, "_cuda_isCurrentStreamCapturing", torch.cuda.is_current_stream_capturing)
 
 
 def launch(index: int, entry, *args):
