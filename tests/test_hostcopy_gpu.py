@@ -41,6 +41,20 @@ def test_results_in_reused_blocks():
     _hostpool.release()
 
 
+def test_results_beyond_the_pool():
+    """More than the pool keeps, in one array and in several."""
+    from trspmm import _hostpool
+    dev = torch.device("cuda", 0)
+    _hostpool.release()
+    src = [torch.arange(n, dtype=torch.int32, device=dev) for n in (70 * MB + 3, 30 * MB, 30 * MB + 1, 20 * MB)]
+    for k in range(2):
+        got = _lib.copy_to_host([s + k for s in src], dev)
+        for a, b in zip(got, src):
+            assert torch.equal(a, (b + k).cpu())
+        assert sum(b.bytes for b in _hostpool._idle) <= _hostpool.KEEP_BYTES
+    _hostpool.release()
+
+
 def test_result_dropped_while_it_is_copied():
     """A caller queues a copy of a result behind work on a stream of its own and drops the result: the next results
     must not reach the copy."""
