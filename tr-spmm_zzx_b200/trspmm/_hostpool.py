@@ -29,6 +29,11 @@ _idle: list = []         # storages idle or still in use, oldest first
 class _Block:
     def __init__(self, n: int):
         self.bytes = n
+        # The C library serves arrays up to the largest one freed so far (32 MB at most) from its heap, which keeps their
+        # pages.  A result that is kept is never freed, so it is once in advance, as it would be by any program that drops
+        # it: otherwise the program's own arrays of such sizes fault their pages in every time (a format's copy to
+        # the CPU, 45 MB in 29 arrays: 38 against 8 ms).
+        torch.empty(n, dtype=torch.uint8, device="cpu")
         self.storage = torch.empty(n, dtype=torch.uint8, device="cpu").untyped_storage()
 
     def in_use(self) -> bool:
