@@ -129,3 +129,29 @@ def test_array_that_cannot_be_had(error, strict, monkeypatch):
         if calls[0] <= k:
             break
     assert 10 < k < 40
+
+
+@pytest.mark.parametrize("long_row", [0, 33, 0.6])
+@pytest.mark.parametrize("entries,bits", [(entries, bits) for cap, bits in ((256, 23), (512, 22), (1024, 21), (2048, 20))
+                                          for entries in (cap - 1, cap, cap + 1) for bits in (bits, bits + 1)])
+def test_warp_sort_borders(entries, bits, long_row):
+    """Windows on both sides of the classes that a warp sorts, with equal rows (each takes two lanes), with rows longer than
+    that, and columns up to the last one of the widest that fit into its keys and of the next power of two."""
+    g = torch.Generator().manual_seed(entries + bits)
+    per_row = torch.full((16,), entries // 16)
+    per_row[:entries % 16] += 1
+    more = int(long_row * entries) if long_row < 1 else long_row
+    for r in range(15):   # the last row takes from the others
+        take = min(int(per_row[r]) - 1, -(-more // 15))
+        per_row[r] -= take
+        per_row[15] += take
+    shared = torch.randint(0, 1 << bits, (entries // 2,), generator=g)
+    cols = []
+    for r in range(16):
+        few = torch.cat([shared[torch.randperm(shared.numel(), generator=g)][:int(per_row[r]) // 2],
+                         torch.randint(0, 1 << bits, (3 * int(per_row[r]) + 64,), generator=g)]).unique()
+        cols.append(few[torch.randperm(few.numel(), generator=g)][:int(per_row[r])].sort().values)
+    cols[15][-1] = (1 << bits) - 1
+    rowptr = torch.zeros(17, dtype=torch.int32)
+    rowptr[1:] = torch.cumsum(per_row, 0)
+    _check(rowptr, torch.cat(cols).to(torch.int32), torch.randn(entries, generator=g))

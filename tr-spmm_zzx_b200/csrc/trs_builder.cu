@@ -38,6 +38,7 @@
 #include <string.h>
 
 #include <algorithm>
+#include <atomic>
 #include <mutex>
 #include <vector>
 
@@ -58,17 +59,28 @@ struct BuildCfg {
 // ---------------------------------------------------------------------------------------------
 // 0. the sizes, the row pointers and the windows by size: one pass, one read-back
 // ---------------------------------------------------------------------------------------------
-// Size classes of windows by number of entries: sorted by one CTA in shared memory up to the last sort_cap, by
-// device-wide passes over all larger ones together beyond (hub windows).
-constexpr int kSortClasses = 4;
-__host__ __device__ constexpr int sort_cap(int c) { return c == 0 ? 256 : c == 1 ? 1024 : c == 2 ? 4096 : 8192; }
+// Classes of windows: up to 256 entries, and up to 512 and 1024 where no row has more than a sixteenth of that, sorted by
+// one warp in registers; up to 1024 otherwise and then up to 8192 by one CTA in shared memory; by device-wide passes over all
+// larger ones together beyond (hub windows).  A power-law graph's windows above 256 have one long row nearly always, and
+// sorted from scratch by a warp they take longer than a CTA merging their rows (builds of R-MAT 15 / 18 505 / 1163 against 493 /
+// 1140 us); windows of equal rows of 1025 to 2048 entries are as fast in a CTA (703 and 698 us).
+constexpr int kSortClasses = 7, kWarpClasses = 3;
+__host__ __device__ constexpr int sort_cap(int c) { return c < kWarpClasses ? 256 << c : 1024 << (c - kWarpClasses); }
+__device__ __forceinline__ int sort_class_of(long long n, int longest_row) {
+    if (n <= 0) return kSortClasses + 1;   // no class
+    if (n <= sort_cap(0)) return 0;
+    for (int c = 1; c < kWarpClasses; ++c)
+        if (n <= sort_cap(c) && longest_row <= sort_cap(c) / 16) return c;
+    for (int c = kWarpClasses; c < kSortClasses; ++c)
+        if (n <= sort_cap(c)) return c;
+    return kSortClasses;
+}
 
 struct InputInfo {
     int first, last;  // rowptr[0], rowptr[n_rows]
     int max_col;
     int err;          // 1: decreasing row pointer, 2: columns negative, not ascending or repeated
     int windows[kSortClasses + 1];   // windows per class, hubs last
-    int pad;
     u64 hub_entries;
 };
 
@@ -85,16 +97,20 @@ __global__ void kb_input_info(const int* __restrict__ rowptr, const int* __restr
     for (long long w0 = t0 - lane; w0 < W; w0 += step) {   // whole warps
         const long long w = w0 + lane;
         long long n = 0;
+        int longest_row = 0;
         if (w < W) {
-            n = (long long)rowptr[min((w + 1) * window, (long long)n_rows)] - rowptr[w * window];
+            const long long r1 = min((w + 1) * window, (long long)n_rows);
+            int from = rowptr[w * window];
+            n = (long long)rowptr[r1] - from;
             ncol[w] = 0;
+            if (n > sort_cap(0) && n <= sort_cap(kWarpClasses - 1))
+                for (long long r = w * window + 1; r <= r1; ++r) {
+                    const int to = rowptr[r];
+                    longest_row = max(longest_row, to - from);
+                    from = to;
+                }
         }
-        int c = kSortClasses + 1;   // empty: no class
-        if (n > 0) {
-            c = kSortClasses;
-            for (int i = kSortClasses - 1; i >= 0; --i)
-                if (n <= sort_cap(i)) c = i;
-        }
+        const int c = sort_class_of(n, longest_row);
         for (int i = 0; i <= kSortClasses; ++i) {
             const unsigned in = __ballot_sync(0xffffffffu, c == i);
             if (!in) continue;
@@ -134,7 +150,7 @@ struct WindowOut {
     int* ncol;
 };
 
-// One CTA per window of at most CAP entries, everything in shared memory; 12 bytes read and 4 + 17 per column written
+// Windows that do not go to kb_sort_warp: one CTA per window of at most CAP entries, everything in shared memory; 12 bytes read and 4 + 17 per column written
 // per entry.  The rows of a window are sorted already, so four rounds merge them two by two: a thread finds where its
 // outputs begin by binary search along the diagonal (merge path) and then takes them one by one.  A record's place in the
 // (count desc, column asc) order is counted, not sorted.
@@ -145,7 +161,7 @@ struct WindowOut {
 // takes 201 (windows of 780 entries), and 32 in place of 53 on windows of 510.
 template <int T, int CAP, class Key>
 struct WindowSort {
-    static constexpr int PB = CAP <= 256 ? 8 : CAP <= 1024 ? 10 : CAP <= 4096 ? 12 : 13;   // bits of a place in the window
+    static constexpr int PB = CAP <= 256 ? 8 : CAP <= 512 ? 9 : CAP <= 1024 ? 10 : CAP <= 2048 ? 11 : CAP <= 4096 ? 12 : 13;   // bits of a place in the window
     static_assert(CAP <= 1 << PB, "");
     struct Smem {
         Key key[2][CAP];           // column << PB | place in the window
@@ -331,6 +347,244 @@ __global__ void __launch_bounds__(T) kb_sort_window(const int* __restrict__ rowp
         out.cnt[o] = (unsigned char)(16 - k);
     }
     if (tid == 0) out.ncol[w] = D;
+}
+
+// One warp per window of at most 32 KPL entries, the keys in registers, KPL consecutive ones per lane: a bitonic merge whose
+// stages are two min / max per pair of keys (and a shuffle where the pair lies in two lanes), without an address, a bank or
+// a branch.  Every row takes two lanes, so that only the four rounds that merge rows are left; where a row has more than 2 KPL
+// entries, which the classes leave to KPL = 8, the keys are sorted from scratch.  The mask of a record is the difference of
+// two prefix sums over 1 << row: rows of one column are distinct.
+//
+// What bounds it: issue.  The merge of a CTA in shared memory (kb_sort_window) took 11900 warp instructions per window of the
+// clustered graph (780 entries) and 201 us at 89 % of the issue slots; this takes 5400 and 151 us at 60 % (its code does not stay in
+// the innermost instruction cache).  The loads of all keys go out at once: eight at a time took 202 us.
+template <int KPL>
+struct WarpSort {
+    static constexpr int CAP = 32 * KPL;
+    static constexpr int PB = KPL == 8 ? 8 : KPL == 16 ? 9 : 10;
+    static constexpr int LP = PB - 4;     // rows of 2 KPL places
+    static_assert(1 << PB == CAP, "");
+    struct __align__(16) Smem {   // the keys are read and written 16 bytes at a time
+        unsigned key[CAP];                // key i at at(i)
+        unsigned short before[CAP + 2];   // of the records: sum of 1 << row over the entries before, modulo 2^16
+        unsigned short start[CAP + 2];    // of the records
+        union {
+            unsigned char row[CAP];                // of an entry, where rows have no places of their own
+            unsigned short cells[16 * KPL];        // afterwards: records per count and chunk of 32
+        };
+        int bound[17];                    // first entry of every row, from the window's first
+    };
+    // The four keys that a lane reads or writes at a time lie where the eight lanes of a phase meet eight different bank groups,
+    // and 32 consecutive keys are still in 32 different banks.
+    __device__ static __forceinline__ int swizzle(int owner) { return KPL == 8 ? (owner >> 2) & 1 : KPL == 16 ? (owner >> 1) & 3 : owner & 7; }
+    __device__ static __forceinline__ int at(int i) { return i ^ (swizzle(i / KPL) << 2); }
+    static constexpr int CTAS = KPL <= 16 ? 9 : 6;   // of kSortWarps, by shared memory and registers
+};
+
+template <int N, int P, int K, int J = 0>
+__device__ __forceinline__ void odd_even_stage(unsigned (&v)[N]) {   // Batcher's odd-even merge: pairs K apart, runs of P
+#pragma unroll
+    for (int x = K % P; x + K < N; ++x)
+        if ((x - K % P) / K % 2 == 0 && x / (2 * P) == (x + K) / (2 * P)) {
+            const unsigned a = v[x], b = v[x + K];
+            v[x] = min(a, b);
+            v[x + K] = max(a, b);
+        }
+    if constexpr (K > 1) odd_even_stage<N, P, K / 2>(v);
+    else if constexpr (2 * P < N) odd_even_stage<N, 2 * P, 2 * P>(v);
+}
+
+constexpr int kSortWarps = 4;
+template <int KPL>
+__global__ void __launch_bounds__(32 * kSortWarps, WarpSort<KPL>::CTAS) kb_sort_warp(const int* __restrict__ rowptr, const int* __restrict__ col,
+                                                                const float* __restrict__ val, int n_rows, int window,
+                                                                const int* __restrict__ sel, int count, WindowOut out,
+                                                                InputInfo* __restrict__ info) {
+    using S = WarpSort<KPL>;
+    constexpr int PB = S::PB, LP = S::LP, CAP = S::CAP;
+    constexpr unsigned kPad = 0xffffffffu;   // columns have 31 - PB bits at most
+    extern __shared__ __align__(16) unsigned char smem_raw[];
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    typename S::Smem& s = reinterpret_cast<typename S::Smem*>(smem_raw)[wid];
+    const int which = blockIdx.x * kSortWarps + wid;
+    if (which >= count) return;
+    const int w = sel[which];
+    const int base = rowptr[(size_t)w * window];
+    if (lane < 17) s.bound[lane] = rowptr[min((long long)w * window + min(lane, window), (long long)n_rows)] - base;
+    __syncwarp();
+    const int n = s.bound[16];
+    const bool rows_fit = KPL > 8 || __reduce_max_sync(0xffffffffu, lane < 16 ? s.bound[lane + 1] - s.bound[lane] : 0) <= 2 * KPL;
+    unsigned v[KPL];
+    bool bad = false;
+    if (rows_fit) {
+#pragma unroll
+        for (int i = 0; i < KPL; ++i) {
+            const int place = i * 32 + lane, row = place >> LP, e = s.bound[row] + (place & (2 * KPL - 1));
+            const bool have = e < s.bound[row + 1];
+            const int c = have ? col[base + e] : 0;
+            bad |= c < 0;
+            v[i] = have ? (unsigned)c << PB | (unsigned)place : kPad;
+        }
+    } else {
+#pragma unroll 4
+        for (int i = 0; i < KPL; ++i) {
+            const int e = i * 32 + lane;
+            unsigned key = kPad;
+            if (e < n) {
+                const int c = col[base + e];
+                int row = 0;
+#pragma unroll
+                for (int d = 8; d; d >>= 1)
+                    if (row + d < window && s.bound[row + d] <= e) row += d;
+                s.row[e] = (unsigned char)row;
+                key = (unsigned)c << PB | (unsigned)e;
+                bad |= c < 0 || (e + 1 < s.bound[row + 1] && col[base + e + 1] <= c);
+            }
+            s.key[S::at(e)] = key;
+        }
+    }
+    if (rows_fit) {
+#pragma unroll
+        for (int i = 0; i < KPL; ++i) s.key[S::at(i * 32 + lane)] = v[i];
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < KPL; i += 4) {
+        const uint4 x = *(const uint4*)(s.key + S::at(lane * KPL + i));
+        v[i] = x.x; v[i + 1] = x.y; v[i + 2] = x.z; v[i + 3] = x.w;
+    }
+    if (rows_fit) {   // a row's columns ascend: pairs of neighbours, behind the row's end a pad
+#pragma unroll
+        for (int i = 0; i + 1 < KPL; ++i) bad |= v[i] != kPad && (v[i] >> PB) >= (v[i + 1] >> PB);
+        const unsigned across = __shfl_down_sync(0xffffffffu, v[0], 1);
+        bad |= (lane & 1) == 0 && v[KPL - 1] != kPad && (v[KPL - 1] >> PB) >= (across >> PB);
+    }
+    if (__any_sync(0xffffffffu, bad)) {   // nothing below holds for unsorted rows
+        if (lane == 0) atomicOr(&info->err, 2);
+        return;
+    }
+    auto inner = [&]() {   // the last stages of a merge, inside the lanes
+#pragma unroll
+        for (int d = KPL / 2; d; d >>= 1)
+#pragma unroll
+            for (int i = 0; i < KPL; ++i)
+                if (!(i & d)) {
+                    const unsigned a = v[i], b = v[i + d];
+                    v[i] = min(a, b);
+                    v[i + d] = max(a, b);
+                }
+    };
+    if (!rows_fit) odd_even_stage<KPL, 1, 1>(v);
+    // sorted runs of m lanes become runs of 2 m: the first stage pairs a run with the next one backwards, so that all stages ascend
+#pragma unroll 1
+    for (int m = rows_fit ? 2 : 1; m < 32; m <<= 1) {
+        const bool low = !(lane & m);
+#pragma unroll
+        for (int i = 0; i < KPL / 2; ++i) {
+            const unsigned a = v[i], b = v[KPL - 1 - i];
+            const unsigned x = __shfl_xor_sync(0xffffffffu, b, 2 * m - 1), y = __shfl_xor_sync(0xffffffffu, a, 2 * m - 1);
+            v[i] = (a < x) == low ? a : x;
+            v[KPL - 1 - i] = (b < y) == low ? b : y;
+        }
+#pragma unroll 1
+        for (int d = m >> 1; d; d >>= 1) {
+            const bool first = !(lane & d);
+#pragma unroll
+            for (int i = 0; i < KPL; ++i) {
+                const unsigned x = __shfl_xor_sync(0xffffffffu, v[i], d);
+                v[i] = (v[i] < x) == first ? v[i] : x;
+            }
+        }
+        inner();
+    }
+    __syncwarp();
+#pragma unroll
+    for (int i = 0; i < KPL; i += 4) *(uint4*)(s.key + S::at(lane * KPL + i)) = make_uint4(v[i], v[i + 1], v[i + 2], v[i + 3]);
+    // records begin where the column changes
+    const int mine = min(max(n - lane * KPL, 0), KPL);
+    unsigned rowbit_sum = 0;
+    int heads = 0;
+    const unsigned last = __shfl_up_sync(0xffffffffu, v[KPL - 1], 1);
+    auto is_head = [&](int i) -> bool {
+        if (i >= mine) return false;
+        if (i == 0) return lane == 0 || (v[0] >> PB) != (last >> PB);
+        return (v[i] ^ v[i - 1]) >> PB != 0u;
+    };
+    auto row_bit = [&](int i) -> unsigned { return 1u << (rows_fit ? (v[i] >> LP) & 15u : (unsigned)s.row[v[i] & (CAP - 1)]); };
+#pragma unroll
+    for (int i = 0; i < KPL; ++i) {
+        heads += is_head(i);
+        if (i < mine) rowbit_sum += row_bit(i);
+    }
+    int r = heads;
+    unsigned sum = rowbit_sum;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const int y = __shfl_up_sync(0xffffffffu, r, d);
+        const unsigned z = __shfl_up_sync(0xffffffffu, sum, d);
+        if (lane >= d) { r += y; sum += z; }
+    }
+    const int D = __shfl_sync(0xffffffffu, r, 31);
+    if (lane == 31) { s.start[D] = (unsigned short)n; s.before[D] = (unsigned short)sum; }
+    r -= heads;
+    sum -= rowbit_sum;
+#pragma unroll
+    for (int i = 0; i < KPL; ++i) {
+        if (is_head(i)) {
+            s.start[r] = (unsigned short)(lane * KPL + i);
+            s.before[r] = (unsigned short)sum;
+            ++r;
+        }
+        if (i < mine) sum += row_bit(i);
+    }
+    __syncwarp();
+    auto entry = [&](unsigned key) -> int {   // of the window
+        const int place = (int)(key & (CAP - 1));
+        return rows_fit ? s.bound[place >> LP] + (place & (2 * KPL - 1)) : place;
+    };
+#pragma unroll 1
+    for (int i0 = lane; i0 < n; i0 += 32 * 8) {
+        float x[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) x[i] = i0 + 32 * i < n ? val[base + entry(s.key[S::at(i0 + 32 * i)])] : 0.f;
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+            if (i0 + 32 * i < n) out.sval[base + i0 + 32 * i] = x[i];
+    }
+    // (count desc, column asc), as in kb_sort_window
+    const unsigned lt = (1u << lane) - 1u;
+    const int rchunks = (D + 31) / 32, ncells = 16 * rchunks;
+    for (int i = lane; i < ncells; i += 32) s.cells[i] = 0;
+    __syncwarp();
+    for (int c = 0; c < rchunks; ++c) {
+        const int q = c * 32 + lane, k = q < D ? 16 - (s.start[q + 1] - s.start[q]) : 16;
+        const unsigned same = __match_any_sync(0xffffffffu, k);
+        if (k < 16 && (same & lt) == 0) s.cells[k * rchunks + c] = (unsigned short)__popc(same);
+    }
+    __syncwarp();
+    int before = 0;
+    for (int c0 = 0; c0 < ncells; c0 += 32) {
+        const int i = c0 + lane, x = i < ncells ? s.cells[i] : 0;
+        int incl = x;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, incl, d);
+            if (lane >= d) incl += y;
+        }
+        if (i < ncells) s.cells[i] = (unsigned short)(before + incl - x);
+        before += __shfl_sync(0xffffffffu, incl, 31);
+    }
+    __syncwarp();
+    for (int c = 0; c < rchunks; ++c) {
+        const int q = c * 32 + lane, st = q < D ? s.start[q] : 0, k = q < D ? 16 - (s.start[q + 1] - st) : 16;
+        const unsigned same = __match_any_sync(0xffffffffu, k);
+        if (k == 16) continue;
+        const unsigned first = s.key[S::at(st)];
+        const size_t o = (size_t)base + s.cells[k * rchunks + c] + __popc(same & lt);
+        out.rec[o] = Record{(int)(first >> PB), base + st, (unsigned)(unsigned short)(s.before[q + 1] - s.before[q]), val[base + entry(first)]};
+        out.cnt[o] = (unsigned char)(16 - k);
+    }
+    if (lane == 0) out.ncol[w] = D;
 }
 
 // Hub windows: the same through device-wide sorts, keys (hub << col_bits | column), payload the place in the window.
@@ -1711,12 +1965,23 @@ struct Records {   // stages 1 - 3
     int* sel = nullptr;   // [kSortClasses + 1][W]
 };
 
+template <class Kernel>
+int allow_smem(Kernel kernel, int smem, std::atomic<unsigned long long>& done) {   // once per device and kernel
+    int dev = 0;
+    TRS_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (smem <= 48 * 1024 || (dev < 64 && (done.load(std::memory_order_relaxed) & bit))) return 0;
+    TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
+    return 0;
+}
 template <int T, class Key, int C>
 int sort_class_as(const InputInfo& info, const int* rowptr, const int* col, const float* val, const trs_builder* B, const Records& R,
                   InputInfo* d_info, cudaStream_t st) {
     constexpr int CAP = sort_cap(C), smem = (int)sizeof(typename WindowSort<T, CAP, Key>::Smem);
     auto kernel = kb_sort_window<T, CAP, Key>;
-    if (smem > 48 * 1024) TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    static std::atomic<unsigned long long> done{0};
+    TRS_TRY(allow_smem(kernel, smem, done));
     kernel<<<info.windows[C], T, smem, st>>>(rowptr, col, val, B->n_rows, B->cfg.window, R.sel + (size_t)C * B->W, R.w, d_info);
     TRS_LAUNCH_CHECK();
     return 0;
@@ -1725,6 +1990,19 @@ template <int T, int C>
 int sort_class(const InputInfo& info, const int* rowptr, const int* col, const float* val, const trs_builder* B, int col_bits,
                const Records& R, InputInfo* d_info, cudaStream_t st) {
     if (info.windows[C] == 0) return 0;
+    if constexpr (C < kWarpClasses) {
+        using S = WarpSort<sort_cap(C) / 32>;
+        if (col_bits + S::PB <= 31) {   // larger columns would need keys of 64 bits, which a warp has no registers for
+            constexpr int smem = (int)sizeof(typename S::Smem) * kSortWarps;
+            auto kernel = kb_sort_warp<sort_cap(C) / 32>;
+            static std::atomic<unsigned long long> done{0};
+            TRS_TRY(allow_smem(kernel, smem, done));
+            kernel<<<ceil_div(info.windows[C], kSortWarps), 32 * kSortWarps, smem, st>>>(rowptr, col, val, B->n_rows, B->cfg.window,
+                                                                                        R.sel + (size_t)C * B->W, info.windows[C], R.w, d_info);
+            TRS_LAUNCH_CHECK();
+            return 0;
+        }
+    }
     return col_bits + WindowSort<T, sort_cap(C), unsigned>::PB <= 32
                ? sort_class_as<T, unsigned, C>(info, rowptr, col, val, B, R, d_info, st)
                : sort_class_as<T, u64, C>(info, rowptr, col, val, B, R, d_info, st);
@@ -1805,8 +2083,11 @@ int make_records(trs_builder* B, const int* rowptr, const int* col, const float*
         for (cudaStream_t s : side) TRS_CUDA(cudaStreamWaitEvent(s, ready.e, 0));
     }
     auto classes = [&]() -> int {
-        TRS_TRY((sort_class<1024, 3>(info, rowptr, col, val, B, col_bits, *R, d_info, side[0])));
-        TRS_TRY((sort_class<512, 2>(info, rowptr, col, val, B, col_bits, *R, d_info, side[1])));
+        TRS_TRY((sort_class<1024, 6>(info, rowptr, col, val, B, col_bits, *R, d_info, side[0])));
+        TRS_TRY((sort_class<512, 5>(info, rowptr, col, val, B, col_bits, *R, d_info, side[1])));
+        TRS_TRY((sort_class<256, 4>(info, rowptr, col, val, B, col_bits, *R, d_info, side[1])));
+        TRS_TRY((sort_class<128, 3>(info, rowptr, col, val, B, col_bits, *R, d_info, side[0])));
+        TRS_TRY((sort_class<128, 2>(info, rowptr, col, val, B, col_bits, *R, d_info, side[1])));
         TRS_TRY((sort_class<128, 1>(info, rowptr, col, val, B, col_bits, *R, d_info, side[0])));
         return sort_class<64, 0>(info, rowptr, col, val, B, col_bits, *R, d_info, side[1]);
     };
@@ -1926,11 +2207,17 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     };
     // Without large windows the bounds are close enough to start before the sizes have come back (30 us of 870 on the
     // clustered graph).  With them the words of every warp would take the shared memory of many.
-    const bool ahead = info.windows[2] == 0 && info.windows[3] == 0 && info.windows[kSortClasses] == 0;
-    static_assert(sort_cap(1) / 2 <= kWarpUnits, "");
+    bool ahead = true;
+    int largest = 0;
+    for (int c = 0; c <= kSortClasses; ++c) {
+        if (info.windows[c] == 0) continue;
+        largest = c;
+        ahead &= c < kSortClasses - 2;
+    }
+    static_assert(sort_cap(kSortClasses - 3) / 2 <= kWarpUnits, "");
     if (ahead) {
         TRS_TRY(match_arrays((size_t)nnz / 2 + W, (size_t)nnz / 4 + W));
-        TRS_TRY(match_warps(sort_cap(info.windows[1] > 0 ? 1 : 0) / 2));
+        TRS_TRY(match_warps(sort_cap(largest) / 2));
         TRS_TRY(group_sizes());
     }
     TRS_TRY(sized.wait());
@@ -2204,7 +2491,7 @@ extern "C" int trs_build_query(int n_rows, long long nnz, const trs_build_config
     b += e * 72;                      // per-(window, column) records, their two sort buffers, TC / SPTC index maps
     b += (e / 2 + W) * 8 + (e / 4 + W) * 24;   // units, pairs, group column lists
     if (cfg->strict) b += e * 28 + (size_t)n_rows * 8;
-    b += W * 4 * 32;                  // per-window counters and prefixes
+    b += W * 4 * 34;                  // per-window counters and prefixes
     b += e / 2 + ((size_t)64 << 20);  // CUB temporary storage
     // outputs: SPTC groups (196 B each) and tiles (360 B each), TC blocks, CSR parts, fp16 value copies
     b += (e / 4 + W) * 196 + (e / 16 + 2 * W) * 360;
