@@ -135,3 +135,29 @@ def test_windows_beyond_the_entry_lists():
         got = plan.run(X, Y, out_dtype=dtype).float()
         assert float((got - want).abs().max()) <= 2e-3 * float(want.abs().max())
     assert torch.equal(plan.run(X, Y), sddmm(rp, col, X, Y))
+
+
+@pytest.mark.parametrize("K", [24, 64, 160, 256])
+@pytest.mark.parametrize("shape", ["hubs first", "hubs last", "even", "one window"])
+def test_shares_of_equal_cost(shape, K):
+    """Patterns whose quads cost the same (equal numbers per warp) and very different amounts (a table of first quads): every
+    entry is written once, whichever warp has it."""
+    g = torch.Generator().manual_seed(K)
+    n, m = (16, 60000) if shape == "one window" else (24000, 6000)
+    if shape == "one window":
+        rows, cols = torch.randint(0, n, (400000,), generator=g), torch.randint(0, m, (400000,), generator=g)
+    else:
+        rows, cols = torch.arange(n).repeat_interleave(9), torch.randint(0, m, (9 * n,), generator=g)
+        if shape != "even":
+            hub = torch.arange(300) + (n - 300 if shape == "hubs last" else 0)
+            rows = torch.cat([rows, hub.repeat_interleave(2500)])
+            cols = torch.cat([cols, torch.randint(0, m, (300 * 2500,), generator=g)])
+    rp, col = (t.cuda() for t in graphs.coo_to_csr(rows, cols, n, m)[:2])
+    X, Y = torch.randn(n, K, generator=g).half().cuda(), torch.randn(m, K, generator=g).half().cuda()
+    r = torch.repeat_interleave(torch.arange(n, device="cuda"), (rp[1:] - rp[:-1]).long())
+    out = SddmmPlan(rp, col, m).run(X, Y, out=torch.full((col.numel(),), float("nan"), dtype=torch.float16, device="cuda")).float()
+    ref = torch.empty_like(out)
+    for a in range(0, col.numel(), 1 << 18):
+        ref[a:a + (1 << 18)] = (X[r[a:a + (1 << 18)]].float() * Y[col[a:a + (1 << 18)].long()].float()).sum(1)
+    # fp16 results (2^-11) of fp32 sums, whose order differs by less than that
+    assert float((out - ref).abs().max()) <= 2e-3 * float(ref.abs().max())

@@ -269,11 +269,58 @@ __global__ void ksp_columns(const unsigned long long* __restrict__ key, const in
     if ((local & 31) == 0) begin[q] = (int)i;
 }
 
+// CTAs per SM, by shared memory and registers (K = 64 with 8 CTAs of 64 registers spills: 85 against 81 us, clustered).  Single
+// warps take longer to launch than CTAs of four (4096 rows, K = 256: 7.9 against 6.3 us).
+constexpr int kRingClasses = 8, kRingWarps = 4;
+__host__ __device__ constexpr int ring_ctas(int kch) { return kch == 1 ? 8 : kch == 2 ? 7 : kch <= 4 ? 5 : kch <= 6 ? 4 : 3; }
+// What a quad costs a warp: overhead, blocks of 8 rows, entries to put in place, and the rows of X where a window begins (with
+// the wait for them).
+__host__ __device__ constexpr unsigned quad_cost(int blocks, int entries, bool new_window) {
+    return 4 + 2 * blocks + 2 * ((entries + 31) / 32) + (new_window ? 8 : 0);
+}
+// One wave of warps takes equal shares of the quads, or by a table of first quads equal shares of their cost: hub windows
+// have full quads, most windows of a power-law graph one that is nearly empty.  R-MAT 18, K = 32 / 64 / 128 / 256: equal numbers
+// 101 / 127 / 187 / 354 us (SMs busy 73 % of the time), equal cost 82 / 104 / 155 / 322; weights of 4, 2, 1, 4 or of 2, 2, 2, 4 take 5
+// to 10 % more, 16 for a window 4 %.  The table is another load to wait for, so it is used only where the largest share gets
+// smaller by an eighth and warps have two quads or more (40000 clustered rows, K = 64, 6 quads a warp: 13.3 us without, 13.7 with;
+// 4096 uniform rows, K = 256, 1.3 quads a warp: 6.2 and 7.2).
+struct RingShares {
+    int warps;                    // of a wave
+    int offset;                   // of its table, where there is one
+    unsigned worst, worst_cost;   // largest share of equal numbers, of equal cost
+};
+struct RingTables {
+    RingShares of[kRingClasses];
+    int total;
+};
+__device__ __forceinline__ int first_quad(const unsigned* __restrict__ cost_before, int n_quads, int i, int warps) {
+    const unsigned long long want = (unsigned long long)cost_before[n_quads] * (unsigned)i / (unsigned)warps;
+    int lo = 0, hi = n_quads;   // first quad with `want` or more before it
+    while (lo < hi) {
+        const int mid = (lo + hi) >> 1;
+        if (cost_before[mid] < want) lo = mid + 1; else hi = mid;
+    }
+    return lo;
+}
+__global__ void ksp_shares(const unsigned* __restrict__ cost_before, int n_quads, RingTables s, int* __restrict__ starts,
+                           unsigned* __restrict__ worst /* [kRingClasses][2] */) {
+    const int x = blockIdx.x * blockDim.x + threadIdx.x;
+    if (x >= s.total) return;
+    int c = kRingClasses - 1;
+    while (x < s.of[c].offset) --c;
+    const int i = x - s.of[c].offset, warps = s.of[c].warps, per = (n_quads + warps - 1) / warps;
+    const int at = first_quad(cost_before, n_quads, i, warps);
+    starts[x] = at;
+    if (i == warps) return;
+    atomicMax(worst + 2 * c, cost_before[min((long long)(i + 1) * per, (long long)n_quads)] - cost_before[min((long long)i * per, (long long)n_quads)]);
+    atomicMax(worst + 2 * c + 1, cost_before[first_quad(cost_before, n_quads, i + 1, warps)] - cost_before[at]);
+}
+
 // One warp per quad: header, repeated columns, and the entries in CSR order, placed by row masks.
 __global__ void ksp_quads(const unsigned long long* __restrict__ key, const int* __restrict__ ent, const int* __restrict__ pair_idx,
                           const int* __restrict__ first_pair, const int* __restrict__ begin, const int* __restrict__ rowptr,
                           int n_rows, int nnz, int n_quads, SddmmQuad* __restrict__ quads, int* __restrict__ ids,
-                          unsigned* __restrict__ list, int* __restrict__ err) {
+                          unsigned* __restrict__ list, unsigned* __restrict__ cost, int* __restrict__ err) {
     __shared__ unsigned s_mask[8][16];
     __shared__ int s_before[8][16];
     const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
@@ -314,11 +361,15 @@ __global__ void ksp_quads(const unsigned long long* __restrict__ key, const int*
     }
     const int blocks = (cols + 7) / 8;
     if (lane >= cols && lane < blocks * 8) ids[(size_t)q * 32 + lane] = ids[(size_t)q * 32];
-    if (lane == 0) quads[q] = SddmmQuad{w, e0, (e - b) << 3 | blocks, b};
+    if (lane == 0) {
+        quads[q] = SddmmQuad{w, e0, (e - b) << 3 | blocks, b};
+        cost[q] = quad_cost(blocks, e - b, pair0 == first_pair[w]);
+        if (q + 1 == n_quads) cost[n_quads] = 0;
+    }
 }
 
 // One warp walks a contiguous range of quads, one block of 8 columns at a time: the window's X tile (16 x K) sits
-// in registers as A fragments, the 8 gathered Y rows are the B fragments.  Column ids (one per lane) and
+// in registers as A fragments (the next window's is loaded while results are put in place: 5 % of the clustered pattern), the 8 gathered Y rows are the B fragments.  Column ids (one per lane) and
 // headers come from memory two quads ahead, the Y rows kRowAhead blocks ahead as 16-byte cp.async copies into the
 // warp's ring; a lane copies exactly the pieces it reads back, so no lane waits for another.  (The odd Y rows land with
 // the two 64-byte halves of every 128 bytes swapped: chunk c at position c ^ 4.  A 16-byte access is served eight lanes
@@ -340,11 +391,8 @@ struct SddmmRing {
     static constexpr bool SWAP = CPR % 8 == 0;            // rows of 64 (mod 128) bytes alternate halves by themselves
     static constexpr int STAGE = 8 * ROWB;
     static constexpr int WARP_SMEM = kRowStages * STAGE + 16 * kTilePitch;
-    static constexpr int SMEM = 4 * WARP_SMEM;
-    // per SM: shared memory and registers (K = 64 with 8 CTAs of 64 registers spills: 85 against 81 us, clustered)
-    static constexpr int CTAS = KCH == 1 ? 8 : KCH == 2 ? 7 : KCH <= 4 ? 5 : KCH <= 6 ? 4 : 3;
+    static constexpr int SMEM = kRingWarps * WARP_SMEM;
 };
-
 template <int N, int I = 0, class Fn>
 __device__ __forceinline__ void sddmm_for(Fn&& fn) {
     if constexpr (I < N) {
@@ -360,17 +408,17 @@ __device__ __forceinline__ void cp_async16_to(uint32_t dst, const void* src) {
 
 // TAIL: K is not a multiple of 32; the chunks past the end of a row are zero on both sides.
 template <int KCH, bool TAIL, bool F32>
-__global__ void __launch_bounds__(128, SddmmRing<KCH>::CTAS) k_sddmm_tc_ring(
-    const SddmmQuad* __restrict__ quads, const int* __restrict__ ids, const unsigned* __restrict__ list, int n_quads,
-    const __half* __restrict__ X, const __half* __restrict__ Y, void* __restrict__ out, int n_rows, int pieces,
-    int ld16, int quads_per_warp) {
+__global__ void __launch_bounds__(32 * kRingWarps, ring_ctas(KCH)) k_sddmm_tc_ring(
+    const SddmmQuad* __restrict__ quads, const int* __restrict__ ids, const unsigned* __restrict__ list,
+    const int* __restrict__ starts, int n_quads, int quads_per_warp, const __half* __restrict__ X, const __half* __restrict__ Y,
+    void* __restrict__ out, int n_rows, int pieces, int ld16) {
     using R = SddmmRing<KCH>;
     extern __shared__ __align__(128) unsigned char smem[];
-    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    const int g = lane >> 2, t = lane & 3;
-    const int q0 = (blockIdx.x * 4 + wid) * quads_per_warp;
-    if (q0 >= n_quads) return;
-    const int nq = min(quads_per_warp, n_quads - q0);
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, g = lane >> 2, t = lane & 3;
+    const int warp = blockIdx.x * kRingWarps + wid;   // a table has an entry behind the last CTA's last warp
+    const int q0 = starts ? starts[warp] : warp * quads_per_warp;
+    const int nq = (starts ? starts[warp + 1] : min(q0 + quads_per_warp, n_quads)) - q0;
+    if (nq <= 0) return;
     unsigned char* const ring = smem + wid * R::WARP_SMEM;
     unsigned char* const tile = ring + kRowStages * R::STAGE;
     const uint32_t rows0 = smem_u32(ring);
@@ -384,7 +432,11 @@ __global__ void __launch_bounds__(128, SddmmRing<KCH>::CTAS) k_sddmm_tc_ring(
     ids += (size_t)q0 * 32 + lane;
 
     auto load_ids = [&](int q) { return q < nq ? __ldg(ids + (size_t)q * 32) : 0; };
-    auto load_head = [&](int q) { return q < nq ? __ldg((const int4*)(quads + q)) : make_int4(0, 0, 0, 0); };
+    auto load_head = [&](int q) {   // behind the last one: no blocks of the same window
+        int4 h = __ldg((const int4*)(quads + min(q, nq - 1)));
+        if (q >= nq) h.z = 0;
+        return h;
+    };
     auto issue_rows = [&](int c, auto stage) {
         constexpr int S = decltype(stage)::value * R::STAGE;
         const unsigned char* src = Yq + (unsigned long long)(uint32_t)c * pitch;
@@ -411,6 +463,20 @@ __global__ void __launch_bounds__(128, SddmmRing<KCH>::CTAS) k_sddmm_tc_ring(
 #pragma unroll
     for (int c = 0; c < KCH; ++c) xa[c] = xb[c] = make_uint4(0, 0, 0, 0);
 
+    auto load_x = [&](int w) {
+        cur_w = w;
+        const unsigned char* ra = Xq + (size_t)min(w * 16 + g, n_rows - 1) * pitch;
+        const unsigned char* rb = Xq + (size_t)min(w * 16 + g + 8, n_rows - 1) * pitch;
+#pragma unroll
+        for (int ch = 0; ch < KCH; ++ch) {
+            if (!TAIL || 4 * ch + t < pieces) {
+                xa[ch] = __ldg((const uint4*)(ra + ch * 64));
+                xb[ch] = __ldg((const uint4*)(rb + ch * 64));
+            }
+        }
+    };
+    load_x(head.x);
+
     for (int q = 0; q < nq; ++q) {
         const int id2 = load_ids(q + 2);
         const int4 head2 = load_head(q + 2);
@@ -419,18 +485,6 @@ __global__ void __launch_bounds__(128, SddmmRing<KCH>::CTAS) k_sddmm_tc_ring(
         unsigned ent[kListAhead];
 #pragma unroll
         for (int i = 0; i < kListAhead; ++i) ent[i] = 32 * i + lane < n_ent ? __ldg(entries + 32 * i + lane) : 0u;
-        if (head.x != cur_w) {  // warp-uniform
-            cur_w = head.x;
-            const unsigned char* ra = Xq + (size_t)min(cur_w * 16 + g, n_rows - 1) * pitch;
-            const unsigned char* rb = Xq + (size_t)min(cur_w * 16 + g + 8, n_rows - 1) * pitch;
-#pragma unroll
-            for (int ch = 0; ch < KCH; ++ch) {
-                if (!TAIL || 4 * ch + t < pieces) {
-                    xa[ch] = __ldg((const uint4*)(ra + ch * 64));
-                    xb[ch] = __ldg((const uint4*)(rb + ch * 64));
-                }
-            }
-        }
         // group 4 q + b carries the rows of block b; all but the newest kRowAhead - 1 groups are complete
         const bool full = nb == 4 && nb1 == 4;
         auto blocks = [&](auto all) {
@@ -463,6 +517,7 @@ __global__ void __launch_bounds__(128, SddmmRing<KCH>::CTAS) k_sddmm_tc_ring(
         });
         };
         if (full) blocks(std::true_type()); else blocks(std::false_type());
+        if (head1.x != cur_w) load_x(head1.x);   // warp-uniform; under way while the results are put in place
         __syncwarp();
         const long long o = (unsigned)head.y;
         auto put = [&](unsigned e) {
@@ -492,6 +547,8 @@ struct trs_sddmm_plan {
     trs::DevBuf<trs::SddmmQuad> quads;
     trs::DevBuf<int> ids;         // [quads][32]
     trs::DevBuf<unsigned> list;   // [nnz]
+    trs::RingTables shares;
+    const int* starts = nullptr;  // the tables, behind the ids
 };
 
 extern "C" int trs_sddmm_plan_destroy(trs_sddmm_plan* p) {
@@ -524,6 +581,9 @@ extern "C" int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, 
     if (nnz == 0) { *out = p; return TRS_OK; }
 
     const int W = (n_rows + 15) / 16;
+    int dev = 0, sms = 1;
+    TRS_CUDA(cudaGetDevice(&dev));
+    TRS_CUDA(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     TempSpace ts;
     ts.st = st;
     ts.chunk_bytes = (size_t)nnz * 38 + ((size_t)W + 1) * 12 + ((size_t)8 << 20);
@@ -540,10 +600,10 @@ extern "C" int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, 
     if (!rc) rc = ts.get((size_t)W + 1, &quads_of);
     if (!rc) rc = ts.get((size_t)W + 1, &quad_off);
     if (!rc) rc = ts.get(nnz, &begin);
-    if (!rc) rc = ts.get(2, &d_err);   // error bits, number of 8-column blocks
+    if (!rc) rc = ts.get(2 + 2 * kRingClasses, &d_err);   // error bits, number of 8-column blocks, largest shares
     if (rc) return fail(rc);
     auto grid = [](long long n) { return (unsigned)((n + 255) / 256); };
-    cudaMemsetAsync(d_err, 0, 2 * sizeof(int), st);
+    cudaMemsetAsync(d_err, 0, (2 + 2 * kRingClasses) * sizeof(int), st);
     ksp_rows<<<grid(n_rows), 256, 0, st>>>(rowptr, n_rows, d_err);
     ksp_keys<<<grid(nnz), 256, 0, st>>>(rowptr, col, n_rows, n_cols, nnz, key_a, ent_a, d_err);
     {
@@ -559,12 +619,14 @@ extern "C" int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, 
     while ((1ll << wbits) < W) ++wbits;
     cub::DoubleBuffer<unsigned long long> kb(key_a, key_b);
     cub::DoubleBuffer<int> vb(ent_a, ent_b);
-    size_t bytes = 0, bytes2 = 0, bytes3 = 0;
+    size_t bytes = 0, bytes2 = 0, bytes3 = 0, bytes4 = 0;
     cudaError_t e = cub::DeviceRadixSort::SortPairs(nullptr, bytes, kb, vb, (int)nnz, 0, 32 + wbits, st);
     if (e == cudaSuccess) e = cub::DeviceScan::InclusiveSum(nullptr, bytes2, head, pair_idx, (int)nnz, st);
     if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, bytes3, quads_of, quad_off, W + 1, st);
+    // costs of the quads: no more of them than entries
+    if (e == cudaSuccess) e = cub::DeviceScan::ExclusiveSum(nullptr, bytes4, (unsigned*)nullptr, (unsigned*)nullptr, nnz + 1, st);
     if (e != cudaSuccess) return fail((int)e);
-    bytes = std::max(bytes, std::max(bytes2, bytes3));
+    bytes = std::max(std::max(bytes, bytes4), std::max(bytes2, bytes3));
     unsigned char* tmp;
     if ((rc = ts.get(bytes + 16, &tmp))) return fail(rc);
     e = cub::DeviceRadixSort::SortPairs(tmp, bytes, kb, vb, (int)nnz, 0, 32 + wbits, st);
@@ -592,18 +654,36 @@ extern "C" int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, 
     p->n_blocks = n_blocks;
     p->n_pairs = total_pairs;
     rc = p->quads.alloc((size_t)n_quads);
-    if (!rc) rc = p->ids.alloc((size_t)n_quads * 32);
     if (!rc) rc = p->list.alloc((size_t)nnz);
+    RingTables& sh = p->shares;
+    sh.total = 0;
+    for (int c = 0; c < kRingClasses; ++c) {
+        sh.of[c] = RingShares{sms * ring_ctas(c + 1) * kRingWarps, sh.total, 0u, 0u};
+        sh.total += sh.of[c].warps + 1;
+    }
+    if (!rc) rc = p->ids.alloc((size_t)n_quads * 32 + sh.total);
+    int* const starts = p->ids.p + (size_t)n_quads * 32;
+    p->starts = starts;
+    unsigned *cost, *cost_before;
+    if (!rc) rc = ts.get((size_t)n_quads + 1, &cost);
+    if (!rc) rc = ts.get((size_t)n_quads + 1, &cost_before);
     if (rc) return fail(rc);
     ksp_columns<<<grid(nnz), 256, 0, st>>>(key, pair_idx, head, first_pair, quad_off, nnz, p->ids.p, begin);
     ksp_quads<<<(unsigned)ceil_div(n_quads, 8), 256, 0, st>>>(key, ent, pair_idx, first_pair, begin, rowptr, n_rows, (int)nnz, n_quads,
-                                                              p->quads.p, p->ids.p, p->list.p, d_err);
-    int herr = 0;
-    e = cudaMemcpyAsync(&herr, d_err, sizeof(int), cudaMemcpyDeviceToHost, st);
+                                                              p->quads.p, p->ids.p, p->list.p, cost, d_err);
+    e = cub::DeviceScan::ExclusiveSum(tmp, bytes, cost, cost_before, n_quads + 1, st);
+    if (e != cudaSuccess) return fail((int)e);
+    ksp_shares<<<grid(sh.total), 256, 0, st>>>(cost_before, n_quads, sh, starts, (unsigned*)d_err + 2);
+    int back[2 + 2 * kRingClasses];
+    e = cudaMemcpyAsync(back, d_err, sizeof(back), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return fail((int)e);
-    p->wide = (herr & 4) != 0;
+    p->wide = (back[0] & 4) != 0;
+    for (int c = 0; c < kRingClasses; ++c) {
+        sh.of[c].worst = (unsigned)back[2 + 2 * c];
+        sh.of[c].worst_cost = (unsigned)back[3 + 2 * c];
+    }
     *out = p;
     return TRS_OK;
 } TRS_CATCH
@@ -690,10 +770,12 @@ int launch_ring(const trs_sddmm_plan* p, const Operands& o, void* out, int K, cu
         TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM));
         if (dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
     }
-    // one wave of warps with equal shares (48 blocks a warp left the last of 2.4 waves nearly empty)
-    const int per_warp = ceil_div(p->n_quads, sm_count() * R::CTAS * 4);
-    kernel<<<ceil_div(ceil_div(p->n_quads, per_warp), 4), 128, R::SMEM, st>>>(p->quads.p, p->ids.p, p->list.p, p->n_quads, o.X, o.Y,
-                                                                             out, p->n_rows, (K + 7) / 8, o.ld / 8, per_warp);
+    const RingShares& sh = p->shares.of[KCH - 1];
+    const bool table = p->n_quads / 2 >= sh.warps && sh.worst_cost + sh.worst_cost / 8 < sh.worst;
+    const int per_warp = ceil_div(p->n_quads, sh.warps);
+    const int warps = table ? sh.warps : ceil_div(p->n_quads, per_warp);
+    kernel<<<ceil_div(warps, kRingWarps), 32 * kRingWarps, R::SMEM, st>>>(p->quads.p, p->ids.p, p->list.p, table ? p->starts + sh.offset : nullptr,
+                                                                        p->n_quads, per_warp, o.X, o.Y, out, p->n_rows, (K + 7) / 8, o.ld / 8);
     TRS_LAUNCH_CHECK();
     return TRS_OK;
 }
