@@ -175,6 +175,28 @@ __device__ __forceinline__ void cp_async_wait() {
     asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
+// A kernel launched behind another one of the same call (`behind`) is brought onto the SMs as that one's CTAs leave them; it
+// waits for its end before it touches anything that it wrote.  At least one thread has to wait: a later kernel waits only
+// for this one.  (Letting it come earlier, when the first one's CTAs have all started, gained nothing more, and the
+// instruction for that cost short items of the product 5 %: R-MAT 20, F = 13 216 -> 227 us.)
+__device__ __forceinline__ void wait_for_kernel_before() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
+template <class... Params, class... Args>
+int launch_behind(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, bool behind, Args... args) {
+    cudaLaunchAttribute attr;
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(threads);
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = st;
+    cfg.attrs = &attr;
+    cfg.numAttrs = behind ? 1 : 0;
+    TRS_CUDA(cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
+    return TRS_OK;
+}
+
 // D(16x8,f32) += A(16x16 with 2:4 sparsity, stored 16x8 f16) * B(16x8 f16).
 // `meta`: bits 4c..4c+3 = the two kept positions (p0 | p1<<2, p0<p1) of 4-column chunk c for
 // row lane/4; bits 16+4c.. the same for row lane/4+8.  All four lanes of a quad pass the same
