@@ -161,3 +161,37 @@ def test_shares_of_equal_cost(shape, K):
         ref[a:a + (1 << 18)] = (X[r[a:a + (1 << 18)]].float() * Y[col[a:a + (1 << 18)].long()].float()).sum(1)
     # fp16 results (2^-11) of fp32 sums, whose order differs by less than that
     assert float((out - ref).abs().max()) <= 2e-3 * float(ref.abs().max())
+
+
+def test_row_pointer_ends():
+    """What the product's kernel says about the ends of the row pointers: errors, no entries, calls from several threads and
+    streams at a time, and a capture, which has nothing to say."""
+    import threading
+    rp, col = (t.cuda() for t in _pattern("rmat"))
+    X = torch.randn(1024, 64, generator=torch.Generator().manual_seed(2)).half().cuda()
+    want = sddmm(rp, col, X, X)
+    for bad in (rp + 1, -rp):
+        with pytest.raises(TrsError) as e:
+            sddmm(bad, col, X, X)
+        assert e.value.code == -3
+    assert sddmm(torch.zeros_like(rp), col[:0], X, X).numel() == 0
+    failed = []
+
+    def calls(k):
+        with torch.cuda.stream(torch.cuda.Stream()):
+            torch.cuda._sleep(100000 * k)
+            for _ in range(50):
+                if not torch.equal(sddmm(rp, col, X, X), want):
+                    failed.append(k)
+
+    threads = [threading.Thread(target=calls, args=(k,)) for k in range(6)]
+    torch.cuda.synchronize()
+    [t.start() for t in threads]
+    [t.join() for t in threads]
+    assert not failed
+    out = torch.zeros_like(want)
+    with pytest.raises(Exception):
+        with torch.cuda.graph(torch.cuda.CUDAGraph()):
+            sddmm(rp, col, X, X, out=out)
+    torch.cuda.synchronize()
+    assert torch.equal(sddmm(rp, col, X, X), want)
