@@ -155,3 +155,14 @@ def test_warp_sort_borders(entries, bits, long_row):
     rowptr = torch.zeros(17, dtype=torch.int32)
     rowptr[1:] = torch.cumsum(per_row, 0)
     _check(rowptr, torch.cat(cols).to(torch.int32), torch.randn(entries, generator=g))
+
+
+@pytest.mark.parametrize("windows", [1, 1023, 1024, 4095, 4096, 4607, 4608, 9000])
+def test_scan_borders(windows):
+    """Sums over windows on both sides of a round of the one-CTA scan, and of its largest number of values."""
+    g = torch.Generator().manual_seed(windows)
+    n = 16 * windows - 3
+    rows = torch.cat([torch.arange(0, n, 5), torch.randint(0, n, (n,), generator=g)])
+    cols = torch.randint(0, 300, (rows.numel(),), generator=g)
+    rp, col, _ = graphs.coo_to_csr(rows, cols, n, 300)
+    _check(rp, col, torch.randn(col.numel(), generator=g))

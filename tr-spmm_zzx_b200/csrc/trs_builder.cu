@@ -84,9 +84,23 @@ struct InputInfo {
     u64 hub_entries;
 };
 
+// Words that the host looks at, copied into pinned memory by the kernel that finishes them.
+struct Publish {
+    const int* a;
+    int* host_a;
+    int na;
+    const int* b;
+    int* host_b;
+    int nb;
+    __device__ __forceinline__ void by_block() const {
+        for (int i = threadIdx.x; i < na; i += blockDim.x) host_a[i] = __ldcg(a + i);
+        for (int i = threadIdx.x; i < nb; i += blockDim.x) host_b[i] = __ldcg(b + i);
+    }
+};
+
 __global__ void kb_input_info(const int* __restrict__ rowptr, const int* __restrict__ col, int n_rows, int window, int W,
                               int* __restrict__ sel /* [kSortClasses + 1][W] */, int* __restrict__ ncol /* [W], cleared */,
-                              InputInfo* __restrict__ info) {
+                              InputInfo* info, unsigned* done /* cleared */, Publish pub) {
     const long long t0 = (long long)blockIdx.x * blockDim.x + threadIdx.x, step = (long long)gridDim.x * blockDim.x;
     const int first = rowptr[0], nnz = rowptr[n_rows];
     if (t0 == 0) { info->first = first; info->last = nnz; }
@@ -121,12 +135,93 @@ __global__ void kb_input_info(const int* __restrict__ rowptr, const int* __restr
         }
         if (c == kSortClasses) atomicAdd(&info->hub_entries, (u64)n);
     }
-    if (first != 0 || !col) return;
-    int m = -1;
-    for (long long e = t0; e < nnz; e += step) m = max(m, col[e]);
-    m = __reduce_max_sync(0xffffffffu, m);
-    if (lane == 0 && m > info->max_col) atomicMax(&info->max_col, m);
+    if (first == 0 && col) {
+        int m = -1;
+        for (long long e = t0; e < nnz; e += step) m = max(m, col[e]);
+        m = __reduce_max_sync(0xffffffffu, m);
+        if (lane == 0 && m > __ldcg(&info->max_col)) atomicMax(&info->max_col, m);
+    }
+    // the last block to get here passes everything on to the host
+    __shared__ bool s_last;
+    __threadfence();
+    __syncthreads();
+    if (threadIdx.x == 0) s_last = atomicAdd(done, 1u) + 1 == gridDim.x;
+    __syncthreads();
+    if (!s_last) return;
+    __threadfence();
+    pub.by_block();
 }
+
+// Exclusive scan of a few thousand values by one CTA: the device-wide scan and the copy of its sum for the host are three
+// launches, this is one.  What bounds it is one SM's load and store rate, so up to 4608 values (builds of 9000 uniform rows 222 ->
+// 201 us, of 20000 clustered ones 278 -> 252, with the other read-backs made by the kernels that finish them; 16385 windows of
+// four words a build of 567 -> 612).
+constexpr int kSmallScan = 4608;
+template <class T, class Shuffle>
+__device__ __forceinline__ T shuffle_words(const T& x, Shuffle&& shuffle) {
+    static_assert(sizeof(T) % 4 == 0, "");
+    T y;
+#pragma unroll
+    for (int i = 0; i < (int)(sizeof(T) / 4); ++i) ((int*)&y)[i] = shuffle(((const int*)&x)[i]);
+    return y;
+}
+template <class T, class Op>
+__device__ __forceinline__ T warp_inclusive(T x, Op op, int lane) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const T y = shuffle_words(x, [&](int w) { return __shfl_up_sync(0xffffffffu, w, d); });
+        if (lane >= d) x = op(y, x);
+    }
+    return x;
+}
+template <class T, class Op, class In, class Out>
+__global__ void __launch_bounds__(1024) kb_scan_small(In in, Out out, Op op, T zero, int n, Publish pub) {
+    constexpr int kItems = 4;   // consecutive ones per thread and round (one: 1.2 us a round of 1024 four-word values)
+    __shared__ T s_warp[2][32];
+    const int tid = threadIdx.x, lane = tid & 31, wid = tid >> 5;
+    T before = zero, next[kItems];
+    auto load = [&](int base) {
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) next[i] = base + tid * kItems + i < n ? in(base + tid * kItems + i) : zero;
+    };
+    load(0);
+    for (int base = 0, k = 0; base < n; base += 1024 * kItems, k ^= 1) {
+        T x[kItems];
+        T mine = zero;
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) { x[i] = next[i]; mine = op(mine, x[i]); }
+        load(base + 1024 * kItems);
+        const T incl = warp_inclusive(mine, op, lane);
+        if (lane == 31) s_warp[k][wid] = incl;
+        __syncthreads();
+        const T warps = warp_inclusive(s_warp[k][lane], op, lane);
+        T at = before;   // everything before this thread's values
+        if (wid > 0) at = op(at, shuffle_words(warps, [&](int w) { return __shfl_sync(0xffffffffu, w, max(wid - 1, 0)); }));
+        const T prev = shuffle_words(incl, [&](int w) { return __shfl_up_sync(0xffffffffu, w, 1); });
+        if (lane > 0) at = op(at, prev);
+#pragma unroll
+        for (int i = 0; i < kItems; ++i) {
+            if (base + tid * kItems + i < n) out(base + tid * kItems + i, at);
+            at = op(at, x[i]);
+        }
+        before = op(before, shuffle_words(warps, [&](int w) { return __shfl_sync(0xffffffffu, w, 31); }));
+    }
+    __syncthreads();
+    pub.by_block();
+}
+template <class T>
+struct FromArray {
+    const T* p;
+    __device__ __forceinline__ T operator()(int i) const { return p[i]; }
+};
+template <class T>
+struct ToArray {
+    T* p;
+    __device__ __forceinline__ void operator()(int i, const T& x) const { p[i] = x; }
+};
+struct IntSum {
+    __host__ __device__ __forceinline__ int operator()(int a, int b) const { return a + b; }
+};
 
 // ---------------------------------------------------------------------------------------------
 // 1. - 3. the columns of every window
@@ -611,12 +706,13 @@ __device__ __forceinline__ int local_row(const int* __restrict__ rowptr, int n_r
     return lo;
 }
 
-__global__ void kb_hub_sizes(const int* __restrict__ rowptr, int n_rows, int window, const int* __restrict__ sel, int H,
-                             int* __restrict__ size) {
-    const int h = blockIdx.x * blockDim.x + threadIdx.x;
-    if (h > H) return;
-    size[h] = h < H ? rowptr[min((long long)(sel[h] + 1) * window, (long long)n_rows)] - rowptr[(size_t)sel[h] * window] : 0;
-}
+struct HubSizes {
+    const int *rowptr, *sel;
+    int n_rows, window, n;
+    __device__ __forceinline__ int operator()(int h) const {
+        return h < n ? rowptr[min((long long)(sel[h] + 1) * window, (long long)n_rows)] - rowptr[(size_t)sel[h] * window] : 0;
+    }
+};
 
 template <class Key>
 __global__ void kb_hub_keys(const int* __restrict__ rowptr, const int* __restrict__ col, int n_rows, int window, HubView hub, int E,
@@ -1316,6 +1412,14 @@ struct GroupsTilesSum {
 struct WithTiles {
     __host__ __device__ __forceinline__ GroupsTiles operator()(int groups) const { return GroupsTiles{groups, (groups + 3) / 4}; }
 };
+struct GroupsFrom {
+    const int* groups;
+    __device__ __forceinline__ GroupsTiles operator()(int i) const { return WithTiles()(groups[i]); }
+};
+struct GroupsTo {
+    int *groups, *tiles;
+    __device__ __forceinline__ void operator()(int i, const GroupsTiles& x) const { groups[i] = x.groups; tiles[i] = x.tiles; }
+};
 struct ToTuple {
     __host__ __device__ __forceinline__ thrust::tuple<int, int> operator()(const GroupsTiles& g) const { return {g.groups, g.tiles}; }
 };
@@ -1714,8 +1818,9 @@ struct PartsOut {
 // extras, by column.  One thread per row writes its parts and the unit's entries, one per extra its place:
 // its rank among the row's extras plus the unit entries before it (a hub row has thousands).
 __global__ void kb_cuda_rows(int n_rows, int window, int part_c, int short_size, const int* __restrict__ win_cuda_unit,
-                             WindowView v, RecordView r, Extras x, PartsAt off, PartsOut po) {
+                             WindowView v, RecordView r, Extras x, PartsAt off, PartsOut po, Publish pub) {
     int row = blockIdx.x * blockDim.x + threadIdx.x;
+    if (blockIdx.x == 0) pub.by_block();
     if (row == 0) { po.c_row_offset[0] = 0; po.cs_row_offset[0] = 0; }
     if (row >= n_rows) return;
     const Parts o = off[row], e = off[row + 1];
@@ -1758,13 +1863,9 @@ __global__ void kb_cuda_extras(int window, const int* __restrict__ win_cuda_unit
     po.put(o, off[row + 1].zl - o.zl, rank, c, r.sval[x.at[i]]);
 }
 
-// Two runs of words into pinned host memory: a copy of a few words took 3.4 us behind a gap of up to 8 on the copy
+// Words for the host where no kernel above can do it: a copy of a few words took 3.4 us behind a gap of up to 8 on the copy
 // engine, this takes 2 behind 1.
-__global__ void kb_publish(const int* __restrict__ a, int na, int* __restrict__ host_a, const int* __restrict__ b, int nb,
-                           int* __restrict__ host_b) {
-    for (int i = threadIdx.x; i < na; i += blockDim.x) host_a[i] = a[i];
-    for (int i = threadIdx.x; i < nb; i += blockDim.x) host_b[i] = b[i];
-}
+__global__ void kb_publish(Publish p) { p.by_block(); }
 
 __global__ void kb_to_half(const float* __restrict__ src, long long n, __half* __restrict__ dst) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
@@ -1860,9 +1961,6 @@ struct Cub {
     int exclusive_scan(In in, Out out, Op op, T zero, long long n) {
         return run([&](void* t, size_t& b) { return cub::DeviceScan::ExclusiveScan(t, b, in, out, op, zero, n, st); });
     }
-    int exclusive_sum(const int* in, int* out, long long n) {
-        return run([&](void* t, size_t& b) { return cub::DeviceScan::ExclusiveSum(t, b, in, out, n, st); });
-    }
     template <class K, class V>
     int sort_pairs(K* k_in, K* k_out, V* v_in, V* v_out, long long n, int end_bit, K** k_res, V** v_res) {
         cub::DoubleBuffer<K> kb(k_in, k_out);
@@ -1901,20 +1999,19 @@ struct Mirror {
 
 // what a build reads back, from the device into a Mirror; the host may look after an event or a synchronisation behind it
 template <class A, class B>
-int publish(const A* a, A* host_a, const B* b, B* host_b, cudaStream_t st) {
-    kb_publish<<<1, 128, 0, st>>>((const int*)a, (int)(sizeof(A) / 4), (int*)host_a, (const int*)b, (int)(sizeof(B) / 4), (int*)host_b);
-    TRS_LAUNCH_CHECK();
-    return 0;
+Publish words(const A* a, A* host_a, const B* b, B* host_b) {
+    return Publish{(const int*)a, (int*)host_a, (int)(sizeof(A) / 4), (const int*)b, (int*)host_b, (int)(sizeof(B) / 4)};
 }
 template <class T>
-int publish(const T* dev, T* host, cudaStream_t st) {
-    kb_publish<<<1, 128, 0, st>>>((const int*)dev, (int)(sizeof(T) / 4), (int*)host, nullptr, 0, nullptr);
+Publish words(const T* dev, T* host) { return Publish{(const int*)dev, (int*)host, (int)(sizeof(T) / 4), nullptr, nullptr, 0}; }
+int publish(const Publish& p, cudaStream_t st) {
+    kb_publish<<<1, 128, 0, st>>>(p);
     TRS_LAUNCH_CHECK();
     return 0;
 }
 template <class T>
 int read_back(const T* dev, T* host, cudaStream_t st) {
-    TRS_TRY(publish(dev, host, st));
+    TRS_TRY(publish(words(dev, host), st));
     TRS_CUDA(cudaStreamSynchronize(st));
     return 0;
 }
@@ -2015,18 +2112,16 @@ int sort_hubs(trs_builder* B, const int* rowptr, const int* col, const float* va
     const int H = info.windows[kSortClasses], E = (int)info.hub_entries, n = B->n_rows, window = B->cfg.window;
     const int h_bits = bits_for(H - 1);
     const int* sel = R.sel + (size_t)kSortClasses * B->W;
-    int *size, *off, *first_rec, *place_a, *place_b, *place;
+    int *off, *first_rec, *place_a, *place_b, *place;
     Key *keys_a, *keys_b, *keys;
-    TRS_TRY(ts.get((size_t)H + 1, &size));
     TRS_TRY(ts.get((size_t)H + 1, &off));
     TRS_TRY(ts.get((size_t)H, &first_rec));
     TRS_TRY(ts.get(E, &keys_a));
     TRS_TRY(ts.get(E, &keys_b));
     TRS_TRY(ts.get(E, &place_a));
     TRS_TRY(ts.get(E, &place_b));
-    kb_hub_sizes<<<grid_for(H + 1), 256, 0, st>>>(rowptr, n, window, sel, H, size);
+    kb_scan_small<<<1, 1024, 0, st>>>(HubSizes{rowptr, sel, n, window, H}, ToArray<int>{off}, IntSum(), 0, H + 1, Publish{});
     TRS_LAUNCH_CHECK();
-    TRS_TRY(cub_.exclusive_sum(size, off, H + 1));
     const HubView hub{sel, off, H};
     kb_hub_keys<Key><<<grid_for(E), 256, 0, st>>>(rowptr, col, n, window, hub, E, col_bits, keys_a, place_a, d_info);
     TRS_LAUNCH_CHECK();
@@ -2037,7 +2132,7 @@ int sort_hubs(trs_builder* B, const int* rowptr, const int* col, const float* va
     TRS_TRY(cub_.run([&](void* t, size_t& b) {
         return cub::DeviceSelect::If(t, b, thrust::counting_iterator<int>(0), start, d_count, E, is_head, st);
     }));
-    TRS_TRY(publish((const int*)d_count, &back->records, (const int*)&d_info->err, &back->err, st));
+    TRS_TRY(publish(words((const int*)d_count, &back->records, (const int*)&d_info->err, &back->err), st));
     TRS_TRY(meanwhile());
     TRS_CUDA(cudaStreamSynchronize(st));
     if (back->err & 2) return TRS_E_NOT_CANONICAL;   // a repeated column may have more entries than a record counts
@@ -2134,7 +2229,7 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
 
     // ---- sizes of the input ---------------------------------------------------------------------
     struct Counts { InputInfo info; MatchCounts mc; };
-    struct Head { Counts counts; u64 dropped[kDropCounters]; int hub_records, pad; };
+    struct Head { Counts counts; u64 dropped[kDropCounters]; int hub_records; unsigned info_blocks; };
     struct Back { Head head; HubBack hub; Win total; Parts parts; int groups, tiles, tc_nnz; };   // what the host sees of it
     static_assert(sizeof(Back) <= Mirror::kBytes, "");
     Mirror mirror;
@@ -2146,9 +2241,10 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     Records R;
     TRS_TRY(ts.get((size_t)(kSortClasses + 1) * W, &R.sel));
     TRS_TRY(ts.get((size_t)W, &R.w.ncol));
-    kb_input_info<<<2 * sms, 512, 0, st>>>(rowptr, col, n, window, W, R.sel, R.w.ncol, &d_head->counts.info);
+    kb_input_info<<<2 * sms, 512, 0, st>>>(rowptr, col, n, window, W, R.sel, R.w.ncol, &d_head->counts.info, &d_head->info_blocks,
+                                         words(&d_head->counts.info, &back->head.counts.info));
     TRS_LAUNCH_CHECK();
-    TRS_TRY(read_back(&d_head->counts.info, &back->head.counts.info, st));
+    TRS_CUDA(cudaStreamSynchronize(st));
     const InputInfo info = back->head.counts.info;
     if (info.first != 0 || info.last < 0 || (info.err & 1)) return TRS_E_OFFSETS;
     const long long nnz = B->nnz = info.last;
@@ -2160,6 +2256,17 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     TRS_TRY(make_records(B, rowptr, col, val, info, &d_head->counts.info, &d_head->hub_records, &back->hub, ts, cub_, st, &R));
     const RecordView rv{R.w.rec, R.w.sval};
 
+    // Scans by one CTA where they are short (`from`, `to`), by device-wide passes over the iterators otherwise; `pub` goes to the
+    // host behind them.
+    auto scan = [&](auto from, auto to, auto in, auto out, auto op, auto zero, long long count, const Publish& pub) -> int {
+        if (count <= kSmallScan) {
+            kb_scan_small<<<1, 1024, 0, st>>>(from, to, op, zero, (int)count, pub);
+            TRS_LAUNCH_CHECK();
+            return 0;
+        }
+        TRS_TRY(cub_.exclusive_scan(in, out, op, zero, count));
+        return pub.na > 0 ? publish(pub, st) : 0;
+    };
     // ---- 4., 5. TC columns, units, sizes per window ---------------------------------------------
     int *rec, *end, *tc, *sel_block, *sel_huge;
     Win *win, *pre;
@@ -2172,10 +2279,10 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     TRS_TRY(ts.get((size_t)W + 1, &sel_huge));
     kb_windows<<<grid_for(W + 1, 128), 128, 0, st>>>(rowptr, R.w.ncol, R.w.cnt, W, cfg, rec, end, tc, win, sel_block, sel_huge, &d_head->counts.mc);
     TRS_LAUNCH_CHECK();
-    TRS_TRY(cub_.exclusive_scan(win, pre, WinSum(), Win{0, 0, 0, 0}, W + 1));
+    TRS_TRY(scan(FromArray<Win>{win}, ToArray<Win>{pre}, win, pre, WinSum(), Win{0, 0, 0, 0}, W + 1,
+                 words(&d_head->counts, &back->head.counts, (const Win*)pre + W, &back->total)));
     const WindowView v{rec, end, tc, pre};
     Event sized, grouped, counted;
-    TRS_TRY(publish(&d_head->counts, &back->head.counts, (const Win*)pre + W, &back->total, st));
     TRS_TRY(sized.record(st));
 
     // ---- 6. matching ------------------------------------------------------------------------------
@@ -2201,8 +2308,8 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
         const auto both = thrust::make_transform_iterator((const int*)mo.groups, WithTiles());
         const auto out = thrust::make_transform_output_iterator(
             thrust::make_zip_iterator(thrust::make_tuple(B->s_offset.p, B->s_window_tile_offset.p)), ToTuple());
-        TRS_TRY(cub_.exclusive_scan(both, out, GroupsTilesSum(), GroupsTiles{0, 0}, W + 1));
-        TRS_TRY(publish((const int*)B->s_offset.p + W, &back->groups, (const int*)B->s_window_tile_offset.p + W, &back->tiles, st));
+        TRS_TRY(scan(GroupsFrom{mo.groups}, GroupsTo{B->s_offset.p, B->s_window_tile_offset.p}, both, out, GroupsTilesSum(), GroupsTiles{0, 0}, W + 1,
+                     words((const int*)B->s_offset.p + W, &back->groups, (const int*)B->s_window_tile_offset.p + W, &back->tiles)));
         return grouped.record(st);
     };
     // Without large windows the bounds are close enough to start before the sizes have come back (30 us of 870 on the
@@ -2269,7 +2376,8 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     TRS_TRY(B->out(B->t_binary, 6, (size_t)NB * 2));
     kb_tc_blocks<<<grid_for(NB + 1, 128), 128, 0, st>>>(v, rv, W, NB, B->t_column.p, B->t_binary.p, blk_nnz, slot_rec);
     TRS_LAUNCH_CHECK();
-    TRS_TRY(cub_.exclusive_sum(blk_nnz, B->t_block_offset.p, (long long)NB + 1));
+    TRS_TRY(scan(FromArray<int>{blk_nnz}, ToArray<int>{B->t_block_offset.p}, (const int*)blk_nnz, B->t_block_offset.p, IntSum(), 0, (long long)NB + 1,
+                 Publish{}));
     if (!ahead) {   // the hub windows are matched by now
         if (mc.n_huge > 0) { TRS_TRY(done[0].record(side[0])); TRS_CUDA(cudaStreamWaitEvent(st, done[0].e, 0)); }
         if (mc.n_block > 0) { TRS_TRY(done[1].record(side[1])); TRS_CUDA(cudaStreamWaitEvent(st, done[1].e, 0)); }
@@ -2290,16 +2398,15 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     TRS_TRY(ts.get((size_t)part_blocks + 1, &before));
     const PartsAt off{inside, before};
     Extras x{nullptr, nullptr, 0};
-    auto count_parts = [&]() -> int {
+    auto count_parts = [&](const Publish& pub) -> int {
         kb_cuda_count<<<part_blocks, kPartRows, 0, st>>>(n, window, cfg.part_c, cfg.short_size, mo.cuda_unit, v, rv, x, inside, block);
         TRS_LAUNCH_CHECK();
-        return cub_.exclusive_scan(block, before, PartsSum(), Parts{0, 0, 0, 0}, (long long)part_blocks + 1);
+        return scan(FromArray<Parts>{block}, ToArray<Parts>{before}, block, before, PartsSum(), Parts{0, 0, 0, 0}, (long long)part_blocks + 1, pub);
     };
-    if (!cfg.strict) TRS_TRY(count_parts());
     if (cfg.strict) {
-        TRS_TRY(publish((const int*)B->t_block_offset.p + NB, &back->tc_nnz, st));
+        TRS_TRY(publish(words((const int*)B->t_block_offset.p + NB, &back->tc_nnz), st));
     } else {
-        TRS_TRY(publish((const int*)B->t_block_offset.p + NB, &back->tc_nnz, (const Parts*)before + part_blocks, &back->parts, st));
+        TRS_TRY(count_parts(words((const int*)B->t_block_offset.p + NB, &back->tc_nnz, (const Parts*)before + part_blocks, &back->parts)));
     }
     TRS_TRY(counted.record(st));
 
@@ -2362,8 +2469,8 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
             TRS_TRY(cub_.sort_pairs(xkey_a, xkey_b, xat_a, xat_b, (long long)n_extra, 32 + bits_for(n), &key, &at));
             x = Extras{key, at, (int)n_extra};
         }
-        TRS_TRY(count_parts());
-        TRS_TRY(read_back((const Parts*)before + part_blocks, &back->parts, st));
+        TRS_TRY(count_parts(words((const Parts*)before + part_blocks, &back->parts)));
+        TRS_CUDA(cudaStreamSynchronize(st));
     }
     const Parts p = back->parts;
     TRS_TRY(B->out(B->c_row_offset, 7, (size_t)p.nl + 1));
@@ -2378,13 +2485,14 @@ int do_build(trs_builder* B, const int* rowptr, const int* col, const float* val
     TRS_TRY(B->out(B->cs_value, 16, p.zs));
     const PartsOut po{B->c_row_offset.p, B->c_row.p, B->c_atomic.p, B->c_column.p, B->c_value.p,
                       B->cs_row_offset.p, B->cs_row.p, B->cs_atomic.p, B->cs_column.p, B->cs_value.p};
-    kb_cuda_rows<<<grid_for(n), 256, 0, st>>>(n, window, cfg.part_c, cfg.short_size, mo.cuda_unit, v, rv, x, off, po);
+    kb_cuda_rows<<<grid_for(n), 256, 0, st>>>(n, window, cfg.part_c, cfg.short_size, mo.cuda_unit, v, rv, x, off, po,
+                                             words(&d_head->dropped, &back->head.dropped));
     TRS_LAUNCH_CHECK();
     if (x.n > 0) {
         kb_cuda_extras<<<grid_for(x.n), 256, 0, st>>>(window, mo.cuda_unit, v, rv, x, off, po);
         TRS_LAUNCH_CHECK();
     }
-    TRS_TRY(read_back(&d_head->dropped, &back->head.dropped, st));
+    TRS_CUDA(cudaStreamSynchronize(st));
     mirror.pending = false;
     B->dropped = 0;
     if (!cfg.strict)   // nothing is lost in strict mode
