@@ -164,3 +164,22 @@ def test_nearly_empty_matrices(entries):
     for w0, w1 in ((0, 300), (300, 4000), (4000, n // 16)):
         plan.run_windows(B.cuda(), parts, w0, w1)
     assert torch.equal(parts, out)
+
+
+@pytest.mark.parametrize("F", [50, 64])
+@pytest.mark.parametrize("per_row", [1, 3, 9, 40])
+def test_first_column_ids(F, per_row):
+    """Enough items for a warp each, with less than a block of eight steps, a block, and more; windows without entries between
+    them: the ids beside the items are those of the stream."""
+    n = 40000
+    g = torch.Generator().manual_seed(per_row)
+    rows = torch.arange(n).repeat_interleave(per_row)
+    rows = rows[(rows // 16) % 5 != 2]
+    rp, col, _ = graphs.coo_to_csr(rows, torch.randint(0, n, (rows.numel(),), generator=g), n, n)
+    val = torch.randn(col.numel(), generator=g)
+    B = torch.randn(n, F, generator=g).half()
+    fmt = build_format(rp.cuda(), col.cuda(), val.cuda(), strict=True)[0]
+    out = SpmmPlan(fmt, n, n).run(B.cuda(), out_dtype=torch.float32).cpu()
+    ref = torch.sparse_csr_tensor(rp.long(), col.long(), val.half().double(), (n, n)) @ B.double()
+    # fp32 sums of exact products of fp16 values
+    assert float((out - ref).abs().max()) <= 2e-5 * float(ref.abs().max())

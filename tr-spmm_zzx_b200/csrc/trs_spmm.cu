@@ -66,6 +66,7 @@ struct KernelArgs {
     int n_items;
     int w_begin, w_end;            // window range of this run (RANGE instances: items outside return at once)
     const int* ids;                // [steps + kIdSpare][16] column ids of the step stream
+    const int* first_ids;          // [n_items][kIdBlock][16] those of the first block of every item, or null
     const uint32_t* packed_a;      // [tiles][64]
     const uint32_t* packed_meta;   // [tiles][8]
     const uint4* dense;            // [dense steps][32] A tiles in fragment order, one uint4 per lane
@@ -337,6 +338,12 @@ __global__ void k_fill_steps(trs_format f, WindowRanges wr, const Item* __restri
     }
 }
 
+// The first block of column ids of every item, one warp each (it may go past the item's and the stream's end: kIdSpare).
+__global__ void k_first_ids(const Item* __restrict__ items, int n_items, const int* __restrict__ ids, int* __restrict__ first) {
+    const int i = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, lane = threadIdx.x & 31;
+    if (i < n_items) ((int4*)first)[(size_t)i * 32 + lane] = ((const int4*)(ids + (size_t)items[i].step0 * 16))[lane];
+}
+
 // Validation: every violated rule ORs one bit into *err.
 enum { V_OFFSETS = 1, V_COLUMN = 2, V_ROW = 4, V_SHAPE = 8 };
 
@@ -533,6 +540,11 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
     unsigned char* const smem = smem_all + wid * T::SMEM;
     const int fbase = blockIdx.y * FS;
 
+    // The first column ids do not wait for the item where they lie beside it: a start is one trip to memory shorter.  64 features
+    // alone: the instance spills less with it too (262144 clustered rows 63.7 -> 61.7 us, 131072 uniform ones 34.9 -> 33.3, R-MAT 18
+    // lossless 93.3 -> 90.4); 128 gain nothing, 16, 32 and 96 lose 2 to 7 %.
+    const bool beside = FS == 64 && WPI == 1 && ALIGNED && !RANGE && a.first_ids;
+    if (beside) cp_async16(smem_u32(smem) + T::STAGE * STAGES + lane * 16, a.first_ids + (size_t)blockIdx.x * (kIdBlock * 16) + lane * 4);
     const Item it = a.items[blockIdx.x];
     if constexpr (RANGE) {   // a test in the whole-matrix instance costs up to 20 % (it delays the first ids of short items)
         if (it.window < a.w_begin || it.window >= a.w_end) return;
@@ -656,7 +668,7 @@ __global__ void __launch_bounds__(32 * WPI, MINB) k_window_spmm_warp(const Kerne
     };
 
     if (nsteps > 0) {
-        issue_ids(0);
+        if (!beside) issue_ids(0);
         cp_async_commit();
         wait_for_kernel_before();   // the copy of B, where there is one
         cp_async_wait<0>();
@@ -842,6 +854,7 @@ struct trs_spmm_plan {
     int per_sample = 1;
     std::vector<int> item_at, heavy_at, step_at;
     int* ids = nullptr;      // [steps + kIdSpare][16] column ids of the step stream
+    int* first_ids = nullptr;   // [fine items][kIdBlock][16] the first ones of the items in launch order
     uint4* dense = nullptr;  // [dense steps][32] A tiles of the dense steps in fragment order
     int n_steps, sms;        // of all items; SMs of the device
 };
@@ -1033,14 +1046,18 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
         coarse.longest = info.coarse.longest;
     }
     const size_t ids_bytes = ((size_t)n_steps + kIdSpare) * 64, dense_bytes = (size_t)n_dense * 512;
+    // 512 bytes an item, so not where most have next to no steps
+    const size_t first_bytes = n_steps / 2 >= n_items ? (size_t)n_items * (kIdBlock * 64) : 0;
     const size_t items_bytes = ((size_t)2 * n_items + coarse.n_items) * sizeof(Item);
     const size_t heavy_bytes = ((size_t)n_heavy + coarse.n_heavy) * sizeof(Heavy);
     // the kernels read the packed values 8 bytes per lane; an array that does not allow that is copied
     const size_t packed_bytes = ((uintptr_t)f.s_packed_a & 7) != 0 ? (size_t)f.tiles * 256 : 0;
     auto fail = [&](int code) { trs_spmm_plan_destroy(p); return code; };
-    if ((rc = pool_alloc(&p->block, ids_bytes + dense_bytes + packed_bytes + items_bytes + heavy_bytes, st))) return fail(rc);
+    if ((rc = pool_alloc(&p->block, ids_bytes + first_bytes + dense_bytes + packed_bytes + items_bytes + heavy_bytes, st))) return fail(rc);
     unsigned char* at = (unsigned char*)p->block;
     p->ids = (int*)at; at += ids_bytes;
+    if (first_bytes) p->first_ids = (int*)at;
+    at += first_bytes;
     p->dense = (uint4*)at; at += dense_bytes;
     if (packed_bytes) {
         const cudaError_t copied = cudaMemcpyAsync(at, f.s_packed_a, packed_bytes, cudaMemcpyDeviceToDevice, st);
@@ -1071,6 +1088,7 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
             k_fill_coarse<<<grid(W), 256, 0, st>>>(f, W, off, open, &d_info->made, coarse.items, coarse.heavy);
         e = sort(sort_tmp);
     }
+    if (e == cudaSuccess && p->first_ids) k_first_ids<<<grid((long long)n_items * 32), 256, 0, st>>>(fine.items, n_items, p->ids, p->first_ids);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return fail((int)e);
@@ -1273,6 +1291,7 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
     }
     a.w_begin = w0; a.w_end = w1;
     a.ids = p->ids; a.dense = p->dense;
+    a.first_ids = a.items == p->fine.items ? p->first_ids : nullptr;
     a.packed_a = p->f.s_packed_a; a.packed_meta = p->f.s_packed_meta;
     a.B = (const __half*)B; a.C = C; a.scratch = (float*)workspace;
     a.ldb = F; a.ldS = scratch_ld(F); a.F = F; a.bchunks = ceil_div(F, 8);
