@@ -552,18 +552,26 @@ struct trs_sddmm_plan {
     long long nnz = 0, n_blocks = 0, n_pairs = 0;
     int n_quads = 0;
     bool wide = false;   // a window with too many entries for the lists
-    trs::DevBuf<trs::SddmmQuad> quads;
-    trs::DevBuf<int> ids;         // [quads][32]
-    trs::DevBuf<unsigned> list;   // [nnz]
+    int device = 0;
+    void* block = nullptr;        // pool memory of the arrays below (a cudaMalloc each took up to milliseconds)
+    trs::SddmmQuad* quads = nullptr;
+    int* ids = nullptr;           // [quads][32]
+    unsigned* list = nullptr;     // [nnz]
     trs::RingTables shares;
     const int* starts = nullptr;  // the tables, behind the ids
 };
 
 extern "C" int trs_sddmm_plan_destroy(trs_sddmm_plan* p) {
     if (!p) return TRS_OK;
-    p->quads.release();
-    p->ids.release();
-    p->list.release();
+    if (p->block) {
+        // kernels on any stream may still read the plan: wait as cudaFree would
+        int dev = 0;
+        cudaGetDevice(&dev);
+        if (dev != p->device) cudaSetDevice(p->device);
+        cudaDeviceSynchronize();
+        trs::pool_free(p->block, nullptr);
+        if (dev != p->device) cudaSetDevice(dev);
+    }
     delete p;
     return TRS_OK;
 }
@@ -661,24 +669,29 @@ extern "C" int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, 
     p->n_quads = n_quads;
     p->n_blocks = n_blocks;
     p->n_pairs = total_pairs;
-    rc = p->quads.alloc((size_t)n_quads);
-    if (!rc) rc = p->list.alloc((size_t)nnz);
     RingTables& sh = p->shares;
     sh.total = 0;
     for (int c = 0; c < kRingClasses; ++c) {
         sh.of[c] = RingShares{sms * ring_ctas(c + 1) * kRingWarps, sh.total, 0u, 0u};
         sh.total += sh.of[c].warps + 1;
     }
-    if (!rc) rc = p->ids.alloc((size_t)n_quads * 32 + sh.total);
-    int* const starts = p->ids.p + (size_t)n_quads * 32;
-    p->starts = starts;
+    p->device = dev;
+    const size_t quad_bytes = (size_t)n_quads * sizeof(SddmmQuad), id_bytes = (size_t)n_quads * 32 * sizeof(int);
+    const size_t start_bytes = (size_t)sh.total * sizeof(int);
+    if ((rc = pool_alloc(&p->block, quad_bytes + id_bytes + start_bytes + (size_t)nnz * sizeof(unsigned), st))) return fail(rc);
+    unsigned char* at = (unsigned char*)p->block;
+    p->quads = (SddmmQuad*)at; at += quad_bytes;
+    p->ids = (int*)at; at += id_bytes;
+    int* const starts = (int*)at;
+    p->starts = starts; at += start_bytes;
+    p->list = (unsigned*)at;
     unsigned *cost, *cost_before;
-    if (!rc) rc = ts.get((size_t)n_quads + 1, &cost);
+    rc = ts.get((size_t)n_quads + 1, &cost);
     if (!rc) rc = ts.get((size_t)n_quads + 1, &cost_before);
     if (rc) return fail(rc);
-    ksp_columns<<<grid(nnz), 256, 0, st>>>(key, pair_idx, head, first_pair, quad_off, nnz, p->ids.p, begin);
+    ksp_columns<<<grid(nnz), 256, 0, st>>>(key, pair_idx, head, first_pair, quad_off, nnz, p->ids, begin);
     ksp_quads<<<(unsigned)ceil_div(n_quads, 8), 256, 0, st>>>(key, ent, pair_idx, first_pair, begin, rowptr, n_rows, (int)nnz, n_quads,
-                                                              p->quads.p, p->ids.p, p->list.p, cost, d_err);
+                                                              p->quads, p->ids, p->list, cost, d_err);
     e = cub::DeviceScan::ExclusiveSum(tmp, bytes, cost, cost_before, n_quads + 1, st);
     if (e != cudaSuccess) return fail((int)e);
     ksp_shares<<<grid(sh.total), 256, 0, st>>>(cost_before, n_quads, sh, starts, (unsigned*)d_err + 2);
@@ -785,7 +798,7 @@ int launch_ring(const trs_sddmm_plan* p, const Operands& o, void* out, int K, cu
     const bool table = p->n_quads / 2 >= sh.warps && sh.worst_cost + sh.worst_cost / 8 < sh.worst;
     const int per_warp = ceil_div(p->n_quads, sh.warps);
     const int warps = table ? sh.warps : ceil_div(p->n_quads, per_warp);
-    kernel<<<ceil_div(warps, kRingWarps), 32 * kRingWarps, R::SMEM, st>>>(p->quads.p, p->ids.p, p->list.p, table ? p->starts + sh.offset : nullptr,
+    kernel<<<ceil_div(warps, kRingWarps), 32 * kRingWarps, R::SMEM, st>>>(p->quads, p->ids, p->list, table ? p->starts + sh.offset : nullptr,
                                                                         p->n_quads, per_warp, o.X, o.Y, out, p->n_rows, (K + 7) / 8, o.ld / 8);
     TRS_LAUNCH_CHECK();
     return TRS_OK;
