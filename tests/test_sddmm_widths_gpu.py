@@ -189,3 +189,32 @@ def test_row_pointer_ends():
     [t.start() for t in threads]
     [t.join() for t in threads]
     assert not failed
+
+
+def _runtime():
+    """The CUDA runtime that the library and torch share: what one of them leaves as a thread's last error, the other finds."""
+    import ctypes
+    return ctypes.CDLL("libcudart.so.12")
+
+
+def test_refused_under_capture():
+    """A one-use product under capture is an error (its row pointers cannot be looked at); the error is that call's and is not
+    found by a later launch."""
+    rp, col = (t.cuda() for t in _pattern("rmat"))
+    X = torch.randn(1024, 64, generator=torch.Generator().manual_seed(3)).half().cuda()
+    want = sddmm(rp, col, X, X)
+    out = torch.zeros_like(want)
+    for _ in range(3):
+        with pytest.raises(TrsError) as e:
+            with torch.cuda.graph(torch.cuda.CUDAGraph()):
+                try:
+                    sddmm(rp, col, X, X, out=out)
+                finally:
+                    left = _runtime().cudaPeekAtLastError()
+        assert e.value.code == 900 and left == 0   # cudaErrorStreamCaptureUnsupported
+        assert torch.equal(sddmm(rp, col, X, X), want)
+        with pytest.raises(TrsError) as e:
+            sddmm(rp + 1, col, X, X)
+        assert e.value.code == -3
+    torch.cuda.synchronize()
+    assert not out.any()

@@ -11,10 +11,14 @@
 
 #include "trspmm.h"
 
+// An error that a call returns does not stay the thread's last one: the check behind a later launch would return it again.
 #define TRS_CUDA(expr)                                     \
     do {                                                   \
         cudaError_t _e = (expr);                           \
-        if (_e != cudaSuccess) return (int)_e;             \
+        if (_e != cudaSuccess) {                           \
+            (void)cudaGetLastError();                      \
+            return (int)_e;                                \
+        }                                                  \
     } while (0)
 
 #define TRS_LAUNCH_CHECK()                                 \
@@ -137,8 +141,8 @@ struct DevBuf {
             return p ? 0 : TRS_E_WORKSPACE;
         }
         owned = true;
-        cudaError_t e = cudaMalloc((void**)&p, count * sizeof(T));
-        return e == cudaSuccess ? 0 : (int)e;
+        TRS_CUDA(cudaMalloc((void**)&p, count * sizeof(T)));
+        return 0;
     }
     void release() {
         if (p && owned) cudaFree(p);

@@ -694,8 +694,8 @@ struct Bag {
     template <class T>
     int get(size_t n, T** out) {
         void* d = nullptr;
-        cudaError_t e = cudaMalloc(&d, (n ? n : 1) * sizeof(T));
-        if (e != cudaSuccess) { *out = nullptr; return (int)e; }
+        *out = nullptr;
+        TRS_CUDA(cudaMalloc(&d, (n ? n : 1) * sizeof(T)));
         ptrs.push_back(d);
         *out = (T*)d;
         return 0;

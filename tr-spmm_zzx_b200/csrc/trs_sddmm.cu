@@ -843,14 +843,14 @@ void give_ends(const EndsWord& w) {
     std::lock_guard<std::mutex> lock(g_ends_mutex);
     g_ends.push_back(w);
 }
-// Until the device has written the word; an error of the stream (a capture among them) ends the wait.
+// Until the device has written the word; an error of the stream ends the wait.
 cudaError_t wait_for_ends(const EndsWord& w, cudaStream_t st) {
     for (unsigned i = 1; !w.p[2]; ++i) {
         if (i % 4096 != 0) continue;
         const cudaError_t e = cudaStreamQuery(st);
-        if (e == cudaErrorNotReady) (void)cudaGetLastError();   // not an error of a later launch
-        else if (e != cudaSuccess) return e;
-        else if (!w.p[2]) return cudaErrorUnknown;              // all done, and nothing was written
+        if (e != cudaSuccess) (void)cudaGetLastError();   // not an error of a later launch
+        if (e != cudaSuccess && e != cudaErrorNotReady) return e;
+        if (e == cudaSuccess && !w.p[2]) return cudaErrorUnknown;   // all done, and nothing was written
     }
     std::atomic_thread_fence(std::memory_order_acquire);
     return cudaSuccess;
@@ -897,6 +897,11 @@ extern "C" int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_ha
     // The ends of rowptr decide whether this is an error, and only the device has them.  The product's own kernel looks at
     // them and passes them on as it begins; the host waits for that, after earlier work of the stream, and for nothing else.  (A kernel
     // of their own before the product took 3 of 28 us: uniform 50 021 rows, K = 96.)
+    // A graph has no row pointers to look at when it is captured: refused before anything is queued, so that nothing is
+    // left that could write the words later.
+    cudaStreamCaptureStatus capture;
+    TRS_CUDA(cudaStreamIsCapturing(st, &capture));
+    if (capture != cudaStreamCaptureStatusNone) return (int)cudaErrorStreamCaptureUnsupported;
     EndsWord ends;
     int rc = take_ends(&ends);
     if (rc) return rc;
