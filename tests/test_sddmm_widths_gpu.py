@@ -218,3 +218,25 @@ def test_refused_under_capture():
         assert e.value.code == -3
     torch.cuda.synchronize()
     assert not out.any()
+
+
+def test_error_of_an_earlier_call():
+    """An error that another call left with the thread is not the product's: it runs, behind work that takes a while, and the calls
+    after it get their own row pointers."""
+    rp, col = (t.cuda() for t in _pattern("rmat"))
+    X = torch.randn(1024, 64, generator=torch.Generator().manual_seed(4)).half().cuda()
+    want, out = sddmm(rp, col, X, X), torch.zeros(col.numel(), dtype=torch.float16, device="cuda")
+    stream = torch.cuda.Stream()
+    torch.cuda.synchronize()
+    for _ in range(20):
+        with torch.cuda.stream(stream):
+            torch.cuda._sleep(1000000)
+            assert _runtime().cudaSetDevice(4096) == 101   # cudaErrorInvalidDevice, now the thread's last error
+            sddmm(rp, col, X, X, out=out)
+        with pytest.raises(TrsError) as e:
+            sddmm(rp + 1, col, X, X)
+        assert e.value.code == -3
+        stream.synchronize()
+        assert torch.equal(out, want)
+        out.zero_()
+        torch.cuda.synchronize()

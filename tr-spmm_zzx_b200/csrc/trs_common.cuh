@@ -200,6 +200,11 @@ int launch_behind(void (*kernel)(Params...), dim3 grid, int threads, size_t smem
     TRS_CUDA(cudaLaunchKernelEx(&cfg, kernel, Params(args)...));
     return TRS_OK;
 }
+// A launch whose error is its own: cudaGetLastError behind one also returns what an earlier call left with the thread.
+template <class... Params, class... Args>
+int launch(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
+    return launch_behind(kernel, grid, threads, smem, st, false, args...);
+}
 
 // D(16x8,f32) += A(16x16 with 2:4 sparsity, stored 16x8 f16) * B(16x8 f16).
 // `meta`: bits 4c..4c+3 = the two kept positions (p0 | p1<<2, p0<p1) of 4-column chunk c for

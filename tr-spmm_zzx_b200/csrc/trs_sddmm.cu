@@ -761,27 +761,25 @@ int sm_count() {
     return n > 0 ? n : 1;
 }
 
-// `ends`: three words of pinned memory for publish_ends, or null
+// `ends`: three words of pinned memory for publish_ends, or null.  An error is the launch's own, not one that an earlier call left
+// with the thread: it says that nothing will write the words.
 int launch_entries(const int32_t* rowptr, const int32_t* col, const Operands& o, void* out, int out_f32, int n_rows, int n_cols,
                    int K, int* ends, cudaStream_t st) {
     if (o.ld == 0) {
-        k_sddmm_plain<<<sm_count() * 8, 256, 0, st>>>(rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K);
-        TRS_LAUNCH_CHECK();
-        if (ends) k_sddmm_ends<<<1, 1, 0, st>>>(rowptr, n_rows, ends);
-        TRS_LAUNCH_CHECK();
-        return TRS_OK;
+        const int rc = launch(k_sddmm_plain, dim3(sm_count() * 8), 256, 0, st, rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K);
+        return rc || !ends ? rc : launch(k_sddmm_ends, dim3(1), 1, 0, st, rowptr, n_rows, ends);
     }
-    auto go = [&](auto kernel, int ctas) { kernel<<<sm_count() * ctas, 32 * kEntryWarps, 0, st>>>(rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K, o.ld, ends); };
-    if (K == 32) go(k_sddmm<1, true>, entry_ctas(1));
-    else if (K < 32) go(k_sddmm<1, false>, entry_ctas(1));
-    else if (K == 64) go(k_sddmm<2, true>, entry_ctas(2));
-    else if (K < 64) go(k_sddmm<2, false>, entry_ctas(2));
-    else if (K == 96) go(k_sddmm<3, true>, entry_ctas(3));
-    else if (K < 96) go(k_sddmm<3, false>, entry_ctas(3));
-    else if (K == 128) go(k_sddmm<4, true>, entry_ctas(4));
-    else go(k_sddmm<4, false>, entry_ctas(4));
-    TRS_LAUNCH_CHECK();
-    return TRS_OK;
+    auto go = [&](auto kernel, int ctas) {
+        return launch(kernel, dim3(sm_count() * ctas), 32 * kEntryWarps, 0, st, rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K, o.ld, ends);
+    };
+    if (K == 32) return go(k_sddmm<1, true>, entry_ctas(1));
+    if (K < 32) return go(k_sddmm<1, false>, entry_ctas(1));
+    if (K == 64) return go(k_sddmm<2, true>, entry_ctas(2));
+    if (K < 64) return go(k_sddmm<2, false>, entry_ctas(2));
+    if (K == 96) return go(k_sddmm<3, true>, entry_ctas(3));
+    if (K < 96) return go(k_sddmm<3, false>, entry_ctas(3));
+    if (K == 128) return go(k_sddmm<4, true>, entry_ctas(4));
+    return go(k_sddmm<4, false>, entry_ctas(4));
 }
 
 template <int KCH, bool TAIL, bool F32>
@@ -910,10 +908,9 @@ extern "C" int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_ha
         rc = o.prepare(X, Y, n_rows, n_cols, K, st);
         if (!rc) rc = launch_entries(rowptr, col, o, out, 0, n_rows, n_cols, K, (int*)ends.p, st);
     } else {
-        k_sddmm_ends<<<1, 1, 0, st>>>(rowptr, n_rows, (int*)ends.p);
-        rc = (int)cudaGetLastError();
+        rc = launch(k_sddmm_ends, dim3(1), 1, 0, st, rowptr, n_rows, (int*)ends.p);
     }
-    if (rc) {   // nothing that writes to the words is queued
+    if (rc) {   // the kernel that writes the words was refused, or not asked for
         give_ends(ends);
         return rc;
     }
