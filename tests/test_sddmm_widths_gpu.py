@@ -240,3 +240,41 @@ def test_error_of_an_earlier_call():
         assert torch.equal(out, want)
         out.zero_()
         torch.cuda.synchronize()
+
+
+def test_no_memory_for_copies_and_no_wait():
+    """The product without copies tells the row pointers' ends as it begins as well: the call does not wait for its end."""
+    import time
+    from trspmm import _lib
+    n, K = 1 << 20, 47
+    rp = torch.arange(n + 1, dtype=torch.int32, device="cuda") * 24
+    col = torch.randint(0, n, (24 * n,), device="cuda", dtype=torch.int32)
+    X = torch.randn(n, K, device="cuda", dtype=torch.float16)
+    out = torch.empty(col.numel(), dtype=torch.float16, device="cuda")
+    sddmm(rp, col, X, X, out=out)
+    want = out.clone()
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    _lib.check(_lib.load().trs_pool_trim())
+    hog = [torch.empty(torch.cuda.mem_get_info()[0] - (64 << 20), dtype=torch.uint8, device="cuda")]
+    while True:
+        try:
+            hog.append(torch.empty(4 << 20, dtype=torch.uint8, device="cuda"))
+        except torch.OutOfMemoryError:
+            break
+    try:
+        times = []
+        for _ in range(5):
+            out.zero_()
+            torch.cuda.synchronize()
+            t = [time.perf_counter()]
+            sddmm(rp, col, X, X, out=out)
+            t.append(time.perf_counter())
+            torch.cuda.synchronize()
+            t.append(time.perf_counter())
+            times.append((t[1] - t[0]) / (t[2] - t[0]))
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert float((out.float() - want.float()).abs().max()) <= 2e-3 * float(want.abs().max())
+    assert min(times) < 0.5, times   # a tenth; all of it where the call waits for the product's end

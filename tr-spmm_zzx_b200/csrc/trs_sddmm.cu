@@ -152,7 +152,8 @@ __global__ void __launch_bounds__(32 * kEntryWarps, entry_ctas(KCH)) k_sddmm(con
 // The same product on rows of any alignment, a warp per entry, where there is no memory for copies of X and Y.
 __global__ void __launch_bounds__(256) k_sddmm_plain(const int* __restrict__ rowptr, const int* __restrict__ col,
                                                      const __half* __restrict__ X, const __half* __restrict__ Y,
-                                                     void* __restrict__ out, int out_f32, int n_rows, int n_cols, int K) {
+                                                     void* __restrict__ out, int out_f32, int n_rows, int n_cols, int K, int* ends) {
+    if (ends && blockIdx.x == 0 && threadIdx.x == 0) publish_ends(rowptr, n_rows, ends);
     const int lane = threadIdx.x & 31, nnz = rowptr[0] == 0 ? rowptr[n_rows] : 0;
     const long long step = (long long)gridDim.x * 8;
     for (long long e = (long long)blockIdx.x * 8 + (threadIdx.x >> 5); e < nnz; e += step) {
@@ -765,10 +766,8 @@ int sm_count() {
 // with the thread: it says that nothing will write the words.
 int launch_entries(const int32_t* rowptr, const int32_t* col, const Operands& o, void* out, int out_f32, int n_rows, int n_cols,
                    int K, int* ends, cudaStream_t st) {
-    if (o.ld == 0) {
-        const int rc = launch(k_sddmm_plain, dim3(sm_count() * 8), 256, 0, st, rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K);
-        return rc || !ends ? rc : launch(k_sddmm_ends, dim3(1), 1, 0, st, rowptr, n_rows, ends);
-    }
+    if (o.ld == 0)
+        return launch(k_sddmm_plain, dim3(sm_count() * 8), 256, 0, st, rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K, ends);
     auto go = [&](auto kernel, int ctas) {
         return launch(kernel, dim3(sm_count() * ctas), 32 * kEntryWarps, 0, st, rowptr, col, o.X, o.Y, out, out_f32, n_rows, n_cols, K, o.ld, ends);
     };
