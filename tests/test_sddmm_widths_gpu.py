@@ -278,3 +278,21 @@ def test_no_memory_for_copies_and_no_wait():
         torch.cuda.empty_cache()
     assert float((out.float() - want.float()).abs().max()) <= 2e-3 * float(want.abs().max())
     assert min(times) < 0.5, times   # a tenth; all of it where the call waits for the product's end
+
+
+def test_wait_behind_a_long_queue():
+    """A call that waits for earlier work of its stream leaves the core to others, and is not late when the work ends."""
+    import time
+    rp, col = (t.cuda() for t in _pattern("rmat"))
+    X = torch.randn(1024, 64, generator=torch.Generator().manual_seed(5)).half().cuda()
+    want = sddmm(rp, col, X, X)
+    torch.cuda.synchronize()
+    for cycles in (100_000, 3_000_000, 500_000_000):   # 50 us, 2 ms, 0.3 s
+        done = torch.cuda.Event()
+        wall, cpu = time.perf_counter(), time.thread_time()
+        torch.cuda._sleep(cycles)
+        done.record()
+        got = sddmm(rp, col, X, X)
+        wall, cpu = time.perf_counter() - wall, time.thread_time() - cpu
+        assert done.query() and torch.equal(got, want)
+    assert wall > 0.1 and cpu < 0.25 * wall, (wall, cpu)
