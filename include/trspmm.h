@@ -354,6 +354,10 @@ int trs_sddmm_plan_run_ex(const trs_sddmm_plan* plan, const trs_half* X, const t
                           int out_dtype, void* stream);
 /* distinct (window, column) pairs and 8-column blocks of the plan */
 int trs_sddmm_plan_info(const trs_sddmm_plan* plan, long long* n_pairs, long long* n_blocks);
+/* How a product of width K <= 256 is divided: the warps of its wave, the largest share of the work (in the plan's own
+ * units) if all take equal numbers of quads and if all take equal cost (0: the plan did not look, the pattern is too small),
+ * and whether it goes by cost. */
+int trs_sddmm_plan_shares(const trs_sddmm_plan* plan, int K, int* warps, unsigned* by_number, unsigned* by_cost, int* table);
 int trs_sddmm_plan_destroy(trs_sddmm_plan* plan);
 
 #ifdef __cplusplus

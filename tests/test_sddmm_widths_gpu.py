@@ -296,3 +296,35 @@ def test_wait_behind_a_long_queue():
         wall, cpu = time.perf_counter() - wall, time.thread_time() - cpu
         assert done.query() and torch.equal(got, want)
     assert wall > 0.1 and cpu < 0.25 * wall, (wall, cpu)
+
+
+def _shares(plan, K):
+    """(warps, largest share by number of quads, by cost, goes by cost) of a plan at width K."""
+    import ctypes
+    warps, table = ctypes.c_int(), ctypes.c_int()
+    number, cost = ctypes.c_uint(), ctypes.c_uint()
+    assert plan.lib.trs_sddmm_plan_shares(plan._handle, K, ctypes.byref(warps), ctypes.byref(number), ctypes.byref(cost),
+                                          ctypes.byref(table)) == 0
+    return warps.value, number.value, cost.value, bool(table.value)
+
+
+def test_shares_are_looked_at_where_they_can_be_used():
+    """Patterns of one quad a window, around the number of quads from which the smallest wave gets two a warp: the shares of a
+    wave are those of its quads (16 each: one block, up to 32 entries, a new window), and not looked at below."""
+    sms = torch.cuda.get_device_properties(0).multi_processor_count
+    least = 12 * sms
+    for n_quads in (1, 2 * least - 1, 2 * least, 2 * least + 1, 40 * sms, 2 * 32 * sms):
+        rp = torch.arange(16 * n_quads + 1, dtype=torch.int32, device="cuda")
+        col = (torch.arange(16 * n_quads, dtype=torch.int32, device="cuda") // 2) % 8   # 16 entries, 8 columns a window
+        plan = SddmmPlan(rp, col, 8)
+        for K in (24, 64, 96, 128, 160, 192, 224, 256):
+            warps, number, cost, table = _shares(plan, K)
+            assert warps % (4 * sms) == 0 and warps >= least and not table
+            if n_quads // 2 < warps:
+                assert (number, cost) == (0, 0)
+            else:
+                assert number == 16 * -(-n_quads // warps) and cost in (number, number - 16, number + 16)
+        X = torch.randn(16 * n_quads, 64, device="cuda").half()
+        out, want = plan.run(X, X[:8].contiguous()).float(), (X.float() * X.float()[col.long()]).sum(1)
+        # fp16 results (2^-11) of fp32 sums, whose order differs by less than that
+        assert float((out - want).abs().max()) <= 2e-3 * float(want.abs().max())

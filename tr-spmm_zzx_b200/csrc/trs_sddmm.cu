@@ -8,6 +8,7 @@
 // lane (g, t) takes bytes [64 c + 16 t, +16) of its row for every 32-feature chunk c - the same feature
 // positions on both sides, which is all the MMA needs (the order of k inside a chunk is free).
 // Rows that do not start on 16-byte boundaries are copied to padded ones first.
+#include <limits.h>
 #include <stdlib.h>
 #include <string.h>
 #if defined(__SSE2__)
@@ -318,18 +319,28 @@ __device__ __forceinline__ int first_quad(const unsigned* __restrict__ cost_befo
     }
     return lo;
 }
+// A wave that gets less than two quads a warp has no table; without any such wave (fewer than 24 quads per SM) the costs are not
+// summed either.
+__host__ __device__ __forceinline__ bool may_have_table(int n_quads, int warps) { return n_quads / 2 >= warps; }
 __global__ void ksp_shares(const unsigned* __restrict__ cost_before, int n_quads, RingTables s, int* __restrict__ starts,
                            unsigned* __restrict__ worst /* [kRingClasses][2] */) {
-    const int x = blockIdx.x * blockDim.x + threadIdx.x;
-    if (x >= s.total) return;
-    int c = kRingClasses - 1;
-    while (x < s.of[c].offset) --c;
-    const int i = x - s.of[c].offset, warps = s.of[c].warps, per = (n_quads + warps - 1) / warps;
-    const int at = first_quad(cost_before, n_quads, i, warps);
-    starts[x] = at;
-    if (i == warps) return;
-    atomicMax(worst + 2 * c, cost_before[min((long long)(i + 1) * per, (long long)n_quads)] - cost_before[min((long long)i * per, (long long)n_quads)]);
-    atomicMax(worst + 2 * c + 1, cost_before[first_quad(cost_before, n_quads, i + 1, warps)] - cost_before[at]);
+    const int c = blockIdx.y, i = blockIdx.x * blockDim.x + threadIdx.x, warps = s.of[c].warps;
+    if (!may_have_table(n_quads, warps)) return;
+    unsigned number = 0, cost = 0;
+    if (i <= warps) {
+        const int at = first_quad(cost_before, n_quads, i, warps);
+        starts[s.of[c].offset + i] = at;
+        if (i < warps) {
+            const long long per = (n_quads + warps - 1) / warps, end = min((i + 1) * per, (long long)n_quads);
+            number = cost_before[end] - cost_before[min(i * per, end)];
+            cost = cost_before[first_quad(cost_before, n_quads, i + 1, warps)] - cost_before[at];
+        }
+    }
+    number = __reduce_max_sync(0xffffffffu, number);
+    cost = __reduce_max_sync(0xffffffffu, cost);
+    if ((threadIdx.x & 31) != 0) return;
+    atomicMax(worst + 2 * c, number);
+    atomicMax(worst + 2 * c + 1, cost);
 }
 
 // One warp per quad: header, repeated columns, and the entries in CSR order, placed by row masks.
@@ -379,8 +390,10 @@ __global__ void ksp_quads(const unsigned long long* __restrict__ key, const int*
     if (lane >= cols && lane < blocks * 8) ids[(size_t)q * 32 + lane] = ids[(size_t)q * 32];
     if (lane == 0) {
         quads[q] = SddmmQuad{w, e0, (e - b) << 3 | blocks, b};
-        cost[q] = quad_cost(blocks, e - b, pair0 == first_pair[w]);
-        if (q + 1 == n_quads) cost[n_quads] = 0;
+        if (cost) {
+            cost[q] = quad_cost(blocks, e - b, pair0 == first_pair[w]);
+            if (q + 1 == n_quads) cost[n_quads] = 0;
+        }
     }
 }
 
@@ -566,7 +579,12 @@ struct trs_sddmm_plan {
     int* ids = nullptr;           // [quads][32]
     unsigned* list = nullptr;     // [nnz]
     trs::RingTables shares;
-    const int* starts = nullptr;  // the tables, behind the ids
+    const int* starts = nullptr;  // the tables, behind the ids; null where no wave can have one
+    // whether a wave of the kernel for `kch` chunks goes by its table
+    bool by_table(int kch) const {
+        const trs::RingShares& sh = shares.of[kch - 1];
+        return starts && trs::may_have_table(n_quads, sh.warps) && sh.worst_cost + sh.worst_cost / 8 < sh.worst;
+    }
 };
 
 extern "C" int trs_sddmm_plan_destroy(trs_sddmm_plan* p) {
@@ -679,30 +697,36 @@ extern "C" int trs_sddmm_plan_create(const int32_t* rowptr, const int32_t* col, 
     p->n_pairs = total_pairs;
     RingTables& sh = p->shares;
     sh.total = 0;
+    int least = INT_MAX, most = 0;   // warps of a wave
     for (int c = 0; c < kRingClasses; ++c) {
         sh.of[c] = RingShares{sms * ring_ctas(c + 1) * kRingWarps, sh.total, 0u, 0u};
         sh.total += sh.of[c].warps + 1;
+        least = std::min(least, sh.of[c].warps);
+        most = std::max(most, sh.of[c].warps);
     }
+    const bool tables = may_have_table(n_quads, least);
     p->device = dev;
     const size_t quad_bytes = (size_t)n_quads * sizeof(SddmmQuad), id_bytes = (size_t)n_quads * 32 * sizeof(int);
-    const size_t start_bytes = (size_t)sh.total * sizeof(int);
+    const size_t start_bytes = tables ? (size_t)sh.total * sizeof(int) : 0;
     if ((rc = pool_alloc(&p->block, quad_bytes + id_bytes + start_bytes + (size_t)nnz * sizeof(unsigned), st))) return fail(rc);
     unsigned char* at = (unsigned char*)p->block;
     p->quads = (SddmmQuad*)at; at += quad_bytes;
     p->ids = (int*)at; at += id_bytes;
     int* const starts = (int*)at;
-    p->starts = starts; at += start_bytes;
+    if (tables) p->starts = starts;
+    at += start_bytes;
     p->list = (unsigned*)at;
-    unsigned *cost, *cost_before;
-    rc = ts.get((size_t)n_quads + 1, &cost);
-    if (!rc) rc = ts.get((size_t)n_quads + 1, &cost_before);
-    if (rc) return fail(rc);
+    unsigned *cost = nullptr, *cost_before = nullptr;
+    if (tables && (rc = ts.get((size_t)n_quads + 1, &cost))) return fail(rc);
+    if (tables && (rc = ts.get((size_t)n_quads + 1, &cost_before))) return fail(rc);
     ksp_columns<<<grid(nnz), 256, 0, st>>>(key, pair_idx, head, first_pair, quad_off, nnz, p->ids, begin);
     ksp_quads<<<(unsigned)ceil_div(n_quads, 8), 256, 0, st>>>(key, ent, pair_idx, first_pair, begin, rowptr, n_rows, (int)nnz, n_quads,
                                                               p->quads, p->ids, p->list, cost, d_err);
-    e = cub::DeviceScan::ExclusiveSum(tmp, bytes, cost, cost_before, n_quads + 1, st);
-    if (e != cudaSuccess) return fail((int)e);
-    ksp_shares<<<grid(sh.total), 256, 0, st>>>(cost_before, n_quads, sh, starts, (unsigned*)d_err + 2);
+    if (tables) {
+        e = cub::DeviceScan::ExclusiveSum(tmp, bytes, cost, cost_before, n_quads + 1, st);
+        if (e != cudaSuccess) return fail((int)e);
+        ksp_shares<<<dim3(grid(most + 1), kRingClasses), 256, 0, st>>>(cost_before, n_quads, sh, starts, (unsigned*)d_err + 2);
+    }
     int back[2 + 2 * kRingClasses];
     e = cudaMemcpyAsync(back, d_err, sizeof(back), cudaMemcpyDeviceToHost, st);
     if (e == cudaSuccess) e = cudaStreamSynchronize(st);
@@ -721,6 +745,17 @@ extern "C" int trs_sddmm_plan_info(const trs_sddmm_plan* p, long long* n_pairs, 
     if (!p) return TRS_E_ARG;
     if (n_pairs) *n_pairs = p->n_pairs;
     if (n_blocks) *n_blocks = p->n_blocks;
+    return TRS_OK;
+}
+
+extern "C" int trs_sddmm_plan_shares(const trs_sddmm_plan* p, int K, int* warps, unsigned* by_number, unsigned* by_cost, int* table) {
+    const int kch = (K + 31) / 32;
+    if (!p || K <= 0 || kch > trs::kRingClasses) return TRS_E_ARG;
+    const trs::RingShares none{0, 0, 0u, 0u}, &sh = p->nnz > 0 ? p->shares.of[kch - 1] : none;
+    if (warps) *warps = sh.warps;
+    if (by_number) *by_number = sh.worst;
+    if (by_cost) *by_cost = sh.worst_cost;
+    if (table) *table = p->nnz > 0 && p->by_table(kch);
     return TRS_OK;
 }
 
@@ -799,7 +834,7 @@ int launch_ring(const trs_sddmm_plan* p, const Operands& o, void* out, int K, cu
         if (dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
     }
     const RingShares& sh = p->shares.of[KCH - 1];
-    const bool table = p->n_quads / 2 >= sh.warps && sh.worst_cost + sh.worst_cost / 8 < sh.worst;
+    const bool table = p->by_table(KCH);
     const int per_warp = ceil_div(p->n_quads, sh.warps);
     const int warps = table ? sh.warps : ceil_div(p->n_quads, per_warp);
     kernel<<<ceil_div(warps, kRingWarps), 32 * kRingWarps, R::SMEM, st>>>(p->quads, p->ids, p->list, table ? p->starts + sh.offset : nullptr,

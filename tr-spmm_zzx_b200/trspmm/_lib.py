@@ -113,8 +113,10 @@ def load():
     lib.trs_sddmm_plan_run.argtypes = [vp, vp, vp, vp, i32, vp]
     lib.trs_sddmm_plan_run_ex.argtypes = [vp, vp, vp, vp, i32, i32, vp]
     lib.trs_sddmm_plan_info.argtypes = [vp, C.POINTER(C.c_longlong), C.POINTER(C.c_longlong)]
+    lib.trs_sddmm_plan_shares.argtypes = [vp, i32, C.POINTER(i32), C.POINTER(C.c_uint), C.POINTER(C.c_uint), C.POINTER(i32)]
     lib.trs_sddmm_plan_destroy.argtypes = [vp]
-    for name in ("trs_sddmm_plan_create", "trs_sddmm_plan_run", "trs_sddmm_plan_run_ex", "trs_sddmm_plan_info", "trs_sddmm_plan_destroy"):
+    for name in ("trs_sddmm_plan_create", "trs_sddmm_plan_run", "trs_sddmm_plan_run_ex", "trs_sddmm_plan_info", "trs_sddmm_plan_shares",
+                 "trs_sddmm_plan_destroy"):
         getattr(lib, name).restype = i32
     lib.trs_build_create.argtypes = [vp, vp, vp, i32, C.POINTER(TrsBuildConfig), vp, C.POINTER(vp)]
     lib.trs_copy_to_host.argtypes = [i32, C.POINTER(vp), C.POINTER(vp), C.POINTER(sz), vp]
