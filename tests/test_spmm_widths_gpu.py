@@ -183,3 +183,27 @@ def test_first_column_ids(F, per_row):
     ref = torch.sparse_csr_tensor(rp.long(), col.long(), val.half().double(), (n, n)) @ B.double()
     # fp32 sums of exact products of fp16 values
     assert float((out - ref).abs().max()) <= 2e-5 * float(ref.abs().max())
+
+
+@pytest.mark.parametrize("windows", [1 << 16, 1 << 19])
+def test_plan_without_room_for_first_column_ids(windows):
+    """A plan fits where its arrays fit: the ids beside the items (512 bytes an item, more than the rest of this plan) are left out,
+    and the results are the same."""
+    n, g = 16 * windows, torch.Generator(device="cuda").manual_seed(1)
+    rp = torch.arange(n + 1, dtype=torch.int32, device="cuda") * 3
+    col = torch.randint(0, 1 << 12, (n, 3), generator=g, device="cuda") + (torch.arange(3, device="cuda") << 12)
+    fmt = build_format(rp, col.flatten().to(torch.int32), torch.randn(3 * n, generator=g, device="cuda"))[0]
+    B = torch.randn(3 << 12, 64, generator=g, device="cuda").half()
+    want = SpmmPlan(fmt, n, 3 << 12).run(B)
+    del rp, col
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    _lib.check(_lib.load().trs_pool_trim())
+    hog = torch.empty(torch.cuda.mem_get_info()[0] - 640 * windows, dtype=torch.uint8, device="cuda")
+    try:
+        plan = SpmmPlan(fmt, n, 3 << 12)
+    finally:
+        del hog
+        torch.cuda.empty_cache()
+    assert torch.equal(plan.run(B), want)
+    assert torch.equal(plan.run(B[:, :50].contiguous()), want[:, :50])

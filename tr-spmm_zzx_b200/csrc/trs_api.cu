@@ -186,7 +186,7 @@ class PlanThread {
     int rc_ = TRS_OK;
 
 public:
-    int start(const trs_format& dev, int m_rows, int k_cols, int window, cudaStream_t after, trs_spmm_plan** out) {
+    int start(const trs_format& dev, int m_rows, int k_cols, int window, bool first_ids, cudaStream_t after, trs_spmm_plan** out) {
         const int rc = take_side(&side_);
         if (rc) return rc;
         TRS_CUDA(cudaEventRecord(side_.ready, after));
@@ -194,7 +194,7 @@ public:
         try {
             t_ = std::thread([=] {
                 const cudaError_t e = cudaSetDevice(side_.device);
-                rc_ = e != cudaSuccess ? (int)e : trs_spmm_plan_create(&dev, m_rows, k_cols, window, 1, side_.st, out);
+                rc_ = e != cudaSuccess ? (int)e : spmm_plan_create(&dev, m_rows, k_cols, window, 1, first_ids, side_.st, out);
             });
         } catch (const std::system_error&) {   // no thread to be had: the caller makes the plan itself
         }
@@ -344,7 +344,8 @@ int slot_init(trs_resident* h, int i) {
 
 int resident_finish_create(trs_resident* h, int mOri, int kOri, int window, int max_dimN) {
     h->m_rows = mOri; h->k_cols = kOri; h->max_dim = max_dimN; h->window = window;
-    int rc = trs_spmm_plan_create(&h->dev, mOri, kOri, window, 1, nullptr, &h->plan);
+    // (slabs of a wider product are 64 features wide)
+    int rc = spmm_plan_create(&h->dev, mOri, kOri, window, 1, max_dimN >= kFirstIdsFrom, nullptr, &h->plan);
     if (!rc) rc = trs_spmm_workspace_bytes(h->plan, max_dimN, &h->ws_bytes);
     if (!rc) rc = h->up.now<unsigned char>(h->ws_bytes, (unsigned char**)&h->d_ws);
     if (!rc) rc = slot_init(h, 0);  // the second slot is allocated by the first overlapping submit
@@ -637,10 +638,11 @@ extern "C" int trs_spmm_forward_host(const trs_format* host_format, const trs_ha
     // the plan needs the format only: it is made (some twenty small kernels and two read-backs) while the dense operand goes up
     {
         PlanThread maker;
-        if (rhs_bytes >= ((size_t)2 << 20)) rc = maker.start(dev, mOri, kOri, window, st, &plan.p);
+        const bool first_ids = dimN >= kFirstIdsFrom && dimN <= kFirstIdsTo;
+        if (rhs_bytes >= ((size_t)2 << 20)) rc = maker.start(dev, mOri, kOri, window, first_ids, st, &plan.p);
         const HostSegment in{(void*)rhs_host, d_rhs, rhs_bytes};
         if (!rc) rc = copy_to_device(&in, 1, st);
-        const int plan_rc = maker.started() ? maker.join() : (rc ? rc : trs_spmm_plan_create(&dev, mOri, kOri, window, 1, st, &plan.p));
+        const int plan_rc = maker.started() ? maker.join() : (rc ? rc : spmm_plan_create(&dev, mOri, kOri, window, 1, first_ids, st, &plan.p));
         if (rc || plan_rc) return rc ? rc : plan_rc;
     }
     size_t ws_bytes = 0;

@@ -240,6 +240,11 @@ int copy_to_host(const HostSegment* seg, int n, cudaStream_t st);
 int copy_to_device(const HostSegment* seg, int n, cudaStream_t st);
 void release_host_ring();
 
+// trs_spmm.cu: trs_spmm_plan_create for callers that know whether a width is to come that reads `first_ids` (49 to 64).
+constexpr int kFirstIdsFrom = 49, kFirstIdsTo = 64;
+int spmm_plan_create(const trs_format* dev_format, int m_rows, int k_cols, int window, int validate, bool first_ids, cudaStream_t st,
+                     trs_spmm_plan** out);
+
 // trs_spmm.cu: trs_spmm_run_windows for callers that cut one product into several runs.
 struct SpmmHow {
     int width = 0;   // the product's own width where `F` is a slab of it: what goes by the width goes by that

@@ -854,7 +854,7 @@ struct trs_spmm_plan {
     int per_sample = 1;
     std::vector<int> item_at, heavy_at, step_at;
     int* ids = nullptr;      // [steps + kIdSpare][16] column ids of the step stream
-    int* first_ids = nullptr;   // [fine items][kIdBlock][16] the first ones of the items in launch order
+    int* first_ids = nullptr;   // [fine items][kIdBlock][16] the first ones of the items in launch order, or null
     uint4* dense = nullptr;  // [dense steps][32] A tiles of the dense steps in fragment order
     int n_steps, sms;        // of all items; SMs of the device
 };
@@ -951,11 +951,25 @@ static int validate_on_device(const trs_format& f, int m_rows, int k_cols, int n
     return TRS_OK;
 }
 
+// First ids beside the items take 512 bytes an item.  Nobody is to miss that room: beyond 32 MB they are left out where they would be more
+// than a sixteenth of what the device has left (asking for that takes 60 us, a plan of 9000 rows 190), and no plan fails for want of them.
+static bool room_for_first_ids(size_t bytes) {
+    if (bytes <= (size_t)32 << 20) return true;
+    size_t left = 0, total = 0;
+    if (cudaMemGetInfo(&left, &total) != cudaSuccess) { (void)cudaGetLastError(); return false; }
+    return bytes <= left / 16;
+}
+
 // CSR value-count checks need the last prefix entry; done with the column range check so that a
 // short column array cannot be over-read: the caller states the lengths implicitly through the
 // prefix arrays, exactly as the reference does (mGCN_online.cpp:982-1042 copies numel() items).
 extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, int k_cols, int window, int validate,
-                                    void* stream, trs_spmm_plan** out_plan) try {
+                                    void* stream, trs_spmm_plan** out_plan) {
+    return spmm_plan_create(dev_format, m_rows, k_cols, window, validate, true, (cudaStream_t)stream, out_plan);
+}
+
+int trs::spmm_plan_create(const trs_format* dev_format, int m_rows, int k_cols, int window, int validate, bool first_ids,
+                          cudaStream_t st, trs_spmm_plan** out_plan) try {
     if (!dev_format || !out_plan) return TRS_E_ARG;
     *out_plan = nullptr;
     if (m_rows <= 0 || k_cols <= 0) return TRS_E_ARG;
@@ -973,7 +987,6 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
     int ndev = 0;
     if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) return TRS_E_NO_DEVICE;
 
-    cudaStream_t st = (cudaStream_t)stream;
     const int W = max(ceil_div(m_rows, window), f.num_windows);
     TempSpace ts;
     ts.st = st;
@@ -1046,14 +1059,34 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
         coarse.longest = info.coarse.longest;
     }
     const size_t ids_bytes = ((size_t)n_steps + kIdSpare) * 64, dense_bytes = (size_t)n_dense * 512;
-    // 512 bytes an item, so not where most have next to no steps
-    const size_t first_bytes = n_steps / 2 >= n_items ? (size_t)n_items * (kIdBlock * 64) : 0;
     const size_t items_bytes = ((size_t)2 * n_items + coarse.n_items) * sizeof(Item);
     const size_t heavy_bytes = ((size_t)n_heavy + coarse.n_heavy) * sizeof(Heavy);
     // the kernels read the packed values 8 bytes per lane; an array that does not allow that is copied
     const size_t packed_bytes = ((uintptr_t)f.s_packed_a & 7) != 0 ? (size_t)f.tiles * 256 : 0;
     auto fail = [&](int code) { trs_spmm_plan_destroy(p); return code; };
-    if ((rc = pool_alloc(&p->block, ids_bytes + first_bytes + dense_bytes + packed_bytes + items_bytes + heavy_bytes, st))) return fail(rc);
+    // the temporaries first: what the plan can do without comes last
+    int* open;
+    unsigned char *cls, *sort_tmp;
+    size_t sort_bytes = 0;
+    Item*& by_window = p->by_window;
+    auto sort = [&](void* t) {
+        return cub::DeviceRadixSort::SortPairs(t, sort_bytes, cls, cls + n_items, by_window, fine.items, n_items, 0, kClassBits, st);
+    };
+    rc = ts.get((size_t)2 * n_items, &cls);
+    if (!rc) rc = ts.get((size_t)W, &open);
+    if (rc) return fail(rc);
+    cudaError_t e = sort(nullptr);
+    if (e == cudaSuccess && (rc = ts.get(sort_bytes + 16, &sort_tmp))) return fail(rc);
+    const size_t needed = ids_bytes + dense_bytes + packed_bytes + items_bytes + heavy_bytes;
+    // 512 bytes an item, so not where most have next to no steps
+    size_t first_bytes = first_ids && n_steps / 2 >= n_items ? (size_t)n_items * (kIdBlock * 64) : 0;
+    if (!room_for_first_ids(first_bytes)) first_bytes = 0;
+    rc = pool_alloc(&p->block, needed + first_bytes, st);
+    if (rc == (int)cudaErrorMemoryAllocation && first_bytes > 0) {
+        first_bytes = 0;
+        rc = pool_alloc(&p->block, needed, st);
+    }
+    if (rc) return fail(rc);
     unsigned char* at = (unsigned char*)p->block;
     p->ids = (int*)at; at += ids_bytes;
     if (first_bytes) p->first_ids = (int*)at;
@@ -1064,21 +1097,9 @@ extern "C" int trs_spmm_plan_create(const trs_format* dev_format, int m_rows, in
         if (copied != cudaSuccess) return fail((int)copied);
         p->f.s_packed_a = (const uint32_t*)at; at += packed_bytes;
     }
-    p->by_window = (Item*)at; fine.items = p->by_window + n_items; coarse.items = fine.items + n_items; at += items_bytes;
+    by_window = (Item*)at; fine.items = by_window + n_items; coarse.items = fine.items + n_items; at += items_bytes;
     fine.heavy = (Heavy*)at; coarse.heavy = fine.heavy + n_heavy;
 
-    Item* const by_window = p->by_window;
-    int* open;
-    unsigned char *cls, *sort_tmp;
-    size_t sort_bytes = 0;
-    rc = ts.get((size_t)2 * n_items, &cls);
-    if (!rc) rc = ts.get((size_t)W, &open);
-    if (rc) return fail(rc);
-    auto sort = [&](void* t) {
-        return cub::DeviceRadixSort::SortPairs(t, sort_bytes, cls, cls + n_items, by_window, fine.items, n_items, 0, kClassBits, st);
-    };
-    cudaError_t e = sort(nullptr);
-    if (e == cudaSuccess && (rc = ts.get(sort_bytes + 16, &sort_tmp))) return fail(rc);
     if (e == cudaSuccess) e = cudaMemsetAsync(open, 0x7f, sizeof(int) * (size_t)W, st);
     if (e == cudaSuccess) {
         k_fill_items<<<grid(W), 256, 0, st>>>(f, W, off, by_window, fine.heavy);
