@@ -5,6 +5,7 @@ import torch
 
 from oracle import oracle as O
 from trspmm import TrsError, build_format, graphs
+from window_slices import compare_window, slice_window, window_segment
 
 pytestmark = pytest.mark.gpu
 
@@ -166,3 +167,23 @@ def test_scan_borders(windows):
     cols = torch.randint(0, 300, (rows.numel(),), generator=g)
     rp, col, _ = graphs.coo_to_csr(rows, cols, n, 300)
     _check(rp, col, torch.randn(col.numel(), generator=g))
+
+
+def _hub_windows(windows):
+    """Windows of 16 x 513 entries, more than a CTA sorts, over 600 columns."""
+    g = torch.Generator(device="cuda").manual_seed(windows)
+    n = 16 * windows
+    col = torch.cat([torch.rand(a.numel(), 600, generator=g, device="cuda").argsort(1)[:, :513].sort(1).values.to(torch.int32).flatten()
+                     for a in torch.arange(n).split(1 << 15)])
+    rp = torch.arange(n + 1, dtype=torch.int32, device="cuda") * 513
+    return rp, col, torch.randn(col.numel(), generator=g, device="cuda")
+
+
+@pytest.mark.parametrize("windows", [4607, 4608])
+def test_many_hub_windows(windows):
+    """As many hub windows as the one-CTA scan adds up, and one more."""
+    rp, col, val = _hub_windows(windows)
+    named = dict(zip(O.FORMAT_NAMES, build_format(rp, col, val)[0].arrays()))
+    rp = rp.cpu()
+    for w in (0, 1, 1023, 2500, windows - 2, windows - 1):
+        compare_window(window_segment(named, w), O.build_format(*slice_window(rp, col, val, w))[0], f"window {w}")

@@ -709,7 +709,7 @@ __device__ __forceinline__ int local_row(const int* __restrict__ rowptr, int n_r
 struct HubSizes {
     const int *rowptr, *sel;
     int n_rows, window, n;
-    __device__ __forceinline__ int operator()(int h) const {
+    __host__ __device__ __forceinline__ int operator()(int h) const {
         return h < n ? rowptr[min((long long)(sel[h] + 1) * window, (long long)n_rows)] - rowptr[(size_t)sel[h] * window] : 0;
     }
 };
@@ -2120,8 +2120,13 @@ int sort_hubs(trs_builder* B, const int* rowptr, const int* col, const float* va
     TRS_TRY(ts.get(E, &keys_b));
     TRS_TRY(ts.get(E, &place_a));
     TRS_TRY(ts.get(E, &place_b));
-    kb_scan_small<<<1, 1024, 0, st>>>(HubSizes{rowptr, sel, n, window, H}, ToArray<int>{off}, IntSum(), 0, H + 1, Publish{});
-    TRS_LAUNCH_CHECK();
+    const HubSizes size{rowptr, sel, n, window, H};
+    if (H + 1 <= kSmallScan) {
+        kb_scan_small<<<1, 1024, 0, st>>>(size, ToArray<int>{off}, IntSum(), 0, H + 1, Publish{});
+        TRS_LAUNCH_CHECK();
+    } else {
+        TRS_TRY(cub_.exclusive_scan(thrust::make_transform_iterator(thrust::counting_iterator<int>(0), size), off, IntSum(), 0, (long long)H + 1));
+    }
     const HubView hub{sel, off, H};
     kb_hub_keys<Key><<<grid_for(E), 256, 0, st>>>(rowptr, col, n, window, hub, E, col_bits, keys_a, place_a, d_info);
     TRS_LAUNCH_CHECK();
