@@ -2062,23 +2062,13 @@ struct Records {   // stages 1 - 3
     int* sel = nullptr;   // [kSortClasses + 1][W]
 };
 
-template <class Kernel>
-int allow_smem(Kernel kernel, int smem, std::atomic<unsigned long long>& done) {   // once per device and kernel
-    int dev = 0;
-    TRS_CUDA(cudaGetDevice(&dev));
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (smem <= 48 * 1024 || (dev < 64 && (done.load(std::memory_order_relaxed) & bit))) return 0;
-    TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    if (dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
-    return 0;
-}
 template <int T, class Key, int C>
 int sort_class_as(const InputInfo& info, const int* rowptr, const int* col, const float* val, const trs_builder* B, const Records& R,
                   InputInfo* d_info, cudaStream_t st) {
     constexpr int CAP = sort_cap(C), smem = (int)sizeof(typename WindowSort<T, CAP, Key>::Smem);
     auto kernel = kb_sort_window<T, CAP, Key>;
     static std::atomic<unsigned long long> done{0};
-    TRS_TRY(allow_smem(kernel, smem, done));
+    TRS_TRY(allow_smem(kernel, smem, false, done));
     kernel<<<info.windows[C], T, smem, st>>>(rowptr, col, val, B->n_rows, B->cfg.window, R.sel + (size_t)C * B->W, R.w, d_info);
     TRS_LAUNCH_CHECK();
     return 0;
@@ -2093,7 +2083,7 @@ int sort_class(const InputInfo& info, const int* rowptr, const int* col, const f
             constexpr int smem = (int)sizeof(typename S::Smem) * kSortWarps;
             auto kernel = kb_sort_warp<sort_cap(C) / 32>;
             static std::atomic<unsigned long long> done{0};
-            TRS_TRY(allow_smem(kernel, smem, done));
+            TRS_TRY(allow_smem(kernel, smem, false, done));
             kernel<<<ceil_div(info.windows[C], kSortWarps), 32 * kSortWarps, smem, st>>>(rowptr, col, val, B->n_rows, B->cfg.window,
                                                                                         R.sel + (size_t)C * B->W, info.windows[C], R.w, d_info);
             TRS_LAUNCH_CHECK();

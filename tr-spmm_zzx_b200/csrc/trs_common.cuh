@@ -6,6 +6,7 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
 #include <exception>
 #include <new>
 
@@ -204,6 +205,21 @@ int launch_behind(void (*kernel)(Params...), dim3 grid, int threads, size_t smem
 template <class... Params, class... Args>
 int launch(void (*kernel)(Params...), dim3 grid, int threads, size_t smem, cudaStream_t st, Args... args) {
     return launch_behind(kernel, grid, threads, smem, st, false, args...);
+}
+
+// More than 48 KB of dynamic shared memory for a kernel, and with `carveout` as much of an SM's memory as can be for it; once per device
+// and kernel (`done`: the attributes belong to the device's copy of the kernel).
+template <class Kernel>
+int allow_smem(Kernel kernel, int smem, bool carveout, std::atomic<unsigned long long>& done) {
+    if (smem <= 48 * 1024 && !carveout) return TRS_OK;
+    int dev = 0;
+    TRS_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = 1ull << (dev & 63);
+    if (dev < 64 && (done.load(std::memory_order_relaxed) & bit)) return TRS_OK;
+    if (smem > 48 * 1024) TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    if (carveout) TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
+    if (dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
+    return TRS_OK;
 }
 
 // D(16x8,f32) += A(16x16 with 2:4 sparsity, stored 16x8 f16) * B(16x8 f16).

@@ -825,14 +825,9 @@ template <int KCH, bool TAIL, bool F32>
 int launch_ring(const trs_sddmm_plan* p, const Operands& o, void* out, int K, cudaStream_t st) {
     using R = SddmmRing<KCH>;
     auto kernel = k_sddmm_tc_ring<KCH, TAIL, F32>;
-    static std::atomic<unsigned long long> done{0};   // per device
-    int dev = 0;
-    TRS_CUDA(cudaGetDevice(&dev));
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (!(done.load(std::memory_order_relaxed) & bit)) {
-        TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, R::SMEM));
-        if (dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
-    }
+    static std::atomic<unsigned long long> done{0};
+    const int rc = allow_smem(kernel, R::SMEM, false, done);
+    if (rc) return rc;
     const RingShares& sh = p->shares.of[KCH - 1];
     const bool table = p->by_table(KCH);
     const int per_warp = ceil_div(p->n_quads, sh.warps);

@@ -1175,26 +1175,12 @@ extern "C" int trs_spmm_launches(const trs_spmm_plan* p) {
     return p->fine.n_heavy > 0 ? 2 : 1;
 }
 
-// Dynamic shared memory of a kernel, and as much of an SM's memory as can be for it; once per device and kernel (`done`: the
-// attributes belong to the device's copy of the kernel).
-template <class Kernel>
-static int allow_smem(Kernel kernel, int smem, std::atomic<unsigned long long>& done) {
-    int dev = 0;
-    TRS_CUDA(cudaGetDevice(&dev));
-    const unsigned long long bit = 1ull << (dev & 63);
-    if (dev < 64 && (done.load(std::memory_order_relaxed) & bit)) return TRS_OK;
-    if (smem > 0) TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
-    TRS_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributePreferredSharedMemoryCarveout, cudaSharedmemCarveoutMaxShared));
-    if (dev < 64) done.fetch_or(bit, std::memory_order_relaxed);
-    return TRS_OK;
-}
-
 template <int FS, int STAGES, int WPI, int MINB, bool ALIGNED, bool RANGE, bool RAGGED>
 static int launch_instance(const KernelArgs& a, int slabs, cudaStream_t st) {
     auto kernel = k_window_spmm_warp<FS, STAGES, WPI, MINB, ALIGNED, RANGE, RAGGED>;
     constexpr int smem = WarpTile<FS, STAGES>::SMEM * WPI;
     static std::atomic<unsigned long long> done{0};
-    const int rc = allow_smem(kernel, smem, done);
+    const int rc = allow_smem(kernel, smem, true, done);
     if (rc) return rc;
     return launch_behind(kernel, dim3(a.n_items, slabs), 32 * WPI, smem, st, a.behind, a);
 }
@@ -1339,7 +1325,7 @@ static int run_impl(const trs_spmm_plan* p, const trs_half* B, void* C, int F, i
             // range may have no item that waits, so it is launched when this has ended.
             a.behind = whole;
             static std::atomic<unsigned long long> done{0};
-            const int rc = allow_smem(k_pad_rows, 0, done);
+            const int rc = allow_smem(k_pad_rows, 0, true, done);
             if (rc) return rc;
             k_pad_rows<<<(unsigned)ceil_div64(pieces, 256), 256, 0, st>>>(a.B, pieces, F, a.bchunks, Bp);
             TRS_LAUNCH_CHECK();
