@@ -83,15 +83,48 @@ def test_part_block_borders(rows):
     _check(rowptr.to(torch.int32), col.to(torch.int32), torch.randn(col.numel(), generator=g), window=7, unit_min_nnz=4)
 
 
-@pytest.mark.parametrize("entries", [12, 600])
+@pytest.mark.parametrize("entries", [12, 20, 40, 100, 200, 500, 600])
 def test_repeated_columns_are_refused(entries):
-    """A column repeated in every row, in a window sorted by a CTA and in a hub window: more entries of one column than the
-    window has rows must not get as far as the records."""
+    """A column repeated in every row, in windows sorted by a warp (up to 64 a row), by a CTA and in a hub window (600): more entries of
+    one column than the window has rows must not get as far as the records."""
     rp = torch.arange(17, dtype=torch.int32) * entries
     col = torch.full((16 * entries,), 5, dtype=torch.int32)
     with pytest.raises(TrsError) as e:
         build_format(rp.cuda(), col.cuda(), torch.ones(16 * entries).cuda())
     assert e.value.code == -8
+
+
+# rows of the window, and the place in the first of them whose column does not ascend
+_ORDERS = {"warp of 8 a lane, inside a lane": ([12] * 16, 3), "warp of 8 a lane, two lanes of a row": ([12] * 16, 8),
+           "warp of 8 a lane, rows that do not fit": ([40] + [10] * 15, 33), "warp of 16 a lane, inside a lane": ([20] * 16, 19),
+           "warp of 16 a lane, two lanes of a row": ([20] * 16, 16), "warp of 32 a lane, inside a lane": ([40] * 16, 31),
+           "warp of 32 a lane, two lanes of a row": ([40] * 16, 32), "CTA of 1024": ([400] + [10] * 15, 256),
+           "CTA of 2048": ([100] * 16, 64), "CTA of 4096": ([200] * 16, 128), "CTA of 8192": ([400] * 16, 399), "hub": ([600] * 16, 300)}
+
+
+@pytest.mark.parametrize("fault", ["repeated", "descending", "negative"])
+@pytest.mark.parametrize("where", _ORDERS)
+@pytest.mark.parametrize("bits", [16, 24])   # 24: keys of 64 bits, which a warp does not sort
+def test_one_column_out_of_order(where, fault, bits):
+    """One entry of one row of the middle one of three windows: refused at every place where a sort looks, and the next build is
+    right."""
+    rows, at = _ORDERS[where]
+    g = torch.Generator().manual_seed(len(rows) * at)
+    per_row = torch.tensor(rows * 3)
+    col = torch.cat([torch.randperm(1 << 12, generator=g)[:k].sort().values + 1 for k in per_row.tolist()]).to(torch.int32)
+    col[-1] = (1 << bits) - 1
+    rowptr = torch.zeros(49, dtype=torch.int32)
+    rowptr[1:] = torch.cumsum(per_row, 0)
+    val = torch.randn(col.numel(), generator=g)
+    bad = col.clone()
+    e = int(rowptr[16]) + at
+    if fault == "negative":
+        e -= at
+    bad[e] = {"repeated": bad[e - 1], "descending": bad[e - 1] - 1, "negative": -1}[fault]
+    with pytest.raises(TrsError) as err:
+        build_format(rowptr.cuda(), bad.cuda(), val.cuda())
+    assert err.value.code == -8
+    _check(rowptr, col, val)
 
 
 def test_entries_without_arrays_are_refused():
