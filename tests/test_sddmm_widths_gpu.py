@@ -141,21 +141,24 @@ def test_windows_beyond_the_entry_lists():
 @pytest.mark.parametrize("shape", ["hubs first", "hubs last", "even", "one window"])
 def test_shares_of_equal_cost(shape, K):
     """Patterns whose quads cost the same (equal numbers per warp) and very different amounts (a table of first quads): every
-    entry is written once, whichever warp has it."""
+    entry is written once, whichever warp has it.  The plan says which of the two it is."""
     g = torch.Generator().manual_seed(K)
-    n, m = (16, 60000) if shape == "one window" else (24000, 6000)
+    n, m = (16, 60000) if shape == "one window" else (240000, 6000)
     if shape == "one window":
         rows, cols = torch.randint(0, n, (400000,), generator=g), torch.randint(0, m, (400000,), generator=g)
     else:
         rows, cols = torch.arange(n).repeat_interleave(9), torch.randint(0, m, (9 * n,), generator=g)
         if shape != "even":
-            hub = torch.arange(300) + (n - 300 if shape == "hubs last" else 0)
-            rows = torch.cat([rows, hub.repeat_interleave(2500)])
-            cols = torch.cat([cols, torch.randint(0, m, (300 * 2500,), generator=g)])
-    rp, col = (t.cuda() for t in graphs.coo_to_csr(rows, cols, n, m)[:2])
+            hub = torch.arange(1600) + (n - 1600 if shape == "hubs last" else 0)
+            rows = torch.cat([rows, hub.repeat_interleave(m)])
+            cols = torch.cat([cols, torch.arange(m).repeat(1600)])
+    rp, col = graphs.coo_to_csr(rows.cuda(), cols.cuda(), n, m)[:2]
     X, Y = torch.randn(n, K, generator=g).half().cuda(), torch.randn(m, K, generator=g).half().cuda()
     r = torch.repeat_interleave(torch.arange(n, device="cuda"), (rp[1:] - rp[:-1]).long())
-    out = SddmmPlan(rp, col, m).run(X, Y, out=torch.full((col.numel(),), float("nan"), dtype=torch.float16, device="cuda")).float()
+    plan = SddmmPlan(rp, col, m)
+    warps, number, cost, table = _shares(plan, K)
+    assert table == shape.startswith("hubs") and (number > 1.5 * cost) == table, (warps, number, cost)
+    out = plan.run(X, Y, out=torch.full((col.numel(),), float("nan"), dtype=torch.float16, device="cuda")).float()
     ref = torch.empty_like(out)
     for a in range(0, col.numel(), 1 << 18):
         ref[a:a + (1 << 18)] = (X[r[a:a + (1 << 18)]].float() * Y[col[a:a + (1 << 18)].long()].float()).sum(1)
@@ -164,9 +167,9 @@ def test_shares_of_equal_cost(shape, K):
 
 
 def test_row_pointer_ends():
-    """What the product's kernel says about the ends of the row pointers: errors, no entries, calls from several threads and
-    streams at a time."""
-    import threading
+    """What the product's kernel says about the ends of the row pointers: errors, no entries, and calls from several threads and
+    streams at a time, each of which gets what its own row pointers say."""
+    from concurrent.futures import ThreadPoolExecutor
     rp, col = (t.cuda() for t in _pattern("rmat"))
     X = torch.randn(1024, 64, generator=torch.Generator().manual_seed(2)).half().cuda()
     want = sddmm(rp, col, X, X)
@@ -175,20 +178,28 @@ def test_row_pointer_ends():
             sddmm(bad, col, X, X)
         assert e.value.code == -3
     assert sddmm(torch.zeros_like(rp), col[:0], X, X).numel() == 0
-    failed = []
+    own = []   # threads 0, 3: the whole pattern; 1, 4: its first rows; 2, 5: row pointers that are an error
+    for k in range(6):
+        rows = 1024 if k % 3 == 0 else 100 + k
+        own.append((rp[:rows + 1] + (1 if k % 3 == 2 else 0), X[:rows], want[:int(rp[rows])]))
 
     def calls(k):
+        ptr, x, mine = own[k]
         with torch.cuda.stream(torch.cuda.Stream()):
             torch.cuda._sleep(100000 * k)
-            for _ in range(50):
-                if not torch.equal(sddmm(rp, col, X, X), want):
-                    failed.append(k)
+            for i in range(50):
+                try:
+                    got = sddmm(ptr, col, x, X, out=torch.zeros_like(want))
+                except TrsError as e:
+                    if k % 3 != 2 or e.code != -3:
+                        raise
+                else:
+                    assert k % 3 != 2 and torch.equal(got[:mine.numel()], mine) and not got[mine.numel():].any()
+        return i + 1
 
-    threads = [threading.Thread(target=calls, args=(k,)) for k in range(6)]
     torch.cuda.synchronize()
-    [t.start() for t in threads]
-    [t.join() for t in threads]
-    assert not failed
+    with ThreadPoolExecutor(6) as pool:
+        assert list(pool.map(calls, range(6))) == [50] * 6
 
 
 def _runtime():
