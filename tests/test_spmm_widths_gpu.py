@@ -185,7 +185,7 @@ def test_first_column_ids(F, per_row):
     assert float((out - ref).abs().max()) <= 2e-5 * float(ref.abs().max())
 
 
-@pytest.mark.parametrize("windows", [1 << 16, 1 << 19])
+@pytest.mark.parametrize("windows", [1 << 16, 1 << 20])
 def test_plan_without_room_for_first_column_ids(windows):
     """A plan fits where its arrays fit: the ids beside the items (512 bytes an item, more than the rest of this plan) are left out,
     and the results are the same."""

@@ -951,10 +951,11 @@ static int validate_on_device(const trs_format& f, int m_rows, int k_cols, int n
     return TRS_OK;
 }
 
-// First ids beside the items take 512 bytes an item.  Nobody is to miss that room: beyond 32 MB they are left out where they would be more
-// than a sixteenth of what the device has left (asking for that takes 60 us, a plan of 9000 rows 190), and no plan fails for want of them.
+// First ids beside the items take 512 bytes an item.  Nobody is to miss that room: beyond 256 MB (8 M rows) they are left out where they
+// would be more than a sixteenth of what the device has left, and no plan fails for want of them.  Asking for that takes 60 to 150
+// us, so smaller ones are not asked for (plans of 9000 rows / R-MAT 20 with the question 250 / 1250 us, without 190 / 1060).
 static bool room_for_first_ids(size_t bytes) {
-    if (bytes <= (size_t)32 << 20) return true;
+    if (bytes <= (size_t)256 << 20) return true;
     size_t left = 0, total = 0;
     if (cudaMemGetInfo(&left, &total) != cudaSuccess) { (void)cudaGetLastError(); return false; }
     return bytes <= left / 16;
@@ -1117,9 +1118,10 @@ int trs::spmm_plan_create(const trs_format* dev_format, int m_rows, int k_cols, 
     return TRS_OK;
 } TRS_CATCH
 
-// No kernel of this library waits on a flag or a barrier that another warp or kernel sets (the
-// window kernels synchronise inside one warp or one CTA only), so there is no wait that could
-// give up: the status word is always 0.  Kept for callers of earlier versions.
+// No kernel of this library spins on a flag or a barrier that another kernel sets: the window kernels synchronise inside one warp
+// or one CTA, and what the sums of split windows (and a product behind a copy of B) wait for is the end of the kernel launched before
+// them, which waits for nothing of theirs.  So there is no wait that could give up, and the status word is always 0.  Kept
+// for callers of earlier versions.
 extern "C" int trs_spmm_status(const trs_spmm_plan* p, int* status) {
     if (!p || !status) return TRS_E_ARG;
     *status = 0;
