@@ -529,7 +529,7 @@ def run_ours(args, rank, world, local_rank):
 
 
 def run_sddmm(args):
-    """SDDMM (BASELINE config 3): X, Y dense N x 64 fp16 on the pattern of the chosen workload."""
+    """SDDMM: X, Y dense N x 64 fp16 on the pattern of the chosen workload."""
     from trspmm import sddmm
     dev = torch.device("cuda", 0)
     rp, col, val, _ = make_matrix(args.workload, dev)
@@ -738,7 +738,7 @@ def run_match24(args):
 
 
 def run_gcn(args, rank, world, local_rank):
-    """Two-layer GCN forward (BASELINE config 4 shape): features 256 -> 128 -> 64, ReLU between."""
+    """Two-layer GCN forward: features 256 -> 128 -> 64, ReLU between."""
     import torch.distributed as dist
     from trspmm import ShardedGCN2
     torch.cuda.set_device(local_rank)

@@ -147,9 +147,9 @@ int trs_rows_gemm_bcast(const trs_half* H, const trs_half* W, void* const* dst, 
  * GPU, this one included, so the sender issues each row once whatever the number of ranks. */
 int trs_rows_gemm_mcast(const trs_half* H, const trs_half* W, void* multicast_dst, long long row0, int rows,
                         int K, int N, void* stream);
-/* Health word of the plan's kernels.  No kernel of the library waits on a flag or barrier another
- * warp or kernel sets, so there is no wait that could give up: always 0.  Kept for callers of
- * earlier versions. */
+/* Health word of the plan's kernels.  No kernel of the library spins on a flag or barrier that another
+ * kernel sets (some wait for the end of the kernel launched before them), so there is no wait that could
+ * give up: always 0.  Kept for callers of earlier versions. */
 int trs_spmm_status(const trs_spmm_plan* plan, int* status);
 /* trs_spmm_run for callers that can neither allocate device memory nor be handed any: hosts that
  * gave the whole device to their own memory pool at start-up, and latency-critical loops where
@@ -328,11 +328,11 @@ typedef struct trs_match_stats {
 int trs_match24_stats(int variant, const int32_t* rowptr, const int32_t* col, int n_rows, int window,
                       int dense_threshold, int t_max, void* stream, trs_match_stats* out);
 
-/* ---- SDDMM (no counterpart in the reference; defined by BASELINE config 3) -----------------
+/* ---- SDDMM (no counterpart in the reference) -------------------------------------------------
  * out[e] = fp16( sum_k fp32(X[row(e),k]) * fp32(Y[col(e),k]) ) for every CSR entry e.
- * The call reads rowptr[0] and rowptr[n_rows] back to the host first (one stream synchronise per
- * call; TRS_E_OFFSETS when they are not 0 / non-negative), then launches on `stream`.  The pattern
- * is not validated beyond that: the kernel never reads outside X, Y or rowptr, and an entry whose
+ * The product's kernel tells the host rowptr[0] and rowptr[n_rows] as it begins, and the call waits for
+ * that, so for earlier work of `stream` but not for the product (TRS_E_OFFSETS when they are not 0 /
+ * non-negative: nothing is written then; under capture the call is refused).  The pattern is not validated beyond that: the kernel never reads outside X, Y or rowptr, and an entry whose
  * column lies outside [0, n_cols) comes back as NaN.  Use the plan below for a checked pattern. */
 int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_half* X, const trs_half* Y,
               trs_half* out, int n_rows, int n_cols, int K, void* stream);

@@ -1,6 +1,6 @@
 """The GPU builder pinned at the benchmark sizes, window by window.
 
-BASELINE configs 1, 2 and 4 (clustered N = 262 144, R-MAT scale 21, R-MAT scale 20) are built whole
+The benchmark matrices (clustered N = 262 144, R-MAT scale 21, R-MAT scale 20) are built whole
 on the GPU; the reference's CPU builder cannot do that (its matching is quadratic in the columns
 of a window in time and memory, block_online.cpp:340-352).  Windows are independent
 (block_online.cpp:584-734), so for >= 64 sampled windows per matrix - the 8 heaviest, 8 whose unit

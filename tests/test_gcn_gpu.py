@@ -1,4 +1,4 @@
-"""Two-layer GCN forward (BASELINE config 4 shape, reduced size) against the fp32 CPU expression
+"""Two-layer GCN forward (the benchmark's shape, reduced size) against the fp32 CPU expression
 over the matrix the format encodes; single rank here, two ranks via torchrun when 2 GPUs exist."""
 import os
 import subprocess

@@ -115,7 +115,7 @@ def test_spmm_split_windows_are_deterministic(monkeypatch):
 
 
 def test_spmm_config0_uniform_vs_torch_sparse():
-    """uniform N=4096, F=64.  Checked against the arrays' own meaning (L1) and,
+    """Uniform N=4096, F=64.  Checked against the arrays' own meaning (L1) and,
     on rows without dropped entries, against torch.sparse CSR A.B (L2)."""
     rp, col, val = graphs.uniform_graph(4096, 16, 0)
     n = 4096

@@ -245,15 +245,15 @@ struct WindowOut {
     int* ncol;
 };
 
-// Windows that do not go to kb_sort_warp: one CTA per window of at most CAP entries, everything in shared memory; 12 bytes read and 4 + 17 per column written
-// per entry.  The rows of a window are sorted already, so four rounds merge them two by two: a thread finds where its
+// Windows that do not go to kb_sort_warp: one CTA per window of at most CAP entries, everything in shared memory; 12 bytes read
+// and 4 + 17 per column written per entry.  The rows of a window are sorted already, so four rounds merge them two by two: a thread finds where its
 // outputs begin by binary search along the diagonal (merge path) and then takes them one by one.  A record's place in the
 // (count desc, column asc) order is counted, not sorted.
 //
 // What bounds it: issue and the shared-memory pipe.  Device-wide sorts of (window, column) keys with their key, head and
 // record passes moved ten times the bytes: 0.69 of the 1.30 ms of a build of the clustered graph.  A radix sort of the block
-// instead of the merge took 262 us there whatever its digits, a merge with a binary search per entry and round 305; this
-// takes 201 (windows of 780 entries), and 32 in place of 53 on windows of 510.
+// instead of the merge took 262 us on its windows of 780 entries whatever its digits, a merge with a binary search per entry and
+// round 305, this 201 (a warp, where they go now, 151), and 32 in place of 53 on windows of 510.
 template <int T, int CAP, class Key>
 struct WindowSort {
     static constexpr int PB = CAP <= 256 ? 8 : CAP <= 512 ? 9 : CAP <= 1024 ? 10 : CAP <= 2048 ? 11 : CAP <= 4096 ? 12 : 13;   // bits of a place in the window

@@ -36,7 +36,7 @@ def sddmm(rowptr: torch.Tensor, col: torch.Tensor, X: torch.Tensor, Y: torch.Ten
 class SddmmPlan:
     """trs_sddmm_plan_*: a CSR pattern prepared once for many SDDMMs.  The plan groups the entries
     by (16-row window, column) so that every distinct Y row of a window is gathered once and the
-    dot products run on the tensor cores (K = 32, 64, 128); other K fall back to the entry-parallel
+    dot products run on the tensor cores (K up to 256); wider ones run the entry-parallel
     kernel.  `rowptr` / `col` (canonical CSR, int32, CUDA) are kept alive by the plan."""
 
     def __init__(self, rowptr: torch.Tensor, col: torch.Tensor, n_cols: int):
