@@ -332,8 +332,9 @@ int trs_match24_stats(int variant, const int32_t* rowptr, const int32_t* col, in
  * out[e] = fp16( sum_k fp32(X[row(e),k]) * fp32(Y[col(e),k]) ) for every CSR entry e.
  * The product's kernel tells the host rowptr[0] and rowptr[n_rows] as it begins, and the call waits for
  * that, so for earlier work of `stream` but not for the product (TRS_E_OFFSETS when they are not 0 /
- * non-negative: nothing is written then; under capture the call is refused).  The pattern is not validated beyond that: the kernel never reads outside X, Y or rowptr, and an entry whose
- * column lies outside [0, n_cols) comes back as NaN.  Use the plan below for a checked pattern. */
+ * non-negative: nothing is written then; under capture the call is refused).  The pattern is not
+ * validated beyond that: the kernel never reads outside X, Y or rowptr, and an entry whose column
+ * lies outside [0, n_cols) comes back as NaN.  Use the plan below for a checked pattern. */
 int trs_sddmm(const int32_t* rowptr, const int32_t* col, const trs_half* X, const trs_half* Y,
               trs_half* out, int n_rows, int n_cols, int K, void* stream);
 /* Planned SDDMM for a pattern that is used many times (training epochs): the plan groups the
